@@ -219,7 +219,7 @@ int linear(const lcc_seq_model* m, const void* x, int ldx, const void* W, const 
            bool y_f32, int M, int N, int K, cudaStream_t s, const void* bias_st = nullptr, int act = lcc::ACT_NONE) {
     const int Np = m->d.rows_padded8 ? ld8(N) : N;
     if (act != lcc::ACT_NONE && bias) return -2;
-    if (m->use_tc && m->d.dtype == LCC_DT_BF16 && (!y_f32 || (!bias && act == lcc::ACT_NONE)) && (!bias || bias_st) && M >= 16 &&
+    if (m->use_tc && m->d.dtype == LCC_DT_BF16 && (!y_f32 || (!bias && act == lcc::ACT_NONE)) && (!bias || bias_st) && M > 8 &&
         (Np >= 32 || y_f32) && K >= 64 && (K % 8) == 0 && (Np % 8) == 0 && ldy >= Np && (ldx % 8) == 0 && (ldy % 8) == 0 &&
         ((uintptr_t)x % 16) == 0 && ((uintptr_t)y % 16) == 0) {   // (a slice of a wider row may start anywhere)
         lcc::GemmArgs a;
@@ -950,7 +950,9 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
     if (n_want > 0) {
         const lcc::NormSpec fn{d.norm_kind, d.final_norm_f32, d.final_norm_bias_f32, d.final_norm_alpha, d.eps};
         STEP(lcc::gather_norm(dt, hc ? xsum : x32, want_rows, fn, xf, n_want, W, s), "final norm");
-        STEP(lcc::linear_any(dt, xf, W, d.head, W, nullptr, logits, d.vocab, true, n_want, d.vocab, W, s), "output head");
+        // scored prompts ask for many rows: the head is then a product like any other. 128 rows x 32768 outputs of width 2048: 648 us
+        // as CUDA-core tiles; decode steps (up to 8 rows) keep the weight-streaming kernel, which `linear` falls back to.
+        STEP(linear(m, xf, W, d.head, nullptr, logits, d.vocab, true, n_want, d.vocab, W, s), "output head");
         STEP(lcc::softcap(logits, (int64_t)n_want * d.vocab, d.logit_softcap, s, d.logit_scale != 0.f ? d.logit_scale : 1.f), "logit soft cap / scale");
         if (logits_copy &&
             cudaMemcpyAsync(logits_copy, logits, (size_t)n_want * d.vocab * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess)

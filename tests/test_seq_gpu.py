@@ -380,3 +380,27 @@ def test_trace_replay_command_line(tmp_path):
     g2 = torch.from_numpy(np.fromfile(out / "2.f32", dtype="<f4")).reshape(1, -1)
     g3 = torch.from_numpy(np.fromfile(out / "3.f32", dtype="<f4")).reshape(1, -1)
     assert rel(g0, la[[0, 32]]) < F32_TOL and rel(g2, la[[49]]) < F32_TOL and rel(g3, lb[[6]]) < F32_TOL
+
+
+@pytest.mark.parametrize("vocab", [32, 200, 203])
+@pytest.mark.parametrize("rows", [9, 16, 17, 64, 129, 257])
+def test_output_head_for_many_rows_equals_the_head_row_by_row(vocab, rows):
+    """Scored prompts ask for many rows of logits at once (a tensor-core product where the shapes allow it), decode steps for one (the
+    weight-streaming kernel). Both multiply the same bf16 rows and add in fp32: they differ by the order of 72 sums at most."""
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    d = seq_cases.config([seq_cases.ssd(heads=2, vdim=8, state=8, groups=1)], width=72, vocab=vocab, softcap=0.0)
+    m = SeqLMForCausalLM.from_state_dict(SeqModelConfig.from_json(d), synthetic_seq_tensors(SeqModelConfig.from_json(d), seed=3), "bfloat16")
+    toks = seq_cases.tokens(rows, vocab, seed=rows)
+
+    def logits(want):
+        c = m.new_cache()
+        out = m.forward_step([(c, toks)], [want])
+        c.release()
+        return out
+
+    many = logits(list(range(rows)))
+    for k in (0, rows // 2, rows - 1):
+        one = logits([k])[0]
+        # |sum| <= 72 products of |normed row| (rms 1, weight <= 1.25) and |head| (unit rows): order changes it by 72 * 2^-24 of their sum
+        assert (many[k] - one).abs().max() <= 72 * 2.0 ** -23 * 1.25 * 72 ** 0.5, (k, float((many[k] - one).abs().max()))
