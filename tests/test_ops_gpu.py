@@ -377,3 +377,39 @@ def test_embed_gather_never_reads_past_the_video_rows(ctx):
     out2, rank2 = ctx.embed_gather(ids, table, None, vid)
     torch.cuda.synchronize()
     assert torch.equal(out2, table[ids]) and int(rank2[ids.numel()]) == 0
+
+
+@pytest.mark.parametrize("V", [1, 7, 8191, 32768 + 5, 152064])
+@pytest.mark.parametrize("hist", [0, 1, 8193, 70001])
+def test_sample_greedy_sizes(ctx, V, hist):
+    """The selection is shared out over the CTAs of a cluster: vocabularies smaller than a CTA, remainders behind the 4-wide part,
+    histories from none to several passes, ties whose copies lie in different CTAs (the lowest index wins), the threshold's sum."""
+    g = torch.Generator(device=DEV).manual_seed(V + hist)
+    raw = torch.randn(V, device=DEV, generator=g)
+    ties = torch.randint(0, V, (4,), device=DEV, generator=g)
+    raw[ties] = 9.0
+    ids = torch.randint(0, V, (hist,), device=DEV, generator=g)
+    ids[ids == ties.min()] = (int(ties.min()) + 1) % V if V > 1 else 0
+    seq = torch.zeros(hist + 2, dtype=torch.int64, device=DEV)
+    seq[:hist] = ids
+    ref = raw.clone()
+    s = ref[ids]
+    ref[ids] = torch.where(s < 0, s * 1.25, s * 0.8)
+    for thr in (-1, int(ref.argmax())):
+        sc = torch.zeros(A.SC_COUNT, dtype=torch.int32, device=DEV)
+        sc[A.SC_SEQ_LEN] = hist
+        want = ref.clone()
+        if thr >= 0:      # the share of the best token lies between the two bases
+            share = float(torch.softmax(ref.double(), 0)[thr])
+            for base, masked in ((share * 0.999, False), (share * 1.001, True)):
+                proc, sc2 = raw.clone(), sc.clone()
+                ctx.sample_greedy(raw, proc, seq, sc2, A.Sampling(1.25, thr, base, 0.0, -1, 16, 0.8, -1), 0, torch.zeros((V, 8), dtype=torch.bfloat16, device=DEV),
+                                  torch.zeros(8, dtype=torch.bfloat16, device=DEV))
+                assert bool(torch.isinf(proc[thr])) == masked
+            continue
+        proc = raw.clone()
+        ctx.sample_greedy(raw, proc, seq, sc, A.Sampling(1.25, -1, 0.0, 0.0, -1, 16, 0.8, -1), 1, torch.zeros((V, 8), dtype=torch.bfloat16, device=DEV),
+                          torch.zeros(8, dtype=torch.bfloat16, device=DEV))
+        assert torch.equal(proc, want)
+        assert int(seq[hist]) == int((want == want.max()).nonzero()[0])
+        assert sc.tolist()[:6] == [1, 1, 0, 1, hist + 1, int(seq[hist])]
