@@ -258,36 +258,312 @@ __global__ void __launch_bounds__(128) attn_chunk_sink_kernel(const float* __res
     }
 }
 
-// Few rows over many keys (decode steps of plain causal attention, where the window is the whole sequence and, in a
-// replayed step, only the device knows its length): one CTA per (row, head, split). The CTA walks key tiles split,
-// split + n_splits, ... of kSplitKeys keys each (so any length works with any grid; the grid only sets the parallelism), keeps
-// the running (max, sum, output) over its tiles, and leaves them in the workspace; the CTA that arrives last at the
-// (row, head) counter merges the splits with the sink's term, applies the gate and writes the row. The counter goes back to
-// zero for the next launch. With two maps per head (opt.maps = 2) the grid has one CTA per (row, head, map, split), the
-// counter is the head's, and the last CTA merges both maps and writes their normed difference.
-// Keys are numbered as the row sees them: the kept first positions, then the window's.
-constexpr int kSplitKeys = 128, kSplitMaxOut = 4;   // output channels per thread: DV <= 128 * kSplitMaxOut
+// Few rows (decode steps, portions of fewer than kAttnTiledMin rows), 16-byte aligned head rows: one CTA per (row, group of up to HB
+// heads of one key/value head, key split). What bounds a step of one row is latency and, where heads share keys, reading them once per
+// head: so a K or V element is loaded once for all HB heads, straight into registers, and a tile of 32 keys costs one round trip to
+// the pages. Eight warps take 4 keys each: eight lanes per key form its HB scores, a warp per head runs the softmax over the tile,
+// then every lane adds its 16-byte pieces of its keys' value rows into HB running outputs. A CTA walks the tiles
+// split, split + n_splits, ... (any length works with any grid) and leaves (out, max, sum) per head in the workspace; the CTA
+// that arrives last at the row's counter merges the splits with the sink's term, applies the gate or takes the maps' difference, and
+// puts the counter back to zero. One split writes the row itself. A decode
+// step of 16 heads over 2 key/value heads of 128 channels, 130 to 160 keys: with a CTA per (row, head) and a chain of loads per key the
+// two attention layers of a 32-token generation cost 1.0 ms more (7.36 -> 6.34 ms), one layer with a sink 0.8 ms (11.73 -> 10.93 ms).
+// Keys are numbered as the row sees them: the kept first positions, then the window's or the chunk's.
 // The arrival counters take a fixed area at the head of the workspace, whatever the row and head counts of a call: partials
 // of one call must never lie where another call (a layer with other sizes) keeps its counters.
+constexpr int kRowKeys = 32, kRowSplitsMax = 64, kRowDvMax = 512, kRowSmem = 160 * 1024;
 constexpr int kSplitMaxHeads = 512, kSplitCounters = (kAttnTiledMin - 1) * kSplitMaxHeads;
+constexpr int row_part_stride(int DV) { return (DV + 3) / 4 * 4 + 4; }   // [out: DV | max | sum], 16-byte steps
 template <typename T> struct RowVec;
 template <> struct RowVec<bf16> {
     static constexpr int N = 8;
-    static __device__ __forceinline__ void load(const bf16* p, float (&v)[8]) {
-        const uint4 u = *reinterpret_cast<const uint4*>(p);
+    static __device__ __forceinline__ void unpack(const uint4& u, float (&v)[8]) {
         const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
         v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
     }
 };
 template <> struct RowVec<float> {
     static constexpr int N = 4;
-    static __device__ __forceinline__ void load(const float* p, float (&v)[4]) {
-        const float4 u = *reinterpret_cast<const float4*>(p);
-        v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+    static __device__ __forceinline__ void unpack(const uint4& u, float (&v)[4]) {
+        v[0] = __uint_as_float(u.x); v[1] = __uint_as_float(u.y); v[2] = __uint_as_float(u.z); v[3] = __uint_as_float(u.w);
     }
 };
+// shared memory of attn_rows_kernel in floats: queries, scores, weights, corrections | cross-warp outputs | merge weights
+inline size_t row_smem_floats(int HB, int D, int DV) {
+    return (size_t)HB * D + 2 * HB * kRowKeys + 4 * HB + (size_t)8 * HB * DV + (size_t)HB * DV + 2 * (size_t)kRowSplitsMax * HB;
+}
 
-template <typename T, bool VEC>
+// PL: lanes that share a value row (a piece = 16 bytes each), NP: pieces per lane (DV <= PL * NP * RowVec<T>::N).
+template <typename T, int HB, int PL, int NP>
+__global__ void __launch_bounds__(256) attn_rows_kernel(const float* __restrict__ q, const T* __restrict__ k_pages,
+                                                        const T* __restrict__ v_pages, const int* __restrict__ page_table, int page_size,
+                                                        const T* __restrict__ gate, int ld_gate, T* __restrict__ out, int ld_out, int S,
+                                                        int Hq, int G, int D, int DV, int chunk, float scale, SeqPos pos,
+                                                        const float* __restrict__ sink, int ld_v, float* __restrict__ part,
+                                                        int* __restrict__ counters, AttnOpts opt) {
+    if (seq_done(pos)) return;
+    constexpr int VN = RowVec<T>::N, NVK = 4 * PL / 32;   // value keys per lane: a warp's 4 keys over 32 / PL lane groups
+    extern __shared__ __align__(16) float sm[];
+    __shared__ int last_flag;
+    float* sq = sm;                              // [HB][D]
+    float* sc = sq + HB * D;                     // [HB][kRowKeys]
+    float* pw = sc + HB * kRowKeys;              // [kRowKeys][HB]
+    float* corr_s = pw + HB * kRowKeys;          // [HB]
+    float* m_s = corr_s + HB;                    // [HB] running maximum, then the merged one
+    float* l_s = m_s + HB;                       // [HB] running sum, then 1 / merged sum
+    float* osum = l_s + 2 * HB;                  // [8][HB][DV]
+    float* fin = osum + (size_t)8 * HB * DV;     // [HB][DV]
+    float* wm = fin + (size_t)HB * DV;           // [kRowSplitsMax][HB] split maxima, then weights
+    float* wl = wm + kRowSplitsMax * HB;         // [kRowSplitsMax][HB] split sums
+    const int t = blockIdx.y, z = blockIdx.z, nz = gridDim.z;
+    const int per = Hq / G, groups = (per + HB - 1) / HB;        // (Hq counts the maps too)
+    const int g = blockIdx.x / groups, h0 = g * per + (blockIdx.x % groups) * HB, nh = min(HB, per - (blockIdx.x % groups) * HB);
+    const int npos = seq_past(pos, S) + t + 1;
+    const int kfirst = first_key(npos - 1, chunk, opt.window), nkeep = min(opt.keep_first, kfirst), nkeys = npos - kfirst + nkeep;
+    const int ld_k = D * opt.maps;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, l8 = lane & 7;
+    const float inv_cap = opt.softcap > 0.f ? 1.f / opt.softcap : 0.f;
+    const float* brow = opt.bias && l8 < nh ? opt.bias + (size_t)((h0 + l8) / opt.maps) * opt.bias_len : nullptr;
+    for (int i = threadIdx.x; i < HB * D; i += 256) sq[i] = i / D < nh ? q[((size_t)t * Hq + h0) * D + i] * scale : 0.f;
+    float m = -INFINITY, l = 0.f;                // warp h: head h's running maximum and sum
+    float ov[NP][VN][HB] = {};
+    const int PD = D / VN, PDV = DV / VN;
+    __syncthreads();
+    for (int k0 = z * kRowKeys; k0 < nkeys; k0 += nz * kRowKeys) {
+        const int jk = k0 + warp * 4 + (lane >> 3), jc = min(jk, nkeys - 1);
+        const int pj = jc < nkeep ? jc : kfirst + jc - nkeep;
+        const int row = (int)(((size_t)page_table[pj / page_size] * G + g) * page_size + pj % page_size);
+        const T* kr = k_pages + (size_t)row * ld_k;
+        // the first four pieces of the key row per lane, and all of the lane's value pieces, in flight together. The two maps of a
+        // head read different halves of the key row: with maps the lane's pieces are those of map 0, map 1's follow below.
+        uint4 kq[4], vq[NVK][NP];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int p = l8 + 8 * u;
+            kq[u] = p < PD ? ld_stream16(kr + p * VN) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int it = 0; it < NVK; ++it) {
+            const int vrow = __shfl_sync(0xffffffffu, row, (it * (32 / PL) + lane / PL) * 8);
+#pragma unroll
+            for (int n = 0; n < NP; ++n) {
+                const int c = lane % PL + PL * n;
+                vq[it][n] = c < PDV ? ld_stream16(v_pages + (size_t)vrow * ld_v + c * VN) : make_uint4(0, 0, 0, 0);
+            }
+        }
+        float acc[HB];
+#pragma unroll
+        for (int h = 0; h < HB; ++h) acc[h] = 0.f;
+        auto dots = [&](const uint4& kw, int p, int first, int step) {   // heads first, first + step, ... against one piece
+            float kv[VN];
+            RowVec<T>::unpack(kw, kv);
+#pragma unroll
+            for (int h = 0; h < HB; ++h) {
+                if (step == 2 && (h & 1) != first) continue;
+                const float4* sp = reinterpret_cast<const float4*>(sq + h * D + p * VN);
+#pragma unroll
+                for (int i = 0; i < VN / 4; ++i) {
+                    const float4 w = sp[i];
+                    acc[h] = fmaf(w.x, kv[4 * i], fmaf(w.y, kv[4 * i + 1], fmaf(w.z, kv[4 * i + 2], fmaf(w.w, kv[4 * i + 3], acc[h]))));
+                }
+            }
+        };
+        if (opt.maps == 1) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (l8 + 8 * u < PD) dots(kq[u], l8 + 8 * u, 0, 1);
+            for (int p = l8 + 32; p < PD; p += 8) dots(ld_stream16(kr + p * VN), p, 0, 1);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (l8 + 8 * u < PD) dots(kq[u], l8 + 8 * u, 0, 2);
+            for (int p = l8 + 32; p < PD; p += 8) dots(ld_stream16(kr + p * VN), p, 0, 2);
+            for (int p = l8; p < PD; p += 8) dots(ld_stream16(kr + D + p * VN), p, 1, 2);
+        }
+        float mine = 0.f;
+#pragma unroll
+        for (int h = 0; h < HB; ++h) {
+            float v = acc[h];
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            v += __shfl_xor_sync(0xffffffffu, v, 4);
+            if (l8 == h) mine = v;
+        }
+        if (l8 < nh) {
+            if (opt.softcap > 0.f) mine = soft_cap(mine, opt.softcap, inv_cap);
+            if (brow) mine += bias_at(brow, opt.bias_len, npos - 1 - pj);
+            sc[l8 * kRowKeys + warp * 4 + (lane >> 3)] = jk < nkeys ? mine : -INFINITY;
+        }
+        __syncthreads();
+        if (warp < HB) {
+            if (warp < nh) {
+                const float sv = sc[warp * kRowKeys + lane];
+                const float mn = fmaxf(m, warp_max(sv));          // the tile holds a key: finite
+                const float corr = expf(m - mn), p = expf(sv - mn);   // exp(-inf) = 0 on the first tile and on absent keys
+                l = fmaf(l, corr, warp_sum(p));
+                m = mn;
+                pw[lane * HB + warp] = p;
+                if (lane == 0) corr_s[warp] = corr;
+            } else {
+                pw[lane * HB + warp] = 0.f;
+                if (lane == 0) corr_s[warp] = 1.f;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < HB; ++h) {
+            const float c = corr_s[h];
+#pragma unroll
+            for (int n = 0; n < NP; ++n)
+#pragma unroll
+                for (int i = 0; i < VN; ++i) ov[n][i][h] *= c;
+        }
+#pragma unroll
+        for (int it = 0; it < NVK; ++it) {
+            const float* wk = pw + (warp * 4 + it * (32 / PL) + lane / PL) * HB;
+            float w[HB];
+#pragma unroll
+            for (int h = 0; h < HB; ++h) w[h] = wk[h];
+#pragma unroll
+            for (int n = 0; n < NP; ++n) {
+                float vv[VN];
+                RowVec<T>::unpack(vq[it][n], vv);
+#pragma unroll
+                for (int i = 0; i < VN; ++i)
+#pragma unroll
+                    for (int h = 0; h < HB; ++h) ov[n][i][h] = fmaf(w[h], vv[i], ov[n][i][h]);
+            }
+        }
+    }
+    // the warps' sums, then one value per (head, channel)
+#pragma unroll
+    for (int n = 0; n < NP; ++n) {
+        const int c = (lane % PL + PL * n) * VN;
+#pragma unroll
+        for (int i = 0; i < VN; ++i)
+#pragma unroll
+            for (int h = 0; h < HB; ++h) {
+                float v = ov[n][i][h];
+#pragma unroll
+                for (int o = PL; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane < PL && c < DV) osum[((size_t)warp * HB + h) * DV + c + i] = v;
+            }
+    }
+    if (warp < nh && lane == 0) { m_s[warp] = m; l_s[warp] = l; }
+    __syncthreads();
+    const int stride = row_part_stride(DV);
+    for (int i = threadIdx.x; i < nh * DV; i += 256) {
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += osum[(size_t)w * HB * DV + i];
+        if (nz == 1) fin[i] = v;
+        else part[(((size_t)t * Hq + h0 + i / DV) * nz + z) * stride + i % DV] = v;
+    }
+    if (nz > 1) {
+        if (threadIdx.x < nh) {
+            float* mine = part + (((size_t)t * Hq + h0 + threadIdx.x) * nz + z) * stride + stride - 4;
+            mine[0] = m_s[threadIdx.x]; mine[1] = l_s[threadIdx.x];
+        }
+        __threadfence();
+        __syncthreads();
+        int* counter = counters + t * gridDim.x + blockIdx.x;
+        if (threadIdx.x == 0) last_flag = atomicAdd(counter, 1) == nz - 1;
+        __syncthreads();
+        if (!last_flag) return;
+        __threadfence();
+        if (threadIdx.x == 0) *counter = 0;
+        for (int i = threadIdx.x; i < nz * nh; i += 256) {
+            const float* src = part + (((size_t)t * Hq + h0 + i % nh) * nz + i / nh) * stride + stride - 4;
+            wm[(i / nh) * HB + i % nh] = __ldcg(src);
+            wl[(i / nh) * HB + i % nh] = __ldcg(src + 1);
+        }
+    } else if (threadIdx.x < nh) {
+        wm[threadIdx.x] = m_s[threadIdx.x]; wl[threadIdx.x] = l_s[threadIdx.x];
+    }
+    __syncthreads();
+    if (warp < nh) {   // warp h: the splits' weights and the merged sum, with the sink's term (weight in the denominator, no value)
+        const float sk = opt.no_sink ? -INFINITY : (sink ? sink[h0 + warp] : 0.f);
+        float mt = sk;
+        for (int i = lane; i < nz; i += 32) mt = fmaxf(mt, wm[i * HB + warp]);
+        mt = warp_max(mt);                        // split 0 holds the row's first key: finite
+        float lt = 0.f;
+        for (int i = lane; i < nz; i += 32) {
+            const float w = expf(wm[i * HB + warp] - mt);
+            wm[i * HB + warp] = w;
+            lt = fmaf(wl[i * HB + warp], w, lt);
+        }
+        lt = warp_sum(lt) + expf(sk - mt);
+        if (lane == 0) l_s[warp] = 1.f / lt;
+    }
+    __syncthreads();
+    // (with one split a thread reads what it left itself)
+    for (int i = threadIdx.x; i < nh * DV; i += 256) {
+        const int h = i / DV, c = i % DV;
+        float v = 0.f;
+        if (nz == 1) v = fin[i] * wm[h];
+        else {
+            const float* src = part + ((size_t)t * Hq + h0 + h) * nz * stride + c;
+#pragma unroll 8
+            for (int k = 0; k < nz; ++k) v = fmaf(__ldcg(src + (size_t)k * stride), wm[k * HB + h], v);
+        }
+        v *= l_s[h];
+        if (opt.maps == 2) { fin[i] = v; continue; }
+        const float gv = gate ? gate_of(gate, ld_gate, t, h0 + h, c, DV, opt.gate_channel) : 1.f;
+        stf(out + (size_t)t * ld_out + (size_t)(h0 + h) * DV + c, v * gv);
+    }
+    if (opt.maps != 2) return;
+    __syncthreads();
+    if (warp < nh / 2) {   // both maps of a head lie here: o = a1 - lambda a2, brought to unit rms over the head's channels, times the scale
+        const float* a1 = fin + (size_t)2 * warp * DV;
+        float ss = 0.f;
+        for (int c = lane; c < DV; c += 32) { const float v = fmaf(-opt.lambda, a1[DV + c], a1[c]); ss = fmaf(v, v, ss); }
+        const float rn = opt.diff_scale / sqrtf(warp_sum(ss) / (float)DV + opt.eps);
+        for (int c = lane; c < DV; c += 32)
+            stf(out + (size_t)t * ld_out + (size_t)(h0 / 2 + warp) * DV + c, fmaf(-opt.lambda, a1[DV + c], a1[c]) * rn);
+    }
+}
+
+template <typename T>
+int launch_attn_rows(const float* q, const void* k_pages, const void* v_pages, const int* page_table, int page_size, const void* gate,
+                     int ld_gate, void* out, int ld_out, int S, int Hq, int G, int D, int DV, int chunk, float scale, SeqPos pos,
+                     cudaStream_t s, const float* sink, int ld_v, float* ws, size_t ws_floats, int keys_est, const AttnOpts& opt) {
+    constexpr int VN = RowVec<T>::N;
+    const int per = Hq / G, pieces = DV / VN;
+    const bool wide = DV > 256;                              // 16 running outputs per head and lane: at most 4 heads
+    const int HB = per <= 2 ? 2 : (wide ? 4 : 8);
+    const int ctas = G * ((per + HB - 1) / HB) * S;
+    // splits: a tile of keys per CTA while the SMs have room (about two CTAs each). A replayed step's range grows behind the host's back: at least 8
+    const int tiles = (keys_est + kRowKeys - 1) / kRowKeys;
+    int nz = std::min({pos.kv_len ? std::max(tiles, 8) : tiles, std::max(1, 296 / ctas), kRowSplitsMax});
+    const size_t cnt = kSplitCounters, per_split = (size_t)S * Hq * row_part_stride(DV);
+    nz = std::max(1, (int)std::min<size_t>(nz, ws_floats > cnt ? (ws_floats - cnt) / per_split : 1));
+    const size_t smem = sizeof(float) * row_smem_floats(HB, D, DV);
+    int* counters = reinterpret_cast<int*>(ws);              // zero when the workspace is bound; every launch leaves zeros
+    const dim3 grid(ctas / S, S, nz);
+    count_launch();
+#define LCC_ATTN_ROWS(HBN, PLN, NPN)                                                                                                   do {                                                                                                                                  static SmemAttrOnce once;                                                                                                         if (ensure_dyn_smem(once, attn_rows_kernel<T, HBN, PLN, NPN>, kRowSmem)) return -100;                                             attn_rows_kernel<T, HBN, PLN, NPN><<<grid, 256, smem, s>>>(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,                                                                         (const T*)gate, ld_gate, (T*)out, ld_out, S, Hq, G, D, DV, chunk, scale, pos,                                                                    sink, ld_v, ws + cnt, counters, opt);                              } while (0)
+#define LCC_ATTN_ROWS_HB(PLN, NPN)                                                                                                     do { if (HB == 2) LCC_ATTN_ROWS(2, PLN, NPN); else LCC_ATTN_ROWS(8, PLN, NPN); } while (0)
+    if constexpr (VN == 8) {
+        if (pieces <= 16) LCC_ATTN_ROWS_HB(16, 1);
+        else if (pieces <= 32) LCC_ATTN_ROWS_HB(32, 1);
+        else if (HB == 2) LCC_ATTN_ROWS(2, 32, 2);
+        else LCC_ATTN_ROWS(4, 32, 2);
+    } else {
+        if (pieces <= 32) LCC_ATTN_ROWS_HB(32, 1);
+        else if (pieces <= 64) LCC_ATTN_ROWS_HB(32, 2);
+        else if (HB == 2) LCC_ATTN_ROWS(2, 32, 4);
+        else LCC_ATTN_ROWS(4, 32, 4);
+    }
+#undef LCC_ATTN_ROWS_HB
+#undef LCC_ATTN_ROWS
+    return cudaGetLastError() == cudaSuccess ? 0 : -100;
+}
+
+// The same for head rows without 16-byte alignment, over long or device-known ranges: one CTA per (row, head, split), scalar loads,
+// key tiles of kSplitKeys, thread c owns output channels c, c + 128, ... With two maps per head (opt.maps = 2) the grid has one CTA per
+// (row, head, map, split), the counter is the head's, and the last CTA merges both maps and writes their normed difference.
+constexpr int kSplitKeys = 128, kSplitMaxOut = 4;   // output channels per thread: DV <= 128 * kSplitMaxOut
+template <typename T>
 __global__ void __launch_bounds__(128) attn_split_kernel(const float* __restrict__ q, const T* __restrict__ k_pages,
                                                          const T* __restrict__ v_pages, const int* __restrict__ page_table,
                                                          int page_size, const T* __restrict__ gate, int ld_gate,
@@ -313,10 +589,7 @@ __global__ void __launch_bounds__(128) attn_split_kernel(const float* __restrict
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < D; i += blockDim.x) sq[i] = q[((size_t)t * Hq + h) * D + i] * scale;
     float m = -INFINITY, l = 0.f;
-    float o[kSplitMaxOut] = {};                      // scalar form: thread c owns channels c, c + 128, ...
-    constexpr int VN = VEC ? RowVec<T>::N : 1, NP = VEC ? 128 * kSplitMaxOut / (32 * RowVec<T>::N) : 1;
-    float ov[NP][VN] = {};                           // vector form: a warp's sum over ITS keys of 16-byte pieces lane, lane + 32, ...
-    float* osum = sc + kSplitKeys;                   // [4][DV], vector form only
+    float o[kSplitMaxOut] = {};
     for (int k0 = z * kSplitKeys; k0 < nkeys; k0 += nz * kSplitKeys) {
         const int nk = min(kSplitKeys, nkeys - k0);
         __syncthreads();       // sq is staged; the previous tile's weights are consumed
@@ -329,7 +602,7 @@ __global__ void __launch_bounds__(128) attn_split_kernel(const float* __restrict
         __syncthreads();
         float mx = -INFINITY;
         // a warp takes KG consecutive keys at a time and has all their loads in flight before it sums
-        constexpr int KG = VEC ? 8 : 4;
+        constexpr int KG = 4;
         for (int j0 = warp * KG; j0 < nk; j0 += 4 * KG) {
             const T* kr[KG];
 #pragma unroll
@@ -337,25 +610,12 @@ __global__ void __launch_bounds__(128) attn_split_kernel(const float* __restrict
             float acc[KG];
 #pragma unroll
             for (int j = 0; j < KG; ++j) acc[j] = 0.f;
-            if constexpr (VEC) {
-                constexpr int V = RowVec<T>::N;
-                for (int d = lane * V; d < D; d += 32 * V) {
-                    float kv[KG][V];
+            for (int d = lane; d < D; d += 32) {
+                float kv[KG];
 #pragma unroll
-                    for (int j = 0; j < KG; ++j) RowVec<T>::load(kr[j] + d, kv[j]);
+                for (int j = 0; j < KG; ++j) kv[j] = ldf(kr[j] + d);
 #pragma unroll
-                    for (int j = 0; j < KG; ++j)
-#pragma unroll
-                        for (int i = 0; i < V; ++i) acc[j] = fmaf(sq[d + i], kv[j][i], acc[j]);
-                }
-            } else {
-                for (int d = lane; d < D; d += 32) {
-                    float kv[KG];
-#pragma unroll
-                    for (int j = 0; j < KG; ++j) kv[j] = ldf(kr[j] + d);
-#pragma unroll
-                    for (int j = 0; j < KG; ++j) acc[j] = fmaf(sq[d], kv[j], acc[j]);
-                }
+                for (int j = 0; j < KG; ++j) acc[j] = fmaf(sq[d], kv[j], acc[j]);
             }
 #pragma unroll
             for (int j = 0; j < KG; ++j) {
@@ -382,32 +642,6 @@ __global__ void __launch_bounds__(128) attn_split_kernel(const float* __restrict
         sum = block_sum(sum, red);                  // contains the barrier that publishes sc[]
         l = fmaf(l, corr, sum);
         m = mn;
-        if constexpr (VEC) {
-            // a warp takes eight consecutive keys at a time; its lanes read 16-byte pieces of their value rows, all in flight
-            // together. The four warps' sums are added after the last tile.
-#pragma unroll
-            for (int p = 0; p < NP; ++p)
-#pragma unroll
-                for (int i = 0; i < VN; ++i) ov[p][i] *= corr;
-            for (int j0 = warp * 8; j0 < nk; j0 += 32) {
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    const int c = (lane + 32 * p) * VN;
-                    if (c < DV) {
-                        float vv[8][VN];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) RowVec<T>::load(v_pages + (size_t)row_of[min(j0 + j, nk - 1)] * ld_v + c, vv[j]);
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float wj = j0 + j < nk ? sc[j0 + j] : 0.f;
-#pragma unroll
-                            for (int i = 0; i < VN; ++i) ov[p][i] = fmaf(wj, vv[j][i], ov[p][i]);
-                        }
-                    }
-                }
-            }
-            continue;
-        }
 #pragma unroll
         for (int u = 0; u < kSplitMaxOut; ++u) {
             const int c = threadIdx.x + u * 128;
@@ -429,24 +663,10 @@ __global__ void __launch_bounds__(128) attn_split_kernel(const float* __restrict
     // partials of this split: [max, sum, out[DV]]
     float* mine = part + (((size_t)t * Hq + h) * nz + z) * (DV + 2);
     if (threadIdx.x == 0) { mine[0] = m; mine[1] = l; }
-    if constexpr (VEC) {
-        __syncthreads();                             // the last tile's weights are consumed (osum lies behind them)
 #pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            const int c = (lane + 32 * p) * VN;
-            if (c < DV)
-#pragma unroll
-                for (int i = 0; i < VN; ++i) osum[(size_t)warp * DV + c + i] = ov[p][i];
-        }
-        __syncthreads();
-        for (int c = threadIdx.x; c < DV; c += blockDim.x)
-            mine[2 + c] = (osum[c] + osum[DV + c]) + (osum[2 * DV + c] + osum[3 * DV + c]);
-    } else {
-#pragma unroll
-        for (int u = 0; u < kSplitMaxOut; ++u) {
-            const int c = threadIdx.x + u * 128;
-            if (c < DV) mine[2 + c] = o[u];
-        }
+    for (int u = 0; u < kSplitMaxOut; ++u) {
+        const int c = threadIdx.x + u * 128;
+        if (c < DV) mine[2 + c] = o[u];
     }
     __threadfence();
     __syncthreads();
@@ -1147,7 +1367,7 @@ int qk_norm_kv_append(int dt, const void* proj, int ld, const float* qn_w, const
 }
 
 size_t attn_split_ws_floats(int rows, int Hq, int DV) {
-    return (size_t)kSplitCounters + (size_t)rows * Hq * (DV + 2) * 32;
+    return (size_t)kSplitCounters + (size_t)rows * Hq * row_part_stride(DV) * 32;
 }
 
 int attn_chunk_sink(int dt, const float* q, const void* k_pages, const void* v_pages, const int* page_table,
@@ -1206,6 +1426,16 @@ int attn_masked(int dt, const float* q, const void* k_pages, const void* v_pages
     // few rows without chunks over a long or device-known range of keys: key splits across CTAs
     int keys_est = pos.kv_len ? std::max(key_hint, pos.past + S) : pos.past + S;
     if (window) keys_est = std::min(keys_est, window + keep);
+    static const bool force_tiled = [] { const char* e = getenv("LIVECC_B200_SEQ_ATTN_TILED"); return e && e[0] == '1'; }();
+    if (chunk > 0) keys_est = std::min(keys_est, chunk);
+    const int vn = dt == DT_F32 ? 4 : 8;
+    if (S < kAttnTiledMin && split_ws && split_ws_floats > (size_t)kSplitCounters && DV <= kRowDvMax && Hq <= kSplitMaxHeads &&
+        ((D % vn) | (DV % vn) | (ld_v % vn)) == 0 && (((uintptr_t)k_pages | (uintptr_t)v_pages) % 16) == 0 && !(force_tiled && chunk > 0) &&
+        sizeof(float) * row_smem_floats(Hq / G <= 2 ? 2 : (DV > 256 ? 4 : 8), D, DV) <= (size_t)kRowSmem)
+        return dt == DT_F32 ? launch_attn_rows<float>(q, k_pages, v_pages, page_table, page_size, gate, ld_gate, out, ld_out, S, Hq, G, D, DV, chunk,
+                                                      scale, pos, s, sink, ld_v, split_ws, split_ws_floats, keys_est, o)
+                            : launch_attn_rows<bf16>(q, k_pages, v_pages, page_table, page_size, gate, ld_gate, out, ld_out, S, Hq, G, D, DV, chunk,
+                                                     scale, pos, s, sink, ld_v, split_ws, split_ws_floats, keys_est, o);
     if (chunk <= 0 && S < kAttnTiledMin && split_ws && DV <= 128 * kSplitMaxOut && Hq <= kSplitMaxHeads &&
         ((pos.kv_len && !window) || keys_est > 2 * kSplitKeys || opt.maps == 2)) {
         const size_t per = (size_t)S * Hq * (DV + 2), cnt = kSplitCounters;
@@ -1214,19 +1444,16 @@ int attn_masked(int dt, const float* q, const void* k_pages, const void* v_pages
         if (split_ws_floats > cnt && nz >= 1) {
             int* counters = reinterpret_cast<int*>(split_ws);           // zero when the workspace is bound; every launch leaves zeros
             float* part = split_ws + cnt;
-            const size_t smem = sizeof(float) * ((size_t)D + kSplitKeys + 4 * (size_t)DV);
+            const size_t smem = sizeof(float) * ((size_t)D + kSplitKeys);
             dim3 grid(Hq, S, nz);
             count_launch();
-#define LCC_SPLIT(T, VECB)                                                                                                   \
-    attn_split_kernel<T, VECB><<<grid, 128, smem, s>>>(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size, (const T*)gate,  \
-                                                       ld_gate, (T*)out, ld_out, S, Hq, G, D, DV, scale, pos, sink, ld_v, part, counters, o)
             if (smem > 48 * 1024) return -3;
-            if (dt == DT_F32) {
-                if (((D | DV | ld_v) % 4) == 0 && (((uintptr_t)k_pages | (uintptr_t)v_pages) % 16) == 0) LCC_SPLIT(float, true); else LCC_SPLIT(float, false);
-            } else {
-                if (((D | DV | ld_v) % 8) == 0 && (((uintptr_t)k_pages | (uintptr_t)v_pages) % 16) == 0) LCC_SPLIT(bf16, true); else LCC_SPLIT(bf16, false);
-            }
-#undef LCC_SPLIT
+            if (dt == DT_F32)
+                attn_split_kernel<float><<<grid, 128, smem, s>>>(q, (const float*)k_pages, (const float*)v_pages, page_table, page_size, (const float*)gate,
+                                                                 ld_gate, (float*)out, ld_out, S, Hq, G, D, DV, scale, pos, sink, ld_v, part, counters, o);
+            else
+                attn_split_kernel<bf16><<<grid, 128, smem, s>>>(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, page_size, (const bf16*)gate,
+                                                                ld_gate, (bf16*)out, ld_out, S, Hq, G, D, DV, scale, pos, sink, ld_v, part, counters, o);
             return cudaGetLastError() == cudaSuccess ? 0 : -100;
         }
     }
@@ -1249,7 +1476,6 @@ int attn_masked(int dt, const float* q, const void* k_pages, const void* v_pages
     if (window) max_keys = max_keys > 0 ? std::min(max_keys, window) : window + keep;
     if (!pos.kv_len) max_keys = max_keys > 0 ? std::min(max_keys, pos.past + S) : pos.past + S;
     const size_t smem = sizeof(float) * ((size_t)D + (size_t)std::max(max_keys, 0));
-    static const bool force_tiled = [] { const char* e = getenv("LIVECC_B200_SEQ_ATTN_TILED"); return e && e[0] == '1'; }();
     if (S >= kAttnTiledMin || max_keys < 0 || smem > 160 * 1024 || force_tiled) {
         const bool mma = dt == DT_BF16 && tensor_cores && D <= kAttnMmaMaxDim;
         if (mma && opt.maps == 2 && DV <= 256)

@@ -119,7 +119,7 @@ WsLayout make_layout(const lcc_seq_model* m, int NT, int NW) {
     int wp = 8, wp2 = 8, wm = 8, wy = 8, wq = 8, wf = 8;
     size_t scan_floats = 0;
     int moe_e = 0, moe_top = 0, moe_ff = 0, moe_rows = 0, moe_glu = 0;   // moe_glu: widest hidden row of a gated expert
-    size_t split_floats = 0;   // key-split partials of few-row plain causal attention
+    size_t split_floats = 0;   // key-split partials of few-row attention
     int wvk = 0;
     size_t delta_floats = 0;   // the delta rule's prepared operands (head by head, fp32) share the fp32 query buffer
     for (const lcc_seq_layer& l : m->layers) {
@@ -149,14 +149,13 @@ WsLayout make_layout(const lcc_seq_model* m, int NT, int NW) {
             wq = std::max(wq, l.a_heads * z.a_kd);
             split_floats = std::max(split_floats, lcc::attn_split_ws_floats(lcc::kAttnTiledMin - 1, l.a_heads, l.a_rank));
         }
-        if (l.type == LCC_MIX_PARALLEL && l.l_chunk <= 0)
+        if (l.type == LCC_MIX_PARALLEL)
             split_floats = std::max(split_floats, lcc::attn_split_ws_floats(lcc::kAttnTiledMin - 1, l.l_heads, l.l_vdim));
         if (l.type == LCC_MIX_ATTENTION) {
             wp = std::max(wp, ld8(z.m_proj)); wm = std::max(wm, ld8(z.m_o)); wq = std::max(wq, z.m_nq);
             const int maps = l.m_maps > 1 ? l.m_maps : 1;
             if (maps > 1) wy = std::max(wy, l.m_heads * maps * l.m_vdim);      // the maps' outputs in fp32, where no kernel takes their difference itself
-            if (l.m_chunk <= 0)
-                split_floats = std::max(split_floats, lcc::attn_split_ws_floats(lcc::kAttnTiledMin - 1, l.m_heads * maps, l.m_vdim));
+            split_floats = std::max(split_floats, lcc::attn_split_ws_floats(lcc::kAttnTiledMin - 1, l.m_heads * maps, l.m_vdim));
         }
         if (l.ff_kind == LCC_FF_MOE) {
             const bool glu = l.e_act == LCC_EXPERT_CLAMP_GLU || l.e_act == LCC_EXPERT_SILU_GLU;

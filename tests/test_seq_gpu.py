@@ -404,3 +404,22 @@ def test_output_head_for_many_rows_equals_the_head_row_by_row(vocab, rows):
         one = logits([k])[0]
         # |sum| <= 72 products of |normed row| (rms 1, weight <= 1.25) and |head| (unit rows): order changes it by 72 * 2^-24 of their sum
         assert (many[k] - one).abs().max() <= 72 * 2.0 ** -23 * 1.25 * 72 ** 0.5, (k, float((many[k] - one).abs().max()))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,chunk", [(1, 1, 8, 8, 7), (6, 3, 16, 40, 200), (9, 1, 32, 128, 200), (18, 2, 24, 136, 33), (5, 1, 64, 264, 64),
+                                                           (4, 2, 264, 512, 100)])
+def test_few_row_attention_over_head_groups_and_widths(heads, kv_heads, dim, vdim, chunk, dtype):
+    """Steps of one to three rows: groups of 1 to 9 heads per key/value head (8 at a time, a ragged rest), value rows of one 16-byte piece
+    up to the widest form, key rows longer than the pieces loaded up front, chunks that end inside a tile of 32 keys."""
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    d = seq_cases.config([seq_cases.par(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, chunk=chunk, scale=dim ** -0.5, ff=None)], width=40)
+    cfg = SeqModelConfig.from_json(d)
+    tensors = synthetic_seq_tensors(cfg, seed=5)
+    toks = seq_cases.tokens(102, 96, seed=heads)
+    want, _ = O.forward(d, tensors, toks)
+    m = SeqLMForCausalLM.from_state_dict(cfg, tensors, dtype)
+    cuts = [30, 31, 32, 33, 35, 63, 64, 65, 66, 69, 96, 97, 98, 99, 100, 101]
+    # fp32 storage: the order of sums; bf16: a dozen roundings of 2^-9 on the way from a row to its logits
+    assert rel(run(m, toks, cuts), want) < (2e-5 if dtype == "float32" else 3e-2)
