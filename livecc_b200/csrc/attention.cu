@@ -571,14 +571,24 @@ __device__ __forceinline__ void rope1d_row(const bf16* src, bf16* dst, int lane_
     dst[lane_dim + 64] = f2bf(rbf(rbf(x2 * c) + rbf(x1 * s)));
 }
 
+// The decode kernel's K/V tiles go through kDecBuf shared-memory buffers: while one tile is computed the next two are in flight.
+constexpr int kDecBuf = 3, kDecLds = 136, kDecSmem = (16 + kDecBuf * 2 * 64) * kDecLds * 2;
+
+// CL = 1: `split` of p.nsplit key ranges, the last CTA of a KV group to arrive merges all splits from global memory. CL = 8: the eight
+// CTAs of a cluster hold eight consecutive splits and merge them through their shared memory, one query head each; one partial
+// per cluster goes to global memory, and the last cluster to arrive merges p.nsplit / 8 of them (again one head per CTA). What bounds a
+// step over a short cache is the chain launch -> page -> tile -> merge, over a long one the bytes in flight: with 64 splits of two CTAs per
+// SM and three buffers both get shorter. A merge of 32 partials by one CTA per KV group was the longest link of the chain.
+// 16 tokens of four layers: over 8k tokens 11.20 -> 10.93 ms (4.5 us per launch), over 65k 12.31 -> 11.90 ms (6.8 us).
+template <int CL>
 __device__ __forceinline__ void attn_decode_role(const DecodeAttnParams& p, const int g, const int split,
                                                  uint8_t* smem_attn) {
-    constexpr int D = 128, LDS = D + 8, BN = 64;
+    constexpr int D = 128, LDS = kDecLds, BN = 64;
     pdl_wait();  // qkv of this token comes from the previous kernel
     if (p.finished && *p.finished) return;
     bf16* sq = reinterpret_cast<bf16*>(smem_attn);  // [16][LDS]
-    bf16* sk = sq + 16 * LDS;                        // [2][64][LDS]
-    bf16* sv = sk + 2 * BN * LDS;                    // [2][64][LDS]
+    bf16* sk = sq + 16 * LDS;                        // [kDecBuf][64][LDS]
+    bf16* sv = sk + kDecBuf * BN * LDS;              // [kDecBuf][64][LDS]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = p.Hq / p.Hkv;
     const int kv_old = *p.kv_len;
@@ -590,19 +600,18 @@ __device__ __forceinline__ void attn_decode_role(const DecodeAttnParams& p, cons
     const int tile_begin = split * tiles_per_split;
     const int tile_end = min(n_tiles_total, tile_begin + tiles_per_split);
 
+    const bool empty = tile_begin >= tile_end;
+    // this CTA's merged partial of its split: with a cluster it lies in shared memory behind the warps' partials
     float* po = p.part_o + ((size_t)split * p.Hq + (size_t)g * G) * D;
     float* pml = p.part_ml + ((size_t)split * p.Hq + (size_t)g * G) * 2;
-    const bool empty = tile_begin >= tile_end;
+    if (CL > 1) {
+        po = reinterpret_cast<float*>(sv);           // [8][128]
+        pml = po + 8 * D;                            // [8][2]
+    }
     if (empty) {  // empty split: neutral partial
         if (threadIdx.x < G) { pml[threadIdx.x * 2] = -INFINITY; pml[threadIdx.x * 2 + 1] = 0.f; }
     } else {
 
-    // ---- q: rotate the G heads of this group into smem (rows >= G zero) ----
-    for (int i = threadIdx.x; i < 16 * 64; i += 128) {
-        const int r = i >> 6, j = i & 63;
-        if (r < G) rope1d_row(p.qkv + (size_t)(g * G + r) * D, sq + r * LDS, j, pos, p.inv_freq);
-        else { sq[r * LDS + j] = f2bf(0.f); sq[r * LDS + j + 64] = f2bf(0.f); }
-    }
     // ---- append the new token's k (rotated) and v to the cache (the CTA owning the last tile) ----
     if (tile_end == n_tiles_total) {
         const int page = p.page_table[kv_old / BN], slot = kv_old % BN;
@@ -616,25 +625,37 @@ __device__ __forceinline__ void attn_decode_role(const DecodeAttnParams& p, cons
             *reinterpret_cast<uint4*>(dv + c * 8) = *reinterpret_cast<const uint4*>(vsrc + c * 8);
         }
         __threadfence();
+        __syncthreads();   // the row is written before any thread of this CTA copies the last tile
+    }
+
+    auto load_kv = [&](int tile) {
+        if (tile < tile_end) {
+            const int buf = (tile - tile_begin) % kDecBuf;
+            bf16* dk = sk + buf * BN * LDS;
+            bf16* dv = sv + buf * BN * LDS;
+            const int page = p.page_table[tile];
+            const bf16* gk = p.kc + ((size_t)page * p.Hkv + g) * BN * D;
+            const bf16* gv = p.vc + ((size_t)page * p.Hkv + g) * BN * D;
+            const int t0 = tile * BN;
+            for (int i = threadIdx.x; i < BN * (D / 8); i += 128) {
+                const int r = i >> 4, c = i & 15;
+                const bool ok = (t0 + r) < T;
+                cp_async16(dk + r * LDS + c * 8, gk + (size_t)r * D + c * 8, ok);
+                cp_async16(dv + r * LDS + c * 8, gv + (size_t)r * D + c * 8, ok);
+            }
+        }
+        cp_async_commit();   // (a group per tile slot, empty past the end, so that the waits count alike)
+    };
+#pragma unroll
+    for (int i = 0; i < kDecBuf - 1; ++i) load_kv(tile_begin + i);
+
+    // ---- q: rotate the G heads of this group into smem (rows >= G zero) while the first tiles arrive ----
+    for (int i = threadIdx.x; i < 16 * 64; i += 128) {
+        const int r = i >> 6, j = i & 63;
+        if (r < G) rope1d_row(p.qkv + (size_t)(g * G + r) * D, sq + r * LDS, j, pos, p.inv_freq);
+        else { sq[r * LDS + j] = f2bf(0.f); sq[r * LDS + j + 64] = f2bf(0.f); }
     }
     __syncthreads();
-
-    auto load_kv = [&](int tile, int buf) {
-        bf16* dk = sk + buf * BN * LDS;
-        bf16* dv = sv + buf * BN * LDS;
-        const int page = p.page_table[tile];
-        const bf16* gk = p.kc + ((size_t)page * p.Hkv + g) * BN * D;
-        const bf16* gv = p.vc + ((size_t)page * p.Hkv + g) * BN * D;
-        const int t0 = tile * BN;
-        for (int i = threadIdx.x; i < BN * (D / 8); i += 128) {
-            const int r = i >> 4, c = i & 15;
-            const bool ok = (t0 + r) < T;
-            cp_async16(dk + r * LDS + c * 8, gk + (size_t)r * D + c * 8, ok);
-            cp_async16(dv + r * LDS + c * 8, gv + (size_t)r * D + c * 8, ok);
-        }
-    };
-    load_kv(tile_begin, 0);
-    cp_async_commit();
 
     uint32_t qf[D / 16][4];
 #pragma unroll
@@ -651,11 +672,10 @@ __device__ __forceinline__ void attn_decode_role(const DecodeAttnParams& p, cons
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 
     for (int t = tile_begin; t < tile_end; ++t) {
-        const int buf = (t - tile_begin) & 1;
-        if (t + 1 < tile_end) load_kv(t + 1, buf ^ 1);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
+        const int buf = (t - tile_begin) % kDecBuf;
+        cp_async_wait<kDecBuf - 2>();
+        __syncthreads();   // tile t has landed for everybody, and everybody is done with the buffer of tile t - 1
+        load_kv(t + kDecBuf - 1);
         const bf16* ks = sk + buf * BN * LDS + warp * 16 * LDS;
         const bf16* vs = sv + buf * BN * LDS + warp * 16 * LDS;
         float s[2][4];
@@ -672,8 +692,8 @@ __device__ __forceinline__ void attn_decode_role(const DecodeAttnParams& p, cons
         uint32_t pf[1][4];
         softmax_step<D, 1>(s, p.scale_log2, m, l, o, pf);
         warp_pv<D, LDS, 1>(pf, vs, lane, o);
-        __syncthreads();
     }
+    cp_async_wait<0>();   // (empty groups)
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
@@ -709,6 +729,77 @@ __device__ __forceinline__ void attn_decode_role(const DecodeAttnParams& p, cons
         if (d == 0) { pml[r * 2] = M; pml[r * 2 + 1] = L; }
     }
     }  // !empty
+
+    if (CL > 1) {
+        // ---- cluster: CTA r merges query head r of the cluster's splits, then of all clusters if it arrives last ----
+        pdl_launch_dependents();
+        const int rank = (int)cluster_ctarank(), ncl = p.nsplit / CL;
+        __syncwarp();
+        cluster_sync_all();        // every CTA's partial is in its shared memory
+        float M = -INFINITY, acc = 0.f, L = 0.f;
+        const int d = threadIdx.x;
+        if (rank < G) {
+            float mw[CL], lw[CL], ow[CL];
+#pragma unroll
+            for (int c = 0; c < CL; ++c) {
+                mw[c] = ld_cluster_f32(pml + rank * 2, c);
+                lw[c] = ld_cluster_f32(pml + rank * 2 + 1, c);
+                ow[c] = ld_cluster_f32(po + rank * D + d, c);
+                M = fmaxf(M, mw[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < CL; ++c) {
+                if (mw[c] != -INFINITY) {   // (an empty split left no output)
+                    const float f = exp2f((mw[c] - M) * p.scale_log2);
+                    acc = fmaf(f, ow[c], acc);
+                    L = fmaf(f, lw[c], L);
+                }
+            }
+        }
+        __syncwarp();
+        cluster_arrive();          // this CTA has read its peers; it leaves only when they have read it
+        if (rank < G && ncl == 1) p.out[(size_t)(g * G + rank) * D + d] = f2bf(L > 0.f ? acc / L : 0.f);
+        if (rank < G && ncl > 1) {
+            __shared__ int s_last_row;
+            const size_t row = (size_t)(split / CL) * p.Hq + (size_t)g * G + rank;
+            p.part_o[row * D + d] = acc;
+            if (d == 0) { p.part_ml[row * 2] = M; p.part_ml[row * 2 + 1] = L; }
+            __threadfence();
+            __syncthreads();
+            // the KV group's counter holds one 4-bit arrival count per head (at most 8 clusters)
+            if (d == 0) {
+                const unsigned prev = atomicAdd(reinterpret_cast<unsigned*>(&p.counters[g]), 1u << (4 * rank));
+                s_last_row = ((prev >> (4 * rank)) & 15u) == (unsigned)(ncl - 1);
+                if (s_last_row) atomicSub(reinterpret_cast<unsigned*>(&p.counters[g]), (unsigned)ncl << (4 * rank));   // ready for the next launch
+            }
+            __syncthreads();
+            if (s_last_row) {
+                __threadfence();
+                float mw[CL], lw[CL], ow[CL];
+                M = -INFINITY; acc = 0.f; L = 0.f;
+#pragma unroll
+                for (int c = 0; c < CL; ++c) {
+                    const size_t r = (size_t)min(c, ncl - 1) * p.Hq + (size_t)g * G + rank;
+                    mw[c] = c < ncl ? __ldcg(p.part_ml + r * 2) : -INFINITY;
+                    lw[c] = __ldcg(p.part_ml + r * 2 + 1);
+                    ow[c] = __ldcg(p.part_o + r * D + d);
+                    M = fmaxf(M, mw[c]);
+                }
+#pragma unroll
+                for (int c = 0; c < CL; ++c) {
+                    if (mw[c] != -INFINITY) {
+                        const float f = exp2f((mw[c] - M) * p.scale_log2);
+                        acc = fmaf(f, ow[c], acc);
+                        L = fmaf(f, lw[c], L);
+                    }
+                }
+                p.out[(size_t)(g * G + rank) * D + d] = f2bf(L > 0.f ? acc / L : 0.f);
+            }
+        }
+        __syncwarp();
+        cluster_wait();
+        return;
+    }
 
     // ---- the last CTA of this KV group to arrive merges all splits (replaces a separate combine launch) ----
     pdl_launch_dependents();
@@ -765,7 +856,11 @@ __device__ __forceinline__ void attn_decode_role(const DecodeAttnParams& p, cons
 
 __global__ void __launch_bounds__(128) attn_decode_kernel(const DecodeAttnParams p) {
     extern __shared__ __align__(16) uint8_t smem_attn[];
-    attn_decode_role(p, blockIdx.x, blockIdx.y, smem_attn);
+    attn_decode_role<1>(p, blockIdx.x, blockIdx.y, smem_attn);
+}
+__global__ void __cluster_dims__(1, 8, 1) __launch_bounds__(128) attn_decode_cluster_kernel(const DecodeAttnParams p) {
+    extern __shared__ __align__(16) uint8_t smem_attn[];
+    attn_decode_role<8>(p, blockIdx.x, blockIdx.y, smem_attn);
 }
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
@@ -875,7 +970,7 @@ __device__ __forceinline__ void oproj_role(const DecodeAttnParams& p, const Opro
 __global__ void __launch_bounds__(128) attn_oproj_kernel(const DecodeAttnParams p, const OprojParams o) {
     extern __shared__ __align__(16) uint8_t smem_attn[];
     const int n_attn = p.Hkv * p.nsplit;
-    if ((int)blockIdx.x < n_attn) attn_decode_role(p, blockIdx.x % p.Hkv, blockIdx.x / p.Hkv, smem_attn);
+    if ((int)blockIdx.x < n_attn) attn_decode_role<1>(p, blockIdx.x % p.Hkv, blockIdx.x / p.Hkv, smem_attn);
     else oproj_role(p, o, blockIdx.x - n_attn, smem_attn);
 }
 
@@ -883,16 +978,16 @@ int attn_decode(bf16* qkv, bf16* kc, bf16* vc, const int* page_table, int page_s
                 const int* rope_pos, const int* finished, const float* inv_freq, int Hq, int Hkv, int nsplit,
                 float* part_o, float* part_ml, int* counters, bf16* out, bool pdl, cudaStream_t s) {
     if (page_size != 64 || Hq % Hkv || Hq / Hkv > 8) return -1;
-    constexpr int smem = (16 + 4 * 64) * 136 * 2;
-    static SmemAttrOnce once;
-    if (ensure_dyn_smem(once, attn_decode_kernel, smem)) return -2;
+    const bool cluster = nsplit % 8 == 0;
+    static SmemAttrOnce once, once_cl;
+    if (cluster ? ensure_dyn_smem(once_cl, attn_decode_cluster_kernel, kDecSmem) : ensure_dyn_smem(once, attn_decode_kernel, kDecSmem)) return -2;
     DecodeAttnParams p{};
     p.qkv = qkv; p.kc = kc; p.vc = vc; p.page_table = page_table; p.kv_len = kv_len; p.rope_pos = rope_pos;
     p.finished = finished; p.inv_freq = inv_freq; p.Hq = Hq; p.Hkv = Hkv; p.nsplit = nsplit;
     p.part_o = part_o; p.part_ml = part_ml; p.counters = counters; p.out = out;
     p.scale_log2 = 1.4426950408889634f / sqrtf(128.f);
     count_launch();
-    if (launch_kernel(attn_decode_kernel, dim3(Hkv, nsplit), dim3(128), (size_t)smem, s, pdl, p) != cudaSuccess) return -3;
+    if (launch_kernel(cluster ? attn_decode_cluster_kernel : attn_decode_kernel, dim3(Hkv, nsplit), dim3(128), (size_t)kDecSmem, s, pdl, p) != cudaSuccess) return -3;
     return 0;
 }
 
@@ -902,7 +997,7 @@ int attn_oproj_decode(bf16* qkv, bf16* kc, bf16* vc, const int* page_table, int 
                       float* part_o, float* part_ml, int* counters, bf16* attn_out, const bf16* o_w, int o_ldw,
                       int o_N, bf16* h, int* sync, cudaStream_t s) {
     if (page_size != 64 || Hq % Hkv || Hq / Hkv > 8) return -1;
-    constexpr int smem = (16 + 4 * 64) * 136 * 2;
+    constexpr int smem = kDecSmem;
     if (Hq * 128 * 2 > smem) return -4;
     static SmemAttrOnce once;
     if (ensure_dyn_smem(once, attn_oproj_kernel, smem)) return -2;

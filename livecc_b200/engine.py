@@ -100,8 +100,10 @@ class LiveCCB200ForConditionalGeneration:
         self.use_cuda_graph = os.environ.get("LIVECC_B200_NO_GRAPH", "0") != "1"
         self.use_vit_graph = self.use_cuda_graph and os.environ.get("LIVECC_B200_VIT_GRAPH", "1") != "0"
         self._vit_graphs = {}
-        # split-KV factor of the decode attention: at most one CTA per SM, at least ~8 KV tiles (512 tokens) per split
-        self.max_nsplit = max(1, min(64, (self.ctx.num_sms + t.num_key_value_heads - 1) // t.num_key_value_heads))
+        # split-KV factor of the decode attention: at most two CTAs per SM (they fit side by side), as a power of two
+        self.max_nsplit = 1
+        while self.max_nsplit < 64 and 2 * self.max_nsplit * t.num_key_value_heads <= 2 * self.ctx.num_sms:
+            self.max_nsplit *= 2
         self.nsplit = self.max_nsplit
         self.last_stats = {}
         # per-phase device time of the last generate() (CUDA events on the launch stream) and running totals
@@ -455,8 +457,9 @@ class LiveCCB200ForConditionalGeneration:
     def _pick_nsplit(self, kv_tokens: int) -> int:
         """Split-KV factor of the per-op decode attention (unused by the persistent kernel, which plans its own items)."""
         kv_tiles = (kv_tokens + 63) // 64
-        div = int(os.environ.get("LIVECC_B200_NSPLIT_DIV", "8"))
-        want = max(1, (kv_tiles + div - 1) // div)   # >= ~8 KV tiles (512 tokens) per split
+        div = int(os.environ.get("LIVECC_B200_NSPLIT_DIV", "2"))
+        want = max(1, (kv_tiles + div - 1) // div)   # about 2 KV tiles (128 tokens) per split while the SMs have room
+        want = 1 if want <= 2 else max(want, 8)      # multiples of 8 splits merge inside clusters; up to 4 tiles one CTA per KV head is as fast
         nsplit = 1
         while nsplit < want and nsplit < self.max_nsplit:  # quantised to powers of two: at most 7 captured graphs
             nsplit *= 2

@@ -413,3 +413,32 @@ def test_sample_greedy_sizes(ctx, V, hist):
         assert torch.equal(proc, want)
         assert int(seq[hist]) == int((want == want.max()).nonzero()[0])
         assert sc.tolist()[:6] == [1, 1, 0, 1, hist + 1, int(seq[hist])]
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(28, 4), (8, 1), (3, 3)])
+@pytest.mark.parametrize("nsplit", [8, 16, 24, 64])
+@pytest.mark.parametrize("kv_len", [0, 63, 64, 511, 4095, 9001])
+def test_attn_decode_splits_merged_in_clusters(ctx, kv_len, nsplit, Hq, Hkv):
+    """Multiples of 8 splits merge inside clusters, one query head per CTA: one to eight clusters, empty splits, groups of 1 to 8 heads,
+    the new token alone in its tile; launched twice, since the arrival counts of a launch have to be back at zero."""
+    cache = PagedCache(1, Hkv, kv_len + 1, seed=kv_len)
+    cache.k.fill_(float("nan"))     # (a recycled page may hold anything behind the newest token)
+    cache.v.fill_(float("nan"))
+    pk, pv = _rand((Hkv, max(kv_len, 1), 128), 61), _rand((Hkv, max(kv_len, 1), 128), 62)
+    for t0 in range(0, kv_len, 64):
+        n = min(64, kv_len - t0)
+        pg = int(cache.page_table[t0 // 64])
+        cache.k[0, pg, :, :n], cache.v[0, pg, :, :n] = pk[:, t0:t0 + n], pv[:, t0:t0 + n]
+    qkv = _rand(((Hq + 2 * Hkv) * 128,), 63)
+    sc = torch.zeros(A.SC_COUNT, dtype=torch.int32, device=DEV)
+    sc[A.SC_KV_LEN], sc[A.SC_ROPE_POS] = kv_len, kv_len + 3
+    outs = [ctx.attn_decode(qkv.clone(), cache.k[0], cache.v[0], cache.page_table, sc, _text_inv_freq(), Hq, Hkv, nsplit) for _ in range(2)]
+    assert torch.equal(outs[0], outs[1]) and not ctx._attn_counters.any()
+    q = qkv[: Hq * 128].view(1, Hq, 128).transpose(0, 1)
+    k = qkv[Hq * 128:(Hq + Hkv) * 128].view(1, Hkv, 128).transpose(0, 1)
+    cos, sin = R.mrope_cos_sin(torch.full((3, 1), kv_len + 3, dtype=torch.long, device=DEV), 128, 1e6, torch.bfloat16, (16, 24, 24))
+    q_ref, _ = R.apply_mrope(q, k, cos, sin)
+    kc, vc = cache.gather(0, kv_len + 1)
+    rep = Hq // Hkv
+    kr, vr = (x[:, None].expand(Hkv, rep, kv_len + 1, 128).reshape(Hq, kv_len + 1, 128) for x in (kc, vc))
+    _attn_close(outs[0], _attn_ref_fp32(q_ref, kr, vr, None, 128 ** -0.5).transpose(0, 1).reshape(Hq * 128), "attn_decode")
