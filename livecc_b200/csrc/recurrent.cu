@@ -86,6 +86,46 @@ __global__ void causal_conv_kernel(const TI* __restrict__ in, int ld_in, T* __re
     }
 }
 
+// Long calls in bf16 with 2 to 4 taps and even channels: a thread owns two neighbouring channels over `span` rows, eight rows' loads in
+// flight, the window slides through registers. The form above reads an input 1.9 times (8 rows and 7 before them), two bytes at a time.
+// The sums run in its order. 2048 rows of 6144 channels, 4 taps: 31 us, 64
+// in the form above; 128 rows: 6.8 us for 9.7.
+template <int TAPS, bool SILU>
+__global__ void __launch_bounds__(128) causal_conv_long_kernel(const bf16* __restrict__ in, int ld_in, bf16* __restrict__ out, int ld_out,
+                                                               const float* __restrict__ w, const float* __restrict__ b,
+                                                               const float* __restrict__ carry, int S, int C, int span, SeqPos pos) {
+    if (seq_done(pos)) return;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
+    const int t0 = blockIdx.y * span;
+    if (c >= C) return;
+    float w0[TAPS], w1[TAPS];
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) { w0[j] = w[(size_t)c * TAPS + j]; w1[j] = w[(size_t)(c + 1) * TAPS + j]; }
+    const float b0 = b ? b[c] : 0.f, b1 = b ? b[c + 1] : 0.f;
+    auto row = [&](int t) { return unpack_bf16x2(*reinterpret_cast<const uint32_t*>(in + (size_t)t * ld_in + c)); };
+    float2 win[TAPS - 1 + 8];
+#pragma unroll
+    for (int i = 0; i < TAPS - 1; ++i) {
+        const int t = t0 - (TAPS - 1) + i;   // (below S: t0 is)
+        win[i] = t >= 0 ? row(t) : make_float2(carry[(size_t)c * (TAPS - 1) + (TAPS - 1 + t)], carry[(size_t)(c + 1) * (TAPS - 1) + (TAPS - 1 + t)]);
+    }
+    const int t1 = min(S, t0 + span);
+    for (int t = t0; t < t1; t += 8) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) win[TAPS - 1 + r] = t + r < t1 ? row(t + r) : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            float a0 = b0, a1 = b1;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) { a0 = fmaf(w0[j], win[r + j].x, a0); a1 = fmaf(w1[j], win[r + j].y, a1); }
+            if (t + r < t1)
+                *reinterpret_cast<uint32_t*>(out + (size_t)(t + r) * ld_out + c) = SILU ? pack_bf16x2(silu_f(a0), silu_f(a1)) : pack_bf16x2(a0, a1);
+        }
+#pragma unroll
+        for (int i = 0; i < TAPS - 1; ++i) win[i] = win[8 + i];
+    }
+}
+
 // carry[c, i] <- input at row S - (taps-1) + i (an older carry entry when that row is negative)
 template <typename T>
 __global__ void conv_carry_update_kernel(const T* __restrict__ in, int ld_in, float* __restrict__ carry, int S, int C,
@@ -427,6 +467,8 @@ int causal_conv(int dt, const void* in, int ld_in, void* out, int ld_out, const 
     const bool fused = taps > 1 && S <= kConvRows;
     float* carry_out = fused ? carry : nullptr;
     const bool in32 = opt.in_f32 || dt == DT_F32;
+    const bool pairs = dt == DT_BF16 && !in32 && !opt.add_input && S > kConvRows && taps >= 2 && taps <= 4 && ((C | ld_in | ld_out) % 2) == 0 &&
+                       ((uintptr_t)in % 4) == 0 && ((uintptr_t)out % 4) == 0;
     count_launch();
 #define LCC_CONV(TI, T, SL, AD) causal_conv_kernel<TI, T, SL, AD><<<grid, 128, 0, s>>>((const TI*)in, ld_in, (T*)out, ld_out, w, b, carry, carry_out, S, C, taps, pos)
 #define LCC_CONV2(TI, T)                                                            \
@@ -436,7 +478,21 @@ int causal_conv(int dt, const void* in, int ld_in, void* out, int ld_out, const 
         else if (opt.silu) LCC_CONV(TI, T, true, true);                             \
         else LCC_CONV(TI, T, false, false);                                         \
     } while (0)
-    if (dt == DT_F32) LCC_CONV2(float, float);
+    if (pairs) {
+        const unsigned gx = (C / 2 + 127) / 128;
+        int span = 8;   // more rows per thread (fewer of them read twice) once that leaves every SM a few CTAs
+        while (span < 32 && (uint64_t)gx * ((S + 2 * span - 1) / (2 * span)) >= 4 * 148) span *= 2;
+        const dim3 lg(gx, (S + span - 1) / span);
+#define LCC_CONV_LONG(TP)                                                                                                                    \
+    do {                                                                                                                                     \
+        if (opt.silu) causal_conv_long_kernel<TP, true><<<lg, 128, 0, s>>>((const bf16*)in, ld_in, (bf16*)out, ld_out, w, b, carry, S, C, span, pos);  \
+        else causal_conv_long_kernel<TP, false><<<lg, 128, 0, s>>>((const bf16*)in, ld_in, (bf16*)out, ld_out, w, b, carry, S, C, span, pos);          \
+    } while (0)
+        if (taps == 2) LCC_CONV_LONG(2);
+        else if (taps == 3) LCC_CONV_LONG(3);
+        else LCC_CONV_LONG(4);
+#undef LCC_CONV_LONG
+    } else if (dt == DT_F32) LCC_CONV2(float, float);
     else if (in32) LCC_CONV2(float, bf16);
     else LCC_CONV2(bf16, bf16);
 #undef LCC_CONV2

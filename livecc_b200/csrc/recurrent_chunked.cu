@@ -299,6 +299,230 @@ __global__ void __launch_bounds__(256) chunk_output_kernel(ChunkArgs a, SeqPos p
     }
 }
 
+// ---- the same three products for a decay per head and 16-byte aligned rows ----------------------------------------------
+// The forms above stage 16-deep slices element by element, an exponential per staged element, and a decayed copy of c k^T per head
+// (2048 rows, 64 heads of 64 x 128: 54 + 92 + 157 us). Here a CTA of 128 threads stages 64-deep slabs with 16-byte loads and an 8 x 4 tile
+// per thread multiplies them in packed fp32 pairs (fma.rn.f32x2: each half rounds as a scalar fma does); c k^T is left undecayed once
+// per group of heads, and the decays enter where a head's output tile is staged: 15 + 59 + 112 us, bound by
+// fp32 multiplies (2.1 and 3.2 GFLOP) and the shared-memory reads that feed them. The prefix over blocks: 30 -> 25 us.
+constexpr int SP = 64 + 4;      // pitch of a slab row
+struct Slab {
+    float a[64][SP], b[64][SP]; // [depth][tile row], [depth][tile column]
+};
+struct Acc84 {
+    float2 v[4][4];             // rows (2 i, 2 i + 1) x column j
+};
+__device__ __forceinline__ void slab_fma(const Slab& sh, int depth, int tm, int tn, Acc84& acc) {
+#pragma unroll 8
+    for (int k = 0; k < depth; ++k) {
+        const float4 a0 = *reinterpret_cast<const float4*>(&sh.a[k][tm]), a1 = *reinterpret_cast<const float4*>(&sh.a[k][tm + 4]);
+        const float4 b4 = *reinterpret_cast<const float4*>(&sh.b[k][tn]);
+        const float2 ar[4] = {make_float2(a0.x, a0.y), make_float2(a0.z, a0.w), make_float2(a1.x, a1.y), make_float2(a1.z, a1.w)};
+        const float bj[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 bb = make_float2(bj[j], bj[j]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc.v[i][j] = __ffma2_rn(ar[i], bb, acc.v[i][j]);
+        }
+    }
+}
+// 16 bytes of a row -> floats
+template <typename T> struct Row16;
+template <> struct Row16<bf16> {
+    static constexpr int N = 8;
+    static __device__ __forceinline__ void load(const bf16* p, float (&v)[8]) {
+        const uint4 u = *reinterpret_cast<const uint4*>(p);
+        const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
+    }
+};
+template <> struct Row16<float> {
+    static constexpr int N = 4;
+    static __device__ __forceinline__ void load(const float* p, float (&v)[4]) {
+        const float4 u = *reinterpret_cast<const float4*>(p);
+        v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+    }
+};
+// dst[k][r] = src[r][k0 + k] * f(r) for 64 tile rows (zero from `rows` on) and k < 64 (zero from `cols` on): rows contiguous along k
+template <typename T, typename F>
+__device__ __forceinline__ void slab_across(float (*dst)[SP], const T* src, int ld, int rows, int k0, int cols, F f) {
+    constexpr int V = Row16<T>::N;
+    for (int e = threadIdx.x; e < 64 * (64 / V); e += 128) {
+        const int r = e & 63, k = (e >> 6) * V;
+        float v[V] = {};
+        if (r < rows && k0 + k < cols) {
+            Row16<T>::load(src + (size_t)r * ld + k0 + k, v);
+            const float m = f(r);
+#pragma unroll
+            for (int i = 0; i < V; ++i) v[i] *= m;
+        }
+#pragma unroll
+        for (int i = 0; i < V; ++i) dst[k + i][r] = v[i];
+    }
+}
+// dst[k][c] = src[k][c0 + c] * f(k) for k < 64 (zero from `rows` on) and 64 tile columns (zero from `cols` on): rows contiguous along the tile
+template <typename T, typename F>
+__device__ __forceinline__ void slab_along(float (*dst)[SP], const T* src, int ld, int rows, int c0, int cols, F f) {
+    constexpr int V = Row16<T>::N;
+    for (int e = threadIdx.x; e < 64 * (64 / V); e += 128) {
+        const int k = e / (64 / V), c = (e % (64 / V)) * V;
+        float v[V] = {};
+        if (k < rows && c0 + c < cols) {
+            Row16<T>::load(src + (size_t)k * ld + c0 + c, v);
+            const float m = f(k);
+#pragma unroll
+            for (int i = 0; i < V; ++i) v[i] *= m;
+        }
+#pragma unroll
+        for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(&dst[k][c + i]) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    }
+}
+__device__ __forceinline__ float row_of(const Acc84& acc, int i, int j) { return (i & 1) ? acc.v[i >> 1][j].y : acc.v[i >> 1][j].x; }
+
+// ws_m[blk][group][t][s] = c_t . k_s
+template <typename T>
+__global__ void __launch_bounds__(128) chunk_products_kernel(ChunkArgs a, SeqPos pos) {
+    if (seq_done(pos)) return;
+    __shared__ Slab sh;
+    const int blk = blockIdx.x, g = blockIdx.y, groups = gridDim.y;
+    const int t0 = blk * CL, len = min(CL, a.S - t0);
+    const T* gc = (const T*)a.c + (size_t)(a.row0 + t0) * a.ld_c + (size_t)g * a.N;
+    const T* gk = (const T*)a.k + (size_t)(a.row0 + t0) * a.ld_k + (size_t)g * a.N;
+    const int tm = (threadIdx.x / 16) * 8, tn = (threadIdx.x % 16) * 4;
+    Acc84 acc{};
+    for (int n0 = 0; n0 < a.N; n0 += 64) {
+        __syncthreads();
+        slab_across(sh.a, gc, a.ld_c, len, n0, a.N, [](int) { return 1.f; });
+        slab_across(sh.b, gk, a.ld_k, len, n0, a.N, [](int) { return 1.f; });
+        __syncthreads();
+        slab_fma(sh, min(64, a.N - n0), tm, tn, acc);
+    }
+    float* out = a.ws_m + ((size_t)blk * groups + g) * CL * CL;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float4*>(out + (tm + i) * CL + tn) = make_float4(row_of(acc, i, 0), row_of(acc, i, 1), row_of(acc, i, 2), row_of(acc, i, 3));
+}
+
+// a block's own contribution to the state, stored [p][n]
+template <typename T>
+__global__ void __launch_bounds__(128) chunk_state_head_kernel(ChunkArgs a, SeqPos pos) {
+    if (seq_done(pos)) return;
+    __shared__ Slab sh;
+    __shared__ float rowf[CL];   // per row: the step scale times the decay from the row to the block's end
+    const int blk = blockIdx.x / a.heads, h = blockIdx.x % a.heads, g = h / a.heads_per_group;
+    const int p0 = blockIdx.y * TS;
+    const int t0 = blk * CL, len = min(CL, a.S - t0);
+    const T* gu = (const T*)a.u + (size_t)(a.row0 + t0) * a.ld_u + (size_t)h * a.P;
+    const T* gk = (const T*)a.k + (size_t)(a.row0 + t0) * a.ld_k + (size_t)g * a.N;
+    const float* gb = a.la + (size_t)(a.row0 + t0) * a.heads + h;
+    const int tm = (threadIdx.x / 16) * 8, tn = (threadIdx.x % 16) * 4;
+    if (threadIdx.x < CL) {
+        const int s = threadIdx.x;
+        rowf[s] = s < len ? (a.sc ? a.sc[(size_t)(a.row0 + t0 + s) * a.heads + h] : 1.f) *
+                                expf(fminf(gb[(size_t)(len - 1) * a.heads] - gb[(size_t)s * a.heads], 0.f))
+                          : 0.f;
+    }
+    __syncthreads();
+    slab_along(sh.a, gu, a.ld_u, len, p0, a.P, [&](int s) { return rowf[s]; });
+    float* out = a.ws_s + ((size_t)blk * a.heads + h) * a.P * a.N;
+    for (int n0 = 0; n0 < a.N; n0 += TS) {
+        if (n0) __syncthreads();
+        slab_along(sh.b, gk, a.ld_k, len, n0, a.N, [](int) { return 1.f; });
+        __syncthreads();
+        Acc84 acc{};
+        slab_fma(sh, len, tm, tn, acc);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (p0 + tm + i < a.P && n0 + tn < a.N)
+                *reinterpret_cast<float4*>(out + (size_t)(p0 + tm + i) * a.N + n0 + tn) = make_float4(row_of(acc, i, 0), row_of(acc, i, 1), row_of(acc, i, 2), row_of(acc, i, 3));
+    }
+}
+
+// contributions -> the state that enters each block (chunk_prefix_kernel, four neighbouring entries per thread)
+__global__ void __launch_bounds__(256) chunk_prefix4_kernel(ChunkArgs a, int nblocks, SeqPos pos) {
+    if (seq_done(pos)) return;
+    const size_t per = (size_t)a.heads * a.P * a.N;
+    const size_t idx = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (idx >= per) return;
+    const int h = (int)(idx / ((size_t)a.P * a.N));
+    float4 st = *reinterpret_cast<const float4*>(a.state + idx);
+    for (int b0 = 0; b0 < nblocks; b0 += 8) {
+        float4 d[8];
+        float e[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int b = b0 + i;
+            if (b < nblocks) {
+                d[i] = *reinterpret_cast<const float4*>(a.ws_s + (size_t)b * per + idx);
+                e[i] = a.la[(size_t)(a.row0 + min((b + 1) * CL, a.S) - 1) * a.heads + h];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int b = b0 + i;
+            if (b < nblocks) {
+                *reinterpret_cast<float4*>(a.ws_s + (size_t)b * per + idx) = st;
+                const float f = expf(e[i]);
+                st = make_float4(fmaf(f, st.x, d[i].x), fmaf(f, st.y, d[i].y), fmaf(f, st.z, d[i].z), fmaf(f, st.w, d[i].w));
+            }
+        }
+    }
+    *reinterpret_cast<float4*>(a.state + idx) = st;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128) chunk_output_head_kernel(ChunkArgs a, SeqPos pos) {
+    if (seq_done(pos)) return;
+    __shared__ Slab sh;
+    __shared__ float bt[CL], into[CL], scs[CL];   // per row: cumulative log decay, cs x decay from the block's start, cs x step scale
+    const int blk = blockIdx.x / a.heads, h = blockIdx.x % a.heads, g = h / a.heads_per_group;
+    const int p0 = blockIdx.y * TS;
+    const int t0 = blk * CL, len = min(CL, a.S - t0);
+    const int N = a.N, P = a.P;
+    const T* gu = (const T*)a.u + (size_t)(a.row0 + t0) * a.ld_u + (size_t)h * P;
+    const T* gc = (const T*)a.c + (size_t)(a.row0 + t0) * a.ld_c + (size_t)g * N;
+    const float* sin = a.ws_s + ((size_t)blk * a.heads + h) * P * N;
+    const float* gm = a.ws_m + ((size_t)blk * (a.heads / a.heads_per_group) + g) * CL * CL;
+    const int tm = (threadIdx.x / 16) * 8, tn = (threadIdx.x % 16) * 4;
+    if (threadIdx.x < CL) {
+        const int t = threadIdx.x;
+        const float b = t < len ? a.la[(size_t)(a.row0 + t0 + t) * a.heads + h] : 0.f;
+        bt[t] = b;
+        into[t] = t < len ? a.cs * expf(b) : 0.f;
+        scs[t] = t < len ? a.cs * (a.sc ? a.sc[(size_t)(a.row0 + t0 + t) * a.heads + h] : 1.f) : 0.f;
+    }
+    Acc84 acc{};
+    for (int n0 = 0; n0 < N; n0 += 64) {       // the entering state, seen through the decayed queries
+        __syncthreads();
+        slab_across(sh.a, gc, a.ld_c, len, n0, N, [&](int t) { return into[t]; });
+        slab_across(sh.b, sin + (size_t)p0 * N, N, min(TS, P - p0), n0, N, [](int) { return 1.f; });
+        __syncthreads();
+        slab_fma(sh, min(64, N - n0), tm, tn, acc);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < CL * CL / 4; e += 128) {   // the block's own rows: M[t, s], s <= t
+        const int t = e & 63, s = (e >> 6) * 4;
+        const float4 q = s <= t ? *reinterpret_cast<const float4*>(gm + t * CL + s) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sh.a[s + i][t] = s + i <= t && t < len ? v[i] * scs[s + i] * expf(fminf(bt[t] - bt[s + i], 0.f)) : 0.f;
+    }
+    slab_along(sh.b, gu, a.ld_u, len, p0, P, [](int) { return 1.f; });
+    __syncthreads();
+    slab_fma(sh, len, tm, tn, acc);
+    const float skip = a.skip ? a.skip[h] : 0.f;
+    if (p0 + tn >= P) return;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = tm + i;
+        if (t >= len) continue;
+        const float4 u = *reinterpret_cast<const float4*>(&sh.b[t][tn]);   // the rows' own values are still staged
+        *reinterpret_cast<float4*>(a.y + (size_t)(a.row0 + t0 + t) * a.ld_y + (size_t)h * P + p0 + tn) =
+            make_float4(row_of(acc, i, 0) + skip * u.x, row_of(acc, i, 1) + skip * u.y, row_of(acc, i, 2) + skip * u.z, row_of(acc, i, 3) + skip * u.w);
+    }
+}
+
 template <typename T, bool VEC>
 int run_chunked(const ScanArgs& s, SeqPos pos, cudaStream_t st) {
     const size_t per_block = (size_t)s.heads * ((size_t)CL * CL + (size_t)s.P * s.N);
@@ -316,6 +540,22 @@ int run_chunked(const ScanArgs& s, SeqPos pos, cudaStream_t st) {
         const int ncol = a.heads * a.NV;
         count_launch();
         chunk_cumsum_kernel<<<dim3(nb, (ncol + 127) / 128), 128, 0, st>>>(a, pos);
+        if constexpr (!VEC) {
+            constexpr int V = Row16<T>::N;
+            const bool rows16 = ((s.N | s.P | s.ld_k | s.ld_c | s.ld_u) % V) == 0 && ((s.N | s.P | s.ld_y) % 4) == 0 &&
+                                (((uintptr_t)s.k | (uintptr_t)s.c | (uintptr_t)s.u | (uintptr_t)s.y | (uintptr_t)s.state | (uintptr_t)a.ws_m | (uintptr_t)a.ws_s) % 16) == 0;
+            if (rows16) {
+                count_launch();
+                chunk_products_kernel<T><<<dim3(nb, s.heads / s.heads_per_group), 128, 0, st>>>(a, pos);
+                count_launch();
+                chunk_state_head_kernel<T><<<dim3(nb * s.heads, (s.P + TS - 1) / TS), 128, 0, st>>>(a, pos);
+                count_launch();
+                chunk_prefix4_kernel<<<(unsigned)((per_state / 4 + 255) / 256), 256, 0, st>>>(a, nb, pos);
+                count_launch();
+                chunk_output_head_kernel<T><<<dim3(nb * s.heads, (s.P + TS - 1) / TS), 128, 0, st>>>(a, pos);
+                continue;
+            }
+        }
         count_launch();
         chunk_weights_kernel<T, VEC><<<dim3(nb, VEC ? s.heads : s.heads / s.heads_per_group), 256, 0, st>>>(a, pos);
         count_launch();

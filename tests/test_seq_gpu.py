@@ -423,3 +423,20 @@ def test_few_row_attention_over_head_groups_and_widths(heads, kv_heads, dim, vdi
     cuts = [30, 31, 32, 33, 35, 63, 64, 65, 66, 69, 96, 97, 98, 99, 100, 101]
     # fp32 storage: the order of sums; bf16: a dozen roundings of 2^-9 on the way from a row to its logits
     assert rel(run(m, toks, cuts), want) < (2e-5 if dtype == "float32" else 3e-2)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,vdim,state,groups,taps,norm_groups", [(4, 72, 136, 2, 4, 1), (2, 8, 8, 1, 2, 1), (3, 136, 64, 3, 3, 2), (2, 264, 200, 1, 4, 2)])
+def test_block_form_with_aligned_rows(heads, vdim, state, groups, taps, norm_groups, dtype):
+    """State sizes in multiples of 16 bytes take 64-deep slabs: ragged tiles and slabs, blocks of 64 rows that end anywhere, states carried
+    from portion to portion, convolutions of 2 to 4 taps over long portions, norm groups of 8 to 528 columns."""
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    d = seq_cases.config([seq_cases.ssd(heads=heads, vdim=vdim, state=state, groups=groups, conv=taps, norm_groups=norm_groups, ff=24)], width=40)
+    cfg = SeqModelConfig.from_json(d)
+    tensors = synthetic_seq_tensors(cfg, seed=9)
+    toks = seq_cases.tokens(230, 96, seed=heads)
+    want, _ = O.forward(d, tensors, toks)
+    m = SeqLMForCausalLM.from_state_dict(cfg, tensors, dtype)
+    for cuts in ([], [64, 97, 161], [33, 66, 130]):
+        assert rel(run(m, toks, cuts), want) < (2e-5 if dtype == "float32" else 3e-2)
