@@ -227,6 +227,16 @@ def test_gpu_frame_ingest_is_bit_identical(small):
         b = eng.get_video_features_from_frames(clip.to(DEV))
         torch.cuda.synchronize()
         assert torch.equal(a, b)
+    eng.use_vit_graph = False
+    try:        # frames at an odd address (a clip inside a larger buffer), groups of patch rows with a remainder
+        clip = torch.randint(0, 256, (1, 3, 84, 28), dtype=torch.uint8)
+        buf = torch.zeros(clip.numel() + 1, dtype=torch.uint8, device=DEV)
+        odd = buf[1:].view(clip.shape)
+        odd.copy_(clip)
+        px, grid = patchify_video(clip)
+        assert torch.equal(eng.get_video_features(px.to(DEV), grid), eng.get_video_features_from_frames(odd))
+    finally:
+        eng.use_vit_graph = True
     proc_f = StubProcessor(cfg, emit_frames=True)
     inp = make_turn_inputs(StubProcessor(cfg), 0, 2, (112, 112), 5).to(DEV)
     inp_f = make_turn_inputs(proc_f, 0, 2, (112, 112), 5).to(DEV)

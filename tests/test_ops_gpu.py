@@ -61,6 +61,25 @@ def test_rmsnorm(ctx, rows, dim):
     assert _mismatch(y, ref, 1.0) < 2e-3 and _mismatch(y, ref, 2.0) == 0
 
 
+@pytest.mark.parametrize("rows,dim", [(1, 8), (2400, 8), (5, 512), (2368, 520), (2367, 1536), (2369, 1536), (9, 1544), (700, 4096), (500, 4104), (3, 16392)])
+def test_norms_at_the_edges_of_their_forms(ctx, rows, dim):
+    """teams of 64, 192 and 256 threads, a warp per row, columns beyond the registers; strided rows; a row's result does not depend on
+    how many rows there are"""
+    x = _rand((rows, dim + 8), 3, 2.0)[:, :dim] + 0.5
+    x = torch.cat([x, x[:, :8]], 1)[:, :dim]
+    w, b = 1 + _rand((dim,), 4, 0.1), _rand((dim,), 5, 0.1)
+    x64 = x.double()
+    d = x64 - x64.mean(1, keepdim=True)
+    ln, rms = ctx.layernorm(x, w, b, 1e-6), ctx.rmsnorm(x, w, 1e-6)
+    want = d / (d.square().mean(1, keepdim=True) + 1e-6).sqrt() * w.double() + b.double()
+    # rounding to bf16 (8 significant bits: 2^-8 of the value at most), plus fp32 arithmetic on terms of up to 2^3 (a few ulps of 2^-21)
+    assert ((ln.double() - want).abs() <= 2 ** -7.95 * want.abs() + 2 ** -17).all()
+    want = x64 / (x64.square().mean(1, keepdim=True) + 1e-6).sqrt() * w.double()
+    assert ((rms.double() - want).abs() <= 2 ** -6.95 * want.abs()).all()     # two roundings to bf16
+    n = max(1, rows // 3)
+    assert torch.equal(ctx.layernorm(x[:n], w, b, 1e-6), ln[:n]) and torch.equal(ctx.rmsnorm(x[:n], w, 1e-6), rms[:n])
+
+
 def test_cast(ctx):
     x = torch.randn((1024, 1176), device=DEV)
     assert torch.equal(ctx.cast_f32_bf16(x), x.to(torch.bfloat16))
