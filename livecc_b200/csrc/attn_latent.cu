@@ -31,6 +31,7 @@ __global__ void __launch_bounds__(256) latent_kv_append_kernel(const T* __restri
                                                                float* __restrict__ q_out, T* __restrict__ k_pages,
                                                                const int* __restrict__ page_table, int page_size, int H, int D,
                                                                int DR, int R, SeqPos pos, const T* __restrict__ qsrc, int ld_q, bool pairs) {
+    chain_begin();
     if (seq_done(pos)) return;
     __shared__ float red[32];
     const int t = blockIdx.x;
@@ -72,10 +73,10 @@ int latent_kv_append(int dt, const void* proj, int ld, int has_kv, const float* 
     count_launch();
     const dim3 S_grid(S, S < 32 ? 4 : 1);
     if (dt == DT_F32)
-        latent_kv_append_kernel<float><<<S_grid, 256, 0, s>>>((const float*)proj, ld, has_kv, norm_w, eps, inv_freq, mag, q_out,
+        chained(latent_kv_append_kernel<float>, S_grid, 256, 0, s)((const float*)proj, ld, has_kv, norm_w, eps, inv_freq, mag, q_out,
                                                          (float*)k_pages, page_table, page_size, H, D, DR, R, pos, (const float*)q, ld_q, rot_pairs);
     else
-        latent_kv_append_kernel<bf16><<<S_grid, 256, 0, s>>>((const bf16*)proj, ld, has_kv, norm_w, eps, inv_freq, mag, q_out,
+        chained(latent_kv_append_kernel<bf16>, S_grid, 256, 0, s)((const bf16*)proj, ld, has_kv, norm_w, eps, inv_freq, mag, q_out,
                                                         (bf16*)k_pages, page_table, page_size, H, D, DR, R, pos, (const bf16*)q, ld_q, rot_pairs);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }

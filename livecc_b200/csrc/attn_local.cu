@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(256) qk_headnorm_rope_append_kernel(const T* _
                                                                       T* __restrict__ k_pages, T* __restrict__ v_pages,
                                                                       const int* __restrict__ page_table, int page_size, int S, int Hq,
                                                                       int G, int D, int DV, SeqPos pos, AppendOpts ao) {
+    chain_begin();
     if (seq_done(pos)) return;
     const int t = blockIdx.x;
     const int p = seq_past(pos, S) + t;
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(256) qk_norm_kv_append_kernel(const T* __restr
                                                                 T* __restrict__ k_pages, T* __restrict__ v_pages,
                                                                 const int* __restrict__ page_table, int page_size, int S, int Hq,
                                                                 int G, int D, int DV, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     __shared__ float red[32];
     const int t = blockIdx.x;
@@ -202,6 +204,7 @@ __global__ void __launch_bounds__(128) attn_chunk_sink_kernel(const float* __res
                                                               T* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                               int chunk, float scale, SeqPos pos,
                                                               const float* __restrict__ sink, int ld_v, AttnOpts opt) {
+    chain_begin();
     if (seq_done(pos)) return;
     extern __shared__ float sm[];
     __shared__ float red[32];
@@ -301,6 +304,7 @@ __global__ void __launch_bounds__(256) attn_rows_kernel(const float* __restrict_
                                                         int Hq, int G, int D, int DV, int chunk, float scale, SeqPos pos,
                                                         const float* __restrict__ sink, int ld_v, float* __restrict__ part,
                                                         int* __restrict__ counters, AttnOpts opt) {
+    chain_begin();
     if (seq_done(pos)) return;
     constexpr int VN = RowVec<T>::N, NVK = 4 * PL / 32;   // value keys per lane: a warp's 4 keys over 32 / PL lane groups
     extern __shared__ __align__(16) float sm[];
@@ -541,7 +545,7 @@ int launch_attn_rows(const float* q, const void* k_pages, const void* v_pages, c
     int* counters = reinterpret_cast<int*>(ws);              // zero when the workspace is bound; every launch leaves zeros
     const dim3 grid(ctas / S, S, nz);
     count_launch();
-#define LCC_ATTN_ROWS(HBN, PLN, NPN)                                                                                                   do {                                                                                                                                  static SmemAttrOnce once;                                                                                                         if (ensure_dyn_smem(once, attn_rows_kernel<T, HBN, PLN, NPN>, kRowSmem)) return -100;                                             attn_rows_kernel<T, HBN, PLN, NPN><<<grid, 256, smem, s>>>(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,                                                                         (const T*)gate, ld_gate, (T*)out, ld_out, S, Hq, G, D, DV, chunk, scale, pos,                                                                    sink, ld_v, ws + cnt, counters, opt);                              } while (0)
+#define LCC_ATTN_ROWS(HBN, PLN, NPN)                                                                                                   do {                                                                                                                                  static SmemAttrOnce once;                                                                                                         if (ensure_dyn_smem(once, attn_rows_kernel<T, HBN, PLN, NPN>, kRowSmem)) return -100;                                             chained(attn_rows_kernel<T, HBN, PLN, NPN>, grid, 256, smem, s)(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,                                                                         (const T*)gate, ld_gate, (T*)out, ld_out, S, Hq, G, D, DV, chunk, scale, pos,                                                                    sink, ld_v, ws + cnt, counters, opt);                              } while (0)
 #define LCC_ATTN_ROWS_HB(PLN, NPN)                                                                                                     do { if (HB == 2) LCC_ATTN_ROWS(2, PLN, NPN); else LCC_ATTN_ROWS(8, PLN, NPN); } while (0)
     if constexpr (VN == 8) {
         if (pieces <= 16) LCC_ATTN_ROWS_HB(16, 1);
@@ -570,6 +574,7 @@ __global__ void __launch_bounds__(128) attn_split_kernel(const float* __restrict
                                                          T* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                          float scale, SeqPos pos, const float* __restrict__ sink, int ld_v,
                                                          float* __restrict__ part, int* __restrict__ counters, AttnOpts opt) {
+    chain_begin();
     if (seq_done(pos)) return;
     extern __shared__ float sm[];
     __shared__ float red[32];
@@ -755,6 +760,7 @@ __global__ void __launch_bounds__(256) attn_chunk_sink_tiled_kernel(const float*
                                                                     T* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                                     int chunk, float scale, SeqPos pos,
                                                                     const float* __restrict__ sink, int ld_v, AttnOpts opt) {
+    chain_begin();
     if (seq_done(pos)) return;
     extern __shared__ __align__(16) uint8_t smem_attn[];
     const int dc = min(D, ADC);
@@ -919,7 +925,7 @@ int launch_attn_tiled(const float* q, const void* k_pages, const void* v_pages, 
     if (ensure_dyn_smem(once, attn_chunk_sink_tiled_kernel<T>, (int)smem)) return -100;
     dim3 grid(Hq, (S + AQ - 1) / AQ, (DV + AVW - 1) / AVW);
     count_launch();
-    attn_chunk_sink_tiled_kernel<T><<<grid, 256, attn_tiled_smem<T>(D), s>>>(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,
+    chained(attn_chunk_sink_tiled_kernel<T>, grid, 256, attn_tiled_smem<T>(D), s)(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,
                                                                             (const T*)gate, ld_gate, (T*)out, ld_out, S, Hq, G, D, DV,
                                                                             chunk, scale, pos, sink, ld_v, opt);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
@@ -959,6 +965,7 @@ __global__ void __launch_bounds__(128 * KH, (VEC8 && NBUF == 1 && NV == 1) ? 2 :
                                                                   bf16* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                                   int chunk, float scale, SeqPos pos,
                                                                   const float* __restrict__ sink, int ld_v, AttnOpts opt) {
+    chain_begin();
     if (seq_done(pos)) return;
     extern __shared__ __align__(16) uint8_t smem_attn[];
     // NV output tiles of 128 channels per CTA (NV = 2: values of up to 256 channels against one pass over the scores)
@@ -1278,7 +1285,7 @@ int launch_attn_mma(const float* q, const void* k_pages, const void* v_pages, co
 #define LCC_ATTN_MMA(ONCE, VEC, KHN, NVN, ...)                                                                                  \
     do {                                                                                                                     \
         if (ensure_dyn_smem(ONCE, attn_chunk_sink_mma_kernel<VEC, KHN, NVN, ##__VA_ARGS__>, (int)smem_max)) return -100;          \
-        attn_chunk_sink_mma_kernel<VEC, KHN, NVN, ##__VA_ARGS__><<<grid, 128 * KHN, smem, s>>>(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, \
+        chained(attn_chunk_sink_mma_kernel<VEC, KHN, NVN, ##__VA_ARGS__>, grid, 128 * KHN, smem, s)(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, \
                                                                            page_size, (const bf16*)gate, ld_gate, (bf16*)out, ld_out, \
                                                                            S, Hq, G, D, DV, chunk, scale, pos, sink, ld_v, opt);  \
     } while (0)
@@ -1317,7 +1324,7 @@ int launch_attn_mma_maps(const float* q, const void* k_pages, const void* v_page
 #define LCC_ATTN_MAPS(ONCE, VEC, NVN, NB)                                                                                        \
     do {                                                                                                                         \
         if (ensure_dyn_smem(ONCE, attn_chunk_sink_mma_kernel<VEC, 2, NVN, NB, 2, true>, (int)smem_max)) return -100;                   \
-        attn_chunk_sink_mma_kernel<VEC, 2, NVN, NB, 2, true><<<grid, 256, smem, s>>>(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, page_size, \
+        chained(attn_chunk_sink_mma_kernel<VEC, 2, NVN, NB, 2, true>, grid, 256, smem, s)(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, page_size, \
                                                                                nullptr, 0, (bf16*)out, ld_out, S, Hq, G, D, DV, chunk, scale, pos, \
                                                                                sink, ld_v, opt);                                 \
     } while (0)
@@ -1335,6 +1342,7 @@ int launch_attn_mma_maps(const float* q, const void* k_pages, const void* v_page
 template <typename T>
 __global__ void __launch_bounds__(128) diff_combine_kernel(const float* __restrict__ a, T* __restrict__ out, int ld_out, int S, int H, int DV,
                                                            float lambda, float scale, float eps, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     const int64_t wid = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -1358,10 +1366,10 @@ int qk_norm_kv_append(int dt, const void* proj, int ld, const float* qn_w, const
         return -2;
     count_launch();
     if (dt == DT_F32)
-        qk_norm_kv_append_kernel<float><<<S, 256, 0, s>>>((const float*)proj, ld, qn_w, kn_w, eps, q_out, (float*)k_pages,
+        chained(qk_norm_kv_append_kernel<float>, S, 256, 0, s)((const float*)proj, ld, qn_w, kn_w, eps, q_out, (float*)k_pages,
                                                           (float*)v_pages, page_table, page_size, S, Hq, G, D, DV, pos);
     else
-        qk_norm_kv_append_kernel<bf16><<<S, 256, 0, s>>>((const bf16*)proj, ld, qn_w, kn_w, eps, q_out, (bf16*)k_pages,
+        chained(qk_norm_kv_append_kernel<bf16>, S, 256, 0, s)((const bf16*)proj, ld, qn_w, kn_w, eps, q_out, (bf16*)k_pages,
                                                          (bf16*)v_pages, page_table, page_size, S, Hq, G, D, DV, pos);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
@@ -1396,7 +1404,7 @@ int qk_headnorm_rope_append(int dt, const void* proj, int ld, int v_col, const f
     const bool pairs = (rot_pairs || rot_dims == 0) && (D % 2) == 0 && (ld % 2) == 0 && ((uintptr_t)proj % (2 * es)) == 0 &&
                        ((uintptr_t)k_pages % (2 * es)) == 0 && ((uintptr_t)q_out % 8) == 0;
 #define LCC_APPEND(T, P)                                                                                                      \
-    qk_headnorm_rope_append_kernel<T, P><<<grid, threads, 0, s>>>((const T*)proj, ld, v_col, qn_w, kn_w, eps, inv_freq, mag, rot_dims,  \
+    chained(qk_headnorm_rope_append_kernel<T, P>, grid, threads, 0, s)((const T*)proj, ld, v_col, qn_w, kn_w, eps, inv_freq, mag, rot_dims,  \
                                                                   rot_pairs, q_out, (T*)k_pages, (T*)v_pages, page_table, page_size, S, Hq, \
                                                                   G, D, DV, pos, ao)
     if (dt == DT_F32) { if (pairs) LCC_APPEND(float, true); else LCC_APPEND(float, false); }
@@ -1449,10 +1457,10 @@ int attn_masked(int dt, const float* q, const void* k_pages, const void* v_pages
             count_launch();
             if (smem > 48 * 1024) return -3;
             if (dt == DT_F32)
-                attn_split_kernel<float><<<grid, 128, smem, s>>>(q, (const float*)k_pages, (const float*)v_pages, page_table, page_size, (const float*)gate,
+                chained(attn_split_kernel<float>, grid, 128, smem, s)(q, (const float*)k_pages, (const float*)v_pages, page_table, page_size, (const float*)gate,
                                                                  ld_gate, (float*)out, ld_out, S, Hq, G, D, DV, scale, pos, sink, ld_v, part, counters, o);
             else
-                attn_split_kernel<bf16><<<grid, 128, smem, s>>>(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, page_size, (const bf16*)gate,
+                chained(attn_split_kernel<bf16>, grid, 128, smem, s)(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, page_size, (const bf16*)gate,
                                                                 ld_gate, (bf16*)out, ld_out, S, Hq, G, D, DV, scale, pos, sink, ld_v, part, counters, o);
             return cudaGetLastError() == cudaSuccess ? 0 : -100;
         }
@@ -1463,9 +1471,9 @@ int attn_masked(int dt, const float* q, const void* k_pages, const void* v_pages
         const int blocks = (int)(((int64_t)S * heads + 3) / 4);
         count_launch();
         if (dt == DT_F32)
-            diff_combine_kernel<float><<<blocks, 128, 0, s>>>(opt.raw, (float*)out, ld_out, S, heads, DV, opt.lambda, opt.diff_scale, opt.eps, pos);
+            chained(diff_combine_kernel<float>, blocks, 128, 0, s)(opt.raw, (float*)out, ld_out, S, heads, DV, opt.lambda, opt.diff_scale, opt.eps, pos);
         else
-            diff_combine_kernel<bf16><<<blocks, 128, 0, s>>>(opt.raw, (bf16*)out, ld_out, S, heads, DV, opt.lambda, opt.diff_scale, opt.eps, pos);
+            chained(diff_combine_kernel<bf16>, blocks, 128, 0, s)(opt.raw, (bf16*)out, ld_out, S, heads, DV, opt.lambda, opt.diff_scale, opt.eps, pos);
         return cudaGetLastError() == cudaSuccess ? 0 : -100;
     };
     // The one-CTA-per-row kernel keeps one score per key of the longest range a row of this call can see in shared memory
@@ -1493,12 +1501,12 @@ int attn_masked(int dt, const float* q, const void* k_pages, const void* v_pages
     count_launch();
     if (dt == DT_F32) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(attn_chunk_sink_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attn_chunk_sink_kernel<float><<<grid, 128, smem, s>>>(q, (const float*)k_pages, (const float*)v_pages, page_table,
+        chained(attn_chunk_sink_kernel<float>, grid, 128, smem, s)(q, (const float*)k_pages, (const float*)v_pages, page_table,
                                                               page_size, (const float*)gate, ld_gate, (float*)out, ld_out, S, Hq,
                                                               G, D, DV, chunk, scale, pos, sink, ld_v, o);
     } else {
         if (smem > 48 * 1024) cudaFuncSetAttribute(attn_chunk_sink_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attn_chunk_sink_kernel<bf16><<<grid, 128, smem, s>>>(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table,
+        chained(attn_chunk_sink_kernel<bf16>, grid, 128, smem, s)(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table,
                                                              page_size, (const bf16*)gate, ld_gate, (bf16*)out, ld_out, S, Hq, G,
                                                              D, DV, chunk, scale, pos, sink, ld_v, o);
     }

@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(256) hyper_boundary_kernel(float* __restrict__
                                                              const float* __restrict__ prev, const float* __restrict__ next,
                                                              const float* __restrict__ w, float eps, T* __restrict__ xa,
                                                              float* __restrict__ sum_out, int W) {
+    chain_begin();
     __shared__ float red[32];
     constexpr bool FAST = N > 0 && E > 0;
     const int n = N > 0 ? N : n_rt;
@@ -186,7 +187,7 @@ int launch_boundary(float* xs, int n, const YSource<T>& src, const float* prev, 
     const int per = (W + 255) / 256;
     const bool top_ok = src.y || !src.eo || src.top <= kMaxTop;
     count_launch();
-#define LCC_HB(N, E) hyper_boundary_kernel<T, N, E><<<S, 256, 0, s>>>(xs, n, src, prev, next, w, eps, (T*)xa, sum_out, W)
+#define LCC_HB(N, E) chained(hyper_boundary_kernel<T, N, E>, S, 256, 0, s)(xs, n, src, prev, next, w, eps, (T*)xa, sum_out, W)
 #define LCC_HB_E(N)                                                                                                        \
     do {                                                                                                                   \
         if (per <= 4 && top_ok) LCC_HB(N, 4); else if (per <= 8 && top_ok) LCC_HB(N, 8); else if (per <= 16 && top_ok) LCC_HB(N, 16); else LCC_HB(0, 0); \

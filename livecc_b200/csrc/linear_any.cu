@@ -52,6 +52,7 @@ template <typename T, typename TC>
 __global__ void __launch_bounds__(256) linear_tile_kernel(const T* __restrict__ A, int lda, const T* __restrict__ W, int ldw,
                                                           const float* __restrict__ bias, TC* __restrict__ C, int ldc, int M,
                                                           int N, int K, Grp g) {
+    chain_begin();
     __shared__ float As[BK][BM + 4];
     __shared__ float Ws[BK][BN + 4];
     const int tid = threadIdx.x;
@@ -132,6 +133,30 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
     const int n0 = (blockIdx.x * (blockDim.x >> 5) + warp) * (GLU ? 1 : WR);
     if (n0 >= N) return;
     int row0 = 0, z = blockIdx.y;
+    constexpr int V = Vec16<T>::N;
+    // the weight row behind accumulator r: output columns n0, n0 + 1, ...; in the GLU form (WR = 2) the gate row (r = 0) and
+    // the up row (r = 1) of output column n0
+    auto wrow = [&](int r) -> int {
+        if (GLU) return g.glu_il16 ? ((n0 >> 4) << 5) + (n0 & 15) + 16 * r : n0 + r * g.glu_F;
+        return min(n0 + r, N - 1);
+    };
+    uint4 wq[WR][WU];
+    auto load_weights = [&](int kb) {
+#pragma unroll
+        for (int r = 0; r < WR; ++r)
+#pragma unroll
+            for (int u = 0; u < WU; ++u) {
+                const int k = kb + u * 32 * V;
+                wq[r][u] = k < K ? ld_stream16(W + (size_t)wrow(r) * ldw + k) : make_uint4(0, 0, 0, 0);
+            }
+    };
+    bool loaded = false;
+    if (VEC && !g.row_off) {   // which weights it reads is known before the kernel in front has finished: their first loads don't wait for it
+        W += z * g.w_stride;
+        load_weights(lane * V);
+        loaded = true;
+    }
+    chain_begin();
     if (g.row_off) {
         if (g.compact) {
             // a decode step routes a handful of rows to a handful of lists: the grid has one y per possible non-empty list
@@ -144,7 +169,7 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
         M_all = g.row_off[z + 1] - row0;
     }
     const T* A0 = A + z * g.a_stride;
-    W += z * g.w_stride;
+    if (!loaded) W += z * g.w_stride;
     TC* C0 = C + z * g.c_stride + (size_t)row0 * ldc;
     const int* arow = g.a_rows ? g.a_rows + row0 : nullptr;
     if (!arow) A0 += (size_t)row0 * lda;
@@ -161,26 +186,10 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
     for (int r = 0; r < WR; ++r)
 #pragma unroll
         for (int m = 0; m < MM; ++m) acc[r][m] = 0.f;
-    // the weight row behind accumulator r: output columns n0, n0 + 1, ...; in the GLU form (WR = 2) the gate row (r = 0) and
-    // the up row (r = 1) of output column n0
-    auto wrow = [&](int r) -> int {
-        if (GLU) return g.glu_il16 ? ((n0 >> 4) << 5) + (n0 & 15) + 16 * r : n0 + r * g.glu_F;
-        return min(n0 + r, N - 1);
-    };
     if (VEC) {
-        constexpr int V = Vec16<T>::N;
-        const T* w[WR];
-#pragma unroll
-        for (int r = 0; r < WR; ++r) w[r] = W + (size_t)wrow(r) * ldw;
         for (int kb = lane * V; kb < K; kb += 32 * V * WU) {
-            uint4 wq[WR][WU];
-#pragma unroll
-            for (int r = 0; r < WR; ++r)
-#pragma unroll
-                for (int u = 0; u < WU; ++u) {
-                    const int k = kb + u * 32 * V;
-                    wq[r][u] = k < K ? ld_stream16(w[r] + k) : make_uint4(0, 0, 0, 0);
-                }
+            if (!loaded) load_weights(kb);
+            loaded = false;
 #pragma unroll
             for (int u = 0; u < WU; ++u) {
                 const int k = min(kb + u * 32 * V, K - V);      // past the end the weights are zero; keep the address valid
@@ -254,8 +263,8 @@ int launch_linear(const void* A, int lda, const void* W, int ldw, const float* b
 #define LCC_ROWS(MMN, WRN, WUN, WARPS, GLUB)                                                                                    \
     do {                                                                                                                       \
         const dim3 grid((N + WARPS * (GLUB ? 1 : WRN) - 1) / (WARPS * (GLUB ? 1 : WRN)), grid_y);                              \
-        if (vec) linear_rows_kernel<T, TC, true, MMN, WRN, WUN, GLUB><<<grid, WARPS * 32, 0, s>>>((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g); \
-        else linear_rows_kernel<T, TC, false, MMN, WRN, WUN, GLUB><<<grid, WARPS * 32, 0, s>>>((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g);    \
+        if (vec) chained(linear_rows_kernel<T, TC, true, MMN, WRN, WUN, GLUB>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g); \
+        else chained(linear_rows_kernel<T, TC, false, MMN, WRN, WUN, GLUB>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g);    \
     } while (0)
         if (g.glu_F > 0) {
             if constexpr (std::is_same<T, TC>::value) {
@@ -291,14 +300,14 @@ int launch_linear(const void* A, int lda, const void* W, int ldw, const float* b
         raw.c_stride = 0;
         dim3 grid((2 * N + BN - 1) / BN, (M + BM - 1) / BM, groups);
         count_launch();
-        linear_tile_kernel<T, T><<<grid, 256, 0, s>>>((const T*)A, lda, (const T*)W, ldw, bias, (T*)glu_tmp, ld_tmp, M, 2 * N, K, raw);
+        chained(linear_tile_kernel<T, T>, grid, 256, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (T*)glu_tmp, ld_tmp, M, 2 * N, K, raw);
         if (cudaGetLastError() != cudaSuccess) return -100;
         const int rows = g.row_off ? M_total : M;
         return glu_clamp_swish(sizeof(T) == 4 ? DT_F32 : DT_BF16, glu_tmp, ld_tmp, C, ldc, rows, N, g.glu_limit, s, g.glu_il16 != 0, g.glu_alpha, g.glu_up_bias);
     } else {
         dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, groups);
         count_launch();
-        linear_tile_kernel<T, TC><<<grid, 256, 0, s>>>((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g);
+        chained(linear_tile_kernel<T, TC>, grid, 256, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }

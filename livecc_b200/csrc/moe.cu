@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
                                                         int E, int top, float scale, int* __restrict__ sel,
                                                         float* __restrict__ weight, float* __restrict__ shared_gate,
                                                         int* __restrict__ counts, int* __restrict__ rank, int S, MoeRouterOpts ro) {
+    chain_begin();
     __shared__ float gch[4][kRouteScratch];
     __shared__ unsigned char gkeep[4][kRouteScratch];
     const int warp = threadIdx.x >> 5;
@@ -154,6 +155,7 @@ __global__ void __launch_bounds__(256) moe_route_small_kernel(const float* __res
                                                               float* __restrict__ weight, float* __restrict__ shared_gate,
                                                               int* __restrict__ row_off, int* __restrict__ pos,
                                                               int* __restrict__ src_row, int S, MoeRouterOpts ro) {
+    chain_begin();
     __shared__ int cnt[kSmallRouteExperts + 1];
     __shared__ int rk[kSmallRouteItems];
     __shared__ float gch[8][kRouteScratch];
@@ -195,6 +197,7 @@ __device__ __forceinline__ int padded(int n, int pad) { return (n + pad - 1) / p
 __global__ void moe_index_kernel(const int* __restrict__ sel, const int* __restrict__ rank, const int* __restrict__ counts, int E,
                                  int top, int pad, int* __restrict__ row_off, int* __restrict__ pos, int* __restrict__ src_row,
                                  int* __restrict__ tile_group, int n_tiles, int S) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= E) {
         int o = 0;
@@ -224,6 +227,7 @@ __global__ void moe_index_kernel(const int* __restrict__ sel, const int* __restr
 // out[i, :] = in[src_row[i], :] for every list row (16-byte pieces); padding rows (src_row < 0) are left alone.
 __global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict__ in, int ld_in16, const int* __restrict__ src_row,
                                                          uint4* __restrict__ out, int ld_out16, int n16) {
+    chain_begin();
     const int r = src_row[blockIdx.x];
     if (r < 0) return;
     for (int c = threadIdx.x; c < n16; c += blockDim.x) out[(size_t)blockIdx.x * ld_out16 + c] = in[(size_t)r * ld_in16 + c];
@@ -247,7 +251,7 @@ int moe_route(const float* logits, int ld, const float* correction, int E, int t
         top > E || ld < E + ((shared_gate && !ro.identity) ? 1 : 0) || !router_ok(ro, E, top, shared_gate))
         return -2;
     count_launch();
-    moe_route_kernel<<<(S + 3) / 4, 128, 0, s>>>(logits, ld, correction, E, top, scale, sel, weight, shared_gate, counts, rank, S, ro);
+    chained(moe_route_kernel, (S + 3) / 4, 128, 0, s)(logits, ld, correction, E, top, scale, sel, weight, shared_gate, counts, rank, S, ro);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 
@@ -258,7 +262,7 @@ int moe_route_small(const float* logits, int ld, const float* correction, int E,
         top < 1 || top > E || S * top > kSmallRouteItems || ld < E + ((shared_gate && !ro.identity) ? 1 : 0) || !router_ok(ro, E, top, shared_gate))
         return -2;
     count_launch();
-    moe_route_small_kernel<<<1, 256, 0, s>>>(logits, ld, correction, E, top, scale, sel, weight, shared_gate, row_off, pos, src_row, S, ro);
+    chained(moe_route_small_kernel, 1, 256, 0, s)(logits, ld, correction, E, top, scale, sel, weight, shared_gate, row_off, pos, src_row, S, ro);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 
@@ -269,7 +273,7 @@ int moe_index(const int* sel, const int* rank, const int* counts, int E, int top
     int n = S * top > E + 1 ? S * top : E + 1;
     if (tile_group && n_tiles > n) n = n_tiles;
     count_launch();
-    moe_index_kernel<<<(n + 255) / 256, 256, 0, s>>>(sel, rank, counts, E, top, pad, row_off, pos, src_row, tile_group, n_tiles, S);
+    chained(moe_index_kernel, (n + 255) / 256, 256, 0, s)(sel, rank, counts, E, top, pad, row_off, pos, src_row, tile_group, n_tiles, S);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 
@@ -279,7 +283,7 @@ int moe_gather_rows(int dt, const void* in, int ld_in, const int* src_row, void*
         ((uintptr_t)in % 16) || ((uintptr_t)out % 16))
         return -2;
     count_launch();
-    moe_gather_kernel<<<rows, 128, 0, s>>>((const uint4*)in, ld_in / per16, src_row, (uint4*)out, ld_out / per16, W / per16);
+    chained(moe_gather_kernel, rows, 128, 0, s)((const uint4*)in, ld_in / per16, src_row, (uint4*)out, ld_out / per16, W / per16);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 

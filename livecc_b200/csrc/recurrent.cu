@@ -44,6 +44,7 @@ template <typename TI, typename T, bool SILU, bool ADD>
 __global__ void causal_conv_kernel(const TI* __restrict__ in, int ld_in, T* __restrict__ out, int ld_out,
                                    const float* __restrict__ w, const float* __restrict__ b,
                                    const float* carry, float* carry_out, int S, int C, int taps, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int t0 = blockIdx.y * kConvRows;
@@ -94,6 +95,7 @@ template <int TAPS, bool SILU>
 __global__ void __launch_bounds__(128) causal_conv_long_kernel(const bf16* __restrict__ in, int ld_in, bf16* __restrict__ out, int ld_out,
                                                                const float* __restrict__ w, const float* __restrict__ b,
                                                                const float* __restrict__ carry, int S, int C, int span, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
     const int t0 = blockIdx.y * span;
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(128) causal_conv_long_kernel(const bf16* __res
 template <typename T>
 __global__ void conv_carry_update_kernel(const T* __restrict__ in, int ld_in, float* __restrict__ carry, int S, int C,
                                          int taps, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
@@ -147,6 +150,7 @@ template <typename T>
 __global__ void ssm_step_decay_kernel(const T* __restrict__ raw, int ld, const float* __restrict__ dt_bias,
                                       const float* __restrict__ a_log, float* __restrict__ dt_out,
                                       float* __restrict__ decay_out, int S, int heads) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= S * heads) return;
     const int t = i / heads, h = i % heads;
@@ -158,6 +162,7 @@ __global__ void ssm_step_decay_kernel(const T* __restrict__ raw, int ld, const f
 template <typename T>
 __global__ void gla_decay_kernel(const T* __restrict__ z, int ld, const float* __restrict__ bias, float inv_tau,
                                  float* __restrict__ decay_out, int S, int n) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= S * n) return;
     const int t = i / n, c = i % n;
@@ -177,6 +182,7 @@ constexpr int kScanThreads = 128;
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(kScanThreads) gated_scan_kernel(ScanArgs a, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     extern __shared__ float sm[];
     const int N = a.N, P = a.P, S = a.S;
@@ -255,6 +261,7 @@ __global__ void __launch_bounds__(kScanThreads) gated_scan_kernel(ScanArgs a, Se
 // product k . q, the values as fp32, the decays exp(-exp(a_log[h]) * softplus(z + dt_bias)), and beta = sigmoid(b).
 template <typename T>
 __global__ void __launch_bounds__(128) delta_pack_kernel(DeltaPackArgs a) {
+    chain_begin();
     const int wid = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (wid >= a.S * a.G) return;
     const int t = wid / a.G, g = wid % a.G, N = a.N, P = a.P, hpg = a.H / a.G;
@@ -308,6 +315,7 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
 // loops need no bounds.
 template <int NT_, int CPT>
 __global__ void __launch_bounds__(kScanThreads) delta_scan_kernel(DeltaScanArgs a, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     extern __shared__ __align__(16) float sm[];
     const int N = a.N, P = a.P, S = a.S, TTn = a.TT;
@@ -470,7 +478,7 @@ int causal_conv(int dt, const void* in, int ld_in, void* out, int ld_out, const 
     const bool pairs = dt == DT_BF16 && !in32 && !opt.add_input && S > kConvRows && taps >= 2 && taps <= 4 && ((C | ld_in | ld_out) % 2) == 0 &&
                        ((uintptr_t)in % 4) == 0 && ((uintptr_t)out % 4) == 0;
     count_launch();
-#define LCC_CONV(TI, T, SL, AD) causal_conv_kernel<TI, T, SL, AD><<<grid, 128, 0, s>>>((const TI*)in, ld_in, (T*)out, ld_out, w, b, carry, carry_out, S, C, taps, pos)
+#define LCC_CONV(TI, T, SL, AD) chained(causal_conv_kernel<TI, T, SL, AD>, grid, 128, 0, s)((const TI*)in, ld_in, (T*)out, ld_out, w, b, carry, carry_out, S, C, taps, pos)
 #define LCC_CONV2(TI, T)                                                            \
     do {                                                                            \
         if (opt.silu && !opt.add_input) LCC_CONV(TI, T, true, false);               \
@@ -485,8 +493,8 @@ int causal_conv(int dt, const void* in, int ld_in, void* out, int ld_out, const 
         const dim3 lg(gx, (S + span - 1) / span);
 #define LCC_CONV_LONG(TP)                                                                                                                    \
     do {                                                                                                                                     \
-        if (opt.silu) causal_conv_long_kernel<TP, true><<<lg, 128, 0, s>>>((const bf16*)in, ld_in, (bf16*)out, ld_out, w, b, carry, S, C, span, pos);  \
-        else causal_conv_long_kernel<TP, false><<<lg, 128, 0, s>>>((const bf16*)in, ld_in, (bf16*)out, ld_out, w, b, carry, S, C, span, pos);          \
+        if (opt.silu) chained(causal_conv_long_kernel<TP, true>, lg, 128, 0, s)((const bf16*)in, ld_in, (bf16*)out, ld_out, w, b, carry, S, C, span, pos);  \
+        else chained(causal_conv_long_kernel<TP, false>, lg, 128, 0, s)((const bf16*)in, ld_in, (bf16*)out, ld_out, w, b, carry, S, C, span, pos);          \
     } while (0)
         if (taps == 2) LCC_CONV_LONG(2);
         else if (taps == 3) LCC_CONV_LONG(3);
@@ -500,9 +508,9 @@ int causal_conv(int dt, const void* in, int ld_in, void* out, int ld_out, const 
     if (taps > 1 && !fused) {
         count_launch();
         if (in32)
-            conv_carry_update_kernel<float><<<(C + 127) / 128, 128, 0, s>>>((const float*)in, ld_in, carry, S, C, taps, pos);
+            chained(conv_carry_update_kernel<float>, (C + 127) / 128, 128, 0, s)((const float*)in, ld_in, carry, S, C, taps, pos);
         else
-            conv_carry_update_kernel<bf16><<<(C + 127) / 128, 128, 0, s>>>((const bf16*)in, ld_in, carry, S, C, taps, pos);
+            chained(conv_carry_update_kernel<bf16>, (C + 127) / 128, 128, 0, s)((const bf16*)in, ld_in, carry, S, C, taps, pos);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
@@ -513,8 +521,8 @@ int delta_pack(int dt, const DeltaPackArgs& a, cudaStream_t s) {
         return -2;
     const int warps = a.S * a.G;
     count_launch();
-    if (dt == DT_F32) delta_pack_kernel<float><<<(warps + 3) / 4, 128, 0, s>>>(a);
-    else delta_pack_kernel<bf16><<<(warps + 3) / 4, 128, 0, s>>>(a);
+    if (dt == DT_F32) chained(delta_pack_kernel<float>, (warps + 3) / 4, 128, 0, s)(a);
+    else chained(delta_pack_kernel<bf16>, (warps + 3) / 4, 128, 0, s)(a);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 
@@ -552,7 +560,7 @@ int delta_scan(const DeltaScanArgs& q, SeqPos pos, cudaStream_t s) {
 #define LCC_DSCAN(NTV, CPTV)                                                                                                    \
     do {                                                                                                                        \
         if (smem > 48 * 1024) cudaFuncSetAttribute(delta_scan_kernel<NTV, CPTV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        delta_scan_kernel<NTV, CPTV><<<grid, block, smem, s>>>(a, pos);                                                         \
+        chained(delta_scan_kernel<NTV, CPTV>, grid, block, smem, s)(a, pos);                                                         \
     } while (0)
     if (nt == 4) { if (cpt == 4) LCC_DSCAN(4, 4); else if (cpt == 2) LCC_DSCAN(4, 2); else LCC_DSCAN(4, 1); }
     else if (nt == 8) { if (cpt == 4) LCC_DSCAN(8, 4); else if (cpt == 2) LCC_DSCAN(8, 2); else LCC_DSCAN(8, 1); }
@@ -573,9 +581,9 @@ int ssm_step_decay(int dt, const void* raw, int ld, const float* dt_bias, const 
     const int n = S * heads;
     count_launch();
     if (dt == DT_F32)
-        ssm_step_decay_kernel<float><<<(n + 255) / 256, 256, 0, s>>>((const float*)raw, ld, dt_bias, a_log, dt_out, decay_out, S, heads);
+        chained(ssm_step_decay_kernel<float>, (n + 255) / 256, 256, 0, s)((const float*)raw, ld, dt_bias, a_log, dt_out, decay_out, S, heads);
     else
-        ssm_step_decay_kernel<bf16><<<(n + 255) / 256, 256, 0, s>>>((const bf16*)raw, ld, dt_bias, a_log, dt_out, decay_out, S, heads);
+        chained(ssm_step_decay_kernel<bf16>, (n + 255) / 256, 256, 0, s)((const bf16*)raw, ld, dt_bias, a_log, dt_out, decay_out, S, heads);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 
@@ -585,9 +593,9 @@ int gla_decay(int dt, const void* z, int ld, const float* bias, float tau, float
     const int tot = S * n;
     count_launch();
     if (dt == DT_F32)
-        gla_decay_kernel<float><<<(tot + 255) / 256, 256, 0, s>>>((const float*)z, ld, bias, 1.f / tau, decay_out, S, n);
+        chained(gla_decay_kernel<float>, (tot + 255) / 256, 256, 0, s)((const float*)z, ld, bias, 1.f / tau, decay_out, S, n);
     else
-        gla_decay_kernel<bf16><<<(tot + 255) / 256, 256, 0, s>>>((const bf16*)z, ld, bias, 1.f / tau, decay_out, S, n);
+        chained(gla_decay_kernel<bf16>, (tot + 255) / 256, 256, 0, s)((const bf16*)z, ld, bias, 1.f / tau, decay_out, S, n);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 
@@ -609,7 +617,7 @@ int gated_scan(const ScanArgs& a, SeqPos pos, cudaStream_t s) {
 #define LCC_SCAN(T, V)                                                                                            \
     do {                                                                                                          \
         if (smem > 48 * 1024) cudaFuncSetAttribute(gated_scan_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        gated_scan_kernel<T, V><<<grid, block, smem, s>>>(a, pos);                                                \
+        chained(gated_scan_kernel<T, V>, grid, block, smem, s)(a, pos);                                                \
     } while (0)
     if (a.dt == DT_F32) {
         if (a.vec_decay) LCC_SCAN(float, true); else LCC_SCAN(float, false);

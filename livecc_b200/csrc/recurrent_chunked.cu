@@ -80,6 +80,7 @@ struct ChunkArgs {
 
 // ---- 1: block-local cumulative sums of the log decays ---------------------------------------------------------------
 __global__ void chunk_cumsum_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     const int col = blockIdx.y * blockDim.x + threadIdx.x, ncol = a.heads * a.NV;
     if (col >= ncol) return;
@@ -101,6 +102,7 @@ __global__ void chunk_cumsum_kernel(ChunkArgs a, SeqPos pos) {
 // ---- 2: M[t, s] -------------------------------------------------------------------------------------------------------
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) chunk_weights_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     __shared__ float sc_[KS][PAD], sk_[KS][PAD], sb_[KS][PAD];
     // a decay per head: the product c k^T is the same for every head of a group, so a CTA forms it once per group and
@@ -169,6 +171,7 @@ __global__ void __launch_bounds__(256) chunk_weights_kernel(ChunkArgs a, SeqPos 
 // ---- 3: a block's own contribution to the state, stored [p][n] ----------------------------------------------------------
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) chunk_state_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     __shared__ Tile sh;
     const int blk = blockIdx.x / a.heads, h = blockIdx.x % a.heads, g = h / a.heads_per_group;
@@ -220,6 +223,7 @@ __global__ void __launch_bounds__(256) chunk_state_kernel(ChunkArgs a, SeqPos po
 // ---- 4: contributions -> the state that enters each block; the state after the last block goes back to the slot -----
 template <bool VEC>
 __global__ void chunk_prefix_kernel(ChunkArgs a, int nblocks, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     const size_t per = (size_t)a.heads * a.P * a.N;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -253,6 +257,7 @@ __global__ void chunk_prefix_kernel(ChunkArgs a, int nblocks, SeqPos pos) {
 // ---- 5: outputs ---------------------------------------------------------------------------------------------------------
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) chunk_output_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     __shared__ Tile sh;
     const int blk = blockIdx.x / a.heads, h = blockIdx.x % a.heads, g = h / a.heads_per_group;
@@ -383,6 +388,7 @@ __device__ __forceinline__ float row_of(const Acc84& acc, int i, int j) { return
 // ws_m[blk][group][t][s] = c_t . k_s
 template <typename T>
 __global__ void __launch_bounds__(128) chunk_products_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     __shared__ Slab sh;
     const int blk = blockIdx.x, g = blockIdx.y, groups = gridDim.y;
@@ -407,6 +413,7 @@ __global__ void __launch_bounds__(128) chunk_products_kernel(ChunkArgs a, SeqPos
 // a block's own contribution to the state, stored [p][n]
 template <typename T>
 __global__ void __launch_bounds__(128) chunk_state_head_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     __shared__ Slab sh;
     __shared__ float rowf[CL];   // per row: the step scale times the decay from the row to the block's end
@@ -441,6 +448,7 @@ __global__ void __launch_bounds__(128) chunk_state_head_kernel(ChunkArgs a, SeqP
 
 // contributions -> the state that enters each block (chunk_prefix_kernel, four neighbouring entries per thread)
 __global__ void __launch_bounds__(256) chunk_prefix4_kernel(ChunkArgs a, int nblocks, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     const size_t per = (size_t)a.heads * a.P * a.N;
     const size_t idx = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
@@ -473,6 +481,7 @@ __global__ void __launch_bounds__(256) chunk_prefix4_kernel(ChunkArgs a, int nbl
 
 template <typename T>
 __global__ void __launch_bounds__(128) chunk_output_head_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     __shared__ Slab sh;
     __shared__ float bt[CL], into[CL], scs[CL];   // per row: cumulative log decay, cs x decay from the block's start, cs x step scale
@@ -539,31 +548,31 @@ int run_chunked(const ScanArgs& s, SeqPos pos, cudaStream_t st) {
         a.ws_m = s.ws; a.ws_s = s.ws + (size_t)nb * s.heads * CL * CL;
         const int ncol = a.heads * a.NV;
         count_launch();
-        chunk_cumsum_kernel<<<dim3(nb, (ncol + 127) / 128), 128, 0, st>>>(a, pos);
+        chained(chunk_cumsum_kernel, dim3(nb, (ncol + 127) / 128), 128, 0, st)(a, pos);
         if constexpr (!VEC) {
             constexpr int V = Row16<T>::N;
             const bool rows16 = ((s.N | s.P | s.ld_k | s.ld_c | s.ld_u) % V) == 0 && ((s.N | s.P | s.ld_y) % 4) == 0 &&
                                 (((uintptr_t)s.k | (uintptr_t)s.c | (uintptr_t)s.u | (uintptr_t)s.y | (uintptr_t)s.state | (uintptr_t)a.ws_m | (uintptr_t)a.ws_s) % 16) == 0;
             if (rows16) {
                 count_launch();
-                chunk_products_kernel<T><<<dim3(nb, s.heads / s.heads_per_group), 128, 0, st>>>(a, pos);
+                chained(chunk_products_kernel<T>, dim3(nb, s.heads / s.heads_per_group), 128, 0, st)(a, pos);
                 count_launch();
-                chunk_state_head_kernel<T><<<dim3(nb * s.heads, (s.P + TS - 1) / TS), 128, 0, st>>>(a, pos);
+                chained(chunk_state_head_kernel<T>, dim3(nb * s.heads, (s.P + TS - 1) / TS), 128, 0, st)(a, pos);
                 count_launch();
-                chunk_prefix4_kernel<<<(unsigned)((per_state / 4 + 255) / 256), 256, 0, st>>>(a, nb, pos);
+                chained(chunk_prefix4_kernel, (unsigned)((per_state / 4 + 255) / 256), 256, 0, st)(a, nb, pos);
                 count_launch();
-                chunk_output_head_kernel<T><<<dim3(nb * s.heads, (s.P + TS - 1) / TS), 128, 0, st>>>(a, pos);
+                chained(chunk_output_head_kernel<T>, dim3(nb * s.heads, (s.P + TS - 1) / TS), 128, 0, st)(a, pos);
                 continue;
             }
         }
         count_launch();
-        chunk_weights_kernel<T, VEC><<<dim3(nb, VEC ? s.heads : s.heads / s.heads_per_group), 256, 0, st>>>(a, pos);
+        chained(chunk_weights_kernel<T, VEC>, dim3(nb, VEC ? s.heads : s.heads / s.heads_per_group), 256, 0, st)(a, pos);
         count_launch();
-        chunk_state_kernel<T, VEC><<<dim3(nb * s.heads, (s.P + TS - 1) / TS, (s.N + TS - 1) / TS), 256, 0, st>>>(a, pos);
+        chained(chunk_state_kernel<T, VEC>, dim3(nb * s.heads, (s.P + TS - 1) / TS, (s.N + TS - 1) / TS), 256, 0, st)(a, pos);
         count_launch();
-        chunk_prefix_kernel<VEC><<<(unsigned)((per_state + 255) / 256), 256, 0, st>>>(a, nb, pos);
+        chained(chunk_prefix_kernel<VEC>, (unsigned)((per_state + 255) / 256), 256, 0, st)(a, nb, pos);
         count_launch();
-        chunk_output_kernel<T, VEC><<<dim3(nb * s.heads, (s.P + TS - 1) / TS), 256, 0, st>>>(a, pos);
+        chained(chunk_output_kernel<T, VEC>, dim3(nb * s.heads, (s.P + TS - 1) / TS), 256, 0, st)(a, pos);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }

@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(256) rotary_pack_kernel(const T* __restrict__ 
                                                           Segs segs, const float* __restrict__ inv_freq, float mag,
                                                           const float* __restrict__ fill, float* __restrict__ fill_out, int fill_n,
                                                           SeqPos pos) {
+    chain_begin();
     if (seq_done(pos)) return;
     const int t = blockIdx.x;
     const float p = (float)(seq_past(pos) + t);
@@ -97,7 +98,7 @@ int rotary_pack_f32(int dt, const void* in, int ld_in, float* out, int ld_out, c
         any = any || seg[i].rot_dims == 0;
     }
     vec = vec && any;
-#define LCC_PACK(T, V) rotary_pack_kernel<T, V><<<S_grid, 256, 0, s>>>((const T*)in, ld_in, out, ld_out, g, inv_freq, mag, fill, fill_out, fill_n, pos)
+#define LCC_PACK(T, V) chained(rotary_pack_kernel<T, V>, S_grid, 256, 0, s)((const T*)in, ld_in, out, ld_out, g, inv_freq, mag, fill, fill_out, fill_n, pos)
     if (dt == DT_F32) { if (vec) LCC_PACK(float, true); else LCC_PACK(float, false); }
     else { if (vec) LCC_PACK(bf16, true); else LCC_PACK(bf16, false); }
 #undef LCC_PACK

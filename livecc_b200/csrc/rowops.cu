@@ -46,6 +46,7 @@ template <typename T>
 __global__ void embed_sinusoid_kernel(const int64_t* __restrict__ ids, const int* __restrict__ seq_len, const T* __restrict__ table,
                                       int64_t vocab, float scale, const float* __restrict__ inv_freq, float* __restrict__ x32,
                                       T* __restrict__ xa, int S, int W, SeqPos pos, int copies) {
+    chain_begin();
     if (seq_done(pos)) return;
     const int r = blockIdx.x;
     const int64_t id = seq_len ? ids[*seq_len - S + r] : ids[r];
@@ -71,6 +72,7 @@ __global__ void __launch_bounds__(256) postnorm_residual_kernel(float* __restric
                                                                 int ld_a, const float* __restrict__ wa, const T* __restrict__ b,
                                                                 int ld_b, const float* __restrict__ wb, const float* __restrict__ w,
                                                                 float alpha, float eps, int W) {
+    chain_begin();
     __shared__ float red[32];
     const int r = blockIdx.x;
     float* x = x32 + (size_t)r * W;
@@ -150,6 +152,7 @@ template <typename T, int E, bool VEC>
 __global__ void __launch_bounds__(256) postnorm_branch_kernel(float* __restrict__ x32, T* __restrict__ xa, const T* __restrict__ a, int ld_a,
                                                               bool has_mc, MoeCombine mc, const float* __restrict__ ls,
                                                               const float* __restrict__ w, float alpha, float eps, int W) {
+    chain_begin();
     __shared__ float red[32];
     __shared__ int spos[kCombineTop];
     __shared__ float swt[kCombineTop];
@@ -249,6 +252,7 @@ template <typename T, int TEAM, int E>
 __global__ void __launch_bounds__(256) gated_group_norm_kernel(const float* __restrict__ y, int ld_y, const T* __restrict__ gate,
                                                                int ld_gate, const float* __restrict__ w, int w_len, T* __restrict__ out,
                                                                int ld_out, int S, int n, int group, int gate_first, float eps) {
+    chain_begin();
     __shared__ float red[32];
     const int ngroups = n / group;
     const int wid = TEAM == 32 ? blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x;
@@ -311,6 +315,7 @@ template <typename T, int TEAM, int E>
 __global__ void __launch_bounds__(TEAM == 32 ? 64 : TEAM) gated_group_norm4_kernel(const float* __restrict__ y, int ld_y, const T* __restrict__ gate,
                                                                 int ld_gate, const float* __restrict__ w, int w_len, T* __restrict__ out,
                                                                 int ld_out, int S, int n, int group, int gate_first, float eps) {
+    chain_begin();
     __shared__ float red[32];
     const int ngroups = n / group, wid = TEAM == 32 ? blockIdx.x * 2 + (threadIdx.x >> 5) : blockIdx.x, lane = TEAM == 32 ? (threadIdx.x & 31) : threadIdx.x;
     if (wid >= S * ngroups) return;
@@ -353,6 +358,7 @@ __global__ void __launch_bounds__(TEAM == 32 ? 64 : TEAM) gated_group_norm4_kern
 // four columns per thread where the rows allow it (NV = 4), else one
 template <typename T, int NV>
 __global__ void __launch_bounds__(256) glu_gelu_tanh_kernel(const T* __restrict__ gu, int ld, T* __restrict__ out, int ld_out, int S, int F) {
+    chain_begin();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * NV;
     if (i >= (int64_t)S * F) return;
     const int r = (int)(i / F), c = (int)(i % F);
@@ -369,6 +375,7 @@ __global__ void __launch_bounds__(256) glu_gelu_tanh_kernel(const T* __restrict_
 template <typename T>
 __global__ void __launch_bounds__(256) gather_rmsnorm_kernel(const float* __restrict__ x32, const int* __restrict__ rows,
                                                              const float* __restrict__ w, float eps, T* __restrict__ out, int W) {
+    chain_begin();
     __shared__ float red[32];
     const int i = blockIdx.x;
     const float* x = x32 + (size_t)rows[i] * W;
@@ -383,6 +390,7 @@ __global__ void __launch_bounds__(256) gather_rmsnorm_kernel(const float* __rest
 template <typename T>
 __global__ void __launch_bounds__(128) slice_rmsnorm_kernel(const T* __restrict__ in, int ld_in, const float* __restrict__ w, float eps,
                                                             T* __restrict__ out, int ld_out, int n) {
+    chain_begin();
     __shared__ float red[32];
     const T* x = in + (size_t)blockIdx.x * ld_in;
     float ss = 0.f;
@@ -393,6 +401,7 @@ __global__ void __launch_bounds__(128) slice_rmsnorm_kernel(const T* __restrict_
 }
 
 __global__ void softcap_kernel(float* __restrict__ x, int64_t n, float cap, float inv_cap, float scale) {
+    chain_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = (cap > 0.f ? cap * tanhf(x[i] * inv_cap) : x[i]) * scale;
 }
@@ -404,6 +413,7 @@ __device__ __forceinline__ float norm_apply(const NormSpec& n, float v, float rn
 template <typename T>
 __global__ void __launch_bounds__(256) gather_norm_kernel(const float* __restrict__ x32, const int* __restrict__ rows, NormSpec n,
                                                           T* __restrict__ out, int W) {
+    chain_begin();
     __shared__ float red[32];
     const int i = blockIdx.x;
     const float* x = x32 + (size_t)rows[i] * W;
@@ -430,6 +440,7 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ x32, const T* __restrict__ a, int ld_a,
                                                             const T* __restrict__ b, int ld_b, bool has_mc, MoeCombine mc, NormSpec n,
                                                             T* __restrict__ xa, int W) {
+    chain_begin();
     __shared__ float red[32];
     __shared__ int spos[kCombineTop];
     __shared__ float swt[kCombineTop];
@@ -512,6 +523,7 @@ __global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ 
 template <typename T>
 __global__ void glu_clamp_swish_kernel(const T* __restrict__ gu, int ld, T* __restrict__ out, int ld_out, int S, int F, float limit, bool il16,
                                        float alpha, float up_bias) {
+    chain_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)S * F) return;
     const int r = (int)(i / F), c = (int)(i % F);
@@ -529,6 +541,7 @@ template <typename T, int E, bool VEC>
 __global__ void __launch_bounds__(256) branch_norm_residual_kernel(float* __restrict__ x32, const T* __restrict__ a, int ld_a, bool has_mc,
                                                                    MoeCombine mc, const float* __restrict__ w, float eps,
                                                                    T* __restrict__ xa, int W) {
+    chain_begin();
     __shared__ float red[32];
     __shared__ int spos[kCombineTop];
     __shared__ float swt[kCombineTop];
@@ -623,6 +636,7 @@ __global__ void __launch_bounds__(256) branch_norm_residual_kernel(float* __rest
 template <typename T, int E, bool VEC>
 __global__ void __launch_bounds__(256) sandwich_residual_kernel(float* __restrict__ x32, const T* __restrict__ a, int ld_a, bool has_mc,
                                                                 MoeCombine mc, NormSpec post, NormSpec next, T* __restrict__ xa, int W) {
+    chain_begin();
     __shared__ float red[32];
     __shared__ int spos[kCombineTop];
     __shared__ float swt[kCombineTop];
@@ -752,9 +766,9 @@ int embed_sinusoid(int dt, const int64_t* ids, const int* seq_len, const void* t
     if (!ids || !table || !x32 || S < 1 || W < 1 || copies < 1) return -2;
     count_launch();
     if (dt == DT_F32)
-        embed_sinusoid_kernel<float><<<S, 256, 0, s>>>(ids, seq_len, (const float*)table, vocab, scale, inv_freq, x32, (float*)xa, S, W, pos, copies);
+        chained(embed_sinusoid_kernel<float>, S, 256, 0, s)(ids, seq_len, (const float*)table, vocab, scale, inv_freq, x32, (float*)xa, S, W, pos, copies);
     else
-        embed_sinusoid_kernel<bf16><<<S, 256, 0, s>>>(ids, seq_len, (const bf16*)table, vocab, scale, inv_freq, x32, (bf16*)xa, S, W, pos, copies);
+        chained(embed_sinusoid_kernel<bf16>, S, 256, 0, s)(ids, seq_len, (const bf16*)table, vocab, scale, inv_freq, x32, (bf16*)xa, S, W, pos, copies);
     return done();
 }
 
@@ -772,8 +786,8 @@ int postnorm_residual(int dt, float* x32, void* xa, const void* a, int ld_a, con
                          (!mc || (ok4(m.eo, m.ld_eo) && ok4(m.so, m.ld_so)));
 #define LCC_PNB2(E, VECB)                                                                                                      \
     do {                                                                                                                       \
-        if (dt == DT_F32) postnorm_branch_kernel<float, E, VECB><<<S, 256, 0, s>>>(x32, (float*)xa, (const float*)a, ld_a, mc != nullptr, m, ls, w, alpha, eps, W); \
-        else postnorm_branch_kernel<bf16, E, VECB><<<S, 256, 0, s>>>(x32, (bf16*)xa, (const bf16*)a, ld_a, mc != nullptr, m, ls, w, alpha, eps, W);                 \
+        if (dt == DT_F32) chained(postnorm_branch_kernel<float, E, VECB>, S, 256, 0, s)(x32, (float*)xa, (const float*)a, ld_a, mc != nullptr, m, ls, w, alpha, eps, W); \
+        else chained(postnorm_branch_kernel<bf16, E, VECB>, S, 256, 0, s)(x32, (bf16*)xa, (const bf16*)a, ld_a, mc != nullptr, m, ls, w, alpha, eps, W);                 \
     } while (0)
 #define LCC_PNB(E) do { if (vec) LCC_PNB2(E, true); else LCC_PNB2(E, false); } while (0)
         const int pieces = (W / (vec ? 4 : 1) + 255) / 256;      // per thread: the form depends on the row's width alone
@@ -790,9 +804,9 @@ int postnorm_residual(int dt, float* x32, void* xa, const void* a, int ld_a, con
 #define LCC_PNR(E)                                                                                                          \
     do {                                                                                                                    \
         if (dt == DT_F32)                                                                                                   \
-            postnorm_residual_kernel<float, E><<<S, 256, 0, s>>>(x32, (float*)xa, (const float*)a, ld_a, wa, (const float*)b, ld_b, wb, w, alpha, eps, W); \
+            chained(postnorm_residual_kernel<float, E>, S, 256, 0, s)(x32, (float*)xa, (const float*)a, ld_a, wa, (const float*)b, ld_b, wb, w, alpha, eps, W); \
         else                                                                                                                \
-            postnorm_residual_kernel<bf16, E><<<S, 256, 0, s>>>(x32, (bf16*)xa, (const bf16*)a, ld_a, wa, (const bf16*)b, ld_b, wb, w, alpha, eps, W); \
+            chained(postnorm_residual_kernel<bf16, E>, S, 256, 0, s)(x32, (bf16*)xa, (const bf16*)a, ld_a, wa, (const bf16*)b, ld_b, wb, w, alpha, eps, W); \
     } while (0)
     const int per = (W + 255) / 256;
     if (per <= 2) LCC_PNR(2);
@@ -817,10 +831,10 @@ int gated_group_norm(int dt, const float* y, int ld_y, const void* gate, int ld_
     do {                                                                                                                        \
         const int grid = TEAM == 32 ? (teams + 1) / 2 : teams, block = TEAM == 32 ? 64 : TEAM;                                  \
         if (dt == DT_F32)                                                                                                       \
-            gated_group_norm4_kernel<float, TEAM, E><<<grid, block, 0, s>>>(y, ld_y, (const float*)gate, ld_gate, w, w_len,     \
+            chained(gated_group_norm4_kernel<float, TEAM, E>, grid, block, 0, s)(y, ld_y, (const float*)gate, ld_gate, w, w_len,     \
                                                                             (float*)out, ld_out, S, n, group, gate_first, eps); \
         else                                                                                                                    \
-            gated_group_norm4_kernel<bf16, TEAM, E><<<grid, block, 0, s>>>(y, ld_y, (const bf16*)gate, ld_gate, w, w_len,       \
+            chained(gated_group_norm4_kernel<bf16, TEAM, E>, grid, block, 0, s)(y, ld_y, (const bf16*)gate, ld_gate, w, w_len,       \
                                                                            (bf16*)out, ld_out, S, n, group, gate_first, eps);   \
     } while (0)
         if (group <= 256) LCC_GGN4(32, 2);
@@ -833,10 +847,10 @@ int gated_group_norm(int dt, const float* y, int ld_y, const void* gate, int ld_
 #define LCC_GGN(TEAM, E, GRID)                                                                                            \
     do {                                                                                                                  \
         if (dt == DT_F32)                                                                                                 \
-            gated_group_norm_kernel<float, TEAM, E><<<GRID, 256, 0, s>>>(y, ld_y, (const float*)gate, ld_gate, w, w_len, (float*)out, \
+            chained(gated_group_norm_kernel<float, TEAM, E>, GRID, 256, 0, s)(y, ld_y, (const float*)gate, ld_gate, w, w_len, (float*)out, \
                                                                          ld_out, S, n, group, gate_first, eps);           \
         else                                                                                                              \
-            gated_group_norm_kernel<bf16, TEAM, E><<<GRID, 256, 0, s>>>(y, ld_y, (const bf16*)gate, ld_gate, w, w_len, (bf16*)out,    \
+            chained(gated_group_norm_kernel<bf16, TEAM, E>, GRID, 256, 0, s)(y, ld_y, (const bf16*)gate, ld_gate, w, w_len, (bf16*)out,    \
                                                                         ld_out, S, n, group, gate_first, eps);            \
     } while (0)
     if (group <= 128) {
@@ -861,7 +875,7 @@ int glu_gelu_tanh(int dt, const void* gu, int ld, void* out, int ld_out, int S, 
     const bool quads = ((F | ld | ld_out) % 4) == 0 && ((uintptr_t)gu % (4 * es)) == 0 && ((uintptr_t)out % (4 * es)) == 0;
     const unsigned blocks = (unsigned)((n / (quads ? 4 : 1) + 255) / 256);
     count_launch();
-#define LCC_GLU(T, NV) glu_gelu_tanh_kernel<T, NV><<<blocks, 256, 0, s>>>((const T*)gu, ld, (T*)out, ld_out, S, F)
+#define LCC_GLU(T, NV) chained(glu_gelu_tanh_kernel<T, NV>, blocks, 256, 0, s)((const T*)gu, ld, (T*)out, ld_out, S, F)
     if (dt == DT_F32) { if (quads) LCC_GLU(float, 4); else LCC_GLU(float, 1); }
     else { if (quads) LCC_GLU(bf16, 4); else LCC_GLU(bf16, 1); }
 #undef LCC_GLU
@@ -873,9 +887,9 @@ int gather_rmsnorm(int dt, const float* x32, const int* rows, const float* w, fl
     if (!x32 || !rows || !w || !out || n_rows < 1 || W < 1) return -2;
     count_launch();
     if (dt == DT_F32)
-        gather_rmsnorm_kernel<float><<<n_rows, 256, 0, s>>>(x32, rows, w, eps, (float*)out, W);
+        chained(gather_rmsnorm_kernel<float>, n_rows, 256, 0, s)(x32, rows, w, eps, (float*)out, W);
     else
-        gather_rmsnorm_kernel<bf16><<<n_rows, 256, 0, s>>>(x32, rows, w, eps, (bf16*)out, W);
+        chained(gather_rmsnorm_kernel<bf16>, n_rows, 256, 0, s)(x32, rows, w, eps, (bf16*)out, W);
     return done();
 }
 
@@ -883,9 +897,9 @@ int slice_rmsnorm(int dt, const void* in, int ld_in, const float* w, float eps, 
     if (!in || !w || !out || S < 1 || n < 1 || ld_in < n || ld_out < n) return -2;
     count_launch();
     if (dt == DT_F32)
-        slice_rmsnorm_kernel<float><<<S, 128, 0, s>>>((const float*)in, ld_in, w, eps, (float*)out, ld_out, n);
+        chained(slice_rmsnorm_kernel<float>, S, 128, 0, s)((const float*)in, ld_in, w, eps, (float*)out, ld_out, n);
     else
-        slice_rmsnorm_kernel<bf16><<<S, 128, 0, s>>>((const bf16*)in, ld_in, w, eps, (bf16*)out, ld_out, n);
+        chained(slice_rmsnorm_kernel<bf16>, S, 128, 0, s)((const bf16*)in, ld_in, w, eps, (bf16*)out, ld_out, n);
     return done();
 }
 
@@ -893,7 +907,7 @@ int softcap(float* x, int64_t n, float cap, cudaStream_t s, float scale) {
     if (!x || n < 1) return -2;
     if (!(cap > 0.f) && scale == 1.f) return 0;
     count_launch();
-    softcap_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(x, n, cap > 0.f ? cap : 0.f, cap > 0.f ? 1.f / cap : 0.f, scale);
+    chained(softcap_kernel, (unsigned)((n + 255) / 256), 256, 0, s)(x, n, cap > 0.f ? cap : 0.f, cap > 0.f ? 1.f / cap : 0.f, scale);
     return done();
 }
 
@@ -902,9 +916,9 @@ int gather_norm(int dt, const float* x32, const int* rows, const NormSpec& n, vo
         return -2;
     count_launch();
     if (dt == DT_F32)
-        gather_norm_kernel<float><<<n_rows, 256, 0, s>>>(x32, rows, n, (float*)out, W);
+        chained(gather_norm_kernel<float>, n_rows, 256, 0, s)(x32, rows, n, (float*)out, W);
     else
-        gather_norm_kernel<bf16><<<n_rows, 256, 0, s>>>(x32, rows, n, (bf16*)out, W);
+        chained(gather_norm_kernel<bf16>, n_rows, 256, 0, s)(x32, rows, n, (bf16*)out, W);
     return done();
 }
 
@@ -922,7 +936,7 @@ int residual_norm(int dt, float* x32, const void* a, int ld_a, const void* b, in
     const bool vec = (W % 4) == 0 && ((uintptr_t)x32 % 16) == 0 && ok4(a, ld_a) && ok4(b, ld_b) && ok4(xa, W) &&
                      (!mc || (ok4(m.eo, m.ld_eo) && ok4(m.so, m.ld_so)));
 #define LCC_RN(T, VECB)                                                                                                      \
-    residual_norm_kernel<T, VECB><<<S, 256, 0, s>>>(x32, (const T*)a, ld_a, (const T*)b, ld_b, mc != nullptr, m, next, (T*)xa, W)
+    chained(residual_norm_kernel<T, VECB>, S, 256, 0, s)(x32, (const T*)a, ld_a, (const T*)b, ld_b, mc != nullptr, m, next, (T*)xa, W)
     if (dt == DT_F32) { if (vec) LCC_RN(float, true); else LCC_RN(float, false); }
     else { if (vec) LCC_RN(bf16, true); else LCC_RN(bf16, false); }
 #undef LCC_RN
@@ -941,8 +955,8 @@ int branch_norm_residual(int dt, float* x32, const void* a, int ld_a, const MoeC
                      (!mc || (ok4(m.eo, m.ld_eo) && ok4(m.so, m.ld_so)));
 #define LCC_BNR2(E, VECB)                                                                                                      \
     do {                                                                                                                       \
-        if (dt == DT_F32) branch_norm_residual_kernel<float, E, VECB><<<S, 256, 0, s>>>(x32, (const float*)a, ld_a, mc != nullptr, m, w, eps, (float*)xa, W); \
-        else branch_norm_residual_kernel<bf16, E, VECB><<<S, 256, 0, s>>>(x32, (const bf16*)a, ld_a, mc != nullptr, m, w, eps, (bf16*)xa, W);                 \
+        if (dt == DT_F32) chained(branch_norm_residual_kernel<float, E, VECB>, S, 256, 0, s)(x32, (const float*)a, ld_a, mc != nullptr, m, w, eps, (float*)xa, W); \
+        else chained(branch_norm_residual_kernel<bf16, E, VECB>, S, 256, 0, s)(x32, (const bf16*)a, ld_a, mc != nullptr, m, w, eps, (bf16*)xa, W);                 \
     } while (0)
 #define LCC_BNR(E) do { if (vec) LCC_BNR2(E, true); else LCC_BNR2(E, false); } while (0)
     const int per = (W / (vec ? 4 : 1) + 255) / 256;      // pieces per thread: the form depends on the row's width alone
@@ -970,8 +984,8 @@ int sandwich_residual(int dt, float* x32, const void* a, int ld_a, const MoeComb
                      ok4(xa, W) && (!mc || (ok4(m.eo, m.ld_eo) && ok4(m.so, m.ld_so)));
 #define LCC_SR2(E, VECB)                                                                                                       \
     do {                                                                                                                       \
-        if (dt == DT_F32) sandwich_residual_kernel<float, E, VECB><<<S, 256, 0, s>>>(x32, (const float*)a, ld_a, mc != nullptr, m, post, next, (float*)xa, W); \
-        else sandwich_residual_kernel<bf16, E, VECB><<<S, 256, 0, s>>>(x32, (const bf16*)a, ld_a, mc != nullptr, m, post, next, (bf16*)xa, W);                 \
+        if (dt == DT_F32) chained(sandwich_residual_kernel<float, E, VECB>, S, 256, 0, s)(x32, (const float*)a, ld_a, mc != nullptr, m, post, next, (float*)xa, W); \
+        else chained(sandwich_residual_kernel<bf16, E, VECB>, S, 256, 0, s)(x32, (const bf16*)a, ld_a, mc != nullptr, m, post, next, (bf16*)xa, W);                 \
     } while (0)
 #define LCC_SR(E) do { if (vec) LCC_SR2(E, true); else LCC_SR2(E, false); } while (0)
     const int per = (W / (vec ? 4 : 1) + 255) / 256;      // pieces per thread: the form depends on the row's width alone
@@ -992,9 +1006,9 @@ int glu_clamp_swish(int dt, const void* gu, int ld, void* out, int ld_out, int S
     const int64_t n = (int64_t)S * F;
     count_launch();
     if (dt == DT_F32)
-        glu_clamp_swish_kernel<float><<<(unsigned)((n + 255) / 256), 256, 0, s>>>((const float*)gu, ld, (float*)out, ld_out, S, F, limit, il16, alpha, up_bias);
+        chained(glu_clamp_swish_kernel<float>, (unsigned)((n + 255) / 256), 256, 0, s)((const float*)gu, ld, (float*)out, ld_out, S, F, limit, il16, alpha, up_bias);
     else
-        glu_clamp_swish_kernel<bf16><<<(unsigned)((n + 255) / 256), 256, 0, s>>>((const bf16*)gu, ld, (bf16*)out, ld_out, S, F, limit, il16, alpha, up_bias);
+        chained(glu_clamp_swish_kernel<bf16>, (unsigned)((n + 255) / 256), 256, 0, s)((const bf16*)gu, ld, (bf16*)out, ld_out, S, F, limit, il16, alpha, up_bias);
     return done();
 }
 

@@ -479,6 +479,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
     const lcc_seq_model_desc& d = m->d;
     const int dt = d.dtype, W = d.width;
     const size_t es = lcc::dt_size(dt);
+    const lcc::ChainScope chain;
     const WsLayout L = make_layout(m, m->cap_tokens, m->cap_want);
     uint8_t* ws = m->ws;
     float* x32 = (float*)(ws + L.x32);
@@ -815,6 +816,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
         if (has_ff && hc) STEP(boundary(l.hc2_f32, l.norm2_f32, nullptr), "stream boundary");
         lcc::MoeCombine par_mc{};       // blocks on one stream: the routed feed-forward's row is formed by the layer's residual kernel
         bool par_is_mc = false;
+        if (fork_ff) lcc::chain_break();
         if (l.ff_kind == LCC_FF_MOE) {
             // E real experts own row lists; the router has EO = E + identity outputs
             const bool glu = l.e_act == LCC_EXPERT_CLAMP_GLU || l.e_act == LCC_EXPERT_SILU_GLU;
@@ -843,6 +845,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
             const bool fork = shared && m->side && T <= kForkMaxRows && !fork_ff;
             if (fork && (cudaEventRecord(m->ev_fork, fs) != cudaSuccess || cudaStreamWaitEvent(m->side, m->ev_fork, 0) != cudaSuccess))
                 LCC_FAIL(m->ctx, -100, "stream fork failed");
+            if (fork) lcc::chain_break();
             if (shared) {
                 cudaStream_t ss = fork ? m->side : fs;
                 STEP(linear(m, xa, W, l.e_shared_up, nullptr, mid2, lds, false, T, l.e_shared_ff, W, ss, nullptr,
@@ -857,6 +860,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
             } else {
                 if (cudaMemsetAsync(counts, 0, sizeof(int) * E, fs) != cudaSuccess) LCC_FAIL(m->ctx, -100, "router counters");
                 if (tc && cudaMemsetAsync(src_row, 0xff, sizeof(int) * (size_t)n_tiles * kMoeTile, fs) != cudaSuccess) LCC_FAIL(m->ctx, -100, "row lists");
+                lcc::chain_break();
                 STEP(lcc::moe_route(logit, lde, l.e_correction_f32, EO, K, l.e_scale, sel, wsel, gate_out, counts, rank, T, fs, &ro), "expert choice");
                 STEP(lcc::moe_index(sel, rank, counts, E, K, tc ? kMoeTile : 1, row_off, posn, src_row, tc ? tile_group : nullptr, n_tiles, T, fs), "expert row lists");
             }
@@ -894,6 +898,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
             }
             if (fork && (cudaEventRecord(m->ev_join, m->side) != cudaSuccess || cudaStreamWaitEvent(fs, m->ev_join, 0) != cudaSuccess))
                 LCC_FAIL(m->ctx, -100, "stream join failed");
+            if (fork) lcc::chain_break();
             if (hc) {   // the weighted sum of the experts' rows is formed by the boundary kernel that folds it into the streams
                 pend_mc = lcc::MoeCombine{eo, ldw8, posn, wsel, K, shared ? o2 : nullptr, W, gate_out};
                 pend_is_mc = true;
@@ -919,6 +924,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
         }
         if (fork_ff && (cudaEventRecord(m->ev_join, m->side) != cudaSuccess || cudaStreamWaitEvent(s, m->ev_join, 0) != cudaSuccess))
             LCC_FAIL(m->ctx, -100, "stream join failed");
+        if (fork_ff) lcc::chain_break();
         if (par) {
             // x <- x + (mixer + feed-forward), then the next layer's norm of the new row
             STEP(lcc::residual_norm(dt, x32, o1, W, (has_ff && !par_is_mc) ? o2 : nullptr, W, par_is_mc ? &par_mc : nullptr, norm_of(li + 1),
@@ -939,6 +945,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
         if (layer_dump && !hc) {
             if (cudaMemcpyAsync(layer_dump + (size_t)li * T * W, x32, (size_t)T * W * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
                 LCC_FAIL(m->ctx, -100, "layer dump copy failed");
+            lcc::chain_break();
         }
     }
     if (hc) {
