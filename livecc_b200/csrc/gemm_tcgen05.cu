@@ -582,6 +582,14 @@ int make_tmap_bf16_2d(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t co
     return make_tmap_bf16_2d_box(tm, ptr, rows, cols, ld, BLOCK_K, box_rows, false);
 }
 
+// The clamped GLU has no residual and no bias: those slots carry the clamp, the slope and the offset.
+static void glu_slots(const GemmArgs& a, int& ldr, const bf16*& bias) {
+    memcpy(&ldr, &a.epi_param, sizeof(int));
+    const float ab[2] = {a.epi_alpha, a.epi_up_bias};
+    static_assert(sizeof(bias) == sizeof(ab), "two floats ride in a pointer");
+    memcpy(&bias, ab, sizeof(ab));
+}
+
 template <int EPI>
 static int launch_cfg(const GemmArgs& a, int bn, int num_sms, cudaStream_t stream) {
     const GemmTile cfg = make_tile(bn);
@@ -600,12 +608,7 @@ static int launch_cfg(const GemmArgs& a, int bn, int num_sms, cudaStream_t strea
     lcc::count_launch();
     int ldr = a.ldr;
     const bf16* bias = (const bf16*)a.bias;
-    if (EPI == EPI_CLAMP_GLU) {   // no residual and no bias in this epilogue: the slots carry the clamp, the slope and the offset
-        memcpy(&ldr, &a.epi_param, sizeof(int));
-        const float ab[2] = {a.epi_alpha, a.epi_up_bias};
-        static_assert(sizeof(bias) == sizeof(ab), "two floats ride in a pointer");
-        memcpy(&bias, ab, sizeof(ab));
-    }
+    if (EPI == EPI_CLAMP_GLU) glu_slots(a, ldr, bias);
     kern<<<grid, 384, cfg.smem_bytes, stream>>>(ta, tb, (bf16*)a.C, a.M, a.N, a.K, a.ldc,
                                                 bias, (const bf16*)a.residual,
                                                 ldr, splits, cfg, a.tile_group, batch, a.a_col_stride, a.c_col_stride);
@@ -626,8 +629,10 @@ static int launch_cfg2(const GemmArgs& a, int bn, int num_sms, cudaStream_t stre
     const int units = m_pairs * n_tiles * splits;
     const int pairs = units < num_sms / 2 ? units : num_sms / 2;
     lcc::count_launch();
-    kern<<<2 * pairs, 384, cfg.smem_bytes, stream>>>(ta, tb, (bf16*)a.C, a.M, a.N, a.K, a.ldc, (const bf16*)a.bias,
-                                                     (const bf16*)a.residual, a.ldr, splits, cfg);
+    int ldr = a.ldr;
+    const bf16* bias = (const bf16*)a.bias;
+    if (EPI == EPI_CLAMP_GLU) glu_slots(a, ldr, bias);
+    kern<<<2 * pairs, 384, cfg.smem_bytes, stream>>>(ta, tb, (bf16*)a.C, a.M, a.N, a.K, a.ldc, bias, (const bf16*)a.residual, ldr, splits, cfg);
     return cudaGetLastError() == cudaSuccess ? 0 : -13;
 }
 
@@ -640,6 +645,10 @@ static int launch_epi2(const GemmArgs& a, int bn, int num_sms, cudaStream_t stre
         case EPI_RESIDUAL: return launch_cfg2<EPI_RESIDUAL>(a, bn, num_sms, stream);
         case EPI_BIAS_RESIDUAL: return launch_cfg2<EPI_BIAS_RESIDUAL>(a, bn, num_sms, stream);
         case EPI_SWIGLU: return launch_cfg2<EPI_SWIGLU>(a, bn, num_sms, stream);
+        case EPI_RELU2: return launch_cfg2<EPI_RELU2>(a, bn, num_sms, stream);
+        case EPI_GELU_TANH: return launch_cfg2<EPI_GELU_TANH>(a, bn, num_sms, stream);
+        case EPI_GELU_ERF: return launch_cfg2<EPI_GELU_ERF>(a, bn, num_sms, stream);
+        case EPI_CLAMP_GLU: return launch_cfg2<EPI_CLAMP_GLU>(a, bn, num_sms, stream);
     }
     return -14;
 }
@@ -680,6 +689,30 @@ static int choose_bn(int M, int N, int num_sms) {
         return ((tiles + num_sms - 1) / num_sms) * (long long)(128 + bn);
     };
     return cost(128) <= cost(256) ? 128 : 256;
+}
+
+// Is the CTA pair's kernel the better one, and with which width (0: it is not)? A pair brings in half the bytes per multiplication, so its
+// time per 64-deep k-block grows with the width only: 0.295, 0.30, 0.325, 0.355, 0.37 us for 128, 160, 192, 224, 256 columns, where a CTA
+// alone takes 0.28 us for 128 and 0.41 for 256; against that it has 74 units of 256 rows for 148 of 128, and a launch of 9.5 us for 8. Waves
+// x k-blocks x these plus the launch predict which of the two wins for the shapes of the models (M = 281 to 8192, us, alone | pair):
+// 2048 x 10304 x 2048 75 | 65, 2048 x 5120 x 5120 107 | 92, 1200 x 4608 x 3584 55 | 44, 2090 x 4608 x 3584 66 | 61, 2090 x 3584 x 18944
+// 250 | 219, 8192 x 3840 x 1280 69 | 66, 512 x 10304 x 2048 31 | 27; alone stays for 281 x 37888 x 3584 81 | 91, 1024 x 3840 x 1280 16 | 17,
+// 256 x 5120 x 5120 31 | 33. Where the model sees less than 3 % the two measure the same. Every sum runs over k in the same order.
+static int choose_pair(int M, int N, int K, int num_sms) {
+    const long long nkb = (K + BLOCK_K - 1) / BLOCK_K;
+    auto waves = [](long long units, int at_once) { return (double)((units + at_once - 1) / at_once); };
+    const int bn1 = choose_bn(M, N, num_sms);
+    if (bn1 < 128 || num_sms < 2) return 0;
+    const double alone = 8.0 + waves((long long)((M + BLOCK_M - 1) / BLOCK_M) * ((N + bn1 - 1) / bn1), num_sms) * nkb * (bn1 == 128 ? 0.28 : 0.41);
+    const double per_kb[5] = {0.295, 0.30, 0.325, 0.355, 0.37};
+    double best = 0.97 * alone;
+    int width = 0;
+    for (int i = 0; i < 5; ++i) {
+        const int bn = 128 + 32 * i;
+        const double t = 9.5 + waves((long long)((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + bn - 1) / bn), num_sms / 2) * nkb * per_kb[i];
+        if (t < best) { best = t; width = bn; }
+    }
+    return width;
 }
 
 // Sum of the split-K partials + the fused epilogue (same rounding points as the in-kernel epilogues):
@@ -792,9 +825,11 @@ int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream) {
             forced = e ? atoi(e) : 0;
         }
         block_n = forced > 0 ? forced : choose_bn(a.M, a.N, num_sms);
+        if (forced <= 0 && plain && a.epi != EPI_SIGMOID_GATE)
+            if (const int width = choose_pair(a.M, a.N, a.K, num_sms)) block_n = -width;
     }
-    // block_n < 0 selects the CTA-pair kernel with tile width -block_n (explicit: tests and tuning)
-    const bool pair = block_n < 0 && plain && a.epi != EPI_RELU2 && a.epi != EPI_GELU_TANH && a.epi != EPI_GELU_ERF && a.epi != EPI_CLAMP_GLU && a.epi != EPI_SIGMOID_GATE;
+    // block_n < 0: the CTA pair's kernel with tile width -block_n
+    const bool pair = block_n < 0 && plain && a.epi != EPI_SIGMOID_GATE && (a.epi <= EPI_SWIGLU || block_n % 32 == 0);
     if (block_n < 0) block_n = -block_n;
     if (block_n < 32 || block_n > 256 || (block_n % 16) || ((a.epi == EPI_SWIGLU || a.epi == EPI_CLAMP_GLU) && (block_n % 32))) return -6;
     if (pair) return (block_n % 32) ? -6 : launch_epi2(a, block_n, num_sms, stream);

@@ -116,6 +116,15 @@ def test_gemm_epilogues_every_tile_width(ctx, block_n):
         assert torch.equal(ctx.gemm(a, b, epilogue=epi, block_n=block_n, **kw), ctx.gemm(a, b, epilogue=epi, block_n=256, **kw)), epi
 
 
+@pytest.mark.parametrize("M,N,K,epi", [(2048, 10304, 1160, 8), (2049, 10304, 1096, 9), (2303, 5120, 1224, 11), (1281, 4640, 1096, A.EPI_SWIGLU),
+                                       (2090, 4616, 1088, A.EPI_NONE), (513, 10312, 1344, A.EPI_NONE)])   # 8, 9, 11: relu^2, tanh gelu, erf gelu
+def test_gemm_default_kernel_equals_one_cta(ctx, M, N, K, epi):
+    """Large products run on CTA pairs by default: the same sums in the same order as the one-CTA kernel, every epilogue."""
+    a, b = _ints((M, K), -2, 2, 21), _ints((N, K), -2, 2, 22)
+    a, b = (a * 0.11).to(torch.bfloat16), (b * 0.07).to(torch.bfloat16)
+    assert torch.equal(ctx.gemm(a, b, epilogue=epi), ctx.gemm(a, b, epilogue=epi, block_n=256))
+
+
 def test_gemm_strided_views(ctx):
     """A and C may be column slices of wider buffers (leading dimension > width)."""
     M, N, K = 256, 384, 320
