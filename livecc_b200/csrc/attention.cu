@@ -260,32 +260,31 @@ __global__ void __launch_bounds__(128) flash_fwd_kernel(const FlashParams p) {
     }
 }
 
-// Merge of the split-KV partials of the prefill attention: one CTA per packed row, one thread per dim.
+// Merge of the split-KV partials of the prefill attention (up to 32 of them): one CTA per packed row, one thread per dim. A lane weighs one
+// split; the partials are then read eight at a time.
 __global__ void __launch_bounds__(128) flash_merge_kernel(const float* __restrict__ part_o,
                                                           const float* __restrict__ part_ml, int nsplit, int Hkv,
                                                           int rows_total, int G, float scale_log2,
                                                           bf16* __restrict__ out, int o_ld) {
-    const int rr = blockIdx.x, g = blockIdx.y, d = threadIdx.x;
-    float ms[8], ls[8];
-    float M = -INFINITY;
-#pragma unroll
-    for (int sp = 0; sp < 8; ++sp) {
-        if (sp < nsplit) {
-            const size_t prow = ((size_t)sp * Hkv + g) * rows_total + rr;
-            ms[sp] = part_ml[prow * 2];
-            ls[sp] = part_ml[prow * 2 + 1];
-            M = fmaxf(M, ms[sp]);
-        }
+    const int rr = blockIdx.x, g = blockIdx.y, d = threadIdx.x, lane = threadIdx.x & 31;
+    const size_t row = (size_t)g * rows_total + rr, step = (size_t)Hkv * rows_total;
+    float m = -INFINITY, l = 0.f;
+    if (lane < nsplit) {
+        const float2 ml = *reinterpret_cast<const float2*>(part_ml + (lane * step + row) * 2);
+        m = ml.x;
+        l = ml.y;
     }
-    float acc = 0.f, L = 0.f;
+    const float M = warp_max(m);
+    const float f = m == -INFINITY ? 0.f : exp2f((m - M) * scale_log2);
+    const float L = warp_sum(f * l);
+    const unsigned has = __ballot_sync(0xffffffffu, m != -INFINITY);   // a split without keys wrote no partial
+    float acc = 0.f;
+    for (int s0 = 0; s0 < nsplit; s0 += 8) {
+        float v[8];
 #pragma unroll
-    for (int sp = 0; sp < 8; ++sp) {
-        if (sp < nsplit && ms[sp] != -INFINITY) {
-            const size_t prow = ((size_t)sp * Hkv + g) * rows_total + rr;
-            const float f = exp2f((ms[sp] - M) * scale_log2);
-            acc += f * part_o[prow * 128 + d];
-            L += f * ls[sp];
-        }
+        for (int i = 0; i < 8; ++i) v[i] = has >> (s0 + i) & 1 ? part_o[((s0 + i) * step + row) * 128 + d] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc = fmaf(__shfl_sync(0xffffffffu, f, s0 + i), v[i], acc);
     }
     const int pos = rr / G, hq = g * G + rr % G;
     out[(size_t)pos * o_ld + (size_t)hq * 128 + d] = f2bf(L > 0.f ? acc / L : 0.f);

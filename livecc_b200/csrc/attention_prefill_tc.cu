@@ -12,8 +12,13 @@
 //   * causal mask per row (key index <= past + position), applied only on tiles that reach the diagonal.
 //   * split-KV (blockIdx.z): partial (unnormalised O, m, l) in the format of flash_merge_kernel (attention.cu).
 // The tail of the last page beyond past+S is never unmasked; V there must be finite (mrope_kv_write zeroes it).
-// TMEM (256 columns): S0 @0, S1 @64, O @128 (128 columns).
-#include <stdlib.h>
+// TMEM (256 columns): S0 @0, S1 @64, O @128 (128 columns); a tile's P overwrites the first half of its S and is the A operand of P.V.
+//
+// A thread owns a row, so one CTA has four softmax warps, one per scheduler, and a tile is a serial chain (TMEM load, maximum, 64
+// exponentials, TMEM store, MMA): 1.8 us per 64 keys with one CTA per SM. Two CTAs fill each other's gaps: 98 KB of shared memory (two
+// slots each for K and V, released apart) and half of the TMEM each: 281 rows over 8 k keys 119 -> 48 us (20 us at
+// the tensor rate), 24 rows over 32 k 115 us with one CTA per SM and 8 splits at most.
+#include <algorithm>
 
 #include "common.cuh"
 #include "gemm.h"
@@ -22,21 +27,18 @@
 
 namespace lcc {
 namespace ptc {
-constexpr int D = 128, BM = 128, BN = 64, STAGES = 4;
-// P operand through TMEM instead of shared memory (see attention_tc.cu). LIVECC_B200_ATTN_PTMEM=0/1 overrides.
-constexpr int kPtmemDefault = 1;
+constexpr int D = 128, BM = 128, BN = 64, STAGES = 2;
 constexpr int Q_ATOM_BYTES = BM * 128;       // [128 rows][64 bf16]
 constexpr int Q_BYTES = 2 * Q_ATOM_BYTES;
 constexpr int KV_ATOM_BYTES = BN * 128;      // [64 tokens][64 bf16]
 constexpr int KV_BYTES = 2 * KV_ATOM_BYTES;  // one K or V tile
-constexpr int P_BYTES = BM * 128;            // [128 rows][64 keys]
 constexpr int OFF_Q = 0;
 constexpr int OFF_K = OFF_Q + Q_BYTES;
 constexpr int OFF_V = OFF_K + STAGES * KV_BYTES;
-constexpr int OFF_P = OFF_V + STAGES * KV_BYTES;
-constexpr int OFF_BAR = OFF_P + P_BYTES;
+constexpr int OFF_BAR = OFF_V + STAGES * KV_BYTES;
 constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
-constexpr int COL_S = 0, COL_O = 2 * BN, COL_P = 256;  // P (32 columns of packed bf16x2) only in the PTMEM variant
+constexpr int COL_S = 0, COL_O = 2 * BN, TMEM_COLS = 256;
+constexpr int MAX_SPLIT = 32;
 constexpr float RESCALE_THRESHOLD = 8.f;
 }  // namespace ptc
 
@@ -57,14 +59,10 @@ __device__ __forceinline__ float ex2_ftz_p(float x) {
     return y;
 }
 
-// PTMEM: P goes to TMEM (tcgen05.st) and P.V reads its A operand from TMEM instead of staging P in shared memory
-// (experimental, LIVECC_B200_ATTN_PTMEM=1: written without GPU time at the end of round 1, not validated yet).
-template <bool PTMEM>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(192, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                        const __grid_constant__ CUtensorMap tmap_v, PrefillTcParams p) {
     using namespace ptc;
-    constexpr int TMEM_COLS = PTMEM ? 512 : 256;
     const int kvh = blockIdx.y, split = blockIdx.z;
     const int pos0 = blockIdx.x * p.PT;
     if (pos0 >= p.S) return;
@@ -95,11 +93,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
     uint64_t* q_full = bars;
-    uint64_t* kv_full = bars + 1;
-    uint64_t* kv_empty = kv_full + STAGES;
-    uint64_t* s_full = kv_empty + STAGES;
-    uint64_t* s_empty = s_full + 2;
-    uint64_t* p_full = s_empty + 2;
+    uint64_t* k_full = bars + 1;
+    uint64_t* k_empty = k_full + STAGES;
+    uint64_t* v_full = k_empty + STAGES;
+    uint64_t* v_empty = v_full + STAGES;
+    uint64_t* s_full = v_empty + STAGES;
+    uint64_t* p_full = s_full + 2;
     uint64_t* pv_done = p_full + 1;
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(pv_done + 1);
 
@@ -111,13 +110,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         prefetch_tensormap(&tmap_v);
         mbar_init(q_full, 1);
         for (int i = 0; i < STAGES; ++i) {
-            mbar_init(&kv_full[i], 1);
-            mbar_init(&kv_empty[i], 1);
+            mbar_init(&k_full[i], 1);
+            mbar_init(&k_empty[i], 1);
+            mbar_init(&v_full[i], 1);
+            mbar_init(&v_empty[i], 1);
         }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&s_full[i], 1);
-            mbar_init(&s_empty[i], 4);
-        }
+        for (int i = 0; i < 2; ++i) mbar_init(&s_full[i], 1);
         mbar_init(p_full, 4);
         mbar_init(pv_done, 1);
         fence_barrier_init();
@@ -140,16 +138,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             tma_load_3d(smem + OFF_Q + Q_ATOM_BYTES, &tmap_q, q_full, 64, kvh * p.G, pos0);
             for (int i = 0; i < T; ++i) {
                 const int st = i % STAGES;
-                mbar_wait(&kv_empty[st], (((i / STAGES) & 1) ^ 1));
-                mbar_arrive_expect_tx(&kv_full[st], 2 * KV_BYTES);
+                const uint32_t free = ((i / STAGES) & 1) ^ 1;
                 const int page = p.page_table[tile_lo + i];
                 const int row = (page * p.Hkv + kvh) * BN;
                 uint8_t* sk = smem + OFF_K + st * KV_BYTES;
                 uint8_t* sv = smem + OFF_V + st * KV_BYTES;
-                tma_load_2d(sk, &tmap_k, &kv_full[st], 0, row);
-                tma_load_2d(sk + KV_ATOM_BYTES, &tmap_k, &kv_full[st], 64, row);
-                tma_load_2d(sv, &tmap_v, &kv_full[st], 0, row);
-                tma_load_2d(sv + KV_ATOM_BYTES, &tmap_v, &kv_full[st], 64, row);
+                mbar_wait(&k_empty[st], free);
+                mbar_arrive_expect_tx(&k_full[st], KV_BYTES);
+                tma_load_2d(sk, &tmap_k, &k_full[st], 0, row);
+                tma_load_2d(sk + KV_ATOM_BYTES, &tmap_k, &k_full[st], 64, row);
+                mbar_wait(&v_empty[st], free);
+                mbar_arrive_expect_tx(&v_full[st], KV_BYTES);
+                tma_load_2d(sv, &tmap_v, &v_full[st], 0, row);
+                tma_load_2d(sv + KV_ATOM_BYTES, &tmap_v, &v_full[st], 64, row);
             }
         }
     } else if (warp == 1) {
@@ -157,11 +158,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         constexpr uint32_t idesc_qk = make_idesc_bf16(BM, BN);
         constexpr uint32_t idesc_pv = make_idesc_bf16(BM, D) | (1u << 16);  // B (= V) is MN-major
         const uint32_t q_addr = smem_u32(smem + OFF_Q);
-        const uint32_t p_addr = smem_u32(smem + OFF_P);
         auto issue_qk = [&](int i) {
             const int st = i % STAGES, b = i & 1;
-            mbar_wait(&kv_full[st], (i / STAGES) & 1);
-            mbar_wait(&s_empty[b], (((i >> 1) & 1) ^ 1));
+            mbar_wait(&k_full[st], (i / STAGES) & 1);
+            if (i >= 2) mbar_wait(pv_done, i & 1);   // P of tile i - 2 lies where S of tile i goes (the MMA of tile i - 1 is yet to be issued)
             tc_fence_after();
             if (lane == 0) {
                 const uint32_t k_addr = smem_u32(smem + OFF_K + st * KV_BYTES);
@@ -174,6 +174,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                         umma_bf16_ss(tmem_base + COL_S + b * BN, dq + (uint64_t)(2 * k), dk + (uint64_t)(2 * k), idesc_qk,
                                      (a | k) ? 1u : 0u);
                 }
+                umma_commit(&k_empty[st]);
                 umma_commit(&s_full[b]);
             }
             __syncwarp();
@@ -182,21 +183,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         issue_qk(0);
         for (int i = 0; i < T; ++i) {
             if (i + 1 < T) issue_qk(i + 1);
+            mbar_wait(&v_full[i % STAGES], (i / STAGES) & 1);
             mbar_wait(p_full, i & 1);
             tc_fence_after();
             if (lane == 0) {
                 const int st = i % STAGES;
                 const uint32_t v_addr = smem_u32(smem + OFF_V + st * KV_BYTES);
-                const uint64_t dp = make_sw128_kmajor_desc(p_addr);
 #pragma unroll
                 for (int ks = 0; ks < BN / 16; ++ks) {  // 16 tokens per MMA: +32 B in P rows, +16 token rows in V
                     const uint64_t dv = make_sw128_mnmajor_desc(v_addr + ks * (16 * 128), KV_ATOM_BYTES);
-                    if constexpr (PTMEM)
-                        umma_bf16_ts(tmem_base + COL_O, tmem_base + COL_P + ks * 8, dv, idesc_pv, (i | ks) ? 1u : 0u);
-                    else
-                        umma_bf16_ss(tmem_base + COL_O, dp + (uint64_t)(2 * ks), dv, idesc_pv, (i | ks) ? 1u : 0u);
+                    umma_bf16_ts(tmem_base + COL_O, tmem_base + COL_S + (i & 1) * BN + ks * 8, dv, idesc_pv, (i | ks) ? 1u : 0u);
                 }
-                umma_commit(&kv_empty[st]);
+                umma_commit(&v_empty[st]);
                 umma_commit(pv_done);
             }
             __syncwarp();
@@ -209,8 +207,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         const bool row_ok = row < rows_used;
         const int rpos = row / p.G, rg = row - rpos * p.G;
         const int lim = row_ok ? p.past + pos0 + rpos : -1;  // last visible key index; invalid rows see nothing
-        uint8_t* p_row = smem + OFF_P + row * 128;
-        const int sw = row & 7;
         float m_used = -INFINITY, l = 0.f;
         for (int i = 0; i < T; ++i) {
             const int b = i & 1;
@@ -220,9 +216,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             tmem_ld_32x32b_x32(tmem_base + COL_S + b * BN + lane_off, v[0]);
             tmem_ld_32x32b_x32(tmem_base + COL_S + b * BN + 32 + lane_off, v[1]);
             tmem_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&s_empty[b]);
 
             const int kbase = (tile_lo + i) * BN;
             if (__any_sync(0xffffffffu, kbase + BN - 1 > lim)) {  // tile reaches the diagonal for some row of this warp
@@ -265,7 +258,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
 
             if (i > 0) {
-                mbar_wait(pv_done, (i - 1) & 1);  // P_{i-1} V_{i-1} retired: P buffer free, O up to date
+                mbar_wait(pv_done, (i - 1) & 1);  // P_{i-1} V_{i-1} retired: O up to date
                 tc_fence_after();
                 if (any_need) {
 #pragma unroll
@@ -280,18 +273,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                     tmem_st_wait();
                 }
             }
-            if constexpr (PTMEM) {
-                // P row -> TMEM: word j = keys (2j, 2j+1), lane = row (the A-operand layout of kind::f16)
-                tmem_st_32x32b_x32(tmem_base + COL_P + lane_off, pk);
-                tmem_st_wait();
-            } else {
-                // P row (64 keys = one 128-byte swizzled row: 16-byte chunk index XOR (row & 7))
-#pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    *reinterpret_cast<uint4*>(p_row + ((c ^ sw) << 4)) =
-                        make_uint4(pk[c * 4], pk[c * 4 + 1], pk[c * 4 + 2], pk[c * 4 + 3]);
-                fence_proxy_async_smem();
-            }
+            // P row -> TMEM, over the S it came from: word j = keys (2j, 2j+1), lane = row (the A-operand layout of kind::f16)
+            tmem_st_32x32b_x32(tmem_base + COL_S + b * BN + lane_off, pk);
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full);
@@ -361,31 +345,22 @@ int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, con
     const int ctas = q_tiles * Hkv;
     const int kv_tiles = (past + S + BN - 1) / BN;
     int nsplit = 1;
-    if (part_o && part_ml && ctas < num_sms) {  // one CTA per SM: split the KV range until the SMs are covered
-        nsplit = num_sms / ctas;
-        if (nsplit > 8) nsplit = 8;
-        while (nsplit > 1 && kv_tiles < 8 * nsplit) --nsplit;  // keep >= 8 tiles of work per split
-        if ((size_t)nsplit * Hkv * S * G > part_capacity_rows) nsplit = 1;
+    // two CTAs per SM: split the KV range until those places are taken, with at least 8 tiles of work per split (281 rows x 8 k keys: 4
+    // splits; 24 rows x 32 k keys: 32). Partials that don't fit into the caller's scratch mean fewer splits.
+    if (part_o && part_ml) {
+        nsplit = std::max(1, std::min({2 * num_sms / ctas, MAX_SPLIT, kv_tiles / 8}));
+        nsplit = std::max(1, (int)std::min((size_t)nsplit, part_capacity_rows / ((size_t)Hkv * S * G)));
     }
     CUtensorMap tq, tk, tv;
     if (make_tmap_bf16_3d_sw128(&tq, q, D, Hq, S, D, q_ld, G, PT)) return -10;
     const int64_t pool_rows = (int64_t)1 << 31;  // page ids come from the page table; no meaningful row bound here
     if (make_tmap_bf16_2d_box(&tk, kc, pool_rows, D, D, 64, BN, false)) return -11;
     if (make_tmap_bf16_2d_box(&tv, vc, pool_rows, D, D, 64, BN, false)) return -11;
-    static int ptmem = -1;
-    if (ptmem < 0) {
-        const char* pe = getenv("LIVECC_B200_ATTN_PTMEM");  // "1" / "0" force the variant; unset = kPtmemDefault
-        ptmem = pe ? (pe[0] == '1' ? 1 : 0) : kPtmemDefault;
-    }
-    static SmemAttrOnce once_a, once_b;
-    if (ensure_dyn_smem(once_a, attn_prefill_tc_kernel<false>, SMEM_BYTES) ||
-        ensure_dyn_smem(once_b, attn_prefill_tc_kernel<true>, SMEM_BYTES))
-        return -12;
+    static SmemAttrOnce once;
+    if (ensure_dyn_smem(once, attn_prefill_tc_kernel, SMEM_BYTES)) return -12;
     PrefillTcParams p{out, o_ld, page_table, Hkv, G, PT, S, past, 1.4426950408889634f / sqrtf((float)D), nsplit, part_o, part_ml};
-    if (ptmem)
-        { lcc::count_launch(); attn_prefill_tc_kernel<true><<<dim3(q_tiles, Hkv, nsplit), 192, SMEM_BYTES, s>>>(tq, tk, tv, p); }
-    else
-        { lcc::count_launch(); attn_prefill_tc_kernel<false><<<dim3(q_tiles, Hkv, nsplit), 192, SMEM_BYTES, s>>>(tq, tk, tv, p); }
+    lcc::count_launch();
+    attn_prefill_tc_kernel<<<dim3(q_tiles, Hkv, nsplit), 192, SMEM_BYTES, s>>>(tq, tk, tv, p);
     *nsplit_out = nsplit;
     return 0;
 }

@@ -224,6 +224,31 @@ def test_mrope_kv_write_and_prefill_attention(ctx, S, past, impl, split):
     assert (out.float() - eager.float()).abs().max().item() < 5e-2
 
 
+@pytest.mark.parametrize("S,past,rows", [(1, 16384, 32), (24, 17000, 32), (24, 17000, 5), (19, 1100, 32), (300, 9000, 3), (40, 511, 32), (2, 126, 32)])
+def test_prefill_attention_split_counts(ctx, S, past, rows):
+    """few new rows over a long past: as many splits as there are places for, at least 8 tiles each, and as fit into the scratch (`rows`
+    splits' worth); splits of 1, 2 and more tiles, a last one cut short"""
+    Hq, Hkv = 14, 2
+    T = past + S
+    cache = PagedCache(1, Hkv, T)
+    k, v = _rand((Hkv, T, 128), 31), _rand((Hkv, T, 128), 32)
+    cache.k.zero_(), cache.v.zero_()
+    for t0 in range(0, T, 64):
+        n, pg = min(64, T - t0), int(cache.page_table[t0 // 64])
+        cache.k[0, pg, :, :n], cache.v[0, pg, :, :n] = k[:, t0:t0 + n], v[:, t0:t0 + n]
+    q = _rand((S, Hq * 128), 33)
+    out = torch.empty_like(q)
+    part_o = torch.empty((rows * S * Hq, 128), device=DEV)
+    part_ml = torch.empty((rows * S * Hq, 2), device=DEV)
+    ctx.call("lcc_attn_prefill", A._ptr(q), A._i(q.stride(0)), A._ptr(cache.k[0]), A._ptr(cache.v[0]), A._ptr(cache.page_table), A._i(Hq), A._i(Hkv),
+             A._i(S), A._i(past), A._ptr(out), A._i(out.stride(0)), A._ptr(part_o), A._ptr(part_ml), A.C.c_int64(part_o.shape[0]), A._i(2),
+             ctx.stream_ptr())
+    rep = Hq // Hkv
+    mask = torch.zeros((S, T), device=DEV).masked_fill_(torch.arange(T, device=DEV)[None, :] > torch.arange(past, T, device=DEV)[:, None], float("-inf"))
+    ref = _attn_ref_fp32(q.view(S, Hq, 128).transpose(0, 1), k.repeat_interleave(rep, 0), v.repeat_interleave(rep, 0), mask, 128 ** -0.5)
+    _attn_close(out, ref.transpose(0, 1).reshape(S, Hq * 128), "attn_prefill")
+
+
 @pytest.mark.parametrize("kv_len", [0, 1, 63, 64, 65, 1000, 5000])
 @pytest.mark.parametrize("nsplit", [1, 8, 37])
 def test_attn_decode(ctx, kv_len, nsplit):
