@@ -16,8 +16,11 @@
 // overlaps the main loop of tile i+1.
 //
 // The fused epilogues reproduce the reference's bf16 rounding points (one torch op = one rounding).
-#include <string.h>
 #include <stdlib.h>
+#include <string.h>
+
+#include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "gemm.h"
@@ -526,6 +529,365 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 }
 
 // ----------------------------------------------------------------------------
+// CTA pair with the operands swapped, for few rows: the WEIGHTS are the 256-row operand, the activations the columns.
+//
+// Products of a few hundred rows have too few tiles for the SMs and take every weight tile in once per 128 rows. Here a pair multiplies 256
+// weight rows by up to 512 activation rows (two MMAs of up to 256 columns per k-step, each CTA staging its 128 weight rows and half of the
+// activation rows): M = 281 is ONE tile of 288 columns, and a weight element reaches exactly one SM. The width is a run-time value, a
+// multiple of 32; where the tiles are too few, the pairs of a cluster split K and add their accumulators through distributed shared memory
+// (no partials in global memory, no second launch, fixed order). Which products gain: see choose_swap.
+//
+// Structure (per CTA 384 threads): as the pair kernel above. TMEM lane = weight row = output column, TMEM column = activation row = output
+// row: a thread owns one output column, so its bias is one register; two shuffle rounds turn four threads' columns into 8-byte pieces of
+// an output row, stored (and the residual read) as 64-byte runs. That is dearer than the row-wise store of the other kernels, so many
+// rows stay with those.
+// ----------------------------------------------------------------------------
+struct SwapTile {
+    int bm, n1, n2;      // activation rows per tile = columns of the first and (0: none) second MMA, multiples of 32
+    int stages, bufs;    // ring depth; accumulator buffers in TMEM
+    int tmem_cols;
+    int splits;          // pairs of a cluster that share a tile's K range
+    uint32_t idesc1, idesc2;
+    int stage_bytes, smem_bytes;
+};
+static constexpr int kSwapMax = 512, kSwapSplits = 4;
+static SwapTile make_swap(int bm, int splits, bool many) {
+    SwapTile t;
+    t.bm = bm;
+    t.n1 = bm <= 256 ? bm : (bm / 2 + 31) / 32 * 32;
+    t.n2 = bm - t.n1;
+    t.stage_bytes = A_BYTES + bm / 2 * BLOCK_K * 2;
+    t.stages = (227 * 1024 - 1024 - 256) / t.stage_bytes;
+    if (t.stages > MAX_STAGES) t.stages = MAX_STAGES;
+    t.bufs = many && 2 * bm <= 512 ? 2 : 1;
+    t.tmem_cols = 32;
+    while (t.tmem_cols < t.bufs * bm) t.tmem_cols <<= 1;
+    t.splits = splits;
+    t.idesc1 = make_idesc_bf16(2 * BLOCK_M, t.n1);
+    t.idesc2 = t.n2 ? make_idesc_bf16(2 * BLOCK_M, t.n2) : 0u;
+    t.smem_bytes = t.stages * t.stage_bytes + 1024 /*align slack*/ + 256 /*barriers*/;
+    return t;
+}
+
+// Bounded mbarrier wait (2 s): a signal that never comes raises the CTA's flag, every later wait gives up at its first look at it, and the
+// epilogue stores NaN, so that the kernel ends and the result shows it.
+__device__ __forceinline__ void mbar_wait_or(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
+    unsigned long long t0 = 0, now;
+    for (int it = 0;; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred P1;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, P1;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return;
+        if ((it & 0x3ff) != 0x3ff) continue;
+        if (*gave_up) return;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (t0 == 0) t0 = now;
+        else if (now - t0 > 2000000000ull) { *gave_up = 1; return; }
+    }
+}
+
+__device__ __forceinline__ float ld_cluster_addr_f32(uint32_t cluster_addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
+    return v;
+}
+
+// what an accumulator becomes before it is rounded to bf16 (the activations of EPI_BIAS_QUICKGELU / EPI_BIAS_GELU follow the rounding)
+template <int EPI>
+__device__ __forceinline__ float swap_unary(float x, float bias) {
+    if (EPI == EPI_BIAS || EPI == EPI_BIAS_QUICKGELU || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESIDUAL) x += bias;
+    if (EPI == EPI_RELU2) { x = fmaxf(x, 0.f); x *= x; }
+    if (EPI == EPI_GELU_ERF) x = 0.5f * x * (1.f + erff(x * 0.7071067811865476f));
+    if (EPI == EPI_GELU_TANH) x = 0.5f * x * (1.f + tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x)));
+    if (EPI == EPI_BIAS_QUICKGELU) x = quick_gelu_bf16(rbf(x));
+    if (EPI == EPI_BIAS_GELU) x = gelu_erf_bf16(rbf(x));
+    return x;
+}
+template <int EPI> struct SwapEpi {
+    static constexpr bool kGlu = EPI == EPI_SWIGLU || EPI == EPI_CLAMP_GLU;
+    static constexpr bool kResidual = EPI == EPI_RESIDUAL || EPI == EPI_BIAS_RESIDUAL;
+};
+
+// A warp's chunk: v[j] = accumulator of output row m0 + j, output column n (one per lane). res: the residual's 8-byte pieces at the
+// places this lane will store (rows m0 + 4 k + (lane & 3), columns (n & ~3) ..), EPI_*RESIDUAL only.
+template <int EPI>
+__device__ __forceinline__ void swap_store(const float (&v)[32], bf16* C, int ldc, int M, int N, int m0, int n, int lane, float bias,
+                                           const uint2 (&res)[8], float limit, float alpha, float up_bias) {
+    if (EPI == EPI_PARTIAL_F32) {   // fp32 output: 32 consecutive columns per store
+        float* out = reinterpret_cast<float*>(C);
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if (m0 + j < M && n < N) out[(size_t)(m0 + j) * ldc + n] = v[j];
+        return;
+    }
+    if (SwapEpi<EPI>::kGlu) {
+        // lanes 0..15 hold gate rows, 16..31 the matching up rows: of rows j, j + 1 the lower half makes row j, the upper half row j + 1
+        const bool hi = lane & 16;
+        uint32_t o[8];   // rows j + hi (low half) and j + 2 + hi (high half), j = 0, 4, ...
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            float y[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int j = 4 * k + 2 * e;
+                const float r = __shfl_xor_sync(0xffffffffu, hi ? v[j] : v[j + 1], 16);
+                const float g = hi ? r : v[j], u = hi ? v[j + 1] : r;
+                if (EPI == EPI_SWIGLU) y[e] = silu_bf16(rbf(g)) * rbf(u);
+                else {
+                    const float gc = fminf(g, limit), uc = fminf(fmaxf(u, -limit), limit);
+                    y[e] = gc / (1.f + __expf(-alpha * gc)) * (uc + up_bias);
+                }
+            }
+            o[k] = pack_bf16x2(y[0], y[1]);
+        }
+        const int col = ((n >> 5) << 4) + (lane & 12);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            uint32_t w[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {   // even lane: row 4 k' + hi of two columns, odd lane: row 4 k' + 2 + hi
+                const uint32_t own = o[2 * k + e], other = __shfl_xor_sync(0xffffffffu, own, 1);
+                w[e] = (lane & 1) ? __byte_perm(other, own, 0x7632) : __byte_perm(own, other, 0x5410);
+            }
+            const uint32_t recv = __shfl_xor_sync(0xffffffffu, (lane & 2) ? w[0] : w[1], 2);
+            const uint2 q = (lane & 2) ? make_uint2(recv, w[1]) : make_uint2(w[0], recv);
+            const int row = m0 + 4 * (2 * k + ((lane >> 1) & 1)) + 2 * (lane & 1) + (hi ? 1 : 0);
+            if (row < M && n < N) *reinterpret_cast<uint2*>(C + (size_t)row * ldc + col) = q;
+        }
+        return;
+    }
+    const int col = n & ~3;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        uint32_t w[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {   // rows j, j + 1: the even lane keeps row j of two columns, the odd lane row j + 1
+            const int j = 4 * k + 2 * e;
+            const uint32_t own = pack_bf16x2(swap_unary<EPI>(v[j], bias), swap_unary<EPI>(v[j + 1], bias));
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
+            w[e] = (lane & 1) ? __byte_perm(other, own, 0x7632) : __byte_perm(own, other, 0x5410);
+        }
+        const uint32_t recv = __shfl_xor_sync(0xffffffffu, (lane & 2) ? w[0] : w[1], 2);
+        uint2 q = (lane & 2) ? make_uint2(recv, w[1]) : make_uint2(w[0], recv);
+        const int row = m0 + 4 * k + (lane & 3);
+        if (SwapEpi<EPI>::kResidual) {
+            const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), ra = unpack_bf16x2(res[k].x), rb = unpack_bf16x2(res[k].y);
+            q = make_uint2(pack_bf16x2(a.x + ra.x, a.y + ra.y), pack_bf16x2(b.x + rb.x, b.y + rb.y));
+        }
+        if (row < M && n < N) *reinterpret_cast<uint2*>(C + (size_t)row * ldc + col) = q;
+    }
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(384, 1)
+gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x1,
+                 const __grid_constant__ CUtensorMap tmap_x2, bf16* C, int M, int N, int K, int ldc, const bf16* __restrict__ bias,
+                 const bf16* residual /* may alias C */, int ldr, const SwapTile cfg, float limit, float alpha, float up_bias) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const int STAGES = cfg.stages, STAGE_BYTES = cfg.stage_bytes, S = cfg.splits;
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+    uint64_t* empty_bar = full_bar + MAX_STAGES;
+    uint64_t* tmem_full = empty_bar + MAX_STAGES;
+    uint64_t* tmem_empty = tmem_full + 2;
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+    volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_holder + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t crank = cluster_ctarank();
+    const int rank = crank & 1, split = crank >> 1;        // CTA of the pair; pair of the cluster
+    const uint32_t lead = crank & ~1u;
+    const bool leader = rank == 0;
+    const int cluster = blockIdx.x / (2 * S), num_clusters = gridDim.x / (2 * S);
+
+    const int m_tiles = (M + cfg.bm - 1) / cfg.bm, n_tiles = (N + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
+    const int nkb = (K + BLOCK_K - 1) / BLOCK_K;
+    const int kb0 = (int)((long long)nkb * split / S), kb1 = (int)((long long)nkb * (split + 1) / S);
+    const int units = m_tiles * n_tiles;   // m fastest: the tiles that share weight rows run together. S > 1: one unit per cluster
+
+    if (warp == 0 && lane == 0) {
+        prefetch_tensormap(&tmap_w);
+        prefetch_tensormap(&tmap_x1);
+        if (cfg.n2) prefetch_tensormap(&tmap_x2);
+    }
+    if (warp == 1 && lane == 0) {
+        for (int i = 0; i < STAGES; ++i) {
+            mbar_init(&full_bar[i], 1);   // used in the leader: its producer's arrive.expect_tx (bytes of both CTAs)
+            mbar_init(&empty_bar[i], 1);  // one multicast commit of the leader's MMA warp
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&tmem_full[i], 1);    // one multicast commit
+            mbar_init(&tmem_empty[i], 16);  // used in the leader: 8 epilogue warps of each CTA
+        }
+        *gave_up = 0;
+        fence_barrier_init();
+    }
+    if (warp == 2) {
+        tmem_alloc_cg2(tmem_holder, cfg.tmem_cols);
+        tmem_relinquish_cg2();
+    }
+    tc_fence_before();
+    __syncwarp();        // barrier.cluster is .aligned: the warp must be converged
+    cluster_sync_all();  // barriers of all CTAs are initialised before any remote arrive / TMA credit
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_holder;
+
+    if (warp == 0) {
+        // ===================== TMA producer (both CTAs) =====================
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0;
+            for (int unit = cluster; unit < units; unit += num_clusters) {
+                const int m0 = (unit % m_tiles) * cfg.bm, n0 = (unit / m_tiles) * 2 * BLOCK_M;
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    mbar_wait_or(&empty_bar[stage], phase ^ 1, gave_up);
+                    uint8_t* sw = smem + stage * STAGE_BYTES;
+                    uint8_t* sx = sw + A_BYTES;
+                    if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
+                    const uint32_t bar = mapa_shared(smem_u32(&full_bar[stage]), lead);
+                    tma_load_2d_cg2(sw, &tmap_w, bar, kb * BLOCK_K, n0 + rank * BLOCK_M);
+                    tma_load_2d_cg2(sx, &tmap_x1, bar, kb * BLOCK_K, m0 + rank * (cfg.n1 / 2));
+                    if (cfg.n2)
+                        tma_load_2d_cg2(sx + cfg.n1 / 2 * BLOCK_K * 2, &tmap_x2, bar, kb * BLOCK_K, m0 + cfg.n1 + rank * (cfg.n2 / 2));
+                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ===================== MMA issuer (leader CTA only) =====================
+        if (leader) {
+            int stage = 0, acc = 0;
+            uint32_t phase = 0, acc_phase = 0;
+            const uint16_t both = (uint16_t)(3u << lead);
+            for (int unit = cluster; unit < units; unit += num_clusters) {
+                mbar_wait_or(&tmem_empty[acc], acc_phase ^ 1, gave_up);
+                tc_fence_after();
+                const uint32_t tmem_d = tmem_base + acc * cfg.bm;
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    mbar_wait_or(&full_bar[stage], phase, gave_up);
+                    tc_fence_after();
+                    if (lane == 0) {
+                        const uint32_t sw = smem_u32(smem + stage * STAGE_BYTES);
+                        const uint64_t dw = make_sw128_kmajor_desc(sw);
+                        const uint64_t dx = make_sw128_kmajor_desc(sw + A_BYTES);
+                        const uint64_t dx2 = make_sw128_kmajor_desc(sw + A_BYTES + cfg.n1 / 2 * BLOCK_K * 2);
+#pragma unroll
+                        for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                            const uint32_t add = ((kb - kb0) | k) != 0 ? 1u : 0u;
+                            umma_bf16_ss_cg2(tmem_d, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), cfg.idesc1, add);
+                            if (cfg.n2) umma_bf16_ss_cg2(tmem_d + cfg.n1, dw + (uint64_t)(k * 2), dx2 + (uint64_t)(k * 2), cfg.idesc2, add);
+                        }
+                        umma_commit_cg2(&empty_bar[stage], both);  // frees the slot in both CTAs when the MMAs retire
+                        if (kb == kb1 - 1) umma_commit_cg2(&tmem_full[acc], both);
+                    }
+                    __syncwarp();
+                    if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                }
+                if (++acc == cfg.bufs) { acc = 0; acc_phase ^= 1; }
+            }
+        }
+    } else if (warp >= 4) {
+        // ===================== Epilogue (both CTAs, own 128 weight rows) =====================
+        const int q = warp & 3, half = (warp - 4) >> 2;   // TMEM lane quarter; every other chunk of 32 activation rows
+        const int chunks = cfg.bm >> 5;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        for (int unit = cluster; unit < units; unit += num_clusters) {
+            const int m0 = (unit % m_tiles) * cfg.bm;
+            const int n = (unit / m_tiles) * 2 * BLOCK_M + rank * BLOCK_M + q * 32 + lane;
+            float b = 0.f;
+            if (EPI == EPI_BIAS || EPI == EPI_BIAS_QUICKGELU || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESIDUAL) b = n < N ? bf2f(bias[n]) : 0.f;
+            // the chunks this warp finishes: all of its half, or with a split K range those this pair owns
+            auto owner = [&](int c) { return S == 1 ? 0 : c * S / chunks; };
+            auto mine = [&](int c) { return S == 1 ? (c & 1) == half : owner(c) == split && ((c - (split * chunks + S - 1) / S) & 1) == half; };
+            uint2 res[8];
+            auto fetch = [&](int c) {   // the residual of chunk c, in flight while the accumulators are awaited
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int row = m0 + c * 32 + 4 * k + (lane & 3);
+                    res[k] = row < M && n < N ? *reinterpret_cast<const uint2*>(residual + (size_t)row * ldr + (n & ~3)) : make_uint2(0u, 0u);
+                }
+            };
+            int c = 0;
+            while (c < chunks && !mine(c)) ++c;
+            if (SwapEpi<EPI>::kResidual && c < chunks) fetch(c);
+            mbar_wait_or(&tmem_full[acc], acc_phase, gave_up);
+            tc_fence_after();
+            const uint32_t taddr = tmem_base + (uint32_t)(acc * cfg.bm) + ((uint32_t)(q * 32) << 16);
+            float* red = reinterpret_cast<float*>(smem) + q * 32 + lane;   // [chunk][32 columns][128 weight rows]: over the drained ring
+            if (S > 1) {
+                for (int d = half; d < chunks; d += 2) {
+                    if (owner(d) == split) continue;
+                    uint32_t v[32];
+                    tmem_ld_32x32b_x32(taddr + d * 32, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) red[(size_t)(d * 32 + j) * BLOCK_M] = __uint_as_float(v[j]);
+                }
+                __syncwarp();
+                cluster_sync_all();
+            }
+            while (c < chunks) {
+                int next = c + 1;
+                while (next < chunks && !mine(next)) ++next;
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(taddr + c * 32, v);
+                tmem_ld_wait();
+                float x[32];
+                if (S > 1) {
+                    const uint32_t at = smem_u32(red + (size_t)c * 32 * BLOCK_M);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) x[j] = 0.f;
+                    for (int sp = 0; sp < S; ++sp) {   // in split order, whoever adds
+                        const uint32_t from = mapa_shared(at, 2 * sp + rank);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            x[j] += sp == split ? __uint_as_float(v[j]) : ld_cluster_addr_f32(from + j * BLOCK_M * 4);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(v[j]);
+                }
+                uint2 now[8];
+                if (SwapEpi<EPI>::kResidual) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) now[k] = res[k];
+                    if (next < chunks) fetch(next);
+                }
+                if (*gave_up) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) x[j] = __int_as_float(0x7fc00000);
+                }
+                swap_store<EPI>(x, C, ldc, M, N, m0 + c * 32, n, lane, b, now, limit, alpha, up_bias);
+                c = next;
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tmem_empty[acc]), lead));
+            if (++acc == cfg.bufs) { acc = 0; acc_phase ^= 1; }
+        }
+    }
+
+    if (S > 1 && warp < 4) {
+        __syncwarp();
+        cluster_sync_all();   // the epilogue warps' barrier of the split reduction counts every thread of the cluster
+    }
+    tc_fence_before();
+    __syncwarp();        // lanes that skipped a single-lane role loop wait here for their lane 0
+    cluster_sync_all();  // no CTA may exit (or free TMEM) while the pair's MMAs / remote reads and arrives can still touch it
+    if (warp == 2) {
+        tc_fence_after();
+        tmem_dealloc_cg2(tmem_base, cfg.tmem_cols);
+    }
+}
+
+
+// ----------------------------------------------------------------------------
 // Host side
 // ----------------------------------------------------------------------------
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
@@ -653,6 +1015,75 @@ static int launch_epi2(const GemmArgs& a, int bn, int num_sms, cudaStream_t stre
     return -14;
 }
 
+// Clusters of 2 * splits CTAs (one per SM) that the device holds at once; a hardware fact, asked once per device and size.
+static int max_clusters(int splits, int num_sms) {
+    static std::atomic<int> known[64][kSwapSplits + 1];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = known[dev][splits].load(std::memory_order_relaxed);
+    if (n) return n;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(num_sms / (2 * splits) * 2 * splits);
+    cfg.blockDim = dim3(384);
+    cfg.dynamicSmemBytes = 227 * 1024;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(gemm_swap_kernel<EPI_NONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_swap_kernel<EPI_NONE>, &cfg) != cudaSuccess || n < 1)
+        n = 1;
+    known[dev][splits].store(n, std::memory_order_relaxed);
+    return n;
+}
+
+template <int EPI>
+static int launch_swap(const GemmArgs& a, int bm, int splits, int num_sms, cudaStream_t stream) {
+    const int units = (a.M + bm - 1) / bm * ((a.N + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
+    const int clusters = std::min(units, max_clusters(splits, num_sms));
+    const SwapTile cfg = make_swap(bm, splits, units > clusters);
+    // a shared K range: every unit has its cluster, every pair a k-block, and the partial accumulators fit over the ring
+    if (splits > 1 && (clusters < units || (a.K + BLOCK_K - 1) / BLOCK_K < splits || bm * BLOCK_M * 4 > cfg.stages * cfg.stage_bytes)) return -15;
+    CUtensorMap tw, t1, t2;
+    if (make_tmap_bf16_2d(&tw, a.B, a.N, a.K, a.ldb, BLOCK_M)) return -10;
+    if (make_tmap_bf16_2d(&t1, a.A, a.M, a.K, a.lda, cfg.n1 / 2)) return -11;
+    if (make_tmap_bf16_2d(&t2, a.A, a.M, a.K, a.lda, (cfg.n2 ? cfg.n2 : cfg.n1) / 2)) return -11;
+    auto kern = gemm_swap_kernel<EPI>;
+    static SmemAttrOnce once;
+    if (ensure_dyn_smem(once, kern, 227 * 1024)) return -12;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(clusters * 2 * splits);
+    lc.blockDim = dim3(384);
+    lc.dynamicSmemBytes = cfg.smem_bytes;
+    lc.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    lcc::count_launch();
+    return cudaLaunchKernelEx(&lc, kern, tw, t1, t2, (bf16*)a.C, a.M, a.N, a.K, a.ldc, (const bf16*)a.bias, (const bf16*)a.residual, a.ldr, cfg,
+                              a.epi_param, a.epi_alpha, a.epi_up_bias) == cudaSuccess ? 0 : -13;
+}
+
+static int launch_epi_swap(const GemmArgs& a, int bm, int splits, int num_sms, cudaStream_t stream) {
+    switch (a.epi) {
+        case EPI_NONE: return launch_swap<EPI_NONE>(a, bm, splits, num_sms, stream);
+        case EPI_BIAS: return launch_swap<EPI_BIAS>(a, bm, splits, num_sms, stream);
+        case EPI_BIAS_QUICKGELU: return launch_swap<EPI_BIAS_QUICKGELU>(a, bm, splits, num_sms, stream);
+        case EPI_BIAS_GELU: return launch_swap<EPI_BIAS_GELU>(a, bm, splits, num_sms, stream);
+        case EPI_RESIDUAL: return launch_swap<EPI_RESIDUAL>(a, bm, splits, num_sms, stream);
+        case EPI_BIAS_RESIDUAL: return launch_swap<EPI_BIAS_RESIDUAL>(a, bm, splits, num_sms, stream);
+        case EPI_SWIGLU: return launch_swap<EPI_SWIGLU>(a, bm, splits, num_sms, stream);
+        case EPI_RELU2: return launch_swap<EPI_RELU2>(a, bm, splits, num_sms, stream);
+        case EPI_GELU_TANH: return launch_swap<EPI_GELU_TANH>(a, bm, splits, num_sms, stream);
+        case EPI_GELU_ERF: return launch_swap<EPI_GELU_ERF>(a, bm, splits, num_sms, stream);
+        case EPI_CLAMP_GLU: return launch_swap<EPI_CLAMP_GLU>(a, bm, splits, num_sms, stream);
+    }
+    return -14;
+}
+
 static int launch_epi(const GemmArgs& a, int bn, int num_sms, cudaStream_t stream) {
     switch (a.epi) {
         case EPI_NONE: return launch_cfg<EPI_NONE>(a, bn, num_sms, stream);
@@ -698,10 +1129,11 @@ static int choose_bn(int M, int N, int num_sms) {
 // 2048 x 10304 x 2048 75 | 65, 2048 x 5120 x 5120 107 | 92, 1200 x 4608 x 3584 55 | 44, 2090 x 4608 x 3584 66 | 61, 2090 x 3584 x 18944
 // 250 | 219, 8192 x 3840 x 1280 69 | 66, 512 x 10304 x 2048 31 | 27; alone stays for 281 x 37888 x 3584 81 | 91, 1024 x 3840 x 1280 16 | 17,
 // 256 x 5120 x 5120 31 | 33. Where the model sees less than 3 % the two measure the same. Every sum runs over k in the same order.
-static int choose_pair(int M, int N, int K, int num_sms) {
+static int choose_pair(int M, int N, int K, int num_sms, double* us) {
     const long long nkb = (K + BLOCK_K - 1) / BLOCK_K;
     auto waves = [](long long units, int at_once) { return (double)((units + at_once - 1) / at_once); };
     const int bn1 = choose_bn(M, N, num_sms);
+    *us = 0.;
     if (bn1 < 128 || num_sms < 2) return 0;
     const double alone = 8.0 + waves((long long)((M + BLOCK_M - 1) / BLOCK_M) * ((N + bn1 - 1) / bn1), num_sms) * nkb * (bn1 == 128 ? 0.28 : 0.41);
     const double per_kb[5] = {0.295, 0.30, 0.325, 0.355, 0.37};
@@ -712,7 +1144,32 @@ static int choose_pair(int M, int N, int K, int num_sms) {
         const double t = 9.5 + waves((long long)((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + bn - 1) / bn), num_sms / 2) * nkb * per_kb[i];
         if (t < best) { best = t; width = bn; }
     }
+    *us = width ? best : alone;
     return width;
+}
+
+// Few rows: is the swapped kernel the better one? `other`: the estimate of the best other form (0: none, narrow products). One wave of
+// clusters of 2 s CTAs (two waves where all rows are one tile), max(0.42, rows / 700) us per k-block of a pair's share, 10 us for the launch,
+// 3.5 for the exchange of a split, 0.5 per 64 rows for the store. Measured (us, the other forms | this): 281 rows x 3584 x 18944 58 | 52,
+// x 37888 x 3584 81 | 77, x 3584 x 3584 24 | 22; 24 x 4608 x 3584 21 | 16.5, x 3584 x 3584 20 | 15.5; 256 x 5120 x 5120 31 | 28, x 3584 x 5120
+// 28 | 23; 1024 x 1280 x 5120 31 | 27; 2090 x 3584 x 18944 219 | 196; others stay for 24 x 37888 x 3584 46 | 60, x 3584 x 18944 32 | 44.
+static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_out, int* splits_out) {
+    const int n_tiles = (N + 2 * BLOCK_M - 1) / (2 * BLOCK_M), nkb = (K + BLOCK_K - 1) / BLOCK_K;
+    const int t0 = (M + kSwapMax - 1) / kSwapMax;
+    double best = 0.95 * other;
+    bool found = false;
+    for (int tiles = t0; tiles <= 2 * t0 + 2; ++tiles) {
+        const int bm = ((M + tiles - 1) / tiles + 31) / 32 * 32, m_tiles = (M + bm - 1) / bm, units = m_tiles * n_tiles;
+        for (int sp = 1; sp <= kSwapSplits; ++sp) {
+            const int fit = max_clusters(sp, num_sms), waves = (units + fit - 1) / fit;
+            if (waves > (sp == 1 && m_tiles == 1 ? 2 : 1) || nkb < 4 * sp) continue;
+            const SwapTile t = make_swap(bm, sp, false);
+            if (sp > 1 && bm * BLOCK_M * 4 > t.stages * t.stage_bytes) continue;
+            const double us = 10.0 + waves * ((nkb + sp - 1) / sp) * std::max(0.42, bm / 700.0) + 0.5 * bm / 64 + (sp > 1 ? 3.5 : 0.0);
+            if (us < best) { best = us; *bm_out = bm; *splits_out = sp; found = true; }
+        }
+    }
+    return found;
 }
 
 // Sum of the split-K partials + the fused epilogue (same rounding points as the in-kernel epilogues):
@@ -767,12 +1224,15 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits,
 // with it forced on). Measured (profiles/r02_gemm_shapes.md): it pays only for long K — down_proj (K = 18944) 86.7 -> 60.9 us,
 // while qkv / o_proj (K = 3584) get slower (23 -> 34 us) — so the default applies it for K >= 8192 only.
 // LIVECC_B200_GEMM_SPLITK=1 forces it for every eligible shape, =0 disables it.
-static int try_splitk(const GemmArgs& a, int num_sms, cudaStream_t stream) {
-    static int mode = -1;  // 0 off, 1 forced, 2 default (long K only)
-    if (mode < 0) {
+static int splitk_mode() {
+    static const int mode = [] {   // 0 off, 1 forced, 2 default (long K only)
         const char* e = getenv("LIVECC_B200_GEMM_SPLITK");
-        mode = !e ? 2 : (e[0] == '1' ? 1 : (e[0] == '0' ? 0 : 2));
-    }
+        return !e ? 2 : (e[0] == '1' ? 1 : (e[0] == '0' ? 0 : 2));
+    }();
+    return mode;
+}
+static int try_splitk(const GemmArgs& a, int num_sms, cudaStream_t stream, double* estimate = nullptr) {
+    const int mode = splitk_mode();
     if (!mode || !a.splitk_ws || a.M > 384) return 0;
     if (mode == 2 && a.K < 8192) return 0;
     if (a.epi != EPI_NONE && a.epi != EPI_BIAS && a.epi != EPI_RESIDUAL && a.epi != EPI_BIAS_RESIDUAL) return 0;
@@ -787,6 +1247,10 @@ static int try_splitk(const GemmArgs& a, int num_sms, cudaStream_t stream) {
     while (splits > 1 && (splits - 1) * ((nkb + splits - 1) / splits) >= nkb) --splits;  // no empty split
     while (splits > 1 && (size_t)splits * a.M * a.N * 4 > a.splitk_ws_bytes) --splits;
     if (splits < 2) return 0;
+    if (estimate) {   // two launches, the partials written and read once
+        *estimate = 11.0 + (tiles * splits + num_sms - 1) / num_sms * ((nkb + splits - 1) / splits) * 0.41 + (double)a.M * a.N * splits * 4 / 6.5e6;
+        return 1;
+    }
     GemmArgs p = a;
     p.C = a.splitk_ws;
     p.ldc = a.N;
@@ -815,19 +1279,21 @@ int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream) {
     const bool plain = !a.tile_group && a.batch <= 1 && !a.c_f32;
     if (a.batch > 1 && (a.tile_group || (a.K % BLOCK_K) || (a.a_col_stride % 8) || (a.c_col_stride % 8) || a.a_col_stride < 0 || a.c_col_stride < 0)) return -7;
     if (a.c_f32 && (a.epi != EPI_NONE || (a.ldc % 4))) return -8;
+    static const int forced = [] { const char* e = getenv("LIVECC_B200_GEMM_BN"); return e ? atoi(e) : 0; }();  // tuning hook (0/unset = model)
+    const bool choose = plain && a.block_n == 0 && forced <= 0 && a.epi != EPI_SIGMOID_GATE;
+    int width = 0;
+    if (choose) {
+        double us = 0., split_us = 0.;
+        width = choose_pair(a.M, a.N, a.K, num_sms, &us);
+        if (try_splitk(a, num_sms, stream, &split_us) > 0) us = split_us;
+        int bm = 0, splits = 0;
+        if (splitk_mode() != 1 && a.epi != EPI_PARTIAL_F32 && choose_swap(a.M, a.N, a.K, num_sms, us, &bm, &splits))
+            return launch_epi_swap(a, bm, splits, num_sms, stream);
+    }
     if (plain)
         if (int r = try_splitk(a, num_sms, stream)) return r < 0 ? r : 0;
     int block_n = a.block_n;
-    if (block_n == 0) {
-        static int forced = -1;
-        if (forced < 0) {
-            const char* e = getenv("LIVECC_B200_GEMM_BN");  // tuning hook: force one width (0/unset = model)
-            forced = e ? atoi(e) : 0;
-        }
-        block_n = forced > 0 ? forced : choose_bn(a.M, a.N, num_sms);
-        if (forced <= 0 && plain && a.epi != EPI_SIGMOID_GATE)
-            if (const int width = choose_pair(a.M, a.N, a.K, num_sms)) block_n = -width;
-    }
+    if (block_n == 0) block_n = forced > 0 ? forced : (width ? -width : choose_bn(a.M, a.N, num_sms));
     // block_n < 0: the CTA pair's kernel with tile width -block_n
     const bool pair = block_n < 0 && plain && a.epi != EPI_SIGMOID_GATE && (a.epi <= EPI_SWIGLU || block_n % 32 == 0);
     if (block_n < 0) block_n = -block_n;

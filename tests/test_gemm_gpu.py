@@ -125,6 +125,22 @@ def test_gemm_default_kernel_equals_one_cta(ctx, M, N, K, epi):
     assert torch.equal(ctx.gemm(a, b, epilogue=epi), ctx.gemm(a, b, epilogue=epi, block_n=256))
 
 
+@pytest.mark.parametrize("epi", [A.EPI_NONE, A.EPI_BIAS, A.EPI_BIAS_QUICKGELU, A.EPI_BIAS_GELU, A.EPI_RESIDUAL, A.EPI_BIAS_RESIDUAL, A.EPI_SWIGLU, 8, 9, 11])
+@pytest.mark.parametrize("M,N,K", [(1, 3584, 3584), (24, 4608, 3584), (33, 2080, 4104), (281, 3584, 3592), (288, 3584, 18944), (300, 37888, 512), (1000, 1280, 5120),
+                                   (513, 3584, 4096)])
+def test_gemm_few_rows_every_epilogue(ctx, M, N, K, epi):
+    """Few rows run with the operands swapped, K split inside a cluster: equal to the one-CTA kernel on sums that fp32 holds exactly (so
+    the order of the splits cannot show); ragged rows, columns and k, one and two column groups."""
+    a, b = _ints((M, K), -1, 1, 31), _ints((N, K), -1, 1, 32)
+    kw = {}
+    if epi in (A.EPI_BIAS, A.EPI_BIAS_QUICKGELU, A.EPI_BIAS_GELU, A.EPI_BIAS_RESIDUAL):
+        kw["bias"] = _ints((N,), -8, 8, 33)
+    if epi in (A.EPI_RESIDUAL, A.EPI_BIAS_RESIDUAL):
+        kw["residual"] = _ints((M, N), -8, 8, 34)
+    # (activations: integers are exact before them; the fp32 math after the sum is the same code)
+    assert torch.equal(ctx.gemm(a, b, epilogue=epi, **kw), ctx.gemm(a, b, epilogue=epi, block_n=128, **kw))
+
+
 def test_gemm_strided_views(ctx):
     """A and C may be column slices of wider buffers (leading dimension > width)."""
     M, N, K = 256, 384, 320
