@@ -16,8 +16,8 @@
 //
 // A thread owns a row, so one CTA has four softmax warps, one per scheduler, and a tile is a serial chain (TMEM load, maximum, 64
 // exponentials, TMEM store, MMA): 1.8 us per 64 keys with one CTA per SM. Two CTAs fill each other's gaps: 98 KB of shared memory (two
-// slots each for K and V, released apart) and half of the TMEM each: 281 rows over 8 k keys 119 -> 48 us (20 us at
-// the tensor rate), 24 rows over 32 k 115 us with one CTA per SM and 8 splits at most.
+// slots each for K and V, released apart) and half of the TMEM each: 281 rows over 17 k keys 119 -> 89 us (42 us at the
+// tensor rate). Four layers of 24 rows over 64 k keys: 245 us less, of 4 x 115 with 8 splits at most (the keys and values alone: 21 us each).
 #include <algorithm>
 
 #include "common.cuh"
@@ -345,9 +345,9 @@ int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, con
     const int ctas = q_tiles * Hkv;
     const int kv_tiles = (past + S + BN - 1) / BN;
     int nsplit = 1;
-    // two CTAs per SM: split the KV range until those places are taken, with at least 8 tiles of work per split (281 rows x 8 k keys: 4
-    // splits; 24 rows x 32 k keys: 32). Partials that don't fit into the caller's scratch mean fewer splits.
-    if (part_o && part_ml) {
+    // two CTAs per SM: split the KV range until those places are taken, with at least 8 tiles of work per split (281 rows: 4 splits; 24
+    // rows over 64 k keys: 32). Partials that don't fit into the caller's scratch mean fewer splits.
+    if (part_o && part_ml && ((uintptr_t)part_o % 16) == 0 && ((uintptr_t)part_ml % 8) == 0) {
         nsplit = std::max(1, std::min({2 * num_sms / ctas, MAX_SPLIT, kv_tiles / 8}));
         nsplit = std::max(1, (int)std::min((size_t)nsplit, part_capacity_rows / ((size_t)Hkv * S * G)));
     }
