@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(256) latent_kv_append_kernel(const T* __restri
                                                                float* __restrict__ q_out, T* __restrict__ k_pages,
                                                                const int* __restrict__ page_table, int page_size, int H, int D,
                                                                int DR, int R, SeqPos pos, const T* __restrict__ qsrc, int ld_q, bool pairs) {
-    chain_begin();
+    chain_begin(proj, page_table, qsrc);
     if (seq_done(pos)) return;
     __shared__ float red[32];
     const int t = blockIdx.x;

@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256) qk_headnorm_rope_append_kernel(const T* _
                                                                       T* __restrict__ k_pages, T* __restrict__ v_pages,
                                                                       const int* __restrict__ page_table, int page_size, int S, int Hq,
                                                                       int G, int D, int DV, SeqPos pos, AppendOpts ao) {
-    chain_begin();
+    chain_begin(proj, page_table);
     if (seq_done(pos)) return;
     const int t = blockIdx.x;
     const int p = seq_past(pos, S) + t;
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(256) qk_norm_kv_append_kernel(const T* __restr
                                                                 T* __restrict__ k_pages, T* __restrict__ v_pages,
                                                                 const int* __restrict__ page_table, int page_size, int S, int Hq,
                                                                 int G, int D, int DV, SeqPos pos) {
-    chain_begin();
+    chain_begin(proj, page_table);
     if (seq_done(pos)) return;
     __shared__ float red[32];
     const int t = blockIdx.x;
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(128) attn_chunk_sink_kernel(const float* __res
                                                               T* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                               int chunk, float scale, SeqPos pos,
                                                               const float* __restrict__ sink, int ld_v, AttnOpts opt) {
-    chain_begin();
+    chain_begin(q, k_pages, v_pages, page_table, gate);
     if (seq_done(pos)) return;
     extern __shared__ float sm[];
     __shared__ float red[32];
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(256) attn_rows_kernel(const float* __restrict_
                                                         int Hq, int G, int D, int DV, int chunk, float scale, SeqPos pos,
                                                         const float* __restrict__ sink, int ld_v, float* __restrict__ part,
                                                         int* __restrict__ counters, AttnOpts opt) {
-    chain_begin();
+    chain_begin(q, k_pages, v_pages, page_table, gate);
     if (seq_done(pos)) return;
     constexpr int VN = RowVec<T>::N, NVK = 4 * PL / 32;   // value keys per lane: a warp's 4 keys over 32 / PL lane groups
     extern __shared__ __align__(16) float sm[];
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(256) attn_rows_kernel(const float* __restrict_
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int p = l8 + 8 * u;
-            kq[u] = p < PD ? ld_stream16(kr + p * VN) : make_uint4(0, 0, 0, 0);
+            kq[u] = p < PD ? ld_pages16(kr + p * VN) : make_uint4(0, 0, 0, 0);
         }
 #pragma unroll
         for (int it = 0; it < NVK; ++it) {
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(256) attn_rows_kernel(const float* __restrict_
 #pragma unroll
             for (int n = 0; n < NP; ++n) {
                 const int c = lane % PL + PL * n;
-                vq[it][n] = c < PDV ? ld_stream16(v_pages + (size_t)vrow * ld_v + c * VN) : make_uint4(0, 0, 0, 0);
+                vq[it][n] = c < PDV ? ld_pages16(v_pages + (size_t)vrow * ld_v + c * VN) : make_uint4(0, 0, 0, 0);
             }
         }
         float acc[HB];
@@ -376,13 +376,13 @@ __global__ void __launch_bounds__(256) attn_rows_kernel(const float* __restrict_
 #pragma unroll
             for (int u = 0; u < 4; ++u)
                 if (l8 + 8 * u < PD) dots(kq[u], l8 + 8 * u, 0, 1);
-            for (int p = l8 + 32; p < PD; p += 8) dots(ld_stream16(kr + p * VN), p, 0, 1);
+            for (int p = l8 + 32; p < PD; p += 8) dots(ld_pages16(kr + p * VN), p, 0, 1);
         } else {
 #pragma unroll
             for (int u = 0; u < 4; ++u)
                 if (l8 + 8 * u < PD) dots(kq[u], l8 + 8 * u, 0, 2);
-            for (int p = l8 + 32; p < PD; p += 8) dots(ld_stream16(kr + p * VN), p, 0, 2);
-            for (int p = l8; p < PD; p += 8) dots(ld_stream16(kr + D + p * VN), p, 1, 2);
+            for (int p = l8 + 32; p < PD; p += 8) dots(ld_pages16(kr + p * VN), p, 0, 2);
+            for (int p = l8; p < PD; p += 8) dots(ld_pages16(kr + D + p * VN), p, 1, 2);
         }
         float mine = 0.f;
 #pragma unroll
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(128) attn_split_kernel(const float* __restrict
                                                          T* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                          float scale, SeqPos pos, const float* __restrict__ sink, int ld_v,
                                                          float* __restrict__ part, int* __restrict__ counters, AttnOpts opt) {
-    chain_begin();
+    chain_begin(q, k_pages, v_pages, page_table, gate);
     if (seq_done(pos)) return;
     extern __shared__ float sm[];
     __shared__ float red[32];
@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(256) attn_chunk_sink_tiled_kernel(const float*
                                                                     T* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                                     int chunk, float scale, SeqPos pos,
                                                                     const float* __restrict__ sink, int ld_v, AttnOpts opt) {
-    chain_begin();
+    chain_begin(q, k_pages, v_pages, page_table, gate);
     if (seq_done(pos)) return;
     extern __shared__ __align__(16) uint8_t smem_attn[];
     const int dc = min(D, ADC);
@@ -965,7 +965,7 @@ __global__ void __launch_bounds__(128 * KH, (VEC8 && NBUF == 1 && NV == 1) ? 2 :
                                                                   bf16* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                                   int chunk, float scale, SeqPos pos,
                                                                   const float* __restrict__ sink, int ld_v, AttnOpts opt) {
-    chain_begin();
+    chain_begin(q, k_pages, v_pages, page_table, gate);
     if (seq_done(pos)) return;
     extern __shared__ __align__(16) uint8_t smem_attn[];
     // NV output tiles of 128 channels per CTA (NV = 2: values of up to 256 channels against one pass over the scores)
@@ -1342,7 +1342,7 @@ int launch_attn_mma_maps(const float* q, const void* k_pages, const void* v_page
 template <typename T>
 __global__ void __launch_bounds__(128) diff_combine_kernel(const float* __restrict__ a, T* __restrict__ out, int ld_out, int S, int H, int DV,
                                                            float lambda, float scale, float eps, SeqPos pos) {
-    chain_begin();
+    chain_begin(a);
     if (seq_done(pos)) return;
     const int64_t wid = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;

@@ -57,13 +57,23 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // ----------------------------------------------------------------------------
-// Streaming 16-byte loads (weights / KV are read once per step: bypass L1)
+// Streaming 16-byte loads of weights (read once per step: bypass L1; the non-coherent path)
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     uint4 r;
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                  : "l"(p));
+    return r;
+}
+
+// the same for data of this pass (K/V pages): coherent, and not before the asm statements in front of it
+__device__ __forceinline__ uint4 ld_pages16(const void* p) {
+    uint4 r;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+                 : "l"(p)
+                 : "memory");
     return r;
 }
 
@@ -374,7 +384,22 @@ __device__ __forceinline__ void pdl_wait() {}
 // the wait fills the SMs with kernels that only wait: a step of the recurrent design 254 us instead of 231.)
 __device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void chain_begin() { chain_wait(); chain_open(); }
+// Such a kernel is on the SMs while the one before it still writes, so the non-coherent path (ld.global.nc, __ldg, and what the compiler
+// makes of a load through a `const __restrict__` parameter) is for weights and tables alone: the path asks that nobody writes the data while
+// the kernel lives, and its loads may be moved across the wait. Every `__restrict__` pointer to data that an earlier kernel or copy of the
+// pass wrote is therefore named in chain_begin: from the wait on it is a value the compiler knows nothing about, read by coherent loads only.
+template <typename P>
+__device__ __forceinline__ void chain_fresh(P& p) {
+    size_t at = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(at));
+    p = static_cast<P>(__cvta_global_to_generic(at));
+}
+template <typename... P>
+__device__ __forceinline__ void chain_begin(P&... written_before) {
+    chain_wait();
+    chain_open();
+    (chain_fresh(written_before), ...);
+}
 
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred = 0;

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) hyper_boundary_kernel(float* __restrict__
                                                              const float* __restrict__ prev, const float* __restrict__ next,
                                                              const float* __restrict__ w, float eps, T* __restrict__ xa,
                                                              float* __restrict__ sum_out, int W) {
-    chain_begin();
+    chain_begin(xs);
     __shared__ float red[32];
     constexpr bool FAST = N > 0 && E > 0;
     const int n = N > 0 ? N : n_rt;

@@ -52,7 +52,7 @@ template <typename T, typename TC>
 __global__ void __launch_bounds__(256) linear_tile_kernel(const T* __restrict__ A, int lda, const T* __restrict__ W, int ldw,
                                                           const float* __restrict__ bias, TC* __restrict__ C, int ldc, int M,
                                                           int N, int K, Grp g) {
-    chain_begin();
+    chain_begin(A);
     __shared__ float As[BK][BM + 4];
     __shared__ float Ws[BK][BN + 4];
     const int tid = threadIdx.x;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
         load_weights(lane * V);
         loaded = true;
     }
-    chain_begin();
+    chain_begin(A);
     if (g.row_off) {
         if (g.compact) {
             // a decode step routes a handful of rows to a handful of lists: the grid has one y per possible non-empty list
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
                 for (int m = 0; m < MM; ++m) {
                     if (m < M) {
                         float av[V];
-                        Vec16<T>::unpack(__ldg(reinterpret_cast<const uint4*>(arp[m] + k)), av);
+                        Vec16<T>::unpack(*reinterpret_cast<const uint4*>(arp[m] + k), av);
 #pragma unroll
                         for (int r = 0; r < WR; ++r)
 #pragma unroll

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
                                                         int E, int top, float scale, int* __restrict__ sel,
                                                         float* __restrict__ weight, float* __restrict__ shared_gate,
                                                         int* __restrict__ counts, int* __restrict__ rank, int S, MoeRouterOpts ro) {
-    chain_begin();
+    chain_begin(logits);
     __shared__ float gch[4][kRouteScratch];
     __shared__ unsigned char gkeep[4][kRouteScratch];
     const int warp = threadIdx.x >> 5;
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256) moe_route_small_kernel(const float* __res
                                                               float* __restrict__ weight, float* __restrict__ shared_gate,
                                                               int* __restrict__ row_off, int* __restrict__ pos,
                                                               int* __restrict__ src_row, int S, MoeRouterOpts ro) {
-    chain_begin();
+    chain_begin(logits);
     __shared__ int cnt[kSmallRouteExperts + 1];
     __shared__ int rk[kSmallRouteItems];
     __shared__ float gch[8][kRouteScratch];
@@ -197,7 +197,7 @@ __device__ __forceinline__ int padded(int n, int pad) { return (n + pad - 1) / p
 __global__ void moe_index_kernel(const int* __restrict__ sel, const int* __restrict__ rank, const int* __restrict__ counts, int E,
                                  int top, int pad, int* __restrict__ row_off, int* __restrict__ pos, int* __restrict__ src_row,
                                  int* __restrict__ tile_group, int n_tiles, int S) {
-    chain_begin();
+    chain_begin(sel, rank, counts);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= E) {
         int o = 0;
@@ -227,7 +227,7 @@ __global__ void moe_index_kernel(const int* __restrict__ sel, const int* __restr
 // out[i, :] = in[src_row[i], :] for every list row (16-byte pieces); padding rows (src_row < 0) are left alone.
 __global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict__ in, int ld_in16, const int* __restrict__ src_row,
                                                          uint4* __restrict__ out, int ld_out16, int n16) {
-    chain_begin();
+    chain_begin(in, src_row);
     const int r = src_row[blockIdx.x];
     if (r < 0) return;
     for (int c = threadIdx.x; c < n16; c += blockDim.x) out[(size_t)blockIdx.x * ld_out16 + c] = in[(size_t)r * ld_in16 + c];

@@ -44,7 +44,7 @@ template <typename TI, typename T, bool SILU, bool ADD>
 __global__ void causal_conv_kernel(const TI* __restrict__ in, int ld_in, T* __restrict__ out, int ld_out,
                                    const float* __restrict__ w, const float* __restrict__ b,
                                    const float* carry, float* carry_out, int S, int C, int taps, SeqPos pos) {
-    chain_begin();
+    chain_begin(in);
     if (seq_done(pos)) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int t0 = blockIdx.y * kConvRows;
@@ -95,7 +95,7 @@ template <int TAPS, bool SILU>
 __global__ void __launch_bounds__(128) causal_conv_long_kernel(const bf16* __restrict__ in, int ld_in, bf16* __restrict__ out, int ld_out,
                                                                const float* __restrict__ w, const float* __restrict__ b,
                                                                const float* __restrict__ carry, int S, int C, int span, SeqPos pos) {
-    chain_begin();
+    chain_begin(in, carry);
     if (seq_done(pos)) return;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 2;
     const int t0 = blockIdx.y * span;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(128) causal_conv_long_kernel(const bf16* __res
 template <typename T>
 __global__ void conv_carry_update_kernel(const T* __restrict__ in, int ld_in, float* __restrict__ carry, int S, int C,
                                          int taps, SeqPos pos) {
-    chain_begin();
+    chain_begin(in, carry);
     if (seq_done(pos)) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
@@ -150,7 +150,7 @@ template <typename T>
 __global__ void ssm_step_decay_kernel(const T* __restrict__ raw, int ld, const float* __restrict__ dt_bias,
                                       const float* __restrict__ a_log, float* __restrict__ dt_out,
                                       float* __restrict__ decay_out, int S, int heads) {
-    chain_begin();
+    chain_begin(raw);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= S * heads) return;
     const int t = i / heads, h = i % heads;
@@ -162,7 +162,7 @@ __global__ void ssm_step_decay_kernel(const T* __restrict__ raw, int ld, const f
 template <typename T>
 __global__ void gla_decay_kernel(const T* __restrict__ z, int ld, const float* __restrict__ bias, float inv_tau,
                                  float* __restrict__ decay_out, int S, int n) {
-    chain_begin();
+    chain_begin(z);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= S * n) return;
     const int t = i / n, c = i % n;

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(256) rotary_pack_kernel(const T* __restrict__ 
                                                           Segs segs, const float* __restrict__ inv_freq, float mag,
                                                           const float* __restrict__ fill, float* __restrict__ fill_out, int fill_n,
                                                           SeqPos pos) {
-    chain_begin();
+    chain_begin(in, fill);
     if (seq_done(pos)) return;
     const int t = blockIdx.x;
     const float p = (float)(seq_past(pos) + t);

@@ -46,7 +46,7 @@ template <typename T>
 __global__ void embed_sinusoid_kernel(const int64_t* __restrict__ ids, const int* __restrict__ seq_len, const T* __restrict__ table,
                                       int64_t vocab, float scale, const float* __restrict__ inv_freq, float* __restrict__ x32,
                                       T* __restrict__ xa, int S, int W, SeqPos pos, int copies) {
-    chain_begin();
+    chain_begin(ids, seq_len);
     if (seq_done(pos)) return;
     const int r = blockIdx.x;
     const int64_t id = seq_len ? ids[*seq_len - S + r] : ids[r];
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) postnorm_residual_kernel(float* __restric
                                                                 int ld_a, const float* __restrict__ wa, const T* __restrict__ b,
                                                                 int ld_b, const float* __restrict__ wb, const float* __restrict__ w,
                                                                 float alpha, float eps, int W) {
-    chain_begin();
+    chain_begin(x32, a, b);
     __shared__ float red[32];
     const int r = blockIdx.x;
     float* x = x32 + (size_t)r * W;
@@ -152,7 +152,7 @@ template <typename T, int E, bool VEC>
 __global__ void __launch_bounds__(256) postnorm_branch_kernel(float* __restrict__ x32, T* __restrict__ xa, const T* __restrict__ a, int ld_a,
                                                               bool has_mc, MoeCombine mc, const float* __restrict__ ls,
                                                               const float* __restrict__ w, float alpha, float eps, int W) {
-    chain_begin();
+    chain_begin(x32, a);
     __shared__ float red[32];
     __shared__ int spos[kCombineTop];
     __shared__ float swt[kCombineTop];
@@ -252,7 +252,7 @@ template <typename T, int TEAM, int E>
 __global__ void __launch_bounds__(256) gated_group_norm_kernel(const float* __restrict__ y, int ld_y, const T* __restrict__ gate,
                                                                int ld_gate, const float* __restrict__ w, int w_len, T* __restrict__ out,
                                                                int ld_out, int S, int n, int group, int gate_first, float eps) {
-    chain_begin();
+    chain_begin(y, gate);
     __shared__ float red[32];
     const int ngroups = n / group;
     const int wid = TEAM == 32 ? blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x;
@@ -315,7 +315,7 @@ template <typename T, int TEAM, int E>
 __global__ void __launch_bounds__(TEAM == 32 ? 64 : TEAM) gated_group_norm4_kernel(const float* __restrict__ y, int ld_y, const T* __restrict__ gate,
                                                                 int ld_gate, const float* __restrict__ w, int w_len, T* __restrict__ out,
                                                                 int ld_out, int S, int n, int group, int gate_first, float eps) {
-    chain_begin();
+    chain_begin(y, gate);
     __shared__ float red[32];
     const int ngroups = n / group, wid = TEAM == 32 ? blockIdx.x * 2 + (threadIdx.x >> 5) : blockIdx.x, lane = TEAM == 32 ? (threadIdx.x & 31) : threadIdx.x;
     if (wid >= S * ngroups) return;
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(TEAM == 32 ? 64 : TEAM) gated_group_norm4_kern
 // four columns per thread where the rows allow it (NV = 4), else one
 template <typename T, int NV>
 __global__ void __launch_bounds__(256) glu_gelu_tanh_kernel(const T* __restrict__ gu, int ld, T* __restrict__ out, int ld_out, int S, int F) {
-    chain_begin();
+    chain_begin(gu);
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * NV;
     if (i >= (int64_t)S * F) return;
     const int r = (int)(i / F), c = (int)(i % F);
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(256) glu_gelu_tanh_kernel(const T* __restrict_
 template <typename T>
 __global__ void __launch_bounds__(256) gather_rmsnorm_kernel(const float* __restrict__ x32, const int* __restrict__ rows,
                                                              const float* __restrict__ w, float eps, T* __restrict__ out, int W) {
-    chain_begin();
+    chain_begin(x32, rows);
     __shared__ float red[32];
     const int i = blockIdx.x;
     const float* x = x32 + (size_t)rows[i] * W;
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(256) gather_rmsnorm_kernel(const float* __rest
 template <typename T>
 __global__ void __launch_bounds__(128) slice_rmsnorm_kernel(const T* __restrict__ in, int ld_in, const float* __restrict__ w, float eps,
                                                             T* __restrict__ out, int ld_out, int n) {
-    chain_begin();
+    chain_begin(in);
     __shared__ float red[32];
     const T* x = in + (size_t)blockIdx.x * ld_in;
     float ss = 0.f;
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(128) slice_rmsnorm_kernel(const T* __restrict_
 }
 
 __global__ void softcap_kernel(float* __restrict__ x, int64_t n, float cap, float inv_cap, float scale) {
-    chain_begin();
+    chain_begin(x);
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) x[i] = (cap > 0.f ? cap * tanhf(x[i] * inv_cap) : x[i]) * scale;
 }
@@ -413,7 +413,7 @@ __device__ __forceinline__ float norm_apply(const NormSpec& n, float v, float rn
 template <typename T>
 __global__ void __launch_bounds__(256) gather_norm_kernel(const float* __restrict__ x32, const int* __restrict__ rows, NormSpec n,
                                                           T* __restrict__ out, int W) {
-    chain_begin();
+    chain_begin(x32, rows);
     __shared__ float red[32];
     const int i = blockIdx.x;
     const float* x = x32 + (size_t)rows[i] * W;
@@ -440,7 +440,7 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ x32, const T* __restrict__ a, int ld_a,
                                                             const T* __restrict__ b, int ld_b, bool has_mc, MoeCombine mc, NormSpec n,
                                                             T* __restrict__ xa, int W) {
-    chain_begin();
+    chain_begin(x32, a, b);
     __shared__ float red[32];
     __shared__ int spos[kCombineTop];
     __shared__ float swt[kCombineTop];
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(256) residual_norm_kernel(float* __restrict__ 
 template <typename T>
 __global__ void glu_clamp_swish_kernel(const T* __restrict__ gu, int ld, T* __restrict__ out, int ld_out, int S, int F, float limit, bool il16,
                                        float alpha, float up_bias) {
-    chain_begin();
+    chain_begin(gu);
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)S * F) return;
     const int r = (int)(i / F), c = (int)(i % F);
@@ -541,7 +541,7 @@ template <typename T, int E, bool VEC>
 __global__ void __launch_bounds__(256) branch_norm_residual_kernel(float* __restrict__ x32, const T* __restrict__ a, int ld_a, bool has_mc,
                                                                    MoeCombine mc, const float* __restrict__ w, float eps,
                                                                    T* __restrict__ xa, int W) {
-    chain_begin();
+    chain_begin(x32, a);
     __shared__ float red[32];
     __shared__ int spos[kCombineTop];
     __shared__ float swt[kCombineTop];
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(256) branch_norm_residual_kernel(float* __rest
 template <typename T, int E, bool VEC>
 __global__ void __launch_bounds__(256) sandwich_residual_kernel(float* __restrict__ x32, const T* __restrict__ a, int ld_a, bool has_mc,
                                                                 MoeCombine mc, NormSpec post, NormSpec next, T* __restrict__ xa, int W) {
-    chain_begin();
+    chain_begin(x32, a);
     __shared__ float red[32];
     __shared__ int spos[kCombineTop];
     __shared__ float swt[kCombineTop];

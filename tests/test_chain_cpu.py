@@ -1,0 +1,73 @@
+"""Chained launches of the hybrid sequence models, read from the sources: a kernel that lies on the SMs while the one before it still writes
+may take the non-coherent read path (ld.global.nc: explicit, `__ldg`, or a load through a `const __restrict__` parameter) for weights and
+tables alone."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "livecc_b200" / "csrc"
+FILES = ["rowops", "recurrent", "recurrent_chunked", "attn_local", "attn_latent", "hyper", "moe", "rotary", "linear_any"]
+
+# `__restrict__` parameters that no kernel or copy of a pass writes before the kernel reads them: weights and tables, and what it only writes
+WEIGHTS = {
+    "embed_sinusoid_kernel": "table inv_freq", "postnorm_residual_kernel": "wa wb w", "postnorm_branch_kernel": "ls w",
+    "gated_group_norm_kernel": "w", "gated_group_norm4_kernel": "w", "gather_rmsnorm_kernel": "w", "slice_rmsnorm_kernel": "w",
+    "branch_norm_residual_kernel": "w", "causal_conv_kernel": "w b", "causal_conv_long_kernel": "w b", "ssm_step_decay_kernel": "dt_bias a_log",
+    "gla_decay_kernel": "bias", "qk_headnorm_rope_append_kernel": "qn_w kn_w inv_freq", "qk_norm_kv_append_kernel": "qn_w kn_w",
+    "attn_chunk_sink_kernel": "sink", "attn_rows_kernel": "sink", "attn_split_kernel": "sink", "attn_chunk_sink_tiled_kernel": "sink",
+    "attn_chunk_sink_mma_kernel": "sink", "latent_kv_append_kernel": "norm_w inv_freq", "hyper_boundary_kernel": "prev next w",
+    "moe_route_kernel": "correction", "moe_route_small_kernel": "correction", "rotary_pack_kernel": "inv_freq",
+    "linear_tile_kernel": "W bias", "linear_rows_kernel": "W bias",
+}
+WRITTEN = {
+    "embed_sinusoid_kernel": "x32 xa", "postnorm_residual_kernel": "xa", "postnorm_branch_kernel": "xa", "gated_group_norm_kernel": "out",
+    "gated_group_norm4_kernel": "out", "glu_gelu_tanh_kernel": "out", "gather_rmsnorm_kernel": "out", "slice_rmsnorm_kernel": "out",
+    "gather_norm_kernel": "out", "residual_norm_kernel": "xa", "glu_clamp_swish_kernel": "out", "branch_norm_residual_kernel": "xa",
+    "sandwich_residual_kernel": "xa", "causal_conv_kernel": "out", "causal_conv_long_kernel": "out", "ssm_step_decay_kernel": "dt_out decay_out",
+    "gla_decay_kernel": "decay_out", "qk_headnorm_rope_append_kernel": "q_out k_pages v_pages", "qk_norm_kv_append_kernel": "q_out k_pages v_pages",
+    "attn_chunk_sink_kernel": "out", "attn_rows_kernel": "out part counters", "attn_split_kernel": "out part counters",
+    "attn_chunk_sink_tiled_kernel": "out", "attn_chunk_sink_mma_kernel": "out", "diff_combine_kernel": "out",
+    "latent_kv_append_kernel": "q_out k_pages", "hyper_boundary_kernel": "xa sum_out", "moe_route_kernel": "sel weight shared_gate counts rank",
+    "moe_route_small_kernel": "sel weight shared_gate row_off pos src_row", "moe_index_kernel": "row_off pos src_row tile_group",
+    "moe_gather_kernel": "out", "rotary_pack_kernel": "out fill_out", "linear_tile_kernel": "C", "linear_rows_kernel": "C",
+}
+
+
+def kernels(name):
+    """(kernel name, parameter text, body) of every __global__ function of a file."""
+    src = re.sub(r"//[^\n]*", "", (CSRC / f"{name}.cu").read_text())
+    out = []
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\(([^{]*)\)\s*\{", src):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(src[i], 0)
+            i += 1
+        out.append((m.group(1), m.group(2), src[m.end():i]))
+    return src, out
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_chained_kernels_wait_and_name_what_was_written_before(name):
+    src, found = kernels(name)
+    chained = set(re.findall(r"chained\(\s*(\w+)", src))
+    assert chained and chained <= {k for k, _, _ in found}
+    for kernel, params, body in found:
+        if kernel not in chained:
+            continue
+        begin = re.findall(r"chain_begin\(([^)]*)\);", body)
+        assert len(begin) == 1, kernel
+        if kernel != "linear_rows_kernel":     # (that one loads weights before it waits)
+            assert body.lstrip().startswith("chain_begin("), kernel
+        restrict = set(re.findall(r"\*\s*__restrict__\s+(\w+)", params))
+        named = set(filter(None, re.split(r"[,\s]+", begin[0])))
+        rest = set((WEIGHTS.get(kernel, "") + " " + WRITTEN.get(kernel, "")).split())
+        assert named | rest == restrict and not named & rest, f"{kernel}: {sorted(restrict - named - rest)} may be read non-coherently"
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_explicit_non_coherent_loads_are_of_weights(name):
+    src, _ = kernels(name)
+    allowed = {"linear_any": ["W + (size_t)wrow(r) * ldw + k"], "attn_local": ["row + min(dist, len - 1)"]}   # weights; the distance table
+    loads = [a for a in re.findall(r"(?:ld_stream16|__ldg)\(((?:[^()]|\([^()]*\))*)\)", src)]
+    assert [a for a in loads if a not in allowed.get(name, [])] == []
