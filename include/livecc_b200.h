@@ -85,6 +85,16 @@ int lcc_gemm_bf16(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, 
                   int M, int N, int K, const void* bias, const void* residual, int ldr, int epilogue,
                   int block_n, void* splitk_ws, int64_t splitk_ws_bytes, lcc_stream_t stream);
 
+/* Which kernel block_n = 0 takes without split-K scratch: plan[0] = 0 one CTA per tile, 1 CTA pairs, 2 CTA pairs with the weights as the
+ * 256-row operand; plan[1] = tile width (for 2: rows of A per tile); plan[2] = pairs of a cluster that share a tile's K. */
+int lcc_gemm_plan(int num_sms, int M, int N, int K, int32_t* plan);
+/* lcc_gemm_bf16 with one explicit kernel (form, width and splits as in lcc_gemm_plan; any epilogue but the per-head gate), for tests and
+ * tuning. limit, alpha and up_bias: epilogue 10, gate and up rows interleaved by 16 as for LCC_EPI_SWIGLU:
+ * g = min(gate, limit), u = clamp(up, +-limit), C = g * sigmoid(alpha * g) * (u + up_bias). */
+int lcc_gemm_form(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K, const void* bias,
+                  const void* residual, int ldr, int epilogue, int form, int width, int splits, float limit, float alpha, float up_bias,
+                  lcc_stream_t stream);
+
 /* hidden_states.to(bf16) of the f32 patch rows (mq2vl.py:309). */
 int lcc_cast_f32_bf16(lcc_ctx* ctx, const float* in, void* out, int64_t n, lcc_stream_t stream);
 

@@ -18,6 +18,7 @@ PAGE_SIZE = 64
 
 # epilogue codes (LCC_EPI_*)
 EPI_NONE, EPI_BIAS, EPI_BIAS_QUICKGELU, EPI_BIAS_GELU, EPI_RESIDUAL, EPI_BIAS_RESIDUAL, EPI_SWIGLU = range(7)
+EPI_CLAMP_GLU = 10
 # stream scalar slots (LCC_SC_*)
 SC_KV_LEN, SC_ROPE_POS, SC_FINISHED, SC_N_GENERATED, SC_SEQ_LEN, SC_LAST_TOKEN, SC_VIDEO_TOKENS, SC_NATIVE_ERROR = range(8)
 SC_COUNT = 8
@@ -147,6 +148,7 @@ def _declare(lib: C.CDLL):
     sig("lcc_destroy", None, [C.c_void_p])
     sig("lcc_last_error", C.c_char_p, [C.c_void_p])
     sig("lcc_num_sms", None, [C.c_void_p])
+    sig("lcc_gemm_plan", None, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p])
     sig("lcc_launch_count", C.c_uint64, [])
     sig("lcc_model_create", C.c_void_p, [C.c_void_p, C.POINTER(ModelConfig), C.POINTER(ModelWeights)])
     sig("lcc_model_destroy", None, [C.c_void_p])
@@ -292,6 +294,24 @@ class Context:
                   _i(M), _i(N), _i(K), _ptr(bias), _ptr(residual), _i(ldr), _i(epilogue), _i(block_n), _ptr(splitk_ws),
                   C.c_int64(splitk_ws.numel() * splitk_ws.element_size() if splitk_ws is not None else 0),
                   self.stream_ptr())
+        return out
+
+    def gemm_plan(self, M, N, K):
+        """(form, width, splits) that gemm() takes for a plain product: form 0 one CTA per tile, 1 CTA pairs, 2 swapped operands."""
+        plan = (C.c_int32 * 3)()
+        self.check(self.lib.lcc_gemm_plan(self.num_sms, int(M), int(N), int(K), plan), "lcc_gemm_plan")
+        return tuple(plan)
+
+    def gemm_form(self, a, b, form, width, splits=1, bias=None, residual=None, epilogue=EPI_NONE, limit=0.0, alpha=1.702, up_bias=1.0, out=None):
+        """gemm() by one explicit kernel (tests and tuning); epilogue 10 is the clamped gated activation."""
+        import torch
+
+        (M, K), N = a.shape, b.shape[0]
+        if out is None:
+            out = torch.empty((M, N // 2 if epilogue in (EPI_SWIGLU, EPI_CLAMP_GLU) else N), dtype=torch.bfloat16, device=a.device)
+        self.call("lcc_gemm_form", _ptr(a), _i(a.stride(0)), _ptr(b), _i(b.stride(0)), _ptr(out), _i(out.stride(0)), _i(M), _i(N), _i(K),
+                  _ptr(bias), _ptr(residual), _i(residual.stride(0) if residual is not None else 0), _i(epilogue), _i(form), _i(width),
+                  _i(splits), C.c_float(limit), C.c_float(alpha), C.c_float(up_bias), self.stream_ptr())
         return out
 
     def cast_f32_bf16(self, x):

@@ -51,6 +51,30 @@ int lcc_gemm_bf16(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, 
     return 0;
 }
 
+int lcc_gemm_plan(int num_sms, int M, int N, int K, int32_t* plan) {
+    if (!plan || num_sms < 2 || M < 1 || N < 1 || K < 1) return -1;
+    lcc::GemmArgs a{};
+    a.M = M; a.N = N; a.K = K;
+    a.epi = lcc::EPI_NONE;
+    const lcc::GemmPlan p = lcc::gemm_plan(a, num_sms);
+    plan[0] = p.form; plan[1] = p.width; plan[2] = p.splits;
+    return 0;
+}
+
+int lcc_gemm_form(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K, const void* bias,
+                  const void* residual, int ldr, int epilogue, int form, int width, int splits, float limit, float alpha, float up_bias,
+                  lcc_stream_t stream) {
+    if (!ctx) return -1;
+    lcc::GemmArgs a{};
+    a.A = A; a.B = B; a.C = C;
+    a.M = M; a.N = N; a.K = K;
+    a.lda = lda; a.ldb = ldb; a.ldc = ldc;
+    a.bias = bias; a.residual = residual; a.ldr = ldr;
+    a.epi = epilogue; a.epi_param = limit; a.epi_alpha = alpha; a.epi_up_bias = up_bias;
+    int r = form < lcc::FORM_ONE || form > lcc::FORM_SWAP ? -6 : lcc::gemm_bf16_tn_form(a, (lcc::GemmForm)form, width, splits, ctx->num_sms, (cudaStream_t)stream);
+    if (r) LCC_FAIL(ctx, r, "lcc_gemm_form failed (code %d; M=%d N=%d K=%d epi=%d form=%d width=%d splits=%d)", r, M, N, K, epilogue, form, width, splits);
+    return 0;
+}
 
 #define OP_RET(ctx, expr, name)                                              \
     do {                                                                     \

@@ -59,6 +59,14 @@ struct GemmArgs {
 
 int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream);
 
+// The kernels of a plain product: one CTA per 128-row tile; CTA pairs with 256-row tiles; pairs with the weights as the 256-row operand,
+// `width` activation rows per tile and K split over `splits` pairs of a cluster.
+enum GemmForm { FORM_ONE = 0, FORM_PAIR = 1, FORM_SWAP = 2 };
+struct GemmPlan { GemmForm form = FORM_ONE; int width = 0, splits = 1; };
+GemmPlan gemm_plan(const GemmArgs& a, int num_sms);   // what block_n = 0 takes
+// One explicit form (tests, tuning): width a multiple of 32, up to 256 (FORM_SWAP: 512)
+int gemm_bf16_tn_form(const GemmArgs& a, GemmForm form, int width, int splits, int num_sms, cudaStream_t stream);
+
 // TMA descriptor of a row-major bf16 matrix [rows, cols] (row stride ld elements) with box [box_rows, box_cols];
 // box_cols*2 bytes must equal the swizzle span: 128 (SWIZZLE_128B) or 32 (swizzle32 = SWIZZLE_32B).
 // Out-of-range rows/cols are zero-filled.

@@ -544,14 +544,14 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 // ----------------------------------------------------------------------------
 struct SwapTile {
     int bm, n1, n2;      // activation rows per tile = columns of the first and (0: none) second MMA, multiples of 32
-    int stages, bufs;    // ring depth; accumulator buffers in TMEM
+    int stages;          // ring depth
     int tmem_cols;
     int splits;          // pairs of a cluster that share a tile's K range
     uint32_t idesc1, idesc2;
     int stage_bytes, smem_bytes;
 };
 static constexpr int kSwapMax = 512, kSwapSplits = 4;
-static SwapTile make_swap(int bm, int splits, bool many) {
+static SwapTile make_swap(int bm, int splits) {
     SwapTile t;
     t.bm = bm;
     t.n1 = bm <= 256 ? bm : (bm / 2 + 31) / 32 * 32;
@@ -559,9 +559,8 @@ static SwapTile make_swap(int bm, int splits, bool many) {
     t.stage_bytes = A_BYTES + bm / 2 * BLOCK_K * 2;
     t.stages = (227 * 1024 - 1024 - 256) / t.stage_bytes;
     if (t.stages > MAX_STAGES) t.stages = MAX_STAGES;
-    t.bufs = many && 2 * bm <= 512 ? 2 : 1;
     t.tmem_cols = 32;
-    while (t.tmem_cols < t.bufs * bm) t.tmem_cols <<= 1;
+    while (t.tmem_cols < bm) t.tmem_cols <<= 1;
     t.splits = splits;
     t.idesc1 = make_idesc_bf16(2 * BLOCK_M, t.n1);
     t.idesc2 = t.n2 ? make_idesc_bf16(2 * BLOCK_M, t.n2) : 0u;
@@ -618,13 +617,6 @@ template <int EPI> struct SwapEpi {
 template <int EPI>
 __device__ __forceinline__ void swap_store(const float (&v)[32], bf16* C, int ldc, int M, int N, int m0, int n, int lane, float bias,
                                            const uint2 (&res)[8], float limit, float alpha, float up_bias) {
-    if (EPI == EPI_PARTIAL_F32) {   // fp32 output: 32 consecutive columns per store
-        float* out = reinterpret_cast<float*>(C);
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (m0 + j < M && n < N) out[(size_t)(m0 + j) * ldc + n] = v[j];
-        return;
-    }
     if (SwapEpi<EPI>::kGlu) {
         // lanes 0..15 hold gate rows, 16..31 the matching up rows: of rows j, j + 1 the lower half makes row j, the upper half row j + 1
         const bool hi = lane & 16;
@@ -694,8 +686,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
     uint64_t* empty_bar = full_bar + MAX_STAGES;
     uint64_t* tmem_full = empty_bar + MAX_STAGES;
-    uint64_t* tmem_empty = tmem_full + 2;
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+    uint64_t* tmem_empty = tmem_full + 1;
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 1);
     volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -720,10 +712,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             mbar_init(&full_bar[i], 1);   // used in the leader: its producer's arrive.expect_tx (bytes of both CTAs)
             mbar_init(&empty_bar[i], 1);  // one multicast commit of the leader's MMA warp
         }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&tmem_full[i], 1);    // one multicast commit
-            mbar_init(&tmem_empty[i], 16);  // used in the leader: 8 epilogue warps of each CTA
-        }
+        mbar_init(tmem_full, 1);    // one multicast commit
+        mbar_init(tmem_empty, 16);  // used in the leader: 8 epilogue warps of each CTA
         *gave_up = 0;
         fence_barrier_init();
     }
@@ -761,13 +751,12 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     } else if (warp == 1) {
         // ===================== MMA issuer (leader CTA only) =====================
         if (leader) {
-            int stage = 0, acc = 0;
+            int stage = 0;
             uint32_t phase = 0, acc_phase = 0;
             const uint16_t both = (uint16_t)(3u << lead);
             for (int unit = cluster; unit < units; unit += num_clusters) {
-                mbar_wait_or(&tmem_empty[acc], acc_phase ^ 1, gave_up);
+                mbar_wait_or(tmem_empty, acc_phase ^ 1, gave_up);
                 tc_fence_after();
-                const uint32_t tmem_d = tmem_base + acc * cfg.bm;
                 for (int kb = kb0; kb < kb1; ++kb) {
                     mbar_wait_or(&full_bar[stage], phase, gave_up);
                     tc_fence_after();
@@ -779,23 +768,22 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 #pragma unroll
                         for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
                             const uint32_t add = ((kb - kb0) | k) != 0 ? 1u : 0u;
-                            umma_bf16_ss_cg2(tmem_d, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), cfg.idesc1, add);
-                            if (cfg.n2) umma_bf16_ss_cg2(tmem_d + cfg.n1, dw + (uint64_t)(k * 2), dx2 + (uint64_t)(k * 2), cfg.idesc2, add);
+                            umma_bf16_ss_cg2(tmem_base, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), cfg.idesc1, add);
+                            if (cfg.n2) umma_bf16_ss_cg2(tmem_base + cfg.n1, dw + (uint64_t)(k * 2), dx2 + (uint64_t)(k * 2), cfg.idesc2, add);
                         }
                         umma_commit_cg2(&empty_bar[stage], both);  // frees the slot in both CTAs when the MMAs retire
-                        if (kb == kb1 - 1) umma_commit_cg2(&tmem_full[acc], both);
+                        if (kb == kb1 - 1) umma_commit_cg2(tmem_full, both);
                     }
                     __syncwarp();
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
-                if (++acc == cfg.bufs) { acc = 0; acc_phase ^= 1; }
+                acc_phase ^= 1;
             }
         }
     } else if (warp >= 4) {
         // ===================== Epilogue (both CTAs, own 128 weight rows) =====================
         const int q = warp & 3, half = (warp - 4) >> 2;   // TMEM lane quarter; every other chunk of 32 activation rows
         const int chunks = cfg.bm >> 5;
-        int acc = 0;
         uint32_t acc_phase = 0;
         for (int unit = cluster; unit < units; unit += num_clusters) {
             const int m0 = (unit % m_tiles) * cfg.bm;
@@ -816,9 +804,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             int c = 0;
             while (c < chunks && !mine(c)) ++c;
             if (SwapEpi<EPI>::kResidual && c < chunks) fetch(c);
-            mbar_wait_or(&tmem_full[acc], acc_phase, gave_up);
+            mbar_wait_or(tmem_full, acc_phase, gave_up);
             tc_fence_after();
-            const uint32_t taddr = tmem_base + (uint32_t)(acc * cfg.bm) + ((uint32_t)(q * 32) << 16);
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
             float* red = reinterpret_cast<float*>(smem) + q * 32 + lane;   // [chunk][32 columns][128 weight rows]: over the drained ring
             if (S > 1) {
                 for (int d = half; d < chunks; d += 2) {
@@ -868,8 +856,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tmem_empty[acc]), lead));
-            if (++acc == cfg.bufs) { acc = 0; acc_phase ^= 1; }
+            if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(tmem_empty), lead));
+            acc_phase ^= 1;
         }
     }
 
@@ -1042,7 +1030,7 @@ template <int EPI>
 static int launch_swap(const GemmArgs& a, int bm, int splits, int num_sms, cudaStream_t stream) {
     const int units = (a.M + bm - 1) / bm * ((a.N + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
     const int clusters = std::min(units, max_clusters(splits, num_sms));
-    const SwapTile cfg = make_swap(bm, splits, units > clusters);
+    const SwapTile cfg = make_swap(bm, splits);
     // a shared K range: every unit has its cluster, every pair a k-block, and the partial accumulators fit over the ring
     if (splits > 1 && (clusters < units || (a.K + BLOCK_K - 1) / BLOCK_K < splits || bm * BLOCK_M * 4 > cfg.stages * cfg.stage_bytes)) return -15;
     CUtensorMap tw, t1, t2;
@@ -1163,7 +1151,7 @@ static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_
         for (int sp = 1; sp <= kSwapSplits; ++sp) {
             const int fit = max_clusters(sp, num_sms), waves = (units + fit - 1) / fit;
             if (waves > (sp == 1 && m_tiles == 1 ? 2 : 1) || nkb < 4 * sp) continue;
-            const SwapTile t = make_swap(bm, sp, false);
+            const SwapTile t = make_swap(bm, sp);
             if (sp > 1 && bm * BLOCK_M * 4 > t.stages * t.stage_bytes) continue;
             const double us = 10.0 + waves * ((nkb + sp - 1) / sp) * std::max(0.42, bm / 700.0) + 0.5 * bm / 64 + (sp > 1 ? 3.5 : 0.0);
             if (us < best) { best = us; *bm_out = bm; *splits_out = sp; found = true; }
@@ -1267,7 +1255,20 @@ static int try_splitk(const GemmArgs& a, int num_sms, cudaStream_t stream, doubl
     return cudaGetLastError() == cudaSuccess ? 1 : -13;
 }
 
-int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream) {
+// The form that a plain product of block_n = 0 takes (a split K in global memory counts as FORM_ONE; try_splitk decides on it).
+GemmPlan gemm_plan(const GemmArgs& a, int num_sms) {
+    GemmPlan p;
+    double us = 0., split_us = 0.;
+    const int width = choose_pair(a.M, a.N, a.K, num_sms, &us);
+    p.width = width ? width : choose_bn(a.M, a.N, num_sms);
+    if (width) p.form = FORM_PAIR;
+    if (try_splitk(a, num_sms, nullptr, &split_us) > 0) { us = split_us; p.form = FORM_ONE; }
+    int bm = 0, splits = 0;
+    if (splitk_mode() != 1 && a.epi != EPI_PARTIAL_F32 && choose_swap(a.M, a.N, a.K, num_sms, us, &bm, &splits)) p = GemmPlan{FORM_SWAP, bm, splits};
+    return p;
+}
+
+static int check_args(const GemmArgs& a) {
     if (a.M <= 0 || a.N <= 0 || a.K <= 0) return -1;
     if ((a.K % 8) || (a.lda % 8) || (a.ldb % 8) || (a.N % 8) || (a.ldc % (a.c_f32 ? 4 : 8))) return -2;
     if ((a.epi == EPI_SWIGLU || a.epi == EPI_CLAMP_GLU) && (a.N % 32)) return -3;
@@ -1276,19 +1277,32 @@ int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream) {
     if ((a.epi == EPI_BIAS || a.epi == EPI_BIAS_QUICKGELU || a.epi == EPI_BIAS_GELU ||
          a.epi == EPI_BIAS_RESIDUAL) && !a.bias) return -5;
     if (a.tile_group && a.groups < 1) return -1;
-    const bool plain = !a.tile_group && a.batch <= 1 && !a.c_f32;
     if (a.batch > 1 && (a.tile_group || (a.K % BLOCK_K) || (a.a_col_stride % 8) || (a.c_col_stride % 8) || a.a_col_stride < 0 || a.c_col_stride < 0)) return -7;
     if (a.c_f32 && (a.epi != EPI_NONE || (a.ldc % 4))) return -8;
+    return 0;
+}
+
+int gemm_bf16_tn_form(const GemmArgs& a, GemmForm form, int width, int splits, int num_sms, cudaStream_t stream) {
+    if (int r = check_args(a)) return r;
+    if (a.tile_group || a.batch > 1 || a.c_f32 || a.epi == EPI_SIGMOID_GATE || a.epi == EPI_PARTIAL_F32 || width < 32 || (width % 32)) return -6;
+    if (form == FORM_SWAP) {
+        if (width > kSwapMax || splits < 1 || splits > kSwapSplits) return -6;
+        return launch_epi_swap(a, width, splits, num_sms, stream);
+    }
+    if (width > 256) return -6;
+    return form == FORM_PAIR ? launch_epi2(a, width, num_sms, stream) : launch_epi(a, width, num_sms, stream);
+}
+
+int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream) {
+    if (int r = check_args(a)) return r;
+    const bool plain = !a.tile_group && a.batch <= 1 && !a.c_f32;
     static const int forced = [] { const char* e = getenv("LIVECC_B200_GEMM_BN"); return e ? atoi(e) : 0; }();  // tuning hook (0/unset = model)
     const bool choose = plain && a.block_n == 0 && forced <= 0 && a.epi != EPI_SIGMOID_GATE;
     int width = 0;
     if (choose) {
-        double us = 0., split_us = 0.;
-        width = choose_pair(a.M, a.N, a.K, num_sms, &us);
-        if (try_splitk(a, num_sms, stream, &split_us) > 0) us = split_us;
-        int bm = 0, splits = 0;
-        if (splitk_mode() != 1 && a.epi != EPI_PARTIAL_F32 && choose_swap(a.M, a.N, a.K, num_sms, us, &bm, &splits))
-            return launch_epi_swap(a, bm, splits, num_sms, stream);
+        const GemmPlan p = gemm_plan(a, num_sms);
+        if (p.form == FORM_SWAP) return launch_epi_swap(a, p.width, p.splits, num_sms, stream);
+        if (p.form == FORM_PAIR) width = p.width;
     }
     if (plain)
         if (int r = try_splitk(a, num_sms, stream)) return r < 0 ? r : 0;

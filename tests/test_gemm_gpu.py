@@ -1,5 +1,7 @@
 """tcgen05 GEMM core vs torch on the GPU: bit-exact on integer-valued operands (fp32 accumulation is
 exact there, so any descriptor/swizzle/tile bug shows as a hard mismatch), tolerance on random ones."""
+import math
+
 import pytest
 import torch
 
@@ -129,8 +131,9 @@ def test_gemm_default_kernel_equals_one_cta(ctx, M, N, K, epi):
 @pytest.mark.parametrize("M,N,K", [(1, 3584, 3584), (24, 4608, 3584), (33, 2080, 4104), (281, 3584, 3592), (288, 3584, 18944), (300, 37888, 512), (1000, 1280, 5120),
                                    (513, 3584, 4096)])
 def test_gemm_few_rows_every_epilogue(ctx, M, N, K, epi):
-    """Few rows run with the operands swapped, K split inside a cluster: equal to the one-CTA kernel on sums that fp32 holds exactly (so
-    the order of the splits cannot show); ragged rows, columns and k, one and two column groups."""
+    """Few rows, most of them with the operands swapped, K split inside a cluster: equal to the one-CTA kernel on sums that fp32 holds
+    exactly (so the order of the splits cannot show); ragged rows, columns and k. (The shapes that must take the swapped kernel, and its
+    forms one by one, are in the two tests behind this one.)"""
     a, b = _ints((M, K), -1, 1, 31), _ints((N, K), -1, 1, 32)
     kw = {}
     if epi in (A.EPI_BIAS, A.EPI_BIAS_QUICKGELU, A.EPI_BIAS_GELU, A.EPI_BIAS_RESIDUAL):
@@ -139,6 +142,54 @@ def test_gemm_few_rows_every_epilogue(ctx, M, N, K, epi):
         kw["residual"] = _ints((M, N), -8, 8, 34)
     # (activations: integers are exact before them; the fp32 math after the sum is the same code)
     assert torch.equal(ctx.gemm(a, b, epilogue=epi, **kw), ctx.gemm(a, b, epilogue=epi, block_n=128, **kw))
+
+
+@pytest.mark.parametrize("M,N,K", [(24, 4608, 3584), (281, 3584, 3584), (281, 3584, 18944), (256, 5120, 5120), (281, 37888, 3584)])
+def test_gemm_plan_takes_the_swapped_kernel(ctx, M, N, K):
+    """The shapes the rule was measured on take the swapped form, the last one with more tiles than clusters; sums held exactly."""
+    assert ctx.gemm_plan(M, N, K)[0] == 2
+    a, b = _ints((M, K), -1, 1, 41), _ints((N, K), -1, 1, 42)
+    assert torch.equal(ctx.gemm(a, b), ctx.gemm_form(a, b, 0, 128))
+
+
+# M, N, K, width, splits: one and two column groups (width up to and above 256), ragged rows, columns and k, more tiles than clusters (one
+# tile of rows and several), every split, the whole tile range of rows
+SWAP_FORMS = [(1, 288, 72, 32, 1), (33, 544, 200, 64, 1), (33, 544, 328, 64, 2), (97, 320, 1224, 128, 3), (128, 288, 520, 128, 4),
+              (250, 1056, 328, 256, 1), (281, 1312, 1224, 288, 2), (500, 544, 136, 512, 1), (300, 544, 392, 160, 2), (40, 20512, 200, 64, 1),
+              (281, 7712, 136, 96, 1), (290, 19232, 328, 320, 1)]
+
+
+@pytest.mark.parametrize("epi,limit", [(A.EPI_NONE, 0), (A.EPI_BIAS, 0), (A.EPI_BIAS_QUICKGELU, 0), (A.EPI_BIAS_GELU, 0), (A.EPI_RESIDUAL, 0), (A.EPI_BIAS_RESIDUAL, 0),
+                                       (A.EPI_SWIGLU, 0), (8, 0), (9, 0), (11, 0), (A.EPI_CLAMP_GLU, 7.0), (A.EPI_CLAMP_GLU, math.inf)])
+@pytest.mark.parametrize("M,N,K,width,splits", SWAP_FORMS)
+def test_gemm_swapped_form(ctx, M, N, K, width, splits, epi, limit):
+    """Every form of the swapped kernel equals the one-CTA kernel on sums that fp32 holds exactly, whatever the rule would choose."""
+    a, b = _ints((M, K), -1, 1, 43), _ints((N, K), -1, 1, 44)
+    kw = dict(epilogue=epi)
+    if epi in (A.EPI_BIAS, A.EPI_BIAS_QUICKGELU, A.EPI_BIAS_GELU, A.EPI_BIAS_RESIDUAL):
+        kw["bias"] = _ints((N,), -8, 8, 45)
+    if epi in (A.EPI_RESIDUAL, A.EPI_BIAS_RESIDUAL):
+        kw["residual"] = _ints((M, N), -8, 8, 46)
+    if epi == A.EPI_CLAMP_GLU:
+        kw.update(limit=limit, alpha=1.702 if limit < 8 else 1.0, up_bias=1.0 if limit < 8 else 0.0)
+    assert torch.equal(ctx.gemm_form(a, b, 2, width, splits, **kw), ctx.gemm_form(a, b, 0, 128, **kw))
+
+
+@pytest.mark.parametrize("form,width,splits", [(0, 96, 1), (1, 128, 1), (1, 224, 1), (2, 96, 2)])
+@pytest.mark.parametrize("limit", [7.0, math.inf])
+def test_gemm_clamped_glu(ctx, form, width, splits, limit):
+    """Epilogue 10 of each kernel against float64: gate and up rows interleaved by 16; one rounding to bf16 (2^-9) and fp32 sums before it."""
+    from livecc_b200.checkpoint import interleave_gate_up
+
+    g = torch.Generator(device="cuda").manual_seed(47)
+    M, F, K = 281, 656, 520
+    a = torch.randn((M, K), device="cuda", generator=g).to(torch.bfloat16)
+    wg, wu = ((torch.randn((F, K), device="cuda", generator=g) * 0.2).to(torch.bfloat16) for _ in range(2))
+    gate, up = (a.double() @ w.double().T for w in (wg, wu))
+    gate, up = gate.clamp(max=limit), up.clamp(-limit, limit)
+    ref = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+    out = ctx.gemm_form(a, interleave_gate_up(wg, wu), form, width, splits, epilogue=A.EPI_CLAMP_GLU, limit=limit)
+    assert ((out.double() - ref).norm() / ref.norm()).item() < 2.0 ** -9
 
 
 def test_gemm_strided_views(ctx):
