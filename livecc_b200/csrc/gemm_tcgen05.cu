@@ -1003,12 +1003,12 @@ static int launch_epi2(const GemmArgs& a, int bn, int num_sms, cudaStream_t stre
     return -14;
 }
 
-// Clusters of 2 * splits CTAs (one per SM) that the device holds at once; a hardware fact, asked once per device and size.
-static int max_clusters(int splits, int num_sms) {
+// Clusters of 2 * splits CTAs (one per SM) that the device holds at once, 0 when that cannot be asked; a hardware fact, kept per device and
+// size once it is known.
+static int max_clusters(int dev, int splits, int num_sms) {
     static std::atomic<int> known[64][kSwapSplits + 1];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    int n = known[dev][splits].load(std::memory_order_relaxed);
+    if (dev < 0) return 0;
+    int n = dev < 64 ? known[dev][splits].load(std::memory_order_relaxed) : 0;
     if (n) return n;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(num_sms / (2 * splits) * 2 * splits);
@@ -1020,16 +1020,25 @@ static int max_clusters(int splits, int num_sms) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (cudaFuncSetAttribute(gemm_swap_kernel<EPI_NONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, gemm_swap_kernel<EPI_NONE>, &cfg) != cudaSuccess || n < 1)
-        n = 1;
-    known[dev][splits].store(n, std::memory_order_relaxed);
+        cudaOccupancyMaxActiveClusters(&n, gemm_swap_kernel<EPI_NONE>, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();   // the question's error is not the caller's
+        return 0;
+    }
+    if (dev < 64) known[dev][splits].store(n, std::memory_order_relaxed);
     return n;
+}
+static int current_device() {
+    int dev = -1;
+    if (cudaGetDevice(&dev) == cudaSuccess) return dev;
+    cudaGetLastError();
+    return -1;
 }
 
 template <int EPI>
 static int launch_swap(const GemmArgs& a, int bm, int splits, int num_sms, cudaStream_t stream) {
     const int units = (a.M + bm - 1) / bm * ((a.N + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
-    const int clusters = std::min(units, max_clusters(splits, num_sms));
+    const int clusters = std::min(units, max_clusters(current_device(), splits, num_sms));
+    if (clusters < 1) return -15;
     const SwapTile cfg = make_swap(bm, splits);
     // a shared K range: every unit has its cluster, every pair a k-block, and the partial accumulators fit over the ring
     if (splits > 1 && (clusters < units || (a.K + BLOCK_K - 1) / BLOCK_K < splits || bm * BLOCK_M * 4 > cfg.stages * cfg.stage_bytes)) return -15;
@@ -1144,12 +1153,18 @@ static int choose_pair(int M, int N, int K, int num_sms, double* us) {
 static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_out, int* splits_out) {
     const int n_tiles = (N + 2 * BLOCK_M - 1) / (2 * BLOCK_M), nkb = (K + BLOCK_K - 1) / BLOCK_K;
     const int t0 = (M + kSwapMax - 1) / kSwapMax;
+    // (the fewest tiles there can be, against the most clusters and waves: most products of thousands of rows end here)
+    if ((long long)t0 * n_tiles > (long long)num_sms / 2 * (t0 == 1 ? 2 : 1)) return false;
+    const int dev = current_device();
+    int fit[kSwapSplits + 1];
+    for (int sp = 1; sp <= kSwapSplits; ++sp) fit[sp] = max_clusters(dev, sp, num_sms);
     double best = 0.95 * other;
     bool found = false;
     for (int tiles = t0; tiles <= 2 * t0 + 2; ++tiles) {
         const int bm = ((M + tiles - 1) / tiles + 31) / 32 * 32, m_tiles = (M + bm - 1) / bm, units = m_tiles * n_tiles;
         for (int sp = 1; sp <= kSwapSplits; ++sp) {
-            const int fit = max_clusters(sp, num_sms), waves = (units + fit - 1) / fit;
+            if (fit[sp] < 1) continue;
+            const int waves = (units + fit[sp] - 1) / fit[sp];
             if (waves > (sp == 1 && m_tiles == 1 ? 2 : 1) || nkb < 4 * sp) continue;
             const SwapTile t = make_swap(bm, sp);
             if (sp > 1 && bm * BLOCK_M * 4 > t.stages * t.stage_bytes) continue;

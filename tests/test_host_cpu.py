@@ -1,5 +1,6 @@
 """CPU suite, part 2: C-ABI exports, host orchestration (streaming mirror with a mock model, page pool,
 livecc_utils surface) and the world_size-2 gloo path of the multi-GPU runner. No GPU compute."""
+import ast
 import os
 import subprocess
 import sys
@@ -22,6 +23,18 @@ def test_library_loads_and_exports_every_header_symbol():
     for s in syms:
         assert hasattr(lib, s), f"liblivecc_sm100a.so does not export {s}"
     assert lib.lcc_abi_version() == _cabi.ABI_VERSION
+
+
+def test_gemm_plan_without_an_answer_about_clusters():
+    """Where the device cannot be asked how many clusters fit (here: none is there), no product takes the kernel that needs them, and the
+    others are planned as ever. In a process of its own: a division by that number would end it."""
+    code = ("from livecc_b200 import _cabi; import ctypes as C; lib = _cabi.load_library(); p = (C.c_int32 * 3)();"
+            "print([(lib.lcc_gemm_plan(148, m, n, k, p), *p) for m, n, k in [(24, 4608, 3584), (281, 3584, 3584), (2048, 10304, 2048)]])")
+    env = dict(os.environ, CUDA_VISIBLE_DEVICES="")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, cwd=ROOT)
+    assert r.returncode == 0, r.stderr
+    plans = ast.literal_eval(r.stdout)
+    assert [p[:2] for p in plans] == [(0, 0), (0, 0), (0, 1)] and plans[2][3] == 1
 
 
 def test_product_path_fails_loudly_without_a_gpu():
