@@ -212,13 +212,13 @@ WsLayout make_layout(const lcc_seq_model* m, int NT, int NW) {
     } while (0)
 
 // y[M, N] = x[M, K] W^T (+ bias). Large bf16 products with 8-aligned shapes run on the tensor cores; everything else on
-// the CUDA-core kernels. bias is fp32; the tensor-core epilogue takes a copy in the storage type (bias_st; without one a
-// biased product stays on the CUDA cores). A ragged N runs on the tensor cores when the matrix rows are padded to 8.
+// the CUDA-core kernels. bias is fp32; the tensor-core epilogue takes a copy in the storage type (bias_st; without one, or with
+// fewer than 16 rows, a biased product stays on the CUDA cores, which add the bias itself). A ragged N runs on the tensor cores when the matrix rows are padded to 8.
 int linear(const lcc_seq_model* m, const void* x, int ldx, const void* W, const float* bias, void* y, int ldy,
            bool y_f32, int M, int N, int K, cudaStream_t s, const void* bias_st = nullptr, int act = lcc::ACT_NONE) {
     const int Np = m->d.rows_padded8 ? ld8(N) : N;
     if (act != lcc::ACT_NONE && bias) return -2;
-    if (m->use_tc && m->d.dtype == LCC_DT_BF16 && (!y_f32 || (!bias && act == lcc::ACT_NONE)) && (!bias || bias_st) && M > 8 &&
+    if (m->use_tc && m->d.dtype == LCC_DT_BF16 && (!y_f32 || (!bias && act == lcc::ACT_NONE)) && (!bias || (bias_st && M >= 16)) && M > 8 &&
         (Np >= 32 || y_f32) && K >= 64 && (K % 8) == 0 && (Np % 8) == 0 && ldy >= Np && (ldx % 8) == 0 && (ldy % 8) == 0 &&
         ((uintptr_t)x % 16) == 0 && ((uintptr_t)y % 16) == 0) {   // (a slice of a wider row may start anywhere)
         lcc::GemmArgs a;

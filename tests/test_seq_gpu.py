@@ -98,6 +98,28 @@ def test_bf16_storage_stays_within_rounding_on_both_linear_paths(name, monkeypat
     assert rel(outs[0], outs[1].double()) < BF16_TOL
 
 
+@pytest.mark.parametrize("rows", [1, 8, 9, 12, 15])
+def test_few_rows_add_the_bias_in_fp32(rows):
+    """A bias of an fp32 checkpoint that bf16 cannot hold: 1 + 2^-8 beside a product of 2^-8 is 1 + 2^-7 after one rounding and 1 with the
+    bias rounded first. The embedding is zero, so the last channel of a row is its slowest cosine, 1 in bf16 for the first positions; the
+    value rows of the cache show the sum."""
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    d = seq_cases.config([seq_cases.par()], width=64)
+    cfg = SeqModelConfig.from_json(d)
+    t = {k: v.float() for k, v in synthetic_seq_tensors(cfg, seed=5).items()}
+    t["embed"].zero_()
+    t["l0.mix.left.v"].zero_()
+    t["l0.mix.left.v"][:, -1] = 2.0 ** -8
+    t["l0.mix.left.v.b"].fill_(1 + 2.0 ** -8)
+    m = SeqLMForCausalLM.from_state_dict(cfg, t, "bfloat16")
+    c = m.new_cache()
+    m.forward_step([(c, seq_cases.tokens(rows, d["vocab"]))], [[rows - 1]])
+    v = m.pool.v[0][c.pages[0]][:, :rows].float()
+    c.release()
+    assert bool((v == 1 + 2.0 ** -7).all()), v.unique()
+
+
 # ---- prefill against decoding, portions, first tokens ---------------------------------------------------------------------
 @pytest.mark.parametrize("name", ["ssd_only", "parallel_only", "mixed", "odd"])
 def test_token_by_token_decoding_equals_the_whole_prompt(name):
