@@ -220,7 +220,7 @@ int linear(const lcc_seq_model* m, const void* x, int ldx, const void* W, const 
     if (act != lcc::ACT_NONE && bias) return -2;
     if (m->use_tc && m->d.dtype == LCC_DT_BF16 && (!y_f32 || (!bias && act == lcc::ACT_NONE)) && (!bias || (bias_st && M >= 16)) && M > 8 &&
         (Np >= 32 || y_f32) && K >= 64 && (K % 8) == 0 && (Np % 8) == 0 && ldy >= Np && (ldx % 8) == 0 && (ldy % 8) == 0 &&
-        ((uintptr_t)x % 16) == 0 && ((uintptr_t)y % 16) == 0) {   // (a slice of a wider row may start anywhere)
+        ((uintptr_t)x % 16) == 0 && ((uintptr_t)y % 16) == 0 && ((uintptr_t)W % 16) == 0) {   // (a slice of a wider row, or a head, may start anywhere)
         lcc::GemmArgs a;
         a.c_f32 = y_f32;
         a.A = x; a.B = W; a.C = y; a.M = M; a.N = Np; a.K = K; a.lda = ldx; a.ldb = K; a.ldc = ldy;

@@ -120,6 +120,29 @@ def test_few_rows_add_the_bias_in_fp32(rows):
     assert bool((v == 1 + 2.0 ** -7).all()), v.unique()
 
 
+@pytest.mark.parametrize("want", [3, 12, 40])
+def test_a_head_at_any_address(want):
+    """The output head is read where it lies: a matrix that starts two bytes behind a 16-byte boundary serves any number of wanted rows."""
+    from livecc_b200.seq_engine import SeqLMForCausalLM, SeqWeights
+
+    d = seq_cases.config([seq_cases.par(ff=None)], width=64)
+    cfg = SeqModelConfig.from_json(d)
+    t = synthetic_seq_tensors(cfg, seed=6)
+    toks = seq_cases.tokens(40, d["vocab"])
+    out = []
+    for shift in (0, 1):
+        w = SeqWeights(cfg, t, torch.bfloat16, torch.device("cuda", torch.cuda.current_device()))
+        room = torch.empty(w.head.numel() + 8, dtype=torch.bfloat16, device="cuda")
+        head = room[shift:shift + w.head.numel()].view_as(w.head)
+        head.copy_(w.head)
+        w.head = head
+        m = SeqLMForCausalLM(cfg, w, torch.device("cuda", torch.cuda.current_device()))
+        c = m.new_cache()
+        out.append(m.forward_step([(c, toks)], [list(range(40 - want, 40))]).clone())
+        c.release()
+    assert rel(out[1], out[0].double().cpu()) < F32_TOL      # fp32 sums of the same bf16 products
+
+
 # ---- prefill against decoding, portions, first tokens ---------------------------------------------------------------------
 @pytest.mark.parametrize("name", ["ssd_only", "parallel_only", "mixed", "odd"])
 def test_token_by_token_decoding_equals_the_whole_prompt(name):
