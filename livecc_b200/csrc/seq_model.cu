@@ -211,6 +211,19 @@ WsLayout make_layout(const lcc_seq_model* m, int NT, int NW) {
         if (rc__) LCC_FAIL(m->ctx, rc__, "%s failed (code %d)", what, rc__);                  \
     } while (0)
 
+// Copies and clears between the kernels of a pass. The kernel behind one is launched in the ordinary way (launch.h: a chained kernel's
+// predecessor is a kernel).
+int copy_f32(float* dst, const float* src, size_t n, cudaStream_t s) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
+    lcc::chain_break();
+    return e == cudaSuccess ? 0 : -100;
+}
+int fill_i32(int* dst, int byte, size_t n, cudaStream_t s) {
+    const cudaError_t e = cudaMemsetAsync(dst, byte, n * sizeof(int), s);
+    lcc::chain_break();
+    return e == cudaSuccess ? 0 : -100;
+}
+
 // y[M, N] = x[M, K] W^T (+ bias). Large bf16 products with 8-aligned shapes run on the tensor cores; everything else on
 // the CUDA-core kernels. bias is fp32; the tensor-core epilogue takes a copy in the storage type (bias_st; without one, or with
 // fewer than 16 rows, a biased product stays on the CUDA cores, which add the bias itself). A ragged N runs on the tensor cores when the matrix rows are padded to 8.
@@ -858,9 +871,8 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
                 STEP(lcc::moe_route_small(logit, lde, l.e_correction_f32, EO, K, l.e_scale, sel, wsel, gate_out, row_off, posn,
                                           src_row, T, fs, &ro), "expert choice + row lists");
             } else {
-                if (cudaMemsetAsync(counts, 0, sizeof(int) * E, fs) != cudaSuccess) LCC_FAIL(m->ctx, -100, "router counters");
-                if (tc && cudaMemsetAsync(src_row, 0xff, sizeof(int) * (size_t)n_tiles * kMoeTile, fs) != cudaSuccess) LCC_FAIL(m->ctx, -100, "row lists");
-                lcc::chain_break();
+                STEP(fill_i32(counts, 0, E, fs), "router counters");
+                if (tc) STEP(fill_i32(src_row, 0xff, (size_t)n_tiles * kMoeTile, fs), "row lists");
                 STEP(lcc::moe_route(logit, lde, l.e_correction_f32, EO, K, l.e_scale, sel, wsel, gate_out, counts, rank, T, fs, &ro), "expert choice");
                 STEP(lcc::moe_index(sel, rank, counts, E, K, tc ? kMoeTile : 1, row_off, posn, src_row, tc ? tile_group : nullptr, n_tiles, T, fs), "expert row lists");
             }
@@ -942,16 +954,11 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
             else STEP(lcc::postnorm_residual(dt, x32, xa, par_is_mc ? nullptr : o1, W, nullptr, nullptr, 0, nullptr, l.norm2_f32, d.alpha, d.eps, T, W, s,
                                              l.ls2_f32, par_is_mc ? &par_mc : nullptr), "norm2");
         }
-        if (layer_dump && !hc) {
-            if (cudaMemcpyAsync(layer_dump + (size_t)li * T * W, x32, (size_t)T * W * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-                LCC_FAIL(m->ctx, -100, "layer dump copy failed");
-            lcc::chain_break();
-        }
+        if (layer_dump && !hc) STEP(copy_f32(layer_dump + (size_t)li * T * W, x32, (size_t)T * W, s), "layer dump copy");
     }
     if (hc) {
         STEP(boundary(nullptr, nullptr, xsum), "stream sum");
-        if (layer_dump && cudaMemcpyAsync(layer_dump + (size_t)(d.n_layers - 1) * T * W, xsum, (size_t)T * W * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-            LCC_FAIL(m->ctx, -100, "layer dump copy failed");
+        if (layer_dump) STEP(copy_f32(layer_dump + (size_t)(d.n_layers - 1) * T * W, xsum, (size_t)T * W, s), "layer dump copy");
     }
     if (n_want > 0) {
         const lcc::NormSpec fn{d.norm_kind, d.final_norm_f32, d.final_norm_bias_f32, d.final_norm_alpha, d.eps};
@@ -960,9 +967,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
         // as CUDA-core tiles; decode steps (up to 8 rows) keep the weight-streaming kernel, which `linear` falls back to.
         STEP(linear(m, xf, W, d.head, nullptr, logits, d.vocab, true, n_want, d.vocab, W, s), "output head");
         STEP(lcc::softcap(logits, (int64_t)n_want * d.vocab, d.logit_softcap, s, d.logit_scale != 0.f ? d.logit_scale : 1.f), "logit soft cap / scale");
-        if (logits_copy &&
-            cudaMemcpyAsync(logits_copy, logits, (size_t)n_want * d.vocab * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-            LCC_FAIL(m->ctx, -100, "logits copy failed");
+        if (logits_copy) STEP(copy_f32(logits_copy, logits, (size_t)n_want * d.vocab, s), "logits copy");
     }
     LCC_CHECK_LAUNCH(m->ctx, "lcc_seq_forward");
     return 0;

@@ -71,3 +71,24 @@ def test_explicit_non_coherent_loads_are_of_weights(name):
     allowed = {"linear_any": ["W + (size_t)wrow(r) * ldw + k"], "attn_local": ["row + min(dist, len - 1)"]}   # weights; the distance table
     loads = [a for a in re.findall(r"(?:ld_stream16|__ldg)\(((?:[^()]|\([^()]*\))*)\)", src)]
     assert [a for a in loads if a not in allowed.get(name, [])] == []
+
+
+def test_the_kernel_behind_a_copy_a_clear_a_fork_or_a_join_is_not_chained():
+    """lcc_seq_forward copies and clears through helpers that break the chain; a fork's or a join's wait on another stream's event is followed
+    by a break before anything is launched."""
+    src = re.sub(r"//[^\n]*", "", (CSRC / "seq_model.cu").read_text())
+    for helper in re.findall(r"\n(?:int|void) \w+\([^)]*cudaStream_t s\) \{[^{}]*cudaMem(?:cpy|set)Async[^{}]*\}", src):
+        assert helper.index("Async") < helper.index("chain_break()")
+    forward = src[src.index("int lcc_seq_forward("):]
+    assert not re.search(r"cudaMem(?:cpy|set)\w*\(", forward)
+    waits = [w for w in re.finditer(r"cudaStreamWaitEvent\((\S+), m->(ev_\w+), 0\)", forward)]
+    assert len(waits) == 4
+    for w in waits:
+        rest = forward[w.end():]
+        # the branch that forks from the main stream goes on there (same predecessor kernel); its first launch on the side stream follows a break
+        stop = rest.index("chain_break()")
+        between = rest[:stop]
+        if w.group(2) == "ev_join" or "fork_ff" not in forward[max(0, w.start() - 120):w.start()]:
+            assert "STEP(" not in between, w.group(0)
+        else:
+            assert not re.search(r"STEP\([^;]*\bfs\b", between), w.group(0)
