@@ -402,8 +402,9 @@ __global__ void __launch_bounds__(256) attn_rows_kernel(const float* __restrict_
         if (warp < HB) {
             if (warp < nh) {
                 const float sv = sc[warp * kRowKeys + lane];
-                const float mn = fmaxf(m, warp_max(sv));          // the tile holds a key: finite
-                const float corr = expf(m - mn), p = expf(sv - mn);   // exp(-inf) = 0 on the first tile and on absent keys
+                const float mn = fmaxf(m, warp_max(sv));
+                const float at = mn == -INFINITY ? 0.f : mn;      // so far a distance table hides every key: no weight, and no -inf - -inf
+                const float corr = expf(m - at), p = expf(sv - at);   // exp(-inf) = 0 on the first tile and on absent keys
                 l = fmaf(l, corr, warp_sum(p));
                 m = mn;
                 pw[lane * HB + warp] = p;
@@ -489,7 +490,7 @@ __global__ void __launch_bounds__(256) attn_rows_kernel(const float* __restrict_
         const float sk = opt.no_sink ? -INFINITY : (sink ? sink[h0 + warp] : 0.f);
         float mt = sk;
         for (int i = lane; i < nz; i += 32) mt = fmaxf(mt, wm[i * HB + warp]);
-        mt = warp_max(mt);                        // split 0 holds the row's first key: finite
+        mt = warp_max(mt);                        // the row sees itself: finite unless its own key is hidden too
         float lt = 0.f;
         for (int i = lane; i < nz; i += 32) {
             const float w = expf(wm[i * HB + warp] - mt);

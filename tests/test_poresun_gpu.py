@@ -96,6 +96,19 @@ def routed(d):
     return any(L["mlp"] and L["mlp"]["kind"] == "moe" for L in d["layers"])
 
 
+@pytest.mark.parametrize("portion", [1, 8, 15])
+def test_distances_hidden_by_the_table(portion):
+    """A distance table may hide everything beyond some distance with -inf: whole tiles of keys then have no weight, in portions and steps."""
+    d = K.config([K.att(heads=2, kv_heads=1, dim=8, vdim=8, window=0, cap=0.0, far=20, rows=16, mlp=None),
+                  K.att(heads=4, kv_heads=2, dim=8, vdim=16, window=0, cap=3.0, far=30, rows=12, mlp=None)], width=16)
+    tensors = make(d)
+    for i, b in ((0, 10), (1, 8)):
+        tensors[f"l{i}.mix.rel"][b:] = -torch.inf
+    toks = K.tokens(120, d["vocab"])
+    want, _ = O.forward(d, tensors, toks, layer_outputs=True)
+    assert rel(run(build(d, tensors), toks, range(portion, 120, portion)), want) < F32_TOL
+
+
 # ---- every mechanism alone, and together, against the oracle ------------------------------------------------------------
 @pytest.mark.parametrize("name", ALL)
 def test_whole_prompt_every_layer_matches_the_oracle_fp32(name):
