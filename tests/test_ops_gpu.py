@@ -354,7 +354,7 @@ def test_sample_greedy(ctx):
         bad = (proc != ref).nonzero().flatten()
         print("penalty mismatches vs torch:", bad.numel(), "vs true division:", int((proc != ref_div).sum()),
               [(int(i), float(raw[i]), float(proc[i]), float(ref[i])) for i in bad[:4]])
-    assert torch.equal(proc, ref)  # bit-exact with torch's CUDA semantics (tools/penalty_probe.py)
+    assert torch.equal(proc, ref)  # bit-exact with torch's CUDA semantics
     assert int(seq[5000]) == tok and torch.equal(h, embed[tok])
     assert sc.tolist()[:6] == [5001, 4001, 0, 1, 5001, tok]
     # threshold processor: force -inf on the would-be argmax token
