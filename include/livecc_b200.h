@@ -67,6 +67,9 @@ lcc_ctx* lcc_create(int device);
 void lcc_destroy(lcc_ctx* ctx);
 const char* lcc_last_error(lcc_ctx* ctx);
 int lcc_num_sms(lcc_ctx* ctx);
+/* Non-zero once a bounded wait inside one of the context's matrix products has given up (a signal that never came): the product holds NaN,
+ * later calls of the context fail. To be asked behind a synchronisation. */
+int lcc_check_fault(lcc_ctx* ctx);
 /* Kernel launches issued by this library in this process so far (launches recorded into a CUDA graph count once,
  * at capture). */
 uint64_t lcc_launch_count(void);
@@ -90,10 +93,10 @@ int lcc_gemm_bf16(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, 
 int lcc_gemm_plan(int num_sms, int M, int N, int K, int32_t* plan);
 /* lcc_gemm_bf16 with one explicit kernel (form, width and splits as in lcc_gemm_plan; any epilogue but the per-head gate), for tests and
  * tuning. limit, alpha and up_bias: epilogue 10, gate and up rows interleaved by 16 as for LCC_EPI_SWIGLU:
- * g = min(gate, limit), u = clamp(up, +-limit), C = g * sigmoid(alpha * g) * (u + up_bias). */
+ * g = min(gate, limit), u = clamp(up, +-limit), C = g * sigmoid(alpha * g) * (u + up_bias). wait_ns: limit of a wait inside kernel 2, 0 = 2 s. */
 int lcc_gemm_form(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K, const void* bias,
                   const void* residual, int ldr, int epilogue, int form, int width, int splits, float limit, float alpha, float up_bias,
-                  lcc_stream_t stream);
+                  int64_t wait_ns, lcc_stream_t stream);
 
 /* hidden_states.to(bf16) of the f32 patch rows (mq2vl.py:309). */
 int lcc_cast_f32_bf16(lcc_ctx* ctx, const float* in, void* out, int64_t n, lcc_stream_t stream);

@@ -266,6 +266,10 @@ class Context:
             msg = self.lib.lcc_last_error(C.c_void_p(self.handle)).decode()
             raise LiveCCNativeError(f"{what} failed ({rc}): {msg}")
 
+    def check_fault(self):
+        """Raises if a matrix product of this context gave up on a signal (asked behind a synchronisation)."""
+        self.check(self.lib.lcc_check_fault(C.c_void_p(self.handle)), "lcc_check_fault")
+
     def call(self, name: str, *args):
         rc = getattr(self.lib, name)(C.c_void_p(self.handle), *args)
         self.check(rc, name)
@@ -302,7 +306,7 @@ class Context:
         self.check(self.lib.lcc_gemm_plan(self.num_sms, int(M), int(N), int(K), plan), "lcc_gemm_plan")
         return tuple(plan)
 
-    def gemm_form(self, a, b, form, width, splits=1, bias=None, residual=None, epilogue=EPI_NONE, limit=0.0, alpha=1.702, up_bias=1.0, out=None):
+    def gemm_form(self, a, b, form, width, splits=1, bias=None, residual=None, epilogue=EPI_NONE, limit=0.0, alpha=1.702, up_bias=1.0, wait_ns=0, out=None):
         """gemm() by one explicit kernel (tests and tuning); epilogue 10 is the clamped gated activation."""
         import torch
 
@@ -311,7 +315,7 @@ class Context:
             out = torch.empty((M, N // 2 if epilogue in (EPI_SWIGLU, EPI_CLAMP_GLU) else N), dtype=torch.bfloat16, device=a.device)
         self.call("lcc_gemm_form", _ptr(a), _i(a.stride(0)), _ptr(b), _i(b.stride(0)), _ptr(out), _i(out.stride(0)), _i(M), _i(N), _i(K),
                   _ptr(bias), _ptr(residual), _i(residual.stride(0) if residual is not None else 0), _i(epilogue), _i(form), _i(width),
-                  _i(splits), C.c_float(limit), C.c_float(alpha), C.c_float(up_bias), self.stream_ptr())
+                  _i(splits), C.c_float(limit), C.c_float(alpha), C.c_float(up_bias), C.c_int64(wait_ns), self.stream_ptr())
         return out
 
     def cast_f32_bf16(self, x):

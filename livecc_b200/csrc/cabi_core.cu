@@ -23,10 +23,26 @@ lcc_ctx* lcc_create(int device) {
     c->device = device;
     c->num_sms = prop.multiProcessorCount;
     c->err[0] = 0;
+    c->fault = nullptr;
+    if (cudaHostAlloc((void**)&c->fault, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        delete c;
+        return nullptr;
+    }
+    *c->fault = 0;
     return c;
 }
 
-void lcc_destroy(lcc_ctx* ctx) { delete ctx; }
+void lcc_destroy(lcc_ctx* ctx) {
+    if (!ctx) return;
+    cudaFreeHost(ctx->fault);
+    delete ctx;
+}
+
+int lcc_check_fault(lcc_ctx* ctx) {
+    if (!ctx) return -1;
+    LCC_CHECK_FAULT(ctx, "lcc_check_fault");
+    return 0;
+}
 
 const char* lcc_last_error(lcc_ctx* ctx) { return ctx ? ctx->err : "null ctx"; }
 
@@ -45,9 +61,10 @@ int lcc_gemm_bf16(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, 
     a.M = M; a.N = N; a.K = K;
     a.lda = lda; a.ldb = ldb; a.ldc = ldc;
     a.bias = bias; a.residual = residual; a.ldr = ldr;
-    a.epi = epilogue; a.block_n = block_n;
+    a.epi = epilogue; a.block_n = block_n; a.fault = ctx->fault;
     int r = lcc::gemm_bf16_tn(a, ctx->num_sms, (cudaStream_t)stream);
     if (r) LCC_FAIL(ctx, r, "lcc_gemm_bf16 failed (code %d; M=%d N=%d K=%d epi=%d)", r, M, N, K, epilogue);
+    LCC_CHECK_FAULT(ctx, "lcc_gemm_bf16");
     return 0;
 }
 
@@ -63,9 +80,10 @@ int lcc_gemm_plan(int num_sms, int M, int N, int K, int32_t* plan) {
 
 int lcc_gemm_form(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, void* C, int ldc, int M, int N, int K, const void* bias,
                   const void* residual, int ldr, int epilogue, int form, int width, int splits, float limit, float alpha, float up_bias,
-                  lcc_stream_t stream) {
-    if (!ctx) return -1;
+                  int64_t wait_ns, lcc_stream_t stream) {
+    if (!ctx || wait_ns < 0) return -1;
     lcc::GemmArgs a{};
+    a.fault = ctx->fault; a.wait_ns = (uint64_t)wait_ns;
     a.A = A; a.B = B; a.C = C;
     a.M = M; a.N = N; a.K = K;
     a.lda = lda; a.ldb = ldb; a.ldc = ldc;
@@ -73,6 +91,7 @@ int lcc_gemm_form(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, 
     a.epi = epilogue; a.epi_param = limit; a.epi_alpha = alpha; a.epi_up_bias = up_bias;
     int r = form < lcc::FORM_ONE || form > lcc::FORM_SWAP ? -6 : lcc::gemm_bf16_tn_form(a, (lcc::GemmForm)form, width, splits, ctx->num_sms, (cudaStream_t)stream);
     if (r) LCC_FAIL(ctx, r, "lcc_gemm_form failed (code %d; M=%d N=%d K=%d epi=%d form=%d width=%d splits=%d)", r, M, N, K, epilogue, form, width, splits);
+    LCC_CHECK_FAULT(ctx, "lcc_gemm_form");
     return 0;
 }
 

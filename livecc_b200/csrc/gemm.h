@@ -55,6 +55,9 @@ struct GemmArgs {
     bool c_f32 = false;
     float epi_param = 0.f;   // EPI_CLAMP_GLU: the clamp
     float epi_alpha = 1.702f, epi_up_bias = 1.f;
+    // kernels with bounded waits (the swapped form): a host-visible word that they set when a signal did not come, or null; the limit in ns, 0 = 2 s
+    int* fault = nullptr;
+    uint64_t wait_ns = 0;
 };
 
 int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream);

@@ -568,26 +568,60 @@ static SwapTile make_swap(int bm, int splits) {
     return t;
 }
 
-// Bounded mbarrier wait (2 s): a signal that never comes raises the CTA's flag, every later wait gives up at its first look at it, and the
-// epilogue stores NaN, so that the kernel ends and the result shows it.
-__device__ __forceinline__ void mbar_wait_or(uint64_t* bar, uint32_t parity, volatile int* gave_up) {
-    unsigned long long t0 = 0, now;
-    for (int it = 0;; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred P1;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, P1;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (ok) return;
-        if ((it & 0x3ff) != 0x3ff) continue;
-        if (*gave_up) return;
+// Bounded waits. When a signal of the swapped kernel does not come in time, the thread that waits raises the flag of every CTA of its
+// cluster and the library's fault word. Every wait that has to wait sees the flag and gives up too; nothing more is loaded or multiplied; the
+// epilogue writes NaN over every value that it did not see completed (with a split K: of every value of the cluster, whose shares are
+// all in it); copies and products under way get a limited time to end; then tensor memory is freed and the kernel returns.
+constexpr unsigned long long kWaitNs = 2000000000ull, kDrainNs = 20000000ull;
+struct GiveUp {
+    volatile int* flag;           // in this CTA's shared memory
+    int ctas;                     // of the cluster
+    unsigned long long ns;        // limit of a wait
+    int* fault;                   // host-visible word, or null
+};
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity, uint32_t hint_ns) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred P1;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, P1;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(hint_ns)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, const GiveUp& g) {
+    // (without the hint a try may sleep for longer than a whole product; products of 24 to 1024 rows take 3 to 6 % less time with it and
+    // one lane issuing the products: 281 x 3584 x 18944 50.7 -> 47.5 us)
+    if (mbar_try(bar, parity, 1000u)) return true;
+    unsigned long long t0, now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for (;;) {
+        if (mbar_try(bar, parity, 1000u)) return true;
+        if (*g.flag) return false;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-        if (t0 == 0) t0 = now;
-        else if (now - t0 > 2000000000ull) { *gave_up = 1; return; }
+        if (now - t0 <= g.ns) continue;
+        for (int c = 0; c < g.ctas; ++c)
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapa_shared(smem_u32(const_cast<const int*>(g.flag)), c)), "r"(1) : "memory");
+        if (g.fault) {
+            *reinterpret_cast<volatile int*>(g.fault) = 1;
+            __threadfence_system();
+        }
+        return false;
     }
+}
+// the same for a whole warp: all lanes or none
+__device__ __forceinline__ bool warp_wait_for(uint64_t* bar, uint32_t parity, const GiveUp& g) {
+    return __all_sync(0xffffffffu, mbar_wait_for(bar, parity, g));
+}
+// what is under way ends, or its time does; the flag does not cut it short
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+    unsigned long long t0, now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    do {
+        if (mbar_try(bar, parity, 1000u)) return;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    } while (now - t0 <= kDrainNs);
 }
 
 __device__ __forceinline__ float ld_cluster_addr_f32(uint32_t cluster_addr) {
@@ -679,7 +713,8 @@ template <int EPI>
 __global__ void __launch_bounds__(384, 1)
 gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x1,
                  const __grid_constant__ CUtensorMap tmap_x2, bf16* C, int M, int N, int K, int ldc, const bf16* __restrict__ bias,
-                 const bf16* residual /* may alias C */, int ldr, const SwapTile cfg, float limit, float alpha, float up_bias) {
+                 const bf16* residual /* may alias C */, int ldr, const SwapTile cfg, float limit, float alpha, float up_bias,
+                 unsigned long long wait_ns, int* fault) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int STAGES = cfg.stages, STAGE_BYTES = cfg.stage_bytes, S = cfg.splits;
@@ -687,8 +722,9 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     uint64_t* empty_bar = full_bar + MAX_STAGES;
     uint64_t* tmem_full = empty_bar + MAX_STAGES;
     uint64_t* tmem_empty = tmem_full + 1;
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty + 1);
-    volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_holder + 1);
+    uint64_t* drained = tmem_empty + 1;
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(drained + 1);
+    const GiveUp g{reinterpret_cast<volatile int*>(tmem_holder + 1), 2 * S, wait_ns, fault};
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t crank = cluster_ctarank();
@@ -714,7 +750,8 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
         mbar_init(tmem_full, 1);    // one multicast commit
         mbar_init(tmem_empty, 16);  // used in the leader: 8 epilogue warps of each CTA
-        *gave_up = 0;
+        mbar_init(drained, 1);      // the leader's last commit
+        *g.flag = 0;
         fence_barrier_init();
     }
     if (warp == 2) {
@@ -730,12 +767,14 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     if (warp == 0) {
         // ===================== TMA producer (both CTAs) =====================
         if (lane == 0) {
-            int stage = 0;
+            int stage = 0, issued = 0;
             uint32_t phase = 0;
-            for (int unit = cluster; unit < units; unit += num_clusters) {
+            bool ok = true;
+            for (int unit = cluster; ok && unit < units; unit += num_clusters) {
                 const int m0 = (unit % m_tiles) * cfg.bm, n0 = (unit / m_tiles) * 2 * BLOCK_M;
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    mbar_wait_or(&empty_bar[stage], phase ^ 1, gave_up);
+                    ok = mbar_wait_for(&empty_bar[stage], phase ^ 1, g);
+                    if (!ok) break;
                     uint8_t* sw = smem + stage * STAGE_BYTES;
                     uint8_t* sx = sw + A_BYTES;
                     if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * STAGE_BYTES);
@@ -745,40 +784,51 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     if (cfg.n2)
                         tma_load_2d_cg2(sx + cfg.n1 / 2 * BLOCK_K * 2, &tmap_x2, bar, kb * BLOCK_K, m0 + cfg.n1 + rank * (cfg.n2 / 2));
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                    ++issued;
                 }
             }
+            // no CTA leaves while copies into it are under way: the leader's barriers count those of both CTAs
+            for (int i = max(0, issued - STAGES); leader && i < issued; ++i) {
+                const uint32_t p = (i / STAGES) & 1;
+                if (!mbar_wait_for(&full_bar[i % STAGES], p, g)) mbar_drain(&full_bar[i % STAGES], p);
+            }
+            if (!ok) __nanosleep(1000000);   // (one CTA may have issued a few more than the other)
         }
     } else if (warp == 1) {
-        // ===================== MMA issuer (leader CTA only) =====================
-        if (leader) {
+        // ===================== MMA issuer (one lane of the leader CTA) =====================
+        if (leader && lane == 0) {
             int stage = 0;
             uint32_t phase = 0, acc_phase = 0;
             const uint16_t both = (uint16_t)(3u << lead);
+            bool ok = true;
             for (int unit = cluster; unit < units; unit += num_clusters) {
-                mbar_wait_or(tmem_empty, acc_phase ^ 1, gave_up);
+                ok = mbar_wait_for(tmem_empty, acc_phase ^ 1, g);
+                if (!ok) break;
                 tc_fence_after();
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    mbar_wait_or(&full_bar[stage], phase, gave_up);
+                    ok = mbar_wait_for(&full_bar[stage], phase, g);
+                    if (!ok) break;
                     tc_fence_after();
-                    if (lane == 0) {
-                        const uint32_t sw = smem_u32(smem + stage * STAGE_BYTES);
-                        const uint64_t dw = make_sw128_kmajor_desc(sw);
-                        const uint64_t dx = make_sw128_kmajor_desc(sw + A_BYTES);
-                        const uint64_t dx2 = make_sw128_kmajor_desc(sw + A_BYTES + cfg.n1 / 2 * BLOCK_K * 2);
+                    const uint32_t sw = smem_u32(smem + stage * STAGE_BYTES);
+                    const uint64_t dw = make_sw128_kmajor_desc(sw);
+                    const uint64_t dx = make_sw128_kmajor_desc(sw + A_BYTES);
+                    const uint64_t dx2 = make_sw128_kmajor_desc(sw + A_BYTES + cfg.n1 / 2 * BLOCK_K * 2);
 #pragma unroll
-                        for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-                            const uint32_t add = ((kb - kb0) | k) != 0 ? 1u : 0u;
-                            umma_bf16_ss_cg2(tmem_base, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), cfg.idesc1, add);
-                            if (cfg.n2) umma_bf16_ss_cg2(tmem_base + cfg.n1, dw + (uint64_t)(k * 2), dx2 + (uint64_t)(k * 2), cfg.idesc2, add);
-                        }
-                        umma_commit_cg2(&empty_bar[stage], both);  // frees the slot in both CTAs when the MMAs retire
-                        if (kb == kb1 - 1) umma_commit_cg2(tmem_full, both);
+                    for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                        const uint32_t add = ((kb - kb0) | k) != 0 ? 1u : 0u;
+                        umma_bf16_ss_cg2(tmem_base, dw + (uint64_t)(k * 2), dx + (uint64_t)(k * 2), cfg.idesc1, add);
+                        if (cfg.n2) umma_bf16_ss_cg2(tmem_base + cfg.n1, dw + (uint64_t)(k * 2), dx2 + (uint64_t)(k * 2), cfg.idesc2, add);
                     }
-                    __syncwarp();
+                    umma_commit_cg2(&empty_bar[stage], both);  // frees the slot in both CTAs when the MMAs retire
+                    if (kb == kb1 - 1) umma_commit_cg2(tmem_full, both);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
+                if (!ok) break;
                 acc_phase ^= 1;
             }
+            // the products read both CTAs' shared memory and write both halves of tensor memory: they end before either CTA leaves
+            umma_commit_cg2(drained, (uint16_t)(1u << lead));
+            if (!mbar_wait_for(drained, 0, g)) mbar_drain(drained, 0);
         }
     } else if (warp >= 4) {
         // ===================== Epilogue (both CTAs, own 128 weight rows) =====================
@@ -804,7 +854,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             int c = 0;
             while (c < chunks && !mine(c)) ++c;
             if (SwapEpi<EPI>::kResidual && c < chunks) fetch(c);
-            mbar_wait_or(tmem_full, acc_phase, gave_up);
+            bool lost = !warp_wait_for(tmem_full, acc_phase, g);
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
             float* red = reinterpret_cast<float*>(smem) + q * 32 + lane;   // [chunk][32 columns][128 weight rows]: over the drained ring
@@ -819,6 +869,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 }
                 __syncwarp();
                 cluster_sync_all();
+                lost = __any_sync(0xffffffffu, lost || *g.flag);   // a share of any pair of the cluster is missing
             }
             while (c < chunks) {
                 int next = c + 1;
@@ -847,12 +898,15 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     for (int k = 0; k < 8; ++k) now[k] = res[k];
                     if (next < chunks) fetch(next);
                 }
-                if (*gave_up) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) x[j] = __int_as_float(0x7fc00000);
-                }
                 swap_store<EPI>(x, C, ldc, M, N, m0 + c * 32, n, lane, b, now, limit, alpha, up_bias);
                 c = next;
+            }
+            if (lost) {   // (behind the stores: a test per value inside them costs 3 to 5 % of a product)
+                __syncwarp();
+                const int col = SwapEpi<EPI>::kGlu ? ((n >> 5) << 4) + (lane & 15) : n;
+                for (int d = 0; d < chunks; ++d)
+                    for (int j = 0; mine(d) && j < 32; ++j)
+                        if (m0 + d * 32 + j < M && n < N) C[(size_t)(m0 + d * 32 + j) * ldc + col] = __ushort_as_bfloat16(0x7fff);
             }
             tc_fence_before();
             __syncwarp();
@@ -1061,7 +1115,7 @@ static int launch_swap(const GemmArgs& a, int bm, int splits, int num_sms, cudaS
     lc.numAttrs = 1;
     lcc::count_launch();
     return cudaLaunchKernelEx(&lc, kern, tw, t1, t2, (bf16*)a.C, a.M, a.N, a.K, a.ldc, (const bf16*)a.bias, (const bf16*)a.residual, a.ldr, cfg,
-                              a.epi_param, a.epi_alpha, a.epi_up_bias) == cudaSuccess ? 0 : -13;
+                              a.epi_param, a.epi_alpha, a.epi_up_bias, a.wait_ns ? (unsigned long long)a.wait_ns : kWaitNs, a.fault) == cudaSuccess ? 0 : -13;
 }
 
 static int launch_epi_swap(const GemmArgs& a, int bm, int splits, int num_sms, cudaStream_t stream) {

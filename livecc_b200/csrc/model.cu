@@ -109,6 +109,7 @@ int gemm(lcc_model* m, const void* A, int lda, const void* B, int ldb, void* C, 
     lcc::GemmArgs a;
     a.A = A; a.B = B; a.C = C; a.M = M; a.N = N; a.K = K; a.lda = lda; a.ldb = ldb; a.ldc = ldc;
     a.bias = bias; a.residual = res; a.ldr = ldr; a.epi = epi; a.block_n = 0;
+    a.fault = m->ctx->fault;
     a.splitk_ws = splitk_ws; a.splitk_ws_bytes = splitk_ws_bytes;  // used only with LIVECC_B200_GEMM_SPLITK=1
     return lcc::gemm_bf16_tn(a, m->ctx->num_sms, s);
 }

@@ -235,6 +235,7 @@ int linear(const lcc_seq_model* m, const void* x, int ldx, const void* W, const 
         (Np >= 32 || y_f32) && K >= 64 && (K % 8) == 0 && (Np % 8) == 0 && ldy >= Np && (ldx % 8) == 0 && (ldy % 8) == 0 &&
         ((uintptr_t)x % 16) == 0 && ((uintptr_t)y % 16) == 0 && ((uintptr_t)W % 16) == 0) {   // (a slice of a wider row, or a head, may start anywhere)
         lcc::GemmArgs a;
+        a.fault = m->ctx->fault;
         a.c_f32 = y_f32;
         a.A = x; a.B = W; a.C = y; a.M = M; a.N = Np; a.K = K; a.lda = ldx; a.ldb = K; a.ldc = ldy;
         a.bias = bias ? bias_st : nullptr; a.residual = nullptr; a.ldr = 0; a.block_n = 0;
@@ -260,6 +261,7 @@ int linear_heads(const lcc_seq_model* m, const void* x, int ldx, int a_stride, c
     if (m->use_tc && m->d.dtype == LCC_DT_BF16 && M >= 16 && N >= 32 && (K % 64) == 0 && (N % 8) == 0 && (ldx % 8) == 0 &&
         (ldy % 8) == 0 && (a_stride % 8) == 0 && (c_stride % 8) == 0 && (!gate || (!y_f32 && (ld_gate % 8) == 0 && ((uintptr_t)gate % 16) == 0))) {
         lcc::GemmArgs a;
+        a.fault = m->ctx->fault;
         a.A = x; a.B = W; a.C = y; a.M = M; a.N = N; a.K = K; a.lda = ldx; a.ldb = K; a.ldc = ldy;
         a.bias = nullptr; a.residual = nullptr; a.ldr = 0; a.epi = lcc::EPI_NONE; a.block_n = 0;
         a.batch = heads; a.a_col_stride = a_stride; a.c_col_stride = c_stride; a.c_f32 = y_f32;
@@ -283,6 +285,7 @@ int linear_clamp_glu(const lcc_seq_model* m, const void* x, int ldx, const void*
                     (ldh % 8) == 0 && (ldr % 8) == 0;
     if (tc) {
         lcc::GemmArgs a;
+        a.fault = m->ctx->fault;
         a.A = x; a.B = W; a.C = il16 ? h : raw; a.M = M; a.N = 2 * F; a.K = K; a.lda = ldx; a.ldb = K; a.ldc = il16 ? ldh : ldr;
         a.bias = nullptr; a.residual = nullptr; a.ldr = 0; a.block_n = 0;
         a.epi = il16 ? lcc::EPI_CLAMP_GLU : lcc::EPI_NONE;
@@ -879,6 +882,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
             if (tc) {
                 STEP(lcc::moe_gather_rows(dt, xa, W, src_row, ex, ldw8, n_tiles * kMoeTile, W, fs), "expert row gather");
                 lcc::GemmArgs a;
+                a.fault = m->ctx->fault;
                 // gated experts with interleaved rows: the activation is the up product's epilogue and the hidden rows land in eg
                 const bool epi_glu = glu && l.e_up_il16;
                 a.A = ex; a.B = l.e_up; a.C = epi_glu ? eg : eh; a.M = n_tiles * kMoeTile; a.N = NH; a.K = W; a.lda = ldw8; a.ldb = W;

@@ -527,6 +527,7 @@ class LiveCCB200ForConditionalGeneration:
 
     def _finish_stream(self, rec, sc, logits_out, logits_hist, output_logits) -> GenerateOutput:
         cache, L, past = rec["cache"], rec["L"], rec["past"]
+        self.ctx.check_fault()
         if sc[_cabi.SC_NATIVE_ERROR]:
             raise _cabi.LiveCCNativeError(f"persistent decode kernel gave up on a bounded wait (code "
                                           f"{sc[_cabi.SC_NATIVE_ERROR]}); the results of this call are invalid")

@@ -660,6 +660,7 @@ class SeqLMForCausalLM:
             self._run_decode(cache, raw, sp, n_steps, hist)
         ev[2].record()
         sc = cache.scalars.tolist()                      # the one host sync of the decode phase
+        self.ctx.check_fault()
         n_gen = sc[_cabi.SC_N_GENERATED]
         # the device advanced the position; pages behind the last chunk go back as in a teacher-forced step
         cache.seq_len = L

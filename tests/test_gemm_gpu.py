@@ -175,6 +175,32 @@ def test_gemm_swapped_form(ctx, M, N, K, width, splits, epi, limit):
     assert torch.equal(ctx.gemm_form(a, b, 2, width, splits, **kw), ctx.gemm_form(a, b, 0, 128, **kw))
 
 
+@pytest.mark.parametrize("splits", [1, 2, 3])
+@pytest.mark.parametrize("epi", [A.EPI_NONE, A.EPI_RESIDUAL, A.EPI_SWIGLU, 8, A.EPI_CLAMP_GLU])
+def test_gemm_swapped_wait_that_runs_out(epi, splits):
+    """A limit of 1 us on waits for sums that take some 100 us: the kernel ends, every value it stores is NaN (also where the activation would
+    turn a NaN into a number), the context says so from then on, and others go on."""
+    ctx = A.Context(0)
+    M, N, K = 97, 544, 65536
+    a, b = _ints((M, K), -1, 1, 48), _ints((N, K), -1, 1, 49)
+    out = torch.zeros((M, N // 2 if epi in (A.EPI_SWIGLU, A.EPI_CLAMP_GLU) else N), dtype=torch.bfloat16, device="cuda")
+    res = _ints((M, N), -8, 8, 50) if epi == A.EPI_RESIDUAL else None
+    ctx.check_fault()
+    try:      # (the launch itself may find the word set already)
+        ctx.gemm_form(a, b, 2, 128, splits, epilogue=epi, residual=res, limit=7.0, wait_ns=1000, out=out)
+    except A.LiveCCNativeError:
+        pass
+    torch.cuda.synchronize()
+    assert bool(torch.isnan(out).all())
+    with pytest.raises(A.LiveCCNativeError, match="gave up"):
+        ctx.check_fault()
+    with pytest.raises(A.LiveCCNativeError, match="gave up"):
+        ctx.gemm(a, b)
+    other = A.Context(0)
+    assert torch.equal(other.gemm_form(a, b, 2, 128, splits), other.gemm_form(a, b, 0, 128))
+    other.check_fault()
+
+
 @pytest.mark.parametrize("form,width,splits", [(0, 96, 1), (1, 128, 1), (1, 224, 1), (2, 96, 2)])
 @pytest.mark.parametrize("limit", [7.0, math.inf])
 def test_gemm_clamped_glu(ctx, form, width, splits, limit):
