@@ -1,10 +1,10 @@
 #!/usr/bin/env python
-"""bench.py — LiveCC streaming hot path on B200 (see DESIGN.md §Measurement).
+"""bench.py — LiveCC streaming hot path on B200.
 
 One *step* = one full pass of the hot path over one synthetic 2 fps clip stream: the 6-frame first
 chunk, then 2-frame chunks, each chunk = ViT -> prefill -> <=16 greedy decode steps with
 repetition_penalty 1.05 (REF/demo/infer.py:62-180, REF/demo/cli.py:13-24).  Default workload =
-BASELINE.json configs[1]: LiveCC-7B dims, 60 s clip (120 frames, 58 chunks) at 448x448, bf16, synthetic
+LiveCC-7B dims, 60 s clip (120 frames, 58 chunks) at 448x448, bf16, synthetic
 checkpoint (no weights exist offline) and synthetic frames.
 
   value : tokens/s of the whole job with the chunk inputs already resident in HBM
@@ -172,7 +172,7 @@ def run_stream_device(eng, chunks_dev, max_new, keep_cache=False):
 
 
 def run_streams_batched(eng, chunks_dev, max_new, B, n_chunks=None):
-    """B concurrent streams on ONE GPU through generate_batch (SURVEY.md §8(f) rank 2): per chunk the ViT and the prefill
+    """B concurrent streams on ONE GPU through generate_batch: per chunk the ViT and the prefill
     run per stream, the decode steps run batched in the persistent kernel (weights read once per step for all B)."""
     caches, pasts = [None] * B, [None] * B
     n_tok = n_frames = 0
@@ -281,7 +281,7 @@ def time_persistent_kernel(eng, chunks_dev, max_new, iters=20):
     Timed alone with CUDA events on its launch stream (the sub-range hook of the C ABI launches exactly the kernel the
     CUDA-graph step contains, without the token selection, so the stream state does not advance and every launch
     re-reads the same bytes): algorithmic bytes per launch = all decoder weights + lm_head + the stream's KV at the
-    clip's final length (SURVEY.md §8(d)); inputs (14 GB) >> L2 (126 MB)."""
+    clip's final length; inputs (14 GB) >> L2 (126 MB)."""
     from livecc_b200 import _cabi
 
     t = eng.config.text_config
@@ -311,7 +311,7 @@ def time_persistent_kernel(eng, chunks_dev, max_new, iters=20):
 
 
 def time_ingest_kernel(eng, peak, iters=20):
-    """GPU frame ingest (SURVEY.md §8(f) rank 1): resize_bicubic_aa_u8_kernel on a 2-frame 1080p chunk -> 448x796 (what
+    """GPU frame ingest: resize_bicubic_aa_u8_kernel on a 2-frame 1080p chunk -> 448x796 (what
     get_smart_resized_clip does for a 16:9 source, video_process_patch.py:150-155), rotated over > L2 of distinct clips,
     CUDA events; beside it the reference's host call (torchvision, all host threads) on the same clip, and whether the
     two results are identical. Algorithmic bytes = source + destination planes; the kernel is fp32-issue bound."""
@@ -626,7 +626,7 @@ def main():
         if args.model == "7b":
             tr = json.load(open(os.path.join(ROOT, "profiles", "r01_gateup_ncu.json")))
             traffic = tr["dram_bytes_read"] + tr["dram_bytes_write"]
-            traffic_src = "static: one `ncu --set full` capture of this kernel (profiles/r01_gateup_ncu.json), not measured in this run"
+            traffic_src = "static: one `ncu --set full` capture of this kernel, not measured in this run"
     except Exception:
         traffic = None
     t = cfg.text_config

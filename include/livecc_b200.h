@@ -4,7 +4,7 @@
  *
  * The reference (showlab/livecc) has no native/FFI boundary of its own: the path sits behind Python
  * surfaces (REF/demo/infer.py:43-50,165-174 -> transformers Qwen2VLForConditionalGeneration). This
- * header is therefore the boundary *we* define one level below that surface (SURVEY.md §8(b) B5);
+ * header is therefore the boundary *we* define one level below that surface;
  * each entry point cites the reference interface (file:line) whose arithmetic it replaces.
  *   mq2vl.py     = transformers/models/qwen2_vl/modeling_qwen2_vl.py   (transformers 5.5.0)
  *   gen/utils.py = transformers/generation/utils.py
@@ -185,7 +185,7 @@ typedef struct {
     int32_t eos_token_id;
     int32_t max_new_tokens;
     float inv_repetition_penalty; /* fp32(1.0 / (double)penalty): torch's CUDA `tensor / python_float` multiplies by
-                                     this value (measured: tools/penalty_probe.py); 0 = derive as 1.0f / repetition_penalty */
+                                     this value (measured); 0 = derive as 1.0f / repetition_penalty */
     int32_t eos_token_id2;        /* second stop id (generation_config.json eos_token_id = [151645, 151643] in the
                                      Qwen2-VL family; gen/utils.py stops on any of them), < 0 = none */
 } lcc_sampling;
@@ -273,7 +273,7 @@ int lcc_prefill(lcc_model* m, const lcc_stream_state* st, const int64_t* ids, co
 int lcc_decode_steps(lcc_model* m, const lcc_stream_state* st, int n_steps, int nsplit, const lcc_sampling* sp,
                      lcc_stream_t stream);
 
-/* Batched decode (SURVEY.md §8(f) rank 2; the reference demo admits 5 concurrent sessions on one model,
+/* Batched decode (the reference demo admits 5 concurrent sessions on one model,
  * REF/demo/app.py:178): n_steps x (one persistent kernel = every decoder layer + lm_head for all n_streams <= 8 streams,
  * each weight byte read once per step, then one token selection per stream). states[b] must have been prefilled with
  * slot = b and share one page pool. A stream's ids and logits are bit-identical to decoding it alone (same kernel,
@@ -286,7 +286,7 @@ int lcc_decode_batch(lcc_model* m, const lcc_stream_state* states, int n_streams
 int lcc_decode_mega_debug(lcc_model* m, const lcc_stream_state* states, int n_streams, int layer_begin, int layer_end,
                           int phase_mask, int do_head, lcc_stream_t stream);
 
-/* ---- frame ingest (SURVEY.md §8(f) rank 1) ------------------------------------------------------------------------------
+/* ---- frame ingest ------------------------------------------------------------------------------
  * transforms.functional.resize(clip, [H, W], interpolation=BICUBIC, antialias=True) on a uint8 TCHW clip
  * (REF/livecc-utils/src/livecc_utils/video_process_patch.py:101-106 and :150-155), bit-identical to torchvision 0.26 /
  * ATen's CPU kernel: float32 width pass, float32 height pass, clamp, round half to even, uint8. */

@@ -1,7 +1,7 @@
 """Builds liblivecc_sm100a.so in-tree with nvcc for sm_100a (no torch dependency in the library).
 
 `python -m livecc_b200.build` or `livecc_b200.build.build()`; nvcc cross-compiles without a GPU.
-The .so is git-ignored but travels to the GPU box with the gpurun snapshot.
+The .so is git-ignored but travels with a copy of the tree.
 """
 from __future__ import annotations
 

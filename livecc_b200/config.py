@@ -82,7 +82,7 @@ class LiveCCConfig:
     # -- factories --------------------------------------------------------------------------
     @staticmethod
     def livecc_7b() -> "LiveCCConfig":
-        """LiveCC-7B = Qwen2-VL-7B dims (SURVEY.md §8 header)."""
+        """LiveCC-7B = Qwen2-VL-7B dims."""
         return LiveCCConfig()
 
     @staticmethod

@@ -539,15 +539,26 @@ int launch_attn_rows(const float* q, const void* k_pages, const void* v_pages, c
     const int ctas = G * ((per + HB - 1) / HB) * S;
     // splits: a tile of keys per CTA while the SMs have room (about two CTAs each). A replayed step's range grows behind the host's back: at least 8
     const int tiles = (keys_est + kRowKeys - 1) / kRowKeys;
-    int nz = std::min({pos.kv_len ? std::max(tiles, 8) : tiles, std::max(1, 296 / ctas), kRowSplitsMax});
+    int nz = std::min({pos.kv_len ? std::max(tiles, 8) : tiles, std::max(1, 2 * kSms / ctas), kRowSplitsMax});
     const size_t cnt = kSplitCounters, per_split = (size_t)S * Hq * row_part_stride(DV);
     nz = std::max(1, (int)std::min<size_t>(nz, ws_floats > cnt ? (ws_floats - cnt) / per_split : 1));
     const size_t smem = sizeof(float) * row_smem_floats(HB, D, DV);
     int* counters = reinterpret_cast<int*>(ws);              // zero when the workspace is bound; every launch leaves zeros
     const dim3 grid(ctas / S, S, nz);
     count_launch();
-#define LCC_ATTN_ROWS(HBN, PLN, NPN)                                                                                                   do {                                                                                                                                  static SmemAttrOnce once;                                                                                                         if (ensure_dyn_smem(once, attn_rows_kernel<T, HBN, PLN, NPN>, kRowSmem)) return -100;                                             chained(attn_rows_kernel<T, HBN, PLN, NPN>, grid, 256, smem, s)(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,                                                                         (const T*)gate, ld_gate, (T*)out, ld_out, S, Hq, G, D, DV, chunk, scale, pos,                                                                    sink, ld_v, ws + cnt, counters, opt);                              } while (0)
-#define LCC_ATTN_ROWS_HB(PLN, NPN)                                                                                                     do { if (HB == 2) LCC_ATTN_ROWS(2, PLN, NPN); else LCC_ATTN_ROWS(8, PLN, NPN); } while (0)
+#define LCC_ATTN_ROWS(HBN, PLN, NPN)                                                                                                        \
+    do {                                                                                                                                    \
+        static SmemAttrOnce once;                                                                                                           \
+        if (ensure_dyn_smem(once, attn_rows_kernel<T, HBN, PLN, NPN>, kRowSmem)) return -100;                                               \
+        chained(attn_rows_kernel<T, HBN, PLN, NPN>, grid, 256, smem, s)(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,     \
+                                                                       (const T*)gate, ld_gate, (T*)out, ld_out, S, Hq, G, D, DV, chunk,    \
+                                                                       scale, pos, sink, ld_v, ws + cnt, counters, opt);                    \
+    } while (0)
+#define LCC_ATTN_ROWS_HB(PLN, NPN)                                                                                                          \
+    do {                                                                                                                                    \
+        if (HB == 2) LCC_ATTN_ROWS(2, PLN, NPN);                                                                                            \
+        else LCC_ATTN_ROWS(8, PLN, NPN);                                                                                                    \
+    } while (0)
     if constexpr (VN == 8) {
         if (pieces <= 16) LCC_ATTN_ROWS_HB(16, 1);
         else if (pieces <= 32) LCC_ATTN_ROWS_HB(32, 1);

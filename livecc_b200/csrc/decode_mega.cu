@@ -2,7 +2,7 @@
 // for up to 8 independent streams (Qwen2VLDecoderLayer.forward x L + norm + lm_head, mq2vl.py:613-662, 905, 1437;
 // the loop body of GenerationMixin._sample, gen/utils.py:2743-2805). It replaces the 6 kernels per layer of the
 // per-op path (gemv.cu + attention.cu), whose launch / first-load / tail latency kept the step at 70 % of the HBM
-// roofline (DESIGN.md §7), and it is what makes multi-stream batching (SURVEY.md §8(f) rank 2) a weight-read-once
+// roofline, and it is what makes multi-stream batching a weight-read-once
 // operation.
 //
 // Structure (grid = #SMs, one CTA per SM, 384 threads):

@@ -37,7 +37,7 @@ int cast_f32_bf16(const float* in, bf16* out, int64_t n, int num_sms, cudaStream
 }
 
 // ------------------------------------------------------------------------------------------
-// GPU frame ingest (SURVEY.md §8(f) rank 1): uint8 frames [T,3,H,W] -> bf16 patch rows [N, 3*2*14*14] in one pass,
+// GPU frame ingest: uint8 frames [T,3,H,W] -> bf16 patch rows [N, 3*2*14*14] in one pass,
 // replacing the host-side rescale/normalize/patchify of Qwen2VLVideoProcessor._preprocess
 // (video_processing_qwen2_vl.py:240-272; fused mean/std: image_processing_backends.py:301-304,327) plus the
 // f32 H2D copy and the bf16 cast (mq2vl.py:309). Bit-identical to cast_bf16(host patchify): the value is
@@ -248,7 +248,7 @@ static int norm_rows(const bf16* x, int ldx, const bf16* w, const bf16* b, bf16*
     if (dim % 8 || ldx % 8 || ldy % 8) return -1;
     lcc::count_launch();
     // (one wave: a CTA walks over further rows with the weights it has, the next row's loads in flight)
-    const int sms = 148;
+    const int sms = kSms;
     if (dim <= 1536 && rows >= 16 * sms) norm_rows_warp_kernel<RMS><<<(rows + 7) / 8, 256, 0, s>>>(x, ldx, w, b, y, ldy, rows, dim, eps);
     else if (dim <= 512) norm_rows_kernel<RMS, 64, 1><<<min(rows, 16 * sms), 64, 0, s>>>(x, ldx, w, b, y, ldy, rows, dim, eps);
     else if (dim <= 1536) norm_rows_kernel<RMS, 192, 1><<<min(rows, 5 * sms), 192, 0, s>>>(x, ldx, w, b, y, ldy, rows, dim, eps);

@@ -1153,7 +1153,7 @@ static int launch_epi(const GemmArgs& a, int bn, int num_sms, cudaStream_t strea
     return -14;
 }
 
-// Tile-width choice. What the B200 measurements say (profiles/r02_gemm_shapes.md, r02_gemm_vs_cublas.md):
+// Tile-width choice. What the B200 measurements say:
 //  * with one CTA per SM the main loop is bound by SHARED-MEMORY bandwidth, not by the tensor pipe: per 64-deep k-block the
 //    TMA writes 16 KB (A) + bn*128 B (B) into shared memory and the four MMAs read the same bytes back: 2*(16384 + 128*bn) B
 //    at 128 B/clk = 256 + 2*bn clocks against the tensor floor of 2*bn (bn = 256: 67 %, 128: 50 %, 64: 33 % — the measured
@@ -1277,8 +1277,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits,
 
 // Split-K for small-M GEMMs whose tile count cannot occupy the SMs (prefill down_proj at M ~ 281: 84 tiles on 148 SMs).
 // Returns 1 if it handled the GEMM, 0 if the caller should run the plain path, < 0 on error.
-// Validated on B200 in round 2 (bit-exact on integer operands, test_gemm_splitk_exact_integer_operands; whole-model parity
-// with it forced on). Measured (profiles/r02_gemm_shapes.md): it pays only for long K — down_proj (K = 18944) 86.7 -> 60.9 us,
+// Bit-exact on integer operands (test_gemm_splitk_exact_integer_operands), whole-model parity with it forced on. Measured on B200: it pays only for long K — down_proj (K = 18944) 86.7 -> 60.9 us,
 // while qkv / o_proj (K = 3584) get slower (23 -> 34 us) — so the default applies it for K >= 8192 only.
 // LIVECC_B200_GEMM_SPLITK=1 forces it for every eligible shape, =0 disables it.
 static int splitk_mode() {

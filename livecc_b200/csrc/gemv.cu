@@ -1,5 +1,5 @@
 // Decode-step (M = 1) projections: weight-streaming GEMV kernels, HBM-bound by construction
-// (14.1 GB of bf16 weights per generated token at 7B, SURVEY.md §8(d)). CUDA cores only — a 1-row
+// (14.1 GB of bf16 weights per generated token at 7B). CUDA cores only — a 1-row
 // operand cannot feed a tensor-core tile — with 16-byte non-allocating loads, >= 8 independent loads
 // in flight per lane, the activation vector staged once per CTA in shared memory, and the
 // RMSNorm / bias / SwiGLU / residual work fused around the dot products.
@@ -12,7 +12,7 @@
 //   gemv_rows_kernel  : K <= 8192.  Each warp owns ROWS consecutive weight rows (full K).
 //   gemv_splitk_kernel: large K (down_proj, K = 18944). A CTA owns ROWS rows; its 8 warps split K.
 // (A persistent one-CTA-per-SM variant was measured slower — 3.87 vs 3.29 ms/step — because it gives up the
-//  thread-level parallelism that hides the load->use latency; see DESIGN.md.)
+//  thread-level parallelism that hides the load->use latency.)
 #include <stdlib.h>
 
 #include "common.cuh"

@@ -13,6 +13,9 @@ namespace lcc {
 inline std::atomic<uint64_t> g_launches{0};
 inline void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
+// SMs of a B200, for the sizes of grids whose kernels run whatever the number is (the entry points take the device's own count).
+constexpr int kSms = 148;
+
 // cudaFuncAttributeMaxDynamicSharedMemorySize is a per-device attribute of a kernel: remember per (kernel
 // instantiation, device) that it was raised, so a second engine on another device of the same process works.
 struct SmemAttrOnce {

@@ -163,7 +163,7 @@ lcc_model* lcc_model_create(lcc_ctx* ctx, const lcc_model_config* cfg, const lcc
     m->w.vit_blocks = m->vit_blocks.data();
     m->w.layers = m->layers.data();
     const char* mega_env = getenv("LIVECC_B200_MEGA");
-    // Measured on B200 (profiles/r02_decode_paths.md): for ONE stream the per-op kernels are 5 % faster than the persistent
+    // Measured on B200: for ONE stream the per-op kernels are 5 % faster than the persistent
     // kernel (3.21 vs 3.37 ms/step in situ), so lcc_decode_steps keeps them by default; lcc_decode_batch (2..8 streams) is
     // always the persistent kernel.
     m->use_mega = mega_env && mega_env[0] == '1';

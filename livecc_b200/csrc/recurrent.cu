@@ -489,7 +489,7 @@ int causal_conv(int dt, const void* in, int ld_in, void* out, int ld_out, const 
     if (pairs) {
         const unsigned gx = (C / 2 + 127) / 128;
         int span = 8;   // more rows per thread (fewer of them read twice) once that leaves every SM a few CTAs
-        while (span < 32 && (uint64_t)gx * ((S + 2 * span - 1) / (2 * span)) >= 4 * 148) span *= 2;
+        while (span < 32 && (uint64_t)gx * ((S + 2 * span - 1) / (2 * span)) >= 4 * kSms) span *= 2;
         const dim3 lg(gx, (S + span - 1) / span);
 #define LCC_CONV_LONG(TP)                                                                                                                    \
     do {                                                                                                                                     \

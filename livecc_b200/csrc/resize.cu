@@ -1,4 +1,4 @@
-// GPU frame ingest (SURVEY.md §8(f) rank 1): the antialiased bicubic resize of
+// GPU frame ingest: the antialiased bicubic resize of
 //   REF/livecc-utils/src/livecc_utils/video_process_patch.py:101-106,150-155
 //   transforms.functional.resize(clip_u8_TCHW, [H, W], BICUBIC, antialias=True)
 // reproduced bit for bit: torchvision casts uint8 -> float32, ATen's CPU upsample_bicubic2d_aa runs a width pass then a

@@ -1,4 +1,4 @@
-"""B1/B2 of the drop-in boundary (SURVEY.md §8(b)): a model object with the surface
+"""B1/B2 of the drop-in boundary: a model object with the surface
 `LiveCCDemoInfer` uses on `Qwen2VLForConditionalGeneration` (REF/demo/infer.py:43-50,158,165-174):
 
     model = LiveCCB200ForConditionalGeneration.from_pretrained(path, torch_dtype="auto", device_map="cuda")
@@ -343,7 +343,7 @@ class LiveCCB200ForConditionalGeneration:
     def generate_batch(self, requests: List[dict], repetition_penalty: float = 1.0, logits_processor=None,
                        max_new_tokens: int = 16, do_sample: Optional[bool] = None, output_logits: bool = False,
                        pad_token_id: Optional[int] = None) -> List[GenerateOutput]:
-        """Multi-stream batching (SURVEY.md §8(f) rank 2): one generate() for up to 8 independent streams of this model
+        """Multi-stream batching: one generate() for up to 8 independent streams of this model
         (the reference demo admits 5 concurrent sessions on one model object, REF/demo/app.py:178, and serves them one
         after another). Every request is a dict with the per-stream arguments of generate() (`input_ids` [1, L],
         `pixel_values_videos` | `video_frames`, `video_grid_thw`, `past_key_values`). The ViT and the prefill run per
@@ -394,7 +394,7 @@ class LiveCCB200ForConditionalGeneration:
         """The single-forward multiple-choice scoring of the reference's evaluators
         (REF/evaluation/distributed_mcq_predictor.py:72-105): a LEFT-padded batch (`padding_side='left'`,
         REF/evaluation/videomme/distributed_evaluate_videomme.py:39-42), one forward, the logits of the last position
-        restricted to the answer-letter token ids, argmax. No decode loop: ViT + prefill only (BASELINE config #5).
+        restricted to the answer-letter token ids, argmax. No decode loop: ViT + prefill only.
 
         input_ids / attention_mask: [B, L] (pads on the left, mask 0 there); pixel_values_videos: the processor's rows of
         all samples concatenated; video_grid_thw: [n_videos, 3], one video per sample that contains <|video_pad|> ids,

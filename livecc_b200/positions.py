@@ -1,6 +1,6 @@
 """Position-id bookkeeping of the streaming path (host integers fed to the kernels).
 
-Three regimes (probe A5):
+Three regimes:
   * first turn (empty cache): 3-D M-RoPE ids from `get_rope_index`, and rope_delta = max_pos + 1 - L,
     computed once and kept in the per-stream cache (the reference keeps it on the *model*,
     mq2vl.py:923,1207,1518, which makes two interleaved streams corrupt each other);

@@ -145,7 +145,7 @@ class StubProcessor:
     def __init__(self, config=None, merge_size: int = 2, patch_size: int = 14, temporal_patch_size: int = 2,
                  emit_frames: bool = False):
         """`config`: optional LiveCCConfig supplying (possibly relocated) special ids and vocab size.
-        `emit_frames=True` (GPU frame ingest, SURVEY.md §8(f)): uint8 clips are passed through as `video_frames`
+        `emit_frames=True` (GPU frame ingest): uint8 clips are passed through as `video_frames`
         (4x fewer H2D bytes than f32 patch rows) and the engine normalises + patchifies them on the device."""
         self.emit_frames = emit_frames
         if config is not None:

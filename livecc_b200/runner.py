@@ -1,4 +1,4 @@
-"""Multi-GPU driver: independent video streams, one process per GPU (SURVEY.md §8(e)).
+"""Multi-GPU driver: independent video streams, one process per GPU.
 
 The path is embarrassingly data-parallel, exactly like the reference's evaluation driver, which shards
 `idxs[device_id::num_workers]` over one process per GPU with no communication

@@ -3,12 +3,12 @@
 Drives the *installed* third-party implementation that carries the reference's arithmetic:
 `transformers.Qwen2VLForConditionalGeneration` (transformers 5.5.0, un-vendored dependency of
 showlab/livecc: REF/demo/infer.py:4,43-47; REF/README.md:25). The reference repo holds no model code and
-no tests for this path (SURVEY.md §4), so parity is pinned against this model object, built with the
+no tests for this path, so parity is pinned against this model object, built with the
 same synthetic checkpoint the engine loads (livecc_b200/checkpoint.py), through a restated
 `LiveCCDemoInfer.live_cc` chunk loop (REF/demo/infer.py:105-180).
 
 Version caveat recorded next to every parity number: oracle = transformers 5.5.0 semantics (first-turn
-M-RoPE of t>1 grids differs from the 4.5x stack LiveCC shipped with; SURVEY.md §0.4).
+M-RoPE of t>1 grids differs from the 4.5x stack LiveCC shipped with).
 """
 from __future__ import annotations
 
@@ -48,7 +48,7 @@ _LIGER_APPLIED = [False]
 
 
 def apply_liger():
-    """Oracle variant (B) of SURVEY.md §7: the reference's real GPU path calls
+    """Oracle variant (B): the reference's real GPU path calls
     `liger_kernel.transformers.apply_liger_kernel_to_qwen2_vl()` before the model is built (REF/demo/infer.py:2-3,
     REF/inference.md:14). The patch swaps module-level symbols of transformers for the rest of the process, so a
     test that uses it must run after every variant-(A) test of the same process."""

@@ -10,7 +10,7 @@ transformers/generation/utils.py). It imports no HF modeling code. Two uses:
   * GPU bf16: per-op reference for the CUDA kernels — the ops are issued in the same order as the HF
     eager graph so every bf16 rounding point coincides.
 
-Parity status: the reference repo has no tests or golden vectors for this path (SURVEY.md §4), so the
+Parity status: the reference repo has no tests or golden vectors for this path, so the
 restatement is pinned against outputs of the installed HF implementation, generated by
 tests/golden/make_golden.py (committed with its outputs).
 """

@@ -2,7 +2,7 @@
 (transformers Qwen2VLForConditionalGeneration + Qwen2VLVideoProcessor, fp32 on CPU).
 
 Run here (no GPU needed):  python tests/golden/make_golden.py
-The reference repo holds no tests or golden vectors for this path (SURVEY.md §4), so these files pin the
+The reference repo holds no tests or golden vectors for this path, so these files pin the
 oracle restatement (oracle/restated.py) and the host logic (positions, patchify) against outputs of the
 third-party code the reference actually executes. Version: transformers 5.5.0.
 """

@@ -2,7 +2,7 @@
 tokenizer without merges (ids 0..255 = bytes) + the Qwen2-VL special tokens, the stock `Qwen2VLImageProcessor` /
 `Qwen2VLVideoProcessor`, and a chat template with the Qwen2-VL layout, saved with `save_pretrained` so that
 `AutoProcessor.from_pretrained(dir, use_fast=False)` -- the call REF/demo/infer.py:48 makes -- loads it. Used to run the
-unmodified HF processor code under LiveCCDemoInfer (SURVEY.md §8 a4 / B4)."""
+unmodified HF processor code under LiveCCDemoInfer."""
 import copy
 
 SPECIALS = ["<|im_end|>", "<|endoftext|>", "<|im_start|>", "<|vision_start|>", "<|vision_end|>", "<|vision_pad|>",

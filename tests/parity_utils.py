@@ -1,4 +1,4 @@
-"""Shared helpers of the GPU parity tests: the margin-aware comparison rule of DESIGN.md §2.
+"""Shared helpers of the GPU parity tests: the margin-aware comparison rule.
 
 free-running ids must be IDENTICAL to the oracle's, except that a divergence is accepted at a step where the oracle's
 own top-1/top-2 margin after logits processing is <= 2 * atol (two correct bf16 implementations may legitimately pick

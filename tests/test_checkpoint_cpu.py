@@ -1,4 +1,4 @@
-"""Checkpoint plumbing on the CPU (SURVEY.md §8(f) rank 4): an HF-named safetensors directory in the pre-5.x and the
+"""Checkpoint plumbing on the CPU: an HF-named safetensors directory in the pre-5.x and the
 5.x naming round-trips into the engine weight layout (q/k/v fused, gate/up interleaved), config.json /
 generation_config.json are honoured, tied checkpoints fall back to the embedding table and broken ones fail with a
 readable message. The GPU half (from_pretrained -> identical ids) is tests/test_engine_gpu.py::test_from_pretrained_round_trip."""

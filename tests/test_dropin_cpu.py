@@ -2,7 +2,7 @@
 describes and diffs everything it does against livecc_b200.streaming.LiveCCDemoInfer: every generate() call
 (ids, cache length, pixel rows, kwargs incl. the ThresholdLogitsProcessor the canonical caller REF/demo/cli.py:16-19
 asks for), every yielded ((start, stop), text) and the `state` contract. The model is a deterministic recording mock
-(this is the host-side boundary test for SURVEY.md §8 B1-B3; the arithmetic behind generate() is covered by the
+(this is the host-side boundary test; the arithmetic behind generate() is covered by the
 `-m gpu` parity tests). Runs only where /root/reference exists (the build container); the GPU box has no reference."""
 import importlib
 import importlib.util

@@ -2,7 +2,7 @@
 
 Oracles: (1) the plain-torch restatement in bf16 on the same GPU (same rounding points as HF eager),
 (2) the installed HF Qwen2VLForConditionalGeneration in bf16 on the GPU, both fed the same synthetic
-checkpoint. Protocol (SURVEY.md §7 "hard parts"): teacher-forced logits within a stated bf16 tolerance,
+checkpoint. Protocol: teacher-forced logits within a stated bf16 tolerance,
 top-1 agreement wherever the oracle's margin exceeds twice that tolerance, free-running ids compared
 with every divergence required to sit on a sub-tolerance margin."""
 import pytest
@@ -63,7 +63,7 @@ def test_vit_forward_matches_restatement(small):
         cos = torch.nn.functional.cosine_similarity(o, r, dim=1)
         stats = dict(p50=ulps.median().item(), p99=ulps.flatten().kthvalue(int(0.99 * ulps.numel())).values.item(),
                      max=ulps.max().item(), min_cos=cos.min().item())
-        # measured on B200 (gpurun call 29): p50 0.51, p99 2.2-2.4, max 4.1-5.1 ulps, min cosine 0.99999
+        # measured on B200: p50 0.51, p99 2.2-2.4, max 4.1-5.1 ulps, min cosine 0.99999
         assert stats["min_cos"] > 0.9999, stats
         assert stats["p50"] < 0.8 and stats["p99"] < 4.0 and stats["max"] < 12.0, stats
 

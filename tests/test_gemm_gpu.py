@@ -238,7 +238,7 @@ def test_gemm_splitk_exact_integer_operands(ctx, M, N, K):
     """split-K (fp32 partial tiles + reduce kernel with the fused epilogue): integer operands keep every partial sum
     exact, so the result must be bit-identical to the unsplit reference for all four supported epilogues. By default
     the dispatch splits only K >= 8192 (the first shape); LIVECC_B200_GEMM_SPLITK=1 forces it for all of them (both
-    modes were run on B200 in round 2, profiles/r02_parity_7b.md)."""
+    modes were run on B200)."""
     a = _ints((M, K), -2, 2, 11)
     b = _ints((N, K), -1, 1, 12)
     bias = _ints((N,), -8, 8, 13)

@@ -80,7 +80,7 @@ def test_synthetic_checkpoint_is_device_independent_and_complete():
         for s in shape:
             numel *= s
         n[k] = n.get(k, 0) + numel
-    # parameter counts of SURVEY.md §8 (verified there by instantiating the HF modules)
+    # parameter counts (those of the instantiated HF modules)
     assert n["vit"] == 675_759_104 and n["layer0"] == 233_057_792 and n["lm_head"] == 544_997_376
     total = sum(__import__("math").prod(s) for _, s, _ in hf_param_specs(cfg7))
     assert total == 8_291_375_616
@@ -110,7 +110,7 @@ def _turn_inputs(proc, turn, frames, hw, seed):
 
 def test_restated_streaming_matches_hf_golden(small_fp32):
     """3 streaming turns: greedy ids bit-exact, top-5 logits to fp32 round-off, cache length and the
-    turn-0 rope_delta persistence (SURVEY.md probe A2/A5)."""
+    turn-0 rope_delta persistence."""
     cfg, sd, rs = small_fp32
     gold = GOLD["streaming"]
     proc = StubProcessor(cfg)

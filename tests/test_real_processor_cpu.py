@@ -1,4 +1,4 @@
-"""The real-processor branch (SURVEY.md §8 a4/B4): `AutoProcessor.from_pretrained(model_path, use_fast=False)`
+"""The real-processor branch: `AutoProcessor.from_pretrained(model_path, use_fast=False)`
 (REF/demo/infer.py:48-49) with the UNMODIFIED transformers Qwen2VLProcessor / tokenizer / video processor, built offline by
 tests/hf_tiny_processor.py, driven by (a) livecc_b200.streaming.LiveCCDemoInfer and (b) the unmodified reference
 orchestrator, on a recording mock model. Also pins the offline StubProcessor against it: identical pixel rows, grids and

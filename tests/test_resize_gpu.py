@@ -1,4 +1,4 @@
-"""GPU frame ingest (SURVEY.md §8(f) rank 1): lcc_resize_bicubic_aa_u8 through the C ABI against the oracle, the golden
+"""GPU frame ingest: lcc_resize_bicubic_aa_u8 through the C ABI against the oracle, the golden
 digests of the reference's torchvision call, and live torchvision. Bar: bit-exact (uint8)."""
 import json
 import os

@@ -1,4 +1,4 @@
-"""Event timing of gemm_bf16_tn_kernel at the shapes of the streaming path (SURVEY.md §8): decoder prefill at M = 281 and
+"""Event timing of gemm_bf16_tn_kernel at the shapes of the streaming path: decoder prefill at M = 281 and
 the ViT at M = 1024 / 3072, with the epilogues the model uses. CASE=<name> runs one shape twice (for `ncu -k regex:gemm`)."""
 import os
 import sys

@@ -1,9 +1,9 @@
-"""BASELINE config #5 (offline batch-32 16-frame MCQ, VideoMME shape, synthetic): ViT + prefill only, no decode loop,
+"""Offline batch-32 16-frame MCQ, VideoMME shape, synthetic: ViT + prefill only, no decode loop,
 through `LiveCCB200ForConditionalGeneration.forward_mcq` = the reference's single-forward scoring
 (REF/evaluation/distributed_mcq_predictor.py:72-105): left-padded batch, last-position logits over the letter ids.
 Sweeps the batch size 1..32; per batch the vision tower runs once over all B*8 temporal segments (B*8192 patches) and the
 decoder prefill once per sample (2090 tokens each). Reports samples/s, frames/s and the achieved tensor throughput
-against the sustained bf16 peak (algorithmic FLOPs: SURVEY.md §8(d): 1.49 TFLOP per 1024-patch segment;
+against the sustained bf16 peak (algorithmic FLOPs: 1.49 TFLOP per 1024-patch segment;
 2*6.525e9*S + 4*S*(S/2)*3584*28 per prefill)."""
 import argparse
 import json

@@ -1,4 +1,4 @@
-"""Head-to-head with "the kernel to beat" (SURVEY.md §2.3 K4/K11, §8(d)): flash-attn 2 (the reference's attention,
+"""Head-to-head with "the kernel to beat": flash-attn 2 (the reference's attention,
 REF/demo/infer.py:46) vs the tcgen05/TMEM kernels of this repo at the
 §8 shapes, on the same B200, CUDA-event timed, L2 flushed between iterations. Writes a markdown table to stdout
 (copy under profiles/). flash-attn is LIBRARY code used here only as the measured competitor."""

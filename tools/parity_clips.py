@@ -1,7 +1,7 @@
 """Greedy-id parity over many synthetic clips: engine vs the installed HF model (bf16, same GPU).
 Writes a JSON summary: exact-match rate of free-running ids, worst teacher-forced |dlogit|, and for every
 diverging step the oracle's top-1/top-2 margin (divergences must sit on sub-tolerance margins).
-usage: python tools/parity_clips.py [--clips 100] [--model small] [--out profiles/r01_parity_clips.json]"""
+usage: python tools/parity_clips.py [--clips 100] [--model small] [--out parity_clips.json]"""
 import argparse
 import json
 import os
@@ -21,7 +21,7 @@ ap.add_argument("--clips", type=int, default=100)
 ap.add_argument("--model", default="small")
 ap.add_argument("--size", type=int, default=112)
 ap.add_argument("--tokens", type=int, default=8)
-ap.add_argument("--out", default="profiles/r01_parity_clips.json")
+ap.add_argument("--out", default="parity_clips.json")
 args = ap.parse_args()
 DEV = "cuda"
 cfg = LiveCCConfig.livecc_7b() if args.model == "7b" else LiveCCConfig.small()
