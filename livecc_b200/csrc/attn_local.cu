@@ -937,6 +937,7 @@ int launch_attn_tiled(const float* q, const void* k_pages, const void* v_pages, 
     if (ensure_dyn_smem(once, attn_chunk_sink_tiled_kernel<T>, (int)smem)) return -100;
     dim3 grid(Hq, (S + AQ - 1) / AQ, (DV + AVW - 1) / AVW);
     count_launch();
+    chain_break();
     chained(attn_chunk_sink_tiled_kernel<T>, grid, 256, attn_tiled_smem<T>(D), s)(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,
                                                                             (const T*)gate, ld_gate, (T*)out, ld_out, S, Hq, G, D, DV,
                                                                             chunk, scale, pos, sink, ld_v, opt);
@@ -1297,6 +1298,7 @@ int launch_attn_mma(const float* q, const void* k_pages, const void* v_pages, co
 #define LCC_ATTN_MMA(ONCE, VEC, KHN, NVN, ...)                                                                                  \
     do {                                                                                                                     \
         if (ensure_dyn_smem(ONCE, attn_chunk_sink_mma_kernel<VEC, KHN, NVN, ##__VA_ARGS__>, (int)smem_max)) return -100;          \
+        chain_break();                                                                                                       \
         chained(attn_chunk_sink_mma_kernel<VEC, KHN, NVN, ##__VA_ARGS__>, grid, 128 * KHN, smem, s)(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, \
                                                                            page_size, (const bf16*)gate, ld_gate, (bf16*)out, ld_out, \
                                                                            S, Hq, G, D, DV, chunk, scale, pos, sink, ld_v, opt);  \
@@ -1336,6 +1338,7 @@ int launch_attn_mma_maps(const float* q, const void* k_pages, const void* v_page
 #define LCC_ATTN_MAPS(ONCE, VEC, NVN, NB)                                                                                        \
     do {                                                                                                                         \
         if (ensure_dyn_smem(ONCE, attn_chunk_sink_mma_kernel<VEC, 2, NVN, NB, 2, true>, (int)smem_max)) return -100;                   \
+        chain_break();                                                                                                           \
         chained(attn_chunk_sink_mma_kernel<VEC, 2, NVN, NB, 2, true>, grid, 256, smem, s)(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, page_size, \
                                                                                nullptr, 0, (bf16*)out, ld_out, S, Hq, G, D, DV, chunk, scale, pos, \
                                                                                sink, ld_v, opt);                                 \

@@ -92,3 +92,13 @@ def test_the_kernel_behind_a_copy_a_clear_a_fork_or_a_join_is_not_chained():
             assert "STEP(" not in between, w.group(0)
         else:
             assert not re.search(r"STEP\([^;]*\bfs\b", between), w.group(0)
+
+
+def test_prompt_attention_is_launched_in_the_ordinary_way():
+    """Its few large CTAs would be placed on the SMs that the kernel in front leaves free, two to an SM."""
+    src, _ = kernels("attn_local")
+    flat = re.sub(r"[\\\s]+", " ", src)
+    launches = [m.start() for m in re.finditer(r"chained\(attn_chunk_sink_(?:mma|tiled)_kernel", flat)]
+    assert len(launches) == 3
+    for at in launches:
+        assert flat[:at].rstrip().endswith("chain_break();")
