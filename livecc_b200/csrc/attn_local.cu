@@ -537,7 +537,7 @@ int launch_attn_rows(const float* q, const void* k_pages, const void* v_pages, c
     const bool wide = DV > 256;                              // 16 running outputs per head and lane: at most 4 heads
     const int HB = per <= 2 ? 2 : (wide ? 4 : 8);
     const int ctas = G * ((per + HB - 1) / HB) * S;
-    // splits: a tile of keys per CTA while the SMs have room (about two CTAs each). A replayed step's range grows behind the host's back: at least 8
+    // splits: a tile of keys per CTA while the SMs have room (two CTAs each; the eight-head forms, 230 registers, fit once). A replayed step's range grows behind the host's back: at least 8
     const int tiles = (keys_est + kRowKeys - 1) / kRowKeys;
     int nz = std::min({pos.kv_len ? std::max(tiles, 8) : tiles, std::max(1, 2 * kSms / ctas), kRowSplitsMax});
     const size_t cnt = kSplitCounters, per_split = (size_t)S * Hq * row_part_stride(DV);
@@ -772,7 +772,6 @@ __global__ void __launch_bounds__(256) attn_chunk_sink_tiled_kernel(const float*
                                                                     T* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                                     int chunk, float scale, SeqPos pos,
                                                                     const float* __restrict__ sink, int ld_v, AttnOpts opt) {
-    chain_begin(q, k_pages, v_pages, page_table, gate);
     if (seq_done(pos)) return;
     extern __shared__ __align__(16) uint8_t smem_attn[];
     const int dc = min(D, ADC);
@@ -937,8 +936,7 @@ int launch_attn_tiled(const float* q, const void* k_pages, const void* v_pages, 
     if (ensure_dyn_smem(once, attn_chunk_sink_tiled_kernel<T>, (int)smem)) return -100;
     dim3 grid(Hq, (S + AQ - 1) / AQ, (DV + AVW - 1) / AVW);
     count_launch();
-    chain_break();
-    chained(attn_chunk_sink_tiled_kernel<T>, grid, 256, attn_tiled_smem<T>(D), s)(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,
+    attn_chunk_sink_tiled_kernel<T><<<grid, 256, attn_tiled_smem<T>(D), s>>>(q, (const T*)k_pages, (const T*)v_pages, page_table, page_size,
                                                                             (const T*)gate, ld_gate, (T*)out, ld_out, S, Hq, G, D, DV,
                                                                             chunk, scale, pos, sink, ld_v, opt);
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
@@ -978,7 +976,6 @@ __global__ void __launch_bounds__(128 * KH, (VEC8 && NBUF == 1 && NV == 1) ? 2 :
                                                                   bf16* __restrict__ out, int ld_out, int S, int Hq, int G, int D, int DV,
                                                                   int chunk, float scale, SeqPos pos,
                                                                   const float* __restrict__ sink, int ld_v, AttnOpts opt) {
-    chain_begin(q, k_pages, v_pages, page_table, gate);
     if (seq_done(pos)) return;
     extern __shared__ __align__(16) uint8_t smem_attn[];
     // NV output tiles of 128 channels per CTA (NV = 2: values of up to 256 channels against one pass over the scores)
@@ -1298,8 +1295,7 @@ int launch_attn_mma(const float* q, const void* k_pages, const void* v_pages, co
 #define LCC_ATTN_MMA(ONCE, VEC, KHN, NVN, ...)                                                                                  \
     do {                                                                                                                     \
         if (ensure_dyn_smem(ONCE, attn_chunk_sink_mma_kernel<VEC, KHN, NVN, ##__VA_ARGS__>, (int)smem_max)) return -100;          \
-        chain_break();                                                                                                       \
-        chained(attn_chunk_sink_mma_kernel<VEC, KHN, NVN, ##__VA_ARGS__>, grid, 128 * KHN, smem, s)(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, \
+        attn_chunk_sink_mma_kernel<VEC, KHN, NVN, ##__VA_ARGS__><<<grid, 128 * KHN, smem, s>>>(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, \
                                                                            page_size, (const bf16*)gate, ld_gate, (bf16*)out, ld_out, \
                                                                            S, Hq, G, D, DV, chunk, scale, pos, sink, ld_v, opt);  \
     } while (0)
@@ -1338,8 +1334,7 @@ int launch_attn_mma_maps(const float* q, const void* k_pages, const void* v_page
 #define LCC_ATTN_MAPS(ONCE, VEC, NVN, NB)                                                                                        \
     do {                                                                                                                         \
         if (ensure_dyn_smem(ONCE, attn_chunk_sink_mma_kernel<VEC, 2, NVN, NB, 2, true>, (int)smem_max)) return -100;                   \
-        chain_break();                                                                                                           \
-        chained(attn_chunk_sink_mma_kernel<VEC, 2, NVN, NB, 2, true>, grid, 256, smem, s)(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, page_size, \
+        attn_chunk_sink_mma_kernel<VEC, 2, NVN, NB, 2, true><<<grid, 256, smem, s>>>(q, (const bf16*)k_pages, (const bf16*)v_pages, page_table, page_size, \
                                                                                nullptr, 0, (bf16*)out, ld_out, S, Hq, G, D, DV, chunk, scale, pos, \
                                                                                sink, ld_v, opt);                                 \
     } while (0)

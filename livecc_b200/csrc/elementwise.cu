@@ -103,8 +103,8 @@ int patchify_u8(const uint8_t* frames, int T, int H, int W, bf16* out, const flo
 // RMSNorm over rows (Qwen2VLRMSNorm, mq2vl.py:126-131): y = w * bf16(x * rsqrt(mean(x^2) + eps)).
 // dim % 8 == 0. The rows of a step are few and short, so latency bounds them: a row is read once, all of its 16-byte loads (and those of
 // the weights) in flight together, and stays in registers through the passes. The team depends on the width alone, so a row's sums do
-// not depend on how many rows there are. With a warp per row and three passes over memory, a cold RMSNorm of 24 rows of 3584 took 12.3 us and
-// 2090 rows 14.3; now 6.2 and 12.3 (the launch alone: about 4).
+// not depend on how many rows there are. With a warp per row and three passes over memory, an RMSNorm of 24 rows of 3584 took 5.3 us
+// back to back, of 281 rows 5.7 and of 2090 rows 8.1; now 1.9, 2.6 and 7.7.
 // Columns beyond what the registers hold (TEAM x 8 x KEEP) are read again in each pass.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ float sum8(const uint4& u) {
@@ -443,7 +443,7 @@ __device__ __forceinline__ void mrope_cos_sin(int j /*0..63*/, int pt, int ph, i
 }
 
 // One warp per (token, slice of kMropeHeads heads): the token's 64 angles are the same for every head, so a lane forms its two once and
-// walks the slice with them. (A warp per head formed them 36 times per token: 6.5 us for 281 tokens and 25 for 2090, now 6.0 and 16.)
+// walks the slice with them. (A warp per head formed them 36 times per token: 4.5 us for 281 tokens and 23.4 for 2090, back to back; now 3.7 and 13.0.)
 constexpr int kMropeHeads = 9;
 __global__ void __launch_bounds__(256) mrope_kv_write_kernel(bf16* __restrict__ qkv, int ld, const int* __restrict__ pos3, int S,
                                       const float* __restrict__ inv_freq, MropeSections sec, int Hq, int Hkv,

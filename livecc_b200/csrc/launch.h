@@ -51,10 +51,11 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
 // A chain of short kernels: inside a ChainScope each may be set up while the one before it in the stream still runs (programmatic dependent
 // launch), and its first statement, chain_begin() in common.cuh, waits for that one. A step of the hybrid models is some 45 kernels of 3 to
 // 10 us on one row; as ordinary graph nodes, kernels that return at once cost 2.7 to 4 us each. Chained, and with the first
-// weights of a linear layer loaded before the wait, a step of the recurrent design takes 231 us for 234, of the routed one 128 for 133.
-// Kernels of few and large CTAs (prompt attention: one or two per SM) are launched behind chain_break(): chained, their CTAs go where there is
-// room while the kernel in front still holds the other SMs, and stay there two to an SM. 281 rows behind 4000 tokens of four layers with
-// distance tables took 2.58 ms unchained, 2.76 with every kernel chained.
+// weights of a linear layer loaded before the wait, a prompt of 128 tokens and 31 replayed steps take 8.29 ms for 8.48 (recurrent design, four
+// layers) and 4.86 for 5.14 (routed, two layers), one step launched by the host 0.32 ms for 0.38 and 0.33 for 0.36 (four layers each).
+// Kernels of few and large CTAs (prompt attention: one or two per SM) stay outside: chained, their CTAs go where there is room while the
+// kernel in front still holds the other SMs, and stay there two to an SM. 281 rows behind 4000 tokens of four layers with distance tables
+// took 2.60 ms unchained, 2.76 with every kernel chained. (An ordinary kernel of a scope lets the one behind it in when it is complete.)
 // The first launch of a scope and the one after chain_break() (behind a copy, a fork or a join with another stream) are ordinary: whatever
 // was enqueued before is complete when they start. Outside a scope every launch is.
 enum class Chain { off, broken, on };
