@@ -1201,9 +1201,10 @@ static int choose_pair(int M, int N, int K, int num_sms, double* us) {
 
 // Few rows: is the swapped kernel the better one? `other`: the estimate of the best other form (0: none, narrow products). One wave of
 // clusters of 2 s CTAs (two waves where all rows are one tile), max(0.42, rows / 700) us per k-block of a pair's share, 10 us for the launch,
-// 3.5 for the exchange of a split, 0.5 per 64 rows for the store. Measured (us, the other forms | this): 281 rows x 3584 x 18944 58 | 52,
-// x 37888 x 3584 81 | 77, x 3584 x 3584 24 | 22; 24 x 4608 x 3584 21 | 16.5, x 3584 x 3584 20 | 15.5; 256 x 5120 x 5120 31 | 28, x 3584 x 5120
-// 28 | 23; 1024 x 1280 x 5120 31 | 27; 2090 x 3584 x 18944 219 | 196; others stay for 24 x 37888 x 3584 46 | 60, x 3584 x 18944 32 | 44.
+// 3.5 for the exchange of a split, 0.5 per 64 rows for the store. Measured (us, best of the other forms | this, back to back): 281 rows x 3584
+// x 18944 58 | 46, x 37888 x 3584 85 | 71, x 3584 x 3584 21.0 | 19.7; 24 x 4608 x 3584 18.8 | 16.0, x 3584 x 3584 18.7 | 14.5; 256 x 5120 x 5120
+// 27 | 25, x 3584 x 5120 26 | 21; 1024 x 1280 x 5120 27 | 24; 2090 x 3584 x 18944 219 | 210; others stay for 24 x 37888 x 3584 46 | 55, x 3584
+// x 18944 31 | 40.
 static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_out, int* splits_out) {
     const int n_tiles = (N + 2 * BLOCK_M - 1) / (2 * BLOCK_M), nkb = (K + BLOCK_K - 1) / BLOCK_K;
     const int t0 = (M + kSwapMax - 1) / kSwapMax;

@@ -614,6 +614,10 @@ int gated_scan(const ScanArgs& a, SeqPos pos, cudaStream_t s) {
                                          (size_t)TT * cols);
     if (smem > 200 * 1024) return -3;
     count_launch();
+    // A scan of more than 8 tokens is long, with about one CTA per SM: chained, the CTAs go two to an SM where the kernel in front has left room.
+    // Four layers, 24 and 31 rows behind 200 tokens: 1.29 | 1.18 and 1.46 | 1.34 ms chained | not (two rotated recurrences), 0.59 | 0.56 and
+    // 0.68 | 0.60 (three state-space layers); 8 rows the same either way.
+    if (a.S > 8) chain_break();
 #define LCC_SCAN(T, V)                                                                                            \
     do {                                                                                                          \
         if (smem > 48 * 1024) cudaFuncSetAttribute(gated_scan_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
