@@ -6,7 +6,40 @@
 #include "launch.h"
 #include "ops.h"
 
+#include <deque>
+#include <mutex>
+
 using lcc::bf16;
+
+namespace {
+
+// Fault words of the contexts, in mapped host memory that every device sees. Allocating such memory waits for whatever the GPU is doing (a
+// context beside running work took 340 ms for 3), so a page is taken once and its words go round: the one given back last is handed out last,
+// 1024 contexts later, when no kernel of its former owner can be under way. Pages stay for the life of the process (one per 1024 live contexts).
+std::mutex g_words_mu;
+std::deque<int*>& words() {
+    static auto* w = new std::deque<int*>;
+    return *w;
+}
+int* take_fault_word() {
+    std::lock_guard<std::mutex> lock(g_words_mu);
+    if (words().empty()) {
+        int* page = nullptr;
+        constexpr int n = 1024;
+        if (cudaHostAlloc((void**)&page, n * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+        for (int i = 0; i < n; ++i) words().push_back(page + i);
+    }
+    int* w = words().front();
+    words().pop_front();
+    *w = 0;
+    return w;
+}
+void give_fault_word(int* w) {
+    std::lock_guard<std::mutex> lock(g_words_mu);
+    words().push_back(w);
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -23,18 +56,17 @@ lcc_ctx* lcc_create(int device) {
     c->device = device;
     c->num_sms = prop.multiProcessorCount;
     c->err[0] = 0;
-    c->fault = nullptr;
-    if (cudaHostAlloc((void**)&c->fault, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    c->fault = take_fault_word();
+    if (!c->fault) {
         delete c;
         return nullptr;
     }
-    *c->fault = 0;
     return c;
 }
 
 void lcc_destroy(lcc_ctx* ctx) {
     if (!ctx) return;
-    cudaFreeHost(ctx->fault);
+    give_fault_word(ctx->fault);
     delete ctx;
 }
 

@@ -196,7 +196,9 @@ def test_gemm_swapped_wait_that_runs_out(epi, splits):
         ctx.check_fault()
     with pytest.raises(A.LiveCCNativeError, match="gave up"):
         ctx.gemm(a, b)
+    del ctx
     other = A.Context(0)
+    other.check_fault()
     assert torch.equal(other.gemm_form(a, b, 2, 128, splits), other.gemm_form(a, b, 0, 128))
     other.check_fault()
 

@@ -486,3 +486,21 @@ def test_attn_decode_splits_merged_in_clusters(ctx, kv_len, nsplit, Hq, Hkv):
     rep = Hq // Hkv
     kr, vr = (x[:, None].expand(Hkv, rep, kv_len + 1, 128).reshape(Hq, kv_len + 1, 128) for x in (kc, vc))
     _attn_close(outs[0], _attn_ref_fp32(q_ref, kr, vr, None, 128 ** -0.5).transpose(0, 1).reshape(Hq * 128), "attn_decode")
+
+
+def test_a_context_does_not_wait_for_the_gpu():
+    """A context beside running work: nothing of its creation or its end synchronises (some 300 ms of products lie in front)."""
+    import time
+
+    A.Context(0)          # (the first one of a process may)
+    x = torch.randn((8192, 8192), device="cuda")
+    x @ x
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    for _ in range(20):
+        x = torch.tanh(x @ x)
+    done.record()
+    for _ in range(3):
+        A.Context(0)
+    assert not done.query()
+    torch.cuda.synchronize()
