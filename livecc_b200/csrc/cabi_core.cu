@@ -26,7 +26,10 @@ int* take_fault_word() {
     if (words().empty()) {
         int* page = nullptr;
         constexpr int n = 1024;
-        if (cudaHostAlloc((void**)&page, n * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+        if (cudaHostAlloc((void**)&page, n * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;   // (no pinned memory to be had: a lost signal then shows as NaN only)
+        }
         for (int i = 0; i < n; ++i) words().push_back(page + i);
     }
     int* w = words().front();
@@ -35,6 +38,7 @@ int* take_fault_word() {
     return w;
 }
 void give_fault_word(int* w) {
+    if (!w) return;
     std::lock_guard<std::mutex> lock(g_words_mu);
     words().push_back(w);
 }
@@ -57,10 +61,6 @@ lcc_ctx* lcc_create(int device) {
     c->num_sms = prop.multiProcessorCount;
     c->err[0] = 0;
     c->fault = take_fault_word();
-    if (!c->fault) {
-        delete c;
-        return nullptr;
-    }
     return c;
 }
 
