@@ -55,7 +55,7 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
 // layers) and 4.86 for 5.14 (routed, two layers), one step launched by the host 0.32 ms for 0.38 and 0.33 for 0.36 (four layers each).
 // Kernels of few and large CTAs (prompt attention: one or two per SM) stay outside: chained, their CTAs go where there is room while the
 // kernel in front still holds the other SMs, and stay there two to an SM. 281 rows behind 4000 tokens of four layers with distance tables
-// took 2.60 ms unchained, 2.76 with every kernel chained. (An ordinary kernel of a scope lets the one behind it in when it is complete.)
+// took 2.59 ms unchained, 2.76 with every kernel chained, 2.52 now. (An ordinary kernel of a scope lets the one behind it in when it is complete.)
 // The first launch of a scope and the one after chain_break() (behind a copy, a fork or a join with another stream) are ordinary: whatever
 // was enqueued before is complete when they start. Outside a scope every launch is.
 enum class Chain { off, broken, on };
