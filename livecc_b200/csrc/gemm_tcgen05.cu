@@ -834,6 +834,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         // ===================== Epilogue (both CTAs, own 128 weight rows) =====================
         const int q = warp & 3, half = (warp - 4) >> 2;   // TMEM lane quarter; every other chunk of 32 activation rows
         const int chunks = cfg.bm >> 5;
+        bool lost = false;
         uint32_t acc_phase = 0;
         for (int unit = cluster; unit < units; unit += num_clusters) {
             const int m0 = (unit % m_tiles) * cfg.bm;
@@ -854,7 +855,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             int c = 0;
             while (c < chunks && !mine(c)) ++c;
             if (SwapEpi<EPI>::kResidual && c < chunks) fetch(c);
-            bool lost = !warp_wait_for(tmem_full, acc_phase, g);
+            lost = !warp_wait_for(tmem_full, acc_phase, g) || lost;   // (behind a phase that never ended the next one's parity reads as past)
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
             float* red = reinterpret_cast<float*>(smem) + q * 32 + lane;   // [chunk][32 columns][128 weight rows]: over the drained ring

@@ -175,13 +175,13 @@ def test_gemm_swapped_form(ctx, M, N, K, width, splits, epi, limit):
     assert torch.equal(ctx.gemm_form(a, b, 2, width, splits, **kw), ctx.gemm_form(a, b, 0, 128, **kw))
 
 
-@pytest.mark.parametrize("splits", [1, 2, 3])
+@pytest.mark.parametrize("N,K,splits", [(544, 65536, 1), (544, 65536, 2), (544, 65536, 3), (20512, 8192, 1)])
 @pytest.mark.parametrize("epi", [A.EPI_NONE, A.EPI_RESIDUAL, A.EPI_SWIGLU, 8, A.EPI_CLAMP_GLU])
-def test_gemm_swapped_wait_that_runs_out(epi, splits):
-    """A limit of 1 us on waits for sums that take some 100 us: the kernel ends, every value it stores is NaN (also where the activation would
-    turn a NaN into a number), the context says so from then on, and others go on."""
+def test_gemm_swapped_wait_that_runs_out(epi, N, K, splits):
+    """A limit of 1 us on waits for sums that take 50 us and more: the kernel ends, every value it stores is NaN (also where the activation would
+    turn a NaN into a number, and in a cluster's second tile), the context says so from then on, and others go on."""
     ctx = A.Context(0)
-    M, N, K = 97, 544, 65536
+    M = 97
     a, b = _ints((M, K), -1, 1, 48), _ints((N, K), -1, 1, 49)
     out = torch.zeros((M, N // 2 if epi in (A.EPI_SWIGLU, A.EPI_CLAMP_GLU) else N), dtype=torch.bfloat16, device="cuda")
     res = _ints((M, N), -8, 8, 50) if epi == A.EPI_RESIDUAL else None
