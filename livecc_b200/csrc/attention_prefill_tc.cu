@@ -345,11 +345,19 @@ int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, con
     const int ctas = q_tiles * Hkv;
     const int kv_tiles = (past + S + BN - 1) / BN;
     int nsplit = 1;
-    // two CTAs per SM: split the KV range until those places are taken, with at least 8 tiles of work per split (281 rows: 4 splits; 24
-    // rows over 64 k keys: 32). Partials that don't fit into the caller's scratch mean fewer splits.
+    // Key splits, up to two CTAs per SM, with at least 8 tiles per split and partials that fit into the caller's scratch. A tile takes 0.8 us
+    // with one CTA per SM and 1.15 with two; the partials cost a launch of 3.5 us and are written and read once. (281 rows over 4 k keys: 4
+    // splits; 24 rows over 64 k: 32.) Filling the places whatever the range is cost 400 to 640 rows behind 600 to 1500 tokens up to a quarter:
+    // 400 and 600 rows behind 600 | 1000 | 3000 tokens 17.4 | 22.3 | 47.5 and 20.1 | 24.6 | 50.3 us unsplit, 21.7 | 25.4 | 34.4 and 25.6 | 28.6 |
+    // 45.8 with every place taken.
     if (part_o && part_ml && ((uintptr_t)part_o % 16) == 0 && ((uintptr_t)part_ml % 8) == 0) {
-        nsplit = std::max(1, std::min({2 * num_sms / ctas, MAX_SPLIT, kv_tiles / 8}));
-        nsplit = std::max(1, (int)std::min((size_t)nsplit, part_capacity_rows / ((size_t)Hkv * S * G)));
+        const size_t rows = (size_t)Hkv * S * G;
+        const int most = (int)std::min((size_t)std::min({2 * num_sms / ctas, MAX_SPLIT, kv_tiles / 8}), part_capacity_rows / rows);
+        double best = 0.8 * kv_tiles;   // (more CTAs than SMs are never split)
+        for (int n = 2; n <= most; ++n) {
+            const double us = (double)kv_tiles / n * (ctas * n > num_sms ? 1.15 : 0.8) + 3.5 + (double)rows * n * 1024 / 6.5e6;
+            if (us < best) { best = us; nsplit = n; }
+        }
     }
     CUtensorMap tq, tk, tv;
     if (make_tmap_bf16_3d_sw128(&tq, q, D, Hq, S, D, q_ld, G, PT)) return -10;
