@@ -268,17 +268,30 @@ int lcc_vit_forward_frames(lcc_model* m, const uint8_t* frames, int T, int H, in
 int lcc_prefill(lcc_model* m, const lcc_stream_state* st, const int64_t* ids, const int32_t* pos3, int S,
                 int past, const void* video_embeds, int n_video_rows, const lcc_sampling* sp, int slot, lcc_stream_t stream);
 
+/* The same for the new tokens of up to 8 streams in one pass, so that every weight byte is read once for all of them: stream b gets slot
+ * first_slot + b. States share one page pool; the workspace holds the sum of the S. Sums are taken in the order that the
+ * number of rows calls for, so a stream's last bits may differ from those of lcc_prefill. */
+typedef struct {
+    lcc_stream_state st;
+    const int64_t* ids;
+    const int32_t* pos3;
+    int32_t S, past;
+    const void* video_embeds;
+    int32_t n_video_rows;
+} lcc_prefill_request;
+int lcc_prefill_batch(lcc_model* m, const lcc_prefill_request* requests, int n_streams, const lcc_sampling* sp, int first_slot, lcc_stream_t stream);
+
 /* n_steps x (one-token forward + token selection) (the loop body of _sample, gen/utils.py:2743-2805).
  * No-ops once scalars[LCC_SC_FINISHED] is set. Capturable in a CUDA graph. nsplit: KV splits (1..64). */
 int lcc_decode_steps(lcc_model* m, const lcc_stream_state* st, int n_steps, int nsplit, const lcc_sampling* sp,
                      lcc_stream_t stream);
 
 /* Batched decode (the reference demo admits 5 concurrent sessions on one model,
- * REF/demo/app.py:178): n_steps x (one persistent kernel = every decoder layer + lm_head for all n_streams <= 8 streams,
- * each weight byte read once per step, then one token selection per stream). states[b] must have been prefilled with
- * slot = b and share one page pool. A stream's ids and logits are bit-identical to decoding it alone (same kernel,
- * same reduction order). lcc_decode_steps (one stream) uses the per-op kernels unless LIVECC_B200_MEGA=1: they are ~5 % faster
- * for a single stream (measured); with 2..8 streams the persistent kernel reads every weight byte once per step for all. */
+ * REF/demo/app.py:178): n_steps x (every decoder layer + lm_head for all n_streams <= 8 streams, each weight byte read once per
+ * step, then one token selection per stream). states[b] must have been prefilled with slot = b and share one page pool. A finished
+ * stream's state stays as it is. LIVECC_B200_MEGA=1 (read at lcc_model_create) runs every step as one persistent kernel, lcc_decode_steps too: a
+ * stream's ids and logits are then bit-identical to decoding it alone. The kernels per operation that run otherwise are faster (see
+ * decode_batch_ops in model.cu); they sum in another order than lcc_decode_steps does. */
 int lcc_decode_batch(lcc_model* m, const lcc_stream_state* states, int n_streams, int n_steps, const lcc_sampling* sp,
                      lcc_stream_t stream);
 /* Test hook: run layers [layer_begin, layer_end) and the phases in phase_mask (1 qkv, 2 attention, 4 o_proj,

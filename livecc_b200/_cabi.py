@@ -64,6 +64,12 @@ class StreamState(C.Structure):
                 ("page_table", C.c_void_p), ("scalars", C.c_void_p), ("seq", C.c_void_p)]
 
 
+class PrefillRequest(C.Structure):
+    """lcc_prefill_request"""
+    _fields_ = [("st", StreamState), ("ids", C.c_void_p), ("pos3", C.c_void_p), ("S", C.c_int32), ("past", C.c_int32),
+                ("video_embeds", C.c_void_p), ("n_video_rows", C.c_int32)]
+
+
 class SeqLayer(C.Structure):
     """lcc_seq_layer"""
     _fields_ = [("type", C.c_int32), ("ff", C.c_int32)] + \
@@ -542,6 +548,15 @@ class NativeModel:
         n_rows = video_embeds.shape[0] if video_embeds is not None else 0
         self._call("lcc_prefill", C.byref(st), _ptr(ids), _ptr(pos3), _i(S), _i(past), _ptr(video_embeds), _i(n_rows),
                    C.byref(sampling), _i(slot), Context.stream_ptr())
+
+    def prefill_batch(self, requests, sampling: Sampling, first_slot: int):
+        """requests: list of (StreamState, ids, pos3, S, past, video_embeds) (<= MAX_BATCH); stream b gets slot first_slot + b."""
+        arr = (PrefillRequest * len(requests))()
+        for r, (st, ids, pos3, S, past, video) in zip(arr, requests):
+            r.st, r.ids, r.pos3, r.S, r.past = st, _ptr(ids), _ptr(pos3), int(S), int(past)
+            if video is not None:
+                r.video_embeds, r.n_video_rows = _ptr(video), video.shape[0]
+        self._call("lcc_prefill_batch", arr, _i(len(requests)), C.byref(sampling), _i(first_slot), Context.stream_ptr())
 
     def decode_steps(self, st: StreamState, n_steps, nsplit, sampling: Sampling):
         self._call("lcc_decode_steps", C.byref(st), _i(n_steps), _i(nsplit), C.byref(sampling), Context.stream_ptr())

@@ -15,6 +15,7 @@
 // Softmax statistics are fp32; P is rounded to bf16 before P·V (as the reference does, :370).
 #include <stdlib.h>
 
+#include "../../include/livecc_b200.h"
 #include "common.cuh"
 #include "launch.h"
 #include "mma.cuh"
@@ -492,6 +493,33 @@ int vit_attention(const bf16* qkv, int ld, int64_t n_rows, bf16* out, int o_ld, 
     return launch_flash<80, false, false>(p, grid, s);
 }
 
+int attn_prefill_streams(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const PrefillStreams& ps, int page_size, int Hq, int Hkv, bf16* out,
+                         int o_ld, float* part_o, float* part_ml, size_t part_capacity_rows, int num_sms, int impl, cudaStream_t s) {
+    if (page_size != 64) return -1;
+    if (impl == 0) {
+        const char* e = getenv("LIVECC_B200_PREFILL_ATTN");  // "mma" forces the mma.sync kernel
+        impl = (e && e[0] == 'm') ? 1 : 2;
+    }
+    if (impl == 1) {
+        for (int b = 0; b < ps.n; ++b) {
+            const PrefillStream& st = ps.st[b];
+            if (int r = attn_prefill_paged(q + (size_t)st.row0 * q_ld, q_ld, kc, vc, st.page_table, page_size, Hq, Hkv, st.S, st.past,
+                                           out + (size_t)st.row0 * o_ld, o_ld, part_o, part_ml, part_capacity_rows, num_sms, 1, s))
+                return r;
+        }
+        return 0;
+    }
+    int ns = 1;
+    if (int r = attn_prefill_tc(q, q_ld, kc, vc, ps, Hq, Hkv, out, o_ld, part_o, part_ml, part_capacity_rows, num_sms, &ns, s)) return r;
+    if (ns > 1) {
+        const int G = Hq / Hkv;
+        lcc::count_launch();
+        flash_merge_kernel<<<dim3((ps.rows * G + kMergeRows - 1) / kMergeRows, Hkv), 32 * kMergeRows, 0, s>>>(part_o, part_ml, ns, Hkv, ps.rows * G, G,
+                                                            1.4426950408889634f / sqrtf(128.f), out, o_ld);
+    }
+    return 0;
+}
+
 // Decoder prefill: q rows of the fused qkv buffer (already rotated), K/V in the paged cache
 // (already containing the S new tokens at positions past..past+S-1).
 int attn_prefill_paged(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const int* page_table,
@@ -504,17 +532,10 @@ int attn_prefill_paged(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, 
         impl = (e && e[0] == 'm') ? 1 : 2;
     }
     if (impl == 2) {
-        int ns = 1;
-        if (int r = attn_prefill_tc(q, q_ld, kc, vc, page_table, Hq, Hkv, S, past, out, o_ld, part_o, part_ml,
-                                    part_capacity_rows, num_sms, &ns, s))
-            return r;
-        if (ns > 1) {
-            const int G = Hq / Hkv;
-            lcc::count_launch();
-            flash_merge_kernel<<<dim3((S * G + kMergeRows - 1) / kMergeRows, Hkv), 32 * kMergeRows, 0, s>>>(part_o, part_ml, ns, Hkv, S * G, G,
-                                                                1.4426950408889634f / sqrtf(128.f), out, o_ld);
-        }
-        return 0;
+        PrefillStreams ps{};
+        ps.n = 1; ps.rows = S;
+        ps.st[0].page_table = page_table; ps.st[0].S = S; ps.st[0].past = past;
+        return attn_prefill_streams(q, q_ld, kc, vc, ps, page_size, Hq, Hkv, out, o_ld, part_o, part_ml, part_capacity_rows, num_sms, impl, s);
     }
     FlashParams p{};
     p.q = q; p.q_ld = q_ld; p.kc = kc; p.vc = vc; p.page_table = page_table; p.Hkv = Hkv;
@@ -875,6 +896,28 @@ __global__ void __cluster_dims__(1, 8, 1) __launch_bounds__(128) attn_decode_clu
     attn_decode_role<8>(p, blockIdx.x, blockIdx.y, smem_attn);
 }
 
+// One slice of the grid (z) per stream of a batched step.
+struct DecodeAttnBatchParams {
+    DecodeAttnParams one;
+    AttnStream st[kBatchStreams];
+    int qkv_ld, out_ld;
+};
+__global__ void __cluster_dims__(1, 8, 1) __launch_bounds__(128) attn_decode_batch_kernel(const __grid_constant__ DecodeAttnBatchParams bp) {
+    extern __shared__ __align__(16) uint8_t smem_attn[];
+    const int b = blockIdx.z;
+    DecodeAttnParams p = bp.one;
+    p.qkv += (size_t)b * bp.qkv_ld;
+    p.out += (size_t)b * bp.out_ld;
+    p.page_table = bp.st[b].page_table;
+    p.kv_len = bp.st[b].scalars + LCC_SC_KV_LEN;
+    p.rope_pos = bp.st[b].scalars + LCC_SC_ROPE_POS;
+    p.finished = bp.st[b].scalars + LCC_SC_FINISHED;
+    p.part_o += (size_t)b * 8 * p.Hq * 128;
+    p.part_ml += (size_t)b * 8 * p.Hq * 2;
+    p.counters += b * p.Hkv;
+    attn_decode_role<8>(p, blockIdx.x, blockIdx.y, smem_attn);
+}
+
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -1001,6 +1044,22 @@ int attn_decode(bf16* qkv, bf16* kc, bf16* vc, const int* page_table, int page_s
     count_launch();
     if (launch_kernel(cluster ? attn_decode_cluster_kernel : attn_decode_kernel, dim3(Hkv, nsplit), dim3(128), (size_t)kDecSmem, s, pdl, p) != cudaSuccess) return -3;
     return 0;
+}
+
+int attn_decode_batch(bf16* qkv, int qkv_ld, bf16* kc, bf16* vc, const AttnStream* streams, int B, int page_size, const float* inv_freq,
+                      int Hq, int Hkv, int nsplit, float* part_o, float* part_ml, int* counters, bf16* out, int out_ld, cudaStream_t s) {
+    if (page_size != 64 || Hq % Hkv || Hq / Hkv > 8 || B < 1 || B > kBatchStreams || nsplit < 8 || nsplit > 64 || nsplit % 8) return -1;
+    static SmemAttrOnce once;
+    if (ensure_dyn_smem(once, attn_decode_batch_kernel, kDecSmem)) return -2;
+    DecodeAttnBatchParams bp{};
+    DecodeAttnParams& p = bp.one;
+    p.qkv = qkv; p.kc = kc; p.vc = vc; p.inv_freq = inv_freq; p.Hq = Hq; p.Hkv = Hkv; p.nsplit = nsplit;
+    p.part_o = part_o; p.part_ml = part_ml; p.counters = counters; p.out = out;
+    p.scale_log2 = 1.4426950408889634f / sqrtf(128.f);
+    for (int b = 0; b < B; ++b) bp.st[b] = streams[b];
+    bp.qkv_ld = qkv_ld; bp.out_ld = out_ld;
+    count_launch();
+    return launch_kernel(attn_decode_batch_kernel, dim3(Hkv, nsplit, B), dim3(128), (size_t)kDecSmem, s, false, bp) == cudaSuccess ? 0 : -3;
 }
 
 // Fused attention + o_proj launch (see attn_oproj_kernel). sync: device int[2], zero-initialised once.

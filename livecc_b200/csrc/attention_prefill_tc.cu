@@ -45,12 +45,12 @@ constexpr float RESCALE_THRESHOLD = 8.f;
 struct PrefillTcParams {
     bf16* out;
     int o_ld;
-    const int* page_table;
-    int Hkv, G, PT, S, past;
+    int Hkv, G, PT;
     float scale_log2;
     int nsplit;
-    float* part_o;   // [nsplit, Hkv, S*G, 128] unnormalised fp32
-    float* part_ml;  // [nsplit, Hkv, S*G, 2]    (raw max, sum)
+    float* part_o;   // [nsplit, Hkv, rows*G, 128] unnormalised fp32
+    float* part_ml;  // [nsplit, Hkv, rows*G, 2]    (raw max, sum)
+    PrefillStreams ps;
 };
 
 __device__ __forceinline__ float ex2_ftz_p(float x) {
@@ -61,20 +61,21 @@ __device__ __forceinline__ float ex2_ftz_p(float x) {
 
 __global__ void __launch_bounds__(192, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                       const __grid_constant__ CUtensorMap tmap_v, PrefillTcParams p) {
+                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ PrefillTcParams p) {
     using namespace ptc;
-    const int kvh = blockIdx.y, split = blockIdx.z;
-    const int pos0 = blockIdx.x * p.PT;
-    if (pos0 >= p.S) return;
-    const int npos = min(p.PT, p.S - pos0);
+    const PrefillStream& st = p.ps.st[blockIdx.z / p.nsplit];
+    const int kvh = blockIdx.y, split = blockIdx.z % p.nsplit;
+    const int pos0 = blockIdx.x * p.PT, S = st.S, past = st.past;
+    if (pos0 >= S) return;
+    const int npos = min(p.PT, S - pos0);
     const int rows_used = npos * p.G;
-    const int rows_total = p.S * p.G;
-    const int row_base = pos0 * p.G;  // packed row index of this tile's row 0
+    const int rows_total = p.ps.rows * p.G;
+    const int row_base = (st.row0 + pos0) * p.G;  // packed row index of this tile's row 0
     // KV tiles this CTA needs: keys 0 .. past + last position (causal), restricted to its split
-    const int n_tiles = (p.past + pos0 + npos + BN - 1) / BN;
+    const int n_tiles = (past + pos0 + npos + BN - 1) / BN;
     int tile_lo = 0, tile_hi = n_tiles;
     if (p.nsplit > 1) {
-        const int tiles_total = (p.past + p.S + BN - 1) / BN;
+        const int tiles_total = (past + S + BN - 1) / BN;
         const int tps = (tiles_total + p.nsplit - 1) / p.nsplit;
         tile_lo = split * tps;
         tile_hi = min(n_tiles, tile_lo + tps);
@@ -132,14 +133,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     if (warp == 0) {
         // ===================== TMA producer =====================
         if (lane == 0) {
-            // the box is always (64, G, PT): rows beyond S are zero-filled but still counted
+            // the box is always (64, G, PT): rows beyond the stream's are the next one's, or zero-filled but still counted; nothing of them is kept
             mbar_arrive_expect_tx(q_full, 2u * 64u * (uint32_t)p.G * (uint32_t)p.PT * 2u);
-            tma_load_3d(smem + OFF_Q, &tmap_q, q_full, 0, kvh * p.G, pos0);
-            tma_load_3d(smem + OFF_Q + Q_ATOM_BYTES, &tmap_q, q_full, 64, kvh * p.G, pos0);
+            tma_load_3d(smem + OFF_Q, &tmap_q, q_full, 0, kvh * p.G, st.row0 + pos0);
+            tma_load_3d(smem + OFF_Q + Q_ATOM_BYTES, &tmap_q, q_full, 64, kvh * p.G, st.row0 + pos0);
+            const int* page_table = st.page_table;
             for (int i = 0; i < T; ++i) {
                 const int st = i % STAGES;
                 const uint32_t free = ((i / STAGES) & 1) ^ 1;
-                const int page = p.page_table[tile_lo + i];
+                const int page = page_table[tile_lo + i];
                 const int row = (page * p.Hkv + kvh) * BN;
                 uint8_t* sk = smem + OFF_K + st * KV_BYTES;
                 uint8_t* sv = smem + OFF_V + st * KV_BYTES;
@@ -206,7 +208,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         const bool row_ok = row < rows_used;
         const int rpos = row / p.G, rg = row - rpos * p.G;
-        const int lim = row_ok ? p.past + pos0 + rpos : -1;  // last visible key index; invalid rows see nothing
+        const int lim = row_ok ? past + pos0 + rpos : -1;  // last visible key index; invalid rows see nothing
         float m_used = -INFINITY, l = 0.f;
         for (int i = 0; i < T; ++i) {
             const int b = i & 1;
@@ -303,7 +305,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             }
         } else {
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            bf16* dst = p.out + (size_t)(pos0 + rpos) * p.o_ld + (size_t)(kvh * p.G + rg) * D;
+            bf16* dst = p.out + (size_t)(st.row0 + pos0 + rpos) * p.o_ld + (size_t)(kvh * p.G + rg) * D;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 uint32_t o32[32];
@@ -334,16 +336,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 
 // q: rotated rows of the fused qkv buffer [S, >= Hq*128] (row stride q_ld); kc/vc: one layer of the page pool
 // [pages, Hkv, 64, 128].  Returns the split count used through *nsplit_out (the caller merges when > 1).
-int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const int* page_table, int Hq, int Hkv,
-                    int S, int past, bf16* out, int o_ld, float* part_o, float* part_ml, size_t part_capacity_rows,
-                    int num_sms, int* nsplit_out, cudaStream_t s) {
+int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const PrefillStreams& ps, int Hq, int Hkv, bf16* out, int o_ld,
+                    float* part_o, float* part_ml, size_t part_capacity_rows, int num_sms, int* nsplit_out, cudaStream_t s) {
     using namespace ptc;
     const int G = Hq / Hkv;
     if (G < 1 || G > 128 || Hq % Hkv || (q_ld % 8) || (o_ld % 8)) return -1;
     const int PT = BM / G;
-    const int q_tiles = (S + PT - 1) / PT;
-    const int ctas = q_tiles * Hkv;
-    const int kv_tiles = (past + S + BN - 1) / BN;
+    int q_tiles = 0, ctas = 0, kv_tiles = 0;   // of the longest stream, of all, of the longest range
+    for (int b = 0; b < ps.n; ++b) {
+        const int t = (ps.st[b].S + PT - 1) / PT;
+        q_tiles = std::max(q_tiles, t);
+        ctas += t * Hkv;
+        kv_tiles = std::max(kv_tiles, (ps.st[b].past + ps.st[b].S + BN - 1) / BN);
+    }
     int nsplit = 1;
     // Key splits, up to two CTAs per SM, with at least 8 tiles per split and partials that fit into the caller's scratch. A tile takes 0.8 us
     // with one CTA per SM and 1.15 with two; the partials cost a launch of 3.5 us and are written and read once. (281 rows over 4 k keys: 4
@@ -351,7 +356,7 @@ int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, con
     // 400 and 600 rows behind 600 | 1000 | 3000 tokens 17.4 | 22.3 | 47.5 and 20.1 | 24.6 | 50.3 us unsplit, 21.7 | 25.4 | 34.4 and 25.6 | 28.6 |
     // 45.8 with every place taken.
     if (part_o && part_ml && ((uintptr_t)part_o % 16) == 0 && ((uintptr_t)part_ml % 8) == 0) {
-        const size_t rows = (size_t)Hkv * S * G;
+        const size_t rows = (size_t)Hkv * ps.rows * G;
         const int most = (int)std::min((size_t)std::min({2 * num_sms / ctas, MAX_SPLIT, kv_tiles / 8}), part_capacity_rows / rows);
         double best = 0.8 * kv_tiles;   // (more CTAs than SMs are never split)
         for (int n = 2; n <= most; ++n) {
@@ -360,15 +365,15 @@ int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, con
         }
     }
     CUtensorMap tq, tk, tv;
-    if (make_tmap_bf16_3d_sw128(&tq, q, D, Hq, S, D, q_ld, G, PT)) return -10;
+    if (make_tmap_bf16_3d_sw128(&tq, q, D, Hq, ps.rows, D, q_ld, G, PT)) return -10;
     const int64_t pool_rows = (int64_t)1 << 31;  // page ids come from the page table; no meaningful row bound here
     if (make_tmap_bf16_2d_box(&tk, kc, pool_rows, D, D, 64, BN, false)) return -11;
     if (make_tmap_bf16_2d_box(&tv, vc, pool_rows, D, D, 64, BN, false)) return -11;
     static SmemAttrOnce once;
     if (ensure_dyn_smem(once, attn_prefill_tc_kernel, SMEM_BYTES)) return -12;
-    PrefillTcParams p{out, o_ld, page_table, Hkv, G, PT, S, past, 1.4426950408889634f / sqrtf((float)D), nsplit, part_o, part_ml};
+    const PrefillTcParams p{out, o_ld, Hkv, G, PT, 1.4426950408889634f / sqrtf((float)D), nsplit, part_o, part_ml, ps};
     lcc::count_launch();
-    attn_prefill_tc_kernel<<<dim3(q_tiles, Hkv, nsplit), 192, SMEM_BYTES, s>>>(tq, tk, tv, p);
+    attn_prefill_tc_kernel<<<dim3(q_tiles, Hkv, nsplit * ps.n), 192, SMEM_BYTES, s>>>(tq, tk, tv, p);
     *nsplit_out = nsplit;
     return 0;
 }

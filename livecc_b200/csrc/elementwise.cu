@@ -357,8 +357,12 @@ int vit_rope_apply(bf16* qkv, int ld, const float* cos_t, const float* sin_t, in
 // out[s] = is_video(ids[s]) ? video_embeds[rank of s among video tokens] : table[ids[s]].
 // Kernel 1 (single CTA) computes the exclusive rank by a block scan; kernel 2 copies rows.
 // ------------------------------------------------------------------------------------------
-__global__ void video_rank_kernel(const int64_t* __restrict__ ids, int S, int64_t video_id,
-                                  int* __restrict__ rank, int* __restrict__ total) {
+__global__ void video_rank_kernel(const __grid_constant__ PrefillStreams ps, int64_t video_id, int* __restrict__ rank) {
+    const PrefillStream& st = ps.st[blockIdx.x];
+    const int64_t* __restrict__ ids = st.ids;
+    const int S = st.S;
+    if (!st.video) video_id = -1;
+    rank += st.row0;
     __shared__ int warp_tot[32];
     __shared__ int carry;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -391,16 +395,17 @@ __global__ void video_rank_kernel(const int64_t* __restrict__ ids, int S, int64_
         if (threadIdx.x == 0) carry += warp_tot[(blockDim.x >> 5) - 1];
         __syncthreads();
     }
-    if (threadIdx.x == 0 && total) *total = carry;
+    if (threadIdx.x == 0 && st.total_video) *st.total_video = carry;
 }
 
-__global__ void embed_gather_kernel(const int64_t* __restrict__ ids, const int* __restrict__ rank,
-                                    const bf16* __restrict__ table, const bf16* __restrict__ video,
-                                    bf16* __restrict__ out, int S, int H, int64_t vocab, int n_video_rows) {
+__global__ void embed_gather_kernel(const __grid_constant__ PrefillStreams ps, const int* __restrict__ rank, const bf16* __restrict__ table,
+                                    bf16* __restrict__ out, int H, int64_t vocab) {
     const int row = blockIdx.x;
-    if (row >= S) return;
+    const PrefillStream& st = ps.st[ps.of_row(row)];
+    const bf16* __restrict__ video = st.video;
+    const int n_video_rows = video ? st.n_video : 0;
     const int rk = rank[row];
-    int64_t id = ids[row];
+    int64_t id = st.ids[row - st.row0];
     if (id < 0) id = 0;
     if (id >= vocab) id = vocab - 1;
     // A placeholder beyond the last feature row (more <|video_pad|> ids than ViT rows) keeps its text embedding:
@@ -414,10 +419,18 @@ __global__ void embed_gather_kernel(const int64_t* __restrict__ ids, const int* 
 int embed_gather(const int64_t* ids, const bf16* table, const bf16* video, int n_video_rows, int64_t video_id, bf16* out,
                  int* rank_ws, int* total_video, int S, int H, int64_t vocab, cudaStream_t s) {
     if (S <= 0) return 0;
+    PrefillStreams ps{};
+    ps.n = 1; ps.rows = S;
+    ps.st[0].ids = ids; ps.st[0].video = video; ps.st[0].n_video = n_video_rows; ps.st[0].total_video = total_video; ps.st[0].S = S;
+    return embed_gather_streams(ps, table, video_id, out, rank_ws, H, vocab, s);
+}
+
+int embed_gather_streams(const PrefillStreams& ps, const bf16* table, int64_t video_id, bf16* out, int* rank_ws, int H, int64_t vocab, cudaStream_t s) {
     if (H % 8) return -1;
-    { lcc::count_launch(); video_rank_kernel<<<1, 1024, 0, s>>>(ids, S, video ? video_id : (int64_t)-1, rank_ws, total_video); }
     lcc::count_launch();
-    embed_gather_kernel<<<S, 128, 0, s>>>(ids, rank_ws, table, video, out, S, H, vocab, video ? n_video_rows : 0);
+    video_rank_kernel<<<ps.n, 1024, 0, s>>>(ps, video_id, rank_ws);
+    lcc::count_launch();
+    embed_gather_kernel<<<ps.rows, 128, 0, s>>>(ps, rank_ws, table, out, H, vocab);
     return 0;
 }
 
@@ -445,17 +458,20 @@ __device__ __forceinline__ void mrope_cos_sin(int j /*0..63*/, int pt, int ph, i
 // One warp per (token, slice of kMropeHeads heads): the token's 64 angles are the same for every head, so a lane forms its two once and
 // walks the slice with them. (A warp per head formed them 36 times per token: 4.5 us for 281 tokens and 23.4 for 2090, back to back; now 3.7 and 13.0.)
 constexpr int kMropeHeads = 9;
-__global__ void __launch_bounds__(256) mrope_kv_write_kernel(bf16* __restrict__ qkv, int ld, const int* __restrict__ pos3, int S,
+__global__ void __launch_bounds__(256) mrope_kv_write_kernel(bf16* __restrict__ qkv, int ld, const __grid_constant__ PrefillStreams ps,
                                       const float* __restrict__ inv_freq, MropeSections sec, int Hq, int Hkv,
-                                      bf16* __restrict__ kc, bf16* __restrict__ vc,
-                                      const int* __restrict__ page_table, int page_size, int kv_start) {
+                                      bf16* __restrict__ kc, bf16* __restrict__ vc, int page_size) {
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int heads_total = Hq + 2 * Hkv, slices = (heads_total + kMropeHeads - 1) / kMropeHeads;
-    if (gw >= S * slices) return;
-    const int s_idx = gw / slices, h0 = gw % slices * kMropeHeads, h1 = min(heads_total, h0 + kMropeHeads);
-    bf16* row = qkv + (size_t)s_idx * ld;
-    const int tok = kv_start + s_idx;
+    if (gw >= ps.rows * slices) return;
+    const int h0 = gw % slices * kMropeHeads, h1 = min(heads_total, h0 + kMropeHeads);
+    bf16* row = qkv + (size_t)(gw / slices) * ld;
+    const PrefillStream& st = ps.st[ps.of_row(gw / slices)];
+    const int s_idx = gw / slices - st.row0, S = st.S;
+    const int* __restrict__ pos3 = st.pos3;
+    const int* __restrict__ page_table = st.page_table;
+    const int tok = st.past + s_idx;
     const int page = page_table[tok / page_size], slot = tok % page_size;
     // lane owns rotation pairs j = 2*lane, 2*lane+1  (x[j], x[j+64])
     uint32_t lo[kMropeHeads], hi[kMropeHeads];
@@ -500,12 +516,20 @@ int mrope_kv_write(bf16* qkv, int ld, const int* pos3, int S, const float* inv_f
                    int Hq, int Hkv, bf16* kc, bf16* vc, const int* page_table, int page_size, int kv_start,
                    cudaStream_t s) {
     if (S <= 0) return 0;
-    const int64_t warps = (int64_t)S * ((Hq + 2 * Hkv + kMropeHeads - 1) / kMropeHeads);
+    PrefillStreams ps{};
+    ps.n = 1; ps.rows = S;
+    ps.st[0].pos3 = pos3; ps.st[0].page_table = page_table; ps.st[0].S = S; ps.st[0].past = kv_start;
+    return mrope_kv_write_streams(qkv, ld, ps, inv_freq, sec_t, sec_h, Hq, Hkv, kc, vc, page_size, s);
+}
+
+int mrope_kv_write_streams(bf16* qkv, int ld, const PrefillStreams& ps, const float* inv_freq, int sec_t, int sec_h, int Hq, int Hkv, bf16* kc,
+                           bf16* vc, int page_size, cudaStream_t s) {
+    const int64_t warps = (int64_t)ps.rows * ((Hq + 2 * Hkv + kMropeHeads - 1) / kMropeHeads);
     const int wpb = 8;
     MropeSections sec{sec_t, sec_h};
     lcc::count_launch();
     mrope_kv_write_kernel<<<(int)((warps + wpb - 1) / wpb), wpb * 32, 0, s>>>(
-        qkv, ld, pos3, S, inv_freq, sec, Hq, Hkv, kc, vc, page_table, page_size, kv_start);
+        qkv, ld, ps, inv_freq, sec, Hq, Hkv, kc, vc, page_size);
     return 0;
 }
 

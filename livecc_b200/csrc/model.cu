@@ -46,6 +46,7 @@ struct WsLayout {
     size_t vx, vh, vn, vqkv, vattn, vmlp, vcos, vsin, vcu;  // ViT
     size_t hid, normed, qkv, attn, act, rank, pf_part_o, pf_part_ml, pf_splitk;  // prefill
     size_t h1, qkv1, attn1, act1, logits_raw, logits_proc, part_o, part_ml, attn_cnt;  // decode (8 stream rows each)
+    size_t normed1, batch_cnt;  // batched decode: normalised rows, arrival counters
     size_t mg_part_o, mg_part_ml, mg_cnt, mg_tmaps, mg_layers, mg_trace;  // persistent decode kernel
     size_t total;
 };
@@ -88,6 +89,8 @@ WsLayout make_layout(const lcc_model_config& c, int NP, int NT) {
     L.part_o = take((size_t)kMaxSplit * c.q_heads * 128 * 4);
     L.part_ml = take((size_t)kMaxSplit * c.q_heads * 2 * 4);
     L.attn_cnt = take(64 * 4);
+    L.normed1 = take((size_t)lcc::kBatchStreams * c.hidden * 2);
+    L.batch_cnt = take((size_t)lcc::kBatchStreams * c.kv_heads * 4);
     L.mg_part_o = take((size_t)lcc::MG_MAXB * c.kv_heads * lcc::MG_MAX_ITEMS * 8 * 128 * 4);
     L.mg_part_ml = take((size_t)lcc::MG_MAXB * c.kv_heads * lcc::MG_MAX_ITEMS * 8 * 2 * 4);
     L.mg_cnt = take(128 * 4);  // [0, 8*kv_heads): pair counters; [96]: grid barrier; [97]: sticky error flag
@@ -264,13 +267,24 @@ int lcc_vit_forward_frames(lcc_model* m, const uint8_t* frames, int T, int H, in
     return vit_forward_impl(m, nullptr, frames, T, (T + 1) / 2, H / 14, W / 14, mean255, std255, out, stream);
 }
 
-int lcc_prefill(lcc_model* m, const lcc_stream_state* st, const int64_t* ids, const int32_t* pos3, int S,
-                int past, const void* video_embeds, int n_video_rows, const lcc_sampling* sp, int slot, lcc_stream_t stream) {
-    if (!m || !st || !sp) return -1;
-    if (slot < 0 || slot >= lcc::MG_MAXB) LCC_FAIL(m->ctx, -2, "lcc_prefill: slot must be in [0,%d)", lcc::MG_MAXB);
+static int prefill_impl(lcc_model* m, const lcc_prefill_request* rq, int n, const lcc_sampling* sp, int slot, lcc_stream_t stream) {
     const lcc_model_config& c = m->cfg;
     cudaStream_t s = (cudaStream_t)stream;
-    if (S <= 0) LCC_FAIL(m->ctx, -2, "lcc_prefill: S must be positive");
+    if (slot < 0 || n < 1 || slot + n > lcc::MG_MAXB) LCC_FAIL(m->ctx, -2, "lcc_prefill: slots must be in [0,%d)", lcc::MG_MAXB);
+    lcc::PrefillStreams ps{};
+    ps.n = n;
+    int last[lcc::kBatchStreams];
+    for (int b = 0; b < n; ++b) {
+        const lcc_prefill_request& r = rq[b];
+        if (r.S <= 0) LCC_FAIL(m->ctx, -2, "lcc_prefill: S must be positive");
+        if (r.st.k_pool != rq[0].st.k_pool || r.st.v_pool != rq[0].st.v_pool || r.st.layer_stride != rq[0].st.layer_stride)
+            LCC_FAIL(m->ctx, -5, "lcc_prefill_batch: streams must share one page pool");
+        ps.st[b] = {r.ids, r.pos3, r.st.page_table, (const bf16*)r.video_embeds, r.st.scalars + LCC_SC_VIDEO_TOKENS, r.n_video_rows, r.S, r.past, ps.rows};
+        ps.rows += r.S;
+        last[b] = ps.rows - 1;
+    }
+    const int S = ps.rows;
+    const lcc_stream_state* st = &rq[0].st;
     WsLayout L;
     if (get_layout(m, 0, S, &L)) LCC_FAIL(m->ctx, -3, "lcc_prefill: no workspace bound or too small for %d tokens", S);
     uint8_t* ws = m->ws;
@@ -280,32 +294,55 @@ int lcc_prefill(lcc_model* m, const lcc_stream_state* st, const int64_t* ids, co
     void* skw = ws + L.pf_splitk;  // split-K scratch of the small-N projections (opt-in, see gemm_tcgen05.cu::try_splitk)
     const size_t skb = kSplitKRows * (size_t)(qkv_dim > H ? qkv_dim : H) * 4;
 
-    STEP(lcc::embed_gather(ids, (const bf16*)m->w.embed, (const bf16*)video_embeds, n_video_rows, c.video_token_id, hid, rank,
-                           st->scalars + LCC_SC_VIDEO_TOKENS, S, H, c.vocab, s), "embed gather");
+    STEP(lcc::embed_gather_streams(ps, (const bf16*)m->w.embed, c.video_token_id, hid, rank, H, c.vocab, s), "embed gather");
     for (int i = 0; i < c.layers; ++i) {
         const lcc_layer_weights& lw = m->layers[i];
         bf16* kc = (bf16*)st->k_pool + (size_t)i * st->layer_stride;
         bf16* vc = (bf16*)st->v_pool + (size_t)i * st->layer_stride;
         STEP(lcc::rmsnorm(hid, H, (const bf16*)lw.ln1_w, normed, H, S, H, c.rms_eps, s), "input_layernorm");
         STEP(gemm(m, normed, H, lw.qkv_w, H, qkv, qkv_dim, S, qkv_dim, H, lw.qkv_b, nullptr, 0, lcc::EPI_BIAS, s, skw, skb), "qkv proj");
-        STEP(lcc::mrope_kv_write(qkv, qkv_dim, pos3, S, m->w.text_inv_freq, c.mrope_t, c.mrope_h, Hq, Hkv, kc, vc,
-                                 st->page_table, LCC_PAGE_SIZE, past, s), "mrope + kv write");
-        STEP(lcc::attn_prefill_paged(qkv, qkv_dim, kc, vc, st->page_table, LCC_PAGE_SIZE, Hq, Hkv, S, past, attn,
-                                     Hq * 128, (float*)(ws + L.pf_part_o), (float*)(ws + L.pf_part_ml),
-                                     kPrefillSplitRows * (size_t)Hq, m->ctx->num_sms, 0, s), "prefill attention");
+        STEP(lcc::mrope_kv_write_streams(qkv, qkv_dim, ps, m->w.text_inv_freq, c.mrope_t, c.mrope_h, Hq, Hkv, kc, vc, LCC_PAGE_SIZE, s), "mrope + kv write");
+        STEP(lcc::attn_prefill_streams(qkv, qkv_dim, kc, vc, ps, LCC_PAGE_SIZE, Hq, Hkv, attn, Hq * 128, (float*)(ws + L.pf_part_o),
+                                       (float*)(ws + L.pf_part_ml), kPrefillSplitRows * (size_t)Hq, m->ctx->num_sms, 0, s), "prefill attention");
         STEP(gemm(m, attn, Hq * 128, lw.o_w, Hq * 128, hid, H, S, H, Hq * 128, nullptr, hid, H, lcc::EPI_RESIDUAL, s, skw, skb), "o_proj");
         STEP(lcc::rmsnorm(hid, H, (const bf16*)lw.ln2_w, normed, H, S, H, c.rms_eps, s), "post_attention_layernorm");
         STEP(gemm(m, normed, H, lw.gate_up_w, H, act, c.inter, S, 2 * c.inter, H, nullptr, nullptr, 0, lcc::EPI_SWIGLU, s), "gate_up");
         STEP(gemm(m, act, c.inter, lw.down_w, c.inter, hid, H, S, H, c.inter, nullptr, hid, H, lcc::EPI_RESIDUAL, s, skw, skb), "down_proj");
     }
-    // final norm + lm_head on the last position only (logits_to_keep = 1, gen/utils.py:2487-2491)
-    STEP(lcc::gemv_norm_logits((const bf16*)m->w.lm_head, H, hid + (size_t)(S - 1) * H, (const bf16*)m->w.final_norm_w,
-                               c.rms_eps, (float*)(ws + L.logits_raw) + (size_t)slot * c.vocab,
-                               (float*)(ws + L.logits_proc) + (size_t)slot * c.vocab, c.vocab, H,
-                               nullptr, m->ctx->num_sms, false, s), "lm_head");
-    STEP(lcc::sample_greedy(make_sample(m, st, sp, ws, L, 0, slot), s), "token selection");
+    // final norm + lm_head on the last position of each stream only (logits_to_keep = 1, gen/utils.py:2487-2491)
+    float *raw = (float*)(ws + L.logits_raw) + (size_t)slot * c.vocab, *proc = (float*)(ws + L.logits_proc) + (size_t)slot * c.vocab;
+    if (n == 1) {
+        STEP(lcc::gemv_norm_logits((const bf16*)m->w.lm_head, H, hid + (size_t)(S - 1) * H, (const bf16*)m->w.final_norm_w, c.rms_eps, raw, proc, c.vocab, H,
+                                   nullptr, m->ctx->num_sms, false, s), "lm_head");
+        STEP(lcc::sample_greedy(make_sample(m, st, sp, ws, L, 0, slot), s), "token selection");
+    } else {
+        const int* open[lcc::kBatchStreams];
+        lcc::SampleBatch sb{};
+        sb.B = n;
+        for (int b = 0; b < n; ++b) {
+            open[b] = rq[b].st.scalars + LCC_SC_FINISHED;
+            sb.seq[b] = rq[b].st.seq; sb.scalars[b] = rq[b].st.scalars;
+        }
+        STEP(lcc::rmsnorm(hid, H, (const bf16*)m->w.final_norm_w, normed, H, S, H, c.rms_eps, s), "final norm");
+        const lcc::GemvBatch a{(const bf16*)m->w.lm_head, normed, c.vocab, H, H, n, open, last, nullptr, 0};
+        STEP(lcc::gemv_batch_logits(a, raw, proc, c.vocab, s), "lm_head");
+        STEP(lcc::sample_greedy_batch(make_sample(m, nullptr, sp, ws, L, 0, slot), sb, s), "token selection");
+    }
     LCC_CHECK_LAUNCH(m->ctx, "lcc_prefill");
     return 0;
+}
+
+int lcc_prefill(lcc_model* m, const lcc_stream_state* st, const int64_t* ids, const int32_t* pos3, int S,
+                int past, const void* video_embeds, int n_video_rows, const lcc_sampling* sp, int slot, lcc_stream_t stream) {
+    if (!m || !st || !sp) return -1;
+    const lcc_prefill_request r{*st, ids, pos3, S, past, video_embeds, n_video_rows};
+    return prefill_impl(m, &r, 1, sp, slot, stream);
+}
+
+int lcc_prefill_batch(lcc_model* m, const lcc_prefill_request* requests, int n_streams, const lcc_sampling* sp, int first_slot, lcc_stream_t stream) {
+    if (!m || !requests || !sp) return -1;
+    if (n_streams > 1 && !m->mega_ok) LCC_FAIL(m->ctx, -4, "lcc_prefill_batch: model geometry is not supported by the batched kernels");
+    return prefill_impl(m, requests, n_streams, sp, first_slot, stream);
 }
 
 // ---- persistent decode-step kernel (decode_mega.cu) --------------------------------------------------------------
@@ -353,6 +390,57 @@ static int mega_launch(lcc_model* m, const lcc::MegaParams& p, cudaStream_t s) {
     return lcc::decode_mega_launch(p, p.k_pool, p.v_pool, pool_rows, m->ctx->num_sms, s);
 }
 
+// Per-op kernels of a batched step: every weight byte is read once for all streams (gemv_batch.cu), attention is one grid over streams, KV
+// heads and splits. A step of eight streams over 8k tokens each, four layers, takes 0.69 ms; the persistent kernel, whose grid barriers and
+// attention phase leave HBM idle half of the time, took 1.09 (two streams 0.56 for 0.63).
+static int decode_batch_ops(lcc_model* m, const lcc_stream_state* sts, int B, int n_steps, const lcc_sampling* sp, const WsLayout& L, cudaStream_t s) {
+    const lcc_model_config& c = m->cfg;
+    uint8_t* ws = m->ws;
+    for (int b = 1; b < B; ++b)
+        if (sts[b].k_pool != sts[0].k_pool || sts[b].v_pool != sts[0].v_pool || sts[b].layer_stride != sts[0].layer_stride)
+            LCC_FAIL(m->ctx, -5, "lcc_decode_batch: streams must share one page pool");
+    bf16 *h = (bf16*)(ws + L.h1), *qkv = (bf16*)(ws + L.qkv1), *attn = (bf16*)(ws + L.attn1), *act = (bf16*)(ws + L.act1), *normed = (bf16*)(ws + L.normed1);
+    const int H = c.hidden, Hq = c.q_heads, Hkv = c.kv_heads, qkv_dim = (Hq + 2 * Hkv) * 128;
+    lcc::AttnStream st[lcc::kBatchStreams];
+    const int* fin[lcc::kBatchStreams];
+    lcc::SampleBatch sb{};
+    sb.B = B;
+    for (int b = 0; b < B; ++b) {
+        st[b] = {sts[b].page_table, sts[b].scalars};
+        fin[b] = sts[b].scalars + LCC_SC_FINISHED;
+        sb.seq[b] = sts[b].seq; sb.scalars[b] = sts[b].scalars;
+    }
+    int nsplit = 8;   // about two attention CTAs per SM, whatever the caches' lengths (they grow under a captured graph)
+    while (nsplit < kMaxSplit && 2 * nsplit * B * Hkv <= 2 * m->ctx->num_sms) nsplit *= 2;
+    // the head of the next kernel's weights goes into L2 while a kernel's last CTAs run (see gemv.cu)
+    const size_t kPf = 32u << 20;
+    auto ops = [&](const void* W, int N, int K, const bf16* x, const void* next, size_t next_bytes) {
+        return lcc::GemvBatch{(const bf16*)W, x, N, K, K, B, fin, nullptr, next, next_bytes < kPf ? next_bytes : kPf};
+    };
+    for (int step = 0; step < n_steps; ++step) {
+        for (int i = 0; i < c.layers; ++i) {
+            const lcc_layer_weights& lw = m->layers[i];
+            bf16* kc = (bf16*)sts[0].k_pool + (size_t)i * sts[0].layer_stride;
+            bf16* vc = (bf16*)sts[0].v_pool + (size_t)i * sts[0].layer_stride;
+            const bool last = i + 1 == c.layers;
+            STEP(lcc::rmsnorm(h, H, (const bf16*)lw.ln1_w, normed, H, B, H, c.rms_eps, s), "batched decode input_layernorm");
+            STEP(lcc::gemv_batch_bias(ops(lw.qkv_w, qkv_dim, H, normed, lw.o_w, (size_t)H * Hq * 256), (const bf16*)lw.qkv_b, qkv, qkv_dim, s), "batched decode qkv");
+            STEP(lcc::attn_decode_batch(qkv, qkv_dim, kc, vc, st, B, LCC_PAGE_SIZE, m->w.text_inv_freq, Hq, Hkv, nsplit, (float*)(ws + L.part_o),
+                                        (float*)(ws + L.part_ml), (int*)(ws + L.batch_cnt), attn, Hq * 128, s), "batched decode attention");
+            STEP(lcc::gemv_batch_residual(ops(lw.o_w, H, Hq * 128, attn, lw.gate_up_w, (size_t)4 * c.inter * H), h, H, s), "batched decode o_proj");
+            STEP(lcc::rmsnorm(h, H, (const bf16*)lw.ln2_w, normed, H, B, H, c.rms_eps, s), "batched decode post_attention_layernorm");
+            STEP(lcc::gemv_batch_swiglu(ops(lw.gate_up_w, 2 * c.inter, H, normed, lw.down_w, (size_t)2 * c.inter * H), act, c.inter, s), "batched decode gate_up");
+            STEP(lcc::gemv_batch_residual(ops(lw.down_w, H, c.inter, act, last ? m->w.lm_head : m->layers[i + 1].qkv_w,
+                                              last ? (size_t)c.vocab * H * 2 : (size_t)qkv_dim * H * 2), h, H, s), "batched decode down_proj");
+        }
+        STEP(lcc::rmsnorm(h, H, (const bf16*)m->w.final_norm_w, normed, H, B, H, c.rms_eps, s), "batched decode final norm");
+        STEP(lcc::gemv_batch_logits(ops(m->w.lm_head, c.vocab, H, normed, nullptr, 0), (float*)(ws + L.logits_raw), (float*)(ws + L.logits_proc), c.vocab, s), "batched decode lm_head");
+        STEP(lcc::sample_greedy_batch(make_sample(m, nullptr, sp, ws, L, 1), sb, s), "batched token selection");
+    }
+    LCC_CHECK_LAUNCH(m->ctx, "lcc_decode_batch");
+    return 0;
+}
+
 int lcc_decode_batch(lcc_model* m, const lcc_stream_state* states, int n_streams, int n_steps, const lcc_sampling* sp,
                      lcc_stream_t stream) {
     if (!m || !states || !sp) return -1;
@@ -361,6 +449,7 @@ int lcc_decode_batch(lcc_model* m, const lcc_stream_state* states, int n_streams
     WsLayout L;
     if (get_layout(m, 0, 0, &L)) LCC_FAIL(m->ctx, -3, "lcc_decode_batch: no workspace bound");
     cudaStream_t s = (cudaStream_t)stream;
+    if (!m->use_mega) return decode_batch_ops(m, states, n_streams, n_steps, sp, L, s);
     lcc::MegaParams p;
     if (mega_step_params(m, states, n_streams, L, &p)) LCC_FAIL(m->ctx, -5, "lcc_decode_batch: streams must share one page pool");
     lcc::SampleBatch sb{};
@@ -467,7 +556,9 @@ extern "C" int lcc_model_bind_workspace(lcc_model* m, void* ws, size_t ws_bytes,
     m->ws = reinterpret_cast<uint8_t*>(ws);
     m->ws_bytes = ws_bytes;
     // split-KV arrival counters start at zero (the attention kernel re-zeroes them itself)
-    if (cudaMemset(m->ws + make_layout(m->cfg, max_patches, max_tokens).attn_cnt, 0, 64 * 4) != cudaSuccess)
+    const WsLayout L0 = make_layout(m->cfg, max_patches, max_tokens);
+    if (cudaMemset(m->ws + L0.attn_cnt, 0, 64 * 4) != cudaSuccess ||
+        cudaMemset(m->ws + L0.batch_cnt, 0, (size_t)lcc::kBatchStreams * m->cfg.kv_heads * 4) != cudaSuccess)
         LCC_FAIL(m->ctx, -3, "lcc_model_bind_workspace: cudaMemset failed");
     m->cap_patches = max_patches;
     m->cap_tokens = max_tokens;

@@ -21,6 +21,30 @@ int vit_rope_table(float* cos_t, float* sin_t, int t, int h, int w, int merge, i
                    const float* inv_freq, cudaStream_t s);
 int vit_rope_apply(bf16* qkv, int ld, const float* cos_t, const float* sin_t, int N, int heads, int hd,
                    cudaStream_t s);
+// The new tokens of up to 8 streams as the rows of one pass: stream b has rows [row0, row0 + S), its tokens follow `past` cached ones.
+constexpr int kBatchStreams = 8;
+struct PrefillStream {
+    const int64_t* ids;       // [S]
+    const int* pos3;          // [3, S]
+    const int* page_table;
+    const bf16* video;        // feature rows, or null
+    int* total_video;
+    int n_video, S, past, row0;
+};
+struct PrefillStreams {
+    int n, rows;
+    PrefillStream st[kBatchStreams];
+#ifdef __CUDACC__
+    __device__ __forceinline__ int of_row(int row) const {
+        int b = 0;
+        while (b + 1 < n && row >= st[b + 1].row0) ++b;
+        return b;
+    }
+#endif
+};
+int embed_gather_streams(const PrefillStreams& ps, const bf16* table, int64_t video_id, bf16* out, int* rank_ws, int H, int64_t vocab, cudaStream_t s);
+int mrope_kv_write_streams(bf16* qkv, int ld, const PrefillStreams& ps, const float* inv_freq, int sec_t, int sec_h, int Hq, int Hkv, bf16* kc,
+                           bf16* vc, int page_size, cudaStream_t s);
 int embed_gather(const int64_t* ids, const bf16* table, const bf16* video, int n_video_rows, int64_t video_id, bf16* out,
                  int* rank_ws, int* total_video, int S, int H, int64_t vocab, cudaStream_t s);
 int mrope_kv_write(bf16* qkv, int ld, const int* pos3, int S, const float* inv_freq, int sec_t, int sec_h,
@@ -38,13 +62,24 @@ int vit_attention_tc(const bf16* qkv, int ld, int64_t n_rows, bf16* out, int o_l
 int attn_prefill_paged(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const int* page_table,
                        int page_size, int Hq, int Hkv, int S, int past, bf16* out, int o_ld, float* part_o,
                        float* part_ml, size_t part_capacity_rows, int num_sms, int impl, cudaStream_t s);
+// the same for the rows of several streams: one launch, and one merge
+int attn_prefill_streams(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const PrefillStreams& ps, int page_size, int Hq, int Hkv, bf16* out,
+                         int o_ld, float* part_o, float* part_ml, size_t part_capacity_rows, int num_sms, int impl, cudaStream_t s);
 // attention_prefill_tc.cu
-int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const int* page_table, int Hq, int Hkv,
-                    int S, int past, bf16* out, int o_ld, float* part_o, float* part_ml, size_t part_capacity_rows,
-                    int num_sms, int* nsplit_out, cudaStream_t s);
+int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const PrefillStreams& ps, int Hq, int Hkv, bf16* out, int o_ld,
+                    float* part_o, float* part_ml, size_t part_capacity_rows, int num_sms, int* nsplit_out, cudaStream_t s);
 int attn_decode(bf16* qkv, bf16* kc, bf16* vc, const int* page_table, int page_size, const int* kv_len,
                 const int* rope_pos, const int* finished, const float* inv_freq, int Hq, int Hkv, int nsplit,
                 float* part_o, float* part_ml, int* counters, bf16* out, bool pdl, cudaStream_t s);
+
+// the same for B streams, one grid slice each: rows b of qkv / out, nsplit a multiple of 8, part_o / part_ml / counters for 8 streams
+// of nsplit / 8 <= 8 rows and Hkv counters each
+struct AttnStream {
+    const int* page_table;
+    const int* scalars;   // LCC_SC_*
+};
+int attn_decode_batch(bf16* qkv, int qkv_ld, bf16* kc, bf16* vc, const AttnStream* streams, int B, int page_size, const float* inv_freq,
+                      int Hq, int Hkv, int nsplit, float* part_o, float* part_ml, int* counters, bf16* out, int out_ld, cudaStream_t s);
 
 int attn_oproj_decode(bf16* qkv, bf16* kc, bf16* vc, const int* page_table, int page_size, const int* kv_len,
                       const int* rope_pos, const int* finished, const float* inv_freq, int Hq, int Hkv, int nsplit,
@@ -62,6 +97,21 @@ int gemv_norm_swiglu(const bf16* W_gu, int ldw, const bf16* x, const bf16* norm_
                      cudaStream_t s);
 int gemv_norm_logits(const bf16* W, int ldw, const bf16* x, const bf16* norm_w, float eps, float* logits,
                      float* logits_copy, int N, int K, const int* finished, int num_sms, bool pdl, cudaStream_t s);
+
+// gemv_batch.cu: the projections of a decode step for B <= 8 streams (rows of x, ldx elements apart). N % 32 == 0, K % 64 == 0, W dense.
+struct GemvBatch {
+    const bf16* W;
+    const bf16* x;
+    int N, K, ldx, B;
+    const int* const* finished;   // [B] device flags: a finished stream's rows stay as they are
+    const int* x_rows;            // [B] rows of x, or null: 0, 1, ...
+    const void* pf_ptr;           // L2 prefetch of the next kernel's weights
+    size_t pf_bytes;
+};
+int gemv_batch_bias(const GemvBatch& a, const bf16* bias, bf16* out, int ldo, cudaStream_t s);
+int gemv_batch_residual(const GemvBatch& a, bf16* h_inout, int ldo, cudaStream_t s);
+int gemv_batch_swiglu(const GemvBatch& a, bf16* act, int ldo, cudaStream_t s);   // gate / up rows interleaved by 16
+int gemv_batch_logits(const GemvBatch& a, float* logits, float* logits_copy, int ldo, cudaStream_t s);
 
 // sampling.cu
 struct SampleArgs {

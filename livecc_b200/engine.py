@@ -93,6 +93,7 @@ class LiveCCB200ForConditionalGeneration:
         self._native = self._build_native()
         self.pool = PagePool(t.num_hidden_layers, t.num_key_value_heads, device)
         self._cap_patches, self._cap_tokens = 0, 0
+        self._persistent_decode = os.environ.get("LIVECC_B200_MEGA", "")[:1] == "1"   # (as lcc_model_create reads it)
         self._ensure_workspace(3072, 1024)
         self._graphs = {}
         self._captured_launches = 0   # launches recorded into graphs (counted by the library at capture, never executed then)
@@ -346,10 +347,12 @@ class LiveCCB200ForConditionalGeneration:
         """Multi-stream batching: one generate() for up to 8 independent streams of this model
         (the reference demo admits 5 concurrent sessions on one model object, REF/demo/app.py:178, and serves them one
         after another). Every request is a dict with the per-stream arguments of generate() (`input_ids` [1, L],
-        `pixel_values_videos` | `video_frames`, `video_grid_thw`, `past_key_values`). The ViT and the prefill run per
-        stream; all decode steps run batched in the persistent decode kernel, which reads every weight byte once per
-        step for all streams. Each stream's ids, logits and cache are bit-identical to calling generate() on it alone
-        (tests/test_engine_gpu.py::test_batched_decode_equals_sequential)."""
+        `pixel_values_videos` | `video_frames`, `video_grid_thw`, `past_key_values`). The ViT runs per stream; the new
+        tokens of all streams are prefilled in one pass (up to PREFILL_ROWS of them at a time), and every decode step is one pass
+        too: each weight byte is read once for all streams. The sums of a pass are taken in an order that depends on its rows, so
+        a stream's logits may differ from generate()'s in their last bits. With LIVECC_B200_MEGA=1 streams are prefilled one by
+        one and decoded by the persistent kernel: ids, logits and caches are then bit-identical to generate() on each
+        alone (tests/test_mega_gpu.py::test_batched_decode_equals_sequential)."""
         if not 1 <= len(requests) <= _cabi.MAX_BATCH:
             raise ValueError(f"generate_batch takes 1..{_cabi.MAX_BATCH} streams")
         self._check_common(None, None, do_sample, max_new_tokens)
@@ -363,11 +366,14 @@ class LiveCCB200ForConditionalGeneration:
             if set(rq) - allowed:
                 raise TypeError(f"request {b} has unsupported keys {sorted(set(rq) - allowed)}")
             recs.append(self._begin_stream(rq.get("input_ids"), rq.get("pixel_values_videos"), rq.get("video_grid_thw"),
-                                           rq.get("past_key_values"), rq.get("video_frames"), sp, max_new_tokens, slot=b))
+                                           rq.get("past_key_values"), rq.get("video_frames"), sp, max_new_tokens, slot=b,
+                                           defer=len(requests) > 1 and not self._persistent_decode))
         if len({id(r["cache"]) for r in recs}) != len(recs):
             raise ValueError("the same cache object appears in two requests of one batch")
         for r in recs:   # a later stream's page allocation may have moved the pool: take the pointers after all of them
             r["st"] = r["cache"].stream_state()
+        if "pos3" in recs[0]:
+            self._prefill_streams(recs, sp)
         V = self.config.text_config.vocab_size
         B = len(recs)
         first_logits = self._raw_logits_all()[:B].clone() if output_logits else None
@@ -467,9 +473,10 @@ class LiveCCB200ForConditionalGeneration:
         return self.nsplit
 
     def _begin_stream(self, input_ids, pixel_values_videos, video_grid_thw, past_key_values, video_frames, sp,
-                      max_new_tokens, slot, timed=False, video_embeds=None):
+                      max_new_tokens, slot, timed=False, video_embeds=None, defer=False):
         """Everything of one stream's turn up to and including the prefill and the first token selection; the first
-        token's embedding and logits land in row `slot` of the decode-step buffers."""
+        token's embedding and logits land in row `slot` of the decode-step buffers. defer: all but the prefill, whose inputs
+        are returned (the vision tower's rows are then this call's own: the next stream's pass overwrites the static ones)."""
         if input_ids is None or input_ids.dim() != 2 or input_ids.shape[0] != 1:
             raise ValueError("input_ids must be [1, L] (one stream per call)")
         cfg = self.config
@@ -505,15 +512,16 @@ class LiveCCB200ForConditionalGeneration:
         if pixel_values_videos is not None:
             if video_grid_thw is None:
                 raise ValueError("video_grid_thw is required with pixel_values_videos")
-            video_embeds = self.get_video_features(pixel_values_videos, video_grid_thw, _static_ok=True)  # consumed by this prefill
+            video_embeds = self.get_video_features(pixel_values_videos, video_grid_thw, _static_ok=not defer)  # consumed by this prefill
             n_video_expected = video_embeds.shape[0]
         elif video_frames is not None:
-            video_embeds = self.get_video_features_from_frames(video_frames, _static_ok=True)
+            video_embeds = self.get_video_features_from_frames(video_frames, _static_ok=not defer)
             n_video_expected = video_embeds.shape[0]
         if timed:
             self._ev[1].record()
         # ---- capacity, buffers, device scalars ----
-        self._ensure_workspace(0, S)
+        if not defer:
+            self._ensure_workspace(0, S)
         cache.ensure_tokens(past + S + max_new_tokens)
         cache.ensure_seq_capacity(L + max_new_tokens + 1)
         cache.seq_buf[:L].copy_(ids_dev[0])
@@ -521,9 +529,28 @@ class LiveCCB200ForConditionalGeneration:
         cache.scalars.copy_(sc_host, non_blocking=False)
         st = cache.stream_state()
         new_ids = cache.seq_buf[past:L]
+        if defer:
+            return dict(cache=cache, L=L, S=S, past=past, n_video_expected=n_video_expected, n_gen=0, pos3=pos3_dev, video=video_embeds)
         # ---- prefill + first token ----
         self._native.prefill(st, new_ids, pos3_dev, S, past, video_embeds, sp, slot=slot)
         return dict(cache=cache, st=st, L=L, S=S, past=past, n_video_expected=n_video_expected, n_gen=0)
+
+    # new tokens of one pass over several streams: enough to keep the tensor cores busy, with the workspace of a clip's question
+    PREFILL_ROWS = 2048
+
+    def _prefill_streams(self, recs, sp):
+        """Prefill of the streams of a batch, as many of them at a time as have PREFILL_ROWS new tokens together."""
+        groups, rows = [], 0
+        for b, r in enumerate(recs):
+            if not groups or rows + r["S"] > self.PREFILL_ROWS:
+                groups.append([])
+                rows = 0
+            groups[-1].append(b)
+            rows += r["S"]
+        self._ensure_workspace(0, max(sum(recs[b]["S"] for b in g) for g in groups))
+        for g in groups:
+            self._native.prefill_batch([(recs[b]["st"], recs[b]["cache"].seq_buf[recs[b]["past"]:recs[b]["L"]], recs[b]["pos3"], recs[b]["S"],
+                                         recs[b]["past"], recs[b]["video"]) for b in g], sp, g[0])
 
     def _finish_stream(self, rec, sc, logits_out, logits_hist, output_logits) -> GenerateOutput:
         cache, L, past = rec["cache"], rec["L"], rec["past"]
