@@ -22,7 +22,7 @@ OBJ_DIR = PKG_DIR / "build"
 # family alone compiles nothing else. The full library (profile None) holds every source and exports a superset.
 PROFILES = {
     "seq": ["cabi_core", "gemm_tcgen05", "sampling", "linear_any", "recurrent", "recurrent_chunked", "attn_local", "rowops", "rotary", "attn_latent",
-            "hyper", "moe", "seq_model"],
+            "attention_prefill_tc", "hyper", "moe", "seq_model"],
 }
 
 

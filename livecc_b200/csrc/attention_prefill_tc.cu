@@ -24,6 +24,7 @@
 #include "gemm.h"
 #include "launch.h"
 #include "ops.h"
+#include "seqmix.h"
 
 namespace lcc {
 namespace ptc {
@@ -59,13 +60,36 @@ __device__ __forceinline__ float ex2_ftz_p(float x) {
     return y;
 }
 
+// LOCAL: the attention of the hybrid models (plain masks): fp32 queries, rounded to bf16 as they are staged, a window and / or chunks, a sink
+// in the softmax, gated output. Their pages are not cleared behind the newest token, and a tile may begin before the first visible
+// key: what P = 0 would meet there is zeroed in the staged V tile. (1024 rows of 16 heads on 2, window 1024: 24 us; mma.sync tiles of one
+// head and 64 rows, eight of which staged the same keys, took 80. 2048 rows in chunks of 1024: 24 for 102.) A prompt has few tiles per
+// CTA, so most of this kernel's code runs once, and fetching it is what it costs: with the staging of Q and the gated output unrolled
+// and whole divisions in it, one tile took 36 us for 11.
+struct PrefillLocal {
+    const float* q;       // [S, Hq, 128]
+    SeqPos pos;
+    const float* sink;    // [Hq], or null: 0
+    const bf16* gate;
+    int ld_gate, chunk, window;
+    bool no_sink, gate_channel;
+    __device__ __forceinline__ int first_key(int p) const {
+        const int lo = chunk > 0 ? p / chunk * chunk : 0;
+        return window > 0 ? max(lo, p - window + 1) : lo;
+    }
+};
+
+template <bool LOCAL>
 __global__ void __launch_bounds__(192, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ PrefillTcParams p) {
+                       const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ PrefillTcParams p, const PrefillLocal lp) {
     using namespace ptc;
-    const PrefillStream& st = p.ps.st[blockIdx.z / p.nsplit];
-    const int kvh = blockIdx.y, split = blockIdx.z % p.nsplit;
-    const int pos0 = blockIdx.x * p.PT, S = st.S, past = st.past;
+    if (LOCAL && lp.pos.finished && *lp.pos.finished) return;
+    const PrefillStream& st = p.ps.st[LOCAL ? 0 : blockIdx.z / p.nsplit];
+    const int kvh = blockIdx.y, split = LOCAL ? 0 : blockIdx.z % p.nsplit;
+    // (with a window or chunks the last rows see the most keys: they start first)
+    const int pos0 = (LOCAL ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * p.PT, S = st.S;
+    const int past = LOCAL && lp.pos.kv_len ? *lp.pos.kv_len : st.past;
     if (pos0 >= S) return;
     const int npos = min(p.PT, S - pos0);
     const int rows_used = npos * p.G;
@@ -74,7 +98,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     // KV tiles this CTA needs: keys 0 .. past + last position (causal), restricted to its split
     const int n_tiles = (past + pos0 + npos + BN - 1) / BN;
     int tile_lo = 0, tile_hi = n_tiles;
-    if (p.nsplit > 1) {
+    const int key0 = LOCAL ? lp.first_key(past + pos0) : 0, key1 = past + pos0 + npos;   // no row of this CTA sees a key outside [key0, key1)
+    if (LOCAL) tile_lo = key0 / BN;
+    if (!LOCAL && p.nsplit > 1) {
         const int tiles_total = (past + S + BN - 1) / BN;
         const int tps = (tiles_total + p.nsplit - 1) / p.nsplit;
         tile_lo = split * tps;
@@ -106,10 +132,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (warp == 0 && lane == 0) {
-        prefetch_tensormap(&tmap_q);
+        if (!LOCAL) prefetch_tensormap(&tmap_q);
         prefetch_tensormap(&tmap_k);
         prefetch_tensormap(&tmap_v);
-        mbar_init(q_full, 1);
+        mbar_init(q_full, LOCAL ? 4 : 1);
         for (int i = 0; i < STAGES; ++i) {
             mbar_init(&k_full[i], 1);
             mbar_init(&k_empty[i], 1);
@@ -134,9 +160,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         // ===================== TMA producer =====================
         if (lane == 0) {
             // the box is always (64, G, PT): rows beyond the stream's are the next one's, or zero-filled but still counted; nothing of them is kept
-            mbar_arrive_expect_tx(q_full, 2u * 64u * (uint32_t)p.G * (uint32_t)p.PT * 2u);
-            tma_load_3d(smem + OFF_Q, &tmap_q, q_full, 0, kvh * p.G, st.row0 + pos0);
-            tma_load_3d(smem + OFF_Q + Q_ATOM_BYTES, &tmap_q, q_full, 64, kvh * p.G, st.row0 + pos0);
+            if (!LOCAL) {
+                mbar_arrive_expect_tx(q_full, 2u * 64u * (uint32_t)p.G * (uint32_t)p.PT * 2u);
+                tma_load_3d(smem + OFF_Q, &tmap_q, q_full, 0, kvh * p.G, st.row0 + pos0);
+                tma_load_3d(smem + OFF_Q + Q_ATOM_BYTES, &tmap_q, q_full, 64, kvh * p.G, st.row0 + pos0);
+            }
             const int* page_table = st.page_table;
             for (int i = 0; i < T; ++i) {
                 const int st = i % STAGES;
@@ -186,6 +214,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         for (int i = 0; i < T; ++i) {
             if (i + 1 < T) issue_qk(i + 1);
             mbar_wait(&v_full[i % STAGES], (i / STAGES) & 1);
+            if (LOCAL) {
+                const int k0 = (tile_lo + i) * BN, cut_lo = max(key0 - k0, 0), cut_hi = min(key1 - k0, BN);   // the tile's rows in [cut_lo, cut_hi) count
+                if (cut_lo > 0 || cut_hi < BN) {
+                    uint8_t* sv = smem + OFF_V + (i % STAGES) * KV_BYTES;
+                    for (int u = lane; u < BN * 16; u += 32) {
+                        const int r = u >> 4, c = u & 15;   // 16 bytes of token row r: eight in each 64-channel half
+                        if (r < cut_lo || r >= cut_hi)
+                            *reinterpret_cast<uint4*>(sv + (c >> 3) * KV_ATOM_BYTES + r * 128 + (c & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                }
+            }
             mbar_wait(p_full, i & 1);
             tc_fence_after();
             if (lane == 0) {
@@ -209,7 +250,36 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         const bool row_ok = row < rows_used;
         const int rpos = row / p.G, rg = row - rpos * p.G;
         const int lim = row_ok ? past + pos0 + rpos : -1;  // last visible key index; invalid rows see nothing
+        const int first = LOCAL && row_ok ? lp.first_key(lim) : 0;
         float m_used = -INFINITY, l = 0.f;
+        if (LOCAL) {
+            if (!lp.no_sink && row_ok) {   // the sink's term starts the sum
+                m_used = (lp.sink ? lp.sink[kvh * p.G + rg] : 0.f) * 1.4426950408889634f;
+                l = 1.f;
+            }
+            // queries: a warp takes its 32 rows one by one, four channels per lane, into the K-major 128-byte-swizzled tile
+            const int Hq = p.Hkv * p.G, c = lane & 15;   // lanes 0..15: channels 0..63 in 8-byte pieces
+            uint8_t* sq = smem + OFF_Q + (lane >> 4) * Q_ATOM_BYTES;
+            int qg = quarter * 32 % p.G;
+            const float* src = lp.q + ((size_t)(pos0 + quarter * 32 / p.G) * Hq + kvh * p.G + qg) * D + lane * 4;
+            for (int r0 = quarter * 32; r0 < quarter * 32 + 32; r0 += 8) {
+                float4 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    v[j] = r0 + j < rows_used ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const bool next = ++qg == p.G;   // the next position's first head of this group
+                    src += next ? (Hq - p.G + 1) * D : D;
+                    qg = next ? 0 : qg;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    *reinterpret_cast<uint2*>(sq + (r0 + j) * 128 + (((c >> 1) ^ j) << 4) + (c & 1) * 8) =
+                        make_uint2(pack_bf16x2(v[j].x, v[j].y), pack_bf16x2(v[j].z, v[j].w));
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(q_full);
+        }
         for (int i = 0; i < T; ++i) {
             const int b = i & 1;
             mbar_wait(&s_full[b], (i >> 1) & 1);
@@ -220,12 +290,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             tmem_ld_wait();
 
             const int kbase = (tile_lo + i) * BN;
-            if (__any_sync(0xffffffffu, kbase + BN - 1 > lim)) {  // tile reaches the diagonal for some row of this warp
+            if (__any_sync(0xffffffffu, kbase + BN - 1 > lim || (LOCAL && kbase < first))) {  // tile reaches the diagonal (or the first key) of some row of this warp
 #pragma unroll
                 for (int c = 0; c < 2; ++c)
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
-                        if (kbase + c * 32 + j > lim) v[c][j] = __float_as_uint(-INFINITY);
+                        if (kbase + c * 32 + j > lim || (LOCAL && kbase + c * 32 + j < first)) v[c][j] = __float_as_uint(-INFINITY);
             }
             float mx[8];
 #pragma unroll
@@ -282,9 +352,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full);
         }
+        const bf16* gate = LOCAL && lp.gate && row_ok
+                               ? lp.gate + (size_t)(pos0 + rpos) * lp.ld_gate + (lp.gate_channel ? (size_t)(kvh * p.G + rg) * D : (size_t)(kvh * p.G + rg)) : nullptr;
+        auto sigmoid = [](float x) { return __fdividef(1.f, 1.f + expf(-x)); };
         mbar_wait(pv_done, (T - 1) & 1);
         tc_fence_after();
-        if (p.nsplit > 1) {
+        if (!LOCAL && p.nsplit > 1) {
             const size_t prow = ((size_t)split * p.Hkv + kvh) * rows_total + row_base + row;
             float* dst = p.part_o + prow * D;
 #pragma unroll
@@ -304,13 +377,32 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 p.part_ml[prow * 2 + 1] = l;
             }
         } else {
-            const float inv = l > 0.f ? 1.f / l : 0.f;
+            float inv = l > 0.f ? 1.f / l : 0.f;
+            const bool wide_gate = LOCAL && gate && lp.gate_channel;
+            if (LOCAL && gate && !wide_gate) inv *= sigmoid(bf2f(*gate));
             bf16* dst = p.out + (size_t)(st.row0 + pos0 + rpos) * p.o_ld + (size_t)(kvh * p.G + rg) * D;
-#pragma unroll
+#pragma unroll LOCAL ? 1 : 4
             for (int c = 0; c < 4; ++c) {
                 uint32_t o32[32];
                 tmem_ld_32x32b_x32(tmem_base + COL_O + c * 32 + lane_off, o32);
+                uint4 z[4];
+                if (wide_gate) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) z[j] = *reinterpret_cast<const uint4*>(gate + c * 32 + j * 8);
+                }
                 tmem_ld_wait();
+                if (wide_gate) {
+#pragma unroll
+                    for (int g8 = 0; g8 < 4; ++g8) {
+                        const uint32_t zw[4] = {z[g8].x, z[g8].y, z[g8].z, z[g8].w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float2 f = unpack_bf16x2(zw[j]);
+                            o32[g8 * 8 + 2 * j] = __float_as_uint(__uint_as_float(o32[g8 * 8 + 2 * j]) * sigmoid(f.x));
+                            o32[g8 * 8 + 2 * j + 1] = __float_as_uint(__uint_as_float(o32[g8 * 8 + 2 * j + 1]) * sigmoid(f.y));
+                        }
+                    }
+                }
                 if (row_ok) {
 #pragma unroll
                     for (int g8 = 0; g8 < 4; ++g8) {
@@ -370,12 +462,40 @@ int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, con
     if (make_tmap_bf16_2d_box(&tk, kc, pool_rows, D, D, 64, BN, false)) return -11;
     if (make_tmap_bf16_2d_box(&tv, vc, pool_rows, D, D, 64, BN, false)) return -11;
     static SmemAttrOnce once;
-    if (ensure_dyn_smem(once, attn_prefill_tc_kernel, SMEM_BYTES)) return -12;
+    if (ensure_dyn_smem(once, attn_prefill_tc_kernel<false>, SMEM_BYTES)) return -12;
     const PrefillTcParams p{out, o_ld, Hkv, G, PT, 1.4426950408889634f / sqrtf((float)D), nsplit, part_o, part_ml, ps};
     lcc::count_launch();
-    attn_prefill_tc_kernel<<<dim3(q_tiles, Hkv, nsplit * ps.n), 192, SMEM_BYTES, s>>>(tq, tk, tv, p);
+    attn_prefill_tc_kernel<false><<<dim3(q_tiles, Hkv, nsplit * ps.n), 192, SMEM_BYTES, s>>>(tq, tk, tv, p, PrefillLocal{});
     *nsplit_out = nsplit;
     return 0;
+}
+
+bool attn_local_tc_takes(const float* q, const void* k_pages, const void* v_pages, int page_size, const void* gate, int ld_gate, const void* out,
+                         int ld_out, int Hq, int G, int D, int DV, int ld_v, const AttnOpts& opt) {
+    const bool plain = opt.softcap <= 0.f && opt.keep_first <= 0 && opt.maps == 1 && !opt.raw && !opt.bias;
+    const bool wide_gate = gate && opt.gate_channel;
+    return plain && D == ptc::D && DV == ptc::D && ld_v == ptc::D && page_size == ptc::BN && Hq / G <= ptc::BM && ld_out % 8 == 0 && (!wide_gate || ld_gate % 8 == 0) &&
+           (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)out | (wide_gate ? (uintptr_t)gate : 0)) & 15) == 0;
+}
+
+int attn_local_tc(const float* q, const void* k_pages, const void* v_pages, const int* page_table, const void* gate, int ld_gate, void* out,
+                  int ld_out, int S, int Hq, int G, int chunk, float scale, SeqPos pos, cudaStream_t s, const float* sink, const AttnOpts& opt) {
+    using namespace ptc;
+    PrefillTcParams p{};
+    p.out = (bf16*)out; p.o_ld = ld_out; p.Hkv = G; p.G = Hq / G; p.PT = BM / p.G;
+    p.scale_log2 = scale * 1.4426950408889634f;
+    p.nsplit = 1;
+    p.ps.n = 1; p.ps.rows = S;
+    p.ps.st[0].page_table = page_table; p.ps.st[0].S = S; p.ps.st[0].past = pos.past;
+    const PrefillLocal lp{q, pos, sink, (const bf16*)gate, ld_gate, chunk > 0 ? chunk : 0, opt.window > 0 ? opt.window : 0, opt.no_sink, opt.gate_channel};
+    CUtensorMap tk, tv;
+    const int64_t pool_rows = (int64_t)1 << 31;  // (as above)
+    if (make_tmap_bf16_2d_box(&tk, k_pages, pool_rows, D, D, 64, BN, false) || make_tmap_bf16_2d_box(&tv, v_pages, pool_rows, D, D, 64, BN, false)) return -100;
+    static SmemAttrOnce once;
+    if (ensure_dyn_smem(once, attn_prefill_tc_kernel<true>, SMEM_BYTES)) return -100;
+    count_launch();
+    attn_prefill_tc_kernel<true><<<dim3((S + p.PT - 1) / p.PT, G), 192, SMEM_BYTES, s>>>(tk, tk, tv, p, lp);
+    return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 
 }  // namespace lcc
