@@ -71,130 +71,165 @@ __device__ __forceinline__ float gelu_erf_bf16(float x) {
 }
 __device__ __forceinline__ float silu_bf16(float x) { return rbf(__fdividef(x, 1.0f + __expf(-x))); }
 
-// Fused epilogue of one 32-column chunk of one accumulator row: v = the fp32 bits of columns [col0, col0 + 32) of output row
-// `row` (one thread per row); columns >= tile_end belong to the next tile (or are padding) and are dropped.
+// Fused epilogue of a warp's 32 x 32 chunk of accumulators. Tensor memory gives a thread one row: v = the fp32 bits of columns [col0, col0 + 32) of
+// row row0 + lane. Bias, activation and rounding happen there; four lanes then exchange their rows' 16-byte pieces, so that a store (and
+// a load of the residual) covers 64 bytes of 8 rows instead of 16 of 32, half a sector each. Bias and residual are fetched while the accumulators
+// arrive. Columns >= tile_end belong to the next tile (or are padding) and are dropped. Where K is short this is what a product costs:
+// GEMM_FIGURES.
+template <int EPI> struct RowEpi {
+    static constexpr bool kBias = EPI == EPI_BIAS || EPI == EPI_BIAS_QUICKGELU || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESIDUAL;
+    static constexpr bool kResidual = EPI == EPI_RESIDUAL || EPI == EPI_BIAS_RESIDUAL;
+};
+struct EpiFetch { uint4 bias[4], res[4]; };
+
 template <int EPI>
-__device__ __forceinline__ void epilogue_chunk(const uint32_t (&v)[32], bf16* C, int ldc, int M, int row, bool row_ok, int col0,
+__device__ __forceinline__ void epilogue_fetch(EpiFetch& f, int M, int row0, int lane, int col0, int tile_end, const bf16* __restrict__ bias,
+                                               const bf16* residual, int ldr) {
+    if (RowEpi<EPI>::kBias) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) f.bias[g] = col0 + g * 8 < tile_end ? *reinterpret_cast<const uint4*>(bias + col0 + g * 8) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (RowEpi<EPI>::kResidual) {
+        const int col = col0 + (lane & 3) * 8;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int row = row0 + (lane & ~3) + k;
+            f.res[k] = row < M && col < tile_end ? *reinterpret_cast<const uint4*>(residual + (size_t)row * ldr + col) : make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+}
+
+// lanes l and l ^ bit exchange: the lane with the bit clear gives b for the other's a
+__device__ __forceinline__ void swap_pieces(uint4& a, uint4& b, int bit, int lane) {
+    const bool up = lane & bit;
+    auto word = [&](uint32_t& x, uint32_t& y) {
+        const uint32_t r = __shfl_xor_sync(0xffffffffu, up ? x : y, bit);
+        if (up) x = r; else y = r;
+    };
+    word(a.x, b.x); word(a.y, b.y); word(a.z, b.z); word(a.w, b.w);
+}
+// p[i] of lane 4 m + k becomes p[k] of lane 4 m + i
+__device__ __forceinline__ void quad_transpose(uint4 (&p)[4], int lane) {
+    swap_pieces(p[0], p[1], 1, lane); swap_pieces(p[2], p[3], 1, lane);
+    swap_pieces(p[0], p[2], 2, lane); swap_pieces(p[1], p[3], 2, lane);
+}
+
+template <int EPI>
+__device__ __forceinline__ void epilogue_chunk(const uint32_t (&v)[32], const EpiFetch& f, bf16* C, int ldc, int M, int row0, int lane, int col0,
                                                int tile_end, int ks, const bf16* __restrict__ bias, const bf16* residual,
                                                int ldr) {
     if (EPI == EPI_PARTIAL_F32) {
         // fp32 partial tile of split ks: P[ks][row][col] (C is the partial buffer, ldc == N)
-        if (row_ok) {
-            float* dst = reinterpret_cast<float*>(C) + ((size_t)ks * M + row) * (size_t)ldc + col0;
+        float* base = reinterpret_cast<float*>(C) + (size_t)ks * M * (size_t)ldc;
 #pragma unroll
-            for (int g = 0; g < 8; ++g)
-                if (col0 + g * 4 < tile_end)
-                    *reinterpret_cast<uint4*>(dst + g * 4) =
-                        make_uint4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
-        }
-    } else if (EPI == EPI_SWIGLU) {
-        // Weight rows are interleaved in 32-row groups: 16 gate rows then the 16
-        // matching up rows. out[j] = bf16(silu_bf16(bf16 gate) * bf16 up)  (mq2vl.py:503)
-        if (row_ok && col0 < tile_end) {  // BLOCK_N % 32 == 0 for this epilogue: whole chunks only
-            const int ocol0 = (col0 >> 5) << 4;
-            uint32_t o[8];
+        for (int h = 0; h < 2; ++h) {
+            uint4 p[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float g0 = rbf(__uint_as_float(v[2 * j])), g1 = rbf(__uint_as_float(v[2 * j + 1]));
-                float u0 = rbf(__uint_as_float(v[16 + 2 * j])), u1 = rbf(__uint_as_float(v[16 + 2 * j + 1]));
-                o[j] = pack_bf16x2(silu_bf16(g0) * u0, silu_bf16(g1) * u1);
+            for (int g = 0; g < 4; ++g) p[g] = make_uint4(v[h * 16 + g * 4], v[h * 16 + g * 4 + 1], v[h * 16 + g * 4 + 2], v[h * 16 + g * 4 + 3]);
+            quad_transpose(p, lane);
+            const int col = col0 + h * 16 + (lane & 3) * 4;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int row = row0 + (lane & ~3) + k;
+                if (row < M && col < tile_end) *reinterpret_cast<uint4*>(base + (size_t)row * ldc + col) = p[k];
             }
-            uint4* dst = reinterpret_cast<uint4*>(C + (size_t)row * ldc + ocol0);
-            dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-            dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
         }
-    } else if (EPI == EPI_CLAMP_GLU) {
-        // the same 32-row interleave; the activation runs in fp32 on the accumulators and is rounded once. The clamp rides in
-        // the (otherwise unused) residual stride as float bits, the sigmoid's slope and the offset of the up half in the
-        // (otherwise unused) bias pointer's bits.
-        if (row_ok && col0 < tile_end) {
-            const float limit = __int_as_float(ldr);
-            const unsigned long long pb = (unsigned long long)bias;
-            const float alpha = __uint_as_float((unsigned)(pb & 0xffffffffull)), up_bias = __uint_as_float((unsigned)(pb >> 32));
-            const int ocol0 = (col0 >> 5) << 4;
-            uint32_t o[8];
+    } else if (EPI == EPI_SWIGLU || EPI == EPI_CLAMP_GLU) {
+        // Weight rows are interleaved in 32-row groups: 16 gate rows then the 16
+        // matching up rows. EPI_SWIGLU: out[j] = bf16(silu_bf16(bf16 gate) * bf16 up)  (mq2vl.py:503). EPI_CLAMP_GLU: the activation runs
+        // in fp32 on the accumulators and is rounded once; the clamp rides in the (otherwise unused) residual stride as float bits, the
+        // sigmoid's slope and the offset of the up half in the (otherwise unused) bias pointer's bits.
+        const float limit = __int_as_float(ldr);
+        const unsigned long long pb = (unsigned long long)bias;
+        const float alpha = __uint_as_float((unsigned)(pb & 0xffffffffull)), up_bias = __uint_as_float((unsigned)(pb >> 32));
+        uint32_t o[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float y[2];
+        for (int j = 0; j < 8; ++j) {
+            float y[2];
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const float g = fminf(__uint_as_float(v[2 * j + e]), limit);
-                    const float u = fminf(fmaxf(__uint_as_float(v[16 + 2 * j + e]), -limit), limit);
+            for (int e = 0; e < 2; ++e) {
+                const float g0 = __uint_as_float(v[2 * j + e]), u0 = __uint_as_float(v[16 + 2 * j + e]);
+                if (EPI == EPI_SWIGLU) {
+                    y[e] = silu_bf16(rbf(g0)) * rbf(u0);
+                } else {
+                    const float g = fminf(g0, limit), u = fminf(fmaxf(u0, -limit), limit);
                     y[e] = g / (1.f + __expf(-alpha * g)) * (u + up_bias);
                 }
-                o[j] = pack_bf16x2(y[0], y[1]);
             }
-            uint4* dst = reinterpret_cast<uint4*>(C + (size_t)row * ldc + ocol0);
-            dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-            dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+            o[j] = pack_bf16x2(y[0], y[1]);
+        }
+        uint4 p0 = make_uint4(o[0], o[1], o[2], o[3]), p1 = make_uint4(o[4], o[5], o[6], o[7]);
+        swap_pieces(p0, p1, 1, lane);   // two lanes: 32 bytes of one row, then of the other
+        const int row = row0 + (lane & ~1), col = ((col0 >> 5) << 4) + (lane & 1) * 8;
+        if (col0 < tile_end) {  // BLOCK_N % 32 == 0 for these epilogues: whole chunks only
+            if (row < M) *reinterpret_cast<uint4*>(C + (size_t)row * ldc + col) = p0;
+            if (row + 1 < M) *reinterpret_cast<uint4*>(C + (size_t)(row + 1) * ldc + col) = p1;
         }
     } else {
+        uint4 p[4];
 #pragma unroll
         for (int g = 0; g < 4; ++g) {  // 4 groups of 8 columns (16 B of bf16 each)
-            const int col = col0 + g * 8;
-            if (row_ok && col < tile_end) {
-                float x[8];
+            float x[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[g * 8 + j]);
-                if (EPI == EPI_BIAS || EPI == EPI_BIAS_QUICKGELU || EPI == EPI_BIAS_GELU ||
-                    EPI == EPI_BIAS_RESIDUAL) {
-                    const uint4 bb = *reinterpret_cast<const uint4*>(bias + col);
-                    const uint32_t bw[4] = {bb.x, bb.y, bb.z, bb.w};
+            for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v[g * 8 + j]);
+            if (RowEpi<EPI>::kBias) {
+                const uint32_t bw[4] = {f.bias[g].x, f.bias[g].y, f.bias[g].z, f.bias[g].w};
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        float2 f = unpack_bf16x2(bw[j]);
-                        x[2 * j] += f.x;
-                        x[2 * j + 1] += f.y;
-                    }
+                for (int j = 0; j < 4; ++j) {
+                    const float2 b = unpack_bf16x2(bw[j]);
+                    x[2 * j] += b.x;
+                    x[2 * j + 1] += b.y;
                 }
-                if (EPI == EPI_RELU2) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) { x[j] = fmaxf(x[j], 0.f); x[j] *= x[j]; }
-                }
-                if (EPI == EPI_SIGMOID_GATE) {
-                    const uint4 gg = *reinterpret_cast<const uint4*>(residual + (size_t)row * ldr + col);
-                    const uint32_t gw[4] = {gg.x, gg.y, gg.z, gg.w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float2 f = unpack_bf16x2(gw[j]);
-                        x[2 * j] = __fdividef(x[2 * j], 1.f + __expf(-f.x));
-                        x[2 * j + 1] = __fdividef(x[2 * j + 1], 1.f + __expf(-f.y));
-                    }
-                }
-                if (EPI == EPI_GELU_ERF) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) x[j] = 0.5f * x[j] * (1.f + erff(x[j] * 0.7071067811865476f));
-                }
-                if (EPI == EPI_GELU_TANH) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) x[j] = 0.5f * x[j] * (1.f + tanhf(0.7978845608028654f * (x[j] + 0.044715f * x[j] * x[j] * x[j])));
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = rbf(x[j]);
-                if (EPI == EPI_BIAS_QUICKGELU) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) x[j] = quick_gelu_bf16(x[j]);
-                } else if (EPI == EPI_BIAS_GELU) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) x[j] = gelu_erf_bf16(x[j]);
-                } else if (EPI == EPI_RESIDUAL || EPI == EPI_BIAS_RESIDUAL) {
-                    const uint4 rr =
-                        *reinterpret_cast<const uint4*>(residual + (size_t)row * ldr + col);
-                    const uint32_t rw[4] = {rr.x, rr.y, rr.z, rr.w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        float2 f = unpack_bf16x2(rw[j]);
-                        x[2 * j] += f.x;
-                        x[2 * j + 1] += f.y;
-                    }
-                }
-                uint4 o;
-                o.x = pack_bf16x2(x[0], x[1]);
-                o.y = pack_bf16x2(x[2], x[3]);
-                o.z = pack_bf16x2(x[4], x[5]);
-                o.w = pack_bf16x2(x[6], x[7]);
-                *reinterpret_cast<uint4*>(C + (size_t)row * ldc + col) = o;
             }
+            if (EPI == EPI_RELU2) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) { x[j] = fmaxf(x[j], 0.f); x[j] *= x[j]; }
+            }
+            if (EPI == EPI_SIGMOID_GATE) {
+                const int row = row0 + lane, col = col0 + g * 8;
+                const uint4 gg = row < M && col < tile_end ? *reinterpret_cast<const uint4*>(residual + (size_t)row * ldr + col) : make_uint4(0u, 0u, 0u, 0u);
+                const uint32_t gw[4] = {gg.x, gg.y, gg.z, gg.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 s = unpack_bf16x2(gw[j]);
+                    x[2 * j] = __fdividef(x[2 * j], 1.f + __expf(-s.x));
+                    x[2 * j + 1] = __fdividef(x[2 * j + 1], 1.f + __expf(-s.y));
+                }
+            }
+            if (EPI == EPI_GELU_ERF) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = 0.5f * x[j] * (1.f + erff(x[j] * 0.7071067811865476f));
+            }
+            if (EPI == EPI_GELU_TANH) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = 0.5f * x[j] * (1.f + tanhf(0.7978845608028654f * (x[j] + 0.044715f * x[j] * x[j] * x[j])));
+            }
+            if (EPI == EPI_BIAS_QUICKGELU) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = quick_gelu_bf16(rbf(x[j]));
+            }
+            if (EPI == EPI_BIAS_GELU) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = gelu_erf_bf16(rbf(x[j]));
+            }
+            p[g] = make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+        }
+        quad_transpose(p, lane);
+        const int col = col0 + (lane & 3) * 8;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int row = row0 + (lane & ~3) + k;
+            if (RowEpi<EPI>::kResidual) {
+                const uint32_t aw[4] = {p[k].x, p[k].y, p[k].z, p[k].w}, rw[4] = {f.res[k].x, f.res[k].y, f.res[k].z, f.res[k].w};
+                uint32_t o[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 a = unpack_bf16x2(aw[j]), r = unpack_bf16x2(rw[j]);
+                    o[j] = pack_bf16x2(a.x + r.x, a.y + r.y);
+                }
+                p[k] = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+            if (row < M && col < tile_end) *reinterpret_cast<uint4*>(C + (size_t)row * ldc + col) = p[k];
         }
     }
 }
@@ -335,8 +370,7 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmap_a,
             if (tile_group && tile_group[m_blk] < 0) continue;
             mbar_wait(&tmem_full[acc], acc_phase);
             tc_fence_after();
-            const int row = m_blk * BLOCK_M + q * 32 + lane;
-            const bool row_ok = row < M;
+            const int row0 = m_blk * BLOCK_M + q * 32;
             const int tile_end = min(N, (n_blk + 1) * BLOCK_N);  // columns past it belong to the next tile (or are padding)
 #pragma unroll 1
             for (int c = c_begin; c < c_end; ++c) {
@@ -344,12 +378,14 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmap_a,
                 const uint32_t taddr =
                     tmem_base + (uint32_t)(acc * BLOCK_N + c * 32) + ((uint32_t)(q * 32) << 16);
                 tmem_ld_32x32b_x32(taddr, v);
-                tmem_ld_wait();
                 const int col0 = n_blk * BLOCK_N + c * 32;
+                EpiFetch f;
+                epilogue_fetch<EPI>(f, M, row0, lane, col0, tile_end, bias, residual, ldr);
+                tmem_ld_wait();
                 // batched: entry z's columns start at z * c_col_stride (floats when the output is fp32)
                 bf16* Cz = (EPI == EPI_PARTIAL_F32) ? reinterpret_cast<bf16*>(reinterpret_cast<float*>(C) + (size_t)z * c_col_stride)
                                                     : C + (size_t)z * c_col_stride;
-                epilogue_chunk<EPI>(v, Cz, ldc, M, row, row_ok, col0, tile_end, ks, bias,
+                epilogue_chunk<EPI>(v, f, Cz, ldc, M, row0, lane, col0, tile_end, ks, bias,
                                     EPI == EPI_SIGMOID_GATE ? residual + (size_t)z * c_col_stride : residual, ldr);
             }
             tc_fence_before();
@@ -500,17 +536,18 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             const int m_pair = unit % m_pairs, ks = (unit / m_pairs) % splits, n_blk = unit / (m_pairs * splits);
             mbar_wait(&tmem_full[acc], acc_phase);
             tc_fence_after();
-            const int row = m_pair * 2 * BLOCK_M + (int)rank * BLOCK_M + q * 32 + lane;
-            const bool row_ok = row < M;
+            const int row0 = m_pair * 2 * BLOCK_M + (int)rank * BLOCK_M + q * 32;
             const int tile_end = min(N, (n_blk + 1) * BLOCK_N);
 #pragma unroll 1
             for (int c = c_begin; c < c_end; ++c) {
                 uint32_t v[32];
                 const uint32_t taddr = tmem_base + (uint32_t)(acc * BLOCK_N + c * 32) + ((uint32_t)(q * 32) << 16);
                 tmem_ld_32x32b_x32(taddr, v);
-                tmem_ld_wait();
                 const int col0 = n_blk * BLOCK_N + c * 32;
-                epilogue_chunk<EPI>(v, C, ldc, M, row, row_ok, col0, tile_end, ks, bias, residual, ldr);
+                EpiFetch f;
+                epilogue_fetch<EPI>(f, M, row0, lane, col0, tile_end, bias, residual, ldr);
+                tmem_ld_wait();
+                epilogue_chunk<EPI>(v, f, C, ldc, M, row0, lane, col0, tile_end, ks, bias, residual, ldr);
             }
             tc_fence_before();
             __syncwarp();
