@@ -74,8 +74,8 @@ __device__ __forceinline__ float silu_bf16(float x) { return rbf(__fdividef(x, 1
 // Fused epilogue of a warp's 32 x 32 chunk of accumulators. Tensor memory gives a thread one row: v = the fp32 bits of columns [col0, col0 + 32) of
 // row row0 + lane. Bias, activation and rounding happen there; four lanes then exchange their rows' 16-byte pieces, so that a store (and
 // a load of the residual) covers 64 bytes of 8 rows instead of 16 of 32, half a sector each. Bias and residual are fetched while the accumulators
-// arrive. Columns >= tile_end belong to the next tile (or are padding) and are dropped. Where K is short this is what a product costs:
-// GEMM_FIGURES.
+// arrive. Columns >= tile_end belong to the next tile (or are padding) and are dropped. Where K is short this is what a product costs: with a
+// row's pieces stored by its own thread 8192 x 5120 x 1280 took 111 us, now 96, and 1024 x 1280 x 1280 14.7, now 11.3.
 template <int EPI> struct RowEpi {
     static constexpr bool kBias = EPI == EPI_BIAS || EPI == EPI_BIAS_QUICKGELU || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESIDUAL;
     static constexpr bool kResidual = EPI == EPI_RESIDUAL || EPI == EPI_BIAS_RESIDUAL;
@@ -1200,7 +1200,7 @@ static int launch_epi(const GemmArgs& a, int bn, int num_sms, cudaStream_t strea
 //    the un-overlapped epilogue of the last tile), which is 30-60 % of the M = 281 / 1024 GEMMs of the streaming path;
 //  * because of that fixed part, filling the last wave exactly (widths like 224 or 144, which the run-time width allows)
 //    measured within noise of the simple rule below (prefill qkv: 96 -> 24.3 us, 128 -> 23.5, 192 -> 25.3, 256 -> 29.5).
-// So: 64-wide tiles never win; between 128 and 256 the cost is (waves over the SMs) x (128 + bn), ties to the narrower tile.
+// So, for grouped and batched products and those with a gate: 64-wide tiles never win; between 128 and 256 the cost is (waves over the SMs) x (128 + bn), ties to the narrower tile.
 static int choose_bn(int M, int N, int num_sms) {
     if (N <= 64) return 64;
     const long long m_tiles = (M + BLOCK_M - 1) / BLOCK_M;
@@ -1211,34 +1211,47 @@ static int choose_bn(int M, int N, int num_sms) {
     return cost(128) <= cost(256) ? 128 : 256;
 }
 
-// Is the CTA pair's kernel the better one, and with which width (0: it is not)? A pair brings in half the bytes per multiplication, so its
-// time per 64-deep k-block grows with the width only: 0.295, 0.30, 0.325, 0.355, 0.37 us for 128, 160, 192, 224, 256 columns, where a CTA
-// alone takes 0.28 us for 128 and 0.41 for 256; against that it has 74 units of 256 rows for 148 of 128, and a launch of 9.5 us for 8. Waves
-// x k-blocks x these plus the launch predict which of the two wins for the shapes of the models (M = 281 to 8192, us, alone | pair):
-// 2048 x 10304 x 2048 75 | 65, 2048 x 5120 x 5120 107 | 92, 1200 x 4608 x 3584 55 | 44, 2090 x 4608 x 3584 66 | 61, 2090 x 3584 x 18944
-// 250 | 219, 8192 x 3840 x 1280 69 | 66, 512 x 10304 x 2048 31 | 27; alone stays for 281 x 37888 x 3584 81 | 91, 1024 x 3840 x 1280 16 | 17,
-// 256 x 5120 x 5120 31 | 33. Where the model sees less than 3 % the two measure the same. Every sum runs over k in the same order.
-static int choose_pair(int M, int N, int K, int num_sms, double* us) {
-    const long long nkb = (K + BLOCK_K - 1) / BLOCK_K;
-    auto waves = [](long long units, int at_once) { return (double)((units + at_once - 1) / at_once); };
-    const int bn1 = choose_bn(M, N, num_sms);
-    *us = 0.;
-    if (bn1 < 128 || num_sms < 2) return 0;
-    const double alone = 8.0 + waves((long long)((M + BLOCK_M - 1) / BLOCK_M) * ((N + bn1 - 1) / bn1), num_sms) * nkb * (bn1 == 128 ? 0.28 : 0.41);
-    const double per_kb[5] = {0.295, 0.30, 0.325, 0.355, 0.37};
-    double best = 0.97 * alone;
+// Plain products: one CTA per tile, or a CTA pair, and how wide a tile. Waves of tiles x 64-deep k-blocks x the time of one, plus a launch: 6.5 us and
+// 0.26, 0.275, 0.285, 0.30, 0.345, 0.385 us for 96 to 256 columns of a CTA, 8 us and 0.31, 0.31, 0.325, 0.345, 0.335 for 128 to 256 of a pair,
+// which brings in half the bytes per multiplication and has 74 units of 256 rows for 148 of 128. What gains by a width in between is a
+// last wave that is filled. Measured (us, back to back; one CTA of 128 or 256 columns | its best width | pair | taken):
+// 1024 x 5120 x 1280 25 | 160: 21.6 | 23.2 | 21.6, 2048 x 1280 x 5120 31.3 | 192: 27.9 | 31.2 | 160: 29.3, 2090 x 4608 x 3584 66 | 192: 58 | 61 | 58,
+// 2090 x 3584 x 3584 47.7 | 224: 44.2 | 46 | 44.2, 8192 x 1280 x 5120 107 | 224: 95 | 98 | 95, 512 x 10304 x 2048 29 | 160: 24 | 26 | 24,
+// 8192 x 3840 x 1280 66 | 256: 66 | 62.4 | pair, 2090 x 37888 x 3584 432 | 224: 424 | 389 | pair, 600 x 37888 x 3584 128 | 256: 128 | 139 | 128.
+// Every sum runs over k in the same order.
+static double tile_us(int M, int N, int K, int rows, int bn, int at_once, double per_kb) {
+    const long long units = (long long)((M + rows - 1) / rows) * ((N + bn - 1) / bn), nkb = (K + BLOCK_K - 1) / BLOCK_K;
+    return (double)((units + at_once - 1) / at_once * nkb) * per_kb;
+}
+// width of one CTA's tile, and its estimate
+static int choose_alone(int M, int N, int K, int num_sms, double* us) {
+    static constexpr double per_kb[6] = {0.26, 0.275, 0.285, 0.30, 0.345, 0.385};
+    int width = 64;
+    if (N <= 64) { *us = 0.; return width; }
+    *us = 1e300;
+    for (int i = 0; i < 6; ++i) {
+        const double t = 6.5 + tile_us(M, N, K, BLOCK_M, 96 + 32 * i, num_sms, per_kb[i]);
+        if (t < *us) { *us = t; width = 96 + 32 * i; }
+    }
+    return width;
+}
+// width of a pair's tile, 0 where one CTA (estimate `alone`) is not slower
+static int choose_pair(int M, int N, int K, int num_sms, double alone, double* us) {
+    static constexpr double per_kb[5] = {0.31, 0.31, 0.325, 0.345, 0.335};
+    *us = alone;
+    if (N <= 64 || num_sms < 2) return 0;
+    double best = alone;
     int width = 0;
     for (int i = 0; i < 5; ++i) {
-        const int bn = 128 + 32 * i;
-        const double t = 9.5 + waves((long long)((M + 2 * BLOCK_M - 1) / (2 * BLOCK_M)) * ((N + bn - 1) / bn), num_sms / 2) * nkb * per_kb[i];
-        if (t < best) { best = t; width = bn; }
+        const double t = 8.0 + tile_us(M, N, K, 2 * BLOCK_M, 128 + 32 * i, num_sms / 2, per_kb[i]);
+        if (t < best) { best = t; width = 128 + 32 * i; }
     }
-    *us = width ? best : alone;
+    if (width) *us = best;
     return width;
 }
 
 // Few rows: is the swapped kernel the better one? `other`: the estimate of the best other form (0: none, narrow products). One wave of
-// clusters of 2 s CTAs (two waves where all rows are one tile), max(0.42, rows / 700) us per k-block of a pair's share, 10 us for the launch,
+// clusters of 2 s CTAs (two waves where all rows are one tile), max(0.42, rows / 700) us per k-block of a pair's share, 7 us for the launch,
 // 3.5 for the exchange of a split, 0.5 per 64 rows for the store. Measured (us, best of the other forms | this, back to back): 281 rows x 3584
 // x 18944 58 | 46, x 37888 x 3584 85 | 71, x 3584 x 3584 21.0 | 19.7; 24 x 4608 x 3584 18.8 | 16.0, x 3584 x 3584 18.7 | 14.5; 256 x 5120 x 5120
 // 27 | 25, x 3584 x 5120 26 | 21; 1024 x 1280 x 5120 27 | 24; 2090 x 3584 x 18944 219 | 210; others stay for 24 x 37888 x 3584 46 | 55, x 3584
@@ -1251,7 +1264,7 @@ static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_
     const int dev = current_device();
     int fit[kSwapSplits + 1];
     for (int sp = 1; sp <= kSwapSplits; ++sp) fit[sp] = max_clusters(dev, sp, num_sms);
-    double best = 0.95 * other;
+    double best = 0.98 * other;
     bool found = false;
     for (int tiles = t0; tiles <= 2 * t0 + 2; ++tiles) {
         const int bm = ((M + tiles - 1) / tiles + 31) / 32 * 32, m_tiles = (M + bm - 1) / bm, units = m_tiles * n_tiles;
@@ -1261,7 +1274,7 @@ static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_
             if (waves > (sp == 1 && m_tiles == 1 ? 2 : 1) || nkb < 4 * sp) continue;
             const SwapTile t = make_swap(bm, sp);
             if (sp > 1 && bm * BLOCK_M * 4 > t.stages * t.stage_bytes) continue;
-            const double us = 10.0 + waves * ((nkb + sp - 1) / sp) * std::max(0.42, bm / 700.0) + 0.5 * bm / 64 + (sp > 1 ? 3.5 : 0.0);
+            const double us = 7.0 + waves * ((nkb + sp - 1) / sp) * std::max(0.42, bm / 700.0) + 0.5 * bm / 64 + (sp > 1 ? 3.5 : 0.0);
             if (us < best) { best = us; *bm_out = bm; *splits_out = sp; found = true; }
         }
     }
@@ -1366,8 +1379,9 @@ static int try_splitk(const GemmArgs& a, int num_sms, cudaStream_t stream, doubl
 GemmPlan gemm_plan(const GemmArgs& a, int num_sms) {
     GemmPlan p;
     double us = 0., split_us = 0.;
-    const int width = choose_pair(a.M, a.N, a.K, num_sms, &us);
-    p.width = width ? width : choose_bn(a.M, a.N, num_sms);
+    p.width = choose_alone(a.M, a.N, a.K, num_sms, &us);
+    const int width = choose_pair(a.M, a.N, a.K, num_sms, us, &us);
+    if (width) p.width = width;
     if (width) p.form = FORM_PAIR;
     if (try_splitk(a, num_sms, nullptr, &split_us) > 0) { us = split_us; p.form = FORM_ONE; }
     int bm = 0, splits = 0;
@@ -1409,12 +1423,12 @@ int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream) {
     if (choose) {
         const GemmPlan p = gemm_plan(a, num_sms);
         if (p.form == FORM_SWAP) return launch_epi_swap(a, p.width, p.splits, num_sms, stream);
-        if (p.form == FORM_PAIR) width = p.width;
+        width = p.form == FORM_PAIR ? -p.width : p.width;
     }
     if (plain)
         if (int r = try_splitk(a, num_sms, stream)) return r < 0 ? r : 0;
     int block_n = a.block_n;
-    if (block_n == 0) block_n = forced > 0 ? forced : (width ? -width : choose_bn(a.M, a.N, num_sms));
+    if (block_n == 0) block_n = forced > 0 ? forced : (width ? width : choose_bn(a.M, a.N, num_sms));
     // block_n < 0: the CTA pair's kernel with tile width -block_n
     const bool pair = block_n < 0 && plain && a.epi != EPI_SIGMOID_GATE && (a.epi <= EPI_SWIGLU || block_n % 32 == 0);
     if (block_n < 0) block_n = -block_n;

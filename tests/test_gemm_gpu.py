@@ -254,3 +254,18 @@ def test_gemm_splitk_exact_integer_operands(ctx, M, N, K):
     assert torch.equal(out, (acc.to(torch.bfloat16).float() + res.float()).to(torch.bfloat16))
     out = ctx.gemm(a, b, bias=bias, residual=res, epilogue=A.EPI_BIAS_RESIDUAL, splitk_ws=ws)
     assert torch.equal(out, ((acc + bias.float()).to(torch.bfloat16).float() + res.float()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("M,N,K,width", [(1024, 1280, 1176, 96), (1000, 5112, 1280, 160), (2090, 4600, 3584, 192), (1020, 3832, 1288, 224)])
+@pytest.mark.parametrize("epi", [A.EPI_NONE, A.EPI_BIAS, A.EPI_BIAS_RESIDUAL])
+def test_gemm_widths_between_128_and_256(ctx, M, N, K, width, epi):
+    """Products whose last wave only a width in between fills take one CTA per tile of that width, with ragged rows, columns and k; sums of
+    integers are exact, so they equal the 128-column kernel's bit for bit."""
+    assert ctx.gemm_plan(M, N, K)[:2] == (0, width)
+    a, b = _ints((M, K), -1, 1, 51), _ints((N, K), -1, 1, 52)
+    kw = {}
+    if epi != A.EPI_NONE:
+        kw["bias"] = _ints((N,), -8, 8, 53)
+    if epi == A.EPI_BIAS_RESIDUAL:
+        kw["residual"] = _ints((M, N), -8, 8, 54)
+    assert torch.equal(ctx.gemm(a, b, epilogue=epi, **kw), ctx.gemm(a, b, epilogue=epi, block_n=128, **kw))
