@@ -9,11 +9,13 @@
 // over blocks that turns them into the state entering each block, and the outputs. All arithmetic is fp32 on the
 // CUDA cores (the recurrence's operands are fp32 by the models' precision rules); the three products are register-
 // tiled 64 x 64 tiles whose operands are formed (decay factors applied) while they are staged into shared memory.
+#include <type_traits>
 #include <math.h>
 
 #include <algorithm>
 
 #include "common.cuh"
+#include "mma.cuh"
 #include "launch.h"
 #include "seqmix.h"
 
@@ -532,6 +534,252 @@ __global__ void __launch_bounds__(128) chunk_output_head_kernel(ChunkArgs a, Seq
     }
 }
 
+// ---- the three products of bf16 rows on the tensor cores -------------------------------------------------------------------
+// Rows of c, k and u are bf16, so one operand of every product is exact; the other is fp32 (a state, decayed weights) and is cut into
+// three bf16 values that hold all its 24 bits (truncated, so that none overflows): the products of mma.sync are then exact too, and only the
+// order of the fp32 sums differs from the kernels above (which fp32 rows keep). Decays and scales stay fp32. Bound by the bytes of the
+// block states, and the cuts (2048 rows, 64 heads of 64 x 128): 7.6 + 32 + 78 us for 16 + 66 + 119 of the fp32 kernels.
+__device__ __forceinline__ float low_part(float x) {   // x minus its leading 8 bits; nothing behind an infinity or NaN
+    return fabsf(x) < INFINITY ? x - __uint_as_float(__float_as_uint(x) & 0xffff0000u) : 0.f;
+}
+__device__ __forceinline__ void cut3(float x0, float x1, uint32_t (&c)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        c[i] = __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632);
+        if (i < 2) { x0 = low_part(x0); x1 = low_part(x1); }
+    }
+}
+constexpr int UP = 64 + 8;      // pitch of a staged bf16 tile row: ldmatrix rows fall into different banks
+// four consecutive k of rows r and r + 8 as an A fragment: which of a product's 16 places a k takes does not matter, as long as B agrees
+__device__ __forceinline__ void rows_a(uint32_t (&a)[4], const bf16* src, int ld, int r, int rows, int k, int cols) {
+    const uint2 z = make_uint2(0u, 0u);
+    const uint2 lo = r < rows && k < cols ? *reinterpret_cast<const uint2*>(src + (size_t)r * ld + k) : z;
+    const uint2 hi = r + 8 < rows && k < cols ? *reinterpret_cast<const uint2*>(src + (size_t)(r + 8) * ld + k) : z;
+    a[0] = lo.x; a[1] = hi.x; a[2] = lo.y; a[3] = hi.y;
+}
+
+__global__ void __launch_bounds__(128) chunk_products_tc_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
+    if (seq_done(pos)) return;
+    const int blk = blockIdx.x, g = blockIdx.y, groups = gridDim.y;
+    const int t0 = blk * CL, len = min(CL, a.S - t0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+    const bf16* gc = (const bf16*)a.c + (size_t)(a.row0 + t0) * a.ld_c + (size_t)g * a.N;
+    const bf16* gk = (const bf16*)a.k + (size_t)(a.row0 + t0) * a.ld_k + (size_t)g * a.N;
+    float acc[4][2][4] = {};
+#pragma unroll 2
+    for (int n0 = 0; n0 < a.N; n0 += 16) {
+        uint32_t kb[4], ca[4][4];   // rows s of this warp's two tiles of 8
+        rows_a(kb, gk, a.ld_k, warp * 16 + gq, len, n0 + 4 * tq, a.N);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rows_a(ca[i], gc, a.ld_c, i * 16 + gq, len, n0 + 4 * tq, a.N);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            mma_bf16_16816(acc[i][0], ca[i], kb[0], kb[2]);
+            mma_bf16_16816(acc[i][1], ca[i], kb[1], kb[3]);
+        }
+    }
+    float* out = a.ws_m + ((size_t)blk * groups + g) * CL * CL + warp * 16 + 2 * tq;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            *reinterpret_cast<float2*>(out + (i * 16 + gq) * CL + j * 8) = make_float2(acc[i][j][0], acc[i][j][1]);
+            *reinterpret_cast<float2*>(out + (i * 16 + gq + 8) * CL + j * 8) = make_float2(acc[i][j][2], acc[i][j][3]);
+        }
+}
+
+// a warp: 16 of the tile's 64 channels p, 64 key channels n at a time
+__global__ void __launch_bounds__(128) chunk_state_tc_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
+    if (seq_done(pos)) return;
+    __shared__ __align__(16) bf16 su[3][CL][UP], sk[CL][UP];   // [row s][p], cut in three; [row s][n]
+    __shared__ float rowf[CL];   // per row: the step scale times the decay from the row to the block's end
+    const int blk = blockIdx.x / a.heads, h = blockIdx.x % a.heads, g = h / a.heads_per_group;
+    const int p0 = blockIdx.y * TS;
+    const int t0 = blk * CL, len = min(CL, a.S - t0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+    const bf16* gu = (const bf16*)a.u + (size_t)(a.row0 + t0) * a.ld_u + (size_t)h * a.P + p0;
+    const bf16* gk = (const bf16*)a.k + (size_t)(a.row0 + t0) * a.ld_k + (size_t)g * a.N;
+    const float* gb = a.la + (size_t)(a.row0 + t0) * a.heads + h;
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    uint4 ur[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int e = threadIdx.x + i * 128, r = e >> 3, c = (e & 7) * 8;
+        ur[i] = r < len && p0 + c < a.P ? *reinterpret_cast<const uint4*>(gu + (size_t)r * a.ld_u + c) : z;
+    }
+    if (threadIdx.x < CL) {
+        const int s = threadIdx.x;
+        rowf[s] = s < len ? (a.sc ? a.sc[(size_t)(a.row0 + t0 + s) * a.heads + h] : 1.f) *
+                                expf(fminf(gb[(size_t)(len - 1) * a.heads] - gb[(size_t)s * a.heads], 0.f))
+                          : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int e = threadIdx.x + i * 128, r = e >> 3, c = (e & 7) * 8;
+        const uint32_t w[4] = {ur[i].x, ur[i].y, ur[i].z, ur[i].w};
+        uint32_t q[3][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 f = unpack_bf16x2(w[j]);
+            uint32_t t[3];
+            cut3(f.x * rowf[r], f.y * rowf[r], t);
+            q[0][j] = t[0]; q[1][j] = t[1]; q[2][j] = t[2];
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint4*>(&su[k][r][c]) = make_uint4(q[k][0], q[k][1], q[k][2], q[k][3]);
+    }
+    float* out = a.ws_s + ((size_t)blk * a.heads + h) * a.P * a.N;
+    const int p = p0 + warp * 16 + gq;
+    for (int n0 = 0; n0 < a.N; n0 += 64) {
+        uint4 kr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int e = threadIdx.x + i * 128, r = e >> 3, c = (e & 7) * 8;
+            kr[i] = r < len && n0 + c < a.N ? *reinterpret_cast<const uint4*>(gk + (size_t)r * a.ld_k + n0 + c) : z;
+        }
+        if (n0) __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int e = threadIdx.x + i * 128;
+            *reinterpret_cast<uint4*>(&sk[e >> 3][(e & 7) * 8]) = kr[i];
+        }
+        __syncthreads();
+        float acc[8][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < CL; ks += 16) {
+            uint32_t b[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                ldmatrix_x4_trans(b[j][0], b[j][1], b[j][2], b[j][3], &sk[ks + (lane & 7) + ((lane >> 3) & 1) * 8][j * 16 + (lane >> 4) * 8]);
+#pragma unroll
+            for (int k = 2; k >= 0; --k) {   // the smallest part first
+                uint32_t w[4];
+                ldmatrix_x4_trans(w[0], w[1], w[2], w[3], &su[k][ks + (lane & 7) + (lane >> 4) * 8][warp * 16 + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    mma_bf16_16816(acc[2 * j], w, b[j][0], b[j][1]);
+                    mma_bf16_16816(acc[2 * j + 1], w, b[j][2], b[j][3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int n = n0 + j * 8 + 2 * tq;
+            if (n >= a.N) continue;
+            if (p < a.P) *reinterpret_cast<float2*>(out + (size_t)p * a.N + n) = make_float2(acc[j][0], acc[j][1]);
+            if (p + 8 < a.P) *reinterpret_cast<float2*>(out + (size_t)(p + 8) * a.N + n) = make_float2(acc[j][2], acc[j][3]);
+        }
+    }
+}
+
+// a warp: all 64 rows of 16 of the tile's channels, so that every state is cut once
+__global__ void __launch_bounds__(128) chunk_output_tc_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
+    if (seq_done(pos)) return;
+    __shared__ __align__(16) bf16 sm[3][CL][UP], su[CL][UP];   // the block's own weights [t][s], cut in three; [row s][p]
+    __shared__ float bt[CL], into[CL], scs[CL];   // per row: cumulative log decay, cs x decay from the block's start, cs x step scale
+    const int blk = blockIdx.x / a.heads, h = blockIdx.x % a.heads, g = h / a.heads_per_group;
+    const int p0 = blockIdx.y * TS;
+    const int t0 = blk * CL, len = min(CL, a.S - t0);
+    const int N = a.N, P = a.P;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+    const bf16* gu = (const bf16*)a.u + (size_t)(a.row0 + t0) * a.ld_u + (size_t)h * P + p0;
+    const bf16* gc = (const bf16*)a.c + (size_t)(a.row0 + t0) * a.ld_c + (size_t)g * N;
+    const float* sin = a.ws_s + ((size_t)blk * a.heads + h) * P * N;
+    const float* gm = a.ws_m + ((size_t)blk * (a.heads / a.heads_per_group) + g) * CL * CL;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int e = threadIdx.x + i * 128, r = e >> 3, c = (e & 7) * 8;
+        *reinterpret_cast<uint4*>(&su[r][c]) = r < len && p0 + c < P ? *reinterpret_cast<const uint4*>(gu + (size_t)r * a.ld_u + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (threadIdx.x < CL) {
+        const int t = threadIdx.x;
+        const float b = t < len ? a.la[(size_t)(a.row0 + t0 + t) * a.heads + h] : 0.f;
+        bt[t] = b;
+        into[t] = t < len ? a.cs * expf(b) : 0.f;
+        scs[t] = t < len ? a.cs * (a.sc ? a.sc[(size_t)(a.row0 + t0 + t) * a.heads + h] : 1.f) : 0.f;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < CL * CL / 4; e += 128) {   // the block's own rows: M[t, s], s <= t
+        const int t = e >> 4, s = (e & 15) * 4;
+        const float4 q = s <= t ? *reinterpret_cast<const float4*>(gm + t * CL + s) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float v[4] = {q.x, q.y, q.z, q.w};
+        float m[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m[i] = s + i <= t && t < len ? v[i] * scs[s + i] * expf(fminf(bt[t] - bt[s + i], 0.f)) : 0.f;
+        uint32_t c0[3], c1[3];
+        cut3(m[0], m[1], c0);
+        cut3(m[2], m[3], c1);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(&sm[k][t][s]) = make_uint2(c0[k], c1[k]);
+    }
+    float acc[4][2][4] = {};
+#pragma unroll 2
+    for (int n0 = 0; n0 < N; n0 += 16) {       // the entering state, seen through the queries
+        const int n = n0 + 4 * tq;
+        float4 st[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int p = p0 + warp * 16 + j * 8 + gq;
+            st[j] = p < P && n < N ? *reinterpret_cast<const float4*>(sin + (size_t)p * N + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        uint32_t ca[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rows_a(ca[i], gc, a.ld_c, i * 16 + gq, len, n, N);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            uint32_t b0[3], b1[3];
+            cut3(st[j].x, st[j].y, b0);
+            cut3(st[j].z, st[j].w, b1);
+#pragma unroll
+            for (int k = 2; k >= 0; --k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mma_bf16_16816(acc[i][j], ca[i], b0[k], b1[k]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float f0 = into[i * 16 + gq], f1 = into[i * 16 + gq + 8];
+            acc[i][j][0] *= f0; acc[i][j][1] *= f0;
+            acc[i][j][2] *= f1; acc[i][j][3] *= f1;
+        }
+    __syncthreads();
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b[0], b[1], b[2], b[3], &su[ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][warp * 16 + (lane >> 4) * 8]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i < ks) continue;   // rows above these keys
+#pragma unroll
+            for (int k = 2; k >= 0; --k) {
+                uint32_t w[4];
+                ldmatrix_x4(w[0], w[1], w[2], w[3], &sm[k][i * 16 + (lane & 15)][ks * 16 + (lane >> 4) * 8]);
+                mma_bf16_16816(acc[i][0], w, b[0], b[1]);
+                mma_bf16_16816(acc[i][1], w, b[2], b[3]);
+            }
+        }
+    }
+    const float skip = a.skip ? a.skip[h] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int t = i * 16 + gq + 8 * r, c = warp * 16 + j * 8 + 2 * tq;
+                if (t >= len || p0 + c >= P) continue;
+                const float2 u = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&su[t][c]));
+                *reinterpret_cast<float2*>(a.y + (size_t)(a.row0 + t0 + t) * a.ld_y + (size_t)h * P + p0 + c) =
+                    make_float2(acc[i][j][2 * r] + skip * u.x, acc[i][j][2 * r + 1] + skip * u.y);
+            }
+}
+
 template <typename T, bool VEC>
 int run_chunked(const ScanArgs& s, SeqPos pos, cudaStream_t st) {
     const size_t per_block = (size_t)s.heads * ((size_t)CL * CL + (size_t)s.P * s.N);
@@ -554,14 +802,20 @@ int run_chunked(const ScanArgs& s, SeqPos pos, cudaStream_t st) {
             const bool rows16 = ((s.N | s.P | s.ld_k | s.ld_c | s.ld_u) % V) == 0 && ((s.N | s.P | s.ld_y) % 4) == 0 &&
                                 (((uintptr_t)s.k | (uintptr_t)s.c | (uintptr_t)s.u | (uintptr_t)s.y | (uintptr_t)s.state | (uintptr_t)a.ws_m | (uintptr_t)a.ws_s) % 16) == 0;
             if (rows16) {
-                count_launch();
-                chained(chunk_products_kernel<T>, dim3(nb, s.heads / s.heads_per_group), 128, 0, st)(a, pos);
-                count_launch();
-                chained(chunk_state_head_kernel<T>, dim3(nb * s.heads, (s.P + TS - 1) / TS), 128, 0, st)(a, pos);
-                count_launch();
-                chained(chunk_prefix4_kernel, (unsigned)((per_state / 4 + 255) / 256), 256, 0, st)(a, nb, pos);
-                count_launch();
-                chained(chunk_output_head_kernel<T>, dim3(nb * s.heads, (s.P + TS - 1) / TS), 128, 0, st)(a, pos);
+                const dim3 tiles(nb * s.heads, (s.P + TS - 1) / TS), pairs(nb, s.heads / s.heads_per_group);
+                const unsigned prefix = (unsigned)((per_state / 4 + 255) / 256);
+                for (int i = 0; i < 4; ++i) count_launch();
+                if constexpr (std::is_same_v<T, bf16>) {
+                    chained(chunk_products_tc_kernel, pairs, 128, 0, st)(a, pos);
+                    chained(chunk_state_tc_kernel, tiles, 128, 0, st)(a, pos);
+                    chained(chunk_prefix4_kernel, prefix, 256, 0, st)(a, nb, pos);
+                    chained(chunk_output_tc_kernel, tiles, 128, 0, st)(a, pos);
+                } else {
+                    chained(chunk_products_kernel<T>, pairs, 128, 0, st)(a, pos);
+                    chained(chunk_state_head_kernel<T>, tiles, 128, 0, st)(a, pos);
+                    chained(chunk_prefix4_kernel, prefix, 256, 0, st)(a, nb, pos);
+                    chained(chunk_output_head_kernel<T>, tiles, 128, 0, st)(a, pos);
+                }
                 continue;
             }
         }
