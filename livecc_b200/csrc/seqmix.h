@@ -176,7 +176,8 @@ int qk_norm_kv_append(int dt, const void* proj, int ld, const float* qn_w, const
 // ld_gate) or null; out: [S, Hq*DV] (storage dt). chunk <= 0 means one chunk (plain causal attention).
 // Three kernels: one CTA per (row, head) for decode steps and portions of fewer than kAttnTiledMin rows; a tiled fp32
 // CUDA-core kernel for longer portions; and, for bf16 storage with head size <= kAttnMmaMaxDim when tensor_cores is set,
-// the same tiling with both products on the tensor cores (bf16 operands, fp32 accumulation, fp32 softmax).
+// the same tiling with both products on the tensor cores (bf16 operands, fp32 accumulation, fp32 softmax); heads of 128 with plain
+// masks take the tcgen05 kernel (attn_local_tc below).
 constexpr int kAttnTiledMin = 16;
 constexpr int kAttnMmaMaxDim = 256;
 // sink: fp32 [Hq] sink logits (null: 0 for every head); the sink adds exp(sink[h]) to the denominator and nothing else.

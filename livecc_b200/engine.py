@@ -461,7 +461,7 @@ class LiveCCB200ForConditionalGeneration:
             raise ValueError("max_new_tokens must be >= 1")
 
     def _pick_nsplit(self, kv_tokens: int) -> int:
-        """Split-KV factor of the per-op decode attention (unused by the persistent kernel, which plans its own items)."""
+        """Split-KV factor of the per-op decode attention (batched steps choose their own)."""
         kv_tiles = (kv_tokens + 63) // 64
         div = int(os.environ.get("LIVECC_B200_NSPLIT_DIV", "2"))
         want = max(1, (kv_tiles + div - 1) // div)   # about 2 KV tiles (128 tokens) per split while the SMs have room
@@ -581,7 +581,7 @@ class LiveCCB200ForConditionalGeneration:
 
     # ------------------------------------------------------------------------------------------
     def _run_decode(self, caches, sts, sp: _cabi.Sampling, n_steps: int, nsplit: int, logits_hist=None):
-        """n_steps decode steps for one stream (caches = [cache]) or a batch (<= 8 caches, persistent kernel)."""
+        """n_steps decode steps for one stream (caches = [cache]) or a batch (<= 8 caches)."""
         B = len(caches)
 
         def launch(n):
