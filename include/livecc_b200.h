@@ -176,6 +176,16 @@ int lcc_gemv_norm_logits(lcc_ctx* ctx, const void* W, int ldw, const void* x, co
                          float* logits, float* logits_copy, int N, int K, const int32_t* scalars,
                          lcc_stream_t stream);
 
+/* The projections of one decode step of B <= 8 streams (lcc_decode_batch), rows ldx / ldo elements apart: W x + bias; out += W x; silu(gate) * up
+ * of rows interleaved by 16, out [B, N/2]; fp32 logits, twice. N a multiple of 32, K of 64, W dense. A stream whose scalars say that it is
+ * finished keeps its row. scalars: B device pointers in a host array. */
+#define LCC_GEMV_BIAS 0
+#define LCC_GEMV_RESIDUAL 1
+#define LCC_GEMV_SWIGLU 2
+#define LCC_GEMV_LOGITS 3
+int lcc_gemv_batch(lcc_ctx* ctx, int kind, const void* W, const void* x, int ldx, int N, int K, int B, const int32_t* const* scalars,
+                   const void* bias, void* out, void* out2, int ldo, lcc_stream_t stream);
+
 /* Logits processing + greedy token selection + stream bookkeeping (gen/utils.py:2762-2805;
  * logits_process.py:407-410; REF/demo/infer.py:10-23). */
 typedef struct {

@@ -478,6 +478,21 @@ class Context:
                   _ptr(lg2), _i(W.shape[0]), _i(W.shape[1]), _ptr(scalars), self.stream_ptr())
         return lg, lg2
 
+    def gemv_batch(self, kind, W, x, scalars, bias=None, out=None):
+        """kind (LCC_GEMV_*): 0 W x + bias, 1 out += W x, 2 silu(gate) * up, 3 fp32 logits; x [B, K], scalars a list of B int32 tensors."""
+        import torch
+
+        B, (N, K) = x.shape[0], W.shape
+        out2 = None
+        if kind == 3:
+            out, out2 = (torch.empty((B, N), dtype=torch.float32, device=W.device) for _ in range(2))
+        elif out is None:
+            out = torch.empty((B, N // 2 if kind == 2 else N), dtype=torch.bfloat16, device=W.device)
+        sc = (C.c_void_p * B)(*[t.data_ptr() for t in scalars])
+        self.call("lcc_gemv_batch", _i(kind), _ptr(W), _ptr(x), _i(x.stride(0)), _i(N), _i(K), _i(B), sc, _ptr(bias), _ptr(out), _ptr(out2),
+                  _i(out.stride(0)), self.stream_ptr())
+        return out if out2 is None else (out, out2)
+
     def sample_greedy(self, logits_raw, logits_proc, seq, scalars, sampling: Sampling, advance_kv, embed, h):
         self.call("lcc_sample_greedy", _ptr(logits_raw), _ptr(logits_proc), _i(logits_raw.numel()), _ptr(seq),
                   _ptr(scalars), C.byref(sampling), _i(advance_kv), _ptr(embed), _ptr(h), _i(embed.shape[1]),

@@ -119,6 +119,23 @@ int lcc_gemv_norm_logits(lcc_ctx* ctx, const void* W, int ldw, const void* x, co
            "lcc_gemv_norm_logits");
 }
 
+int lcc_gemv_batch(lcc_ctx* ctx, int kind, const void* W, const void* x, int ldx, int N, int K, int B, const int32_t* const* scalars,
+                   const void* bias, void* out, void* out2, int ldo, lcc_stream_t stream) {
+    if (!ctx) return -1;
+    if (B < 1 || B > lcc::kBatchStreams || !scalars) LCC_FAIL(ctx, -2, "lcc_gemv_batch: 1..%d streams with their scalars", lcc::kBatchStreams);
+    const int* fin[lcc::kBatchStreams];
+    for (int b = 0; b < B; ++b) fin[b] = scalars[b] + LCC_SC_FINISHED;
+    const lcc::GemvBatch a{(const bf16*)W, (const bf16*)x, N, K, ldx, B, fin, nullptr, nullptr, 0};
+    cudaStream_t s = (cudaStream_t)stream;
+    switch (kind) {
+        case LCC_GEMV_BIAS: OP_RET(ctx, lcc::gemv_batch_bias(a, (const bf16*)bias, (bf16*)out, ldo, s), "lcc_gemv_batch");
+        case LCC_GEMV_RESIDUAL: OP_RET(ctx, lcc::gemv_batch_residual(a, (bf16*)out, ldo, s), "lcc_gemv_batch");
+        case LCC_GEMV_SWIGLU: OP_RET(ctx, lcc::gemv_batch_swiglu(a, (bf16*)out, ldo, s), "lcc_gemv_batch");
+        case LCC_GEMV_LOGITS: OP_RET(ctx, lcc::gemv_batch_logits(a, (float*)out, (float*)out2, ldo, s), "lcc_gemv_batch");
+    }
+    LCC_FAIL(ctx, -2, "lcc_gemv_batch: no projection %d", kind);
+}
+
 // ---- frame ingest: antialiased bicubic uint8 resize (resize.cu) ----
 struct lcc_resize_plan {
     lcc::ResizePlan* impl;

@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(kGbWarps * 32) gemv_batch_kernel(const GemvBat
     __shared__ float part[kGbWarps][MT * 128];   // [row][stream] per warp
     __shared__ float peers[KS][MT * 128];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    if (KS > 1) cluster_arrive();   // waited for in front of the first store into another CTA's shared memory: that CTA has started
     const int tile = blockIdx.x / KS, rank = KS > 1 ? blockIdx.x % KS : 0;
     const int n0 = tile * MT * 16;
     const int units = p.K >> 6, mine = (units + KS - 1) / KS;
@@ -109,6 +110,8 @@ __global__ void __launch_bounds__(kGbWarps * 32) gemv_batch_kernel(const GemvBat
         for (int k = 0; k < kGbWarps; ++k) sum += part[k][i];
     }
     if (KS > 1) {
+        __syncwarp();
+        cluster_wait();
         if (i < MT * 128) {
             const uint32_t a = mapa_shared(smem_u32(&peers[rank][i]), 0);
             asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(sum) : "memory");
