@@ -557,6 +557,16 @@ typedef struct {
     void* const* v_pages;
 } lcc_seq_entry;
 
+/* The gated linear recurrence of the state-space, retention and linear-attention layers by itself (tests and tuning), one state St [N, P] per head:
+ * St <- diag(exp(log_decay_t)) St + k_t (sc_t u_t)^T, y_t = St^T (cs c_t) + skip u_t. k, c: [S, ld], head h reads columns (h / heads_per_group) * N ..;
+ * u: [S, ld_u], columns h * P ..; log_decay: fp32 [S, heads] or, with vec_decay, [S, heads * N], overwritten; sc fp32 [S, heads] or NULL;
+ * skip fp32 [heads] or NULL; state fp32 [heads, P, N], read and written; y fp32 [S, ld_y]. ws (optional): fp32 workspace of
+ * lcc_gated_scan_ws_floats elements, with which 32 rows or more run in blocks of 64. */
+int lcc_gated_scan(lcc_ctx* ctx, int dt, const void* k, int ld_k, const void* c, int ld_c, const void* u, int ld_u, float* log_decay, int vec_decay,
+                   const float* sc, const float* skip, float cs, float* state, float* y, int ld_y, int S, int heads, int heads_per_group, int N, int P,
+                   float* ws, int64_t ws_floats, lcc_stream_t stream);
+int64_t lcc_gated_scan_ws_floats(int S, int heads, int N, int P);
+
 typedef struct lcc_seq_model lcc_seq_model;
 /* sizeof(lcc_seq_layer) (which = 0), sizeof(lcc_seq_model_desc) (1), sizeof(lcc_seq_entry) (2): a binding checks its own layout against them */
 size_t lcc_seq_struct_bytes(int which);

@@ -493,6 +493,23 @@ class Context:
                   _i(out.stride(0)), self.stream_ptr())
         return out if out2 is None else (out, out2)
 
+    def gated_scan(self, k, c, u, log_decay, state, sc=None, skip=None, cs=1.0, blocks=True):
+        """y of the gated linear recurrence; k, c [S, G, N], u [S, H, P] (bf16, or all fp32), log_decay [S, H] or [S, H, N] fp32, state fp32
+        [H, P, N], updated. blocks: the form over blocks of 64 rows (32 rows or more) instead of token by token."""
+        import torch
+
+        (S, G, N), (_, H, P) = k.shape, u.shape
+        y = torch.empty((S, H, P), dtype=torch.float32, device=u.device)
+        la = log_decay.clone()
+        ws = None
+        if blocks:
+            self.lib.lcc_gated_scan_ws_floats.restype = C.c_int64
+            ws = torch.empty(self.lib.lcc_gated_scan_ws_floats(_i(S), _i(H), _i(N), _i(P)), dtype=torch.float32, device=u.device)
+        self.call("lcc_gated_scan", _i(0 if u.dtype == torch.bfloat16 else 1), _ptr(k), _i(k.stride(0)), _ptr(c), _i(c.stride(0)), _ptr(u), _i(u.stride(0)),
+                  _ptr(la), _i(la.dim() == 3), _ptr(sc), _ptr(skip), C.c_float(cs), _ptr(state), _ptr(y), _i(y.stride(0)), _i(S), _i(H), _i(H // G),
+                  _i(N), _i(P), _ptr(ws), C.c_int64(ws.numel() if ws is not None else 0), self.stream_ptr())
+        return y
+
     def sample_greedy(self, logits_raw, logits_proc, seq, scalars, sampling: Sampling, advance_kv, embed, h):
         self.call("lcc_sample_greedy", _ptr(logits_raw), _ptr(logits_proc), _i(logits_raw.numel()), _ptr(seq),
                   _ptr(scalars), C.byref(sampling), _i(advance_kv), _ptr(embed), _ptr(h), _i(embed.shape[1]),

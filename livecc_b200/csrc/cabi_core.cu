@@ -5,6 +5,7 @@
 #include "gemm.h"
 #include "launch.h"
 #include "ops.h"
+#include "seqmix.h"
 
 #include <deque>
 #include <mutex>
@@ -135,6 +136,20 @@ int lcc_gemm_form(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, 
         LCC_CHECK_LAUNCH(ctx, name);                                         \
         return 0;                                                            \
     } while (0)
+
+int lcc_gated_scan(lcc_ctx* ctx, int dt, const void* k, int ld_k, const void* c, int ld_c, const void* u, int ld_u, float* log_decay, int vec_decay,
+                   const float* sc, const float* skip, float cs, float* state, float* y, int ld_y, int S, int heads, int heads_per_group, int N, int P,
+                   float* ws, int64_t ws_floats, lcc_stream_t stream) {
+    lcc::ScanArgs a{};
+    a.dt = dt; a.k = k; a.ld_k = ld_k; a.c = c; a.ld_c = ld_c; a.u = u; a.ld_u = ld_u;
+    a.a = log_decay; a.vec_decay = vec_decay; a.sc = sc; a.skip = skip; a.cs = cs; a.state = state; a.y = y; a.ld_y = ld_y;
+    a.S = S; a.heads = heads; a.heads_per_group = heads_per_group; a.N = N; a.P = P;
+    a.ws = ws; a.ws_floats = ws_floats > 0 ? (size_t)ws_floats : 0;
+    if (dt != lcc::DT_F32 && dt != lcc::DT_BF16) return -1;
+    OP_RET(ctx, lcc::gated_scan(a, lcc::SeqPos{}, (cudaStream_t)stream), "lcc_gated_scan");
+}
+
+int64_t lcc_gated_scan_ws_floats(int S, int heads, int N, int P) { return (int64_t)lcc::gated_scan_ws_floats(S, heads, N, P); }
 
 int lcc_sample_greedy(lcc_ctx* ctx, const float* logits_raw, float* logits_proc, int V, int64_t* seq,
                       int32_t* scalars, const lcc_sampling* sp, int advance_kv, const void* embed, void* h,

@@ -558,6 +558,47 @@ __device__ __forceinline__ void rows_a(uint32_t (&a)[4], const bf16* src, int ld
     a[0] = lo.x; a[1] = hi.x; a[2] = lo.y; a[3] = hi.y;
 }
 
+// What an infinite or NaN entry of the uncut rows touches is summed again in plain fp32: the lower parts of most values are zero, and infinity
+// times zero is not what the product is. A block's state is when its k hold one; an output when it came out non-finite (as it always
+// does then). Not inlined and behind the rest, so that the others' registers and code stay as they are.
+__device__ __forceinline__ void absmax8(__nv_bfloat162& most, const uint4& q) {
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) most = __hmax2_nan(most, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[j])));
+}
+__device__ __noinline__ void state_plain(const bf16* u, int ld_u, const bf16* k, int ld_k, const float* rowf, float* out, int len, int P, int N) {
+    for (int e = threadIdx.x; e < P * N; e += blockDim.x) {
+        const int p = e / N, n = e % N;
+        float acc = 0.f;
+        for (int s = 0; s < len; ++s) acc = fmaf(rowf[s] * bf2f(u[(size_t)s * ld_u + p]), bf2f(k[(size_t)s * ld_k + n]), acc);
+        out[e] = acc;
+    }
+}
+// the 32 outputs of a thread of chunk_output_tc_kernel, those that are not finite
+__device__ __noinline__ void output_plain(const ChunkArgs& a) {
+    const int blk = blockIdx.x / a.heads, h = blockIdx.x % a.heads, g = h / a.heads_per_group;
+    const int row = a.row0 + blk * CL, len = min(CL, a.S - blk * CL), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float* m = a.ws_m + ((size_t)blk * (a.heads / a.heads_per_group) + g) * CL * CL;
+    const float* la = a.la + (size_t)row * a.heads + h;
+    for (int e = 0; e < 32; ++e) {
+        const int t = (e >> 3) * 16 + (lane >> 2) + 8 * ((e >> 1) & 1), p = blockIdx.y * TS + warp * 16 + ((e >> 2) & 1) * 8 + 2 * (lane & 3) + (e & 1);
+        if (t >= len || p >= a.P) continue;
+        float* y = a.y + (size_t)(row + t) * a.ld_y + (size_t)h * a.P + p;
+        if (isfinite(*y)) continue;
+        const bf16* c = (const bf16*)a.c + (size_t)(row + t) * a.ld_c + (size_t)g * a.N;
+        const bf16* u = (const bf16*)a.u + (size_t)row * a.ld_u + (size_t)h * a.P + p;
+        const float* sin = a.ws_s + (((size_t)blk * a.heads + h) * a.P + p) * a.N;
+        const float bt = la[(size_t)t * a.heads], into = a.cs * expf(bt);
+        float acc = 0.f;
+        for (int n = 0; n < a.N; ++n) acc = fmaf(into * bf2f(c[n]), sin[n], acc);
+        for (int s = 0; s <= t; ++s) {
+            const float sc = a.cs * (a.sc ? a.sc[(size_t)(row + s) * a.heads + h] : 1.f);
+            acc = fmaf(m[t * CL + s] * sc * expf(fminf(bt - la[(size_t)s * a.heads], 0.f)), bf2f(u[(size_t)s * a.ld_u]), acc);
+        }
+        *y = acc + (a.skip ? a.skip[h] : 0.f) * bf2f(u[(size_t)t * a.ld_u]);
+    }
+}
+
 __global__ void __launch_bounds__(128) chunk_products_tc_kernel(ChunkArgs a, SeqPos pos) {
     chain_begin();
     if (seq_done(pos)) return;
@@ -590,7 +631,8 @@ __global__ void __launch_bounds__(128) chunk_products_tc_kernel(ChunkArgs a, Seq
 }
 
 // a warp: 16 of the tile's 64 channels p, 64 key channels n at a time
-__global__ void __launch_bounds__(128) chunk_state_tc_kernel(ChunkArgs a, SeqPos pos) {
+// (five CTAs per SM: with six, whose 78 registers the compiler takes otherwise, a chained pass of three layers took 50 us more)
+__global__ void __launch_bounds__(128, 5) chunk_state_tc_kernel(ChunkArgs a, SeqPos pos) {
     chain_begin();
     if (seq_done(pos)) return;
     __shared__ __align__(16) bf16 su[3][CL][UP], sk[CL][UP];   // [row s][p], cut in three; [row s][n]
@@ -602,6 +644,7 @@ __global__ void __launch_bounds__(128) chunk_state_tc_kernel(ChunkArgs a, SeqPos
     const bf16* gu = (const bf16*)a.u + (size_t)(a.row0 + t0) * a.ld_u + (size_t)h * a.P + p0;
     const bf16* gk = (const bf16*)a.k + (size_t)(a.row0 + t0) * a.ld_k + (size_t)g * a.N;
     const float* gb = a.la + (size_t)(a.row0 + t0) * a.heads + h;
+    float* out = a.ws_s + ((size_t)blk * a.heads + h) * a.P * a.N;
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
     uint4 ur[4];
 #pragma unroll
@@ -631,7 +674,6 @@ __global__ void __launch_bounds__(128) chunk_state_tc_kernel(ChunkArgs a, SeqPos
 #pragma unroll
         for (int k = 0; k < 3; ++k) *reinterpret_cast<uint4*>(&su[k][r][c]) = make_uint4(q[k][0], q[k][1], q[k][2], q[k][3]);
     }
-    float* out = a.ws_s + ((size_t)blk * a.heads + h) * a.P * a.N;
     const int p = p0 + warp * 16 + gq;
     for (int n0 = 0; n0 < a.N; n0 += 64) {
         uint4 kr[4];
@@ -641,12 +683,17 @@ __global__ void __launch_bounds__(128) chunk_state_tc_kernel(ChunkArgs a, SeqPos
             kr[i] = r < len && n0 + c < a.N ? *reinterpret_cast<const uint4*>(gk + (size_t)r * a.ld_k + n0 + c) : z;
         }
         if (n0) __syncthreads();
+        __nv_bfloat162 most = __float2bfloat162_rn(0.f);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int e = threadIdx.x + i * 128;
             *reinterpret_cast<uint4*>(&sk[e >> 3][(e & 7) * 8]) = kr[i];
+            absmax8(most, kr[i]);
         }
-        __syncthreads();
+        if (__syncthreads_or(!isfinite(__low2float(most)) || !isfinite(__high2float(most)))) {
+            state_plain(gu, a.ld_u, gk, a.ld_k, rowf, out + (size_t)p0 * a.N, len, min(TS, a.P - p0), a.N);
+            return;
+        }
         float acc[8][4] = {};
 #pragma unroll
         for (int ks = 0; ks < CL; ks += 16) {
@@ -676,7 +723,7 @@ __global__ void __launch_bounds__(128) chunk_state_tc_kernel(ChunkArgs a, SeqPos
 }
 
 // a warp: all 64 rows of 16 of the tile's channels, so that every state is cut once
-__global__ void __launch_bounds__(128) chunk_output_tc_kernel(ChunkArgs a, SeqPos pos) {
+__global__ void __launch_bounds__(128, 4) chunk_output_tc_kernel(const __grid_constant__ ChunkArgs a, SeqPos pos) {
     chain_begin();
     if (seq_done(pos)) return;
     __shared__ __align__(16) bf16 sm[3][CL][UP], su[CL][UP];   // the block's own weights [t][s], cut in three; [row s][p]
@@ -766,6 +813,7 @@ __global__ void __launch_bounds__(128) chunk_output_tc_kernel(ChunkArgs a, SeqPo
         }
     }
     const float skip = a.skip ? a.skip[h] : 0.f;
+    float odd = 0.f;   // NaN once a value is not finite
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -775,9 +823,11 @@ __global__ void __launch_bounds__(128) chunk_output_tc_kernel(ChunkArgs a, SeqPo
                 const int t = i * 16 + gq + 8 * r, c = warp * 16 + j * 8 + 2 * tq;
                 if (t >= len || p0 + c >= P) continue;
                 const float2 u = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&su[t][c]));
-                *reinterpret_cast<float2*>(a.y + (size_t)(a.row0 + t0 + t) * a.ld_y + (size_t)h * P + p0 + c) =
-                    make_float2(acc[i][j][2 * r] + skip * u.x, acc[i][j][2 * r + 1] + skip * u.y);
+                const float2 v = make_float2(acc[i][j][2 * r] + skip * u.x, acc[i][j][2 * r + 1] + skip * u.y);
+                *reinterpret_cast<float2*>(a.y + (size_t)(a.row0 + t0 + t) * a.ld_y + (size_t)h * P + p0 + c) = v;
+                odd = fmaf(0.f, v.x, fmaf(0.f, v.y, odd));
             }
+    if (odd != 0.f) output_plain(a);
 }
 
 template <typename T, bool VEC>
