@@ -2,7 +2,7 @@
 // 8 columns of mma.sync m16n8k16, the weights its 16 rows, straight from global memory into the fragments: a lane's 16-byte load
 // is 8 consecutive k of one weight row, and because the same k are loaded of x, which 4 of a product's 16 places they take does not matter.
 //
-// HBM-bound: 7 TB/s of weights are 24 bytes per clock and SM, 12 products of 1 KB per 43 clocks; eight columns on the CUDA cores would be 96
+// HBM-bound: 7 TB/s of weights are 24 bytes per clock and SM, two products (512 bytes of weights each) per 43 clocks; eight columns on the CUDA cores would be 96
 // multiply-adds per clock and SM beside the unpacking. What a CTA needs is loads in flight: its 8 warps share the K of 16 or 32 rows
 // (a round of them reads 1 KB of each row), 8 to 16 loads of 16 bytes per lane, and add their partials through shared memory. x is read through L1.
 #include "common.cuh"
@@ -30,8 +30,8 @@ struct GemvBatchParams {
 
 constexpr int kGbWarps = 8;
 
-// Measured with 8 streams (hidden 3584; for comparison one stream's CUDA-core kernels): lm_head 160 us (172), gate/up 47 (43), down 28 (25),
-// qkv 9.0 (11.1, RMSNorm included), o 10.3 (9.6).
+// Measured with 8 streams (hidden 3584; for comparison one stream's CUDA-core kernels): lm_head 162 us (172), gate/up 43.9 (43), down 27.0 (25),
+// qkv 9.6 (11.1, RMSNorm included), o 10.9 (9.6; both 0.4 more since the streams' flags are looked at behind the first loads).
 // MT: 16-row tiles per CTA (GB_SWIGLU: 16 gate rows and their 16 up rows). KS: CTAs of a cluster that share K. UN: units of 64 k in flight.
 template <int MT, int KS, int UN, int EPI>
 __global__ void __launch_bounds__(kGbWarps * 32) gemv_batch_kernel(const GemvBatchParams p) {
@@ -73,11 +73,30 @@ __global__ void __launch_bounds__(kGbWarps * 32) gemv_batch_kernel(const GemvBat
         }
     };
     int u = u0 + warp;
-    for (; u + (UN - 1) * kGbWarps < u1; u += UN * kGbWarps) {
+    const int done = lane < p.B ? *p.finished[lane] : 1;
+    bool open = false;
+    auto ended = [&] {   // every stream has ended (a replayed graph): nothing to do, seen while the first weights arrive
+        if (open || !__all_sync(0xffffffffu, done)) { open = true; return false; }
+        if (KS > 1) cluster_wait();
+        return true;
+    };
+    if constexpr (UN == 1) {   // (the loop turned like this: gate/up 43.5 us, 48.4 as below; with 2 units in flight 35 for the 27 of the down projection)
+        if (u < u1) load(u, w[0]);
+        if (ended()) return;
+        while (u < u1) {
+            compute(u, w[0]);
+            u += kGbWarps;
+            if (u < u1) load(u, w[0]);
+        }
+    } else {
+        for (; u + (UN - 1) * kGbWarps < u1; u += UN * kGbWarps) {
 #pragma unroll
-        for (int i = 0; i < UN; ++i) load(u + i * kGbWarps, w[i]);
+            for (int i = 0; i < UN; ++i) load(u + i * kGbWarps, w[i]);
+            if (ended()) return;
 #pragma unroll
-        for (int i = 0; i < UN; ++i) compute(u + i * kGbWarps, w[i]);
+            for (int i = 0; i < UN; ++i) compute(u + i * kGbWarps, w[i]);
+        }
+        if (ended()) return;
     }
     if (UN > 1) {
 #pragma unroll
@@ -187,7 +206,7 @@ int gemv_batch_residual(const GemvBatch& a, bf16* h_inout, int ldo, cudaStream_t
 int gemv_batch_swiglu(const GemvBatch& a, bf16* act, int ldo, cudaStream_t s) {
     GemvBatchParams p = params_of(a);
     p.out = act; p.ldo = ldo;
-    return launch_batch<2, 1, 1, GB_SWIGLU>(p, s);   // (2 units in flight: 48.8 us for 47.3, lm_head 174 for 160: registers)
+    return launch_batch<2, 1, 1, GB_SWIGLU>(p, s);   // (2 units in flight were slower: registers)
 }
 int gemv_batch_logits(const GemvBatch& a, float* logits, float* logits_copy, int ldo, cudaStream_t s) {
     GemvBatchParams p = params_of(a);
