@@ -278,9 +278,10 @@ int lcc_vit_forward_frames(lcc_model* m, const uint8_t* frames, int T, int H, in
 int lcc_prefill(lcc_model* m, const lcc_stream_state* st, const int64_t* ids, const int32_t* pos3, int S,
                 int past, const void* video_embeds, int n_video_rows, const lcc_sampling* sp, int slot, lcc_stream_t stream);
 
-/* The same for the new tokens of up to 8 streams in one pass, so that every weight byte is read once for all of them: stream b gets slot
- * first_slot + b. States share one page pool; the workspace holds the sum of the S. Sums are taken in the order that the
- * number of rows calls for, so a stream's last bits may differ from those of lcc_prefill. */
+/* The same for the new tokens of up to 8 streams in one pass: stream b gets slot first_slot + b. States share one page pool; the workspace holds
+ * the sum of the S. Every stream has the bits that lcc_prefill gives it alone: a product is one launch over the neighbours whose sums it would cut
+ * alike (streams of up to some 130 tokens, or of similar length), attention splits each stream's keys by its own range, and the
+ * output head is read once. */
 typedef struct {
     lcc_stream_state st;
     const int64_t* ids;
@@ -299,9 +300,10 @@ int lcc_decode_steps(lcc_model* m, const lcc_stream_state* st, int n_steps, int 
 /* Batched decode (the reference demo admits 5 concurrent sessions on one model,
  * REF/demo/app.py:178): n_steps x (every decoder layer + lm_head for all n_streams <= 8 streams, each weight byte read once per
  * step, then one token selection per stream). states[b] must have been prefilled with slot = b and share one page pool. A finished
- * stream's state stays as it is. LIVECC_B200_MEGA=1 (read at lcc_model_create) runs every step as one persistent kernel, lcc_decode_steps too: a
- * stream's ids and logits are then bit-identical to decoding it alone. The kernels per operation that run otherwise are faster (see
- * decode_batch_ops in model.cu); they sum in another order than lcc_decode_steps does. */
+ * stream's state stays as it is, and a step behind the end of all of them does nothing. A stream's ids, logits and cache are bit-identical to those of a call with it
+ * alone or with any others. Two paths: kernels per operation, faster (see decode_batch_ops in model.cu), whose sums run in another order than those of
+ * lcc_decode_steps; with LIVECC_B200_MEGA=1 (read at lcc_model_create) one persistent kernel per step, lcc_decode_steps too, so that
+ * the two then agree bit for bit. */
 int lcc_decode_batch(lcc_model* m, const lcc_stream_state* states, int n_streams, int n_steps, const lcc_sampling* sp,
                      lcc_stream_t stream);
 /* Test hook: run layers [layer_begin, layer_end) and the phases in phase_mask (1 qkv, 2 attention, 4 o_proj,

@@ -266,11 +266,15 @@ __global__ void __launch_bounds__(128) flash_fwd_kernel(const FlashParams p) {
 // row with a dim per thread took 15.9.)
 constexpr int kMergeRows = 8;   // rows per CTA
 __global__ void __launch_bounds__(32 * kMergeRows) flash_merge_kernel(const float* __restrict__ part_o,
-                                                                      const float* __restrict__ part_ml, int nsplit, int Hkv,
-                                                                      int rows_total, int G, float scale_log2,
-                                                                      bf16* __restrict__ out, int o_ld) {
+                                                                      const float* __restrict__ part_ml, const __grid_constant__ PrefillStreams ps,
+                                                                      int Hkv, int G, float scale_log2, bf16* __restrict__ out, int o_ld) {
+    const PrefillStream& st = ps.st[blockIdx.z];
     const int rr = blockIdx.x * kMergeRows + (threadIdx.x >> 5), g = blockIdx.y, lane = threadIdx.x & 31;
-    if (rr >= rows_total) return;
+    const int rows_total = st.S * G, nsplit = st.nsplit;
+    if (nsplit < 2 || rr >= rows_total) return;
+    part_o += st.part_row * 128;
+    part_ml += st.part_row * 2;
+    out += (size_t)st.row0 * o_ld;
     const size_t row = (size_t)g * rows_total + rr, step = (size_t)Hkv * rows_total;
     float m = -INFINITY, l = 0.f;
     if (lane < nsplit) {
@@ -509,13 +513,31 @@ int attn_prefill_streams(const bf16* q, int q_ld, const bf16* kc, const bf16* vc
         }
         return 0;
     }
-    int ns = 1;
-    if (int r = attn_prefill_tc(q, q_ld, kc, vc, ps, Hq, Hkv, out, o_ld, part_o, part_ml, part_capacity_rows, num_sms, &ns, s)) return r;
-    if (ns > 1) {
-        const int G = Hq / Hkv;
-        lcc::count_launch();
-        flash_merge_kernel<<<dim3((ps.rows * G + kMergeRows - 1) / kMergeRows, Hkv), 32 * kMergeRows, 0, s>>>(part_o, part_ml, ns, Hkv, ps.rows * G, G,
-                                                            1.4426950408889634f / sqrtf(128.f), out, o_ld);
+    const int G = Hq / Hkv;
+    if (G < 1 || G > 128 || Hq % Hkv || (q_ld % 8) || (o_ld % 8)) return -1;
+    if (!part_o || !part_ml || ((uintptr_t)part_o % 16) || ((uintptr_t)part_ml % 8)) part_capacity_rows = 0;
+    for (int b = 0; b < ps.n;) {   // streams whose partials fit together
+        PrefillStreams some{};
+        some.rows = ps.rows;
+        size_t used = 0;
+        int longest = 0;   // of those with partials
+        for (; b < ps.n; ++b) {
+            PrefillStream& st = some.st[some.n];
+            st = ps.st[b];
+            st.nsplit = attn_prefill_tc_splits(st.S, st.past, Hq, Hkv, part_capacity_rows, num_sms);
+            const size_t need = st.nsplit > 1 ? (size_t)st.nsplit * Hq * st.S : 0;
+            if (used + need > part_capacity_rows) break;
+            st.part_row = used;
+            used += need;
+            if (need) longest = std::max(longest, st.S);
+            ++some.n;
+        }
+        if (int r = attn_prefill_tc(q, q_ld, kc, vc, some, Hq, Hkv, out, o_ld, part_o, part_ml, s)) return r;
+        if (longest) {
+            lcc::count_launch();
+            flash_merge_kernel<<<dim3((longest * G + kMergeRows - 1) / kMergeRows, Hkv, some.n), 32 * kMergeRows, 0, s>>>(
+                part_o, part_ml, some, Hkv, G, 1.4426950408889634f / sqrtf(128.f), out, o_ld);
+        }
     }
     return 0;
 }
@@ -556,8 +578,13 @@ int attn_prefill_paged(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, 
     p.nsplit = nsplit; p.part_o = part_o; p.part_ml = part_ml;
     dim3 grid(q_tiles, Hkv, nsplit);
     if (int r = launch_flash<128, true, true>(p, grid, s)) return r;
-    if (nsplit > 1)
-        { lcc::count_launch(); flash_merge_kernel<<<dim3((S * p.G + kMergeRows - 1) / kMergeRows, Hkv), 32 * kMergeRows, 0, s>>>(part_o, part_ml, nsplit, Hkv, S * p.G, p.G, p.scale_log2, out, o_ld); }
+    if (nsplit > 1) {
+        PrefillStreams ps{};
+        ps.n = 1; ps.rows = S;
+        ps.st[0].S = S; ps.st[0].nsplit = nsplit;
+        lcc::count_launch();
+        flash_merge_kernel<<<dim3((S * p.G + kMergeRows - 1) / kMergeRows, Hkv), 32 * kMergeRows, 0, s>>>(part_o, part_ml, ps, Hkv, p.G, p.scale_log2, out, o_ld);
+    }
     return 0;
 }
 
@@ -896,16 +923,23 @@ __global__ void __cluster_dims__(1, 8, 1) __launch_bounds__(128) attn_decode_clu
     attn_decode_role<8>(p, blockIdx.x, blockIdx.y, smem_attn);
 }
 
-// One slice of the grid (z) per stream of a batched step.
+// Slices of the grid (z) per stream of a batched step. A stream's keys are split by its own length alone, so that its bits do not depend on its
+// neighbours: eight splits, sixteen past kBatchLong tokens (the second cluster of a shorter stream, behind all others in the grid, leaves at once).
+// Eight splits of eight streams are one wave of CTAs, and more cost their fixed part again (us, 8 | 16 | 32 splits: 8 streams of 200, 2000, 8000,
+// 16384 tokens 10.2 | 20.7 | 25.2, 14.8 | 26.6 | 43.8, 30.8 | 41.2 | 59.3, 52.8 | 64.3 | 82.5); few streams of long caches leave SMs idle with
+// eight (4 x 8000 27.3 | 21.5 | 31.4, 2 x 8000 19.8 | 19.1 | 16.5, 2 x 30000 54 | 38 | 31). Chosen by the number of streams before, as low as each row has.
+constexpr int kBatchLong = 16384;
 struct DecodeAttnBatchParams {
     DecodeAttnParams one;
     AttnStream st[kBatchStreams];
-    int qkv_ld, out_ld;
+    int qkv_ld, out_ld, B;
 };
 __global__ void __cluster_dims__(1, 8, 1) __launch_bounds__(128) attn_decode_batch_kernel(const __grid_constant__ DecodeAttnBatchParams bp) {
     extern __shared__ __align__(16) uint8_t smem_attn[];
-    const int b = blockIdx.z;
+    const int b = blockIdx.z % bp.B, cluster = blockIdx.z / bp.B;
     DecodeAttnParams p = bp.one;
+    p.nsplit = bp.st[b].scalars[LCC_SC_KV_LEN] >= kBatchLong ? 16 : 8;
+    if (cluster * 8 >= p.nsplit) return;
     p.qkv += (size_t)b * bp.qkv_ld;
     p.out += (size_t)b * bp.out_ld;
     p.page_table = bp.st[b].page_table;
@@ -915,7 +949,7 @@ __global__ void __cluster_dims__(1, 8, 1) __launch_bounds__(128) attn_decode_bat
     p.part_o += (size_t)b * 8 * p.Hq * 128;
     p.part_ml += (size_t)b * 8 * p.Hq * 2;
     p.counters += b * p.Hkv;
-    attn_decode_role<8>(p, blockIdx.x, blockIdx.y, smem_attn);
+    attn_decode_role<8>(p, blockIdx.x, cluster * 8 + blockIdx.y, smem_attn);
 }
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
@@ -1047,19 +1081,19 @@ int attn_decode(bf16* qkv, bf16* kc, bf16* vc, const int* page_table, int page_s
 }
 
 int attn_decode_batch(bf16* qkv, int qkv_ld, bf16* kc, bf16* vc, const AttnStream* streams, int B, int page_size, const float* inv_freq,
-                      int Hq, int Hkv, int nsplit, float* part_o, float* part_ml, int* counters, bf16* out, int out_ld, cudaStream_t s) {
-    if (page_size != 64 || Hq % Hkv || Hq / Hkv > 8 || B < 1 || B > kBatchStreams || nsplit < 8 || nsplit > 64 || nsplit % 8) return -1;
+                      int Hq, int Hkv, float* part_o, float* part_ml, int* counters, bf16* out, int out_ld, cudaStream_t s) {
+    if (page_size != 64 || Hq % Hkv || Hq / Hkv > 8 || B < 1 || B > kBatchStreams) return -1;
     static SmemAttrOnce once;
     if (ensure_dyn_smem(once, attn_decode_batch_kernel, kDecSmem)) return -2;
     DecodeAttnBatchParams bp{};
     DecodeAttnParams& p = bp.one;
-    p.qkv = qkv; p.kc = kc; p.vc = vc; p.inv_freq = inv_freq; p.Hq = Hq; p.Hkv = Hkv; p.nsplit = nsplit;
+    p.qkv = qkv; p.kc = kc; p.vc = vc; p.inv_freq = inv_freq; p.Hq = Hq; p.Hkv = Hkv;
     p.part_o = part_o; p.part_ml = part_ml; p.counters = counters; p.out = out;
     p.scale_log2 = 1.4426950408889634f / sqrtf(128.f);
     for (int b = 0; b < B; ++b) bp.st[b] = streams[b];
-    bp.qkv_ld = qkv_ld; bp.out_ld = out_ld;
+    bp.qkv_ld = qkv_ld; bp.out_ld = out_ld; bp.B = B;
     count_launch();
-    return launch_kernel(attn_decode_batch_kernel, dim3(Hkv, nsplit, B), dim3(128), (size_t)kDecSmem, s, false, bp) == cudaSuccess ? 0 : -3;
+    return launch_kernel(attn_decode_batch_kernel, dim3(Hkv, 8, 2 * B), dim3(128), (size_t)kDecSmem, s, false, bp) == cudaSuccess ? 0 : -3;
 }
 
 // Fused attention + o_proj launch (see attn_oproj_kernel). sync: device int[2], zero-initialised once.

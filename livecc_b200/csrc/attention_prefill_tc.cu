@@ -48,9 +48,8 @@ struct PrefillTcParams {
     int o_ld;
     int Hkv, G, PT;
     float scale_log2;
-    int nsplit;
-    float* part_o;   // [nsplit, Hkv, rows*G, 128] unnormalised fp32
-    float* part_ml;  // [nsplit, Hkv, rows*G, 2]    (raw max, sum)
+    float* part_o;   // per stream, from its part_row on: [nsplit, Hkv, S*G, 128] unnormalised fp32
+    float* part_ml;  // the same: [nsplit, Hkv, S*G, 2]    (raw max, sum)
     PrefillStreams ps;
 };
 
@@ -85,28 +84,32 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                        const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ PrefillTcParams p, const PrefillLocal lp) {
     using namespace ptc;
     if (LOCAL && lp.pos.finished && *lp.pos.finished) return;
-    const PrefillStream& st = p.ps.st[LOCAL ? 0 : blockIdx.z / p.nsplit];
-    const int kvh = blockIdx.y, split = LOCAL ? 0 : blockIdx.z % p.nsplit;
+    int b = 0, split = LOCAL ? 0 : blockIdx.z;
+    if (!LOCAL)
+        while (split >= p.ps.st[b].nsplit) split -= p.ps.st[b++].nsplit;
+    const PrefillStream& st = p.ps.st[b];
+    const int kvh = blockIdx.y;
+    const bool parts = !LOCAL && st.nsplit > 1;
     // (with a window or chunks the last rows see the most keys: they start first)
     const int pos0 = (LOCAL ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * p.PT, S = st.S;
     const int past = LOCAL && lp.pos.kv_len ? *lp.pos.kv_len : st.past;
     if (pos0 >= S) return;
     const int npos = min(p.PT, S - pos0);
     const int rows_used = npos * p.G;
-    const int rows_total = p.ps.rows * p.G;
-    const int row_base = (st.row0 + pos0) * p.G;  // packed row index of this tile's row 0
+    const int rows_total = S * p.G;
+    const int row_base = pos0 * p.G;  // packed row index of this tile's row 0
     // KV tiles this CTA needs: keys 0 .. past + last position (causal), restricted to its split
     const int n_tiles = (past + pos0 + npos + BN - 1) / BN;
     int tile_lo = 0, tile_hi = n_tiles;
     const int key0 = LOCAL ? lp.first_key(past + pos0) : 0, key1 = past + pos0 + npos;   // no row of this CTA sees a key outside [key0, key1)
     if (LOCAL) tile_lo = key0 / BN;
-    if (!LOCAL && p.nsplit > 1) {
+    if (parts) {
         const int tiles_total = (past + S + BN - 1) / BN;
-        const int tps = (tiles_total + p.nsplit - 1) / p.nsplit;
+        const int tps = (tiles_total + st.nsplit - 1) / st.nsplit;
         tile_lo = split * tps;
         tile_hi = min(n_tiles, tile_lo + tps);
         if (tile_lo >= tile_hi) {  // nothing for this split: neutral partial
-            float* ml = p.part_ml + (((size_t)split * p.Hkv + kvh) * rows_total + row_base) * 2;
+            float* ml = p.part_ml + (st.part_row + ((size_t)split * p.Hkv + kvh) * rows_total + row_base) * 2;
             for (int i = threadIdx.x; i < rows_used; i += blockDim.x) {
                 ml[i * 2] = -INFINITY;
                 ml[i * 2 + 1] = 0.f;
@@ -357,8 +360,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         auto sigmoid = [](float x) { return __fdividef(1.f, 1.f + expf(-x)); };
         mbar_wait(pv_done, (T - 1) & 1);
         tc_fence_after();
-        if (!LOCAL && p.nsplit > 1) {
-            const size_t prow = ((size_t)split * p.Hkv + kvh) * rows_total + row_base + row;
+        if (parts) {
+            const size_t prow = st.part_row + ((size_t)split * p.Hkv + kvh) * rows_total + row_base + row;
             float* dst = p.part_o + prow * D;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -426,35 +429,35 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     }
 }
 
-// q: rotated rows of the fused qkv buffer [S, >= Hq*128] (row stride q_ld); kc/vc: one layer of the page pool
-// [pages, Hkv, 64, 128].  Returns the split count used through *nsplit_out (the caller merges when > 1).
-int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const PrefillStreams& ps, int Hq, int Hkv, bf16* out, int o_ld,
-                    float* part_o, float* part_ml, size_t part_capacity_rows, int num_sms, int* nsplit_out, cudaStream_t s) {
+// Key ranges of one stream's attention, up to two CTAs per SM, with at least 8 tiles per range and partials that fit into the caller's scratch. A tile
+// takes 0.8 us with one CTA per SM and 1.15 with two; the partials cost a launch of 3.5 us and are written and read once. (281 rows over 4 k keys: 4
+// splits; 24 rows over 64 k: 32.) Filling the places whatever the range is cost 400 to 640 rows behind 600 to 1500 tokens up to a quarter:
+// 400 and 600 rows behind 600 | 1000 | 3000 tokens 17.4 | 22.3 | 47.5 and 20.1 | 24.6 | 50.3 us unsplit, 21.7 | 25.4 | 34.4 and 25.6 | 28.6 |
+// 45.8 with every place taken. Other streams of the launch do not count: a stream has the same bits whoever its neighbours are.
+int attn_prefill_tc_splits(int S, int past, int Hq, int Hkv, size_t part_capacity_rows, int num_sms) {
     using namespace ptc;
-    const int G = Hq / Hkv;
-    if (G < 1 || G > 128 || Hq % Hkv || (q_ld % 8) || (o_ld % 8)) return -1;
-    const int PT = BM / G;
-    int q_tiles = 0, ctas = 0, kv_tiles = 0;   // of the longest stream, of all, of the longest range
-    for (int b = 0; b < ps.n; ++b) {
-        const int t = (ps.st[b].S + PT - 1) / PT;
-        q_tiles = std::max(q_tiles, t);
-        ctas += t * Hkv;
-        kv_tiles = std::max(kv_tiles, (ps.st[b].past + ps.st[b].S + BN - 1) / BN);
-    }
+    const int PT = BM / (Hq / Hkv), ctas = (S + PT - 1) / PT * Hkv, kv_tiles = (past + S + BN - 1) / BN;
+    const size_t rows = (size_t)Hq * S;
+    const int most = (int)std::min((size_t)std::min({2 * num_sms / ctas, MAX_SPLIT, kv_tiles / 8}), part_capacity_rows / rows);
     int nsplit = 1;
-    // Key splits, up to two CTAs per SM, with at least 8 tiles per split and partials that fit into the caller's scratch. A tile takes 0.8 us
-    // with one CTA per SM and 1.15 with two; the partials cost a launch of 3.5 us and are written and read once. (281 rows over 4 k keys: 4
-    // splits; 24 rows over 64 k: 32.) Filling the places whatever the range is cost 400 to 640 rows behind 600 to 1500 tokens up to a quarter:
-    // 400 and 600 rows behind 600 | 1000 | 3000 tokens 17.4 | 22.3 | 47.5 and 20.1 | 24.6 | 50.3 us unsplit, 21.7 | 25.4 | 34.4 and 25.6 | 28.6 |
-    // 45.8 with every place taken.
-    if (part_o && part_ml && ((uintptr_t)part_o % 16) == 0 && ((uintptr_t)part_ml % 8) == 0) {
-        const size_t rows = (size_t)Hkv * ps.rows * G;
-        const int most = (int)std::min((size_t)std::min({2 * num_sms / ctas, MAX_SPLIT, kv_tiles / 8}), part_capacity_rows / rows);
-        double best = 0.8 * kv_tiles;   // (more CTAs than SMs are never split)
-        for (int n = 2; n <= most; ++n) {
-            const double us = (double)kv_tiles / n * (ctas * n > num_sms ? 1.15 : 0.8) + 3.5 + (double)rows * n * 1024 / 6.5e6;
-            if (us < best) { best = us; nsplit = n; }
-        }
+    double best = 0.8 * kv_tiles;   // (more CTAs than SMs are never split)
+    for (int n = 2; n <= most; ++n) {
+        const double us = (double)kv_tiles / n * (ctas * n > num_sms ? 1.15 : 0.8) + 3.5 + (double)rows * n * 1024 / 6.5e6;
+        if (us < best) { best = us; nsplit = n; }
+    }
+    return nsplit;
+}
+
+// q: rotated rows of the fused qkv buffer [ps.rows, >= Hq*128] (row stride q_ld); kc/vc: one layer of the page pool
+// [pages, Hkv, 64, 128]. Streams with nsplit > 1 leave partials, which the caller merges.
+int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const PrefillStreams& ps, int Hq, int Hkv, bf16* out, int o_ld,
+                    float* part_o, float* part_ml, cudaStream_t s) {
+    using namespace ptc;
+    const int G = Hq / Hkv, PT = BM / G;
+    int q_tiles = 0, slices = 0;
+    for (int b = 0; b < ps.n; ++b) {
+        q_tiles = std::max(q_tiles, (ps.st[b].S + PT - 1) / PT);
+        slices += ps.st[b].nsplit;
     }
     CUtensorMap tq, tk, tv;
     if (make_tmap_bf16_3d_sw128(&tq, q, D, Hq, ps.rows, D, q_ld, G, PT)) return -10;
@@ -463,10 +466,9 @@ int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, con
     if (make_tmap_bf16_2d_box(&tv, vc, pool_rows, D, D, 64, BN, false)) return -11;
     static SmemAttrOnce once;
     if (ensure_dyn_smem(once, attn_prefill_tc_kernel<false>, SMEM_BYTES)) return -12;
-    const PrefillTcParams p{out, o_ld, Hkv, G, PT, 1.4426950408889634f / sqrtf((float)D), nsplit, part_o, part_ml, ps};
+    const PrefillTcParams p{out, o_ld, Hkv, G, PT, 1.4426950408889634f / sqrtf((float)D), part_o, part_ml, ps};
     lcc::count_launch();
-    attn_prefill_tc_kernel<false><<<dim3(q_tiles, Hkv, nsplit * ps.n), 192, SMEM_BYTES, s>>>(tq, tk, tv, p, PrefillLocal{});
-    *nsplit_out = nsplit;
+    attn_prefill_tc_kernel<false><<<dim3(q_tiles, Hkv, slices), 192, SMEM_BYTES, s>>>(tq, tk, tv, p, PrefillLocal{});
     return 0;
 }
 
@@ -484,8 +486,8 @@ int attn_local_tc(const float* q, const void* k_pages, const void* v_pages, cons
     PrefillTcParams p{};
     p.out = (bf16*)out; p.o_ld = ld_out; p.Hkv = G; p.G = Hq / G; p.PT = BM / p.G;
     p.scale_log2 = scale * 1.4426950408889634f;
-    p.nsplit = 1;
     p.ps.n = 1; p.ps.rows = S;
+    p.ps.st[0].nsplit = 1;
     p.ps.st[0].page_table = page_table; p.ps.st[0].S = S; p.ps.st[0].past = pos.past;
     const PrefillLocal lp{q, pos, sink, (const bf16*)gate, ld_gate, chunk > 0 ? chunk : 0, opt.window > 0 ? opt.window : 0, opt.no_sink, opt.gate_channel};
     CUtensorMap tk, tv;

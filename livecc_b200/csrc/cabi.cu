@@ -125,7 +125,7 @@ int lcc_gemv_batch(lcc_ctx* ctx, int kind, const void* W, const void* x, int ldx
     if (B < 1 || B > lcc::kBatchStreams || !scalars) LCC_FAIL(ctx, -2, "lcc_gemv_batch: 1..%d streams with their scalars", lcc::kBatchStreams);
     const int* fin[lcc::kBatchStreams];
     for (int b = 0; b < B; ++b) fin[b] = scalars[b] + LCC_SC_FINISHED;
-    const lcc::GemvBatch a{(const bf16*)W, (const bf16*)x, N, K, ldx, B, fin, nullptr, nullptr, 0};
+    const lcc::GemvBatch a{(const bf16*)W, (const bf16*)x, N, K, ldx, B, fin, nullptr, 0};
     cudaStream_t s = (cudaStream_t)stream;
     switch (kind) {
         case LCC_GEMV_BIAS: OP_RET(ctx, lcc::gemv_batch_bias(a, (const bf16*)bias, (bf16*)out, ldo, s), "lcc_gemv_batch");

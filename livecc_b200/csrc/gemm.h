@@ -67,6 +67,16 @@ int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream);
 enum GemmForm { FORM_ONE = 0, FORM_PAIR = 1, FORM_SWAP = 2 };
 struct GemmPlan { GemmForm form = FORM_ONE; int width = 0, splits = 1; };
 GemmPlan gemm_plan(const GemmArgs& a, int num_sms);   // what block_n = 0 takes
+// How the sum over K of a plain product is cut: into `ranges` partial sums that are added in order, by the pairs of a cluster or (`scratch`) through
+// the fp32 scratch. Products that are cut alike have the same bits in every form and at every tile width.
+struct SumOrder {
+    int ranges = 1;
+    bool scratch = false;
+    bool operator==(const SumOrder& o) const { return ranges == o.ranges && scratch == o.scratch; }
+};
+SumOrder gemm_sum_order(const GemmArgs& a, int num_sms);   // what block_n = 0 takes
+// The rows of several sequences as one product, cut as each of them alone would be: `order` is gemm_sum_order of the one sequence's rows.
+int gemm_bf16_tn_order(const GemmArgs& a, const SumOrder& order, int num_sms, cudaStream_t stream);
 // One explicit form (tests, tuning): width a multiple of 32, up to 256 (FORM_SWAP: 512)
 int gemm_bf16_tn_form(const GemmArgs& a, GemmForm form, int width, int splits, int num_sms, cudaStream_t stream);
 

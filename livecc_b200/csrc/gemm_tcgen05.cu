@@ -1327,8 +1327,9 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits,
     *reinterpret_cast<uint4*>(C + (size_t)row * ldc + col) = o;
 }
 
+static int splitk_width(const GemmArgs& a) { return a.block_n ? a.block_n : (a.N >= 256 ? 256 : (a.N >= 128 ? 128 : 64)); }
+
 // Split-K for small-M GEMMs whose tile count cannot occupy the SMs (prefill down_proj at M ~ 281: 84 tiles on 148 SMs).
-// Returns 1 if it handled the GEMM, 0 if the caller should run the plain path, < 0 on error.
 // Bit-exact on integer operands (test_gemm_splitk_exact_integer_operands), whole-model parity with it forced on. Measured on B200: it pays only for long K — down_proj (K = 18944) 86.7 -> 60.9 us,
 // while qkv / o_proj (K = 3584) get slower (23 -> 34 us) — so the default applies it for K >= 8192 only.
 // LIVECC_B200_GEMM_SPLITK=1 forces it for every eligible shape, =0 disables it.
@@ -1339,13 +1340,13 @@ static int splitk_mode() {
     }();
     return mode;
 }
-static int try_splitk(const GemmArgs& a, int num_sms, cudaStream_t stream, double* estimate = nullptr) {
+// Into how many ranges (0: not at all)?
+static int splitk_ranges(const GemmArgs& a, int num_sms) {
     const int mode = splitk_mode();
     if (!mode || !a.splitk_ws || a.M > 384) return 0;
     if (mode == 2 && a.K < 8192) return 0;
     if (a.epi != EPI_NONE && a.epi != EPI_BIAS && a.epi != EPI_RESIDUAL && a.epi != EPI_BIAS_RESIDUAL) return 0;
-    const int block_n = a.block_n ? a.block_n : (a.N >= 256 ? 256 : (a.N >= 128 ? 128 : 64));
-    const int m_tiles = (a.M + BLOCK_M - 1) / BLOCK_M, n_tiles = (a.N + block_n - 1) / block_n;
+    const int block_n = splitk_width(a), m_tiles = (a.M + BLOCK_M - 1) / BLOCK_M, n_tiles = (a.N + block_n - 1) / block_n;
     const int tiles = m_tiles * n_tiles;
     const int nkb = (a.K + BLOCK_K - 1) / BLOCK_K;
     if (tiles * 2 > num_sms) return 0;
@@ -1354,11 +1355,9 @@ static int try_splitk(const GemmArgs& a, int num_sms, cudaStream_t stream, doubl
     if (splits > nkb / 4) splits = nkb / 4;  // >= 4 k-blocks per unit
     while (splits > 1 && (splits - 1) * ((nkb + splits - 1) / splits) >= nkb) --splits;  // no empty split
     while (splits > 1 && (size_t)splits * a.M * a.N * 4 > a.splitk_ws_bytes) --splits;
-    if (splits < 2) return 0;
-    if (estimate) {   // two launches, the partials written and read once
-        *estimate = 11.0 + (tiles * splits + num_sms - 1) / num_sms * ((nkb + splits - 1) / splits) * 0.41 + (double)a.M * a.N * splits * 4 / 6.5e6;
-        return 1;
-    }
+    return splits < 2 ? 0 : splits;
+}
+static int run_splitk(const GemmArgs& a, int splits, int num_sms, cudaStream_t stream) {
     GemmArgs p = a;
     p.C = a.splitk_ws;
     p.ldc = a.N;
@@ -1366,24 +1365,28 @@ static int try_splitk(const GemmArgs& a, int num_sms, cudaStream_t stream, doubl
     p.splits = splits;
     p.bias = nullptr;
     p.residual = nullptr;
-    if (int r = launch_cfg<EPI_PARTIAL_F32>(p, block_n, num_sms, stream)) return r;
+    if (int r = launch_cfg<EPI_PARTIAL_F32>(p, splitk_width(a), num_sms, stream)) return r;
     const int64_t threads = (int64_t)a.M * (a.N / 8);
     lcc::count_launch();
     splitk_reduce_kernel<<<(int)((threads + 255) / 256), 256, 0, stream>>>(
         (const float*)a.splitk_ws, splits, a.M, a.N, (const bf16*)a.bias, (const bf16*)a.residual, a.ldr, (bf16*)a.C,
         a.ldc, a.epi);
-    return cudaGetLastError() == cudaSuccess ? 1 : -13;
+    return cudaGetLastError() == cudaSuccess ? 0 : -13;
 }
 
-// The form that a plain product of block_n = 0 takes (a split K in global memory counts as FORM_ONE; try_splitk decides on it).
+// The form that a plain product of block_n = 0 takes (a split K in global memory counts as FORM_ONE; splitk_ranges decides on it).
 GemmPlan gemm_plan(const GemmArgs& a, int num_sms) {
     GemmPlan p;
-    double us = 0., split_us = 0.;
+    double us = 0.;
     p.width = choose_alone(a.M, a.N, a.K, num_sms, &us);
     const int width = choose_pair(a.M, a.N, a.K, num_sms, us, &us);
     if (width) p.width = width;
     if (width) p.form = FORM_PAIR;
-    if (try_splitk(a, num_sms, nullptr, &split_us) > 0) { us = split_us; p.form = FORM_ONE; }
+    if (const int ranges = splitk_ranges(a, num_sms)) {   // two launches, the partials written and read once
+        const int w = splitk_width(a), tiles = (a.M + BLOCK_M - 1) / BLOCK_M * ((a.N + w - 1) / w), nkb = (a.K + BLOCK_K - 1) / BLOCK_K;
+        us = 11.0 + (tiles * ranges + num_sms - 1) / num_sms * ((nkb + ranges - 1) / ranges) * 0.41 + (double)a.M * a.N * ranges * 4 / 6.5e6;
+        p.form = FORM_ONE;
+    }
     int bm = 0, splits = 0;
     if (splitk_mode() != 1 && a.epi != EPI_PARTIAL_F32 && choose_swap(a.M, a.N, a.K, num_sms, us, &bm, &splits)) p = GemmPlan{FORM_SWAP, bm, splits};
     return p;
@@ -1414,10 +1417,57 @@ int gemm_bf16_tn_form(const GemmArgs& a, GemmForm form, int width, int splits, i
     return form == FORM_PAIR ? launch_epi2(a, width, num_sms, stream) : launch_epi(a, width, num_sms, stream);
 }
 
+static int forced_width() {   // tuning hook (0/unset = model)
+    static const int forced = [] { const char* e = getenv("LIVECC_B200_GEMM_BN"); return e ? atoi(e) : 0; }();
+    return forced;
+}
+
+SumOrder gemm_sum_order(const GemmArgs& a, int num_sms) {
+    if (forced_width() <= 0) {
+        const GemmPlan p = gemm_plan(a, num_sms);
+        if (p.form == FORM_SWAP) return SumOrder{p.splits, false};
+    }
+    const int ranges = splitk_ranges(a, num_sms);
+    return ranges ? SumOrder{ranges, true} : SumOrder{};
+}
+
+int gemm_bf16_tn_order(const GemmArgs& a, const SumOrder& order, int num_sms, cudaStream_t stream) {
+    if (int r = check_args(a)) return r;
+    if (a.tile_group || a.batch > 1 || a.c_f32 || a.block_n || a.epi == EPI_SIGMOID_GATE) return -6;
+    if (gemm_sum_order(a, num_sms) == order) return gemm_bf16_tn(a, num_sms, stream);
+    if (order.ranges == 1) {
+        double us = 0.;
+        const int alone = choose_alone(a.M, a.N, a.K, num_sms, &us), pair = choose_pair(a.M, a.N, a.K, num_sms, us, &us);
+        return pair ? launch_epi2(a, pair, num_sms, stream) : launch_epi(a, alone, num_sms, stream);
+    }
+    // as many rows at a time as the scratch, or one wave of clusters, holds
+    int rows, bm = kSwapMax, m_tiles = 1;
+    if (order.scratch) rows = (int)std::min<size_t>(a.splitk_ws_bytes / ((size_t)order.ranges * a.N * 4), 1 << 20) / BLOCK_M * BLOCK_M;
+    else {
+        auto fits = [&](int h) { const SwapTile t = make_swap(h, order.ranges); return h * BLOCK_M * 4 <= t.stages * t.stage_bytes; };
+        while (bm > 32 && !fits(bm)) bm -= 32;
+        m_tiles = max_clusters(current_device(), order.ranges, num_sms) / ((a.N + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
+        rows = m_tiles * bm;
+    }
+    if (rows < 1) return -15;
+    for (int m0 = 0; m0 < a.M; m0 += rows) {
+        GemmArgs p = a;
+        p.M = std::min(rows, a.M - m0);
+        p.A = (const bf16*)a.A + (size_t)m0 * a.lda;
+        p.C = (bf16*)a.C + (size_t)m0 * a.ldc;
+        if (a.residual) p.residual = (const bf16*)a.residual + (size_t)m0 * a.ldr;
+        const int tiles = (p.M + bm - 1) / bm;
+        if (int r = order.scratch ? run_splitk(p, order.ranges, num_sms, stream)
+                                  : launch_epi_swap(p, ((p.M + tiles - 1) / tiles + 31) / 32 * 32, order.ranges, num_sms, stream))
+            return r;
+    }
+    return 0;
+}
+
 int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream) {
     if (int r = check_args(a)) return r;
     const bool plain = !a.tile_group && a.batch <= 1 && !a.c_f32;
-    static const int forced = [] { const char* e = getenv("LIVECC_B200_GEMM_BN"); return e ? atoi(e) : 0; }();  // tuning hook (0/unset = model)
+    const int forced = forced_width();
     const bool choose = plain && a.block_n == 0 && forced <= 0 && a.epi != EPI_SIGMOID_GATE;
     int width = 0;
     if (choose) {
@@ -1426,7 +1476,7 @@ int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream) {
         width = p.form == FORM_PAIR ? -p.width : p.width;
     }
     if (plain)
-        if (int r = try_splitk(a, num_sms, stream)) return r < 0 ? r : 0;
+        if (const int ranges = splitk_ranges(a, num_sms)) return run_splitk(a, ranges, num_sms, stream);
     int block_n = a.block_n;
     if (block_n == 0) block_n = forced > 0 ? forced : (width ? width : choose_bn(a.M, a.N, num_sms));
     // block_n < 0: the CTA pair's kernel with tile width -block_n

@@ -284,6 +284,105 @@ __global__ void __launch_bounds__(256) gemv_splitk_kernel(const GemvParams p) {
     }
 }
 
+// Output head over the rows of NS sequences: one read of the weights, and for every row the sums of gemv_rows_kernel<.., GV_LOGITS, ..> (a lane's pieces of 8
+// in the same order, the same sum over a warp), so that a row has the bits that it has alone. Rows come normalised (head_norm_kernel). Bound by
+// issue on the CUDA cores, which is what these sums ask for: two rows' multiply-adds per instruction (fma.rn.f32x2 rounds each like fmaf). 152064 x 3584,
+// 2 | 4 | 8 rows: 159 | 225 | 344 us (one by one 2, 4 and 8 times 172; without the packed form 174 | 245 | 387; mma.sync, another order, 162).
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+struct HeadRows { int at[kBatchStreams]; };
+__global__ void __launch_bounds__(256) head_norm_kernel(const bf16* __restrict__ x, int ldx, HeadRows rows, const bf16* __restrict__ norm_w, float eps, int K,
+                                                        bf16* __restrict__ out) {
+    extern __shared__ __align__(16) uint8_t smem_gemv[];
+    bf16* xs = reinterpret_cast<bf16*>(smem_gemv);
+    __shared__ float red[32];
+    stage_x<true>(xs, x + (size_t)rows.at[blockIdx.x] * ldx, norm_w, eps, K, red);
+    for (int c = threadIdx.x * 8; c < K; c += blockDim.x * 8) *reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * K + c) = *reinterpret_cast<const uint4*>(xs + c);
+}
+// UNROLL pieces of 4 weight rows in flight per lane, CTAS per SM
+template <int NS, int UNROLL, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) head_rows_kernel(const bf16* __restrict__ W, int ldw, const bf16* __restrict__ x, int B, int N, int K,
+                                                              float* __restrict__ logits, float* __restrict__ logits_copy) {
+    constexpr int ROWS = 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row0 = (blockIdx.x * 8 + warp) * ROWS;
+    if (row0 >= N) return;
+    float acc[ROWS][NS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int s = 0; s < NS; ++s) acc[r][s] = 0.f;
+    const bf16* w0 = W + (size_t)row0 * ldw;
+    for (int c = lane * 8; c < K; c += UNROLL * 256) {
+        uint4 w[UNROLL][ROWS];
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u)
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+                w[u][r] = c + u * 256 < K ? ld_stream16(w0 + (size_t)min(r, N - 1 - row0) * ldw + c + u * 256) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+            const int at = min(c + u * 256, K - 8);
+            unsigned long long wp[ROWS / 2][8];   // rows 2 r and 2 r + 1
+#pragma unroll
+            for (int r = 0; r < ROWS / 2; ++r) {
+                const uint4 lo = w[u][2 * r], hi = w[u][2 * r + 1];
+                const uint32_t a[4] = {lo.x, lo.y, lo.z, lo.w}, b[4] = {hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 fa = unpack_bf16x2(a[j]), fb = unpack_bf16x2(b[j]);
+                    wp[r][2 * j] = pack2(fa.x, fb.x);
+                    wp[r][2 * j + 1] = pack2(fa.y, fb.y);
+                }
+            }
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                const uint4 xv = __ldg(reinterpret_cast<const uint4*>(x + (size_t)min(s, B - 1) * K + at));
+                const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
+                unsigned long long d[ROWS / 2];
+#pragma unroll
+                for (int r = 0; r < ROWS / 2; ++r) d[r] = 0ull;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {   // (as dot8)
+                    const float2 f = unpack_bf16x2(xw[j]);
+                    const unsigned long long x0 = pack2(f.x, f.x), x1 = pack2(f.y, f.y);
+#pragma unroll
+                    for (int r = 0; r < ROWS / 2; ++r) {
+                        d[r] = fma2(wp[r][2 * j], x0, d[r]);
+                        d[r] = fma2(wp[r][2 * j + 1], x1, d[r]);
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < ROWS / 2; ++r) {
+                    acc[2 * r][s] += __uint_as_float((uint32_t)d[r]);
+                    acc[2 * r + 1][s] += __uint_as_float((uint32_t)(d[r] >> 32));
+                }
+            }
+        }
+    }
+    float mine = 0.f;   // lane r NS + s stores row r of sequence s
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const float v = warp_sum(acc[r][s]);
+            if (lane == r * NS + s) mine = rbf(v);
+        }
+    const int s = lane % NS, n = row0 + lane / NS;
+    if (lane < ROWS * NS && s < B && n < N) {
+        logits[(size_t)s * N + n] = mine;
+        logits_copy[(size_t)s * N + n] = mine;
+    }
+}
+
 template <typename Kern>
 static int set_smem(Kern kern, int bytes) {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess ? 0 : -1;
@@ -373,6 +472,24 @@ int gemv_norm_logits(const bf16* W, int ldw, const bf16* x, const bf16* norm_w, 
     if (int r = check_common(p)) return r;
     LCC_LAUNCH((gemv_rows_kernel<4, true, GV_LOGITS, 4>), (N + 31) / 32, K * 2);
     return 0;
+}
+
+int gemv_norm_logits_rows(const bf16* W, int ldw, const bf16* x, int ldx, const int* x_rows, int B, const bf16* norm_w, float eps, bf16* normed,
+                          float* logits, float* logits_copy, int N, int K, cudaStream_t s) {
+    if (B < 1 || B > kBatchStreams || N <= 0 || K <= 0 || (K % 8) || (ldw % 8) || (ldx % 8)) return -1;
+    if (K * 2 > 200 * 1024) return -2;
+    HeadRows rows{};
+    for (int b = 0; b < B; ++b) rows.at[b] = x_rows[b];
+    static SmemAttrOnce once;
+    if (ensure_dyn_smem(once, head_norm_kernel, 200 * 1024)) return -3;
+    count_launch();
+    head_norm_kernel<<<B, 256, K * 2, s>>>(x, ldx, rows, norm_w, eps, K, normed);
+    count_launch();
+    const int grid = (N + 31) / 32;
+    if (B <= 2) head_rows_kernel<2, 2, 3><<<grid, 256, 0, s>>>(W, ldw, normed, B, N, K, logits, logits_copy);
+    else if (B <= 4) head_rows_kernel<4, 2, 2><<<grid, 256, 0, s>>>(W, ldw, normed, B, N, K, logits, logits_copy);
+    else head_rows_kernel<8, 1, 2><<<grid, 256, 0, s>>>(W, ldw, normed, B, N, K, logits, logits_copy);
+    return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
 }  // namespace lcc

@@ -16,9 +16,8 @@ enum { GB_BIAS = 0, GB_RESIDUAL = 1, GB_SWIGLU = 2, GB_LOGITS = 3 };
 
 struct GemvBatchParams {
     const bf16* W;
-    const bf16* x;     // rows x_row[b] of [][ldx]
+    const bf16* x;     // [B][ldx]
     int N, K, ldx, B;
-    int x_row[kBatchStreams];
     const bf16* bias;  // GB_BIAS
     bf16* out;         // [B][ldo]; GB_RESIDUAL: the residual stream, in and out
     int ldo;
@@ -30,11 +29,12 @@ struct GemvBatchParams {
 
 constexpr int kGbWarps = 8;
 
-// Measured with 8 streams (hidden 3584; for comparison one stream's CUDA-core kernels): lm_head 162 us (172), gate/up 43.9 (43), down 27.0 (25),
-// qkv 9.6 (11.1, RMSNorm included), o 10.9 (9.6; both 0.4 more since the streams' flags are looked at behind the first loads).
+// Measured with 8 streams (hidden 3584; for comparison one stream's CUDA-core kernels): lm_head 166 us (172), gate/up 43.8 (43), down 27.0 (25),
+// qkv 9.0 (11.1, RMSNorm included), o 10.1 (9.6).
 // MT: 16-row tiles per CTA (GB_SWIGLU: 16 gate rows and their 16 up rows). KS: CTAs of a cluster that share K. UN: units of 64 k in flight.
+// CTAs per SM are fixed, or a change of a few registers moves these times by a tenth (down at 80 registers 33 us, the head at 68 170).
 template <int MT, int KS, int UN, int EPI>
-__global__ void __launch_bounds__(kGbWarps * 32) gemv_batch_kernel(const GemvBatchParams p) {
+__global__ void __launch_bounds__(kGbWarps * 32, EPI == GB_SWIGLU ? 3 : UN > 2 ? 2 : 4) gemv_batch_kernel(const GemvBatchParams p) {
     __shared__ float part[kGbWarps][MT * 128];   // [row][stream] per warp
     __shared__ float peers[KS][MT * 128];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kGbWarps * 32) gemv_batch_kernel(const GemvBat
     const int units = p.K >> 6, mine = (units + KS - 1) / KS;
     const int u0 = rank * mine, u1 = min(units, u0 + mine);
     const bf16* w0 = p.W + (size_t)(n0 + g) * p.K + t * 8;
-    const bf16* x0 = p.x + (size_t)p.x_row[g < p.B ? g : 0] * p.ldx + t * 8;
+    const bf16* x0 = p.x + (size_t)(g < p.B ? g : 0) * p.ldx + t * 8;
     float acc[MT][4];
 #pragma unroll
     for (int m = 0; m < MT; ++m)
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kGbWarps * 32) gemv_batch_kernel(const GemvBat
         if (KS > 1) cluster_wait();
         return true;
     };
-    if constexpr (UN == 1) {   // (the loop turned like this: gate/up 43.5 us, 48.4 as below; with 2 units in flight 35 for the 27 of the down projection)
+    if constexpr (UN == 1) {   // (the loop turned like this: gate/up 43.8 us, 48.4 as below; with 2 units in flight 35 for the 27 of the down projection)
         if (u < u1) load(u, w[0]);
         if (ended()) return;
         while (u < u1) {
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kGbWarps * 32) gemv_batch_kernel(const GemvBat
         *reinterpret_cast<float2*>(d + 64) = make_float2(acc[m][2], acc[m][3]);
     }
     __syncthreads();
-    if (p.pf_bytes) {
+    if (EPI != GB_LOGITS && p.pf_bytes) {   // (nothing follows the head)
         const unsigned ntail = min(gridDim.x, 296u);
         if (blockIdx.x + ntail >= gridDim.x) {
             const unsigned lines = (p.pf_bytes + 127u) >> 7, per = (lines + ntail - 1) / ntail;
@@ -185,7 +185,7 @@ static int launch_batch(const GemvBatchParams& p, cudaStream_t s) {
 static GemvBatchParams params_of(const GemvBatch& a) {
     GemvBatchParams p{};
     p.W = a.W; p.x = a.x; p.N = a.N; p.K = a.K; p.ldx = a.ldx; p.B = a.B;
-    for (int b = 0; b < a.B && b < kBatchStreams; ++b) { p.finished[b] = a.finished[b]; p.x_row[b] = a.x_rows ? a.x_rows[b] : b; }
+    for (int b = 0; b < a.B && b < kBatchStreams; ++b) p.finished[b] = a.finished[b];
     p.pf_ptr = (const uint8_t*)a.pf_ptr; p.pf_bytes = (unsigned)a.pf_bytes;
     return p;
 }

@@ -293,20 +293,66 @@ static int prefill_impl(lcc_model* m, const lcc_prefill_request* rq, int n, cons
     void* skw = ws + L.pf_splitk;  // split-K scratch of the small-N projections (opt-in, see gemm_tcgen05.cu::try_splitk)
     const size_t skb = kSplitKRows * (size_t)(qkv_dim > H ? qkv_dim : H) * 4;
 
+    // A product of all rows is one launch over the streams that it would cut alike if each were alone (SumOrder): a stream's bits are those of its own pass.
+    struct Runs { int n, row0[lcc::kBatchStreams], rows[lcc::kBatchStreams]; lcc::SumOrder order[lcc::kBatchStreams]; };
+    auto args = [&](const void* A, int lda, const void* B, int ldb, void* C, int ldc, int N, int K, const void* bias, const void* res, int epi, bool split) {
+        lcc::GemmArgs a{};
+        a.A = A; a.B = B; a.C = C; a.M = S; a.N = N; a.K = K; a.lda = lda; a.ldb = ldb; a.ldc = ldc;
+        a.bias = bias; a.residual = res; a.ldr = H; a.epi = epi;
+        a.fault = m->ctx->fault;
+        if (split) { a.splitk_ws = skw; a.splitk_ws_bytes = skb; }
+        return a;
+    };
+    auto runs_of = [&](lcc::GemmArgs a) {
+        Runs r{};
+        for (int b = 0; n > 1 && b < n; ++b) {
+            a.M = ps.st[b].S;
+            const lcc::SumOrder o = lcc::gemm_sum_order(a, m->ctx->num_sms);
+            if (!r.n || !(r.order[r.n - 1] == o)) { r.row0[r.n] = ps.st[b].row0; r.order[r.n++] = o; }
+            r.rows[r.n - 1] += a.M;
+        }
+        return r;
+    };
+    auto product = [&](const lcc::GemmArgs& a, const Runs& r) {
+        if (n == 1) return lcc::gemm_bf16_tn(a, m->ctx->num_sms, s);
+        for (int i = 0; i < r.n; ++i) {
+            lcc::GemmArgs p = a;
+            p.M = r.rows[i];
+            p.A = (const bf16*)a.A + (size_t)r.row0[i] * a.lda;
+            p.C = (bf16*)a.C + (size_t)r.row0[i] * a.ldc;
+            if (a.residual) p.residual = (const bf16*)a.residual + (size_t)r.row0[i] * a.ldr;
+            if (int rc = lcc::gemm_bf16_tn_order(p, r.order[i], m->ctx->num_sms, s)) return rc;
+        }
+        return 0;
+    };
+    auto norm = [&](const void* w) {   // (thousands of narrow rows take a kernel of their own, which a stream alone would not)
+        if (n == 1 || H > 1536) return lcc::rmsnorm(hid, H, (const bf16*)w, normed, H, S, H, c.rms_eps, s);
+        for (int b = 0; b < n; ++b) {
+            const size_t at = (size_t)ps.st[b].row0 * H;
+            if (int rc = lcc::rmsnorm(hid + at, H, (const bf16*)w, normed + at, H, ps.st[b].S, H, c.rms_eps, s)) return rc;
+        }
+        return 0;
+    };
+    Runs r_qkv{}, r_o{}, r_gu{}, r_down{};
     STEP(lcc::embed_gather_streams(ps, (const bf16*)m->w.embed, c.video_token_id, hid, rank, H, c.vocab, s), "embed gather");
     for (int i = 0; i < c.layers; ++i) {
         const lcc_layer_weights& lw = m->layers[i];
         bf16* kc = (bf16*)st->k_pool + (size_t)i * st->layer_stride;
         bf16* vc = (bf16*)st->v_pool + (size_t)i * st->layer_stride;
-        STEP(lcc::rmsnorm(hid, H, (const bf16*)lw.ln1_w, normed, H, S, H, c.rms_eps, s), "input_layernorm");
-        STEP(gemm(m, normed, H, lw.qkv_w, H, qkv, qkv_dim, S, qkv_dim, H, lw.qkv_b, nullptr, 0, lcc::EPI_BIAS, s, skw, skb), "qkv proj");
+        const lcc::GemmArgs a_qkv = args(normed, H, lw.qkv_w, H, qkv, qkv_dim, qkv_dim, H, lw.qkv_b, nullptr, lcc::EPI_BIAS, true);
+        const lcc::GemmArgs a_o = args(attn, Hq * 128, lw.o_w, Hq * 128, hid, H, H, Hq * 128, nullptr, hid, lcc::EPI_RESIDUAL, true);
+        const lcc::GemmArgs a_gu = args(normed, H, lw.gate_up_w, H, act, c.inter, 2 * c.inter, H, nullptr, nullptr, lcc::EPI_SWIGLU, false);
+        const lcc::GemmArgs a_down = args(act, c.inter, lw.down_w, c.inter, hid, H, H, c.inter, nullptr, hid, lcc::EPI_RESIDUAL, true);
+        if (i == 0) { r_qkv = runs_of(a_qkv); r_o = runs_of(a_o); r_gu = runs_of(a_gu); r_down = runs_of(a_down); }
+        STEP(norm(lw.ln1_w), "input_layernorm");
+        STEP(product(a_qkv, r_qkv), "qkv proj");
         STEP(lcc::mrope_kv_write_streams(qkv, qkv_dim, ps, m->w.text_inv_freq, c.mrope_t, c.mrope_h, Hq, Hkv, kc, vc, LCC_PAGE_SIZE, s), "mrope + kv write");
         STEP(lcc::attn_prefill_streams(qkv, qkv_dim, kc, vc, ps, LCC_PAGE_SIZE, Hq, Hkv, attn, Hq * 128, (float*)(ws + L.pf_part_o),
                                        (float*)(ws + L.pf_part_ml), kPrefillSplitRows * (size_t)Hq, m->ctx->num_sms, 0, s), "prefill attention");
-        STEP(gemm(m, attn, Hq * 128, lw.o_w, Hq * 128, hid, H, S, H, Hq * 128, nullptr, hid, H, lcc::EPI_RESIDUAL, s, skw, skb), "o_proj");
-        STEP(lcc::rmsnorm(hid, H, (const bf16*)lw.ln2_w, normed, H, S, H, c.rms_eps, s), "post_attention_layernorm");
-        STEP(gemm(m, normed, H, lw.gate_up_w, H, act, c.inter, S, 2 * c.inter, H, nullptr, nullptr, 0, lcc::EPI_SWIGLU, s), "gate_up");
-        STEP(gemm(m, act, c.inter, lw.down_w, c.inter, hid, H, S, H, c.inter, nullptr, hid, H, lcc::EPI_RESIDUAL, s, skw, skb), "down_proj");
+        STEP(product(a_o, r_o), "o_proj");
+        STEP(norm(lw.ln2_w), "post_attention_layernorm");
+        STEP(product(a_gu, r_gu), "gate_up");
+        STEP(product(a_down, r_down), "down_proj");
     }
     // final norm + lm_head on the last position of each stream only (logits_to_keep = 1, gen/utils.py:2487-2491)
     float *raw = (float*)(ws + L.logits_raw) + (size_t)slot * c.vocab, *proc = (float*)(ws + L.logits_proc) + (size_t)slot * c.vocab;
@@ -315,16 +361,11 @@ static int prefill_impl(lcc_model* m, const lcc_prefill_request* rq, int n, cons
                                    nullptr, m->ctx->num_sms, false, s), "lm_head");
         STEP(lcc::sample_greedy(make_sample(m, st, sp, ws, L, 0, slot), s), "token selection");
     } else {
-        const int* open[lcc::kBatchStreams];
         lcc::SampleBatch sb{};
         sb.B = n;
-        for (int b = 0; b < n; ++b) {
-            open[b] = rq[b].st.scalars + LCC_SC_FINISHED;
-            sb.seq[b] = rq[b].st.seq; sb.scalars[b] = rq[b].st.scalars;
-        }
-        STEP(lcc::rmsnorm(hid, H, (const bf16*)m->w.final_norm_w, normed, H, S, H, c.rms_eps, s), "final norm");
-        const lcc::GemvBatch a{(const bf16*)m->w.lm_head, normed, c.vocab, H, H, n, open, last, nullptr, 0};
-        STEP(lcc::gemv_batch_logits(a, raw, proc, c.vocab, s), "lm_head");
+        for (int b = 0; b < n; ++b) { sb.seq[b] = rq[b].st.seq; sb.scalars[b] = rq[b].st.scalars; }
+        STEP(lcc::gemv_norm_logits_rows((const bf16*)m->w.lm_head, H, hid, H, last, n, (const bf16*)m->w.final_norm_w, c.rms_eps, normed, raw, proc, c.vocab, H, s),
+             "lm_head");
         STEP(lcc::sample_greedy_batch(make_sample(m, nullptr, sp, ws, L, 0, slot), sb, s), "token selection");
     }
     LCC_CHECK_LAUNCH(m->ctx, "lcc_prefill");
@@ -340,7 +381,6 @@ int lcc_prefill(lcc_model* m, const lcc_stream_state* st, const int64_t* ids, co
 
 int lcc_prefill_batch(lcc_model* m, const lcc_prefill_request* requests, int n_streams, const lcc_sampling* sp, int first_slot, lcc_stream_t stream) {
     if (!m || !requests || !sp) return -1;
-    if (n_streams > 1 && !m->mega_ok) LCC_FAIL(m->ctx, -4, "lcc_prefill_batch: model geometry is not supported by the batched kernels");
     return prefill_impl(m, requests, n_streams, sp, first_slot, stream);
 }
 
@@ -409,12 +449,10 @@ static int decode_batch_ops(lcc_model* m, const lcc_stream_state* sts, int B, in
         fin[b] = sts[b].scalars + LCC_SC_FINISHED;
         sb.seq[b] = sts[b].seq; sb.scalars[b] = sts[b].scalars;
     }
-    int nsplit = 8;   // about two attention CTAs per SM, whatever the caches' lengths (they grow under a captured graph)
-    while (nsplit < kMaxSplit && 2 * nsplit * B * Hkv <= 2 * m->ctx->num_sms) nsplit *= 2;
     // the head of the next kernel's weights goes into L2 while a kernel's last CTAs run (see gemv.cu)
     const size_t kPf = 32u << 20;
     auto ops = [&](const void* W, int N, int K, const bf16* x, const void* next, size_t next_bytes) {
-        return lcc::GemvBatch{(const bf16*)W, x, N, K, K, B, fin, nullptr, next, next_bytes < kPf ? next_bytes : kPf};
+        return lcc::GemvBatch{(const bf16*)W, x, N, K, K, B, fin, next, next_bytes < kPf ? next_bytes : kPf};
     };
     for (int step = 0; step < n_steps; ++step) {
         for (int i = 0; i < c.layers; ++i) {
@@ -424,7 +462,7 @@ static int decode_batch_ops(lcc_model* m, const lcc_stream_state* sts, int B, in
             const bool last = i + 1 == c.layers;
             STEP(lcc::rmsnorm(h, H, (const bf16*)lw.ln1_w, normed, H, B, H, c.rms_eps, s), "batched decode input_layernorm");
             STEP(lcc::gemv_batch_bias(ops(lw.qkv_w, qkv_dim, H, normed, lw.o_w, (size_t)H * Hq * 256), (const bf16*)lw.qkv_b, qkv, qkv_dim, s), "batched decode qkv");
-            STEP(lcc::attn_decode_batch(qkv, qkv_dim, kc, vc, st, B, LCC_PAGE_SIZE, m->w.text_inv_freq, Hq, Hkv, nsplit, (float*)(ws + L.part_o),
+            STEP(lcc::attn_decode_batch(qkv, qkv_dim, kc, vc, st, B, LCC_PAGE_SIZE, m->w.text_inv_freq, Hq, Hkv, (float*)(ws + L.part_o),
                                         (float*)(ws + L.part_ml), (int*)(ws + L.batch_cnt), attn, Hq * 128, s), "batched decode attention");
             STEP(lcc::gemv_batch_residual(ops(lw.o_w, H, Hq * 128, attn, lw.gate_up_w, (size_t)4 * c.inter * H), h, H, s), "batched decode o_proj");
             STEP(lcc::rmsnorm(h, H, (const bf16*)lw.ln2_w, normed, H, B, H, c.rms_eps, s), "batched decode post_attention_layernorm");
@@ -444,7 +482,7 @@ int lcc_decode_batch(lcc_model* m, const lcc_stream_state* states, int n_streams
                      lcc_stream_t stream) {
     if (!m || !states || !sp) return -1;
     if (n_streams < 1 || n_streams > lcc::MG_MAXB) LCC_FAIL(m->ctx, -2, "lcc_decode_batch: 1..%d streams per launch", lcc::MG_MAXB);
-    if (!m->mega_ok) LCC_FAIL(m->ctx, -4, "lcc_decode_batch: model geometry is not supported by the persistent decode kernel");
+    if (!m->mega_ok) LCC_FAIL(m->ctx, -4, "lcc_decode_batch: model geometry is not supported by batched decoding (hidden and inter multiples of 256, vocab of 32)");
     WsLayout L;
     if (get_layout(m, 0, 0, &L)) LCC_FAIL(m->ctx, -3, "lcc_decode_batch: no workspace bound");
     cudaStream_t s = (cudaStream_t)stream;

@@ -30,6 +30,8 @@ struct PrefillStream {
     const bf16* video;        // feature rows, or null
     int* total_video;
     int n_video, S, past, row0;
+    int nsplit;               // key ranges of its attention (attn_prefill_streams)
+    size_t part_row;          // their first row of partials
 };
 struct PrefillStreams {
     int n, rows;
@@ -62,24 +64,25 @@ int vit_attention_tc(const bf16* qkv, int ld, int64_t n_rows, bf16* out, int o_l
 int attn_prefill_paged(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const int* page_table,
                        int page_size, int Hq, int Hkv, int S, int past, bf16* out, int o_ld, float* part_o,
                        float* part_ml, size_t part_capacity_rows, int num_sms, int impl, cudaStream_t s);
-// the same for the rows of several streams: one launch, and one merge
+// the same for the rows of several streams, each split as it would be alone: one launch and one merge, more where the partials do not fit together
 int attn_prefill_streams(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const PrefillStreams& ps, int page_size, int Hq, int Hkv, bf16* out,
                          int o_ld, float* part_o, float* part_ml, size_t part_capacity_rows, int num_sms, int impl, cudaStream_t s);
 // attention_prefill_tc.cu
+int attn_prefill_tc_splits(int S, int past, int Hq, int Hkv, size_t part_capacity_rows, int num_sms);
 int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, const PrefillStreams& ps, int Hq, int Hkv, bf16* out, int o_ld,
-                    float* part_o, float* part_ml, size_t part_capacity_rows, int num_sms, int* nsplit_out, cudaStream_t s);
+                    float* part_o, float* part_ml, cudaStream_t s);
 int attn_decode(bf16* qkv, bf16* kc, bf16* vc, const int* page_table, int page_size, const int* kv_len,
                 const int* rope_pos, const int* finished, const float* inv_freq, int Hq, int Hkv, int nsplit,
                 float* part_o, float* part_ml, int* counters, bf16* out, bool pdl, cudaStream_t s);
 
-// the same for B streams, one grid slice each: rows b of qkv / out, nsplit a multiple of 8, part_o / part_ml / counters for 8 streams
-// of nsplit / 8 <= 8 rows and Hkv counters each
+// the same for B streams, split by each stream's own length: rows b of qkv / out, part_o / part_ml / counters for 8 streams of 8 rows and Hkv
+// counters each
 struct AttnStream {
     const int* page_table;
     const int* scalars;   // LCC_SC_*
 };
 int attn_decode_batch(bf16* qkv, int qkv_ld, bf16* kc, bf16* vc, const AttnStream* streams, int B, int page_size, const float* inv_freq,
-                      int Hq, int Hkv, int nsplit, float* part_o, float* part_ml, int* counters, bf16* out, int out_ld, cudaStream_t s);
+                      int Hq, int Hkv, float* part_o, float* part_ml, int* counters, bf16* out, int out_ld, cudaStream_t s);
 
 int attn_oproj_decode(bf16* qkv, bf16* kc, bf16* vc, const int* page_table, int page_size, const int* kv_len,
                       const int* rope_pos, const int* finished, const float* inv_freq, int Hq, int Hkv, int nsplit,
@@ -98,13 +101,16 @@ int gemv_norm_swiglu(const bf16* W_gu, int ldw, const bf16* x, const bf16* norm_
 int gemv_norm_logits(const bf16* W, int ldw, const bf16* x, const bf16* norm_w, float eps, float* logits,
                      float* logits_copy, int N, int K, const int* finished, int num_sms, bool pdl, cudaStream_t s);
 
+// The same for rows x_rows[b] of x, b < B <= 8, with the sums of gemv_norm_logits and one read of W: row b of logits. normed: [B, K] scratch
+int gemv_norm_logits_rows(const bf16* W, int ldw, const bf16* x, int ldx, const int* x_rows, int B, const bf16* norm_w, float eps, bf16* normed,
+                          float* logits, float* logits_copy, int N, int K, cudaStream_t s);
+
 // gemv_batch.cu: the projections of a decode step for B <= 8 streams (rows of x, ldx elements apart). N % 32 == 0, K % 64 == 0, W dense.
 struct GemvBatch {
     const bf16* W;
     const bf16* x;
     int N, K, ldx, B;
     const int* const* finished;   // [B] device flags: a finished stream's rows stay as they are
-    const int* x_rows;            // [B] rows of x, or null: 0, 1, ...
     const void* pf_ptr;           // L2 prefetch of the next kernel's weights
     size_t pf_bytes;
 };

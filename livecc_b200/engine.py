@@ -349,10 +349,10 @@ class LiveCCB200ForConditionalGeneration:
         after another). Every request is a dict with the per-stream arguments of generate() (`input_ids` [1, L],
         `pixel_values_videos` | `video_frames`, `video_grid_thw`, `past_key_values`). The ViT runs per stream; the new
         tokens of all streams are prefilled in one pass (up to PREFILL_ROWS of them at a time), and every decode step is one pass
-        too: each weight byte is read once for all streams. The sums of a pass are taken in an order that depends on its rows, so
-        a stream's logits may differ from generate()'s in their last bits. With LIVECC_B200_MEGA=1 streams are prefilled one by
-        one and decoded by the persistent kernel: ids, logits and caches are then bit-identical to generate() on each
-        alone (tests/test_mega_gpu.py::test_batched_decode_equals_sequential)."""
+        too. A stream's ids, logits and cache do not depend on the other streams, and its first token's logits and its prompt's cache are
+        bit-identical to generate()'s (tests/test_batch_gpu.py). The decode steps of several streams sum in another order than
+        those of one, so later logits may differ from generate()'s in their last bits; with LIVECC_B200_MEGA=1 both decode
+        through the persistent kernel and agree bit for bit (tests/test_mega_gpu.py::test_batched_decode_equals_sequential)."""
         if not 1 <= len(requests) <= _cabi.MAX_BATCH:
             raise ValueError(f"generate_batch takes 1..{_cabi.MAX_BATCH} streams")
         self._check_common(None, None, do_sample, max_new_tokens)

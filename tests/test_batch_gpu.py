@@ -1,6 +1,7 @@
-"""Several streams in one pass (prefill, decode steps, lm_head of each stream's last row) against the same streams taken one by one through
-the one-stream kernels: logits within the rounding of the storage type, ids the same unless the best two logits are that close, caches equal
-in length and content within the same rounding; streams that end early leave the others alone."""
+"""Several streams in one pass (prefill, decode steps, lm_head of each stream's last row): prompts have the bits of a pass of their own (cache and
+first logits), decode steps have the same bits whoever the neighbours are and in whichever place a stream stands; against the one-stream
+decode kernels logits and caches agree within the rounding of the storage type. Ids are the selection that each stream's own logits and history
+give. Streams that end early leave the others alone."""
 import pytest
 import torch
 
@@ -56,6 +57,17 @@ def _rel(a, b):
 TOL = 0.02
 
 
+def _check_ids(out, n, penalty):
+    """Every id is the best of its own logits, those of ids that the stream has seen divided (or multiplied, if negative) by the penalty."""
+    ids = out.sequences[0]
+    for i, lg in enumerate(out.logits):
+        seen = ids[:n + i].unique()
+        lg = lg.clone()
+        lg[seen] = torch.where(lg[seen] < 0, lg[seen] * penalty, lg[seen] / penalty)
+        best = lg.max()
+        assert lg[ids[n + i]] >= best - 1e-6 * best.abs(), (i, int(ids[n + i]), int(lg.argmax()))
+
+
 @pytest.mark.parametrize("which,spec", [
     ("small", [(0, 1, 0), (0, 2, 0)]),                                                       # single new rows
     ("small", [(63, 5, 0), (64, 1, 0), (65, 17, 2)]),                                        # edges of a page, one stream with frames
@@ -76,21 +88,48 @@ def test_streams_together_match_streams_alone(engines, which, spec):
     for b, (a, t, (ids, _, _)) in enumerate(zip(alone, together, reqs)):
         n = ids.shape[1]
         assert t.past_key_values.get_seq_length() == a.past_key_values.get_seq_length() == n + new - 1
-        same = True
+        _check_ids(a, n, 1.05)
+        _check_ids(t, n, 1.05)
+        assert torch.equal(t.logits[0], a.logits[0]), b            # the prompt's pass: the bits of the stream alone
+        same = new
         for i in range(new):
-            if not same:
-                break
             assert _rel(t.logits[i], a.logits[i]) < TOL, (b, i)
-            x, y = int(t.sequences[0, n + i]), int(a.sequences[0, n + i])
-            if x != y:   # only where the best two are within both arms' rounding
-                same = False
-                assert abs(a.logits[i][x] - a.logits[i][y]) < 0.06 * max(1.0, a.logits[i].abs().max().item()), (b, i)
-        m = n if not same else n + new - 1
+            if t.sequences[0, n + i] != a.sequences[0, n + i]:     # (each arm has selected by its own logits: from here on they go apart)
+                same = i
+                break
+        m = n + min(same, new - 1)
         for l, (k, v) in enumerate(kv_alone[b]):
             tk, tv = t.past_key_values.gather(l)
+            assert torch.equal(tk[..., :n, :], k[..., :n, :]) and torch.equal(tv[..., :n, :], v[..., :n, :]), (b, l)
             assert _rel(tk[..., :m, :], k[..., :m, :]) < TOL and _rel(tv[..., :m, :], v[..., :m, :]) < TOL, (b, l)
         a.past_key_values.release()
         t.past_key_values.release()
+
+
+@pytest.mark.parametrize("which,spec,penalty", [
+    ("small", [(0, 9, 2), (130, 3, 0), (1, 1, 0), (64, 64, 0), (200, 2, 2), (0, 300, 0), (40, 18, 6), (7, 11, 0)], 1.6),
+    ("wide", [(4200, 40, 0), (90, 19, 2), (16500, 7, 0), (700, 400, 0), (16300, 90, 0)], 1.05),    # 1, 2 and more key ranges; both sides of the bound
+])
+def test_a_streams_bits_do_not_depend_on_its_neighbours(engines, which, spec, penalty):
+    eng, new = engines[which], 6
+    reqs = _requests(eng, spec, seed=len(spec))
+    def together(of):
+        outs = eng.generate_batch([dict(input_ids=reqs[b][0].to(DEV), past_key_values=c, **({"video_frames": reqs[b][2]} if reqs[b][2] is not None else {}))
+                                   for b, c in zip(of, _caches(eng, [reqs[b] for b in of]))], repetition_penalty=penalty, max_new_tokens=new, output_logits=True)
+        res = {}
+        for b, o in zip(of, outs):
+            _check_ids(o, reqs[b][0].shape[1], penalty)
+            res[b] = (o.sequences.clone(), torch.stack(o.logits), [tuple(x.clone() for x in o.past_key_values.gather(l)) for l in range(eng.config.text_config.num_hidden_layers)])
+            o.past_key_values.release()
+        return res
+
+    every = list(range(len(spec)))
+    full = together(every)
+    for of in ([0, 1], every[::-1], [4, 2, 3], [3, 4]):
+        for b, (seq, logits, kv) in together(of).items():
+            assert torch.equal(seq, full[b][0]) and torch.equal(logits, full[b][1]), (of, b)
+            for l, (k, v) in enumerate(kv):
+                assert torch.equal(k, full[b][2][l][0]) and torch.equal(v, full[b][2][l][1]), (of, b, l)
 
 
 def test_a_stream_that_ends_leaves_the_others_alone(engines):
@@ -117,3 +156,22 @@ def test_a_stream_that_ends_leaves_the_others_alone(engines):
         assert torch.equal(k1, k0[..., :k1.shape[-2], :])
         f.past_key_values.release()
         c.past_key_values.release()
+
+
+def test_one_token_each_of_a_model_that_batched_decoding_refuses():
+    """Prefill of several streams asks for no more than prefill of one; decode steps of several streams need widths of 256."""
+    from livecc_b200._cabi import LiveCCNativeError
+    from livecc_b200.engine import LiveCCB200ForConditionalGeneration
+
+    cfg = LiveCCConfig(text_config=TextConfig(hidden_size=384, intermediate_size=1056, num_hidden_layers=2, num_attention_heads=3, num_key_value_heads=1),
+                       vision_config=VisionConfig(depth=1, embed_dim=320, hidden_size=384, num_heads=4), name="odd").with_vocab(4104)
+    sd = synthetic_state_dict(cfg, dtype=torch.bfloat16, device=DEV, gen_device=DEV)
+    eng = LiveCCB200ForConditionalGeneration.from_state_dict(cfg, sd, DEV)
+    reqs = _requests(eng, [(0, 9, 2), (70, 3, 0), (0, 140, 0)], seed=3)
+    call = lambda new: eng.generate_batch([dict(input_ids=ids.to(DEV), **({"video_frames": v} if v is not None else {})) for ids, _, v in reqs],
+                                          max_new_tokens=new, output_logits=True)
+    for t, (ids, _, v) in zip(call(1), reqs):
+        a = eng.generate(input_ids=ids.to(DEV), max_new_tokens=1, output_logits=True, **({"video_frames": v} if v is not None else {}))
+        assert torch.equal(t.logits[0], a.logits[0]) and torch.equal(t.sequences, a.sequences)
+    with pytest.raises(LiveCCNativeError, match="batched decoding"):
+        call(2)
