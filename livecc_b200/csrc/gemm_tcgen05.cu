@@ -1198,9 +1198,8 @@ static int launch_epi(const GemmArgs& a, int bn, int num_sms, cudaStream_t strea
 //    per-k-block times of every shape in the sweep fit this at the ~1.4 GHz the SMs run under tensor load);
 //  * every launch carries ~8 us that does not depend on the tile (launch gap, barrier/TMEM set-up, first TMA round trip,
 //    the un-overlapped epilogue of the last tile), which is 30-60 % of the M = 281 / 1024 GEMMs of the streaming path;
-//  * because of that fixed part, filling the last wave exactly (widths like 224 or 144, which the run-time width allows)
-//    measured within noise of the simple rule below (prefill qkv: 96 -> 24.3 us, 128 -> 23.5, 192 -> 25.3, 256 -> 29.5).
-// So, for grouped and batched products and those with a gate: 64-wide tiles never win; between 128 and 256 the cost is (waves over the SMs) x (128 + bn), ties to the narrower tile.
+// For grouped and batched products, those with a gate and those with fp32 output: 64-wide tiles never win; between 128 and 256 columns the cost is
+// (waves over the SMs) x (128 + bn), ties to the narrower tile. (Widths in between, which fill a last wave, are weighed for plain products only.)
 static int choose_bn(int M, int N, int num_sms) {
     if (N <= 64) return 64;
     const long long m_tiles = (M + BLOCK_M - 1) / BLOCK_M;
@@ -1218,7 +1217,7 @@ static int choose_bn(int M, int N, int num_sms) {
 // 1024 x 5120 x 1280 25 | 160: 21.6 | 23.2 | 21.6, 2048 x 1280 x 5120 31.3 | 192: 27.9 | 31.2 | 160: 29.3, 2090 x 4608 x 3584 66 | 192: 58 | 61 | 58,
 // 2090 x 3584 x 3584 47.7 | 224: 44.2 | 46 | 44.2, 8192 x 1280 x 5120 107 | 224: 95 | 98 | 95, 512 x 10304 x 2048 29 | 160: 24 | 26 | 24,
 // 8192 x 3840 x 1280 66 | 256: 66 | 62.4 | pair, 2090 x 37888 x 3584 432 | 224: 424 | 389 | pair, 600 x 37888 x 3584 128 | 256: 128 | 139 | 128.
-// Every sum runs over k in the same order.
+// Both forms add over k in the same order at every width.
 static double tile_us(int M, int N, int K, int rows, int bn, int at_once, double per_kb) {
     const long long units = (long long)((M + rows - 1) / rows) * ((N + bn - 1) / bn), nkb = (K + BLOCK_K - 1) / BLOCK_K;
     return (double)((units + at_once - 1) / at_once * nkb) * per_kb;
@@ -1235,12 +1234,12 @@ static int choose_alone(int M, int N, int K, int num_sms, double* us) {
     }
     return width;
 }
-// width of a pair's tile, 0 where one CTA (estimate `alone`) is not slower
+// width of a pair's tile, 0 where one CTA (estimate `alone`) is not slower by more than the estimates' error
 static int choose_pair(int M, int N, int K, int num_sms, double alone, double* us) {
     static constexpr double per_kb[5] = {0.31, 0.31, 0.325, 0.345, 0.335};
     *us = alone;
     if (N <= 64 || num_sms < 2) return 0;
-    double best = alone;
+    double best = 0.98 * alone;
     int width = 0;
     for (int i = 0; i < 5; ++i) {
         const double t = 8.0 + tile_us(M, N, K, 2 * BLOCK_M, 128 + 32 * i, num_sms / 2, per_kb[i]);
@@ -1251,11 +1250,12 @@ static int choose_pair(int M, int N, int K, int num_sms, double alone, double* u
 }
 
 // Few rows: is the swapped kernel the better one? `other`: the estimate of the best other form (0: none, narrow products). One wave of
-// clusters of 2 s CTAs (two waves where all rows are one tile), max(0.42, rows / 700) us per k-block of a pair's share, 7 us for the launch,
-// 3.5 for the exchange of a split, 0.5 per 64 rows for the store. Measured (us, best of the other forms | this, back to back): 281 rows x 3584
-// x 18944 58 | 46, x 37888 x 3584 85 | 71, x 3584 x 3584 21.0 | 19.7; 24 x 4608 x 3584 18.8 | 16.0, x 3584 x 3584 18.7 | 14.5; 256 x 5120 x 5120
-// 27 | 25, x 3584 x 5120 26 | 21; 1024 x 1280 x 5120 27 | 24; 2090 x 3584 x 18944 219 | 210; others stay for 24 x 37888 x 3584 46 | 55, x 3584
-// x 18944 31 | 40.
+// clusters of 2 s CTAs (two waves where all rows are one tile), max(0.42, rows / 700) us per k-block of a pair's share, 6.5 us for the launch,
+// 2.5 and 0.8 per 64 rows for the exchange of a split, 0.5 per 64 rows for the store. Measured (us, best of the other forms | this, back to back):
+// 281 rows x 3584 x 18944 52 | 48, x 37888 x 3584 81 | 72, 24 x 4608 x 3584 19.3 | 15.9, 256 x 5120 x 5120 28.5 | 27.1; others stay for 328 x 3584 x 3584
+// 20.3 | 23.9 (taken while the exchange was held to cost 3.5 whatever the rows), 1288 x 1280 x 5120 27.0 | 28.1, 24 x 3584 x 18944 31 | 40. Over 208
+// products (8 to 2048 rows of the models' shapes) the choice of all forms takes 0.7 % more than the best form of each, at most 11 %.
+// The unsplit forms have the same bits; a split of K changes the order of the sum.
 static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_out, int* splits_out) {
     const int n_tiles = (N + 2 * BLOCK_M - 1) / (2 * BLOCK_M), nkb = (K + BLOCK_K - 1) / BLOCK_K;
     const int t0 = (M + kSwapMax - 1) / kSwapMax;
@@ -1264,7 +1264,7 @@ static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_
     const int dev = current_device();
     int fit[kSwapSplits + 1];
     for (int sp = 1; sp <= kSwapSplits; ++sp) fit[sp] = max_clusters(dev, sp, num_sms);
-    double best = 0.98 * other;
+    double best = other;
     bool found = false;
     for (int tiles = t0; tiles <= 2 * t0 + 2; ++tiles) {
         const int bm = ((M + tiles - 1) / tiles + 31) / 32 * 32, m_tiles = (M + bm - 1) / bm, units = m_tiles * n_tiles;
@@ -1274,7 +1274,7 @@ static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_
             if (waves > (sp == 1 && m_tiles == 1 ? 2 : 1) || nkb < 4 * sp) continue;
             const SwapTile t = make_swap(bm, sp);
             if (sp > 1 && bm * BLOCK_M * 4 > t.stages * t.stage_bytes) continue;
-            const double us = 7.0 + waves * ((nkb + sp - 1) / sp) * std::max(0.42, bm / 700.0) + 0.5 * bm / 64 + (sp > 1 ? 3.5 : 0.0);
+            const double us = 6.5 + waves * ((nkb + sp - 1) / sp) * std::max(0.42, bm / 700.0) + 0.5 * bm / 64 + (sp > 1 ? 2.5 + 0.8 * bm / 64 : 0.0);
             if (us < best) { best = us; *bm_out = bm; *splits_out = sp; found = true; }
         }
     }
@@ -1384,7 +1384,7 @@ GemmPlan gemm_plan(const GemmArgs& a, int num_sms) {
     if (width) p.form = FORM_PAIR;
     if (const int ranges = splitk_ranges(a, num_sms)) {   // two launches, the partials written and read once
         const int w = splitk_width(a), tiles = (a.M + BLOCK_M - 1) / BLOCK_M * ((a.N + w - 1) / w), nkb = (a.K + BLOCK_K - 1) / BLOCK_K;
-        us = 11.0 + (tiles * ranges + num_sms - 1) / num_sms * ((nkb + ranges - 1) / ranges) * 0.41 + (double)a.M * a.N * ranges * 4 / 6.5e6;
+        us = 14.0 + (tiles * ranges + num_sms - 1) / num_sms * ((nkb + ranges - 1) / ranges) * 0.41 + (double)a.M * a.N * ranges * 4 / 6.5e6;
         p.form = FORM_ONE;
     }
     int bm = 0, splits = 0;

@@ -269,3 +269,32 @@ def test_gemm_widths_between_128_and_256(ctx, M, N, K, width, epi):
     if epi == A.EPI_BIAS_RESIDUAL:
         kw["residual"] = _ints((M, N), -8, 8, 54)
     assert torch.equal(ctx.gemm(a, b, epilogue=epi, **kw), ctx.gemm(a, b, epilogue=epi, block_n=128, **kw))
+
+
+@pytest.mark.parametrize("M,N,K,form", [(328, 3584, 3584, 0), (344, 3584, 3584, 0), (328, 4608, 3584, 0), (1288, 1280, 5120, 0), (1400, 1280, 5120, 0),
+                                        (24, 4608, 3584, 2), (281, 3584, 18944, 2), (281, 37888, 3584, 2)])
+def test_plan_weighs_the_exchange_of_a_split(ctx, M, N, K, form):
+    """The swapped form with K split over a cluster where it measured faster (form 2), one CTA per tile where the exchange of many rows costs more
+    than the split gives (328 x 3584 x 3584: 20.3 us, 23.9 split in four)."""
+    assert ctx.gemm_plan(M, N, K)[0] == form
+
+
+@pytest.mark.parametrize("epi", [A.EPI_SWIGLU, A.EPI_CLAMP_GLU])
+@pytest.mark.parametrize("form,width", [(0, 96), (0, 160), (0, 224), (1, 160), (1, 224)])
+@pytest.mark.parametrize("M,N,K", [(130, 224, 192), (1, 96, 64), (700, 1056, 320)])
+def test_gated_epilogues_at_widths_in_between(ctx, epi, form, width, M, N, K):
+    """Two lanes exchange the halves of a row's 16 outputs: every width, ragged rows and columns, the bits of the 128-column kernel."""
+    a, b = _ints((M, K), -1, 1, 61) * 0.25, _ints((N, K), -1, 1, 62) * 0.25
+    kw = dict(epilogue=epi, limit=1.5)
+    want = ctx.gemm_form(a, b, 0, 128, **kw)
+    out = torch.full((M + 2, N // 2), 7.0, dtype=torch.bfloat16, device="cuda")
+    ctx.gemm_form(a, b, form, width, out=out[:M], **kw)
+    assert torch.equal(out[:M], want) and bool((out[M:] == 7.0).all())
+    g, u = (a.double() @ b.double().T).view(M, N // 32, 2, 16).unbind(2)
+    if epi == A.EPI_SWIGLU:
+        y = (g / (1 + (-g).exp())) * u
+    else:
+        g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
+        y = g / (1 + (-1.702 * g).exp()) * (u + 1.0)
+    # bf16 roundings of gate, up, their product (and silu): 2^-9 relative each, 4 of them
+    assert bool(((out[:M].double() - y.reshape(M, -1)).abs() <= y.reshape(M, -1).abs() * 2.0 ** -7 + 1e-6).all())
