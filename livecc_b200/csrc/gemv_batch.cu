@@ -29,20 +29,15 @@ struct GemvBatchParams {
 
 constexpr int kGbWarps = 8;
 
-// Measured with 8 streams (hidden 3584; for comparison one stream's CUDA-core kernels): lm_head 166 us (172), gate/up 43.8 (43), down 27.0 (25),
+// Measured with 8 streams (hidden 3584; for comparison one stream's CUDA-core kernels): lm_head 168 us (172), gate/up 43.8 (43), down 25.3 (25),
 // qkv 9.0 (11.1, RMSNorm included), o 10.1 (9.6).
-// MT: 16-row tiles per CTA (GB_SWIGLU: 16 gate rows and their 16 up rows). KS: CTAs of a cluster that share K. UN: units of 64 k in flight.
-// CTAs per SM are fixed, or a change of a few registers moves these times by a tenth (down at 80 registers 33 us, the head at 68 170).
-template <int MT, int KS, int UN, int EPI>
-__global__ void __launch_bounds__(kGbWarps * 32, EPI == GB_SWIGLU ? 3 : UN > 2 ? 2 : 4) gemv_batch_kernel(const GemvBatchParams p) {
+// MT: 16-row tiles per CTA (GB_SWIGLU: 16 gate rows and their 16 up rows). UN: units of 64 k in flight.
+// CTAs per SM are fixed, or a change of a few registers moves these times by a tenth (the head at 68 registers 170 us).
+template <int MT, int UN, int EPI>
+__global__ void __launch_bounds__(kGbWarps * 32, EPI == GB_SWIGLU ? 3 : UN > 1 ? 2 : 4) gemv_batch_kernel(const GemvBatchParams p) {
     __shared__ float part[kGbWarps][MT * 128];   // [row][stream] per warp
-    __shared__ float peers[KS][MT * 128];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    if (KS > 1) cluster_arrive();   // waited for in front of the first store into another CTA's shared memory: that CTA has started
-    const int tile = blockIdx.x / KS, rank = KS > 1 ? blockIdx.x % KS : 0;
-    const int n0 = tile * MT * 16;
-    const int units = p.K >> 6, mine = (units + KS - 1) / KS;
-    const int u0 = rank * mine, u1 = min(units, u0 + mine);
+    const int tile = blockIdx.x, n0 = tile * MT * 16, units = p.K >> 6;
     const bf16* w0 = p.W + (size_t)(n0 + g) * p.K + t * 8;
     const bf16* x0 = p.x + (size_t)(g < p.B ? g : 0) * p.ldx + t * 8;
     float acc[MT][4];
@@ -72,24 +67,23 @@ __global__ void __launch_bounds__(kGbWarps * 32, EPI == GB_SWIGLU ? 3 : UN > 2 ?
             }
         }
     };
-    int u = u0 + warp;
+    int u = warp;
     const int done = lane < p.B ? *p.finished[lane] : 1;
     bool open = false;
     auto ended = [&] {   // every stream has ended (a replayed graph): nothing to do, seen while the first weights arrive
         if (open || !__all_sync(0xffffffffu, done)) { open = true; return false; }
-        if (KS > 1) cluster_wait();
         return true;
     };
-    if constexpr (UN == 1) {   // (the loop turned like this: gate/up 43.8 us, 48.4 as below; with 2 units in flight 35 for the 27 of the down projection)
-        if (u < u1) load(u, w[0]);
+    if constexpr (UN == 1) {   // (the loop turned like this: gate/up 43.8 us, 48.4 as below)
+        if (u < units) load(u, w[0]);
         if (ended()) return;
-        while (u < u1) {
+        while (u < units) {
             compute(u, w[0]);
             u += kGbWarps;
-            if (u < u1) load(u, w[0]);
+            if (u < units) load(u, w[0]);
         }
     } else {
-        for (; u + (UN - 1) * kGbWarps < u1; u += UN * kGbWarps) {
+        for (; u + (UN - 1) * kGbWarps < units; u += UN * kGbWarps) {
 #pragma unroll
             for (int i = 0; i < UN; ++i) load(u + i * kGbWarps, w[i]);
             if (ended()) return;
@@ -101,12 +95,12 @@ __global__ void __launch_bounds__(kGbWarps * 32, EPI == GB_SWIGLU ? 3 : UN > 2 ?
     if (UN > 1) {
 #pragma unroll
         for (int i = 0; i < UN - 1; ++i)
-            if (u + i * kGbWarps < u1) load(u + i * kGbWarps, w[i]);
+            if (u + i * kGbWarps < units) load(u + i * kGbWarps, w[i]);
 #pragma unroll
         for (int i = 0; i < UN - 1; ++i)
-            if (u + i * kGbWarps < u1) compute(u + i * kGbWarps, w[i]);
+            if (u + i * kGbWarps < units) compute(u + i * kGbWarps, w[i]);
     }
-    // ---- partials: warps in order, then the cluster's CTAs in order ----
+    // ---- partials: warps in order ----
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
         float* d = part[warp] + m * 128 + g * 8 + t * 2;
@@ -127,22 +121,6 @@ __global__ void __launch_bounds__(kGbWarps * 32, EPI == GB_SWIGLU ? 3 : UN > 2 ?
     if (i < MT * 128) {
 #pragma unroll
         for (int k = 0; k < kGbWarps; ++k) sum += part[k][i];
-    }
-    if (KS > 1) {
-        __syncwarp();
-        cluster_wait();
-        if (i < MT * 128) {
-            const uint32_t a = mapa_shared(smem_u32(&peers[rank][i]), 0);
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(sum) : "memory");
-        }
-        __syncwarp();
-        cluster_sync_all();
-        if (rank) return;
-        if (i < MT * 128) {
-            sum = 0.f;
-#pragma unroll
-            for (int k = 0; k < KS; ++k) sum += peers[k][i];
-        }
     }
     if (EPI == GB_SWIGLU) {   // rows 0..15 gate, 16..31 up
         __syncthreads();
@@ -166,20 +144,12 @@ __global__ void __launch_bounds__(kGbWarps * 32, EPI == GB_SWIGLU ? 3 : UN > 2 ?
     else { const float v = rbf(sum); p.out_f32[o] = v; p.out_f32_b[o] = v; }
 }
 
-template <int MT, int KS, int UN, int EPI>
+template <int MT, int UN, int EPI>
 static int launch_batch(const GemvBatchParams& p, cudaStream_t s) {
     if (p.B < 1 || p.B > kBatchStreams || p.N % (MT * 16) || p.K % 64 || p.ldx % 8) return -1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(p.N / (MT * 16) * KS);
-    cfg.blockDim = dim3(kGbWarps * 32);
-    cfg.stream = s;
-    cudaLaunchAttribute a[1];
-    a[0].id = cudaLaunchAttributeClusterDimension;
-    a[0].val.clusterDim.x = KS; a[0].val.clusterDim.y = 1; a[0].val.clusterDim.z = 1;
-    cfg.attrs = a;
-    cfg.numAttrs = KS > 1 ? 1 : 0;
     count_launch();
-    return cudaLaunchKernelEx(&cfg, gemv_batch_kernel<MT, KS, UN, EPI>, p) == cudaSuccess ? 0 : -2;
+    gemv_batch_kernel<MT, UN, EPI><<<p.N / (MT * 16), kGbWarps * 32, 0, s>>>(p);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 static GemvBatchParams params_of(const GemvBatch& a) {
@@ -193,25 +163,24 @@ static GemvBatchParams params_of(const GemvBatch& a) {
 int gemv_batch_bias(const GemvBatch& a, const bf16* bias, bf16* out, int ldo, cudaStream_t s) {
     GemvBatchParams p = params_of(a);
     p.bias = bias; p.out = out; p.ldo = ldo;
-    return launch_batch<1, 1, 4, GB_BIAS>(p, s);
+    return launch_batch<1, 4, GB_BIAS>(p, s);
 }
 int gemv_batch_residual(const GemvBatch& a, bf16* h_inout, int ldo, cudaStream_t s) {
     GemvBatchParams p = params_of(a);
     p.out = h_inout; p.ldo = ldo;
-    // Few rows with a long K (down: 224 tiles of 16 rows x 18944): two CTAs per tile, or the SMs with two tiles keep the others waiting
-    // (28.2 us; one CTA per tile 29.5 with 4 units in flight and 36.5 with 2, 32-row tiles with K in 2 | 4 29 to 38 | 31).
-    if (a.K > 8192) return launch_batch<1, 2, 2, GB_RESIDUAL>(p, s);
-    return launch_batch<1, 1, 4, GB_RESIDUAL>(p, s);
+    // (Two CTAs per tile, sharing K through a cluster, was taken for K > 8192: at two CTAs per SM it never pays, N x K = 1536 to 8192 x 1536 to 27648,
+    // 8 streams: 3584 x 18944 26.4 us either way, 25.3 for 27.0 in a step, 2560 x 18944 22.2 | 21.8, 7168 x 18944 49.6 | 52.2, 1536 x 18944 17.0 | 19.2.)
+    return launch_batch<1, 4, GB_RESIDUAL>(p, s);
 }
 int gemv_batch_swiglu(const GemvBatch& a, bf16* act, int ldo, cudaStream_t s) {
     GemvBatchParams p = params_of(a);
     p.out = act; p.ldo = ldo;
-    return launch_batch<2, 1, 1, GB_SWIGLU>(p, s);   // (2 units in flight were slower: registers)
+    return launch_batch<2, 1, GB_SWIGLU>(p, s);   // (2 units in flight were slower: registers)
 }
 int gemv_batch_logits(const GemvBatch& a, float* logits, float* logits_copy, int ldo, cudaStream_t s) {
     GemvBatchParams p = params_of(a);
     p.out_f32 = logits; p.out_f32_b = logits_copy; p.ldo = ldo;
-    return launch_batch<2, 1, 1, GB_LOGITS>(p, s);
+    return launch_batch<2, 1, GB_LOGITS>(p, s);
 }
 
 }  // namespace lcc

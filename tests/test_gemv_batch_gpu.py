@@ -1,6 +1,5 @@
 """The projections of a decode step of several streams (gemv_batch.cu) by themselves: whole-number operands whose products and sums are exact in
-fp32, so that every order of summation gives the same bits; every number of streams, K on both sides of the bound from which two CTAs share a
-row's K, finished streams. With real-valued operands, a stream's row has the same bits whoever its neighbours are."""
+fp32, so that every order of summation gives the same bits; every number of streams, short and long K, finished streams. With real-valued operands, a stream's row has the same bits whoever its neighbours are."""
 import pytest
 import torch
 
