@@ -568,6 +568,12 @@ int lcc_gated_scan(lcc_ctx* ctx, int dt, const void* k, int ld_k, const void* c,
                    const float* sc, const float* skip, float cs, float* state, float* y, int ld_y, int S, int heads, int heads_per_group, int N, int P,
                    float* ws, int64_t ws_floats, lcc_stream_t stream);
 int64_t lcc_gated_scan_ws_floats(int S, int heads, int N, int P);
+/* The masked attention of the hybrid models by itself (tests and tuning): S new rows at positions past .. over the cached keys of the same chunk (0: one)
+ * and of the last `window` positions (0: all); sink: a score of 0 without a value in the softmax; gate: logits [S, ld_gate], one per head or
+ * (gate_channel) per channel, or NULL. q: fp32 [S, Hq * D]; pages [page][G][page_size][D | DV], dt; out: [S, ld_out], dt. */
+int lcc_attn_masked(lcc_ctx* ctx, int dt, const float* q, const void* k_pages, const void* v_pages, const int32_t* page_table, int page_size, const void* gate,
+                    int ld_gate, int gate_channel, void* out, int ld_out, int S, int past, int Hq, int G, int D, int DV, int chunk, int window, int sink,
+                    float scale, lcc_stream_t stream);
 
 typedef struct lcc_seq_model lcc_seq_model;
 /* sizeof(lcc_seq_layer) (which = 0), sizeof(lcc_seq_model_desc) (1), sizeof(lcc_seq_entry) (2): a binding checks its own layout against them */

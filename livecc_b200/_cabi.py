@@ -493,6 +493,17 @@ class Context:
                   _i(out.stride(0)), self.stream_ptr())
         return out if out2 is None else (out, out2)
 
+    def attn_masked(self, q, k_pages, v_pages, page_table, past, scale, chunk=0, window=0, sink=False, gate=None, gate_channel=False):
+        """q fp32 [S, Hq, D]; pages [page, G, page_size, D | DV] bf16 (or fp32); gate [S, Hq] or [S, Hq * DV] like the pages. -> [S, Hq, DV]"""
+        import torch
+
+        (S, Hq, D), (_, G, ps, DV) = q.shape, v_pages.shape
+        out = torch.empty((S, Hq, DV), dtype=v_pages.dtype, device=q.device)
+        self.call("lcc_attn_masked", _i(0 if v_pages.dtype == torch.bfloat16 else 1), _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(page_table), _i(ps),
+                  _ptr(gate), _i(gate.stride(0) if gate is not None else 0), _i(gate_channel), _ptr(out), _i(Hq * DV), _i(S), _i(past), _i(Hq), _i(G),
+                  _i(D), _i(DV), _i(chunk), _i(window), _i(sink), C.c_float(scale), self.stream_ptr())
+        return out
+
     def gated_scan(self, k, c, u, log_decay, state, sc=None, skip=None, cs=1.0, blocks=True):
         """y of the gated linear recurrence; k, c [S, G, N], u [S, H, P] (bf16, or all fp32), log_decay [S, H] or [S, H, N] fp32, state fp32
         [H, P, N], updated. blocks: the form over blocks of 64 rows (32 rows or more) instead of token by token."""

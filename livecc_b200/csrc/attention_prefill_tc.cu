@@ -68,7 +68,6 @@ __device__ __forceinline__ float ex2_ftz_p(float x) {
 struct PrefillLocal {
     const float* q;       // [S, Hq, 128]
     SeqPos pos;
-    const float* sink;    // [Hq], or null: 0
     const bf16* gate;
     int ld_gate, chunk, window;
     bool no_sink, gate_channel;
@@ -256,10 +255,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         const int first = LOCAL && row_ok ? lp.first_key(lim) : 0;
         float m_used = -INFINITY, l = 0.f;
         if (LOCAL) {
-            if (!lp.no_sink && row_ok) {   // the sink's term starts the sum
-                m_used = (lp.sink ? lp.sink[kvh * p.G + rg] : 0.f) * 1.4426950408889634f;
-                l = 1.f;
-            }
+            if (!lp.no_sink && row_ok) { m_used = 0.f; l = 1.f; }   // the sink (a score of 0 without a value) starts the sum
             // queries: a warp takes its 32 rows one by one, four channels per lane, into the K-major 128-byte-swizzled tile
             const int Hq = p.Hkv * p.G, c = lane & 15;   // lanes 0..15: channels 0..63 in 8-byte pieces
             uint8_t* sq = smem + OFF_Q + (lane >> 4) * Q_ATOM_BYTES;
@@ -357,7 +353,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         }
         const bf16* gate = LOCAL && lp.gate && row_ok
                                ? lp.gate + (size_t)(pos0 + rpos) * lp.ld_gate + (lp.gate_channel ? (size_t)(kvh * p.G + rg) * D : (size_t)(kvh * p.G + rg)) : nullptr;
-        auto sigmoid = [](float x) { return __fdividef(1.f, 1.f + expf(-x)); };
+        // (a denominator of 1 to 2 whatever x is, so that the short reciprocal has its range; one Newton step makes up for its error)
+        auto sigmoid = [](float x) {
+            const float t = expf(-fabsf(x)), d = 1.f + t, r = __fdividef(1.f, d);
+            return (x < 0.f ? t : 1.f) * fmaf(r, fmaf(-d, r, 1.f), r);
+        };
         mbar_wait(pv_done, (T - 1) & 1);
         tc_fence_after();
         if (parts) {
@@ -473,15 +473,15 @@ int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, con
 }
 
 bool attn_local_tc_takes(const float* q, const void* k_pages, const void* v_pages, int page_size, const void* gate, int ld_gate, const void* out,
-                         int ld_out, int Hq, int G, int D, int DV, int ld_v, const AttnOpts& opt) {
-    const bool plain = opt.softcap <= 0.f && opt.keep_first <= 0 && opt.maps == 1 && !opt.raw && !opt.bias;
+                         int ld_out, int Hq, int G, int D, int DV, int ld_v, const float* sink, const AttnOpts& opt) {
+    const bool plain = !sink && opt.softcap <= 0.f && opt.keep_first <= 0 && opt.maps == 1 && !opt.raw && !opt.bias;
     const bool wide_gate = gate && opt.gate_channel;
     return plain && D == ptc::D && DV == ptc::D && ld_v == ptc::D && page_size == ptc::BN && Hq / G <= ptc::BM && ld_out % 8 == 0 && (!wide_gate || ld_gate % 8 == 0) &&
            (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)out | (wide_gate ? (uintptr_t)gate : 0)) & 15) == 0;
 }
 
 int attn_local_tc(const float* q, const void* k_pages, const void* v_pages, const int* page_table, const void* gate, int ld_gate, void* out,
-                  int ld_out, int S, int Hq, int G, int chunk, float scale, SeqPos pos, cudaStream_t s, const float* sink, const AttnOpts& opt) {
+                  int ld_out, int S, int Hq, int G, int chunk, float scale, SeqPos pos, cudaStream_t s, const AttnOpts& opt) {
     using namespace ptc;
     PrefillTcParams p{};
     p.out = (bf16*)out; p.o_ld = ld_out; p.Hkv = G; p.G = Hq / G; p.PT = BM / p.G;
@@ -489,7 +489,7 @@ int attn_local_tc(const float* q, const void* k_pages, const void* v_pages, cons
     p.ps.n = 1; p.ps.rows = S;
     p.ps.st[0].nsplit = 1;
     p.ps.st[0].page_table = page_table; p.ps.st[0].S = S; p.ps.st[0].past = pos.past;
-    const PrefillLocal lp{q, pos, sink, (const bf16*)gate, ld_gate, chunk > 0 ? chunk : 0, opt.window > 0 ? opt.window : 0, opt.no_sink, opt.gate_channel};
+    const PrefillLocal lp{q, pos, (const bf16*)gate, ld_gate, chunk > 0 ? chunk : 0, opt.window > 0 ? opt.window : 0, opt.no_sink, opt.gate_channel};
     CUtensorMap tk, tv;
     const int64_t pool_rows = (int64_t)1 << 31;  // (as above)
     if (make_tmap_bf16_2d_box(&tk, k_pages, pool_rows, D, D, 64, BN, false) || make_tmap_bf16_2d_box(&tv, v_pages, pool_rows, D, D, 64, BN, false)) return -100;

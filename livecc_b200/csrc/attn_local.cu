@@ -1496,8 +1496,8 @@ int attn_masked(int dt, const float* q, const void* k_pages, const void* v_pages
     const size_t smem = sizeof(float) * ((size_t)D + (size_t)std::max(max_keys, 0));
     if (S >= kAttnTiledMin || max_keys < 0 || smem > 160 * 1024 || force_tiled) {
         const bool mma = dt == DT_BF16 && tensor_cores && D <= kAttnMmaMaxDim;
-        if (mma && attn_local_tc_takes(q, k_pages, v_pages, page_size, gate, ld_gate, out, ld_out, Hq, G, D, DV, ld_v, o))
-            return attn_local_tc(q, k_pages, v_pages, page_table, gate, ld_gate, out, ld_out, S, Hq, G, chunk, scale, pos, s, sink, o);
+        if (mma && attn_local_tc_takes(q, k_pages, v_pages, page_size, gate, ld_gate, out, ld_out, Hq, G, D, DV, ld_v, sink, o))
+            return attn_local_tc(q, k_pages, v_pages, page_table, gate, ld_gate, out, ld_out, S, Hq, G, chunk, scale, pos, s, o);
         if (mma && opt.maps == 2 && DV <= 256)
             return launch_attn_mma_maps(q, k_pages, v_pages, page_table, page_size, out, ld_out, S, heads, G, D, DV, chunk, scale, pos, s,
                                         sink, ld_v, o);

@@ -149,6 +149,16 @@ int lcc_gated_scan(lcc_ctx* ctx, int dt, const void* k, int ld_k, const void* c,
     OP_RET(ctx, lcc::gated_scan(a, lcc::SeqPos{}, (cudaStream_t)stream), "lcc_gated_scan");
 }
 
+int lcc_attn_masked(lcc_ctx* ctx, int dt, const float* q, const void* k_pages, const void* v_pages, const int32_t* page_table, int page_size, const void* gate,
+                    int ld_gate, int gate_channel, void* out, int ld_out, int S, int past, int Hq, int G, int D, int DV, int chunk, int window, int sink,
+                    float scale, lcc_stream_t stream) {
+    if (dt != lcc::DT_F32 && dt != lcc::DT_BF16) return -1;
+    lcc::AttnOpts o;
+    o.window = window; o.no_sink = !sink; o.gate_channel = gate_channel != 0;
+    OP_RET(ctx, lcc::attn_masked(dt, q, k_pages, v_pages, page_table, page_size, gate, ld_gate, out, ld_out, S, Hq, G, D, DV, chunk, scale, true,
+                                 lcc::SeqPos{past, nullptr, nullptr}, (cudaStream_t)stream, o), "lcc_attn_masked");
+}
+
 int64_t lcc_gated_scan_ws_floats(int S, int heads, int N, int P) { return (int64_t)lcc::gated_scan_ws_floats(S, heads, N, P); }
 
 int lcc_sample_greedy(lcc_ctx* ctx, const float* logits_raw, float* logits_proc, int V, int64_t* seq,

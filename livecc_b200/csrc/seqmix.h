@@ -227,11 +227,11 @@ struct AppendOpts {
     bool q_only = false;
 };
 // bf16 portions of at least kAttnTiledMin rows on tcgen05 (attention_prefill_tc.cu): heads of 128 channels, pages of 64 tokens, rows on 16-byte
-// boundaries, none of softcap / keep_first / maps / bias.
+// boundaries, none of softcap / keep_first / maps / bias, no sink logits (a sink of score 0 is fine).
 bool attn_local_tc_takes(const float* q, const void* k_pages, const void* v_pages, int page_size, const void* gate, int ld_gate, const void* out,
-                         int ld_out, int Hq, int G, int D, int DV, int ld_v, const AttnOpts& opt);
+                         int ld_out, int Hq, int G, int D, int DV, int ld_v, const float* sink, const AttnOpts& opt);
 int attn_local_tc(const float* q, const void* k_pages, const void* v_pages, const int* page_table, const void* gate, int ld_gate, void* out,
-                  int ld_out, int S, int Hq, int G, int chunk, float scale, SeqPos pos, cudaStream_t s, const float* sink, const AttnOpts& opt);
+                  int ld_out, int S, int Hq, int G, int chunk, float scale, SeqPos pos, cudaStream_t s, const AttnOpts& opt);
 int attn_masked(int dt, const float* q, const void* k_pages, const void* v_pages, const int* page_table, int page_size,
                 const void* gate, int ld_gate, void* out, int ld_out, int S, int Hq, int G, int D, int DV, int chunk, float scale,
                 bool tensor_cores, SeqPos pos, cudaStream_t s, const AttnOpts& opt, const float* sink = nullptr, int ld_v = 0,

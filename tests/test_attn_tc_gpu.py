@@ -59,3 +59,54 @@ def test_windows_and_channel_gates(heads, kv_heads, window, scale, cuts, n):
 def test_chunks_sinks_and_head_gates(heads, kv_heads, chunk, scale, cuts, n):
     d = seq_cases.config([seq_cases.par(heads=heads, kv_heads=kv_heads, dim=128, vdim=128, chunk=chunk, scale=scale) for _ in range(2)], width=40)
     _check(d, seq_oracle, cuts, n, seed=heads + chunk)
+
+
+def _op_case(S, past, Hq, G, seed, vscale=1.0):
+    g = torch.Generator().manual_seed(seed)
+    pages = (past + S + 63) // 64
+    order = torch.randperm(pages, generator=g)
+    kv = torch.full((2, pages, G, 64, 128), float("nan"))
+    flat = torch.randn((2, G, past + S, 128), generator=g)
+    flat[1] *= vscale
+    flat = flat.to(torch.bfloat16).float()
+    for t in range(past + S):
+        kv[:, order[t // 64], :, t % 64] = flat[:, :, t]
+    q = torch.randn((S, Hq, 128), generator=g).to(torch.bfloat16).float()
+    return q.cuda(), kv[0].bfloat16().cuda(), kv[1].bfloat16().cuda(), order.int().cuda(), flat.double().cuda()
+
+
+def _op_want(q, flat, past, scale, chunk, window, sink, gate):
+    S, Hq, _ = q.shape
+    k, v = (x.repeat_interleave(Hq // flat.shape[1], 0) for x in flat)
+    s = torch.einsum("shd,htd->hst", q.double(), k) * scale
+    i, j = torch.arange(past, past + S, device="cuda")[:, None], torch.arange(past + S, device="cuda")[None]
+    see = (j <= i) & ((j > i - window) if window else True) & ((j // chunk == i // chunk) if chunk else True)
+    s = s.masked_fill(~see, float("-inf"))
+    m = s.amax(-1, keepdim=True).clamp_min(0.0 if sink else -1e300)
+    p = (s - m).exp()
+    o = torch.einsum("hst,htd->shd", p / (p.sum(-1, keepdim=True) + ((-m).exp() if sink else 0.0)), v)
+    return o if gate is None else o * torch.sigmoid(gate.double()).view(S, Hq, -1)
+
+
+@pytest.mark.parametrize("S,past,Hq,G,chunk,window", [(70, 0, 8, 1, 100, 30), (130, 77, 4, 2, 128, 64), (65, 191, 6, 2, 64, 1000), (200, 300, 16, 2, 150, 149), (17, 63, 3, 1, 16, 5)])
+@pytest.mark.parametrize("sink", [False, True])
+@pytest.mark.parametrize("gated", [0, 1, 2])
+def test_window_and_chunks_together(ctx, S, past, Hq, G, chunk, window, sink, gated):
+    q, k, v, table, flat = _op_case(S, past, Hq, G, S + past)
+    gate = None if not gated else torch.randn((S, Hq * (128 if gated == 2 else 1)), device="cuda").bfloat16()
+    if gated == 1:    # (a gate per head is one column of a wider row in the models)
+        gate = torch.cat([gate, gate], 1)[:, :Hq]
+    got = ctx.attn_masked(q, k, v, table, past, 0.09, chunk=chunk, window=window, sink=sink, gate=gate, gate_channel=gated == 2)
+    want = _op_want(q, flat, past, 0.09, chunk, window, sink, gate)
+    # softmax weights and the result are rounded to bf16 (2^-9 each, weights relative to values of size 1)
+    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * (want.abs() + 1.0) * 1.5).all())
+
+
+@pytest.mark.parametrize("gated", [1, 2])
+def test_gates_that_are_nearly_shut(ctx, gated):
+    """sigmoid(-88) is 6e-39, a normal quotient of a denominator past 2^126: values of 1e30 come out as 6e-9, not as zeros."""
+    q, k, v, table, flat = _op_case(80, 20, 4, 1, 3, vscale=1e30)
+    gate = torch.full((80, 4 * (128 if gated == 2 else 1)), -88.0, device="cuda").bfloat16()
+    got = ctx.attn_masked(q, k, v, table, 20, 0.09, gate=gate, gate_channel=gated == 2).double()
+    want = _op_want(q, flat, 20, 0.09, 0, 0, False, gate)
+    assert bool(((got - want).abs() <= 2.0 ** -8 * 1.5 * (want.abs() + 1e30 * 6e-39)).all()) and float(got.abs().max()) > 1e-9
