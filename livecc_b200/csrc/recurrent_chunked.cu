@@ -6,9 +6,9 @@
 //     M[t,s]= cs sc_s sum_n c_t[n] k_s[n] exp(b_t[n] - b_s[n])                       (every exponent is <= 0)
 //     S_out = diag(exp(b_last)) S_in + sum_s (k_s * exp(b_last - b_s)) (sc_s u_s)^T
 // Five launches: block-local cumulative log decays, M, the blocks' own state contributions, a short sequential pass
-// over blocks that turns them into the state entering each block, and the outputs. All arithmetic is fp32 on the
-// CUDA cores (the recurrence's operands are fp32 by the models' precision rules); the three products are register-
-// tiled 64 x 64 tiles whose operands are formed (decay factors applied) while they are staged into shared memory.
+// over blocks that turns them into the state entering each block, and the outputs. All arithmetic is fp32 (the recurrence's operands are
+// fp32 by the models' precision rules); the three products are 64 x 64 tiles whose operands are formed (decay factors applied) while
+// they are staged: on the CUDA cores, or, for a decay per head over aligned bf16 rows, on the tensor cores by values cut in three.
 #include <type_traits>
 #include <math.h>
 
@@ -536,9 +536,12 @@ __global__ void __launch_bounds__(128) chunk_output_head_kernel(ChunkArgs a, Seq
 
 // ---- the three products of bf16 rows on the tensor cores -------------------------------------------------------------------
 // Rows of c, k and u are bf16, so one operand of every product is exact; the other is fp32 (a state, decayed weights) and is cut into
-// three bf16 values that hold all its 24 bits (truncated, so that none overflows): the products of mma.sync are then exact too, and only the
-// order of the fp32 sums differs from the kernels above (which fp32 rows keep). Decays and scales stay fp32. Bound by the bytes of the
-// block states, and the cuts (2048 rows, 64 heads of 64 x 128): 7.6 + 32 + 78 us for 16 + 66 + 119 of the fp32 kernels.
+// three bf16 values that hold all its 24 bits (truncated, so that none overflows): the products of mma.sync are then exact too. Its sums are not rounded
+// like fp32 adds, and a running sum kept in its accumulators drifts (2.1e-6 of the summed magnitudes over 136 terms of one sign, where
+// fp32 adds are 1.8e-7 off): 16 terms are summed there, three parts of them one after another, and added to the sum by the CUDA cores (9e-8; random
+// signs 3.0e-9 for 4.5e-9).
+// Decays and scales stay fp32. Bound by the bytes of the block states, and the cuts (2048 rows, 64 heads of 64 x 128): 7.8 + 33 + 77 us for 16 + 66 + 119
+// of the fp32 kernels (6.9 + 31 + 71 with running sums in the accumulators).
 __device__ __forceinline__ float low_part(float x) {   // x minus its leading 8 bits; nothing behind an infinity or NaN
     return fabsf(x) < INFINITY ? x - __uint_as_float(__float_as_uint(x) & 0xffff0000u) : 0.f;
 }
@@ -548,6 +551,14 @@ __device__ __forceinline__ void cut3(float x0, float x1, uint32_t (&c)[3]) {
         c[i] = __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632);
         if (i < 2) { x0 = low_part(x0); x1 = low_part(x1); }
     }
+}
+// acc += the three parts' products, the smallest first
+__device__ __forceinline__ void add_products(float (&acc)[4], const uint32_t (&a)[3][4], uint32_t b0, uint32_t b1) {
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 2; k >= 0; --k) mma_bf16_16816(d, a[k], b0, b1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] += d[i];
 }
 constexpr int UP = 64 + 8;      // pitch of a staged bf16 tile row: ldmatrix rows fall into different banks
 // four consecutive k of rows r and r + 8 as an A fragment: which of a product's 16 places a k takes does not matter, as long as B agrees
@@ -616,8 +627,11 @@ __global__ void __launch_bounds__(128) chunk_products_tc_kernel(ChunkArgs a, Seq
         for (int i = 0; i < 4; ++i) rows_a(ca[i], gc, a.ld_c, i * 16 + gq, len, n0 + 4 * tq, a.N);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            mma_bf16_16816(acc[i][0], ca[i], kb[0], kb[2]);
-            mma_bf16_16816(acc[i][1], ca[i], kb[1], kb[3]);
+            float d[2][4] = {};
+            mma_bf16_16816(d[0], ca[i], kb[0], kb[2]);
+            mma_bf16_16816(d[1], ca[i], kb[1], kb[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { acc[i][0][e] += d[0][e]; acc[i][1][e] += d[1][e]; }
         }
     }
     float* out = a.ws_m + ((size_t)blk * groups + g) * CL * CL + warp * 16 + 2 * tq;
@@ -701,15 +715,14 @@ __global__ void __launch_bounds__(128, 5) chunk_state_tc_kernel(ChunkArgs a, Seq
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 ldmatrix_x4_trans(b[j][0], b[j][1], b[j][2], b[j][3], &sk[ks + (lane & 7) + ((lane >> 3) & 1) * 8][j * 16 + (lane >> 4) * 8]);
+            uint32_t w[3][4];
 #pragma unroll
-            for (int k = 2; k >= 0; --k) {   // the smallest part first
-                uint32_t w[4];
-                ldmatrix_x4_trans(w[0], w[1], w[2], w[3], &su[k][ks + (lane & 7) + (lane >> 4) * 8][warp * 16 + ((lane >> 3) & 1) * 8]);
+            for (int k = 0; k < 3; ++k)
+                ldmatrix_x4_trans(w[k][0], w[k][1], w[k][2], w[k][3], &su[k][ks + (lane & 7) + (lane >> 4) * 8][warp * 16 + ((lane >> 3) & 1) * 8]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    mma_bf16_16816(acc[2 * j], w, b[j][0], b[j][1]);
-                    mma_bf16_16816(acc[2 * j + 1], w, b[j][2], b[j][3]);
-                }
+            for (int j = 0; j < 4; ++j) {
+                add_products(acc[2 * j], w, b[j][0], b[j][1]);
+                add_products(acc[2 * j + 1], w, b[j][2], b[j][3]);
             }
         }
 #pragma unroll
@@ -782,9 +795,13 @@ __global__ void __launch_bounds__(128, 4) chunk_output_tc_kernel(const __grid_co
             cut3(st[j].x, st[j].y, b0);
             cut3(st[j].z, st[j].w, b1);
 #pragma unroll
-            for (int k = 2; k >= 0; --k)
+            for (int i = 0; i < 4; ++i) {
+                float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) mma_bf16_16816(acc[i][j], ca[i], b0[k], b1[k]);
+                for (int k = 2; k >= 0; --k) mma_bf16_16816(d, ca[i], b0[k], b1[k]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[i][j][e] += d[e];
+            }
         }
     }
 #pragma unroll
@@ -803,13 +820,11 @@ __global__ void __launch_bounds__(128, 4) chunk_output_tc_kernel(const __grid_co
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             if (i < ks) continue;   // rows above these keys
+            uint32_t w[3][4];
 #pragma unroll
-            for (int k = 2; k >= 0; --k) {
-                uint32_t w[4];
-                ldmatrix_x4(w[0], w[1], w[2], w[3], &sm[k][i * 16 + (lane & 15)][ks * 16 + (lane >> 4) * 8]);
-                mma_bf16_16816(acc[i][0], w, b[0], b[1]);
-                mma_bf16_16816(acc[i][1], w, b[2], b[3]);
-            }
+            for (int k = 0; k < 3; ++k) ldmatrix_x4(w[k][0], w[k][1], w[k][2], w[k][3], &sm[k][i * 16 + (lane & 15)][ks * 16 + (lane >> 4) * 8]);
+            add_products(acc[i][0], w, b[0], b[1]);
+            add_products(acc[i][1], w, b[2], b[3]);
         }
     }
     const float skip = a.skip ? a.skip[h] : 0.f;

@@ -1,5 +1,5 @@
-"""The gated linear recurrence by itself (bf16 rows, fp32 state and output), in blocks of 64 rows on the tensor cores: infinite entries give what the
-fp32 kernels give for the same values."""
+"""The gated linear recurrence by itself (bf16 rows, fp32 state and output), in blocks of 64 rows on the tensor cores: the error of fp32
+sums against float64, and infinite entries give what the fp32 kernels give for the same values."""
 import pytest
 import torch
 
@@ -34,3 +34,33 @@ def test_infinite_entries(ctx, name, row, value):
         at = torch.isfinite(want)
         # 64 + 72 terms a sum, whatever its order: fp32 rounding of each, all terms of one sign
         assert bool(((got[at] - want[at]).abs() <= want[at].abs() * 2.0 ** -24 * 300).all())
+
+
+def _exact(t, cs):
+    """Outputs and final state token by token in float64, and the magnitudes that are summed for each."""
+    k, c, u, la, st, sc, skip = (t[n].double() for n in ("k", "c", "u", "log_decay", "state", "sc", "skip"))
+    k, c = (x.repeat_interleave(u.shape[1] // k.shape[1], 1) for x in (k, c))
+    s, sa, y, ya = st.clone(), st.abs(), [], []
+    for i in range(k.shape[0]):
+        d = (sc[i][:, None] * u[i])[:, :, None] * k[i][:, None, :]
+        s, sa = la[i].exp()[:, None, None] * s + d, la[i].exp()[:, None, None] * sa + d.abs()
+        q = (cs * c[i])[:, None, :]
+        y.append((s * q).sum(-1) + skip[:, None] * u[i])
+        ya.append((sa * q.abs()).sum(-1) + (skip[:, None] * u[i]).abs())
+    return torch.stack(y), torch.stack(ya), s, sa
+
+
+@pytest.mark.parametrize("sign,state,decay", [(True, 1.0, 0.05), (False, 1.0, 0.05), (True, 1e4, 0.05), (True, 1.0, 3.0), (False, 1.0, 0.002)])
+@pytest.mark.parametrize("S,H,G,N,P", [(200, 4, 2, 136, 72), (64, 2, 1, 64, 64), (129, 2, 2, 16, 8)])
+def test_error_of_the_sums(ctx, S, H, G, N, P, sign, state, decay):
+    """Against float64, relative to the magnitudes summed: some ten fp32 roundings (a block's sums of up to nine groups of 16 terms, decays, the state).
+    Values cut in two instead of three are 1e-5 off, running sums in the tensor cores' accumulators 2e-6. Single values may also be off by what the
+    difference of two running sums of log decays carries, each up to 64 decays and rounded at 2^-24 of that."""
+    t = _inputs(S, H, G, N, P, seed=S, sign=sign)
+    t["state"] *= state
+    t["log_decay"] *= decay / 0.05
+    y, st = _scan(ctx, t, torch.bfloat16)
+    y64, ya, s64, sa = _exact(t, 0.5)
+    for got, want, size in ((y, y64, ya), (st, s64, sa)):
+        err = (got.double() - want).abs()
+        assert float(err.norm() / size.norm()) < 8 * 2.0 ** -24 and float((err / size).max()) < (32 + 64 * decay) * 2.0 ** -24
