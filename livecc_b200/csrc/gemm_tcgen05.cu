@@ -1234,12 +1234,12 @@ static int choose_alone(int M, int N, int K, int num_sms, double* us) {
     }
     return width;
 }
-// width of a pair's tile, 0 where one CTA (estimate `alone`) is not slower by more than the estimates' error
+// width of a pair's tile, 0 where one CTA (estimate `alone`) is not slower
 static int choose_pair(int M, int N, int K, int num_sms, double alone, double* us) {
     static constexpr double per_kb[5] = {0.31, 0.31, 0.325, 0.345, 0.335};
     *us = alone;
     if (N <= 64 || num_sms < 2) return 0;
-    double best = 0.98 * alone;
+    double best = alone;
     int width = 0;
     for (int i = 0; i < 5; ++i) {
         const double t = 8.0 + tile_us(M, N, K, 2 * BLOCK_M, 128 + 32 * i, num_sms / 2, per_kb[i]);
