@@ -172,8 +172,8 @@ def run_stream_device(eng, chunks_dev, max_new, keep_cache=False):
 
 
 def run_streams_batched(eng, chunks_dev, max_new, B, n_chunks=None):
-    """B concurrent streams on ONE GPU through generate_batch: per chunk the ViT and the prefill
-    run per stream, the decode steps run batched in the persistent kernel (weights read once per step for all B)."""
+    """B concurrent streams on ONE GPU through generate_batch: per chunk the ViT runs per stream, the new tokens of all
+    streams are prefilled in one pass and every decode step is one pass of kernels per operation (weights read once for all B)."""
     caches, pasts = [None] * B, [None] * B
     n_tok = n_frames = 0
     for ch in chunks_dev[:n_chunks]:
@@ -276,8 +276,8 @@ def time_gateup_kernel(eng, iters=5):
 
 
 def time_persistent_kernel(eng, chunks_dev, max_new, iters=20):
-    """The persistent decode kernel (decode_mega_kernel; what every batched step runs): one launch = one decode step of one
-    stream (28 layers + lm_head).
+    """The persistent decode kernel (decode_mega_kernel; what decoding runs with LIVECC_B200_MEGA=1): one launch = one decode step of
+    one stream (28 layers + lm_head).
     Timed alone with CUDA events on its launch stream (the sub-range hook of the C ABI launches exactly the kernel the
     CUDA-graph step contains, without the token selection, so the stream state does not advance and every launch
     re-reads the same bytes): algorithmic bytes per launch = all decoder weights + lm_head + the stream's KV at the
@@ -647,7 +647,7 @@ def main():
                      "bytes_per_launch": kbytes,
                      "us_per_launch": ksec * 1e6},
     }
-    line["persistent_kernel"] = {"kernel": "decode_mega_kernel (one launch = 28 layers + lm_head; the batched-decode kernel), 1 stream, "
+    line["persistent_kernel"] = {"kernel": "decode_mega_kernel (one launch = 28 layers + lm_head; opt-in, LIVECC_B200_MEGA=1), 1 stream, "
                                            "kv_len %d" % pk_kv, "bytes_per_launch": pk_bytes, "us_per_launch": pk_sec * 1e6,
                                  "achieved": pk_bytes / pk_sec / 1e9, "unit": "GB/s", "frac": pk_bytes / pk_sec / 1e9 / peak,
                                  "native_error": pk_err}

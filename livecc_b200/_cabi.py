@@ -22,7 +22,7 @@ EPI_CLAMP_GLU = 10
 # stream scalar slots (LCC_SC_*)
 SC_KV_LEN, SC_ROPE_POS, SC_FINISHED, SC_N_GENERATED, SC_SEQ_LEN, SC_LAST_TOKEN, SC_VIDEO_TOKENS, SC_NATIVE_ERROR = range(8)
 SC_COUNT = 8
-MAX_BATCH = 8  # streams per persistent decode launch (MG_MAXB)
+MAX_BATCH = 8  # streams per batched prefill or decode step (MG_MAXB, kBatchStreams)
 
 
 class LiveCCNativeError(RuntimeError):

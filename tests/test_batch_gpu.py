@@ -175,3 +175,18 @@ def test_one_token_each_of_a_model_that_batched_decoding_refuses():
         assert torch.equal(t.logits[0], a.logits[0]) and torch.equal(t.sequences, a.sequences)
     with pytest.raises(LiveCCNativeError, match="batched decoding"):
         call(2)
+
+
+def test_prompts_of_several_streams_through_the_mma_attention(engines, monkeypatch):
+    """LIVECC_B200_PREFILL_ATTN=mma: the mma.sync kernel takes each stream of a joint pass by itself, with the bits of the stream alone."""
+    monkeypatch.setenv("LIVECC_B200_PREFILL_ATTN", "mma")
+    for which, spec in (("small", [(130, 3, 0), (0, 40, 2), (200, 17, 0)]), ("wide", [(2100, 40, 0), (64, 1, 0), (0, 200, 0)])):
+        eng = engines[which]
+        reqs = _requests(eng, spec, seed=8)
+        kw = [dict(input_ids=ids.to(DEV), **({"video_frames": v} if v is not None else {})) for ids, _, v in reqs]
+        alone = [eng.generate(past_key_values=c, max_new_tokens=1, output_logits=True, **k) for k, c in zip(kw, _caches(eng, reqs))]
+        together = eng.generate_batch([dict(k, past_key_values=c) for k, c in zip(kw, _caches(eng, reqs))], max_new_tokens=1, output_logits=True)
+        for a, t in zip(alone, together):
+            assert torch.equal(t.logits[0], a.logits[0]) and torch.equal(t.sequences, a.sequences)
+            a.past_key_values.release()
+            t.past_key_values.release()

@@ -232,9 +232,8 @@ def test_batched_decode_equals_sequential(which, specs, request):
 
 
 def test_persistent_kernel_vs_per_op_path(small):
-    """Same stream through the persistent kernel (`small` engines are built with LIVECC_B200_MEGA=1; every batched step
-    uses it) and through the per-op decode kernels (the one-stream default): logits within bf16 tolerance, cache lengths
-    equal."""
+    """Same stream through the persistent kernel (`small` engines are built with LIVECC_B200_MEGA=1, which runs every step of theirs
+    through it) and through the per-op decode kernels (the default): logits within bf16 tolerance, cache lengths equal."""
     from livecc_b200.engine import LiveCCB200ForConditionalGeneration
 
     cfg, sd, mega = small
