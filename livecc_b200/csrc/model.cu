@@ -430,8 +430,9 @@ static int mega_launch(lcc_model* m, const lcc::MegaParams& p, cudaStream_t s) {
 }
 
 // Per-op kernels of a batched step: every weight byte is read once for all streams (gemv_batch.cu), attention is one grid over streams, KV
-// heads and splits. A step of eight streams over 8k tokens each, four layers, takes 0.69 ms; the persistent kernel, whose grid barriers and
-// attention phase leave HBM idle half of the time, took 1.09 (two streams 0.56 for 0.63).
+// heads and splits. A step of eight streams over 8k tokens each, four layers, takes 0.68 ms; the persistent kernel, whose grid barriers and
+// attention phase leave HBM idle half of the time, took 1.09 (turns of 2, 7 and 8 streams 1.3 to 2.2 times as fast). Nothing here depends on
+// the number of streams or on a stream's place: its bits are the same in every batch.
 static int decode_batch_ops(lcc_model* m, const lcc_stream_state* sts, int B, int n_steps, const lcc_sampling* sp, const WsLayout& L, cudaStream_t s) {
     const lcc_model_config& c = m->cfg;
     uint8_t* ws = m->ws;
