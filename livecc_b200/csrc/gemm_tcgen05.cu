@@ -1249,6 +1249,16 @@ static int choose_pair(int M, int N, int K, int num_sms, double alone, double* u
     return width;
 }
 
+// estimates: the swapped form (waves of tiles of bm rows, nkb k-blocks a share), and K split through the scratch (two launches, the partials written and read once)
+static double swap_us(int bm, int waves, int nkb, int splits) {
+    return 6.5 + waves * nkb * std::max(0.42, bm / 700.0) + 0.5 * bm / 64 + (splits > 1 ? 2.5 + 0.8 * bm / 64 : 0.0);
+}
+static int splitk_width(const GemmArgs& a) { return a.block_n ? a.block_n : (a.N >= 256 ? 256 : (a.N >= 128 ? 128 : 64)); }
+static double scratch_us(const GemmArgs& a, int ranges, int num_sms) {
+    const int w = splitk_width(a), tiles = (a.M + BLOCK_M - 1) / BLOCK_M * ((a.N + w - 1) / w), nkb = (a.K + BLOCK_K - 1) / BLOCK_K;
+    return 14.0 + (tiles * ranges + num_sms - 1) / num_sms * ((nkb + ranges - 1) / ranges) * 0.41 + (double)a.M * a.N * ranges * 4 / 6.5e6;
+}
+
 // Few rows: is the swapped kernel the better one? `other`: the estimate of the best other form (0: none, narrow products). One wave of
 // clusters of 2 s CTAs (two waves where all rows are one tile), max(0.42, rows / 700) us per k-block of a pair's share, 6.5 us for the launch,
 // 2.5 and 0.8 per 64 rows for the exchange of a split, 0.5 per 64 rows for the store. Measured (us, best of the other forms | this, back to back):
@@ -1274,7 +1284,7 @@ static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_
             if (waves > (sp == 1 && m_tiles == 1 ? 2 : 1) || nkb < 4 * sp) continue;
             const SwapTile t = make_swap(bm, sp);
             if (sp > 1 && bm * BLOCK_M * 4 > t.stages * t.stage_bytes) continue;
-            const double us = 6.5 + waves * ((nkb + sp - 1) / sp) * std::max(0.42, bm / 700.0) + 0.5 * bm / 64 + (sp > 1 ? 2.5 + 0.8 * bm / 64 : 0.0);
+            const double us = swap_us(bm, waves, (nkb + sp - 1) / sp, sp);
             if (us < best) { best = us; *bm_out = bm; *splits_out = sp; found = true; }
         }
     }
@@ -1326,8 +1336,6 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits,
     o.w = pack_bf16x2(x[6], x[7]);
     *reinterpret_cast<uint4*>(C + (size_t)row * ldc + col) = o;
 }
-
-static int splitk_width(const GemmArgs& a) { return a.block_n ? a.block_n : (a.N >= 256 ? 256 : (a.N >= 128 ? 128 : 64)); }
 
 // Split-K for small-M GEMMs whose tile count cannot occupy the SMs (prefill down_proj at M ~ 281: 84 tiles on 148 SMs).
 // Bit-exact on integer operands (test_gemm_splitk_exact_integer_operands), whole-model parity with it forced on. Measured on B200: it pays only for long K — down_proj (K = 18944) 86.7 -> 60.9 us,
@@ -1382,9 +1390,8 @@ GemmPlan gemm_plan(const GemmArgs& a, int num_sms) {
     const int width = choose_pair(a.M, a.N, a.K, num_sms, us, &us);
     if (width) p.width = width;
     if (width) p.form = FORM_PAIR;
-    if (const int ranges = splitk_ranges(a, num_sms)) {   // two launches, the partials written and read once
-        const int w = splitk_width(a), tiles = (a.M + BLOCK_M - 1) / BLOCK_M * ((a.N + w - 1) / w), nkb = (a.K + BLOCK_K - 1) / BLOCK_K;
-        us = 14.0 + (tiles * ranges + num_sms - 1) / num_sms * ((nkb + ranges - 1) / ranges) * 0.41 + (double)a.M * a.N * ranges * 4 / 6.5e6;
+    if (const int ranges = splitk_ranges(a, num_sms)) {
+        us = scratch_us(a, ranges, num_sms);
         p.form = FORM_ONE;
     }
     int bm = 0, splits = 0;
@@ -1440,14 +1447,23 @@ int gemm_bf16_tn_order(const GemmArgs& a, const SumOrder& order, int num_sms, cu
         const int alone = choose_alone(a.M, a.N, a.K, num_sms, &us), pair = choose_pair(a.M, a.N, a.K, num_sms, us, &us);
         return pair ? launch_epi2(a, pair, num_sms, stream) : launch_epi(a, alone, num_sms, stream);
     }
-    // as many rows at a time as the scratch, or one wave of clusters, holds
-    int rows, bm = kSwapMax, m_tiles = 1;
-    if (order.scratch) rows = (int)std::min<size_t>(a.splitk_ws_bytes / ((size_t)order.ranges * a.N * 4), 1 << 20) / BLOCK_M * BLOCK_M;
-    else {
+    // as many rows at a time as the scratch, or one wave of clusters, holds. Ranges of equal length may go either way with the same bits (ascending sums
+    // of the same parts, the same roundings behind them); rows that take several waves of clusters are faster through the scratch: two
+    // sequences of 281 rows, x 3584 x 3584 and x 3584 x 18944 together 146 us by clusters, 104 by the scratch.
+    const int nkb = (a.K + BLOCK_K - 1) / BLOCK_K, n_tiles = (a.N + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
+    const bool can_scratch = order.scratch || (a.splitk_ws && nkb % order.ranges == 0 && (a.epi == EPI_NONE || a.epi == EPI_BIAS || a.epi == EPI_RESIDUAL || a.epi == EPI_BIAS_RESIDUAL));
+    const int scratch_rows = can_scratch ? (int)std::min<size_t>(a.splitk_ws_bytes / ((size_t)order.ranges * a.N * 4), 1 << 20) / BLOCK_M * BLOCK_M : 0;
+    bool scratch = order.scratch;
+    int rows = scratch_rows, bm = kSwapMax;
+    if (!scratch) {
         auto fits = [&](int h) { const SwapTile t = make_swap(h, order.ranges); return h * BLOCK_M * 4 <= t.stages * t.stage_bytes; };
         while (bm > 32 && !fits(bm)) bm -= 32;
-        m_tiles = max_clusters(current_device(), order.ranges, num_sms) / ((a.N + 2 * BLOCK_M - 1) / (2 * BLOCK_M));
-        rows = m_tiles * bm;
+        rows = max_clusters(current_device(), order.ranges, num_sms) / n_tiles * bm;
+        if (rows > 0 && scratch_rows > 0) {
+            const int launches = (a.M + rows - 1) / rows, h = std::min(bm, (std::min(rows, a.M) + 31) / 32 * 32);
+            const double clusters_us = launches * swap_us(h, 1, (nkb + order.ranges - 1) / order.ranges, order.ranges);
+            if (a.M > rows && scratch_us(a, order.ranges, num_sms) < clusters_us) { scratch = true; rows = scratch_rows; }
+        }
     }
     if (rows < 1) return -15;
     for (int m0 = 0; m0 < a.M; m0 += rows) {
@@ -1457,8 +1473,8 @@ int gemm_bf16_tn_order(const GemmArgs& a, const SumOrder& order, int num_sms, cu
         p.C = (bf16*)a.C + (size_t)m0 * a.ldc;
         if (a.residual) p.residual = (const bf16*)a.residual + (size_t)m0 * a.ldr;
         const int tiles = (p.M + bm - 1) / bm;
-        if (int r = order.scratch ? run_splitk(p, order.ranges, num_sms, stream)
-                                  : launch_epi_swap(p, ((p.M + tiles - 1) / tiles + 31) / 32 * 32, order.ranges, num_sms, stream))
+        if (int r = scratch ? run_splitk(p, order.ranges, num_sms, stream)
+                            : launch_epi_swap(p, ((p.M + tiles - 1) / tiles + 31) / 32 * 32, order.ranges, num_sms, stream))
             return r;
     }
     return 0;
