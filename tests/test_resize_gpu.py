@@ -120,3 +120,21 @@ def test_plan_rejects_windows_larger_than_shared_memory(ctx):
     with pytest.raises(_cabi.LiveCCNativeError):  # output width 1 with a height change: outside the oracle's domain
         ctx.resize_plan(60, 20, 30, 1)
     ctx.resize_plan(60, 20, 60, 1)  # width only: fine
+
+
+@pytest.mark.parametrize("h,w,H,W", [(40, 52, 60, 84), (61, 157, 28, 70), (64, 160, 33, 66), (120, 400, 30, 100), (97, 401, 30, 97), (90, 550, 28, 100),
+                                     (300, 520, 20, 40), (301, 523, 21, 37), (47, 8, 31, 9), (5, 3, 40, 24)])
+def test_every_form_of_the_width_products(ctx, h, w, H, W):
+    """1 to 4 k-steps and more per window, rows on and off word boundaries, planes that leave a tile ragged; noise (few pixels need the stated order),
+    a checkerboard (half and even sizes: every tile is summed again) and steps of full height (clamped values)."""
+    from oracle import resize_aa
+
+    g = torch.Generator().manual_seed(h * w)
+    noise = torch.randint(0, 256, (3, 1, h, w), generator=g, dtype=torch.uint8)
+    check = ((torch.arange(h)[:, None] + torch.arange(w)[None]) % 2 * 255).to(torch.uint8).expand(2, 1, h, w)
+    steps = ((torch.arange(w) // 7 % 2) * 255).to(torch.uint8).expand(1, 1, h, w)
+    clip = torch.cat([noise, check, steps]).contiguous()
+    want = torch.from_numpy(resize_aa.resize_bicubic_aa_u8(clip.numpy(), (H, W)))
+    assert torch.equal(ctx.resize_bicubic_aa_u8(clip.cuda(), (H, W)).cpu(), want)
+    half = torch.from_numpy(resize_aa.resize_bicubic_aa_u8(check.contiguous().numpy(), (max(h // 2, 2), max(w // 2, 2))))
+    assert torch.equal(ctx.resize_bicubic_aa_u8(check.contiguous().cuda(), (max(h // 2, 2), max(w // 2, 2))).cpu(), half)
