@@ -533,6 +533,25 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
         pend_is_mc = false;
         return rc;
     };
+    // Entries of one token whose layer's recurrence is of a size that one kernel does with all that surrounds it (an entry's bits do not depend on its
+    // neighbours). The rows of the others, in runs: what row kernels are launched over.
+    std::vector<uint8_t> alone(n_entries);
+    auto mark_alone = [&](int li, auto step_of) {
+        int r = 0;
+        for (int e = 0; e < n_entries; r += entries[e++].n_new)
+            alone[e] = entries[e].n_new == 1 && entries[e].layer_state[li] && lcc::scan_step_takes(step_of(entries[e], r));
+    };
+    auto other_rows = [&](auto launch) {      // launch(first row, rows)
+        int r = 0, from = 0;
+        for (int e = 0; e < n_entries; ++e) {
+            if (alone[e]) {
+                if (r > from) { const int rc = launch(from, r - from); if (rc) return rc; }
+                from = r + 1;
+            }
+            r += entries[e].n_new;
+        }
+        return r > from ? launch(from, r - from) : 0;
+    };
     auto pos_of = [&](const lcc_seq_entry& e) {
         lcc::SeqPos p{e.past, nullptr, nullptr};
         if (e.scalars) { p.kv_len = e.scalars + LCC_SC_KV_LEN; p.finished = e.scalars + LCC_SC_FINISHED; }
@@ -733,11 +752,29 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
         } else if (l.type == LCC_MIX_SSD) {
             const int ldp = ld8(z.s_proj), ldm = ld8(z.conv_ch), GN = l.s_groups * l.s_state;
             STEP(linear(m, xa, W, l.s_in, nullptr, proj, ldp, false, T, z.s_proj, W, s), "state-space in-proj");
-            STEP(lcc::ssm_step_decay(dt, proj + (size_t)(z.inner + z.conv_ch) * es, ldp, l.s_dt_bias_f32, l.s_a_log_f32, f1, f2, T,
-                                     l.s_heads, s), "step sizes");
+            const int ldi = ld8(z.inner);
+            auto step_of = [&](const lcc_seq_entry& en, int r) {
+                lcc::ScanStep a{};
+                const uint8_t* pr = proj + (size_t)r * ldp * es;
+                float* st = en.layer_state[li] + st_off;
+                a.dt = dt; a.u = pr + (size_t)z.inner * es; a.dec = pr + (size_t)(z.inner + z.conv_ch) * es;
+                a.conv_w = l.s_conv_w_f32; a.conv_b = l.s_conv_b_f32; a.carry = st; a.taps = l.s_conv;
+                a.dt_bias = l.s_dt_bias_f32; a.a_log = l.s_a_log_f32; a.skip = l.s_skip_f32; a.cs = 1.f;
+                a.state = st + (size_t)z.conv_ch * (l.s_conv - 1);
+                a.gate = pr; a.norm_w = l.s_norm_f32; a.w_len = z.inner; a.out = mid2 + (size_t)r * ldi * es;
+                a.group = z.inner / l.s_norm_groups; a.gate_first = 1; a.eps = d.eps;
+                a.heads = l.s_heads; a.heads_per_group = l.s_heads / l.s_groups; a.N = l.s_state; a.P = l.s_vdim;
+                return a;
+            };
+            mark_alone(li, step_of);
+            STEP(other_rows([&](int r, int n) {
+                return lcc::ssm_step_decay(dt, proj + ((size_t)r * ldp + z.inner + z.conv_ch) * es, ldp, l.s_dt_bias_f32, l.s_a_log_f32, f1 + (size_t)r * l.s_heads,
+                                           f2 + (size_t)r * l.s_heads, n, l.s_heads, s);
+            }), "step sizes");
             int r0 = 0;
             for (int e = 0; e < n_entries; ++e) {
                 const lcc_seq_entry& en = entries[e];
+                if (alone[e]) { STEP(lcc::scan_step(step_of(en, r0++), pos_of(en), s), "state-space step"); continue; }
                 float* st = en.layer_state[li];
                 if (!st) LCC_FAIL(m->ctx, -2, "lcc_seq_forward: entry %d has no state for layer %d", e, li);
                 st += st_off;
@@ -761,9 +798,10 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
                 STEP(lcc::gated_scan(a, pos, s), "state-space recurrence");
                 r0 += en.n_new;
             }
-            const int ldi = ld8(z.inner);
-            STEP(lcc::gated_group_norm(dt, y32, z.inner, proj, ldp, l.s_norm_f32, z.inner, mid2, ldi, T, z.inner,
-                                       z.inner / l.s_norm_groups, 1, d.eps, s), "gated norm");
+            STEP(other_rows([&](int r, int n) {
+                return lcc::gated_group_norm(dt, y32 + (size_t)r * z.inner, z.inner, proj + (size_t)r * ldp * es, ldp, l.s_norm_f32, z.inner,
+                                             mid2 + (size_t)r * ldi * es, ldi, n, z.inner, z.inner / l.s_norm_groups, 1, d.eps, s);
+            }), "gated norm");
             STEP(linear(m, mid2, ldi, l.s_out, nullptr, o1, W, false, T, W, z.inner, s), "state-space out-proj");
         } else {
             // left: chunk-local attention with a sink
@@ -791,10 +829,23 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
             const int ldr = ld8(z.r_proj), ldz = ld8(z.r_nk), ldv = ld8(z.r_nv);
             STEP(linear(m, xa, W, l.r_in, nullptr, proj, ldr, false, T, z.r_proj, W, s), "linear-attention in-proj");
             STEP(linear(m, proj + (size_t)(2 * z.r_nk + 2 * z.r_nv) * es, ldr, l.r_decay_up, l.r_decay_bias_f32, proj2, ldz, false, T, z.r_nk, l.r_rank, s), "decay projection");
-            STEP(lcc::gla_decay(dt, proj2, ldz, nullptr, l.r_tau, f1, T, z.r_nk, s), "decays");
+            auto step_of = [&](const lcc_seq_entry& en, int r) {
+                lcc::ScanStep a{};
+                const uint8_t* pr = proj + (size_t)r * ldr * es;
+                a.dt = dt; a.c = pr; a.k = pr + (size_t)z.r_nk * es; a.u = pr + (size_t)(2 * z.r_nk) * es; a.dec = proj2 + (size_t)r * ldz * es;
+                a.inv_tau = 1.f / l.r_tau; a.cs = 1.f / sqrtf((float)l.r_dim);
+                a.state = en.layer_state[li];
+                a.gate = pr + (size_t)(2 * z.r_nk + z.r_nv) * es; a.norm_w = l.r_norm_f32; a.w_len = l.r_vdim; a.out = mid2 + (size_t)r * ldv * es;
+                a.group = l.r_vdim; a.gate_first = 0; a.eps = d.eps;
+                a.heads = l.r_heads; a.heads_per_group = 1; a.N = l.r_dim; a.P = l.r_vdim;
+                return a;
+            };
+            mark_alone(li, step_of);
+            STEP(other_rows([&](int r, int n) { return lcc::gla_decay(dt, proj2 + (size_t)r * ldz * es, ldz, nullptr, l.r_tau, f1 + (size_t)r * z.r_nk, n, z.r_nk, s); }), "decays");
             r0 = 0;
             for (int e = 0; e < n_entries; ++e) {
                 const lcc_seq_entry& en = entries[e];
+                if (alone[e]) { STEP(lcc::scan_step(step_of(en, r0++), pos_of(en), s), "linear-attention step"); continue; }
                 float* st = en.layer_state[li];
                 if (!st) LCC_FAIL(m->ctx, -2, "lcc_seq_forward: entry %d has no state for layer %d", e, li);
                 uint8_t* pr = proj + (size_t)r0 * ldr * es;
@@ -812,8 +863,10 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
                 STEP(lcc::gated_scan(a, pos_of(en), s), "linear-attention recurrence");
                 r0 += en.n_new;
             }
-            STEP(lcc::gated_group_norm(dt, y32, z.r_nv, proj + (size_t)(2 * z.r_nk + z.r_nv) * es, ldr, l.r_norm_f32, l.r_vdim, mid2, ldv, T,
-                                       z.r_nv, l.r_vdim, 0, d.eps, s), "head norm + gate");
+            STEP(other_rows([&](int r, int n) {
+                return lcc::gated_group_norm(dt, y32 + (size_t)r * z.r_nv, z.r_nv, proj + ((size_t)r * ldr + 2 * z.r_nk + z.r_nv) * es, ldr, l.r_norm_f32, l.r_vdim,
+                                             mid2 + (size_t)r * ldv * es, ldv, n, z.r_nv, l.r_vdim, 0, d.eps, s);
+            }), "head norm + gate");
             STEP(linear(m, mid2, ldv, l.r_out, nullptr, o2, W, false, T, W, z.r_nv, s), "linear-attention out-proj");
             STEP(lcc::postnorm_residual(dt, x32, xa, o1, W, l.l_branch_norm_f32, o2, W, l.r_branch_norm_f32, l.norm1_f32, d.alpha, d.eps,
                                         T, W, s), "branch merge + norm1");

@@ -162,6 +162,23 @@ int gated_scan_chunked(const ScanArgs& a, SeqPos pos, cudaStream_t s);
 // fp32 elements of workspace that let a call of S rows run in the fewest passes
 size_t gated_scan_ws_floats(int S, int heads, int N, int P);
 
+// ---- recurrent_step.cu --------------------------------------------------------------------------------------------------
+// One token of a gated linear recurrence with its convolution, step size, decays, gate and group norm in one kernel, where scan_step_takes the sizes.
+// All rows in the storage type dt. conv_w set: u points to the convolution's inputs [heads*P values | groups*N keys | groups*N read-outs], dec to
+// the step-size logits [heads]; else u, k, c are the recurrence's own rows and dec the decay logits [heads*N]. out[c] as gated_group_norm gives it.
+struct ScanStep {
+    int dt;
+    const void *u, *k, *c, *dec;
+    const float *conv_w, *conv_b; float* carry; int taps;
+    const float *dt_bias, *a_log, *skip;
+    float inv_tau, cs;
+    float* state;                       // [heads, P, N] (n fastest)
+    const void* gate; const float* norm_w; int w_len; void* out; int group, gate_first; float eps;
+    int heads, heads_per_group, N, P;
+};
+bool scan_step_takes(const ScanStep& a);
+int scan_step(const ScanStep& a, SeqPos pos, cudaStream_t s);
+
 // ---- attn_local.cu ------------------------------------------------------------------------------------------------------
 // RMS norm of the whole q projection and of the whole k projection of each row (weights qn_w [Hq*D], kn_w [G*D], fp32),
 // then: normalised q -> q_out fp32 [S, Hq*D]; normalised k and raw v -> the paged cache at positions past..past+S-1.
