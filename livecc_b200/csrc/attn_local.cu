@@ -163,8 +163,21 @@ __global__ void __launch_bounds__(256) qk_headnorm_rope_append_kernel(const T* _
     }
 }
 
-// One CTA per new row.
-template <typename T>
+// Four neighbouring elements of a row
+template <typename T> __device__ __forceinline__ void row4(const T* p, float (&v)[4]);
+template <> __device__ __forceinline__ void row4<float>(const float* p, float (&v)[4]) {
+    const float4 u = *reinterpret_cast<const float4*>(p);
+    v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+}
+template <> __device__ __forceinline__ void row4<bf16>(const bf16* p, float (&v)[4]) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+
+// One CTA per new row. EQ > 0: rows on 4-element boundaries with at most EQ * 256 pieces of four query columns and 256 of key columns; everything
+// the row needs is loaded at once and stays in registers. (One row of 16 + 2 heads of 128: 6.2 us in place of a step's chain element by element, 2.3 so.)
+template <typename T, int EQ>
 __global__ void __launch_bounds__(256) qk_norm_kv_append_kernel(const T* __restrict__ proj, int ld, const float* __restrict__ qn_w,
                                                                 const float* __restrict__ kn_w, float eps, float* __restrict__ q_out,
                                                                 T* __restrict__ k_pages, T* __restrict__ v_pages,
@@ -172,11 +185,55 @@ __global__ void __launch_bounds__(256) qk_norm_kv_append_kernel(const T* __restr
                                                                 int G, int D, int DV, SeqPos pos) {
     chain_begin(proj, page_table);
     if (seq_done(pos)) return;
-    __shared__ float red[32];
+    __shared__ float red[64];
     const int t = blockIdx.x;
-    const int p = seq_past(pos, S) + t;
     const T* row = proj + (size_t)t * ld;
     const int nq = Hq * D, nk = G * D, nv = G * DV;
+    if (EQ > 0) {
+        constexpr int EN = EQ > 0 ? EQ : 1;
+        float vq[EN][4], wq[EN][4], vk[4] = {}, wk[4] = {}, sq = 0.f, sk = 0.f;
+        const int ik = threadIdx.x * 4;
+#pragma unroll
+        for (int e = 0; e < EN; ++e) {
+            const int i = (threadIdx.x + e * 256) * 4;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) vq[e][u] = wq[e][u] = 0.f;
+            if (i < nq) { row4(row + i, vq[e]); row4(qn_w + i, wq[e]); }
+        }
+        if (ik < nk) { row4(row + nq + ik, vk); row4(kn_w + ik, wk); }
+        const int p = seq_past(pos, S) + t, page = page_table[p / page_size], slot = p % page_size;
+        for (int i = threadIdx.x; i < nv; i += 256) {
+            const int g = i / DV, d = i % DV;
+            v_pages[(((size_t)page * G + g) * page_size + slot) * DV + d] = row[nq + nk + i];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+#pragma unroll
+            for (int e = 0; e < EN; ++e) sq = fmaf(vq[e][u], vq[e][u], sq);
+            sk = fmaf(vk[u], vk[u], sk);
+        }
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        sq = warp_sum(sq);
+        sk = warp_sum(sk);
+        if (lane == 0) { red[warp] = sq; red[32 + warp] = sk; }
+        __syncthreads();
+        sq = warp_sum(lane < 8 ? red[lane] : 0.f);
+        sk = warp_sum(lane < 8 ? red[32 + lane] : 0.f);
+        const float rq = 1.f / sqrtf(sq / (float)nq + eps), rk = 1.f / sqrtf(sk / (float)nk + eps);
+#pragma unroll
+        for (int e = 0; e < EN; ++e) {
+            const int i = (threadIdx.x + e * 256) * 4;
+            if (i < nq) *reinterpret_cast<float4*>(q_out + (size_t)t * nq + i) =
+                make_float4(vq[e][0] * rq * wq[e][0], vq[e][1] * rq * wq[e][1], vq[e][2] * rq * wq[e][2], vq[e][3] * rq * wq[e][3]);
+        }
+        if (ik < nk) {
+            T* k = k_pages + (((size_t)page * G + ik / D) * page_size + slot) * D + ik % D;    // (D is a multiple of 4: the piece lies in one head)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) stf(k + u, vk[u] * rk * wk[u]);
+        }
+        return;
+    }
+    const int p = seq_past(pos, S) + t;
     float sq = 0.f, sk = 0.f;
     for (int i = threadIdx.x; i < nq; i += blockDim.x) { const float v = ldf(row + i); sq = fmaf(v, v, sq); }
     for (int i = threadIdx.x; i < nk; i += blockDim.x) { const float v = ldf(row + nq + i); sk = fmaf(v, v, sk); }
@@ -1375,12 +1432,22 @@ int qk_norm_kv_append(int dt, const void* proj, int ld, const float* qn_w, const
         DV < 1 || page_size < 1)
         return -2;
     count_launch();
-    if (dt == DT_F32)
-        chained(qk_norm_kv_append_kernel<float>, S, 256, 0, s)((const float*)proj, ld, qn_w, kn_w, eps, q_out, (float*)k_pages,
-                                                          (float*)v_pages, page_table, page_size, S, Hq, G, D, DV, pos);
-    else
-        chained(qk_norm_kv_append_kernel<bf16>, S, 256, 0, s)((const bf16*)proj, ld, qn_w, kn_w, eps, q_out, (bf16*)k_pages,
-                                                         (bf16*)v_pages, page_table, page_size, S, Hq, G, D, DV, pos);
+    const int nq = Hq * D, nk = G * D;
+    const bool vec = (ld % 4) == 0 && (D % 4) == 0 && ((uintptr_t)proj % (dt == DT_F32 ? 16 : 8)) == 0 &&
+                     (((uintptr_t)qn_w | (uintptr_t)kn_w | (uintptr_t)q_out) % 16) == 0 && nk <= 1024;
+#define LCC_QKN(E)                                                                                                                        \
+    do {                                                                                                                                  \
+        if (dt == DT_F32)                                                                                                                 \
+            chained(qk_norm_kv_append_kernel<float, E>, S, 256, 0, s)((const float*)proj, ld, qn_w, kn_w, eps, q_out, (float*)k_pages,    \
+                                                                      (float*)v_pages, page_table, page_size, S, Hq, G, D, DV, pos);      \
+        else                                                                                                                              \
+            chained(qk_norm_kv_append_kernel<bf16, E>, S, 256, 0, s)((const bf16*)proj, ld, qn_w, kn_w, eps, q_out, (bf16*)k_pages,       \
+                                                                     (bf16*)v_pages, page_table, page_size, S, Hq, G, D, DV, pos);        \
+    } while (0)
+    if (vec && nq <= 2048) LCC_QKN(2);
+    else if (vec && nq <= 4096) LCC_QKN(4);
+    else LCC_QKN(0);
+#undef LCC_QKN
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 

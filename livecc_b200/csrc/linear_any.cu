@@ -34,6 +34,8 @@ struct Grp {
     const void* gate = nullptr;     // the store multiplies by sigmoid(gate[row, z * gate_stride + column]) (no lists)
     int ld_gate = 0;
     int64_t gate_stride = 0;
+    float cap = 0.f, inv_cap = 0.f, scale = 0.f;   // scale != 0 (logits, few-row kernel): the store holds cap * tanh(v / cap) * scale (no cap: v * scale)
+    float* copy = nullptr;                         // ... and a second time here, rows as in C
 };
 template <typename T>
 __device__ __forceinline__ float gated(float v, const Grp& g, int z, int row, int col) {
@@ -109,7 +111,7 @@ __global__ void __launch_bounds__(256) linear_tile_kernel(const T* __restrict__ 
 // accumulators and addresses for eight rows a one-row step had the registers for four loads per weight row only: 32 tokens of four
 // recurrent layers of width 2048 took 10.93 ms and take 8.68 ms, of two routed layers 6.34 and 5.06 ms.
 // Scalar loads when K or a row start is not 16-byte aligned.
-constexpr int kRowsMax = 8;
+constexpr int kRowsMax = kLogitRows;
 template <typename T> struct Vec16;
 template <> struct Vec16<bf16> {
     static constexpr int N = 8;
@@ -241,7 +243,16 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
         for (int m = 0; m < MM; ++m) {
             if (m < M) {
                 const float v = warp_sum(acc[r][m]);
-                if (lane == 0 && n < N) stf(C + (size_t)m * ldc + n, gated<T>(act_of(v + (bias ? bias[n] : 0.f), g.act), g, z, mb + m, n));
+                if (lane != 0 || n >= N) continue;
+                if constexpr (std::is_same<TC, float>::value) {
+                    if (g.scale != 0.f) {
+                        const float lg = (g.cap > 0.f ? g.cap * tanhf(v * g.inv_cap) : v) * g.scale;
+                        C[(size_t)m * ldc + n] = lg;
+                        if (g.copy) g.copy[(size_t)(mb + m) * ldc + n] = lg;
+                        continue;
+                    }
+                }
+                stf(C + (size_t)m * ldc + n, gated<T>(act_of(v + (bias ? bias[n] : 0.f), g.act), g, z, mb + m, n));
             }
         }
     }
@@ -323,6 +334,15 @@ int linear_any(int dt, const void* A, int lda, const void* W, int ldw, const flo
     if (dt == DT_F32) return launch_linear<float, float>(A, lda, W, ldw, bias, C, ldc, M, N, K, s);
     if (c_f32) return launch_linear<bf16, float>(A, lda, W, ldw, bias, C, ldc, M, N, K, s);
     return launch_linear<bf16, bf16>(A, lda, W, ldw, bias, C, ldc, M, N, K, s);
+}
+
+int linear_logits(int dt, const void* A, int lda, const void* W, int ldw, float* C, float* copy, int ldc, int M, int N, int K, float cap, float scale,
+                  cudaStream_t s) {
+    if (!A || !W || !C || M < 1 || M > kRowsMax || N < 1 || K < 1 || lda < K || ldw < K || ldc < N || scale == 0.f) return -2;
+    Grp g{0, 0, 0, nullptr, nullptr, ACT_NONE, 0, 0, 0, 0.f};
+    g.cap = cap > 0.f ? cap : 0.f; g.inv_cap = cap > 0.f ? 1.f / cap : 0.f; g.scale = scale; g.copy = copy;
+    if (dt == DT_F32) return launch_linear<float, float>(A, lda, W, ldw, nullptr, C, ldc, M, N, K, s, 1, g);
+    return launch_linear<bf16, float>(A, lda, W, ldw, nullptr, C, ldc, M, N, K, s, 1, g);
 }
 
 int linear_grouped(const GroupedLinear& q, cudaStream_t s) {

@@ -2,6 +2,8 @@
 // `out` copies in the model's storage type feed the next linear layer.
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "launch.h"
 #include "seqmix.h"
@@ -52,7 +54,7 @@ __global__ void embed_sinusoid_kernel(const int64_t* __restrict__ ids, const int
     const int64_t id = seq_len ? ids[*seq_len - S + r] : ids[r];
     const float p = (float)(seq_past(pos, S) + r);
     const bool ok = id >= 0 && id < vocab;
-    for (int c = threadIdx.x; c < W; c += blockDim.x) {
+    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < W; c += blockDim.x * gridDim.y) {
         float pe = 0.f;
         if (inv_freq) {
             const float ang = p * inv_freq[c >> 1];
@@ -64,83 +66,102 @@ __global__ void embed_sinusoid_kernel(const int64_t* __restrict__ ids, const int
     }
 }
 
-// Two normed branches, averaged, behind a post-norm residual: one CTA per row. Rows of up to 256 * kRowCache elements are read once
-// into registers (E per thread, every load in flight together); wider rows (E = 0) are re-read from L1/L2 in each of the three passes. Every form adds in the same order.
+// Two sums over the CTA behind one pair of barriers (red: 64 floats)
+__device__ __forceinline__ float2 block_sum2(float a, float b, float* red) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
+    a = warp_sum(a);
+    b = warp_sum(b);
+    __syncthreads();
+    if (lane == 0) { red[warp] = a; red[32 + warp] = b; }
+    __syncthreads();
+    a = lane < warps ? red[lane] : 0.f;
+    b = lane < warps ? red[32 + lane] : 0.f;
+    return make_float2(warp_sum(a), warp_sum(b));
+}
+
+// Two normed branches, averaged, behind a post-norm residual: one CTA per row. Rows of up to 256 * kRowCache pieces are read once
+// into registers (E pieces of V columns per thread, every load in flight together, the norms' weights too: behind a sum they would wait once more);
+// wider rows (E = 0) are re-read from L1/L2 in each of the three passes. One row of 2048 columns: 5.7 us in place of a step's chain with single
+// columns, weights loaded where they are used and a sum for each branch; 3.7 here.
 constexpr int kRowCache = 16;
-template <typename T, int E>
+template <typename T, int E, bool VEC>
 __global__ void __launch_bounds__(256) postnorm_residual_kernel(float* __restrict__ x32, T* __restrict__ xa, const T* __restrict__ a,
                                                                 int ld_a, const float* __restrict__ wa, const T* __restrict__ b,
                                                                 int ld_b, const float* __restrict__ wb, const float* __restrict__ w,
                                                                 float alpha, float eps, int W) {
     chain_begin(x32, a, b);
-    __shared__ float red[32];
+    __shared__ float red[64];
     const int r = blockIdx.x;
     float* x = x32 + (size_t)r * W;
     const T* ar = a + (size_t)r * ld_a;
     const T* br = b + (size_t)r * ld_b;
-    constexpr bool CACHE = E > 0;
-    constexpr int EN = E > 0 ? E : 1;
-    float va[EN], vb[EN], vx[EN];
-    if (CACHE) {
+    T* o = xa + (size_t)r * W;
+    constexpr int V = VEC ? 4 : 1, EN = E > 0 ? E : 1;
+    if (E > 0) {
+        float va[EN][V], vb[EN][V], vx[EN][V], ka[EN][V], kb[EN][V], kw[EN][V], sa = 0.f, sb = 0.f;
 #pragma unroll
         for (int i = 0; i < EN; ++i) {
-            const int c = threadIdx.x + i * 256;
-            va[i] = c < W ? ldf(ar + c) : 0.f;
-            vb[i] = c < W ? ldf(br + c) : 0.f;
-            vx[i] = c < W ? x[c] : 0.f;
+            const int c = (threadIdx.x + i * 256) * V;
+            if (c < W) {
+                if (VEC) {
+                    ld4(ar + c, (float(&)[4])va[i]); ld4(br + c, (float(&)[4])vb[i]); ld4(x + c, (float(&)[4])vx[i]);
+                    ld4(wa + c, (float(&)[4])ka[i]); ld4(wb + c, (float(&)[4])kb[i]); ld4(w + c, (float(&)[4])kw[i]);
+                } else {
+                    va[i][0] = ldf(ar + c); vb[i][0] = ldf(br + c); vx[i][0] = x[c];
+                    ka[i][0] = wa[c]; kb[i][0] = wb[c]; kw[i][0] = w[c];
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < V; ++u) va[i][u] = vb[i][u] = vx[i][u] = ka[i][u] = kb[i][u] = kw[i][u] = 0.f;
+            }
         }
+#pragma unroll
+        for (int i = 0; i < EN; ++i)
+#pragma unroll
+            for (int u = 0; u < V; ++u) { sa = fmaf(va[i][u], va[i][u], sa); sb = fmaf(vb[i][u], vb[i][u], sb); }
+        const float2 s = block_sum2(sa, sb, red);
+        const float ra = 1.f / sqrtf(s.x / (float)W + eps), rb = 1.f / sqrtf(s.y / (float)W + eps);
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < EN; ++i)
+#pragma unroll
+            for (int u = 0; u < V; ++u) {
+                const float m = 0.5f * (va[i][u] * ra * ka[i][u] + vb[i][u] * rb * kb[i][u]);
+                vx[i][u] = fmaf(alpha, vx[i][u], m);
+                ss = fmaf(vx[i][u], vx[i][u], ss);
+            }
+        const float rn = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
+#pragma unroll
+        for (int i = 0; i < EN; ++i) {
+            const int c = (threadIdx.x + i * 256) * V;
+            if (c >= W) continue;
+#pragma unroll
+            for (int u = 0; u < V; ++u) vx[i][u] = vx[i][u] * rn * kw[i][u];
+            if (VEC) { st4(x + c, (const float(&)[4])vx[i]); st4(o + c, (const float(&)[4])vx[i]); }
+            else { x[c] = vx[i][0]; stf(o + c, vx[i][0]); }
+        }
+        return;
     }
     float sa = 0.f, sb = 0.f;
-    if (CACHE) {
-#pragma unroll
-        for (int i = 0; i < EN; ++i) { sa = fmaf(va[i], va[i], sa); sb = fmaf(vb[i], vb[i], sb); }
-    } else {
-        for (int c = threadIdx.x; c < W; c += blockDim.x) {
-            const float ta = ldf(ar + c), tb = ldf(br + c);
-            sa = fmaf(ta, ta, sa);
-            sb = fmaf(tb, tb, sb);
-        }
+    for (int c = threadIdx.x; c < W; c += blockDim.x) {
+        const float ta = ldf(ar + c), tb = ldf(br + c);
+        sa = fmaf(ta, ta, sa);
+        sb = fmaf(tb, tb, sb);
     }
-    sa = block_sum(sa, red);
-    sb = block_sum(sb, red);
-    const float ra = 1.f / sqrtf(sa / (float)W + eps), rb = 1.f / sqrtf(sb / (float)W + eps);
+    const float2 s = block_sum2(sa, sb, red);
+    const float ra = 1.f / sqrtf(s.x / (float)W + eps), rb = 1.f / sqrtf(s.y / (float)W + eps);
     float ss = 0.f;
-    if (CACHE) {
-#pragma unroll
-        for (int i = 0; i < EN; ++i) {
-            const int c = threadIdx.x + i * 256;
-            if (c < W) {
-                const float m = 0.5f * (va[i] * ra * wa[c] + vb[i] * rb * wb[c]);
-                vx[i] = fmaf(alpha, vx[i], m);
-                ss = fmaf(vx[i], vx[i], ss);
-            }
-        }
-    } else {
-        for (int c = threadIdx.x; c < W; c += blockDim.x) {
-            const float m = 0.5f * (ldf(ar + c) * ra * wa[c] + ldf(br + c) * rb * wb[c]);
-            const float v = fmaf(alpha, x[c], m);
-            ss = fmaf(v, v, ss);
-        }
+    for (int c = threadIdx.x; c < W; c += blockDim.x) {
+        const float m = 0.5f * (ldf(ar + c) * ra * wa[c] + ldf(br + c) * rb * wb[c]);
+        const float v = fmaf(alpha, x[c], m);
+        ss = fmaf(v, v, ss);
     }
-    ss = block_sum(ss, red);
-    const float rn = 1.f / sqrtf(ss / (float)W + eps);
-    if (CACHE) {
-#pragma unroll
-        for (int i = 0; i < EN; ++i) {
-            const int c = threadIdx.x + i * 256;
-            if (c < W) {
-                const float v = vx[i] * rn * w[c];
-                x[c] = v;
-                stf(xa + (size_t)r * W + c, v);
-            }
-        }
-    } else {
-        for (int c = threadIdx.x; c < W; c += blockDim.x) {
-            const float m = 0.5f * (ldf(ar + c) * ra * wa[c] + ldf(br + c) * rb * wb[c]);
-            const float v = fmaf(alpha, x[c], m) * rn * w[c];
-            x[c] = v;
-            stf(xa + (size_t)r * W + c, v);
-        }
+    const float rn = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
+    for (int c = threadIdx.x; c < W; c += blockDim.x) {
+        const float m = 0.5f * (ldf(ar + c) * ra * wa[c] + ldf(br + c) * rb * wb[c]);
+        const float v = fmaf(alpha, x[c], m) * rn * w[c];
+        x[c] = v;
+        stf(o + c, v);
     }
 }
 
@@ -161,14 +182,18 @@ __global__ void __launch_bounds__(256) postnorm_branch_kernel(float* __restrict_
     float* x = x32 + (size_t)r * W;
     const int top = has_mc ? mc.top : 0;
     const bool cached = top <= kCombineTop;
-    float vx[EN][V];
+    constexpr bool KEEP = E > 0 && E <= 4;      // the norm's weights too (behind the sum they would wait once more)
+    float vx[EN][V], kw[KEEP ? EN : 1][V];
     if (E > 0) {            // the residual row's loads fly while the routed row's places are read
 #pragma unroll
         for (int i = 0; i < EN; ++i) {
             const int c = (threadIdx.x + i * 256) * V;
 #pragma unroll
             for (int u = 0; u < V; ++u) vx[i][u] = 0.f;
-            if (c < W) { if (VEC) ld4(x + c, (float(&)[4])vx[i]); else vx[i][0] = x[c]; }
+            if (c < W) {
+                if (VEC) ld4(x + c, (float(&)[4])vx[i]); else vx[i][0] = x[c];
+                if (KEEP) { if (VEC) ld4(w + c, (float(&)[4])kw[KEEP ? i : 0]); else kw[KEEP ? i : 0][0] = w[c]; }
+            }
         }
     }
     if (has_mc && cached) {
@@ -226,9 +251,13 @@ __global__ void __launch_bounds__(256) postnorm_branch_kernel(float* __restrict_
         }
     }
     const float rn = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
-    auto store = [&](int c, const float (&v)[V]) {
+    auto store = [&](int c, const float (&v)[V], const float* kept) {
         float o[V], t[V];
-        if (VEC) ld4(w + c, (float(&)[4])t); else t[0] = w[c];
+        if (kept) {
+#pragma unroll
+            for (int u = 0; u < V; ++u) t[u] = kept[u];
+        } else if (VEC) ld4(w + c, (float(&)[4])t);
+        else t[0] = w[c];
 #pragma unroll
         for (int u = 0; u < V; ++u) o[u] = v[u] * rn * t[u];
         if (VEC) st4(x + c, (const float(&)[4])o); else x[c] = o[0];
@@ -236,12 +265,12 @@ __global__ void __launch_bounds__(256) postnorm_branch_kernel(float* __restrict_
     };
     if (E > 0) {
 #pragma unroll
-        for (int i = 0; i < EN; ++i) { const int c = (threadIdx.x + i * 256) * V; if (c < W) store(c, vx[i]); }
+        for (int i = 0; i < EN; ++i) { const int c = (threadIdx.x + i * 256) * V; if (c < W) store(c, vx[i], KEEP ? kw[KEEP ? i : 0] : nullptr); }
     } else {
         for (int c = threadIdx.x * V; c < W; c += 256 * V) {
             float v[V];
             if (VEC) ld4(x + c, (float(&)[4])v); else v[0] = x[c];
-            store(c, v);
+            store(c, v, nullptr);
         }
     }
 }
@@ -410,14 +439,53 @@ __device__ __forceinline__ float norm_apply(const NormSpec& n, float v, float rn
     return n.kind == NORM_DYT ? fmaf(tanhf(n.alpha * v), n.w[c], n.b[c]) : v * rn * n.w[c];
 }
 
-template <typename T>
+// One CTA per wanted row. E: pieces of V columns per thread, kept in registers (0: wider rows are read again in each pass). One row of 2048 columns in a
+// step: 5.8 us with single columns and a pass over memory for the sum and one for the result, 3.6 so.
+template <typename T, int E, bool VEC>
 __global__ void __launch_bounds__(256) gather_norm_kernel(const float* __restrict__ x32, const int* __restrict__ rows, NormSpec n,
                                                           T* __restrict__ out, int W) {
     chain_begin(x32, rows);
     __shared__ float red[32];
+    constexpr int V = VEC ? 4 : 1, EN = E > 0 ? E : 1;
     const int i = blockIdx.x;
     const float* x = x32 + (size_t)rows[i] * W;
+    T* o = out + (size_t)i * W;
     float rn = 1.f, mean = 0.f;
+    if (E > 0) {
+        float v[EN][V];
+#pragma unroll
+        for (int e = 0; e < EN; ++e) {
+            const int c = (threadIdx.x + e * 256) * V;
+#pragma unroll
+            for (int u = 0; u < V; ++u) v[e][u] = 0.f;
+            if (c < W) { if (VEC) ld4(x + c, (float(&)[4])v[e]); else v[e][0] = x[c]; }
+        }
+        if (n.kind != NORM_DYT) {
+            if (n.kind == NORM_LAYER) {
+#pragma unroll
+                for (int e = 0; e < EN; ++e)
+#pragma unroll
+                    for (int u = 0; u < V; ++u) mean += v[e][u];
+                mean = block_sum(mean, red) / (float)W;
+            }
+            float ss = 0.f;
+#pragma unroll
+            for (int e = 0; e < EN; ++e)
+#pragma unroll
+                for (int u = 0; u < V; ++u)
+                    if ((threadIdx.x + e * 256) * V < W) ss = fmaf(v[e][u] - mean, v[e][u] - mean, ss);
+            rn = 1.f / sqrtf(block_sum(ss, red) / (float)W + n.eps);
+        }
+#pragma unroll
+        for (int e = 0; e < EN; ++e) {
+            const int c = (threadIdx.x + e * 256) * V;
+            if (c >= W) continue;
+#pragma unroll
+            for (int u = 0; u < V; ++u) v[e][u] = norm_apply(n, v[e][u] - mean, rn, c + u);
+            if (VEC) st4(o + c, (const float(&)[4])v[e]); else stf(o + c, v[e][0]);
+        }
+        return;
+    }
     if (n.kind != NORM_DYT) {
         float ss = 0.f;
         if (n.kind == NORM_LAYER) {
@@ -428,7 +496,7 @@ __global__ void __launch_bounds__(256) gather_norm_kernel(const float* __restric
         ss = block_sum(ss, red);
         rn = 1.f / sqrtf(ss / (float)W + n.eps);
     }
-    for (int c = threadIdx.x; c < W; c += blockDim.x) stf(out + (size_t)i * W + c, norm_apply(n, x[c] - mean, rn, c));
+    for (int c = threadIdx.x; c < W; c += blockDim.x) stf(o + c, norm_apply(n, x[c] - mean, rn, c));
 }
 
 // One CTA per row: pass 1 forms the new residual row (every addend read, also a row of xa that pass 2 rewrites) and, for a
@@ -765,10 +833,12 @@ int embed_sinusoid(int dt, const int64_t* ids, const int* seq_len, const void* t
                    const float* inv_freq, float* x32, void* xa, int S, int W, SeqPos pos, cudaStream_t s, int copies) {
     if (!ids || !table || !x32 || S < 1 || W < 1 || copies < 1) return -2;
     count_launch();
+    // few rows: a column per thread (eight sines one after the other in each thread took 10.1 us for one row of 2048 columns, one takes 2.4)
+    const dim3 grid(S, S <= kSms ? std::min((W + 255) / 256, 8) : 1);
     if (dt == DT_F32)
-        chained(embed_sinusoid_kernel<float>, S, 256, 0, s)(ids, seq_len, (const float*)table, vocab, scale, inv_freq, x32, (float*)xa, S, W, pos, copies);
+        chained(embed_sinusoid_kernel<float>, grid, 256, 0, s)(ids, seq_len, (const float*)table, vocab, scale, inv_freq, x32, (float*)xa, S, W, pos, copies);
     else
-        chained(embed_sinusoid_kernel<bf16>, S, 256, 0, s)(ids, seq_len, (const bf16*)table, vocab, scale, inv_freq, x32, (bf16*)xa, S, W, pos, copies);
+        chained(embed_sinusoid_kernel<bf16>, grid, 256, 0, s)(ids, seq_len, (const bf16*)table, vocab, scale, inv_freq, x32, (bf16*)xa, S, W, pos, copies);
     return done();
 }
 
@@ -801,19 +871,23 @@ int postnorm_residual(int dt, float* x32, void* xa, const void* a, int ld_a, con
 #undef LCC_PNB2
         return done();
     }
-#define LCC_PNR(E)                                                                                                          \
+    auto row4 = [&](const void* p, int ld) { return (ld % 4) == 0 && ((uintptr_t)p % (dt == DT_F32 ? 16 : 8)) == 0; };
+    const bool vec = (W % 4) == 0 && (((uintptr_t)x32 | (uintptr_t)w | (uintptr_t)wa | (uintptr_t)wb) % 16) == 0 && row4(a, ld_a) && row4(b, ld_b) && row4(xa, W);
+#define LCC_PNR2(E, VECB)                                                                                                   \
     do {                                                                                                                    \
         if (dt == DT_F32)                                                                                                   \
-            chained(postnorm_residual_kernel<float, E>, S, 256, 0, s)(x32, (float*)xa, (const float*)a, ld_a, wa, (const float*)b, ld_b, wb, w, alpha, eps, W); \
+            chained(postnorm_residual_kernel<float, E, VECB>, S, 256, 0, s)(x32, (float*)xa, (const float*)a, ld_a, wa, (const float*)b, ld_b, wb, w, alpha, eps, W); \
         else                                                                                                                \
-            chained(postnorm_residual_kernel<bf16, E>, S, 256, 0, s)(x32, (bf16*)xa, (const bf16*)a, ld_a, wa, (const bf16*)b, ld_b, wb, w, alpha, eps, W); \
+            chained(postnorm_residual_kernel<bf16, E, VECB>, S, 256, 0, s)(x32, (bf16*)xa, (const bf16*)a, ld_a, wa, (const bf16*)b, ld_b, wb, w, alpha, eps, W); \
     } while (0)
-    const int per = (W + 255) / 256;
+#define LCC_PNR(E) do { if (vec) LCC_PNR2(E, true); else LCC_PNR2(E, false); } while (0)
+    const int per = (W / (vec ? 4 : 1) + 255) / 256;
     if (per <= 2) LCC_PNR(2);
     else if (per <= 4) LCC_PNR(4);
-    else if (per <= 8) LCC_PNR(8);
-    else if (per <= kRowCache) LCC_PNR(16);
-    else LCC_PNR(0);
+    else if (vec || per > kRowCache) LCC_PNR2(0, false);     // more than 4096 columns
+    else if (per <= 8) LCC_PNR2(8, false);
+    else LCC_PNR2(16, false);
+#undef LCC_PNR2
 #undef LCC_PNR
     return done();
 }
@@ -915,10 +989,19 @@ int gather_norm(int dt, const float* x32, const int* rows, const NormSpec& n, vo
     if (!x32 || !rows || !n.w || !out || n_rows < 1 || W < 1 || (n.kind == NORM_DYT && !n.b) || (n.kind != NORM_DYT && n.kind != NORM_RMS && n.kind != NORM_LAYER))
         return -2;
     count_launch();
-    if (dt == DT_F32)
-        chained(gather_norm_kernel<float>, n_rows, 256, 0, s)(x32, rows, n, (float*)out, W);
-    else
-        chained(gather_norm_kernel<bf16>, n_rows, 256, 0, s)(x32, rows, n, (bf16*)out, W);
+    const bool vec = (W % 4) == 0 && ((uintptr_t)x32 % 16) == 0 && ((uintptr_t)out % 16) == 0;
+    const int pieces = (W / (vec ? 4 : 1) + 255) / 256;
+#define LCC_GN2(E, VECB)                                                                                                  \
+    do {                                                                                                                  \
+        if (dt == DT_F32) chained(gather_norm_kernel<float, E, VECB>, n_rows, 256, 0, s)(x32, rows, n, (float*)out, W);   \
+        else chained(gather_norm_kernel<bf16, E, VECB>, n_rows, 256, 0, s)(x32, rows, n, (bf16*)out, W);                  \
+    } while (0)
+#define LCC_GN(E) do { if (vec) LCC_GN2(E, true); else LCC_GN2(E, false); } while (0)
+    if (pieces <= 2) LCC_GN(2);
+    else if (pieces <= 8) LCC_GN(8);
+    else LCC_GN(0);
+#undef LCC_GN
+#undef LCC_GN2
     return done();
 }
 

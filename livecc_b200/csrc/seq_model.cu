@@ -1020,11 +1020,17 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
     if (n_want > 0) {
         const lcc::NormSpec fn{d.norm_kind, d.final_norm_f32, d.final_norm_bias_f32, d.final_norm_alpha, d.eps};
         STEP(lcc::gather_norm(dt, hc ? xsum : x32, want_rows, fn, xf, n_want, W, s), "final norm");
-        // scored prompts ask for many rows: the head is then a product like any other. 128 rows x 32768 outputs of width 2048: 648 us
-        // as CUDA-core tiles; decode steps (up to 8 rows) keep the weight-streaming kernel, which `linear` falls back to.
-        STEP(linear(m, xf, W, d.head, nullptr, logits, d.vocab, true, n_want, d.vocab, W, s), "output head");
-        STEP(lcc::softcap(logits, (int64_t)n_want * d.vocab, d.logit_softcap, s, d.logit_scale != 0.f ? d.logit_scale : 1.f), "logit soft cap / scale");
-        if (logits_copy) STEP(copy_f32(logits_copy, logits, (size_t)n_want * d.vocab, s), "logits copy");
+        const float scale = d.logit_scale != 0.f ? d.logit_scale : 1.f;
+        if (n_want <= lcc::kLogitRows) {
+            // decode steps: the soft cap, the scale and the second copy ride in the store of the weight-streaming kernel (as kernels of their own 2.5 us of a step)
+            STEP(lcc::linear_logits(dt, xf, W, d.head, W, logits, logits_copy, d.vocab, n_want, d.vocab, W, d.logit_softcap, scale, s), "output head");
+        } else {
+            // scored prompts ask for many rows: the head is then a product like any other. 128 rows x 32768 outputs of width 2048: 648 us
+            // as CUDA-core tiles
+            STEP(linear(m, xf, W, d.head, nullptr, logits, d.vocab, true, n_want, d.vocab, W, s), "output head");
+            STEP(lcc::softcap(logits, (int64_t)n_want * d.vocab, d.logit_softcap, s, scale), "logit soft cap / scale");
+            if (logits_copy) STEP(copy_f32(logits_copy, logits, (size_t)n_want * d.vocab, s), "logits copy");
+        }
     }
     LCC_CHECK_LAUNCH(m->ctx, "lcc_seq_forward");
     return 0;

@@ -40,6 +40,10 @@ struct MoeCombine {
 // c_f32. Any M, N, K >= 1; leading dimensions in elements.
 int linear_any(int dt, const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, bool c_f32,
                int M, int N, int K, cudaStream_t s);
+// The output head of few rows (M <= 8): C = softcap(A x W^T) * scale in fp32 (cap <= 0: none), stored a second time in `copy` (or null).
+constexpr int kLogitRows = 8;
+int linear_logits(int dt, const void* A, int lda, const void* W, int ldw, float* C, float* copy, int ldc, int M, int N, int K, float cap, float scale,
+                  cudaStream_t s);
 
 // The same product for `groups` independent problems in one launch (per-head projections, routed experts). Group z reads
 // A + z * a_stride, W + z * w_stride and writes C + z * c_stride (strides in elements). Without row_off every group has M

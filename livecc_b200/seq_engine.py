@@ -673,8 +673,9 @@ class SeqLMForCausalLM:
         out = GenerateOutput(sequences=seq, past_key_values=cache, logits=logits_out[:n_gen] if output_logits else None)
         return out if return_dict_in_generate else out.sequences
 
-    def _select(self, raw: torch.Tensor, cache: SeqCache, sp: _cabi.Sampling, advance: int):
-        self._logits_proc.copy_(raw[0])
+    def _select(self, raw: torch.Tensor, cache: SeqCache, sp: _cabi.Sampling, advance: int, copied: bool = False):
+        if not copied:
+            self._logits_proc.copy_(raw[0])
         self.ctx.call("lcc_sample_greedy", _cabi._ptr(raw), _cabi._ptr(self._logits_proc), _cabi._i(self.config.vocab),
                       _cabi._ptr(cache.seq_buf), _cabi._ptr(cache.scalars), C.byref(sp), _cabi._i(advance), None, None,
                       _cabi._i(self.config.width), _cabi.Context.stream_ptr())
@@ -683,8 +684,8 @@ class SeqLMForCausalLM:
         """One token, all bookkeeping on the device: the step reads the last id (seq[SEQ_LEN - 1]) and the number of cached
         tokens (KV_LEN) from the sequence's scalars; the selection kernel appends the next id and advances both."""
         ent = self._entry(cache, cache.seq_buf, 1, keep, device_pos=True)
-        self._native.forward([ent], PAGE_SIZE, self._want0, 1, raw, None, None)
-        self._select(raw, cache, sp, advance=1)
+        self._native.forward([ent], PAGE_SIZE, self._want0, 1, raw, self._logits_proc, None)
+        self._select(raw, cache, sp, advance=1, copied=True)
 
     def _run_decode(self, cache: SeqCache, raw: torch.Tensor, sp: _cabi.Sampling, n_steps: int, hist):
         if not hasattr(self, "_want0"):

@@ -1,0 +1,42 @@
+"""Row kernels of a decode step at the widths where their forms meet, the output head's store, and few-row products whose warps share columns, against float64."""
+import pytest
+import torch
+
+import seq_cases
+import seq_oracle as O
+from livecc_b200.checkpoint import synthetic_seq_tensors
+from livecc_b200.config import SeqModelConfig
+from test_seq_gpu import BF16_TOL, F32_TOL, rel, run
+
+pytestmark = pytest.mark.gpu
+
+
+# widths on and off 4-column boundaries, at the ends of the register forms (2 and 4 or 8 pieces of 256 x 4 or 256 columns) and one past them
+@pytest.mark.parametrize("width", [24, 255, 512, 514, 1024, 2046, 2048, 2052, 4096, 4100])
+def test_widths_of_the_row_kernels(width):
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    heads = dict(heads=2, kv_heads=1, dim=12, vdim=8) if width % 4 else dict(heads=4, kv_heads=2, dim=16, vdim=8)
+    d = seq_cases.config([seq_cases.par(**heads, ff=None)], width=width, vocab=70, softcap=8.0)
+    cfg = SeqModelConfig.from_json(d)
+    t = synthetic_seq_tensors(cfg, seed=3)
+    toks = seq_cases.tokens(5, 70, seed=width)
+    want, _ = O.forward(d, t, toks)
+    for dtype, tol in (("float32", F32_TOL), ("bfloat16", BF16_TOL)):
+        m = SeqLMForCausalLM.from_state_dict(cfg, t, dtype)
+        assert rel(run(m, toks, [3, 4]), want) < tol
+
+
+# head sizes of the q/k norm's register forms: 2 x 1024 and 4 x 1024 query columns, one past them, and columns off 4-element boundaries
+@pytest.mark.parametrize("heads,kv,dim", [(2, 1, 10), (8, 2, 256), (9, 3, 228), (16, 4, 256), (17, 1, 256), (4, 4, 260)])
+def test_widths_of_the_query_and_key_norm(heads, kv, dim):
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    d = seq_cases.config([seq_cases.par(heads=heads, kv_heads=kv, dim=dim, vdim=8, scale=dim ** -0.5, ff=None)], width=40)
+    cfg = SeqModelConfig.from_json(d)
+    t = synthetic_seq_tensors(cfg, seed=3)
+    toks = seq_cases.tokens(6, 96, seed=dim)
+    want, _ = O.forward(d, t, toks)
+    for dtype, tol in (("float32", F32_TOL), ("bfloat16", BF16_TOL)):
+        m = SeqLMForCausalLM.from_state_dict(cfg, t, dtype)
+        assert rel(run(m, toks, [4, 5]), want) < tol
