@@ -110,6 +110,8 @@ __global__ void __launch_bounds__(256) linear_tile_kernel(const T* __restrict__ 
 // (column, row of A), so the order of a column's sum does not depend on WR, WU or M. MM is the number of rows the accumulators hold: with
 // accumulators and addresses for eight rows a one-row step had the registers for four loads per weight row only: 32 tokens of four
 // recurrent layers of width 2048 took 10.93 ms and take 8.68 ms, of two routed layers 6.34 and 5.06 ms.
+// KS: warps that share a group of columns, each with every KS-th piece of k; their sums meet in shared memory in a fixed order. A warp of one column reads
+// as much of A from L1 as of W from memory and unpacks both; two columns and half of k halve that with the same loads in flight.
 // Scalar loads when K or a row start is not 16-byte aligned.
 constexpr int kRowsMax = kLogitRows;
 template <typename T> struct Vec16;
@@ -127,13 +129,13 @@ template <> struct Vec16<float> {
     }
 };
 
-template <typename T, typename TC, bool VEC, int MM, int WR, int WU, bool GLU = false>
+template <typename T, typename TC, bool VEC, int MM, int WR, int WU, bool GLU = false, int KS = 1>
 __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ A, int lda, const T* __restrict__ W, int ldw,
                                                           const float* __restrict__ bias, TC* __restrict__ C, int ldc, int M_all,
                                                           int N, int K, Grp g) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = (blockIdx.x * (blockDim.x >> 5) + warp) * (GLU ? 1 : WR);
-    if (n0 >= N) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = warp % KS;
+    const int n0 = (blockIdx.x * ((blockDim.x >> 5) / KS) + warp / KS) * (GLU ? 1 : WR);
+    if (KS == 1 && n0 >= N) return;     // (with KS > 1 all warps meet below; columns past the end read the last one and store nothing)
     int row0 = 0, z = blockIdx.y;
     constexpr int V = Vec16<T>::N;
     // the weight row behind accumulator r: output columns n0, n0 + 1, ...; in the GLU form (WR = 2) the gate row (r = 0) and
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
         for (int r = 0; r < WR; ++r)
 #pragma unroll
             for (int u = 0; u < WU; ++u) {
-                const int k = kb + u * 32 * V;
+                const int k = kb + u * 32 * V * KS;
                 wq[r][u] = k < K ? ld_stream16(W + (size_t)wrow(r) * ldw + k) : make_uint4(0, 0, 0, 0);
             }
     };
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
     bool loaded = false;
     if (EARLY && !g.row_off) {
         W += z * g.w_stride;
-        load_weights(lane * V);
+        load_weights((part * 32 + lane) * V);
         loaded = true;
     }
     chain_begin(A);
@@ -192,12 +194,12 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
 #pragma unroll
         for (int m = 0; m < MM; ++m) acc[r][m] = 0.f;
     if (VEC) {
-        for (int kb = lane * V; kb < K; kb += 32 * V * WU) {
+        for (int kb = (part * 32 + lane) * V; kb < K; kb += 32 * V * WU * KS) {
             if (!EARLY || !loaded) load_weights(kb);
             loaded = false;
 #pragma unroll
             for (int u = 0; u < WU; ++u) {
-                const int k = min(kb + u * 32 * V, K - V);      // past the end the weights are zero; keep the address valid
+                const int k = min(kb + u * 32 * V * KS, K - V);      // past the end the weights are zero; keep the address valid
                 float wv[WR][V];
 #pragma unroll
                 for (int r = 0; r < WR; ++r) Vec16<T>::unpack(wq[r][u], wv[r]);
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
             }
         }
     } else {
-        for (int k = lane; k < K; k += 32) {
+        for (int k = part * 32 + lane; k < K; k += 32 * KS) {
 #pragma unroll
             for (int r = 0; r < WR; ++r) {
                 const float wv = ldf(W + (size_t)wrow(r) * ldw + k);
@@ -236,13 +238,27 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
         }
         continue;
     }
+    __shared__ float sums[KS > 1 ? 8 : 1][WR * MM];
+    if (KS > 1) {
+#pragma unroll
+        for (int r = 0; r < WR; ++r)
+#pragma unroll
+            for (int m = 0; m < MM; ++m) {
+                const float v = m < M ? warp_sum(acc[r][m]) : 0.f;
+                if (lane == 0) sums[warp][r * MM + m] = v;
+            }
+        __syncthreads();
+        if (part != 0) return;          // (one block of rows: KS > 1 is not for lists)
+    }
 #pragma unroll
     for (int r = 0; r < WR; ++r) {
         const int n = n0 + r;
 #pragma unroll
         for (int m = 0; m < MM; ++m) {
             if (m < M) {
-                const float v = warp_sum(acc[r][m]);
+                float v = KS > 1 ? sums[warp][r * MM + m] : warp_sum(acc[r][m]);
+#pragma unroll
+                for (int i = 1; i < KS; ++i) v += sums[KS > 1 ? warp + i : 0][r * MM + m];
                 if (lane != 0 || n >= N) continue;
                 if constexpr (std::is_same<TC, float>::value) {
                     if (g.scale != 0.f) {
@@ -274,12 +290,14 @@ int launch_linear(const void* A, int lda, const void* W, int ldw, const float* b
         count_launch();
         // rows of A that share a weight row: M, or, with lists, at most M of a list's rows (longer lists walk blocks of MM)
         const int mm = M;
-#define LCC_ROWS(MMN, WRN, WUN, WARPS, GLUB)                                                                                    \
+#define LCC_ROWS_KS(MMN, WRN, WUN, WARPS, GLUB, KSN)                                                                           \
     do {                                                                                                                       \
-        const dim3 grid((N + WARPS * (GLUB ? 1 : WRN) - 1) / (WARPS * (GLUB ? 1 : WRN)), grid_y);                              \
-        if (vec) chained(linear_rows_kernel<T, TC, true, MMN, WRN, WUN, GLUB>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g); \
-        else chained(linear_rows_kernel<T, TC, false, MMN, WRN, WUN, GLUB>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g);    \
+        constexpr int per = (WARPS) / (KSN) * (GLUB ? 1 : WRN);                                                                \
+        const dim3 grid((N + per - 1) / per, grid_y);                                                                          \
+        if (vec) chained(linear_rows_kernel<T, TC, true, MMN, WRN, WUN, GLUB, KSN>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g); \
+        else chained(linear_rows_kernel<T, TC, false, MMN, WRN, WUN, GLUB, KSN>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g);    \
     } while (0)
+#define LCC_ROWS(MMN, WRN, WUN, WARPS, GLUB) LCC_ROWS_KS(MMN, WRN, WUN, WARPS, GLUB, 1)
         if (g.glu_F > 0) {
             if constexpr (std::is_same<T, TC>::value) {
                 if (mm == 1) LCC_ROWS(1, 2, 8, 2, true);
@@ -290,12 +308,27 @@ int launch_linear(const void* A, int lda, const void* W, int ldw, const float* b
                 return -2;
             }
         }
-        // Wide matrices: two columns per warp and CTAs of 8 warps. Narrower ones: one column per warp in CTAs of 2 warps, so that the
-        // warps spread evenly over the SMs and the whole matrix is in flight at once; 16 loads per lane cover a 4096-wide bf16 row.
+        // Wide matrices: for one row a column per warp and CTAs of 4 warps, which leave and arrive in small portions; two columns and 8 warps for
+        // more rows. Narrower ones with 1024 to 6144 k (bf16): warps share columns, four by four in matrices of up to 4096 columns, two by two above (one
+        // column for more rows), so that the whole matrix is in flight at once. The rule does not look at M: neither do a row's bits. (Wide matrices two
+        // by two would save one row another us but cost four rows 20 % and eight 25 %: twice the sums across lanes. Longer k, 2048 x 8448, filled
+        // the SMs in front of the attention that runs beside it: a routed step of four sequences 435 us, 394 so, 404 before.) One row in a step,
+        // before | now, us: 2048 columns x 4096: 6.4 | 3.6; 2048 x 5632: 11.0 | 7.0; 2048 x 2048: 4.5 | 3.0; 6208 x 2048: 6.6 | 5.4;
+        // 10304 x 2048: 10.3 | 9.4; 32768 x 2048: 24.4 | 21.0. Steps of 2, 4 and 8 sequences: recurrent 372, 668, 1140 | 285, 541, 870.
         if (N >= 8192) {
-            if (mm == 1) LCC_ROWS(1, 2, 8, 8, false);
+            if (mm == 1) LCC_ROWS(1, 1, 8, 4, false);
             else if (mm <= 2) LCC_ROWS(2, 2, 8, 8, false);
             else LCC_ROWS(8, 2, 4, 8, false);
+        } else if (!g.row_off && K >= 4 * 32 * V && K <= 24 * 32 * V && N <= 4096) {
+            if (mm == 1 && K <= 8 * 32 * V) LCC_ROWS_KS(1, 4, 2, 4, false, 4);
+            else if (mm == 1 && K <= 16 * 32 * V) LCC_ROWS_KS(1, 4, 4, 4, false, 4);
+            else if (mm == 1) LCC_ROWS_KS(1, 4, 6, 4, false, 4);
+            else if (mm <= 2) LCC_ROWS_KS(2, 1, 4, 4, false, 4);
+            else LCC_ROWS_KS(8, 1, 2, 4, false, 4);
+        } else if (!g.row_off && K >= 4 * 32 * V && K <= 24 * 32 * V) {
+            if (mm == 1) LCC_ROWS_KS(1, 2, 4, 4, false, 2);
+            else if (mm <= 2) LCC_ROWS_KS(2, 1, 4, 4, false, 2);
+            else LCC_ROWS_KS(8, 1, 4, 4, false, 2);
         } else if (mm == 1 && K > 8 * 32 * V) {
             LCC_ROWS(1, 1, 16, 2, false);
         } else if (mm == 1) {
@@ -305,6 +338,7 @@ int launch_linear(const void* A, int lda, const void* W, int ldw, const float* b
         } else {
             LCC_ROWS(8, 1, 4, 2, false);
         }
+#undef LCC_ROWS_KS
 #undef LCC_ROWS
     } else if (g.glu_F > 0) {
         // raw gate and up columns into the caller's scratch, then the activation as a row kernel
