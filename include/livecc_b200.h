@@ -101,6 +101,18 @@ int lcc_gemm_form(lcc_ctx* ctx, const void* A, int lda, const void* B, int ldb, 
 /* hidden_states.to(bf16) of the f32 patch rows (mq2vl.py:309). */
 int lcc_cast_f32_bf16(lcc_ctx* ctx, const float* in, void* out, int64_t n, lcc_stream_t stream);
 
+/* What the turns of up to 8 streams bring to the device beside their pixels, in one launch. Per stream: seq[0..L) = ids, pos3 [3, S] = pos_base,
+ * pos_base + 1, .. in each row (pos3 may be null), scalars[0..8) = values. `turns` is host memory, read before the call returns. */
+typedef struct {
+    const int64_t* ids;
+    int64_t* seq;
+    int32_t* pos3;
+    int32_t* scalars;
+    int32_t L, S, pos_base;
+    int32_t values[8];
+} lcc_turn;
+int lcc_turn_setup(lcc_ctx* ctx, const lcc_turn* turns, int n, lcc_stream_t stream);
+
 /* nn.LayerNorm(dim, eps) over rows (ViT norm1/norm2/ln_q, mq2vl.py:464-465,317). */
 int lcc_layernorm(lcc_ctx* ctx, const void* x, int ldx, const void* w, const void* b, void* y, int ldy,
                   int rows, int dim, float eps, lcc_stream_t stream);

@@ -64,6 +64,11 @@ class StreamState(C.Structure):
                 ("page_table", C.c_void_p), ("scalars", C.c_void_p), ("seq", C.c_void_p)]
 
 
+class Turn(C.Structure):
+    _fields_ = [("ids", C.c_void_p), ("seq", C.c_void_p), ("pos3", C.c_void_p), ("scalars", C.c_void_p), ("L", C.c_int32), ("S", C.c_int32),
+                ("pos_base", C.c_int32), ("values", C.c_int32 * 8)]
+
+
 class PrefillRequest(C.Structure):
     """lcc_prefill_request"""
     _fields_ = [("st", StreamState), ("ids", C.c_void_p), ("pos3", C.c_void_p), ("S", C.c_int32), ("past", C.c_int32),
@@ -284,7 +289,19 @@ class Context:
     def stream_ptr():
         import torch
 
-        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        # (torch.cuda.current_stream() builds a stream object: 4 us for a number)
+        return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+
+    def turn_setup(self, turns):
+        """turns: up to 8 tuples (ids [L] int64 contiguous, seq, pos3 [3, S] int32 or None, pos_base, scalars, eight values); per turn
+        seq[:L] = ids, pos3 = pos_base, pos_base + 1, .. in each row, scalars[:8] = values."""
+        arr = (Turn * len(turns))()
+        for t, (ids, seq, pos3, base, scalars, values) in zip(arr, turns):
+            t.ids, t.seq, t.scalars, t.L, t.pos_base = ids.data_ptr(), seq.data_ptr(), scalars.data_ptr(), ids.numel(), base
+            if pos3 is not None:
+                t.pos3, t.S = pos3.data_ptr(), pos3.shape[1]
+            t.values[:] = values
+        self.call("lcc_turn_setup", arr, _i(len(turns)), self.stream_ptr())
 
     # ---- op level ----------------------------------------------------------------------------
     def gemm(self, a, b, out=None, bias=None, residual=None, epilogue=EPI_NONE, block_n=0, splitk_ws=None):

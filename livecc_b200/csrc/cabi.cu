@@ -24,6 +24,10 @@ int lcc_cast_f32_bf16(lcc_ctx* ctx, const float* in, void* out, int64_t n, lcc_s
     OP_RET(ctx, lcc::cast_f32_bf16(in, (bf16*)out, n, ctx->num_sms, (cudaStream_t)stream), "lcc_cast_f32_bf16");
 }
 
+int lcc_turn_setup(lcc_ctx* ctx, const lcc_turn* turns, int n, lcc_stream_t stream) {
+    OP_RET(ctx, lcc::turn_setup(turns, n, (cudaStream_t)stream), "lcc_turn_setup");
+}
+
 int lcc_layernorm(lcc_ctx* ctx, const void* x, int ldx, const void* w, const void* b, void* y, int ldy,
                   int rows, int dim, float eps, lcc_stream_t stream) {
     OP_RET(ctx, lcc::layernorm((const bf16*)x, ldx, (const bf16*)w, (const bf16*)b, (bf16*)y, ldy, rows, dim, eps,

@@ -6,10 +6,13 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "../../include/livecc_b200.h"
+
 namespace lcc {
 typedef __nv_bfloat16 bf16;
 
 // elementwise.cu
+int turn_setup(const lcc_turn* turns, int n, cudaStream_t s);
 int cast_f32_bf16(const float* in, bf16* out, int64_t n, int num_sms, cudaStream_t s);
 int patchify_u8(const uint8_t* frames, int T, int H, int W, bf16* out, const float* mean255, const float* std255,
                 cudaStream_t s);

@@ -106,10 +106,13 @@ class LiveCCB200ForConditionalGeneration:
         while self.max_nsplit < 64 and 2 * self.max_nsplit * t.num_key_value_heads <= 2 * self.ctx.num_sms:
             self.max_nsplit *= 2
         self.nsplit = self.max_nsplit
-        self.last_stats = {}
-        # per-phase device time of the last generate() (CUDA events on the launch stream) and running totals
-        self.phase_ms_total = {"vit": 0.0, "prefill": 0.0, "decode": 0.0, "calls": 0, "decode_steps": 0}
+        # per-phase device time of the last generate() (CUDA events on the launch stream) and running totals. A call's events are read when somebody
+        # asks, or while the next call runs: reading them takes the host longer than a launch, and the device would wait for it
+        self._last_stats = {}
+        self._phase_ms_total = {"vit": 0.0, "prefill": 0.0, "decode": 0.0, "calls": 0, "decode_steps": 0}
+        self._unread_call = None
         self._ev = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
+        self._ev_spare = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
 
     @classmethod
     def from_synthetic(cls, config: LiveCCConfig, seed: int = 1234, device="cuda"):
@@ -214,6 +217,28 @@ class LiveCCB200ForConditionalGeneration:
     def new_cache(self) -> PagedKVCache:
         return PagedKVCache(self.pool)
 
+    @property
+    def last_stats(self) -> dict:
+        self._read_events()
+        return self._last_stats
+
+    @property
+    def phase_ms_total(self) -> dict:
+        self._read_events()
+        return self._phase_ms_total
+
+    def _read_events(self):
+        """Device times of the last finished generate(), if they have not been read yet."""
+        if self._unread_call is None:
+            return
+        ev, stats = self._unread_call
+        self._unread_call = None
+        ph = [ev[i].elapsed_time(ev[i + 1]) for i in range(3)]
+        self._last_stats = {**stats, "vit_ms": ph[0], "prefill_ms": ph[1], "decode_ms": ph[2]}
+        tot = self._phase_ms_total
+        tot["vit"] += ph[0]; tot["prefill"] += ph[1]; tot["decode"] += ph[2]
+        tot["calls"] += 1; tot["decode_steps"] += max(stats["generated"] - 1, 0)
+
     def _sampling(self, repetition_penalty, logits_processor, max_new_tokens) -> _cabi.Sampling:
         thr_token, thr_base, thr_step = -1, 0.0, 0.0
         for proc in logits_processor or []:
@@ -300,15 +325,19 @@ class LiveCCB200ForConditionalGeneration:
             raise TypeError(f"generate() got unsupported arguments {sorted(unsupported)}")
         self._check_common(pixel_values, image_grid_thw, do_sample, max_new_tokens)
         sp = self._sampling(repetition_penalty, logits_processor, max_new_tokens)
-        self._ev[0].record()
+        if self._unread_call is not None and self._unread_call[0] is self._ev_spare:
+            self._read_events()                                   # (a call in between ended in an error)
+        self._ev, self._ev_spare = self._ev_spare, self._ev       # the last call's events may still be unread
+        stream = torch.cuda.current_stream(self.device)
+        self._ev[0].record(stream)
         rec = self._begin_stream(input_ids, pixel_values_videos, video_grid_thw, past_key_values, video_frames, sp,
-                                 max_new_tokens, slot=0, timed=True)
+                                 max_new_tokens, slot=0, timed=stream)
         cache, st, L = rec["cache"], rec["st"], rec["L"]
         logits_out = [self._raw_logits().clone()] if output_logits else None
         if _forced_ids is not None:
             self._force_token(cache, L, 0, _forced_ids, max_new_tokens)
 
-        self._ev[2].record()
+        self._ev[2].record(stream)
         # ---- decode steps ----
         nsplit = self._pick_nsplit(rec["past"] + rec["S"] + max_new_tokens)
         n_steps = max_new_tokens - 1
@@ -329,15 +358,13 @@ class LiveCCB200ForConditionalGeneration:
                                           device=self.device)
             self._run_decode([cache], [st], sp, n_steps, nsplit, logits_hist)
 
-        self._ev[3].record()
+        self._ev[3].record(stream)
+        # while the device works: the times of the call before, and what the caller gets of this one
+        self._read_events()
+        self._take_results(rec, max_new_tokens, logits_hist)
         # ---- one host sync per generate(): read the stream scalars ----
-        out = self._finish_stream(rec, cache.scalars.tolist(), logits_out, logits_hist, output_logits)
-        ph = [self._ev[i].elapsed_time(self._ev[i + 1]) for i in range(3)]
-        self.last_stats = {"prefill_tokens": rec["S"], "generated": rec["n_gen"], "kv_len": cache.seq_len, "vit_ms": ph[0],
-                           "prefill_ms": ph[1], "decode_ms": ph[2]}
-        tot = self.phase_ms_total
-        tot["vit"] += ph[0]; tot["prefill"] += ph[1]; tot["decode"] += ph[2]
-        tot["calls"] += 1; tot["decode_steps"] += max(rec["n_gen"] - 1, 0)
+        out = self._finish_stream(rec, cache.scalars.tolist(), logits_out, output_logits)
+        self._unread_call = (self._ev, {"prefill_tokens": rec["S"], "generated": rec["n_gen"], "kv_len": cache.seq_len})
         return out if return_dict_in_generate else out.sequences
 
     @torch.inference_mode()
@@ -373,6 +400,7 @@ class LiveCCB200ForConditionalGeneration:
         for r in recs:   # a later stream's page allocation may have moved the pool: take the pointers after all of them
             r["st"] = r["cache"].stream_state()
         if "pos3" in recs[0]:
+            self.ctx.turn_setup([r["setup"] for r in recs])
             self._prefill_streams(recs, sp)
         V = self.config.text_config.vocab_size
         B = len(recs)
@@ -383,12 +411,15 @@ class LiveCCB200ForConditionalGeneration:
         if n_steps > 0:
             self._run_decode([r["cache"] for r in recs], [r["st"] for r in recs], sp, n_steps, 1, logits_hist)
         t_ev[2].record()
+        for b, r in enumerate(recs):
+            self._take_results(r, max_new_tokens, logits_hist[:, b] if logits_hist is not None else None)
         scal = torch.stack([r["cache"].scalars for r in recs]).tolist()   # the one host sync of the call
         outs = []
         for b, r in enumerate(recs):
             lo = [first_logits[b]] if output_logits else None
-            outs.append(self._finish_stream(r, scal[b], lo, logits_hist[:, b] if logits_hist is not None else None, output_logits))
-        tot = self.phase_ms_total
+            outs.append(self._finish_stream(r, scal[b], lo, output_logits))
+        self._read_events()
+        tot = self._phase_ms_total
         tot["prefill"] += t_ev[0].elapsed_time(t_ev[1]); tot["decode"] += t_ev[1].elapsed_time(t_ev[2])
         tot["calls"] += B; tot["decode_steps"] += max(max(r["n_gen"] for r in recs) - 1, 0)
         return outs
@@ -441,11 +472,12 @@ class LiveCCB200ForConditionalGeneration:
                 vid += 1
             rec = self._begin_stream(ids_b, None, g, None, None, sp, 1, slot=0, video_embeds=fe)
             out[b].copy_(self._raw_logits()[letters])
+            self._take_results(rec, 1, None)
             caches.append(rec)
         scal = torch.stack([r["cache"].scalars for r in caches]).tolist()   # one host sync for the batch
         try:
             for r, sc in zip(caches, scal):
-                self._finish_stream(r, sc, None, None, False)
+                self._finish_stream(r, sc, None, False)
         finally:
             for r in caches:
                 r["cache"].release()
@@ -473,7 +505,7 @@ class LiveCCB200ForConditionalGeneration:
         return self.nsplit
 
     def _begin_stream(self, input_ids, pixel_values_videos, video_grid_thw, past_key_values, video_frames, sp,
-                      max_new_tokens, slot, timed=False, video_embeds=None, defer=False):
+                      max_new_tokens, slot, timed=None, video_embeds=None, defer=False):
         """Everything of one stream's turn up to and including the prefill and the first token selection; the first
         token's embedding and logits land in row `slot` of the decode-step buffers. defer: all but the prefill, whose inputs
         are returned (the vision tower's rows are then this call's own: the next stream's pass overwrites the static ones)."""
@@ -500,10 +532,9 @@ class LiveCCB200ForConditionalGeneration:
             pos3, delta = get_rope_index(ids_host, grids, cfg.video_token_id, cfg.image_token_id,
                                          cfg.vision_config.spatial_merge_size, self.legacy_4x_positions)
             cache.rope_delta = delta
-            pos3_dev = pos3.to(torch.int32).to(self.device).contiguous()
+            pos3_dev, running = pos3.to(torch.int32).to(self.device).contiguous(), None
         else:
-            base = torch.arange(past + cache.rope_delta, past + cache.rope_delta + S, dtype=torch.int32, device=self.device)
-            pos3_dev = base.view(1, -1).expand(3, -1).contiguous()
+            pos3_dev = running = torch.empty((3, S), dtype=torch.int32, device=self.device)    # (written with the ids and scalars below)
 
         # ---- vision tower ----
         n_video_expected = -1 if video_embeds is None else video_embeds.shape[0]
@@ -517,20 +548,21 @@ class LiveCCB200ForConditionalGeneration:
         elif video_frames is not None:
             video_embeds = self.get_video_features_from_frames(video_frames, _static_ok=not defer)
             n_video_expected = video_embeds.shape[0]
-        if timed:
-            self._ev[1].record()
+        if timed is not None:
+            self._ev[1].record(timed)
         # ---- capacity, buffers, device scalars ----
         if not defer:
             self._ensure_workspace(0, S)
         cache.ensure_tokens(past + S + max_new_tokens)
         cache.ensure_seq_capacity(L + max_new_tokens + 1)
-        cache.seq_buf[:L].copy_(ids_dev[0])
-        sc_host = torch.tensor([past + S, past + S + cache.rope_delta, 0, 0, L, 0, 0, 0], dtype=torch.int32)
-        cache.scalars.copy_(sc_host, non_blocking=False)
+        if ids_dev.dtype != torch.int64 or ids_dev.stride(1) != 1:
+            ids_dev = ids_dev.to(torch.int64).contiguous()
+        setup = (ids_dev, cache.seq_buf, running, past + cache.rope_delta, cache.scalars, (past + S, past + S + cache.rope_delta, 0, 0, L, 0, 0, 0))
+        if defer:
+            return dict(cache=cache, L=L, S=S, past=past, n_video_expected=n_video_expected, n_gen=0, pos3=pos3_dev, video=video_embeds, setup=setup)
+        self.ctx.turn_setup([setup])
         st = cache.stream_state()
         new_ids = cache.seq_buf[past:L]
-        if defer:
-            return dict(cache=cache, L=L, S=S, past=past, n_video_expected=n_video_expected, n_gen=0, pos3=pos3_dev, video=video_embeds)
         # ---- prefill + first token ----
         self._native.prefill(st, new_ids, pos3_dev, S, past, video_embeds, sp, slot=slot)
         return dict(cache=cache, st=st, L=L, S=S, past=past, n_video_expected=n_video_expected, n_gen=0)
@@ -552,7 +584,12 @@ class LiveCCB200ForConditionalGeneration:
             self._native.prefill_batch([(recs[b]["st"], recs[b]["cache"].seq_buf[recs[b]["past"]:recs[b]["L"]], recs[b]["pos3"], recs[b]["S"],
                                          recs[b]["past"], recs[b]["video"]) for b in g], sp, g[0])
 
-    def _finish_stream(self, rec, sc, logits_out, logits_hist, output_logits) -> GenerateOutput:
+    def _take_results(self, rec, max_new_tokens, logits_hist):
+        """Copy of the ids and the steps' logits row by row, before the host waits for the call: how many of them there are is cut behind it."""
+        rec["seq"] = rec["cache"].seq_buf[: rec["L"] + max_new_tokens].clone().view(1, -1)
+        rec["logits"] = list(logits_hist) if logits_hist is not None else None
+
+    def _finish_stream(self, rec, sc, logits_out, output_logits) -> GenerateOutput:
         cache, L, past = rec["cache"], rec["L"], rec["past"]
         self.ctx.check_fault()
         if sc[_cabi.SC_NATIVE_ERROR]:
@@ -572,10 +609,10 @@ class LiveCCB200ForConditionalGeneration:
                 raise ValueError(f"Video features and video tokens do not match, tokens: {n_video_ids}, "
                                  f"features: {rec['n_video_expected']}")
         cache.seq_len = sc[_cabi.SC_KV_LEN]
-        sequences = cache.seq_buf[: L + n_gen].clone().view(1, -1)
+        sequences = rec["seq"][:, : L + n_gen]
         if output_logits and logits_out is not None:
-            if logits_hist is not None:
-                logits_out += list(logits_hist[: max(n_gen - 1, 0)])
+            if rec["logits"] is not None:
+                logits_out += rec["logits"][: max(n_gen - 1, 0)]
             logits_out = logits_out[:n_gen]
         return GenerateOutput(sequences=sequences, past_key_values=cache, logits=logits_out if output_logits else None)
 
