@@ -268,6 +268,7 @@ constexpr int kMergeRows = 8;   // rows per CTA
 __global__ void __launch_bounds__(32 * kMergeRows) flash_merge_kernel(const float* __restrict__ part_o,
                                                                       const float* __restrict__ part_ml, const __grid_constant__ PrefillStreams ps,
                                                                       int Hkv, int G, float scale_log2, bf16* __restrict__ out, int o_ld) {
+    chain_begin(part_o, part_ml);
     const PrefillStream& st = ps.st[blockIdx.z];
     const int rr = blockIdx.x * kMergeRows + (threadIdx.x >> 5), g = blockIdx.y, lane = threadIdx.x & 31;
     const int rows_total = st.S * G, nsplit = st.nsplit;
@@ -535,7 +536,7 @@ int attn_prefill_streams(const bf16* q, int q_ld, const bf16* kc, const bf16* vc
         if (int r = attn_prefill_tc(q, q_ld, kc, vc, some, Hq, Hkv, out, o_ld, part_o, part_ml, s)) return r;
         if (longest) {
             lcc::count_launch();
-            flash_merge_kernel<<<dim3((longest * G + kMergeRows - 1) / kMergeRows, Hkv, some.n), 32 * kMergeRows, 0, s>>>(
+            chained(flash_merge_kernel, dim3((longest * G + kMergeRows - 1) / kMergeRows, Hkv, some.n), 32 * kMergeRows, 0, s)(
                 part_o, part_ml, some, Hkv, G, 1.4426950408889634f / sqrtf(128.f), out, o_ld);
         }
     }
@@ -583,7 +584,7 @@ int attn_prefill_paged(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, 
         ps.n = 1; ps.rows = S;
         ps.st[0].S = S; ps.st[0].nsplit = nsplit;
         lcc::count_launch();
-        flash_merge_kernel<<<dim3((S * p.G + kMergeRows - 1) / kMergeRows, Hkv), 32 * kMergeRows, 0, s>>>(part_o, part_ml, ps, Hkv, p.G, p.scale_log2, out, o_ld);
+        chained(flash_merge_kernel, dim3((S * p.G + kMergeRows - 1) / kMergeRows, Hkv), 32 * kMergeRows, 0, s)(part_o, part_ml, ps, Hkv, p.G, p.scale_log2, out, o_ld);
     }
     return 0;
 }

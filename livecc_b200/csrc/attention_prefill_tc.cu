@@ -157,6 +157,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    chain_begin();
 
     if (warp == 0) {
         // ===================== TMA producer =====================
@@ -468,7 +469,7 @@ int attn_prefill_tc(const bf16* q, int q_ld, const bf16* kc, const bf16* vc, con
     if (ensure_dyn_smem(once, attn_prefill_tc_kernel<false>, SMEM_BYTES)) return -12;
     const PrefillTcParams p{out, o_ld, Hkv, G, PT, 1.4426950408889634f / sqrtf((float)D), part_o, part_ml, ps};
     lcc::count_launch();
-    attn_prefill_tc_kernel<false><<<dim3(q_tiles, Hkv, slices), 192, SMEM_BYTES, s>>>(tq, tk, tv, p, PrefillLocal{});
+    chained(attn_prefill_tc_kernel<false>, dim3(q_tiles, Hkv, slices), 192, SMEM_BYTES, s)(tq, tk, tv, p, PrefillLocal{});
     return 0;
 }
 

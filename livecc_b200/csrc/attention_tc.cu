@@ -126,6 +126,7 @@ vit_attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    chain_begin();
 
     if (warp == 0) {
         // ===================== TMA producer =====================
@@ -358,7 +359,7 @@ static int launch_tc(const bf16* qkv, int ld, int64_t n_rows, const VitTcParams&
     auto kern = vit_attn_tc_kernel<C>;
     static SmemAttrOnce once;  // per instantiation
     if (ensure_dyn_smem(once, kern, C::SMEM_BYTES)) return -12;
-    { lcc::count_launch(); kern<<<grid, 192, C::SMEM_BYTES, s>>>(tq, tkv, p); }
+    { lcc::count_launch(); chained(kern, grid, 192, C::SMEM_BYTES, s)(tq, tkv, p); }
     return 0;
 }
 

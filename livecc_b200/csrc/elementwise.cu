@@ -184,6 +184,7 @@ template <bool RMS, int TEAM, int KEEP>   // KEEP: 16-byte pieces of a row per t
 __global__ void __launch_bounds__(TEAM) norm_rows_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w,
                                                          const bf16* __restrict__ b, bf16* __restrict__ y, int ldy, int rows, int dim,
                                                          float eps) {
+    chain_begin(x);
     __shared__ float red[2][TEAM / 32][32];
     int flip = 0;
     constexpr int STEP = TEAM * 8;
@@ -240,6 +241,7 @@ template <bool RMS>
 __global__ void __launch_bounds__(256) norm_rows_warp_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w,
                                                              const bf16* __restrict__ b, bf16* __restrict__ y, int ldy, int rows, int dim,
                                                              float eps) {
+    chain_begin(x);
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
     const bf16* xr = x + (size_t)row * ldx;
@@ -277,10 +279,10 @@ static int norm_rows(const bf16* x, int ldx, const bf16* w, const bf16* b, bf16*
     lcc::count_launch();
     // (one wave: a CTA walks over further rows with the weights it has, the next row's loads in flight)
     const int sms = kSms;
-    if (dim <= 1536 && rows >= 16 * sms) norm_rows_warp_kernel<RMS><<<(rows + 7) / 8, 256, 0, s>>>(x, ldx, w, b, y, ldy, rows, dim, eps);
-    else if (dim <= 512) norm_rows_kernel<RMS, 64, 1><<<min(rows, 16 * sms), 64, 0, s>>>(x, ldx, w, b, y, ldy, rows, dim, eps);
-    else if (dim <= 1536) norm_rows_kernel<RMS, 192, 1><<<min(rows, 5 * sms), 192, 0, s>>>(x, ldx, w, b, y, ldy, rows, dim, eps);
-    else norm_rows_kernel<RMS, 256, 2><<<min(rows, 3 * sms), 256, 0, s>>>(x, ldx, w, b, y, ldy, rows, dim, eps);
+    if (dim <= 1536 && rows >= 16 * sms) chained(norm_rows_warp_kernel<RMS>, (rows + 7) / 8, 256, 0, s)(x, ldx, w, b, y, ldy, rows, dim, eps);
+    else if (dim <= 512) chained(norm_rows_kernel<RMS, 64, 1>, min(rows, 16 * sms), 64, 0, s)(x, ldx, w, b, y, ldy, rows, dim, eps);
+    else if (dim <= 1536) chained(norm_rows_kernel<RMS, 192, 1>, min(rows, 5 * sms), 192, 0, s)(x, ldx, w, b, y, ldy, rows, dim, eps);
+    else chained(norm_rows_kernel<RMS, 256, 2>, min(rows, 3 * sms), 256, 0, s)(x, ldx, w, b, y, ldy, rows, dim, eps);
     return 0;
 }
 
@@ -303,6 +305,7 @@ int rmsnorm(const bf16* x, int ldx, const bf16* w, bf16* y, int ldy, int rows, i
 __global__ void vit_rope_table_kernel(float* __restrict__ cos_t, float* __restrict__ sin_t, int t, int h,
                                       int w, int merge, int half /* = head_dim/2 */,
                                       const float* __restrict__ inv_freq /* [half/2] */) {
+    chain_begin();
     const int per_frame = h * w;
     const int n = t * per_frame;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -326,7 +329,7 @@ int vit_rope_table(float* cos_t, float* sin_t, int t, int h, int w, int merge, i
     const int half = head_dim / 2;
     const int total = t * h * w * half;
     if (total <= 0) return 0;
-    { lcc::count_launch(); vit_rope_table_kernel<<<(total + 255) / 256, 256, 0, s>>>(cos_t, sin_t, t, h, w, merge, half, inv_freq); }
+    { lcc::count_launch(); chained(vit_rope_table_kernel, (total + 255) / 256, 256, 0, s)(cos_t, sin_t, t, h, w, merge, half, inv_freq); }
     return 0;
 }
 
@@ -334,6 +337,7 @@ int vit_rope_table(float* cos_t, float* sin_t, int t, int h, int w, int merge, i
 // out[i] = x[i]*cos[i] + rot(x)[i]*sin[i], rot(x) = cat(-x[hd/2:], x[:hd/2]); cos[i] = table[i mod hd/2].
 __global__ void vit_rope_apply_kernel(bf16* __restrict__ qkv, int ld, const float* __restrict__ cos_t,
                                       const float* __restrict__ sin_t, int N, int heads, int hd) {
+    chain_begin(qkv, cos_t, sin_t);
     // one thread = 8 consecutive rotation pairs (x[j..j+8), x[j+half..j+half+8)): two 16-byte loads/stores of
     // bf16 and four float4 loads of cos/sin; requires half % 8 == 0 (hd = 80 -> half = 40)
     const int half = hd / 2;
@@ -376,7 +380,7 @@ int vit_rope_apply(bf16* qkv, int ld, const float* cos_t, const float* sin_t, in
     if ((hd / 2) % 8 || ld % 8) return -1;
     const int64_t total = (int64_t)N * 2 * heads * (hd / 16);
     if (total <= 0) return 0;
-    { lcc::count_launch(); vit_rope_apply_kernel<<<(int)((total + 255) / 256), 256, 0, s>>>(qkv, ld, cos_t, sin_t, N, heads, hd); }
+    { lcc::count_launch(); chained(vit_rope_apply_kernel, (int)((total + 255) / 256), 256, 0, s)(qkv, ld, cos_t, sin_t, N, heads, hd); }
     return 0;
 }
 
@@ -386,6 +390,7 @@ int vit_rope_apply(bf16* qkv, int ld, const float* cos_t, const float* sin_t, in
 // Kernel 1 (single CTA) computes the exclusive rank by a block scan; kernel 2 copies rows.
 // ------------------------------------------------------------------------------------------
 __global__ void video_rank_kernel(const __grid_constant__ PrefillStreams ps, int64_t video_id, int* __restrict__ rank) {
+    chain_begin();
     const PrefillStream& st = ps.st[blockIdx.x];
     const int64_t* __restrict__ ids = st.ids;
     const int S = st.S;
@@ -428,6 +433,7 @@ __global__ void video_rank_kernel(const __grid_constant__ PrefillStreams ps, int
 
 __global__ void embed_gather_kernel(const __grid_constant__ PrefillStreams ps, const int* __restrict__ rank, const bf16* __restrict__ table,
                                     bf16* __restrict__ out, int H, int64_t vocab) {
+    chain_begin(rank);
     const int row = blockIdx.x;
     const PrefillStream& st = ps.st[ps.of_row(row)];
     const bf16* __restrict__ video = st.video;
@@ -456,9 +462,9 @@ int embed_gather(const int64_t* ids, const bf16* table, const bf16* video, int n
 int embed_gather_streams(const PrefillStreams& ps, const bf16* table, int64_t video_id, bf16* out, int* rank_ws, int H, int64_t vocab, cudaStream_t s) {
     if (H % 8) return -1;
     lcc::count_launch();
-    video_rank_kernel<<<ps.n, 1024, 0, s>>>(ps, video_id, rank_ws);
+    chained(video_rank_kernel, ps.n, 1024, 0, s)(ps, video_id, rank_ws);
     lcc::count_launch();
-    embed_gather_kernel<<<ps.rows, 128, 0, s>>>(ps, rank_ws, table, out, H, vocab);
+    chained(embed_gather_kernel, ps.rows, 128, 0, s)(ps, rank_ws, table, out, H, vocab);
     return 0;
 }
 
@@ -489,6 +495,7 @@ constexpr int kMropeHeads = 9;
 __global__ void __launch_bounds__(256) mrope_kv_write_kernel(bf16* __restrict__ qkv, int ld, const __grid_constant__ PrefillStreams ps,
                                       const float* __restrict__ inv_freq, MropeSections sec, int Hq, int Hkv,
                                       bf16* __restrict__ kc, bf16* __restrict__ vc, int page_size) {
+    chain_begin(qkv);
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int heads_total = Hq + 2 * Hkv, slices = (heads_total + kMropeHeads - 1) / kMropeHeads;
@@ -556,7 +563,7 @@ int mrope_kv_write_streams(bf16* qkv, int ld, const PrefillStreams& ps, const fl
     const int wpb = 8;
     MropeSections sec{sec_t, sec_h};
     lcc::count_launch();
-    mrope_kv_write_kernel<<<(int)((warps + wpb - 1) / wpb), wpb * 32, 0, s>>>(
+    chained(mrope_kv_write_kernel, (int)((warps + wpb - 1) / wpb), wpb * 32, 0, s)(
         qkv, ld, ps, inv_freq, sec, Hq, Hkv, kc, vc, page_size);
     return 0;
 }

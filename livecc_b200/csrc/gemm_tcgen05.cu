@@ -240,7 +240,7 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmap_a,
                     const __grid_constant__ CUtensorMap tmap_b, bf16* C, int M, int N,
                     int K, int ldc, const bf16* __restrict__ bias,
                     const bf16* residual /* may alias C */, int ldr, int splits_arg /* >= 1 */, const GemmTile cfg,
-                    const int* __restrict__ tile_group /* null: one weight matrix */, int batch, int a_col_stride, int c_col_stride) {
+                    const int* __restrict__ tile_groups /* null: one weight matrix */, int batch, int a_col_stride, int c_col_stride) {
     const int BLOCK_N = cfg.bn;
     const int STAGE_BYTES = A_BYTES + BLOCK_N * BLOCK_K * 2;
     // split-K exists only in the EPI_PARTIAL_F32 instantiations; everywhere else splits is the constant 1 and the
@@ -294,6 +294,8 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmap_a,
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    const int* tile_group = tile_groups;
+    chain_begin(tile_group);   // (barriers, tensor maps and TMEM are ready; only now may the next kernel's CTAs ask for TMEM)
 
     if (warp == 0) {
         // ===================== TMA producer =====================
@@ -467,6 +469,7 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     cluster_sync_all();  // barriers of BOTH CTAs are initialised before any remote arrive / TMA credit
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    chain_begin();
 
     if (warp == 0) {
         // ===================== TMA producer (both CTAs) =====================
@@ -800,6 +803,7 @@ gemm_swap_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     cluster_sync_all();  // barriers of all CTAs are initialised before any remote arrive / TMA credit
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    chain_begin();
 
     if (warp == 0) {
         // ===================== TMA producer (both CTAs) =====================
@@ -1051,9 +1055,8 @@ static int launch_cfg(const GemmArgs& a, int bn, int num_sms, cudaStream_t strea
     int ldr = a.ldr;
     const bf16* bias = (const bf16*)a.bias;
     if (EPI == EPI_CLAMP_GLU) glu_slots(a, ldr, bias);
-    kern<<<grid, 384, cfg.smem_bytes, stream>>>(ta, tb, (bf16*)a.C, a.M, a.N, a.K, a.ldc,
-                                                bias, (const bf16*)a.residual,
-                                                ldr, splits, cfg, a.tile_group, batch, a.a_col_stride, a.c_col_stride);
+    chained(kern, grid, 384, cfg.smem_bytes, stream)(ta, tb, (bf16*)a.C, a.M, a.N, a.K, a.ldc, bias, (const bf16*)a.residual, ldr, splits, cfg,
+                                                     a.tile_group, batch, a.a_col_stride, a.c_col_stride);
     return cudaGetLastError() == cudaSuccess ? 0 : -13;
 }
 
@@ -1074,7 +1077,7 @@ static int launch_cfg2(const GemmArgs& a, int bn, int num_sms, cudaStream_t stre
     int ldr = a.ldr;
     const bf16* bias = (const bf16*)a.bias;
     if (EPI == EPI_CLAMP_GLU) glu_slots(a, ldr, bias);
-    kern<<<2 * pairs, 384, cfg.smem_bytes, stream>>>(ta, tb, (bf16*)a.C, a.M, a.N, a.K, a.ldc, bias, (const bf16*)a.residual, ldr, splits, cfg);
+    chained(kern, 2 * pairs, 384, cfg.smem_bytes, stream)(ta, tb, (bf16*)a.C, a.M, a.N, a.K, a.ldc, bias, (const bf16*)a.residual, ldr, splits, cfg);
     return cudaGetLastError() == cudaSuccess ? 0 : -13;
 }
 
@@ -1146,11 +1149,13 @@ static int launch_swap(const GemmArgs& a, int bm, int splits, int num_sms, cudaS
     lc.blockDim = dim3(384);
     lc.dynamicSmemBytes = cfg.smem_bytes;
     lc.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2 * splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
-    lc.numAttrs = 1;
+    lc.numAttrs = chain_next() ? 2 : 1;
     lcc::count_launch();
     return cudaLaunchKernelEx(&lc, kern, tw, t1, t2, (bf16*)a.C, a.M, a.N, a.K, a.ldc, (const bf16*)a.bias, (const bf16*)a.residual, a.ldr, cfg,
                               a.epi_param, a.epi_alpha, a.epi_up_bias, a.wait_ns ? (unsigned long long)a.wait_ns : kWaitNs, a.fault) == cudaSuccess ? 0 : -13;
@@ -1296,6 +1301,7 @@ static bool choose_swap(int M, int N, int K, int num_sms, double other, int* bm_
 __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, int M, int N,
                                      const bf16* __restrict__ bias, const bf16* residual, int ldr, bf16* C, int ldc,
                                      int epi) {
+    chain_begin(part);
     const int groups = N / 8;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)M * groups) return;
@@ -1376,7 +1382,7 @@ static int run_splitk(const GemmArgs& a, int splits, int num_sms, cudaStream_t s
     if (int r = launch_cfg<EPI_PARTIAL_F32>(p, splitk_width(a), num_sms, stream)) return r;
     const int64_t threads = (int64_t)a.M * (a.N / 8);
     lcc::count_launch();
-    splitk_reduce_kernel<<<(int)((threads + 255) / 256), 256, 0, stream>>>(
+    chained(splitk_reduce_kernel, (int)((threads + 255) / 256), 256, 0, stream)(
         (const float*)a.splitk_ws, splits, a.M, a.N, (const bf16*)a.bias, (const bf16*)a.residual, a.ldr, (bf16*)a.C,
         a.ldc, a.epi);
     return cudaGetLastError() == cudaSuccess ? 0 : -13;

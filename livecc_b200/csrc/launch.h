@@ -53,9 +53,15 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
 // 10 us on one row; as ordinary graph nodes, kernels that return at once cost 2.7 to 4 us each. Chained, and with the first
 // weights of a linear layer loaded before the wait, a prompt of 128 tokens and 31 replayed steps take 8.29 ms for 8.48 (recurrent design, four
 // layers) and 4.86 for 5.14 (routed, two layers), one step launched by the host 0.32 ms for 0.38 and 0.33 for 0.36 (four layers each).
-// Kernels of few and large CTAs (prompt attention: one or two per SM) stay outside: chained, their CTAs go where there is room while the
-// kernel in front still holds the other SMs, and stay there two to an SM. 281 rows behind 4000 tokens of four layers with distance tables
-// took 2.59 ms unchained, 2.76 with every kernel chained, 2.52 now. (An ordinary kernel of a scope lets the one behind it in when it is complete.)
+// Matrix products, row kernels and attention of the vision tower and of a prefill are chained too: what they set up (barriers, tensor memory, tensor
+// maps) and their launch lie beside the kernel in front. A turn that reads 281 tokens behind 17 k 1.42 -> 1.32 ms, 24 behind 8 k 1.00 -> 0.84, eight
+// streams' prefill 2.0 -> 1.6, 1024 and 8192 patches 456 -> 442 and 980 -> 948 us, prompts of the hybrid models 1.72 -> 1.67 and 0.56 -> 0.525 ms.
+// A kernel that takes tensor memory takes it before it opens the door to the next one: that one could otherwise hold what this one waits for.
+// (The first stages' weights asked for before the wait changed little, turn by turn -1 to +0.6 %.) Prompt attention of the hybrid models (few and large
+// CTAs) stays outside: chained, its CTAs go where there is room while the kernel in front still holds the other SMs, and stay there two to an SM.
+// 281 rows behind 4000 tokens of four layers with distance tables took 2.59 ms unchained, 2.76 with every kernel chained, 2.52 now. So do the decoder's
+// decode kernels: each of their thousands of CTAs would pay for the wait with its cached activations (gate/up 44 -> 50 us, lm_head 170 -> 202).
+// (An ordinary kernel of a scope lets the one behind it in when it is complete.)
 // The first launch of a scope and the one after chain_break() (behind a copy, a fork or a join with another stream) are ordinary: whatever
 // was enqueued before is complete when they start. Outside a scope every launch is.
 enum class Chain { off, broken, on };
@@ -68,6 +74,13 @@ struct ChainScope {
     ChainScope& operator=(const ChainScope&) = delete;
 };
 
+// Is the launch that comes next chained? (Asked once for each launch of a scope.)
+inline bool chain_next() {
+    const bool chain = t_chain == Chain::on;
+    if (t_chain == Chain::broken) t_chain = Chain::on;
+    return chain;
+}
+
 template <typename... KArgs>
 struct ChainLaunch {
     void (*kern)(KArgs...);
@@ -76,9 +89,7 @@ struct ChainLaunch {
     cudaStream_t s;
     template <typename... Args>
     void operator()(Args... args) const {
-        const bool chain = t_chain == Chain::on;
-        if (t_chain == Chain::broken) t_chain = Chain::on;
-        launch_kernel(kern, grid, block, smem, s, chain, args...);   // (an error stays in cudaGetLastError, as with <<<>>>)
+        launch_kernel(kern, grid, block, smem, s, chain_next(), args...);   // (an error stays in cudaGetLastError, as with <<<>>>)
     }
 };
 template <typename... KArgs>

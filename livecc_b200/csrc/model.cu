@@ -9,6 +9,7 @@
 
 #include "../../include/livecc_b200.h"
 #include "cabi_common.h"
+#include "common.cuh"
 #include "gemm.h"
 #include "launch.h"
 #include "mega.h"
@@ -102,6 +103,7 @@ WsLayout make_layout(const lcc_model_config& c, int NP, int NT) {
 }
 
 __global__ void fill_cu_seqlens_kernel(int* cu, int t, int hw) {
+    lcc::chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= t) cu[i] = i * hw;
 }
@@ -221,6 +223,7 @@ static int vit_forward_impl(lcc_model* m, const float* pixel_values, const uint8
     float* vcos = (float*)(ws + L.vcos); float* vsin = (float*)(ws + L.vsin);
     int* vcu = (int*)(ws + L.vcu);
     const int dim = c.vit_dim, hd = dim / c.vit_heads;
+    const lcc::ChainScope chain;
 
     if (frames) {
         if (c.patch_dim != 1176) LCC_FAIL(m->ctx, -4, "frame ingest is specialised for 3x2x14x14 patches");
@@ -232,7 +235,7 @@ static int vit_forward_impl(lcc_model* m, const float* pixel_values, const uint8
               lcc::EPI_NONE, s), "vit patch_embed");
     STEP(lcc::vit_rope_table(vcos, vsin, t, h, w, c.merge, hd, m->w.vit_inv_freq, s), "vit rope table");
     lcc::count_launch();
-    fill_cu_seqlens_kernel<<<(t + 256) / 256, 256, 0, s>>>(vcu, t, h * w);
+    lcc::chained(fill_cu_seqlens_kernel, (t + 256) / 256, 256, 0, s)(vcu, t, h * w);
     for (int i = 0; i < c.vit_depth; ++i) {
         const lcc_vit_block_weights& b = m->vit_blocks[i];
         STEP(lcc::layernorm(vh, dim, (const bf16*)b.norm1_w, (const bf16*)b.norm1_b, vn, dim, N, dim, 1e-6f, s), "vit norm1");
@@ -334,6 +337,7 @@ static int prefill_impl(lcc_model* m, const lcc_prefill_request* rq, int n, cons
         return 0;
     };
     Runs r_qkv{}, r_o{}, r_gu{}, r_down{};
+    const lcc::ChainScope chain;
     STEP(lcc::embed_gather_streams(ps, (const bf16*)m->w.embed, c.video_token_id, hid, rank, H, c.vocab, s), "embed gather");
     for (int i = 0; i < c.layers; ++i) {
         const lcc_layer_weights& lw = m->layers[i];
