@@ -102,22 +102,18 @@ __global__ void chunk_cumsum_kernel(ChunkArgs a, SeqPos pos) {
 }
 
 // ---- 2: M[t, s] -------------------------------------------------------------------------------------------------------
-template <typename T, bool VEC>
+// A decay per head: the product c k^T is the same for every head of a group, so a CTA forms it once per group and writes one decayed copy per head.
+template <typename T>
 __global__ void __launch_bounds__(256) chunk_weights_kernel(ChunkArgs a, SeqPos pos) {
     chain_begin();
     if (seq_done(pos)) return;
-    __shared__ float sc_[KS][PAD], sk_[KS][PAD], sb_[KS][PAD];
-    // a decay per head: the product c k^T is the same for every head of a group, so a CTA forms it once per group and
-    // writes one decayed copy per head; a decay per key channel: one CTA per head
-    const int blk = blockIdx.x, g = VEC ? blockIdx.y / a.heads_per_group : blockIdx.y;
-    const int h_first = VEC ? blockIdx.y : g * a.heads_per_group, h_count = VEC ? 1 : a.heads_per_group;
-    const int h = h_first;
+    __shared__ float sc_[KS][PAD], sk_[KS][PAD];
+    const int blk = blockIdx.x, g = blockIdx.y;
     const int t0 = blk * CL, len = min(CL, a.S - t0);
-    const int N = a.N, ncol = a.heads * a.NV;
+    const int N = a.N, ncol = a.heads;
     const int ty = threadIdx.x / 16, tx = threadIdx.x % 16, tm = ty * 4, tn = tx * 4;
     const T* gc = (const T*)a.c + (size_t)(a.row0 + t0) * a.ld_c + (size_t)g * N;
     const T* gk = (const T*)a.k + (size_t)(a.row0 + t0) * a.ld_k + (size_t)g * N;
-    const float* gb = a.la + (size_t)(a.row0 + t0) * ncol + (size_t)h * a.NV;
     const bool live = tn <= tm + 3;            // tiles wholly above the diagonal stay zero
     float acc[4][4] = {};
     for (int n0 = 0; n0 < N; n0 += KS) {
@@ -128,31 +124,23 @@ __global__ void __launch_bounds__(256) chunk_weights_kernel(ChunkArgs a, SeqPos 
             const bool ok = r < len && n < N;
             sc_[kk][r] = ok ? ldf(gc + (size_t)r * a.ld_c + n) : 0.f;
             sk_[kk][r] = ok ? ldf(gk + (size_t)r * a.ld_k + n) : 0.f;
-            if (VEC) sb_[kk][r] = ok ? gb[(size_t)r * ncol + n] : 0.f;
         }
         __syncthreads();
         if (!live) continue;
 #pragma unroll 4
         for (int kk = 0; kk < KS; ++kk) {
-            float cv[4], kv[4], bt[4], bs[4];
+            float cv[4], kv[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) { cv[i] = sc_[kk][tm + i]; kv[i] = sk_[kk][tn + i]; }
-            if (VEC) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) { bt[i] = sb_[kk][tm + i]; bs[i] = sb_[kk][tn + i]; }
-            }
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (VEC) acc[i][j] = fmaf(cv[i] * kv[j], expf(fminf(bt[i] - bs[j], 0.f)), acc[i][j]);
-                    else acc[i][j] = fmaf(cv[i], kv[j], acc[i][j]);
-                }
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(cv[i], kv[j], acc[i][j]);
         }
     }
-    for (int hh = h_first; hh < h_first + h_count; ++hh) {
+    for (int hh = g * a.heads_per_group; hh < (g + 1) * a.heads_per_group; ++hh) {
         float* out = a.ws_m + ((size_t)blk * a.heads + hh) * CL * CL;
-        const float* hb = a.la + (size_t)(a.row0 + t0) * ncol + (size_t)hh * a.NV;
+        const float* hb = a.la + (size_t)(a.row0 + t0) * ncol + hh;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int t = tm + i;
@@ -162,11 +150,120 @@ __global__ void __launch_bounds__(256) chunk_weights_kernel(ChunkArgs a, SeqPos 
                 float v = 0.f;
                 if (s <= t && t < len) {
                     v = acc[i][j] * a.cs * (a.sc ? a.sc[(size_t)(a.row0 + t0 + s) * a.heads + hh] : 1.f);
-                    if (!VEC) v *= expf(fminf(hb[(size_t)t * ncol] - hb[(size_t)s * ncol], 0.f));
+                    v *= expf(fminf(hb[(size_t)t * ncol] - hb[(size_t)s * ncol], 0.f));
                 }
                 out[t * CL + s] = v;
             }
         }
+    }
+}
+
+// A decay per key channel, a CTA per head and block. An exponential per (t, s, n) costs 2080 a channel (145 us for 2048 rows, 8 heads, 128 channels, bound by
+// their instructions; warps on the diagonal ran the half above it too). But exp(b_t - b_s) = exp(b_t - b_m) exp(b_m - b_s) for any m between s and t, and neither
+// exponent is positive: halves of 64, 32, 16 and 8 rows meet in plain products of rows decayed to the first row of the upper half (64 exponentials per level and
+// channel, 1920 of the 2080 weights), and only the tiles of 4 rows on the diagonal keep one per weight (160). Where a factor leaves fp32's normal range the weight
+// is below 2^-126 of its c k. Each 128 threads take a quarter of a slab's 16 channels, and the four sums are added at the end. 26 us (41 with 256 threads and
+// diagonal tiles of 8 rows, 28 with the latter): latency of a slab's loads, exponentials and products behind three barriers.
+template <typename T>
+__global__ void __launch_bounds__(512, 2) chunk_weights_vec_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
+    if (seq_done(pos)) return;
+    constexpr int LEVELS = 4;
+    __shared__ __align__(16) float sh[3 + LEVELS][KS][PAD];   // c, k, cumulative decays; rows decayed per level (upper half: c, lower: k). At the end: the weights
+    auto& sc_ = sh[0]; auto& sk_ = sh[1]; auto& sb_ = sh[2];
+    const int blk = blockIdx.x, h = blockIdx.y, g = h / a.heads_per_group;
+    const int t0 = blk * CL, len = min(CL, a.S - t0), N = a.N, ncol = a.heads * N;
+    const T* gc = (const T*)a.c + (size_t)(a.row0 + t0) * a.ld_c + (size_t)g * N;
+    const T* gk = (const T*)a.k + (size_t)(a.row0 + t0) * a.ld_k + (size_t)g * N;
+    const float* gb = a.la + (size_t)(a.row0 + t0) * ncol + (size_t)h * N;
+    const int part = threadIdx.x >> 7, q = (threadIdx.x ^ (part & 1 ? 127 : 0)) & 127;   // (mirrored, so that no scheduler has all the diagonals)
+    int lv = 0, tm = 0, tn = 0;                               // a thread's 4 x 4 weights below the diagonal tiles (120 of 128 threads)
+    if (q < 64) { lv = 0; tm = 32 + (q >> 3) * 4; tn = (q & 7) * 4; }
+    else if (q < 96) { lv = 1; tm = ((q >> 4) & 1) * 32 + 16 + ((q >> 2) & 3) * 4; tn = ((q >> 4) & 1) * 32 + (q & 3) * 4; }
+    else if (q < 112) { lv = 2; tm = ((q >> 2) & 3) * 16 + 8 + ((q >> 1) & 1) * 4; tn = ((q >> 2) & 3) * 16 + (q & 1) * 4; }
+    else if (q < 120) { lv = 3; tm = (q & 7) * 8 + 4; tn = (q & 7) * 8; }
+    const int dq = (127 - q) / 3, dr = (127 - q) % 3, dt = q >= 80 ? dq * 4 + (dr ? 2 : 0) : 0, ds = q >= 80 ? dq * 4 + (dr == 2 ? 2 : 0) : CL;   // (CL: none)   // and its 2 x 2 on the diagonal
+    float2 acc[2][4] = {};                                    // rows (2 i, 2 i + 1) x column j
+    float diag[2][2] = {};
+    float pc[2], pk[2], pb[2];
+    auto fetch = [&](int n0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int e = threadIdx.x + i * 512, r = e / KS, n = n0 + e % KS;
+            const bool ok = r < len && n < N;
+            pc[i] = ok ? ldf(gc + (size_t)r * a.ld_c + n) : 0.f;
+            pk[i] = ok ? ldf(gk + (size_t)r * a.ld_k + n) : 0.f;
+            pb[i] = ok ? gb[(size_t)r * ncol + n] : 0.f;
+        }
+    };
+    fetch(0);
+    for (int n0 = 0; n0 < N; n0 += KS) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int e = threadIdx.x + i * 512, r = e / KS, kk = e % KS;
+            sc_[kk][r] = pc[i]; sk_[kk][r] = pk[i]; sb_[kk][r] = pb[i];
+        }
+        __syncthreads();
+        if (n0 + KS < N) fetch(n0 + KS);
+#pragma unroll
+        for (int l = 0; l < LEVELS; ++l) {
+            const int L = 32 >> l, r = threadIdx.x & 63, m = (r & ~(2 * L - 1)) + L;
+            const bool up = r & L;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int kk = (threadIdx.x >> 6) + i * 8;
+                const float d = sb_[kk][r] - sb_[kk][m];
+                sh[3 + l][kk][r] = (up ? sc_[kk][r] : sk_[kk][r]) * expf(fminf(up ? d : -d, 0.f));
+            }
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int i8 = 0; i8 < KS / 4; ++i8) {
+            const int kk = part * (KS / 4) + i8;
+            if (q < 120) {
+                const float4 x = *reinterpret_cast<const float4*>(&sh[3 + lv][kk][tm]), y = *reinterpret_cast<const float4*>(&sh[3 + lv][kk][tn]);
+                const float yj[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc[0][j] = __ffma2_rn(make_float2(x.x, x.y), make_float2(yj[j], yj[j]), acc[0][j]);
+                    acc[1][j] = __ffma2_rn(make_float2(x.z, x.w), make_float2(yj[j], yj[j]), acc[1][j]);
+                }
+            }
+            if (ds <= dt) {
+                const float2 c2 = *reinterpret_cast<const float2*>(&sc_[kk][dt]), bt = *reinterpret_cast<const float2*>(&sb_[kk][dt]);
+                const float2 k2 = *reinterpret_cast<const float2*>(&sk_[kk][ds]), bs = *reinterpret_cast<const float2*>(&sb_[kk][ds]);
+                diag[0][0] = fmaf(c2.x * k2.x, expf(fminf(bt.x - bs.x, 0.f)), diag[0][0]);
+                diag[0][1] = fmaf(c2.x * k2.y, expf(fminf(bt.x - bs.y, 0.f)), diag[0][1]);
+                diag[1][0] = fmaf(c2.y * k2.x, expf(fminf(bt.y - bs.x, 0.f)), diag[1][0]);
+                diag[1][1] = fmaf(c2.y * k2.y, expf(fminf(bt.y - bs.y, 0.f)), diag[1][1]);
+            }
+        }
+    }
+    float (*w)[PAD] = reinterpret_cast<float (*)[PAD]>(&sh[0][0][0]);   // [t][s], what lies above the diagonal is not read
+    static_assert((3 + LEVELS) * KS >= CL, "the weights fit");
+    auto each = [&](auto put) {
+        if (q < 120)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) put(w[tm + i][tn + j], (i & 1) ? acc[i >> 1][j].y : acc[i >> 1][j].x);
+        if (ds <= dt)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) put(w[dt + i][ds + j], diag[i][j]);
+    };
+    __syncthreads();
+    for (int p = 0; p < 4; ++p) {
+        if (part == p) each([p](float& x, float v) { x = p ? x + v : v; });
+        __syncthreads();
+    }
+    float* out = a.ws_m + ((size_t)blk * a.heads + h) * CL * CL;
+    const float* gsc = a.sc ? a.sc + (size_t)(a.row0 + t0) * a.heads + h : nullptr;
+    for (int e = threadIdx.x; e < CL * CL; e += 512) {
+        const int t = e / CL, s = e % CL;
+        out[e] = s <= t && t < len ? w[t][s] * a.cs * (gsc ? gsc[(size_t)s * a.heads] : 1.f) : 0.f;
     }
 }
 
@@ -351,6 +448,10 @@ template <> struct Row16<float> {
         v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
     }
 };
+__device__ __forceinline__ void ld4f(const float* p, float* v) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
 // dst[k][r] = src[r][k0 + k] * f(r) for 64 tile rows (zero from `rows` on) and k < 64 (zero from `cols` on): rows contiguous along k
 template <typename T, typename F>
 __device__ __forceinline__ void slab_across(float (*dst)[SP], const T* src, int ld, int rows, int k0, int cols, F f) {
@@ -735,6 +836,212 @@ __global__ void __launch_bounds__(128, 5) chunk_state_tc_kernel(ChunkArgs a, Seq
     }
 }
 
+// The same for a decay per key channel: the decayed k is the operand that is cut, once per 64 key channels and for all value channels (u as it is).
+// 2048 rows, 8 heads of 256 x 128: 25 us for 55 of chunk_state_kernel, which formed every decayed k once per 64 value channels.
+__device__ __noinline__ void state_vec_plain(const ChunkArgs& a, const bf16* u, const bf16* k, const float* b, const float* sc, float* out, int len, int P, int cols) {
+    const int ncol = a.heads * a.N;
+    for (int e = threadIdx.x; e < P * cols; e += blockDim.x) {
+        const int p = e / cols, n = e % cols;
+        float acc = 0.f;
+        for (int s = 0; s < len; ++s) {
+            const float f = expf(fminf(b[(size_t)(len - 1) * ncol + n] - b[(size_t)s * ncol + n], 0.f)) * (sc ? sc[(size_t)s * a.heads] : 1.f);
+            acc = fmaf(bf2f(u[(size_t)s * a.ld_u + p]), bf2f(k[(size_t)s * a.ld_k + n]) * f, acc);
+        }
+        out[(size_t)p * a.N + n] = acc;
+    }
+}
+__global__ void __launch_bounds__(128, 5) chunk_state_vec_tc_kernel(const __grid_constant__ ChunkArgs a, SeqPos pos) {
+    chain_begin();
+    if (seq_done(pos)) return;
+    __shared__ __align__(16) bf16 sk[3][CL][UP], su[CL][UP];   // [row s][n], cut in three; [row s][p]
+    const int blk = blockIdx.x / a.heads, h = blockIdx.x % a.heads, g = h / a.heads_per_group;
+    const int n0 = blockIdx.y * TS, N = a.N, P = a.P, ncol = a.heads * N;
+    const int t0 = blk * CL, len = min(CL, a.S - t0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, tq = lane & 3;
+    const bf16* gu = (const bf16*)a.u + (size_t)(a.row0 + t0) * a.ld_u + (size_t)h * P;
+    const bf16* gk = (const bf16*)a.k + (size_t)(a.row0 + t0) * a.ld_k + (size_t)g * N + n0;
+    const float* gb = a.la + (size_t)(a.row0 + t0) * ncol + (size_t)h * N + n0;
+    const float* gsc = a.sc ? a.sc + (size_t)(a.row0 + t0) * a.heads + h : nullptr;
+    float* out = a.ws_s + ((size_t)blk * a.heads + h) * P * N + n0;
+    {
+        const int c = (threadIdx.x & 7) * 8;                    // a thread's 8 key channels, of every 16th row
+        const bool in = n0 + c < N;
+        float last[8] = {};
+        if (in) { ld4f(gb + (size_t)(len - 1) * ncol + c, last); ld4f(gb + (size_t)(len - 1) * ncol + c + 4, last + 4); }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = (threadIdx.x >> 3) + i * 16;
+            uint32_t q[3][4] = {};
+            if (r < len && in) {
+                float kv[8], b[8];
+                Row16<bf16>::load(gk + (size_t)r * a.ld_k + c, kv);
+                ld4f(gb + (size_t)r * ncol + c, b); ld4f(gb + (size_t)r * ncol + c + 4, b + 4);
+                const float f = gsc ? gsc[(size_t)r * a.heads] : 1.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t t[3];
+                    cut3(kv[2 * j] * (expf(fminf(last[2 * j] - b[2 * j], 0.f)) * f), kv[2 * j + 1] * (expf(fminf(last[2 * j + 1] - b[2 * j + 1], 0.f)) * f), t);
+                    q[0][j] = t[0]; q[1][j] = t[1]; q[2][j] = t[2];
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) *reinterpret_cast<uint4*>(&sk[k][r][c]) = make_uint4(q[k][0], q[k][1], q[k][2], q[k][3]);
+        }
+    }
+    for (int p0 = 0; p0 < P; p0 += TS) {
+        uint4 ur[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int e = threadIdx.x + i * 128, r = e >> 3, c = (e & 7) * 8;
+            ur[i] = r < len && p0 + c < P ? *reinterpret_cast<const uint4*>(gu + (size_t)r * a.ld_u + p0 + c) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        if (p0) __syncthreads();
+        __nv_bfloat162 most = __float2bfloat162_rn(0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int e = threadIdx.x + i * 128;
+            *reinterpret_cast<uint4*>(&su[e >> 3][(e & 7) * 8]) = ur[i];
+            absmax8(most, ur[i]);
+        }
+        if (__syncthreads_or(!isfinite(__low2float(most)) || !isfinite(__high2float(most)))) {
+            state_vec_plain(a, gu + p0, gk, gb, gsc, out + (size_t)p0 * N, len, min(TS, P - p0), min(TS, N - n0));
+            continue;
+        }
+        float acc[8][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < CL; ks += 16) {
+            uint32_t w[4];
+            ldmatrix_x4_trans(w[0], w[1], w[2], w[3], &su[ks + (lane & 7) + (lane >> 4) * 8][warp * 16 + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float d[2][4] = {};
+#pragma unroll
+                for (int k = 2; k >= 0; --k) {
+                    uint32_t b[4];
+                    ldmatrix_x4_trans(b[0], b[1], b[2], b[3], &sk[k][ks + (lane & 7) + ((lane >> 3) & 1) * 8][j * 16 + (lane >> 4) * 8]);
+                    mma_bf16_16816(d[0], w, b[0], b[1]);
+                    mma_bf16_16816(d[1], w, b[2], b[3]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { acc[2 * j][e] += d[0][e]; acc[2 * j + 1][e] += d[1][e]; }
+            }
+        }
+        const int p = p0 + warp * 16 + gq;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int n = j * 8 + 2 * tq;
+            if (n0 + n >= N) continue;
+            if (p < P) *reinterpret_cast<float2*>(out + (size_t)p * N + n) = make_float2(acc[j][0], acc[j][1]);
+            if (p + 8 < P) *reinterpret_cast<float2*>(out + (size_t)(p + 8) * N + n) = make_float2(acc[j][2], acc[j][3]);
+        }
+    }
+}
+
+// Outputs for a decay per key channel: both operands of the product with the state are fp32 (the decays differ along n), so it stays on the CUDA cores:
+// packed fp32 pairs, 8 x (4 NJ) of a tile of 64 rows x 64 NJ channels per thread, so that 16 bytes read from shared memory feed 8 NJ / (2 + NJ) packed products.
+// Slabs of 32: rows of 16-byte pieces are swizzled, so that neither the transposing stores nor the reads meet in a bank.
+// 2048 rows, 8 heads of 256 x 128: 49 us for 79 of chunk_output_kernel (50 in tiles of 64 channels, 54 with three CTAs per SM and no spill).
+template <typename T, int NJ>
+__global__ void __launch_bounds__(128, 4) chunk_output_vec_kernel(ChunkArgs a, SeqPos pos) {
+    chain_begin();
+    if (seq_done(pos)) return;
+    constexpr int D = 32, TP = 64 * NJ, V = Row16<T>::N;
+    __shared__ __align__(16) float sa[D][CL], sb[D][TP];       // [depth][row t], [depth][channel p], swizzled
+    auto at = [](int k, int x) { return x ^ (((k >> 2) & 7) << 2); };
+    const int blk = blockIdx.x / a.heads, h = blockIdx.x % a.heads, g = h / a.heads_per_group;
+    const int p0 = blockIdx.y * TP, t0 = blk * CL, len = min(CL, a.S - t0), N = a.N, P = a.P, ncol = a.heads * N;
+    const T* gu = (const T*)a.u + (size_t)(a.row0 + t0) * a.ld_u + (size_t)h * P + p0;
+    const T* gc = (const T*)a.c + (size_t)(a.row0 + t0) * a.ld_c + (size_t)g * N;
+    const float* gb = a.la + (size_t)(a.row0 + t0) * ncol + (size_t)h * N;
+    const float* sin = a.ws_s + (((size_t)blk * a.heads + h) * P + p0) * N;
+    const float* gm = a.ws_m + ((size_t)blk * a.heads + h) * CL * CL;
+    const int tm = (threadIdx.x >> 4) * 8, tn = (threadIdx.x & 15) * 4;
+    float2 acc[4][4 * NJ] = {};                                // rows (2 i, 2 i + 1) x column j
+    auto product = [&] {
+#pragma unroll 4
+        for (int k = 0; k < D; ++k) {
+            const float4 a0 = *reinterpret_cast<const float4*>(&sa[k][at(k, tm)]), a1 = *reinterpret_cast<const float4*>(&sa[k][at(k, tm + 4)]);
+            const float2 ar[4] = {make_float2(a0.x, a0.y), make_float2(a0.z, a0.w), make_float2(a1.x, a1.y), make_float2(a1.z, a1.w)};
+#pragma unroll
+            for (int m = 0; m < NJ; ++m) {
+                const float4 b4 = *reinterpret_cast<const float4*>(&sb[k][at(k, tn) + 64 * m]);
+                const float bj[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[i][4 * m + j] = __ffma2_rn(ar[i], make_float2(bj[j], bj[j]), acc[i][4 * m + j]);
+            }
+        }
+    };
+    for (int n0 = 0; n0 < N; n0 += D) {        // the entering state, seen through the decayed queries
+        __syncthreads();
+#pragma unroll
+        for (int e = threadIdx.x; e < CL * (D / V); e += 128) {
+            const int r = e / (D / V), k = (e % (D / V)) * V;
+            float v[V] = {};
+            if (r < len && n0 + k < N) {
+                float b[V];
+                Row16<T>::load(gc + (size_t)r * a.ld_c + n0 + k, v);
+#pragma unroll
+                for (int i = 0; i < V; i += 4) ld4f(gb + (size_t)r * ncol + n0 + k + i, b + i);
+#pragma unroll
+                for (int i = 0; i < V; ++i) v[i] = a.cs * v[i] * expf(b[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < V; ++i) sa[k + i][at(k + i, r)] = v[i];
+        }
+#pragma unroll
+        for (int e = threadIdx.x; e < TP * (D / 4); e += 128) {
+            const int r = e / (D / 4), k = (e % (D / 4)) * 4;
+            float v[4] = {};
+            if (p0 + r < P && n0 + k < N) ld4f(sin + (size_t)r * N + n0 + k, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sb[k + i][at(k + i, r)] = v[i];
+        }
+        __syncthreads();
+        product();
+    }
+    for (int s0 = 0; s0 < len; s0 += D) {      // the block's own rows (their weights hold cs, the step scales and the decays)
+        __syncthreads();
+#pragma unroll
+        for (int e = threadIdx.x; e < CL * (D / 4); e += 128) {
+            const int r = e / (D / 4), k = (e % (D / 4)) * 4;
+            float v[4];
+            ld4f(gm + r * CL + s0 + k, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sa[k + i][at(k + i, r)] = v[i];
+        }
+#pragma unroll
+        for (int e = threadIdx.x; e < D * (TP / V); e += 128) {
+            const int k = e / (TP / V), c = (e % (TP / V)) * V;
+            float v[V] = {};
+            if (s0 + k < len && p0 + c < P) Row16<T>::load(gu + (size_t)(s0 + k) * a.ld_u + c, v);
+#pragma unroll
+            for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(&sb[k][at(k, c + i)]) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+        }
+        __syncthreads();
+        product();
+    }
+    const float skip = a.skip ? a.skip[h] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = tm + i;
+        if (t >= len) continue;
+#pragma unroll
+        for (int m = 0; m < NJ; ++m) {
+            const int p = tn + 64 * m;
+            if (p0 + p >= P) continue;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[j] = (i & 1) ? acc[i >> 1][4 * m + j].y : acc[i >> 1][4 * m + j].x;
+                if (a.skip) v[j] += skip * ldf(gu + (size_t)t * a.ld_u + p + j);
+            }
+            *reinterpret_cast<float4*>(a.y + (size_t)(a.row0 + t0 + t) * a.ld_y + (size_t)h * P + p0 + p) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+    }
+}
+
 // a warp: all 64 rows of 16 of the tile's channels, so that every state is cut once
 __global__ void __launch_bounds__(128, 4) chunk_output_tc_kernel(const __grid_constant__ ChunkArgs a, SeqPos pos) {
     chain_begin();
@@ -862,10 +1169,11 @@ int run_chunked(const ScanArgs& s, SeqPos pos, cudaStream_t st) {
         const int ncol = a.heads * a.NV;
         count_launch();
         chained(chunk_cumsum_kernel, dim3(nb, (ncol + 127) / 128), 128, 0, st)(a, pos);
+        constexpr int V = Row16<T>::N;
+        const bool rows16 = ((s.N | s.P | s.ld_k | s.ld_c | s.ld_u) % V) == 0 && ((s.N | s.P | s.ld_y) % 4) == 0 &&
+                            (((uintptr_t)s.k | (uintptr_t)s.c | (uintptr_t)s.u | (uintptr_t)s.y | (uintptr_t)s.state | (uintptr_t)a.ws_m | (uintptr_t)a.ws_s) % 16) == 0 &&
+                            (!VEC || ((uintptr_t)s.a % 16) == 0);
         if constexpr (!VEC) {
-            constexpr int V = Row16<T>::N;
-            const bool rows16 = ((s.N | s.P | s.ld_k | s.ld_c | s.ld_u) % V) == 0 && ((s.N | s.P | s.ld_y) % 4) == 0 &&
-                                (((uintptr_t)s.k | (uintptr_t)s.c | (uintptr_t)s.u | (uintptr_t)s.y | (uintptr_t)s.state | (uintptr_t)a.ws_m | (uintptr_t)a.ws_s) % 16) == 0;
             if (rows16) {
                 const dim3 tiles(nb * s.heads, (s.P + TS - 1) / TS), pairs(nb, s.heads / s.heads_per_group);
                 const unsigned prefix = (unsigned)((per_state / 4 + 255) / 256);
@@ -884,13 +1192,25 @@ int run_chunked(const ScanArgs& s, SeqPos pos, cudaStream_t st) {
                 continue;
             }
         }
-        count_launch();
-        chained(chunk_weights_kernel<T, VEC>, dim3(nb, VEC ? s.heads : s.heads / s.heads_per_group), 256, 0, st)(a, pos);
-        count_launch();
-        chained(chunk_state_kernel<T, VEC>, dim3(nb * s.heads, (s.P + TS - 1) / TS, (s.N + TS - 1) / TS), 256, 0, st)(a, pos);
-        count_launch();
+        for (int i = 0; i < 4; ++i) count_launch();
+        if constexpr (VEC) chained(chunk_weights_vec_kernel<T>, dim3(nb, s.heads), 512, 0, st)(a, pos);
+        else chained(chunk_weights_kernel<T>, dim3(nb, s.heads / s.heads_per_group), 256, 0, st)(a, pos);
+        bool state_done = false;
+        if constexpr (VEC && std::is_same_v<T, bf16>) {
+            if (rows16) {
+                chained(chunk_state_vec_tc_kernel, dim3(nb * s.heads, (s.N + TS - 1) / TS), 128, 0, st)(a, pos);
+                state_done = true;
+            }
+        }
+        if (!state_done) chained(chunk_state_kernel<T, VEC>, dim3(nb * s.heads, (s.P + TS - 1) / TS, (s.N + TS - 1) / TS), 256, 0, st)(a, pos);
         chained(chunk_prefix_kernel<VEC>, (unsigned)((per_state + 255) / 256), 256, 0, st)(a, nb, pos);
-        count_launch();
+        if constexpr (VEC) {
+            if (rows16) {   // channels in tiles of 128 where a head has more than 64
+                if (s.P > 64) chained(chunk_output_vec_kernel<T, 2>, dim3(nb * s.heads, (s.P + 127) / 128), 128, 0, st)(a, pos);
+                else chained(chunk_output_vec_kernel<T, 1>, dim3(nb * s.heads, 1), 128, 0, st)(a, pos);
+                continue;
+            }
+        }
         chained(chunk_output_kernel<T, VEC>, dim3(nb * s.heads, (s.P + TS - 1) / TS), 256, 0, st)(a, pos);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -100;
