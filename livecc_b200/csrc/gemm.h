@@ -22,6 +22,7 @@ enum GemmEpilogue {
                              // C[:, j] = bf16(g * sigmoid(alpha g) * (u + up_bias)) in fp32 on the accumulators; limit = epi_param,
                              // alpha = epi_alpha, up_bias = epi_up_bias (1, 0 and an infinite limit: silu(gate) * up)
     EPI_GELU_ERF = 11,       // C = bf16(gelu_erf(acc)), the activation in fp32 on the accumulator
+    EPI_LOGITS_F32 = 13,     // internal (GemmArgs::logits): c = cap * tanh(acc / cap) * scale in fp32, stored as EPI_PARTIAL_F32 does with one split
     EPI_SIGMOID_GATE = 12,   // C = bf16(acc * sigmoid(residual)): the residual slot carries gate logits (batched: product z reads its columns
                              // z * c_col_stride .. , as it writes C)
 };
@@ -53,6 +54,9 @@ struct GemmArgs {
     int a_col_stride = 0, c_col_stride = 0;
     // fp32 output: C is float [M, ldc] (ldc a multiple of 4), epi must be EPI_NONE
     bool c_f32 = false;
+    // fp32 output of one plain product as logits: c = softcap(acc) * logit_scale (logit_cap <= 0: none)
+    bool logits = false;
+    float logit_cap = 0.f, logit_scale = 1.f;
     float epi_param = 0.f;   // EPI_CLAMP_GLU: the clamp
     float epi_alpha = 1.702f, epi_up_bias = 1.f;
     // kernels with bounded waits (the swapped form): a host-visible word that they set when a signal did not come, or null; the limit in ns, 0 = 2 s

@@ -114,11 +114,18 @@ __device__ __forceinline__ void quad_transpose(uint4 (&p)[4], int lane) {
     swap_pieces(p[0], p[2], 2, lane); swap_pieces(p[1], p[3], 2, lane);
 }
 
+// the logits' cap, its inverse and the scale ride in the slots of the residual's stride and the bias, which they have not (set_logit_slots)
+struct LogitSlots { float cap, inv_cap, scale; };
+__device__ __forceinline__ LogitSlots logit_slots(const bf16* bias, int ldr) {
+    const uint64_t b = reinterpret_cast<uint64_t>(bias);
+    return {__int_as_float(ldr), __uint_as_float((uint32_t)b), __uint_as_float((uint32_t)(b >> 32))};
+}
+
 template <int EPI>
 __device__ __forceinline__ void epilogue_chunk(const uint32_t (&v)[32], const EpiFetch& f, bf16* C, int ldc, int M, int row0, int lane, int col0,
                                                int tile_end, int ks, const bf16* __restrict__ bias, const bf16* residual,
                                                int ldr) {
-    if (EPI == EPI_PARTIAL_F32) {
+    if (EPI == EPI_PARTIAL_F32 || EPI == EPI_LOGITS_F32) {
         // fp32 partial tile of split ks: P[ks][row][col] (C is the partial buffer, ldc == N)
         float* base = reinterpret_cast<float*>(C) + (size_t)ks * M * (size_t)ldc;
 #pragma unroll
@@ -131,7 +138,17 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&v)[32], const Ep
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int row = row0 + (lane & ~3) + k;
-                if (row < M && col < tile_end) *reinterpret_cast<uint4*>(base + (size_t)row * ldc + col) = p[k];
+                if (row < M && col < tile_end) {
+                    if (EPI == EPI_LOGITS_F32) {
+                        const LogitSlots l = logit_slots(bias, ldr);
+                        auto store = [&](uint32_t x) {
+                            const float y = __uint_as_float(x);
+                            return __float_as_uint((l.cap > 0.f ? l.cap * tanhf(y * l.inv_cap) : y) * l.scale);
+                        };
+                        p[k] = make_uint4(store(p[k].x), store(p[k].y), store(p[k].z), store(p[k].w));
+                    }
+                    *reinterpret_cast<uint4*>(base + (size_t)row * ldc + col) = p[k];
+                }
             }
         }
     } else if (EPI == EPI_SWIGLU || EPI == EPI_CLAMP_GLU) {
@@ -1036,6 +1053,12 @@ static void glu_slots(const GemmArgs& a, int& ldr, const bf16*& bias) {
     memcpy(&bias, ab, sizeof(ab));
 }
 
+static void set_logit_slots(const GemmArgs& a, int& ldr, const bf16*& bias) {
+    const float cap = a.logit_cap > 0.f ? a.logit_cap : 0.f, is[2] = {cap > 0.f ? 1.f / cap : 0.f, a.logit_scale};
+    memcpy(&ldr, &cap, sizeof(int));
+    memcpy(&bias, is, sizeof(is));
+}
+
 template <int EPI>
 static int launch_cfg(const GemmArgs& a, int bn, int num_sms, cudaStream_t stream) {
     const GemmTile cfg = make_tile(bn);
@@ -1055,6 +1078,7 @@ static int launch_cfg(const GemmArgs& a, int bn, int num_sms, cudaStream_t strea
     int ldr = a.ldr;
     const bf16* bias = (const bf16*)a.bias;
     if (EPI == EPI_CLAMP_GLU) glu_slots(a, ldr, bias);
+    if (EPI == EPI_LOGITS_F32) set_logit_slots(a, ldr, bias);
     chained(kern, grid, 384, cfg.smem_bytes, stream)(ta, tb, (bf16*)a.C, a.M, a.N, a.K, a.ldc, bias, (const bf16*)a.residual, ldr, splits, cfg,
                                                      a.tile_group, batch, a.a_col_stride, a.c_col_stride);
     return cudaGetLastError() == cudaSuccess ? 0 : -13;
@@ -1509,7 +1533,7 @@ int gemm_bf16_tn(const GemmArgs& a, int num_sms, cudaStream_t stream) {
     if (a.c_f32) {   // the fp32 tile store of the split-K instantiation, as one split
         GemmArgs p = a;
         p.splits = 1;
-        return launch_cfg<EPI_PARTIAL_F32>(p, block_n, num_sms, stream);
+        return a.logits ? launch_cfg<EPI_LOGITS_F32>(p, block_n, num_sms, stream) : launch_cfg<EPI_PARTIAL_F32>(p, block_n, num_sms, stream);
     }
     return launch_epi(a, block_n, num_sms, stream);
 }

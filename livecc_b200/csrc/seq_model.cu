@@ -227,8 +227,10 @@ int fill_i32(int* dst, int byte, size_t n, cudaStream_t s) {
 // y[M, N] = x[M, K] W^T (+ bias). Large bf16 products with 8-aligned shapes run on the tensor cores; everything else on
 // the CUDA-core kernels. bias is fp32; the tensor-core epilogue takes a copy in the storage type (bias_st; without one, or with
 // fewer than 16 rows, a biased product stays on the CUDA cores, which add the bias itself). A ragged N runs on the tensor cores when the matrix rows are padded to 8.
+// logits: fp32 y = softcap(x W^T) * scale (cap <= 0: none), in the tensor cores' store or by a kernel behind the others.
+struct Logits { float cap, scale; };
 int linear(const lcc_seq_model* m, const void* x, int ldx, const void* W, const float* bias, void* y, int ldy,
-           bool y_f32, int M, int N, int K, cudaStream_t s, const void* bias_st = nullptr, int act = lcc::ACT_NONE) {
+           bool y_f32, int M, int N, int K, cudaStream_t s, const void* bias_st = nullptr, int act = lcc::ACT_NONE, const Logits* logits = nullptr) {
     const int Np = m->d.rows_padded8 ? ld8(N) : N;
     if (act != lcc::ACT_NONE && bias) return -2;
     if (m->use_tc && m->d.dtype == LCC_DT_BF16 && (!y_f32 || (!bias && act == lcc::ACT_NONE)) && (!bias || (bias_st && M >= 16)) && M > 8 &&
@@ -237,12 +239,17 @@ int linear(const lcc_seq_model* m, const void* x, int ldx, const void* W, const 
         lcc::GemmArgs a;
         a.fault = m->ctx->fault;
         a.c_f32 = y_f32;
+        if (logits) { a.logits = logits->cap > 0.f || logits->scale != 1.f; a.logit_cap = logits->cap; a.logit_scale = logits->scale; }
         a.A = x; a.B = W; a.C = y; a.M = M; a.N = Np; a.K = K; a.lda = ldx; a.ldb = K; a.ldc = ldy;
         a.bias = bias ? bias_st : nullptr; a.residual = nullptr; a.ldr = 0; a.block_n = 0;
         a.epi = act == lcc::ACT_RELU2 ? lcc::EPI_RELU2
                 : act == lcc::ACT_GELU_TANH ? lcc::EPI_GELU_TANH
                 : act == lcc::ACT_GELU_ERF ? lcc::EPI_GELU_ERF : (bias ? lcc::EPI_BIAS : lcc::EPI_NONE);
         return lcc::gemm_bf16_tn(a, m->ctx->num_sms, s);
+    }
+    if (logits) {
+        const int rc = linear(m, x, ldx, W, bias, y, ldy, y_f32, M, N, K, s);
+        return rc ? rc : lcc::softcap((float*)y, (int64_t)M * ldy, logits->cap, s, logits->scale);
     }
     if (act != lcc::ACT_NONE) {   // the activation rides in the store of the CUDA-core kernels too
         lcc::GroupedLinear g{};
@@ -1026,9 +1033,9 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
             STEP(lcc::linear_logits(dt, xf, W, d.head, W, logits, logits_copy, d.vocab, n_want, d.vocab, W, d.logit_softcap, scale, s), "output head");
         } else {
             // scored prompts ask for many rows: the head is then a product like any other. 128 rows x 32768 outputs of width 2048: 648 us
-            // as CUDA-core tiles
-            STEP(linear(m, xf, W, d.head, nullptr, logits, d.vocab, true, n_want, d.vocab, W, s), "output head");
-            STEP(lcc::softcap(logits, (int64_t)n_want * d.vocab, d.logit_softcap, s, scale), "logit soft cap / scale");
+            // as CUDA-core tiles. The soft cap and the scale ride in its store (as a kernel of their own 17 us for 128 rows, tanh of one logit per thread; here 5 more than the plain store)
+            const Logits ls{d.logit_softcap, scale};
+            STEP(linear(m, xf, W, d.head, nullptr, logits, d.vocab, true, n_want, d.vocab, W, s, nullptr, lcc::ACT_NONE, &ls), "output head");
             if (logits_copy) STEP(copy_f32(logits_copy, logits, (size_t)n_want * d.vocab, s), "logits copy");
         }
     }

@@ -40,3 +40,29 @@ def test_widths_of_the_query_and_key_norm(heads, kv, dim):
     for dtype, tol in (("float32", F32_TOL), ("bfloat16", BF16_TOL)):
         m = SeqLMForCausalLM.from_state_dict(cfg, t, dtype)
         assert rel(run(m, toks, [4, 5]), want) < tol
+
+
+@pytest.mark.parametrize("cap,scale", [(8.0, 1.0), (8.0, 0.7), (0.0, 0.7)])
+@pytest.mark.parametrize("vocab", [32, 200, 203, 1000])
+@pytest.mark.parametrize("rows", [9, 64, 129])
+def test_cap_and_scale_of_many_rows_equal_those_of_one(rows, vocab, cap, scale):
+    """Logits of many rows are capped and scaled in the product's store (or behind it where the tensor cores do not take the sizes), those of one row in
+    another kernel's. The two sums differ by the order of 72 products, which neither a cap (slope at most 1) nor a scale below 1 widens; tanh rounds at 2^-22."""
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    d = seq_cases.config([seq_cases.ssd(heads=2, vdim=8, state=8, groups=1)], width=72, vocab=vocab, softcap=cap)
+    d["logit_scale"] = scale
+    cfg = SeqModelConfig.from_json(d)
+    assert cfg.logit_scale == scale
+    m = SeqLMForCausalLM.from_state_dict(cfg, synthetic_seq_tensors(cfg, seed=3), "bfloat16")
+    toks = seq_cases.tokens(rows, vocab, seed=rows)
+
+    def logits(want):
+        c = m.new_cache()
+        out = m.forward_step([(c, toks)], [want])
+        c.release()
+        return out
+
+    many = logits(list(range(rows)))
+    for k in (0, rows // 2, rows - 1):
+        assert (many[k] - logits([k])[0]).abs().max() <= 72 * 2.0 ** -23 * 1.25 * 72 ** 0.5 + cap * 2.0 ** -22
