@@ -3,6 +3,8 @@
 // grouped linear kernels walk. Router scores, weights and gates are fp32.
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "launch.h"
 #include "seqmix.h"
@@ -224,6 +226,14 @@ __global__ void moe_index_kernel(const int* __restrict__ sel, const int* __restr
     src_row[p] = i / top;
 }
 
+// A kernel, since two memsets in front of the router took 7 us of a chain of kernels and kept the router from being launched early (3 more); 1 us here.
+__global__ void __launch_bounds__(256) moe_clear_kernel(int* __restrict__ counts, int E, int* __restrict__ src_row, int rows) {
+    chain_begin();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < E) counts[i] = 0;
+    if (i < rows) src_row[i] = -1;
+}
+
 // out[i, :] = in[src_row[i], :] for every list row (16-byte pieces); padding rows (src_row < 0) are left alone.
 __global__ void __launch_bounds__(128) moe_gather_kernel(const uint4* __restrict__ in, int ld_in16, const int* __restrict__ src_row,
                                                          uint4* __restrict__ out, int ld_out16, int n16) {
@@ -242,6 +252,13 @@ static bool router_ok(const MoeRouterOpts& ro, int E, int top, const float* shar
     if (ro.group_top < 1 || ro.group_top > 2) return false;
     if (ro.topk_softmax && (ro.identity > 0 || ro.groups > 0 || ro.softmax)) return false;
     return ro.groups >= 0;
+}
+
+int moe_clear(int* counts, int E, int* src_row, int rows, cudaStream_t s) {
+    if (!counts || E < 1 || rows < 0 || (rows && !src_row)) return -2;
+    count_launch();
+    chained(moe_clear_kernel, (std::max(E, rows) + 255) / 256, 256, 0, s)(counts, E, src_row, rows);
+    return cudaGetLastError() == cudaSuccess ? 0 : -100;
 }
 
 int moe_route(const float* logits, int ld, const float* correction, int E, int top, float scale, int* sel, float* weight,

@@ -66,6 +66,33 @@ __global__ void embed_sinusoid_kernel(const int64_t* __restrict__ ids, const int
     }
 }
 
+// Many rows: four columns per thread, so that a pair's sine and cosine share a thread instead of sending every warp through both, and pieces of 16 bytes.
+// 2048 rows of 2048 columns with positions: 24 us with a column per thread and step, 10 here.
+template <typename T>
+__global__ void __launch_bounds__(256) embed_sinusoid4_kernel(const int64_t* __restrict__ ids, const int* __restrict__ seq_len, const T* __restrict__ table,
+                                                              int64_t vocab, float scale, const float* __restrict__ inv_freq, float* __restrict__ x32,
+                                                              T* __restrict__ xa, int S, int W, SeqPos pos, int copies) {
+    chain_begin(ids, seq_len);
+    if (seq_done(pos)) return;
+    const int r = blockIdx.x;
+    const int64_t id = seq_len ? ids[*seq_len - S + r] : ids[r];
+    const float p = (float)(seq_past(pos, S) + r);
+    const bool ok = id >= 0 && id < vocab;
+    for (int c = threadIdx.x * 4; c < W; c += blockDim.x * 4) {
+        float v[4] = {}, pe[4] = {};
+        if (ok) ld4(table + (size_t)id * W + c, v);
+        if (inv_freq) {
+            const float2 f = *reinterpret_cast<const float2*>(inv_freq + (c >> 1));
+            const float a0 = p * f.x, a1 = p * f.y;
+            pe[0] = sinf(a0); pe[1] = cosf(a0); pe[2] = sinf(a1); pe[3] = cosf(a1);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = (ok ? v[j] * scale : 0.f) + pe[j];
+        for (int k = 0; k < copies; ++k) st4(x32 + ((size_t)r * copies + k) * W + c, v);
+        if (xa) st4(xa + (size_t)r * W + c, v);
+    }
+}
+
 // Two sums over the CTA behind one pair of barriers (red: 64 floats)
 __device__ __forceinline__ float2 block_sum2(float a, float b, float* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
@@ -339,7 +366,9 @@ __global__ void __launch_bounds__(256) gated_group_norm_kernel(const float* __re
 
 // Groups of 129 to 1024 columns whose rows allow 16-byte reads of y: four neighbouring columns per thread and load, everything in flight
 // together, one pass; a warp per (row, group), 128 threads above 256 columns (a warp alone takes 6.9 us for one row of 8 groups of 512,
-// 128 threads 4.1, the general form above 4.6). 2048 rows of 4096 in groups of 512: 27 us, 45 in the general form.
+// 128 threads 4.1, the general form above 4.6). 2048 rows of 4096 in groups of 512: 24 us, 45 in the general form; a warp per group takes 23 once there are more
+// groups than CTAs of 128 threads fit on the chip (16 per SM): it needs no barrier, and sums each quarter of the group and then the quarters as those do, so that
+// a row's bits do not depend on how many rows there are.
 template <typename T, int TEAM, int E>
 __global__ void __launch_bounds__(TEAM == 32 ? 64 : TEAM) gated_group_norm4_kernel(const float* __restrict__ y, int ld_y, const T* __restrict__ gate,
                                                                 int ld_gate, const float* __restrict__ w, int w_len, T* __restrict__ out,
@@ -351,7 +380,8 @@ __global__ void __launch_bounds__(TEAM == 32 ? 64 : TEAM) gated_group_norm4_kern
     const int r = wid / ngroups, c0 = (wid % ngroups) * group, wb = c0 % w_len;
     const float* yr = y + (size_t)r * ld_y + c0;
     const T* gr = gate + (size_t)r * ld_gate + c0;
-    float vy[E][4], vg[E][4], vw[E][4], ss = 0.f;
+    constexpr bool QUARTERS = TEAM == 32 && E == 4;
+    float vy[E][4], vg[E][4], vw[E][4], ss = 0.f, sq[4];
 #pragma unroll
     for (int i = 0; i < E; ++i) {
         const int c = (lane + TEAM * i) * 4;
@@ -362,14 +392,17 @@ __global__ void __launch_bounds__(TEAM == 32 ? 64 : TEAM) gated_group_norm4_kern
         }
     }
 #pragma unroll
-    for (int i = 0; i < E; ++i)
+    for (int i = 0; i < E; ++i) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             vg[i][j] = gate_first == 2 ? sigmoid_f(vg[i][j]) : silu_f(vg[i][j]);
             if (gate_first == 1) vy[i][j] *= vg[i][j];
             ss = fmaf(vy[i][j], vy[i][j], ss);
         }
-    const float rn = 1.f / sqrtf((TEAM == 32 ? warp_sum(ss) : block_sum(ss, red)) / (float)group + eps);
+        if (QUARTERS) { sq[i & 3] = warp_sum(ss); ss = 0.f; }
+    }
+    const float sum = QUARTERS ? (sq[0] + sq[2]) + (sq[1] + sq[3]) : TEAM == 32 ? warp_sum(ss) : block_sum(ss, red);
+    const float rn = 1.f / sqrtf(sum / (float)group + eps);
 #pragma unroll
     for (int i = 0; i < E; ++i) {
         const int c = (lane + TEAM * i) * 4;
@@ -833,6 +866,14 @@ int embed_sinusoid(int dt, const int64_t* ids, const int* seq_len, const void* t
                    const float* inv_freq, float* x32, void* xa, int S, int W, SeqPos pos, cudaStream_t s, int copies) {
     if (!ids || !table || !x32 || S < 1 || W < 1 || copies < 1) return -2;
     count_launch();
+    // (up to 148 rows the chip is not full: there a column per thread is the shorter chain)
+    if (S > kSms && (W % 4) == 0 && (((uintptr_t)table | (uintptr_t)x32 | (uintptr_t)xa | (uintptr_t)inv_freq) % 16) == 0) {
+        if (dt == DT_F32)
+            chained(embed_sinusoid4_kernel<float>, S, 256, 0, s)(ids, seq_len, (const float*)table, vocab, scale, inv_freq, x32, (float*)xa, S, W, pos, copies);
+        else
+            chained(embed_sinusoid4_kernel<bf16>, S, 256, 0, s)(ids, seq_len, (const bf16*)table, vocab, scale, inv_freq, x32, (bf16*)xa, S, W, pos, copies);
+        return done();
+    }
     // few rows: a column per thread (eight sines one after the other in each thread took 10.1 us for one row of 2048 columns, one takes 2.4)
     const dim3 grid(S, S <= kSms ? std::min((W + 255) / 256, 8) : 1);
     if (dt == DT_F32)
@@ -912,6 +953,7 @@ int gated_group_norm(int dt, const float* y, int ld_y, const void* gate, int ld_
                                                                            (bf16*)out, ld_out, S, n, group, gate_first, eps);   \
     } while (0)
         if (group <= 256) LCC_GGN4(32, 2);
+        else if (group <= 512 && teams > 16 * kSms) LCC_GGN4(32, 4);
         else if (group <= 512) LCC_GGN4(128, 1);
         else LCC_GGN4(128, 2);
 #undef LCC_GGN4

@@ -211,15 +211,10 @@ WsLayout make_layout(const lcc_seq_model* m, int NT, int NW) {
         if (rc__) LCC_FAIL(m->ctx, rc__, "%s failed (code %d)", what, rc__);                  \
     } while (0)
 
-// Copies and clears between the kernels of a pass. The kernel behind one is launched in the ordinary way (launch.h: a chained kernel's
+// Copies between the kernels of a pass. The kernel behind one is launched in the ordinary way (launch.h: a chained kernel's
 // predecessor is a kernel).
 int copy_f32(float* dst, const float* src, size_t n, cudaStream_t s) {
     const cudaError_t e = cudaMemcpyAsync(dst, src, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
-    lcc::chain_break();
-    return e == cudaSuccess ? 0 : -100;
-}
-int fill_i32(int* dst, int byte, size_t n, cudaStream_t s) {
-    const cudaError_t e = cudaMemsetAsync(dst, byte, n * sizeof(int), s);
     lcc::chain_break();
     return e == cudaSuccess ? 0 : -100;
 }
@@ -934,8 +929,7 @@ int lcc_seq_forward(lcc_seq_model* m, const lcc_seq_entry* entries, int n_entrie
                 STEP(lcc::moe_route_small(logit, lde, l.e_correction_f32, EO, K, l.e_scale, sel, wsel, gate_out, row_off, posn,
                                           src_row, T, fs, &ro), "expert choice + row lists");
             } else {
-                STEP(fill_i32(counts, 0, E, fs), "router counters");
-                if (tc) STEP(fill_i32(src_row, 0xff, (size_t)n_tiles * kMoeTile, fs), "row lists");
+                STEP(lcc::moe_clear(counts, E, src_row, tc ? n_tiles * kMoeTile : 0, fs), "router counters and row lists");
                 STEP(lcc::moe_route(logit, lde, l.e_correction_f32, EO, K, l.e_scale, sel, wsel, gate_out, counts, rank, T, fs, &ro), "expert choice");
                 STEP(lcc::moe_index(sel, rank, counts, E, K, tc ? kMoeTile : 1, row_off, posn, src_row, tc ? tile_group : nullptr, n_tiles, T, fs), "expert row lists");
             }

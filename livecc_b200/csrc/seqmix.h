@@ -320,6 +320,8 @@ int hyper_boundary(int dt, float* xs, int n, const void* y, int ld_y, const floa
 // themselves before scores and choice (not to the shared gate's). group_top: a group scores as the sum of that
 // many of its largest choice scores (1 or 2).
 struct MoeRouterOpts { bool softmax; int identity; int groups; int keep; bool topk_softmax = false; int group_top = 1; const float* logit_bias = nullptr; };
+// counts[0, E) = 0 and src_row[0, rows) = -1: what moe_route counts into and the padding rows of its lists
+int moe_clear(int* counts, int E, int* src_row, int rows, cudaStream_t s);
 int moe_route(const float* logits, int ld, const float* correction, int E, int top, float scale, int* sel, float* weight,
               float* shared_gate, int* counts, int* rank, int S, cudaStream_t s, const MoeRouterOpts* opt = nullptr);
 // moe_route and moe_index (dense lists) in one launch of one CTA, for calls of up to kMoeSmallItems (row, choice) pairs; it

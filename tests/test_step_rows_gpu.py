@@ -66,3 +66,47 @@ def test_cap_and_scale_of_many_rows_equal_those_of_one(rows, vocab, cap, scale):
     many = logits(list(range(rows)))
     for k in (0, rows // 2, rows - 1):
         assert (many[k] - logits([k])[0]).abs().max() <= 72 * 2.0 ** -23 * 1.25 * 72 ** 0.5 + cap * 2.0 ** -22
+
+
+# either side of the rows from which the embedding takes four columns per thread, widths off 4 and past a pass of 1024; norm groups of a warp: up to 128, 256, 512, and past it
+@pytest.mark.parametrize("rows,width", [(148, 24), (149, 24), (149, 255), (150, 1028)])
+def test_embedding_of_many_rows(rows, width):
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    heads = dict(heads=2, kv_heads=1, dim=12, vdim=8) if width % 4 else dict(heads=4, kv_heads=2, dim=16, vdim=8)
+    d = seq_cases.config([seq_cases.par(**heads, ff=None)], width=width, vocab=70, softcap=8.0)
+    cfg = SeqModelConfig.from_json(d)
+    t = synthetic_seq_tensors(cfg, seed=3)
+    toks = seq_cases.tokens(rows, 70, seed=width)
+    want, _ = O.forward(d, t, toks)
+    for dtype, tol in (("float32", F32_TOL), ("bfloat16", BF16_TOL)):
+        m = SeqLMForCausalLM.from_state_dict(cfg, t, dtype)
+        assert rel(run(m, toks, [rows]), want) < tol
+
+
+@pytest.mark.parametrize("heads,vdim,groups", [(1, 132, 1), (2, 128, 1), (4, 65, 1), (4, 128, 1), (8, 128, 2), (4, 129, 1)])
+def test_groups_of_the_gated_norm(heads, vdim, groups):
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    d = seq_cases.config([seq_cases.ssd(heads=heads, vdim=vdim, state=16, groups=1, norm_groups=groups)], width=40, vocab=70)
+    cfg = SeqModelConfig.from_json(d)
+    t = synthetic_seq_tensors(cfg, seed=5)
+    toks = seq_cases.tokens(35, 70, seed=vdim)
+    want, _ = O.forward(d, t, toks)
+    for dtype, tol in (("float32", F32_TOL), ("bfloat16", BF16_TOL)):
+        m = SeqLMForCausalLM.from_state_dict(cfg, t, dtype)
+        assert rel(run(m, toks, [33, 34, 35]), want) < tol
+
+
+@pytest.mark.parametrize("heads,vdim", [(4, 128), (4, 65)])
+def test_gated_norm_has_the_same_bits_for_few_and_many_rows(heads, vdim):
+    """8 groups of rows: 2400 and more (row, group) pairs go a warp to a group, fewer a CTA; both sum in one order. The scan in front is cut at the same
+    blocks of 64 rows, and the products behind one row alone are those of many on the CUDA cores (fp32 storage)."""
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    d = seq_cases.config([seq_cases.ssd(heads=8 * heads, vdim=vdim, state=8, groups=1, norm_groups=8)], width=24, vocab=40)
+    cfg = SeqModelConfig.from_json(d)
+    m = SeqLMForCausalLM.from_state_dict(cfg, synthetic_seq_tensors(cfg, seed=5), "float32", max_tokens=512)
+    toks = seq_cases.tokens(330, 40, seed=vdim)
+    many, few = run(m, toks, [320]), run(m, toks, [128, 256, 320])
+    assert torch.equal(many[:320], few[:320])
