@@ -87,10 +87,10 @@ __global__ void causal_conv_kernel(const TI* __restrict__ in, int ld_in, T* __re
     }
 }
 
-// Long calls in bf16 with 2 to 4 taps and even channels: a thread owns two neighbouring channels over `span` rows, eight rows' loads in
-// flight, the window slides through registers. The form above reads an input 1.9 times (8 rows and 7 before them), two bytes at a time.
-// The sums run in its order. 2048 rows of 6144 channels, 4 taps: 31 us, 64
-// in the form above; 128 rows: 6.8 us for 9.7.
+// Long calls in bf16 with 2 to 4 taps and even channels: a thread owns two neighbouring channels over `span` rows, the next eight rows' loads are in
+// flight while eight are worked on, the window slides through registers. The form above reads an input 1.9 times (8 rows and 7 before them), two bytes
+// at a time. The sums run in its order. 2048 rows of 6144 channels, 4 taps: 64 us in the form above, 21 here between the kernels of a prompt
+// (24 while the eight rows were waited for).
 template <int TAPS, bool SILU>
 __global__ void __launch_bounds__(128) causal_conv_long_kernel(const bf16* __restrict__ in, int ld_in, bf16* __restrict__ out, int ld_out,
                                                                const float* __restrict__ w, const float* __restrict__ b,
@@ -112,9 +112,16 @@ __global__ void __launch_bounds__(128) causal_conv_long_kernel(const bf16* __res
         win[i] = t >= 0 ? row(t) : make_float2(carry[(size_t)c * (TAPS - 1) + (TAPS - 1 + t)], carry[(size_t)(c + 1) * (TAPS - 1) + (TAPS - 1 + t)]);
     }
     const int t1 = min(S, t0 + span);
+    uint32_t nx[8];
+    auto fetch = [&](int t) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) nx[r] = t + r < t1 ? *reinterpret_cast<const uint32_t*>(in + (size_t)(t + r) * ld_in + c) : 0u;
+    };
+    fetch(t0);
     for (int t = t0; t < t1; t += 8) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) win[TAPS - 1 + r] = t + r < t1 ? row(t + r) : make_float2(0.f, 0.f);
+        for (int r = 0; r < 8; ++r) win[TAPS - 1 + r] = unpack_bf16x2(nx[r]);
+        if (t + 8 < t1) fetch(t + 8);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
             float a0 = b0, a1 = b1;
