@@ -49,10 +49,10 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
 }
 
 // A chain of short kernels: inside a ChainScope each may be set up while the one before it in the stream still runs (programmatic dependent
-// launch), and its first statement, chain_begin() in common.cuh, waits for that one. A step of the hybrid models is some 45 kernels of 3 to
-// 10 us on one row; as ordinary graph nodes, kernels that return at once cost 2.7 to 4 us each. Chained, and with the first
-// weights of a linear layer loaded before the wait, a prompt of 128 tokens and 31 replayed steps take 8.29 ms for 8.48 (recurrent design, four
-// layers) and 4.86 for 5.14 (routed, two layers), one step launched by the host 0.32 ms for 0.38 and 0.33 for 0.36 (four layers each).
+// launch), and its first statement, chain_begin() in common.cuh, waits for that one. A step of the hybrid models is 30 (recurrent design, four layers) and 22
+// kernels of 2 to 10 us on one row; as ordinary graph nodes, kernels that return at once cost 2.7 to 4 us each. Chained, and with the first
+// weights of a linear layer loaded before the wait, a prompt of 128 tokens and 31 replayed steps took 8.29 ms for 8.48 (recurrent design, then
+// 45 kernels a step) and 4.86 for 5.14 (routed, two layers), one step launched by the host 0.32 ms for 0.38 and 0.33 for 0.36 (four layers each).
 // Matrix products, row kernels and attention of the vision tower and of a prefill are chained too: what they set up (barriers, tensor memory, tensor
 // maps) and their launch lie beside the kernel in front. A turn that reads 281 tokens behind 17 k 1.42 -> 1.32 ms, 24 behind 8 k 1.00 -> 0.84, eight
 // streams' prefill 2.0 -> 1.6, 1024 and 8192 patches 456 -> 442 and 980 -> 948 us, prompts of the hybrid models 1.72 -> 1.67 and 0.56 -> 0.525 ms.

@@ -227,7 +227,7 @@ __global__ void moe_index_kernel(const int* __restrict__ sel, const int* __restr
 }
 
 // A kernel, since two memsets in front of the router took 7 us of a chain of kernels and kept the router from being launched early (3 more); 1 us here.
-__global__ void __launch_bounds__(256) moe_clear_kernel(int* __restrict__ counts, int E, int* __restrict__ src_row, int rows) {
+__global__ void __launch_bounds__(256) moe_clear_kernel(int* counts, int E, int* src_row, int rows) {
     chain_begin();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i < E) counts[i] = 0;

@@ -8,7 +8,8 @@
 // Five launches: block-local cumulative log decays, M, the blocks' own state contributions, a short sequential pass
 // over blocks that turns them into the state entering each block, and the outputs. All arithmetic is fp32 (the recurrence's operands are
 // fp32 by the models' precision rules); the three products are 64 x 64 tiles whose operands are formed (decay factors applied) while
-// they are staged: on the CUDA cores, or, for a decay per head over aligned bf16 rows, on the tensor cores by values cut in three.
+// they are staged: on the CUDA cores, or, over aligned bf16 rows, on the tensor cores by values cut in three (all three for a decay per head,
+// the blocks' own states for a decay per key channel, whose outputs have two fp32 operands).
 #include <type_traits>
 #include <math.h>
 
@@ -642,7 +643,7 @@ __global__ void __launch_bounds__(128) chunk_output_head_kernel(ChunkArgs a, Seq
 // fp32 adds are 1.8e-7 off): 16 terms are summed there, three parts of them one after another, and added to the sum by the CUDA cores (9e-8; random
 // signs 3.0e-9 for 4.5e-9).
 // Decays and scales stay fp32. Bound by latency (16 to 20 warps per SM; outputs issue in 43 % of the slots and read at 16 % of HBM's rate): 2048 rows, 64 heads of
-// 64 x 128, 7.8 + 33 + 77 us for 16 + 66 + 119 of the fp32 kernels (6.9 + 31 + 71 with running sums in the accumulators).
+// 64 x 128, 7.8 + 33 + 73 us for 16 + 66 + 119 of the fp32 kernels (6.9 + 31 + 71 with running sums in the accumulators).
 __device__ __forceinline__ float low_part(float x) {   // x minus its leading 8 bits; nothing behind an infinity or NaN
     return fabsf(x) < INFINITY ? x - __uint_as_float(__float_as_uint(x) & 0xffff0000u) : 0.f;
 }

@@ -69,9 +69,9 @@ __global__ void embed_sinusoid_kernel(const int64_t* __restrict__ ids, const int
 // Many rows: four columns per thread, so that a pair's sine and cosine share a thread instead of sending every warp through both, and pieces of 16 bytes.
 // 2048 rows of 2048 columns with positions: 24 us with a column per thread and step, 10 here.
 template <typename T>
-__global__ void __launch_bounds__(256) embed_sinusoid4_kernel(const int64_t* __restrict__ ids, const int* __restrict__ seq_len, const T* __restrict__ table,
-                                                              int64_t vocab, float scale, const float* __restrict__ inv_freq, float* __restrict__ x32,
-                                                              T* __restrict__ xa, int S, int W, SeqPos pos, int copies) {
+__global__ void __launch_bounds__(256) embed_sinusoid4_kernel(const int64_t* __restrict__ ids, const int* __restrict__ seq_len, const T* table,
+                                                              int64_t vocab, float scale, const float* inv_freq, float* x32,
+                                                              T* xa, int S, int W, SeqPos pos, int copies) {
     chain_begin(ids, seq_len);
     if (seq_done(pos)) return;
     const int r = blockIdx.x;
