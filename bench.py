@@ -314,7 +314,8 @@ def time_ingest_kernel(eng, peak, iters=20):
     """GPU frame ingest: resize_bicubic_aa_u8_kernel on a 2-frame 1080p chunk -> 448x796 (what
     get_smart_resized_clip does for a 16:9 source, video_process_patch.py:150-155), rotated over > L2 of distinct clips,
     CUDA events; beside it the reference's host call (torchvision, all host threads) on the same clip, and whether the
-    two results are identical. Algorithmic bytes = source + destination planes; the kernel is fp32-issue bound."""
+    two results are identical. Algorithmic bytes = source + destination planes; the kernel is bound by instruction issue and latency
+    (width pass on the tensor cores, height pass in packed fp32)."""
     import time
 
     from torchvision.transforms import InterpolationMode
@@ -346,7 +347,7 @@ def time_ingest_kernel(eng, peak, iters=20):
     nbytes = T * 3 * (h * w + H * W)
     return {"kernel": "resize_bicubic_aa_u8_kernel (bicubic antialias uint8 resize, both passes fused)",
             "workload": "2 frames 3x1080x1920 -> 3x448x796 uint8", "us_per_launch": us, "bytes_per_launch": nbytes,
-            "achieved": nbytes / us / 1e3, "unit": "GB/s", "frac": nbytes / us / 1e3 / peak, "bound": "fp32 issue (22 taps/pixel); HBM frac reported",
+            "achieved": nbytes / us / 1e3, "unit": "GB/s", "frac": nbytes / us / 1e3 / peak, "bound": "instruction issue and latency; HBM frac reported",
             "host_torchvision_ms": cpu_ms, "host_threads": torch.get_num_threads(),
             "identical_to_torchvision": bool(torch.equal(out.cpu(), ref))}
 

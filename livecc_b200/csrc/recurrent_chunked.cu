@@ -642,7 +642,8 @@ __global__ void __launch_bounds__(128) chunk_output_head_kernel(ChunkArgs a, Seq
 // like fp32 adds, and a running sum kept in its accumulators drifts (2.1e-6 of the summed magnitudes over 136 terms of one sign, where
 // fp32 adds are 1.8e-7 off): 16 terms are summed there, three parts of them one after another, and added to the sum by the CUDA cores (9e-8; random
 // signs 3.0e-9 for 4.5e-9).
-// Decays and scales stay fp32. Bound by latency (16 to 20 warps per SM; outputs issue in 43 % of the slots and read at 16 % of HBM's rate): 2048 rows, 64 heads of
+// Decays and scales stay fp32. Bound by each warp's chain of cuts, three products and adds (16 to 20 warps per SM; outputs issue in 43 % of the slots and read at 16 % of HBM's rate;
+// loads a step ahead, the first while the weights are formed, 73 -> 74): 2048 rows, 64 heads of
 // 64 x 128, 7.8 + 33 + 73 us for 16 + 66 + 119 of the fp32 kernels (6.9 + 31 + 71 with running sums in the accumulators).
 __device__ __forceinline__ float low_part(float x) {   // x minus its leading 8 bits; nothing behind an infinity or NaN
     return fabsf(x) < INFINITY ? x - __uint_as_float(__float_as_uint(x) & 0xffff0000u) : 0.f;
