@@ -200,28 +200,41 @@ __global__ void moe_index_kernel(const int* __restrict__ sel, const int* __restr
                                  int top, int pad, int* __restrict__ row_off, int* __restrict__ pos, int* __restrict__ src_row,
                                  int* __restrict__ tile_group, int n_tiles, int S) {
     chain_begin(sel, rank, counts);
+    // every CTA sums the counts once, in one warp: a thread that walked them for its own expert waited for one after the other (16 experts,
+    // 1024 rows x 4: 6.7 us, 2.7 here)
+    __shared__ int off[32 * kMaxExpertsPerLane + 1];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= E) {
-        int o = 0;
-        for (int e = 0; e < i; ++e) o += padded(counts[e], pad);
-        row_off[i] = o;
-    }
-    if (tile_group && i < n_tiles) {
-        // the list that owns rows [i * pad, (i + 1) * pad), or -1 past the last list
-        int o = 0, g = -1;
-        for (int e = 0; e < E; ++e) {
-            const int n = padded(counts[e], pad);
-            if (i * pad >= o && i * pad < o + n) { g = e; break; }
-            o += n;
+    const bool item = i < S * top;
+    const int e = item ? sel[i] : 0, rk = item ? rank[i] : -1;
+    if (threadIdx.x < 32) {
+        int carry = 0;
+        for (int base = 0; base < E; base += 32) {
+            const int x = base + (int)threadIdx.x;
+            int v = x < E ? padded(counts[x], pad) : 0;
+#pragma unroll
+            for (int d = 1; d < 32; d *= 2) {
+                const int up = __shfl_up_sync(0xffffffffu, v, d);
+                if ((int)threadIdx.x >= d) v += up;
+            }
+            if (x < E) off[x + 1] = carry + v;
+            carry += __shfl_sync(0xffffffffu, v, 31);
         }
-        tile_group[i] = g;
+        if (threadIdx.x == 0) off[0] = 0;
     }
-    if (i >= S * top) return;
-    const int e = sel[i];
-    if (rank[i] < 0) { pos[i] = -1; return; }     // an identity expert: no list
-    int o = 0;
-    for (int j = 0; j < e; ++j) o += padded(counts[j], pad);
-    const int p = o + rank[i];
+    __syncthreads();
+    if (i <= E) row_off[i] = off[i];
+    if (tile_group && i < n_tiles) {
+        // the list that owns rows [i * pad, (i + 1) * pad), or -1 past the last list: the last one that starts at or before them (empty ones start where the next does)
+        int lo = 0, hi = E;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (off[mid] <= i * pad) lo = mid; else hi = mid;
+        }
+        tile_group[i] = i * pad < off[E] ? lo : -1;
+    }
+    if (!item) return;
+    if (rk < 0) { pos[i] = -1; return; }     // an identity expert: no list
+    const int p = off[e] + rk;
     pos[i] = p;
     src_row[p] = i / top;
 }
@@ -285,7 +298,7 @@ int moe_route_small(const float* logits, int ld, const float* correction, int E,
 
 int moe_index(const int* sel, const int* rank, const int* counts, int E, int top, int pad, int* row_off, int* pos, int* src_row,
               int* tile_group, int n_tiles, int S, cudaStream_t s) {
-    if (!sel || !rank || !counts || !row_off || !pos || !src_row || S < 1 || E < 1 || top < 1 || pad < 1 || (tile_group && n_tiles < 1))
+    if (!sel || !rank || !counts || !row_off || !pos || !src_row || S < 1 || E < 1 || E > 32 * kMaxExpertsPerLane || top < 1 || pad < 1 || (tile_group && n_tiles < 1))
         return -2;
     int n = S * top > E + 1 ? S * top : E + 1;
     if (tile_group && n_tiles > n) n = n_tiles;
