@@ -108,6 +108,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         tile_lo = split * tps;
         tile_hi = min(n_tiles, tile_lo + tps);
         if (tile_lo >= tile_hi) {  // nothing for this split: neutral partial
+            chain_wait();          // (the kernel in front may be the merge of other streams' partials, in the same scratch)
             float* ml = p.part_ml + (st.part_row + ((size_t)split * p.Hkv + kvh) * rows_total + row_base) * 2;
             for (int i = threadIdx.x; i < rows_used; i += blockDim.x) {
                 ml[i * 2] = -INFINITY;

@@ -76,6 +76,7 @@ def _check_ids(out, n, penalty):
     ("wide", [(300, 24, 0), (512, 1, 0), (0, 33, 0), (90, 19, 2), (1000, 5, 0)]),
     ("small", [(30, 1200, 0), (0, 900, 2), (5, 30, 0)]),                                     # more rows than one pass takes
     ("wide", [(300, 281, 0), (0, 281, 0), (40, 200, 0), (0, 330, 0), (10, 150, 0)]),         # K cut alike, more rows than a wave of clusters takes
+    ("wide", [(16384, 64, 0)] * 7 + [(12932, 50, 0)]),     # attention in two groups that share the partials' scratch; the second has an empty key range
 ])
 def test_streams_together_match_streams_alone(engines, which, spec):
     eng, new = engines[which], 5

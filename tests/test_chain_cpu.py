@@ -7,7 +7,7 @@ from pathlib import Path
 import pytest
 
 CSRC = Path(__file__).resolve().parent.parent / "livecc_b200" / "csrc"
-FILES = ["rowops", "recurrent", "recurrent_chunked", "attn_local", "attn_latent", "hyper", "moe", "rotary", "linear_any"]
+FILES = ["rowops", "recurrent", "recurrent_step", "recurrent_chunked", "attn_local", "attn_latent", "hyper", "moe", "rotary", "linear_any"]
 
 # `__restrict__` parameters that no kernel or copy of a pass writes before the kernel reads them: weights and tables, and what it only writes
 WEIGHTS = {
@@ -37,13 +37,80 @@ def kernels(name):
     """(kernel name, parameter text, body) of every __global__ function of a file."""
     src = re.sub(r"//[^\n]*", "", (CSRC / f"{name}.cu").read_text())
     out = []
-    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\(([^{]*)\)\s*\{", src):
+    for m in re.finditer(r"__global__\s+void\s+(?:__cluster_dims__\([^)]*\)\s*)?(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\(([^{]*)\)\s*\{", src):
         depth, i = 1, m.end()
         while depth:
             depth += {"{": 1, "}": -1}.get(src[i], 0)
             i += 1
         out.append((m.group(1), m.group(2), src[m.end():i]))
     return src, out
+
+
+# What is touched in front of the wait, per kernel: elements of arrays in the launch parameters, shared memory behind a pointer in a struct, and
+# loads of what nothing writes while the kernel in front runs. Nothing at all may be stored to global memory there.
+PARAMETERS = {"attn_prefill_tc_kernel": {"p.ps.st"}}
+SHARED = {"gemm_swap_kernel": {"g.flag"}}
+EARLY_LOADS = {
+    "linear_rows_kernel": {"W"},                          # weights
+    # weights, and the state and the carried inputs: their one writer is the same layer's kernel of the step before, a whole step of kernels away
+    "scan_step_kernel": {"a.conv_w", "a.conv_b", "a.dt_bias", "a.a_log", "a.skip", "a.norm_w", "a.carry", "a.state"},
+    # the form with windows reads its sequence's scalars; it is launched in the ordinary way (test_prompt_attention_is_launched_in_the_ordinary_way)
+    "attn_prefill_tc_kernel": {"lp.pos.finished", "lp.pos.kv_len"},
+    "vit_attn_tc_kernel": {"p.cu_seqlens"},               # written at the start of the pass: layer norm, product and rotary lie between
+}
+
+
+def touched_before_the_wait(body):
+    """(loaded, stored): the pointers through which global memory is reached in front of a kernel's chain_begin; a block's statements behind a
+    chain_wait() of its own do not count. Shared memory, local arrays and pointers to either are left out, a pointer that is a local name for
+    an offset into another counts as that one."""
+    text = body[:body.index("chain_begin(")]
+    while "chain_wait();" in text:
+        at = i = text.index("chain_wait();")
+        depth = 0
+        while i < len(text) and depth >= 0:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+        text = text[:at] + text[i - 1:]
+    near = set(re.findall(r"__shared__[^;]*?(\w+)\[", text)) | {"smem_raw"}
+    for decl in re.findall(r"__shared__([^;]*);", text):
+        near |= set(re.findall(r"(\w+)\s*(?:\[|,|$)", decl))
+    near |= set(re.findall(r"\b(?:float4?|uint4|int|uint32_t)\s+(\w+)\[", text)) | set(re.findall(r"\b(?:float|int)\s[^;=(]*?,\s*(\w+)\[", text))
+    for decl in re.findall(r"\bfloat ((?:\w+\[[^;]*?)+);", text):
+        near |= set(re.findall(r"(\w+)(?:\[\w+\])+", decl))
+    names = {}
+    for m in re.finditer(r"(?:\*|\bauto)\s*(?:const\s+)?(?:__restrict__\s+)?(\w+)\s*=\s*([^;]*);", text):
+        sources = [x for x in re.findall(r"[A-Za-z_][\w.]*", m.group(2))]
+        first = next((x for x in sources if x in near or x in names or "." in x), None)
+        if first in near:
+            near.add(m.group(1))
+        elif first:
+            names[m.group(1)] = names.get(first, first)
+    loaded, stored = set(), set()
+    access = [(m.group(1), m.end()) for m in re.finditer(r"\b([A-Za-z_]\w*(?:\.\w+)*)\s*\[", text)]
+    access += [(m.group(1), m.end()) for m in re.finditer(r"(?<=[=(,&|?:!])\s*\*\s*([A-Za-z_]\w*(?:\.\w+)*)", text)]
+    access += [(m.group(1), m.end()) for m in re.finditer(r"[;{}]\s*\*\s*([A-Za-z_]\w*(?:\.\w+)*)", text)]
+    access += [(m.group(1), m.end()) for m in re.finditer(r"(?:ld_stream16|__ldg|ldf|ld4)\(\s*&?([A-Za-z_]\w*(?:\.\w+)*)", text)]
+    for name, end in access:
+        if name in near:
+            continue
+        depth = text[end - 1] == "["
+        while depth:
+            depth += {"[": 1, "]": -1}.get(text[end], 0)
+            end += 1
+        into = stored if re.match(r"\s*(?:\.\w+\s*)?(?:[-+*/|&^]?=(?!=)|\+\+|--)", text[end:]) else loaded
+        into.add(names.get(name, name))
+    calls = set(re.findall(r"\b(tma_\w+|cp_async\w*|st_\w+|stf|st4|atomic\w+|red_\w+|mbar_wait\w*)\(", text))
+    calls |= {a for a in re.findall(r'asm volatile\("([^"]*)', text) if "global" in a or "bulk" in a}
+    return loaded, stored | calls
+
+
+def check_before_the_wait(kernel, body):
+    loaded, stored = touched_before_the_wait(body)
+    stored -= SHARED.get(kernel, set())
+    assert not stored, f"{kernel} writes in front of its wait: {sorted(stored)}"
+    allowed = PARAMETERS.get(kernel, set()) | EARLY_LOADS.get(kernel, set())
+    assert loaded <= allowed, f"{kernel} reads in front of its wait: {sorted(loaded - allowed)}"
 
 
 @pytest.mark.parametrize("name", FILES)
@@ -56,8 +123,9 @@ def test_chained_kernels_wait_and_name_what_was_written_before(name):
             continue
         begin = re.findall(r"chain_begin\(([^)]*)\);", body)
         assert len(begin) == 1, kernel
-        if kernel != "linear_rows_kernel":     # (that one loads weights before it waits)
+        if kernel not in EARLY_LOADS:
             assert body.lstrip().startswith("chain_begin("), kernel
+        check_before_the_wait(kernel, body)
         restrict = set(re.findall(r"\*\s*__restrict__\s+(\w+)", params))
         named = set(filter(None, re.split(r"[,\s]+", begin[0])))
         rest = set((WEIGHTS.get(kernel, "") + " " + WRITTEN.get(kernel, "")).split())
@@ -99,3 +167,5 @@ def test_prompt_attention_is_launched_in_the_ordinary_way():
     for kernel in ("attn_chunk_sink_mma_kernel", "attn_chunk_sink_tiled_kernel"):
         assert not re.search(rf"chained\(\s*{kernel}", src)
         assert all("chain_begin" not in body for k, _, body in found if k == kernel)
+    src, _ = kernels("attention_prefill_tc")      # the tcgen05 form with windows
+    assert "attn_prefill_tc_kernel<true><<<" in src and "chained(attn_prefill_tc_kernel<true>" not in src

@@ -1,10 +1,10 @@
-"""Chained launches of the vision tower and the prefill, read from the sources: which data a kernel may read non-coherently, and that tensor memory is taken
-before the next kernel is let in."""
+"""Chained launches of the vision tower and the prefill, read from the sources: which data a kernel may read non-coherently, what it touches before it waits
+(nothing that another kernel of the pass writes or still reads), and that tensor memory is taken before the next kernel is let in."""
 import re
 
 import pytest
 
-from test_chain_cpu import CSRC, kernels
+from test_chain_cpu import CSRC, check_before_the_wait, kernels
 
 FILES = ["gemm_tcgen05", "elementwise", "attention", "attention_tc", "attention_prefill_tc"]
 # `__restrict__` parameters that nothing of the pass writes while the kernel is on the SMs (weights, tables), and those that are only written
@@ -15,21 +15,9 @@ WRITTEN = {"norm_rows_kernel": "y", "norm_rows_warp_kernel": "y", "vit_rope_tabl
            "video_rank_kernel": "rank", "mrope_kv_write_kernel": "kc vc", "flash_merge_kernel": "out"}
 
 
-def found_in(name):
-    src, _ = kernels(name)
-    out = []
-    for m in re.finditer(r"__global__\s+void\s+(?:__cluster_dims__\([^)]*\)\s*)?(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\(([^{]*)\)\s*\{", src):
-        depth, i = 1, m.end()
-        while depth:
-            depth += {"{": 1, "}": -1}.get(src[i], 0)
-            i += 1
-        out.append((m.group(1), m.group(2), src[m.end():i]))
-    return src, out
-
-
 @pytest.mark.parametrize("name", FILES)
 def test_chained_kernels_wait_and_name_what_was_written_before(name):
-    src, found = found_in(name)
+    src, found = kernels(name)
     chained = set(re.findall(r"chained\(\s*(\w+)", src)) - {"kern"}
     if "chained(kern" in src or "chain_next()" in src:      # launched through a local name: every kernel of the file that waits
         chained |= {k for k, _, b in found if "chain_begin(" in b}
@@ -51,9 +39,10 @@ def test_chained_kernels_wait_and_name_what_was_written_before(name):
         if "tmem_alloc" in body:
             alloc = body.index("tmem_alloc")
             assert alloc < at and re.search(r"__syncthreads\(\)|cluster_sync_all\(\)", body[alloc:at]), kernel
-            assert "tma_load" not in body[:at] and "residual" not in body[:at], kernel
+            assert "residual" not in body[:at], kernel
         else:
             assert body.lstrip().startswith("chain_begin("), kernel
+        check_before_the_wait(kernel, body)
 
 
 def test_scopes_end_with_the_pass():
