@@ -378,10 +378,13 @@ __device__ __forceinline__ void pdl_launch_dependents() {}
 __device__ __forceinline__ void pdl_wait() {}
 #endif
 
-// First statement of every kernel that is launched through lcc::chained (launch.h): wait until the kernel before it in the stream is
-// complete and its writes are visible, then let the kernel behind it be set up. Nothing but weights is read before. As every kernel of a
-// chain waits, a predecessor being complete means that all before it are. No-ops for ordinary launches. (Letting the next kernel in before
-// the wait fills the SMs with kernels that only wait: a step of the recurrent design 254 us instead of 231.)
+// In every kernel that is launched through lcc::chained (launch.h): wait until the kernel before it in the stream is complete and its writes
+// are visible, then let the kernel behind it be set up. As every kernel of a chain waits, a predecessor being complete means that all before
+// it are. No-ops for ordinary launches. (Letting the next kernel in before the wait fills the SMs with kernels that only wait: a step of the
+// recurrent design 254 us instead of 231.) It is a kernel's first statement, or stands behind the set-up of barriers and tensor memory. In front
+// of it nothing is stored to global memory: the kernel in front may still read there. Nor is anything loaded but weights and, in
+// scan_step_kernel, the state: what is loaded early has its writer at least two kernels back, since the kernel in front, which
+// may still run, let this one in only after its own wait. A CTA that stores or returns early waits by itself (chain_wait) in front of the store.
 __device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Such a kernel is on the SMs while the one before it still writes, so the non-coherent path (ld.global.nc, __ldg, and what the compiler

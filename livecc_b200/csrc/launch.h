@@ -49,7 +49,7 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
 }
 
 // A chain of short kernels: inside a ChainScope each may be set up while the one before it in the stream still runs (programmatic dependent
-// launch), and its first statement, chain_begin() in common.cuh, waits for that one. A step of the hybrid models is 30 (recurrent design, four layers) and 22
+// launch), and chain_begin() in common.cuh, by which it begins, waits for that one. A step of the hybrid models is 30 (recurrent design, four layers) and 22
 // kernels of 2 to 10 us on one row; as ordinary graph nodes, kernels that return at once cost 2.7 to 4 us each. Chained, and with the first
 // weights of a linear layer loaded before the wait, a prompt of 128 tokens and 31 replayed steps took 8.29 ms for 8.48 (recurrent design, then
 // 45 kernels a step) and 4.86 for 5.14 (routed, two layers), one step launched by the host 0.32 ms for 0.38 and 0.33 for 0.36 (four layers each).

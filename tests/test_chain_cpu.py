@@ -56,7 +56,6 @@ EARLY_LOADS = {
     "scan_step_kernel": {"a.conv_w", "a.conv_b", "a.dt_bias", "a.a_log", "a.skip", "a.norm_w", "a.carry", "a.state"},
     # the form with windows reads its sequence's scalars; it is launched in the ordinary way (test_prompt_attention_is_launched_in_the_ordinary_way)
     "attn_prefill_tc_kernel": {"lp.pos.finished", "lp.pos.kv_len"},
-    "vit_attn_tc_kernel": {"p.cu_seqlens"},               # written at the start of the pass: layer norm, product and rotary lie between
 }
 
 
