@@ -519,29 +519,42 @@ ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
     }
     float wmax = 0.f;
     for (float v : ww) wmax = std::max(wmax, fabsf(v));
-    int up = 14;                                             // weights times 2^up stay below half of fp16's range; their low parts are normal numbers
+    int up = 14;                                             // weights times 2^up stay below half of fp16's range
     while (up > -14 && ldexpf(wmax, up) > 32768.f) --up;
     std::vector<__half> frag((size_t)nts * ks * 32 * 8, __float2half_rn(0.f));
-    double split = 0, lo_abs = 0, aw = 0, sum_lo = 1e9, sum_hi = -1e9;
+    // The width pass off its true sums. PTX promises of an mma step products and sums of at least single precision, in an order and with a rounding of the
+    // hardware's choice, so no one form is taken for granted: a step of n products that are not zero, whose magnitudes add up to S with the addend's, is at most
+    // (n + 4) units in the last of S's 24 bits off. That covers fp32 adds one by one in any order (n), however they round or cut, addends aligned to the
+    // largest and cut behind 24 bits, all at once (n + 1, and 1 for the sum) or half by half (n + 2, and 2). The products are exact (11 x 8 bits). What the
+    // hardware does with subnormal operands is left open too: there are none.
+    const double scale = ldexp(1.0, -up);
+    double f_w = 0, sum_lo = 1e9, sum_hi = -1e9;
+    auto normal = [](float v) { return fabsf(v) < 6.103515625e-05f ? 0.f : v; };
     for (int X = 0; X < W; ++X) {
         const int nt = X >> 3, g = X & 7;
-        double es = 0, el = 0, ea = 0, sum = 0;
+        double off = 0, so_far = 0, sum = 0, hs = 0, ls = 0;    // of this k-step: magnitudes of the high and of the low parts
+        int n = 0;
         for (int j = 0; j < nw[X]; ++j) {
             const float v = ww[(size_t)j * W + X], sv = ldexpf(v, up);
-            const __half hi = __float2half_rn(sv), lo = __float2half_rn(sv - __half2float(hi));
+            const __half hi = __float2half_rn(normal(sv)), lo = __float2half_rn(normal(sv - __half2float(hi)));
             const int col = xw[X] + j - win[nt], k = col >> 4, tig = (col & 15) >> 2, b = col & 3;
             __half* f = &frag[(((size_t)nt * ks + k) * 32 + g * 4 + tig) * 8];
             f[b] = hi; f[4 + b] = lo;
-            es += fabs((double)sv - (double)__half2float(hi) - (double)__half2float(lo));
-            el += fabs((double)__half2float(lo));
-            ea += fabs((double)v); sum += v;
+            const double h = __half2float(hi), l = __half2float(lo);
+            off += 128 * scale * fabs((double)sv - h - l);      // bytes minus 128 are -128 .. 127
+            hs += scale * fabs(h); ls += scale * fabs(l); sum += v;
+            ++n;
+            if (j + 1 == nw[X] || ((col + 1) & 15) == 0) {      // (128.1: with the errors up to here)
+                off += (n + 4) * 2 * (half_ulp(128.1 * (hs + ls)) + half_ulp(128.1 * ls));
+                so_far += hs + ls;
+                if (so_far > hs + ls) off += half_ulp(128.1 * so_far);      // the fp32 add of the steps before
+                hs = ls = 0; n = 0;
+            }
         }
-        split = std::max(split, ldexp(es, -up)); lo_abs = std::max(lo_abs, ldexp(el, -up)); aw = std::max(aw, ea);
+        f_w = std::max(f_w, off);
         sum_lo = std::min(sum_lo, sum); sum_hi = std::max(sum_hi, sum);
     }
-    // ---- bound: stated sums off the true ones, the kernel's sums off the true ones, and 128 standing for 128 times the sums of the weights. An mma
-    // step multiplies exactly, aligns its 17 addends to the largest, cuts what lies 24 bits below that one's first, and rounds or cuts the sum once more
-    // (Fasi, Higham, Mikaitis, Pranesh 2021, "Numerical behavior of NVIDIA tensor cores"; 80,000 random steps here stayed below 1/6 of that).
+    // ---- bound: stated sums off the true ones, the kernel's sums off the true ones, and 128 standing for 128 times the sums of the weights
     double e_w = 0, ah = 0, hs_lo = 1e9, hs_hi = -1e9, e_h = 0, f_h = 0;
     double v_lo = 1e9, v_hi = -1e9;      // range of the width pass over bytes
     for (int X = 0; X < W; ++X) {
@@ -557,7 +570,6 @@ ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
         e_h = std::max(e_h, order_error(&wh[y], H, nh[y], v_lo - e_w, v_hi + e_w));
         f_h = std::max(f_h, order_error(&wh[y], H, nh[y], v_lo - 128.01, v_hi - 127.99));
     }
-    const double f_w = 128.0 * split + ks * 2 * (17 * half_ulp(128 * (wmax + lo_abs)) + half_ulp(128 * (aw + lo_abs)) + 18 * half_ulp(128 * lo_abs)) + ks * half_ulp(128 * aw);
     const double off = 128.0 * std::max(std::max(fabs(sum_lo * hs_lo - 1), fabs(sum_hi * hs_hi - 1)), std::max(fabs(sum_lo * hs_hi - 1), fabs(sum_hi * hs_lo - 1)));
     const double bound = 1.02 * (e_w * ah + e_h + f_w * ah + f_h + off) + 1e-6;
 
