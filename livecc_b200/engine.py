@@ -106,13 +106,10 @@ class LiveCCB200ForConditionalGeneration:
         while self.max_nsplit < 64 and 2 * self.max_nsplit * t.num_key_value_heads <= 2 * self.ctx.num_sms:
             self.max_nsplit *= 2
         self.nsplit = self.max_nsplit
-        # per-phase device time of the last generate() (CUDA events on the launch stream) and running totals. A call's events are read when somebody
-        # asks, or while the next call runs: reading them takes the host longer than a launch, and the device would wait for it
-        self._last_stats = {}
-        self._phase_ms_total = {"vit": 0.0, "prefill": 0.0, "decode": 0.0, "calls": 0, "decode_steps": 0}
-        self._unread_call = None
+        self.last_stats = {}
+        # per-phase device time of the last generate() (CUDA events on the launch stream) and running totals
+        self.phase_ms_total = {"vit": 0.0, "prefill": 0.0, "decode": 0.0, "calls": 0, "decode_steps": 0}
         self._ev = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
-        self._ev_spare = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
 
     @classmethod
     def from_synthetic(cls, config: LiveCCConfig, seed: int = 1234, device="cuda"):
@@ -217,28 +214,6 @@ class LiveCCB200ForConditionalGeneration:
     def new_cache(self) -> PagedKVCache:
         return PagedKVCache(self.pool)
 
-    @property
-    def last_stats(self) -> dict:
-        self._read_events()
-        return self._last_stats
-
-    @property
-    def phase_ms_total(self) -> dict:
-        self._read_events()
-        return self._phase_ms_total
-
-    def _read_events(self):
-        """Device times of the last finished generate(), if they have not been read yet."""
-        if self._unread_call is None:
-            return
-        ev, stats = self._unread_call
-        self._unread_call = None
-        ph = [ev[i].elapsed_time(ev[i + 1]) for i in range(3)]
-        self._last_stats = {**stats, "vit_ms": ph[0], "prefill_ms": ph[1], "decode_ms": ph[2]}
-        tot = self._phase_ms_total
-        tot["vit"] += ph[0]; tot["prefill"] += ph[1]; tot["decode"] += ph[2]
-        tot["calls"] += 1; tot["decode_steps"] += max(stats["generated"] - 1, 0)
-
     def _sampling(self, repetition_penalty, logits_processor, max_new_tokens) -> _cabi.Sampling:
         thr_token, thr_base, thr_step = -1, 0.0, 0.0
         for proc in logits_processor or []:
@@ -325,9 +300,6 @@ class LiveCCB200ForConditionalGeneration:
             raise TypeError(f"generate() got unsupported arguments {sorted(unsupported)}")
         self._check_common(pixel_values, image_grid_thw, do_sample, max_new_tokens)
         sp = self._sampling(repetition_penalty, logits_processor, max_new_tokens)
-        if self._unread_call is not None and self._unread_call[0] is self._ev_spare:
-            self._read_events()                                   # (a call in between ended in an error)
-        self._ev, self._ev_spare = self._ev_spare, self._ev       # the last call's events may still be unread
         stream = torch.cuda.current_stream(self.device)
         self._ev[0].record(stream)
         rec = self._begin_stream(input_ids, pixel_values_videos, video_grid_thw, past_key_values, video_frames, sp,
@@ -359,12 +331,17 @@ class LiveCCB200ForConditionalGeneration:
             self._run_decode([cache], [st], sp, n_steps, nsplit, logits_hist)
 
         self._ev[3].record(stream)
-        # while the device works: the times of the call before, and what the caller gets of this one
-        self._read_events()
+        # while the device works: what the caller gets, and the tower's time if that is over (reading a pair of events takes the host 6 us)
         self._take_results(rec, max_new_tokens, logits_hist)
+        vit_ms = self._ev[0].elapsed_time(self._ev[1]) if self._ev[1].query() else None
         # ---- one host sync per generate(): read the stream scalars ----
         out = self._finish_stream(rec, cache.scalars.tolist(), logits_out, output_logits)
-        self._unread_call = (self._ev, {"prefill_tokens": rec["S"], "generated": rec["n_gen"], "kv_len": cache.seq_len})
+        ph = [vit_ms if i == 0 and vit_ms is not None else self._ev[i].elapsed_time(self._ev[i + 1]) for i in range(3)]
+        self.last_stats = {"prefill_tokens": rec["S"], "generated": rec["n_gen"], "kv_len": cache.seq_len, "vit_ms": ph[0],
+                           "prefill_ms": ph[1], "decode_ms": ph[2]}
+        tot = self.phase_ms_total
+        tot["vit"] += ph[0]; tot["prefill"] += ph[1]; tot["decode"] += ph[2]
+        tot["calls"] += 1; tot["decode_steps"] += max(rec["n_gen"] - 1, 0)
         return out if return_dict_in_generate else out.sequences
 
     @torch.inference_mode()
@@ -418,8 +395,7 @@ class LiveCCB200ForConditionalGeneration:
         for b, r in enumerate(recs):
             lo = [first_logits[b]] if output_logits else None
             outs.append(self._finish_stream(r, scal[b], lo, output_logits))
-        self._read_events()
-        tot = self._phase_ms_total
+        tot = self.phase_ms_total
         tot["prefill"] += t_ev[0].elapsed_time(t_ev[1]); tot["decode"] += t_ev[1].elapsed_time(t_ev[2])
         tot["calls"] += B; tot["decode_steps"] += max(max(r["n_gen"] for r in recs) - 1, 0)
         return outs

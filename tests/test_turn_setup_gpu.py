@@ -53,3 +53,15 @@ def test_ids_of_other_types_and_strides_and_the_times_of_a_call():
         assert m.generate(ids, max_new_tokens=1) is not None and m.last_stats["prefill_ms"] > 0
     m.phase_ms_total["calls"] = 0
     assert m.phase_ms_total["calls"] == 0
+
+
+def test_the_times_of_a_call_are_there_when_it_returns_and_can_be_replaced():
+    m = LiveCCB200ForConditionalGeneration.from_synthetic(LiveCCConfig.small())
+    ids = torch.randint(5, 900, (1, 20))
+    held = m.phase_ms_total
+    for n in (1, 2):
+        m.generate(ids, max_new_tokens=3)
+        assert held["calls"] == n and held["decode_steps"] == 2 * n and held["prefill"] > 0
+    m.phase_ms_total, m.last_stats = {k: 0 for k in held}, {}
+    m.generate(ids, max_new_tokens=3)
+    assert m.phase_ms_total["calls"] == 1 and m.last_stats["generated"] == 3 and held["calls"] == 2
