@@ -289,8 +289,9 @@ class Context:
     def stream_ptr():
         import torch
 
-        # (torch.cuda.current_stream() builds a stream object: 4 us for a number)
-        return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+        # (torch.cuda.current_stream() builds a stream object: 4 us for a number. The short way is not part of torch's public interface.)
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        return C.c_void_p(raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream)
 
     def turn_setup(self, turns):
         """turns: up to 8 tuples (ids [L] int64 contiguous, seq, pos3 [3, S] int32 or None, pos_base, scalars, eight values); per turn

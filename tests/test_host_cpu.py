@@ -392,3 +392,16 @@ def test_model_wrappers_pass_as_many_arguments_as_the_header_declares(monkeypatc
     assert len(calls) == 7
     for name, nargs in calls:
         assert nargs + 1 == declared(name), (name, nargs + 1, declared(name))  # + the model / ctx handle
+
+
+def test_stream_without_torchs_private_call(monkeypatch):
+    """The launch stream comes from torch's public interface where its internal shortcut is missing."""
+    import types
+
+    import torch
+
+    from livecc_b200._cabi import Context
+
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: types.SimpleNamespace(cuda_stream=4711))
+    assert Context.stream_ptr().value == 4711
