@@ -53,9 +53,8 @@ int resize_aa_taps(int in_size, int out_size) {
     return (int)ceilf(support) * 2 + 1;
 }
 
-int resize_aa_table(int in_size, int out_size, int32_t* xmin_out, int32_t* xsize_out, float* weights) {
-    const int taps = resize_aa_taps(in_size, out_size);
-    if (taps < 0) return -1;
+// Windows and weights, [out_size][taps].
+static void aa_columns(int in_size, int out_size, int taps, int32_t* xmin_out, int32_t* xsize_out, float* weights) {
     float scale, support, invscale;
     aa_scale(in_size, out_size, scale, support, invscale);
     for (int i = 0; i < out_size; ++i) {
@@ -69,18 +68,29 @@ int resize_aa_table(int in_size, int out_size, int32_t* xmin_out, int32_t* xsize
         if (xsize < 0) xsize = 0;
         if (xsize > taps) xsize = taps;
         float total = 0.0f;
-        for (int j = 0; j < taps; ++j) weights[(size_t)j * out_size + i] = 0.0f;  // tap-major: [taps][out]
+        float* col = weights + (size_t)i * taps;
+        for (int j = (int)xsize; j < taps; ++j) col[j] = 0.0f;
         for (int j = 0; j < (int)xsize; ++j) {
             const float d = (float)(j + xmin) - center;
             const float w = cubic_weight((float)(((double)d + 0.5) * (double)invscale));
-            weights[(size_t)j * out_size + i] = w;
+            col[j] = w;
             total += w;
         }
         if (total != 0.0f)
-            for (int j = 0; j < (int)xsize; ++j) weights[(size_t)j * out_size + i] /= total;
+            for (int j = 0; j < (int)xsize; ++j) col[j] /= total;
         xmin_out[i] = (int32_t)xmin;
         xsize_out[i] = (int32_t)xsize;
     }
+}
+
+int resize_aa_table(int in_size, int out_size, int32_t* xmin_out, int32_t* xsize_out, float* weights) {
+    const int taps = resize_aa_taps(in_size, out_size);
+    if (taps < 0) return -1;
+    std::vector<float> cols((size_t)out_size * taps);
+    aa_columns(in_size, out_size, taps, xmin_out, xsize_out, cols.data());
+    for (int x0 = 0; x0 < out_size; x0 += 16)      // tap-major, in squares that stay in the cache
+        for (int j = 0; j < taps; ++j)
+            for (int x = x0; x < std::min(x0 + 16, out_size); ++x) weights[(size_t)j * out_size + x] = cols[(size_t)x * taps + j];
     return 0;
 }
 
@@ -457,19 +467,38 @@ struct ResizePlan {
 static SmemAttrOnce g_resize_smem[5][2];
 
 // Largest error of rounding (2: of cutting) a number of magnitude up to m to 24 bits: half (one) unit in the last place of m.
-static double half_ulp(double m) { return m > 0 ? ldexp(1.0, std::ilogb(m) - 24) : 0; }
+// (By the exponent's bits: a plan asks some 100,000 times. m is 0 or far from double's limits.)
+static double half_ulp(double m) {
+    uint64_t u;
+    memcpy(&u, &m, 8);
+    u &= 0x7ff0000000000000ull;
+    memcpy(&m, &u, 8);
+    return m * 0x1p-24;
+}
+
+// A float as fp16, rounded to nearest even, by its bits; `back` is its value. 0 stands for what would be subnormal; magnitudes are below 2^15.
+static uint16_t to_half(float v, float* back) {
+    uint32_t u;
+    if (fabsf(v) < 0x1p-14f) v = 0.f;
+    memcpy(&u, &v, 4);
+    const uint32_t r = (u & 0x7fffffffu) + 0xfffu + (u >> 13 & 1), kept = r & ~0x1fffu;
+    const uint32_t whole = v == 0.f ? 0u : kept | (u & 0x80000000u);
+    memcpy(back, &whole, 4);
+    return v == 0.f ? 0 : (uint16_t)((kept >> 13) - (112 << 10) | (u >> 16 & 0x8000u));
+}
 
 // |stated sum - sum without rounding| of an axis, over values in lo .. hi: every product and every sum rounds (the fused steps round once for both).
-static double order_error(const float* wt, int stride, int n, double lo, double hi) {
+static double order_error(const float* wt, int n, double lo, double hi) {
     double e = 0, top = 0, low = 0;      // range of the partial sum
     for (int j = 0; j < n; ++j) {
-        const double w = wt[(size_t)j * stride], a = w * lo, b = w * hi;
+        const double w = wt[j], a = w * lo, b = w * hi;
         top += std::max(a, b); low += std::min(a, b);
         if (j < ((n - 1) >> 2 << 2) + 1) e += half_ulp(std::max(fabs(a), fabs(b)));
-        if (j > 0) e += half_ulp(std::max(top, -low) + e);
+        if (j > 0) e += half_ulp(1.001 * std::max(top, -low));      // (with the errors up to here: fewer than 1000 terms)
     }
     return e;
 }
+
 
 ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
     if (h <= 0 || w <= 0 || H <= 0 || W <= 0 || w > (1 << 15) || h > (1 << 15) || W > (1 << 14) || H > (1 << 14)) return nullptr;
@@ -479,9 +508,9 @@ ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
     if (W == 1 && h != H) return nullptr;
     const int tw_taps = resize_aa_taps(w, W), th_taps = resize_aa_taps(h, H);
     std::vector<int32_t> xw(W), nw(W), xh(H), nh(H);
-    std::vector<float> ww((size_t)tw_taps * W), wh((size_t)th_taps * H);
-    if (resize_aa_table(w, W, xw.data(), nw.data(), ww.data()) || resize_aa_table(h, H, xh.data(), nh.data(), wh.data()))
-        return nullptr;
+    std::vector<float> cw((size_t)((W + 127) & ~127) * tw_taps, 0.f), rw((size_t)H * th_taps);    // weights column by column (padded to whole tiles) and row by row
+    aa_columns(w, W, tw_taps, xw.data(), nw.data(), cw.data());
+    aa_columns(h, H, th_taps, xh.data(), nh.data(), rw.data());
     auto row_windows = [&](int th, std::vector<int32_t>& r0s, std::vector<int32_t>& nrs) {
         int m = 1;
         r0s.clear(); nrs.clear();
@@ -518,29 +547,30 @@ ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
         ks = std::max(ks, (hi - win[nt] + 15) / 16);
     }
     float wmax = 0.f;
-    for (float v : ww) wmax = std::max(wmax, fabsf(v));
+    for (float v : cw) wmax = std::max(wmax, fabsf(v));
     int up = 14;                                             // weights times 2^up stay below half of fp16's range
     while (up > -14 && ldexpf(wmax, up) > 32768.f) --up;
-    std::vector<__half> frag((size_t)nts * ks * 32 * 8, __float2half_rn(0.f));
+    std::vector<uint16_t> frag((size_t)nts * ks * 32 * 8, 0);
     // The width pass off its true sums. PTX promises of an mma step products and sums of at least single precision, in an order and with a rounding of the
     // hardware's choice, so no one form is taken for granted: a step of n products that are not zero, whose magnitudes add up to S with the addend's, is at most
     // (n + 4) units in the last of S's 24 bits off. That covers fp32 adds one by one in any order (n), however they round or cut, addends aligned to the
     // largest and cut behind 24 bits, all at once (n + 1, and 1 for the sum) or half by half (n + 2, and 2). The products are exact (11 x 8 bits). What the
     // hardware does with subnormal operands is left open too: there are none.
     const double scale = ldexp(1.0, -up);
+    const float raise = ldexpf(1.f, up);
     double f_w = 0, sum_lo = 1e9, sum_hi = -1e9;
-    auto normal = [](float v) { return fabsf(v) < 6.103515625e-05f ? 0.f : v; };
     for (int X = 0; X < W; ++X) {
         const int nt = X >> 3, g = X & 7;
         double off = 0, so_far = 0, sum = 0, hs = 0, ls = 0;    // of this k-step: magnitudes of the high and of the low parts
         int n = 0;
         for (int j = 0; j < nw[X]; ++j) {
-            const float v = ww[(size_t)j * W + X], sv = ldexpf(v, up);
-            const __half hi = __float2half_rn(normal(sv)), lo = __float2half_rn(normal(sv - __half2float(hi)));
+            const float v = cw[(size_t)X * tw_taps + j], sv = v * raise;
             const int col = xw[X] + j - win[nt], k = col >> 4, tig = (col & 15) >> 2, b = col & 3;
-            __half* f = &frag[(((size_t)nt * ks + k) * 32 + g * 4 + tig) * 8];
-            f[b] = hi; f[4 + b] = lo;
-            const double h = __half2float(hi), l = __half2float(lo);
+            uint16_t* f = &frag[(((size_t)nt * ks + k) * 32 + g * 4 + tig) * 8];
+            float hi, lo;
+            f[b] = to_half(sv, &hi);
+            f[4 + b] = to_half(sv - hi, &lo);
+            const double h = hi, l = lo;
             off += 128 * scale * fabs((double)sv - h - l);      // bytes minus 128 are -128 .. 127
             hs += scale * fabs(h); ls += scale * fabs(l); sum += v;
             ++n;
@@ -559,16 +589,18 @@ ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
     double v_lo = 1e9, v_hi = -1e9;      // range of the width pass over bytes
     for (int X = 0; X < W; ++X) {
         double lo = 0, hi = 0;
-        for (int j = 0; j < nw[X]; ++j) { const double v = 255.0 * ww[(size_t)j * W + X]; (v < 0 ? lo : hi) += v; }
+        const float* c = &cw[(size_t)X * tw_taps];
+        for (int j = 0; j < nw[X]; ++j) { const double v = 255.0 * c[j]; (v < 0 ? lo : hi) += v; }
         v_lo = std::min(v_lo, lo); v_hi = std::max(v_hi, hi);
-        e_w = std::max(e_w, order_error(&ww[X], W, nw[X], 0.0, 255.0));
+        e_w = std::max(e_w, order_error(c, nw[X], 0.0, 255.0));
     }
     for (int y = 0; y < H; ++y) {
         double a = 0, s = 0;
-        for (int j = 0; j < nh[y]; ++j) { a += fabs((double)wh[(size_t)j * H + y]); s += wh[(size_t)j * H + y]; }
+        const float* r = &rw[(size_t)y * th_taps];
+        for (int j = 0; j < nh[y]; ++j) { a += fabs((double)r[j]); s += r[j]; }
         ah = std::max(ah, a); hs_lo = std::min(hs_lo, s); hs_hi = std::max(hs_hi, s);
-        e_h = std::max(e_h, order_error(&wh[y], H, nh[y], v_lo - e_w, v_hi + e_w));
-        f_h = std::max(f_h, order_error(&wh[y], H, nh[y], v_lo - 128.01, v_hi - 127.99));
+        e_h = std::max(e_h, order_error(r, nh[y], v_lo - e_w, v_hi + e_w));
+        f_h = std::max(f_h, order_error(r, nh[y], v_lo - 128.01, v_hi - 127.99));
     }
     const double off = 128.0 * std::max(std::max(fabs(sum_lo * hs_lo - 1), fabs(sum_hi * hs_hi - 1)), std::max(fabs(sum_lo * hs_hi - 1), fabs(sum_hi * hs_lo - 1)));
     const double bound = 1.02 * (e_w * ah + e_h + f_w * ah + f_h + off) + 1e-6;
@@ -590,12 +622,16 @@ ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
         m = (m + 15 + 3 + 15) >> 4;    // behind a phase of up to 15, and the word that a last word may be cut from
         return (m | 1) << 4;
     };
+    std::vector<std::pair<int, int>> heights;      // rows per CTA, the source rows they cover
+    for (int th : {32, 16, 8, 4, 2, 1}) {
+        const int t = th_override > 0 ? th_override : th;
+        heights.push_back({t, row_windows(t, rr0, rnr)});
+        if (th_override > 0) break;
+    }
     for (int TW : {128, 64, 32, 16, 8}) {
         const int stride = columns(TW);
-        for (int th : {32, 16, 8, 4, 2, 1}) {
-            if (th_override > 0 && th != 32) break;
-            const int t = th_override > 0 ? th_override : th;
-            const int rows = row_windows(t, rr0, rnr), rows16 = (rows + 15) & ~15;
+        for (auto [t, rows] : heights) {
+            const int rows16 = (rows + 15) & ~15;
             const size_t sm = (size_t)rows16 * (stride + (TW + 8) * 4) + ((size_t)tw_taps * TW + ((size_t)th_taps + 1) * t * 2 + 2 * TW + 1) * 4;
             if (sm > kSmem) continue;
             const double ctas = 6.0 * ((W + TW - 1) / TW) * ((H + t - 1) / t), occ = std::min<double>(4, floor(228.0 * 1024 / (sm + 1024)));
@@ -618,12 +654,10 @@ ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
     pl->row_tiles = (int)rr0.size(); pl->col_tiles = (int)cc0.size();
     pl->smem = best.smem;
     // tables: weights column by column (padded to whole tiles) and row by row (each twice), {first tap, taps} pairs
-    std::vector<float> flt((size_t)pl->col_tiles * best.tw * tw_taps + (size_t)H * th_taps * 2, 0.f);
     const size_t o_wh = (size_t)pl->col_tiles * best.tw * tw_taps;
-    for (int j = 0; j < tw_taps; ++j)
-        for (int X = 0; X < W; ++X) flt[(size_t)X * tw_taps + j] = ww[(size_t)j * W + X];
-    for (int j = 0; j < th_taps; ++j)
-        for (int y = 0; y < H; ++y) flt[o_wh + ((size_t)y * th_taps + j) * 2] = flt[o_wh + ((size_t)y * th_taps + j) * 2 + 1] = wh[(size_t)j * H + y];
+    std::vector<float> flt(o_wh + (size_t)H * th_taps * 2);
+    memcpy(flt.data(), cw.data(), o_wh * 4);
+    for (size_t i = 0; i < rw.size(); ++i) flt[o_wh + 2 * i] = flt[o_wh + 2 * i + 1] = rw[i];
     std::vector<int32_t> ints;
     auto put = [&](const std::vector<int32_t>& v) { size_t o = ints.size(); ints.insert(ints.end(), v.begin(), v.end()); return o; };
     auto pairs = [&](const std::vector<int32_t>& a, const std::vector<int32_t>& b) {
@@ -632,7 +666,7 @@ ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
         return o;
     };
     const size_t o_tw = pairs(xw, nw), o_th = pairs(xh, nh), o_c0 = put(cc0), o_cl = put(clen), o_r0 = put(rr0), o_rn = put(rnr), o_wi = put(win);
-    const size_t fb = frag.size() * sizeof(__half), wb = flt.size() * 4, bytes = fb + wb + ints.size() * 4;   // (operands and weights: 16-byte, pairs: 8-byte boundaries)
+    const size_t fb = frag.size() * 2, wb = flt.size() * 4, bytes = fb + wb + ints.size() * 4;   // (operands and weights: 16-byte, pairs: 8-byte boundaries)
     if (cudaMalloc(&pl->dev, bytes) != cudaSuccess) { delete pl; return nullptr; }
     std::vector<uint8_t> host(bytes);
     memcpy(host.data(), frag.data(), fb);

@@ -138,3 +138,36 @@ def test_every_form_of_the_width_products(ctx, h, w, H, W):
     assert torch.equal(ctx.resize_bicubic_aa_u8(clip.cuda(), (H, W)).cpu(), want)
     half = torch.from_numpy(resize_aa.resize_bicubic_aa_u8(check.contiguous().numpy(), (max(h // 2, 2), max(w // 2, 2))))
     assert torch.equal(ctx.resize_bicubic_aa_u8(check.contiguous().cuda(), (max(h // 2, 2), max(w // 2, 2))).cpu(), half)
+
+
+@pytest.mark.parametrize("h,w,H,W", [(1080, 1920, 448, 796), (2160, 3840, 448, 796)])
+def test_a_plan_costs_little_more_than_its_weight_tables(ctx, h, w, H, W):
+    """A size that is met once pays for its plan. Bound: twice the two weight tables for the operands and the error bound, and 150 us for memory and upload.
+    (With an exponent and a power of two by library calls for every tap it took five times the tables.)"""
+    import ctypes as C
+    import time
+
+    lib = ctx.lib
+
+    def least(f):
+        best = 1e9
+        for _ in range(15):
+            t = time.perf_counter()
+            made = f()
+            best = min(best, time.perf_counter() - t)
+            if made:
+                lib.lcc_resize_plan_destroy(C.c_void_p(made))
+        return best * 1e6
+
+    def tables():
+        for n, m in ((w, W), (h, H)):
+            buf = np.empty(m * lib.lcc_resize_aa_taps(n, m), np.float32)
+            at = np.empty((2, m), np.int32)
+            assert lib.lcc_resize_aa_table(n, m, at[0].ctypes.data_as(C.c_void_p), at[1].ctypes.data_as(C.c_void_p), buf.ctypes.data_as(C.c_void_p)) == 0
+
+    def plan():
+        return lib.lcc_resize_plan_create(C.c_void_p(ctx.handle), h, w, H, W, 0)
+
+    kept = plan()      # (its block of device memory serves the others: a fresh one costs the driver some 400 us)
+    assert least(plan) < 3 * least(tables) + 150
+    lib.lcc_resize_plan_destroy(C.c_void_p(kept))
