@@ -126,7 +126,7 @@ struct ResizeParams {
     int taps_w, taps_h, th, tw_log2;    // output rows per CTA, log2 of its columns (8 to 128)
     int rows16;            // staged rows, multiple of 16
     int stride;            // bytes between staged rows (odd multiple of 16: eight rows' words fall into 32 banks)
-    int dense;             // pixels of a warp's 256 up to which the warp sums them one by one (negative: the bound settles nothing)
+    int dense;             // pixels of a warp's 256 up to which the warp sums them one by one (negative: the stated order throughout)
 };
 
 // float(u8) without the quarter-rate I2F: 0x4B000000 | u is the float 2^23 + u (exact), minus 2^23.
@@ -714,6 +714,10 @@ int resize_bicubic_aa_u8(const ResizePlan* pl, const uint8_t* src, int planes, u
     p.win = pl->win; p.frag = pl->frag; p.frag_scale = pl->frag_scale; p.bound = pl->bound; p.ks = pl->ks;
     p.taps_w = pl->taps_w; p.taps_h = pl->taps_h; p.th = pl->th; p.tw_log2 = pl->tw_log2; p.rows16 = pl->rows16; p.stride = pl->stride; p.dense = pl->dense;
     const dim3 grid(pl->col_tiles, pl->row_tiles, planes);
+    // Both axes enlarged (5 taps) and CTAs of one wave (4 per SM): the stated order throughout has fewer steps behind one another than products, test and doubtful
+    // pixels. One frame, products | stated: 360x640 -> 448x796 7.8 | 6.8 us, 300x400 -> 560x784 8.3 | 7.7; two 10.7 | 10.3 and 13.0 | 12.0; three (more
+    // than a wave) 13.8 | 14.2 and 15.9 | 16.1. With an axis made smaller: 480x640 -> 280x784 7.5 | 8.0, 480x854 -> 448x796 8.2 | 8.9.
+    if (pl->taps_w <= 5 && pl->taps_h <= 5 && (size_t)grid.x * grid.y * grid.z <= 4 * kSms) p.dense = -1;
     const bool w4 = ((p.w | (int)reinterpret_cast<uintptr_t>(src)) & 3) == 0;   // every row starts on a word boundary
     switch (pl->ks) {
         case 1: return w4 ? resize_launch<1, true>(p, grid, pl->smem, s) : resize_launch<1, false>(p, grid, pl->smem, s);

@@ -171,3 +171,16 @@ def test_a_plan_costs_little_more_than_its_weight_tables(ctx, h, w, H, W):
     kept = plan()      # (its block of device memory serves the others: a fresh one costs the driver some 400 us)
     assert least(plan) < 3 * least(tables) + 150
     lib.lcc_resize_plan_destroy(C.c_void_p(kept))
+
+
+@pytest.mark.parametrize("h,w,H,W,frames", [(360, 640, 448, 796, (1, 2, 3)), (97, 61, 112, 140, (1, 49, 50)), (28, 28, 28, 28, (1,)), (64, 200, 65, 140, (1, 60))])
+def test_both_sides_of_the_rule_for_enlarged_pictures_of_one_wave(ctx, h, w, H, W, frames):
+    """Enlarged pictures whose CTAs are one wave take the stated order throughout, larger calls (and an axis made smaller) the products: the same bytes."""
+    from oracle import resize_aa
+
+    clip = make_clip("one_wave", max(frames), h, w)
+    clip[:, :, ::2] = 255 * (clip[:, :, ::2] > 127)          # also values on the edge of the range
+    for n in frames:
+        out = ctx.resize_bicubic_aa_u8(clip[:n].cuda(), (H, W)).cpu()
+        for t in {0, n - 1}:
+            assert np.array_equal(out[t].numpy(), resize_aa.resize_bicubic_aa_u8(clip[t:t + 1].numpy(), (H, W))[0]), (n, t)
