@@ -34,7 +34,7 @@ struct Grp {
     const void* gate = nullptr;     // the store multiplies by sigmoid(gate[row, z * gate_stride + column]) (no lists)
     int ld_gate = 0;
     int64_t gate_stride = 0;
-    float cap = 0.f, inv_cap = 0.f, scale = 0.f;   // scale != 0 (logits, few-row kernel): the store holds cap * tanh(v / cap) * scale (no cap: v * scale)
+    float cap = 0.f, inv_cap = 0.f, scale = 0.f;   // logits (few-row kernel, LOGITS): the store holds cap * tanh(v / cap) * scale (no cap: v * scale)
     float* copy = nullptr;                         // ... and a second time here, rows as in C
 };
 template <typename T>
@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(256) linear_tile_kernel(const T* __restrict__ 
 // recurrent layers of width 2048 took 10.93 ms and take 8.68 ms, of two routed layers 6.34 and 5.06 ms.
 // KS: warps that share a group of columns, each with every KS-th piece of k; their sums meet in shared memory in a fixed order. A warp of one column reads
 // as much of A from L1 as of W from memory and unpacks both; two columns and half of k halve that with the same loads in flight.
+// LOGITS: the store caps, scales and copies (a form of its own: tanh in every fp32 store cost the others registers, two rows of 16 x 8448 26 us for 12).
 // Scalar loads when K or a row start is not 16-byte aligned.
 constexpr int kRowsMax = kLogitRows;
 template <typename T> struct Vec16;
@@ -129,7 +130,7 @@ template <> struct Vec16<float> {
     }
 };
 
-template <typename T, typename TC, bool VEC, int MM, int WR, int WU, bool GLU = false, int KS = 1>
+template <typename T, typename TC, bool VEC, int MM, int WR, int WU, bool GLU = false, int KS = 1, bool LOGITS = false>
 __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ A, int lda, const T* __restrict__ W, int ldw,
                                                           const float* __restrict__ bias, TC* __restrict__ C, int ldc, int M_all,
                                                           int N, int K, Grp g) {
@@ -260,22 +261,18 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const T* __restrict__ 
 #pragma unroll
                 for (int i = 1; i < KS; ++i) v += sums[KS > 1 ? warp + i : 0][r * MM + m];
                 if (lane != 0 || n >= N) continue;
-                if constexpr (std::is_same<TC, float>::value) {
-                    if (g.scale != 0.f) {
-                        const float lg = (g.cap > 0.f ? g.cap * tanhf(v * g.inv_cap) : v) * g.scale;
-                        C[(size_t)m * ldc + n] = lg;
-                        if (g.copy) g.copy[(size_t)(mb + m) * ldc + n] = lg;
-                        continue;
-                    }
-                }
-                stf(C + (size_t)m * ldc + n, gated<T>(act_of(v + (bias ? bias[n] : 0.f), g.act), g, z, mb + m, n));
+                if constexpr (LOGITS) {
+                    const float lg = (g.cap > 0.f ? g.cap * tanhf(v * g.inv_cap) : v) * g.scale;
+                    C[(size_t)m * ldc + n] = lg;
+                    if (g.copy) g.copy[(size_t)(mb + m) * ldc + n] = lg;
+                } else stf(C + (size_t)m * ldc + n, gated<T>(act_of(v + (bias ? bias[n] : 0.f), g.act), g, z, mb + m, n));
             }
         }
     }
     }
 }
 
-template <typename T, typename TC>
+template <typename T, typename TC, bool LOGITS = false>
 int launch_linear(const void* A, int lda, const void* W, int ldw, const float* bias, void* C, int ldc, int M, int N, int K,
                   cudaStream_t s, int groups = 1, Grp g = Grp{0, 0, 0, nullptr, nullptr, ACT_NONE, 0, 0, 0, 0.f}, int M_total = 0,
                   void* glu_tmp = nullptr, int ld_tmp = 0) {
@@ -294,8 +291,8 @@ int launch_linear(const void* A, int lda, const void* W, int ldw, const float* b
     do {                                                                                                                       \
         constexpr int per = (WARPS) / (KSN) * (GLUB ? 1 : WRN);                                                                \
         const dim3 grid((N + per - 1) / per, grid_y);                                                                          \
-        if (vec) chained(linear_rows_kernel<T, TC, true, MMN, WRN, WUN, GLUB, KSN>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g); \
-        else chained(linear_rows_kernel<T, TC, false, MMN, WRN, WUN, GLUB, KSN>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g);    \
+        if (vec) chained(linear_rows_kernel<T, TC, true, MMN, WRN, WUN, GLUB, KSN, LOGITS && !(GLUB)>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g); \
+        else chained(linear_rows_kernel<T, TC, false, MMN, WRN, WUN, GLUB, KSN, LOGITS && !(GLUB)>, grid, WARPS * 32, 0, s)((const T*)A, lda, (const T*)W, ldw, bias, (TC*)C, ldc, M, N, K, g);    \
     } while (0)
 #define LCC_ROWS(MMN, WRN, WUN, WARPS, GLUB) LCC_ROWS_KS(MMN, WRN, WUN, WARPS, GLUB, 1)
         if (g.glu_F > 0) {
@@ -375,8 +372,8 @@ int linear_logits(int dt, const void* A, int lda, const void* W, int ldw, float*
     if (!A || !W || !C || M < 1 || M > kRowsMax || N < 1 || K < 1 || lda < K || ldw < K || ldc < N || scale == 0.f) return -2;
     Grp g{0, 0, 0, nullptr, nullptr, ACT_NONE, 0, 0, 0, 0.f};
     g.cap = cap > 0.f ? cap : 0.f; g.inv_cap = cap > 0.f ? 1.f / cap : 0.f; g.scale = scale; g.copy = copy;
-    if (dt == DT_F32) return launch_linear<float, float>(A, lda, W, ldw, nullptr, C, ldc, M, N, K, s, 1, g);
-    return launch_linear<bf16, float>(A, lda, W, ldw, nullptr, C, ldc, M, N, K, s, 1, g);
+    if (dt == DT_F32) return launch_linear<float, float, true>(A, lda, W, ldw, nullptr, C, ldc, M, N, K, s, 1, g);
+    return launch_linear<bf16, float, true>(A, lda, W, ldw, nullptr, C, ldc, M, N, K, s, 1, g);
 }
 
 int linear_grouped(const GroupedLinear& q, cudaStream_t s) {
