@@ -306,30 +306,46 @@ int launch_linear(const void* A, int lda, const void* W, int ldw, const float* b
             }
         }
         // Wide matrices: for one row a column per warp and CTAs of 4 warps, which leave and arrive in small portions; two columns and 8 warps for
-        // more rows. Narrower ones with 1024 to 6144 k (bf16): warps share columns, four by four in matrices of up to 4096 columns, two by two above (one
-        // column for more rows), so that the whole matrix is in flight at once. The rule does not look at M: neither do a row's bits. (Wide matrices two
-        // by two would save one row another us but cost four rows 20 % and eight 25 %: twice the sums across lanes. Longer k, 2048 x 8448, filled
-        // the SMs in front of the attention that runs beside it: a routed step of four sequences 435 us, 394 so, 404 before.) One row in a step,
-        // before | now, us: 2048 columns x 4096: 6.4 | 3.6; 2048 x 5632: 11.0 | 7.0; 2048 x 2048: 4.5 | 3.0; 6208 x 2048: 6.6 | 5.4;
-        // 10304 x 2048: 10.3 | 9.4; 32768 x 2048: 24.4 | 21.0. Steps of 2, 4 and 8 sequences: recurrent 372, 668, 1140 | 285, 541, 870.
+        // more rows. Narrower ones: warps share columns, four by four or two by two, so that the whole matrix is in flight at once. How many share
+        // depends on the matrix alone, never on M: so do a row's bits. Sharing pays where k is long against what it costs (sums that meet in shared
+        // memory) and the columns do not fill the chip by themselves. One | two | four | eight rows in bf16, each warp its own columns -> so, us, products
+        // chained as in a step: by four 64 x 2048 2.8 -> 1.8 | 4.7 -> 2.2 | 9.4 -> 4.1 | 16.1 -> 6.2, 2048 x 4096 6.2 -> 4.1 | 10.5 -> 5.8 | 19.6 -> 16.9 |
+        // 34.0 -> 26.2, 4096 x 4096 12.4 -> 7.5 | 12.1 -> 11.8 | 38.3 -> 26.6 | 64.4 -> 39.7; by two 2048 x 1024 2.7 -> 2.5 | 4.3 -> 4.0 | 6.8 -> 6.2 | 11.1 -> 9.0,
+        // 6208 x 2048 8.4 -> 6.9 | 11.4 -> 10.2 | 21.6 -> 21.9 | 36.3 -> 33.4. It is not free everywhere inside the lines: 4096 x 2048 by two
+        // 4.4 -> 4.2 | 6.2 -> 7.5 | 20.5 -> 16.5 | 34.7 -> 25.1, 3000 x 2048 4.3 -> 3.8 | 6.2 -> 4.7 | 11.8 -> 13.5 | 19.3 -> 21.4. Beyond the lines: by four
+        // 2048 x 1024 2.8 | 3.4 | 10.0 | 14.4, 4096 x 2048 5.1 | 6.9 | 18.0 | 26.4; by two 6208 x 1024 5.2 | 6.5 | 15.9 | 22.7 for 5.6 | 8.3 | 13.0 | 21.0. In fp32,
+        // which costs half as much to unpack, by four 2048 x 2048 3.7 -> 3.5 | 5.8 -> 4.7 | 18.6 -> 15.1 | 28.6 -> 19.7, 2560 x 1024 3.0 -> 2.8 | 3.6 -> 4.3.
+        // Longer k in bf16, 2048 x 8448, filled the SMs in front of the attention that runs beside it: a routed step of four sequences 435 us for 404.
+        // U: what a warp reads of a row of W at once.
+        constexpr int U = 32 * V;
+        constexpr bool F32 = sizeof(T) == 4;
+        const bool shared_k = !g.row_off && (F32 || K <= 24 * U);
+        const bool by4 = shared_k && ((N <= 1024 && K >= 4 * U) || (N <= (F32 ? 2048 : 18 * kSms) && K >= 8 * U) || (!F32 && N <= 4608 && K >= 16 * U));
+        const bool by2 = shared_k && K >= (N <= 2048 ? 4 : 6) * U;
+        // waves of CTAs in a form that has room for so many columns per SM (by its registers). Eight rows: one of 16 columns costs 4/3 of one of 12
+        auto waves = [&](int per_sm) { return (N + per_sm * kSms - 1) / (per_sm * kSms); };
         if (N >= 8192) {
             if (mm == 1) LCC_ROWS(1, 1, 8, 4, false);
             else if (mm <= 2) LCC_ROWS(2, 2, 8, 8, false);
             else LCC_ROWS(8, 2, 4, 8, false);
-        } else if (!g.row_off && K >= 4 * 32 * V && K <= 24 * 32 * V && N <= 4096) {
-            if (mm == 1 && K <= 8 * 32 * V) LCC_ROWS_KS(1, 4, 2, 4, false, 4);
-            else if (mm == 1 && K <= 16 * 32 * V) LCC_ROWS_KS(1, 4, 4, 4, false, 4);
-            else if (mm == 1) LCC_ROWS_KS(1, 4, 6, 4, false, 4);
-            else if (mm <= 2) LCC_ROWS_KS(2, 1, 4, 4, false, 4);
+        } else if (by4) {
+            if (mm == 1 && K <= 8 * U) LCC_ROWS_KS(1, 2, 2, 4, false, 4);
+            else if (mm == 1) LCC_ROWS_KS(1, 2, 4, 4, false, 4);
+            else if (mm <= 2 && N > 1024 && N <= 2048) LCC_ROWS_KS(2, 2, 2, 4, false, 4);
+            else if (mm <= 2 && N <= 1024 && K > 8 * U && (!F32 || N > 256)) LCC_ROWS_KS(2, 1, 4, 4, false, 4);
+            else if (mm <= 2) LCC_ROWS_KS(2, 1, 2, 4, false, 4);
+            else if (N > 6 * kSms && N <= 8 * kSms) LCC_ROWS_KS(8, 2, 2, 4, false, 4);     // one wave of two columns in place of two of one: 1024 x 2048 8.5 -> 6.2 us
             else LCC_ROWS_KS(8, 1, 2, 4, false, 4);
-        } else if (!g.row_off && K >= 4 * 32 * V && K <= 24 * 32 * V) {
+        } else if (by2) {
             if (mm == 1) LCC_ROWS_KS(1, 2, 4, 4, false, 2);
-            else if (mm <= 2) LCC_ROWS_KS(2, 1, 4, 4, false, 2);
+            else if (mm <= 2 && (F32 ? waves(24) <= waves(32) : waves(24) == 1)) LCC_ROWS_KS(2, 2, 4, 4, false, 2);
+            else if (mm <= 2) LCC_ROWS_KS(2, F32 ? 2 : 1, F32 ? 2 : 4, 4, false, 2);
+            else if (F32 || 4 * waves(16) < 3 * waves(12)) LCC_ROWS_KS(8, 2, 2, 4, false, 2);
             else LCC_ROWS_KS(8, 1, 4, 4, false, 2);
-        } else if (mm == 1 && K > 8 * 32 * V) {
+        } else if (mm == 1 && K > 8 * U && N <= 2048) {
             LCC_ROWS(1, 1, 16, 2, false);
         } else if (mm == 1) {
-            LCC_ROWS(1, 1, 8, 2, false);
+            LCC_ROWS(1, 1, 8, 2, false);          // (16 loads a lane above 2048 columns: 4096 x 3072 11.1 us for 6.9)
         } else if (mm <= 2) {
             LCC_ROWS(2, 1, 8, 2, false);
         } else {

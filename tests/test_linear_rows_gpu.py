@@ -13,8 +13,10 @@ pytestmark = pytest.mark.gpu
 
 
 # k of a product (the model's width, the feed-forward's) around 1024, 2048, 4096 and 6144 in bf16 and half of that in fp32; columns (vocabulary, 2 x ff)
-# around 4096 and 8192
-@pytest.mark.parametrize("width,ff,vocab", [(512, 1016, 4095), (520, 2048, 4097), (1016, 2056, 8191), (1024, 4096, 8193), (1032, 4104, 4096), (2048, 6144, 8192), (264, 6152, 333)])
+# around 888, 1024, 1184, 2048, 2664, 4096, 4608 and 8192
+@pytest.mark.parametrize("width,ff,vocab", [(512, 1016, 4095), (520, 2048, 4097), (1016, 2056, 8191), (1024, 4096, 8193), (1032, 4104, 4096), (2048, 6144, 8192), (264, 6152, 333),
+                                            (1024, 2048, 888), (1024, 2056, 896), (1024, 1032, 1184), (1032, 4096, 1192), (2048, 512, 2664), (2048, 4096, 2672),
+                                            (4096, 1024, 4608), (4096, 1016, 4616), (2056, 264, 2048)])
 def test_products_at_the_limits_of_their_forms(width, ff, vocab):
     from livecc_b200.seq_engine import SeqLMForCausalLM
 
