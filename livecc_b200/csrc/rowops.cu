@@ -366,8 +366,9 @@ __global__ void __launch_bounds__(256) gated_group_norm_kernel(const float* __re
 
 // Groups of 129 to 1024 columns whose rows allow 16-byte reads of y: four neighbouring columns per thread and load, everything in flight
 // together, one pass; a warp per (row, group), 128 threads above 256 columns (a warp alone takes 6.9 us for one row of 8 groups of 512,
-// 128 threads 4.1, the general form above 4.6). 2048 rows of 4096 in groups of 512: 24 us, 45 in the general form; a warp per group takes 23 once there are more
-// groups than CTAs of 128 threads fit on the chip (16 per SM): it needs no barrier, and sums each quarter of the group and then the quarters as those do, so that
+// 128 threads 4.1, the general form above 4.6). 2048 rows of 4096 in groups of 512: 24 us, 45 in the general form; a warp per group takes 23 once there are clearly
+// more groups than CTAs of 128 threads fit on the chip (16 per SM; from 20 per SM: 2400 groups 6.8 us and 7.9 by warps, 3000 the same, 4096 10.0 and 8.0): it needs
+// no barrier, and sums each quarter of the group and then the quarters as those do, so that
 // a row's bits do not depend on how many rows there are.
 template <typename T, int TEAM, int E>
 __global__ void __launch_bounds__(TEAM == 32 ? 64 : TEAM) gated_group_norm4_kernel(const float* __restrict__ y, int ld_y, const T* __restrict__ gate,
@@ -953,7 +954,7 @@ int gated_group_norm(int dt, const float* y, int ld_y, const void* gate, int ld_
                                                                            (bf16*)out, ld_out, S, n, group, gate_first, eps);   \
     } while (0)
         if (group <= 256) LCC_GGN4(32, 2);
-        else if (group <= 512 && teams > 16 * kSms) LCC_GGN4(32, 4);
+        else if (group <= 512 && teams > 20 * kSms) LCC_GGN4(32, 4);
         else if (group <= 512) LCC_GGN4(128, 1);
         else LCC_GGN4(128, 2);
 #undef LCC_GGN4

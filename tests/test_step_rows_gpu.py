@@ -100,13 +100,31 @@ def test_groups_of_the_gated_norm(heads, vdim, groups):
 
 @pytest.mark.parametrize("heads,vdim", [(4, 128), (4, 65)])
 def test_gated_norm_has_the_same_bits_for_few_and_many_rows(heads, vdim):
-    """8 groups of rows: 2400 and more (row, group) pairs go a warp to a group, fewer a CTA; both sum in one order. The scan in front is cut at the same
+    """8 groups of rows: more than 2960 (row, group) pairs go a warp to a group, fewer a CTA; both sum in one order. The scan in front is cut at the same
     blocks of 64 rows, and the products behind one row alone are those of many on the CUDA cores (fp32 storage)."""
     from livecc_b200.seq_engine import SeqLMForCausalLM
 
     d = seq_cases.config([seq_cases.ssd(heads=8 * heads, vdim=vdim, state=8, groups=1, norm_groups=8)], width=24, vocab=40)
     cfg = SeqModelConfig.from_json(d)
     m = SeqLMForCausalLM.from_state_dict(cfg, synthetic_seq_tensors(cfg, seed=5), "float32", max_tokens=512)
-    toks = seq_cases.tokens(330, 40, seed=vdim)
-    many, few = run(m, toks, [320]), run(m, toks, [128, 256, 320])
-    assert torch.equal(many[:320], few[:320])
+    toks = seq_cases.tokens(394, 40, seed=vdim)
+    many, few = run(m, toks, [384]), run(m, toks, [128, 256, 384])
+    assert torch.equal(many[:384], few[:384])
+
+
+@pytest.mark.parametrize("rows,width", [(296, 260), (297, 260), (297, 1028), (297, 1030), (1184, 2052), (1185, 2052)])
+@pytest.mark.parametrize("branches", [1, 2])
+def test_post_norms_with_and_without_kept_weights(rows, width, branches):
+    """Rows from which the norms' weights are no longer kept in registers, in rows of one, two and four pieces, on and off 4-column boundaries."""
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    layer = (seq_cases.ssd(heads=2, vdim=8, state=8, groups=1, norm_groups=1) if branches == 1 else
+             seq_cases.par(**(dict(heads=2, kv_heads=1, dim=10, vdim=8) if width % 4 else dict(heads=4, kv_heads=2, dim=16, vdim=8)), ff=None))
+    d = seq_cases.config([layer], width=width, vocab=70)
+    cfg = SeqModelConfig.from_json(d)
+    t = synthetic_seq_tensors(cfg, seed=3)
+    toks = seq_cases.tokens(rows, 70, seed=width)
+    want, _ = O.forward(d, t, toks)
+    for dtype, tol in (("float32", F32_TOL), ("bfloat16", BF16_TOL)):
+        m = SeqLMForCausalLM.from_state_dict(cfg, t, dtype, max_tokens=2048)
+        assert rel(run(m, toks, [rows]), want) < tol
