@@ -176,7 +176,8 @@ template <> __device__ __forceinline__ void row4<bf16>(const bf16* p, float (&v)
 }
 
 // One CTA per new row. EQ > 0: rows on 4-element boundaries with at most EQ * 256 pieces of four query columns and 256 of key columns; everything
-// the row needs is loaded at once and stays in registers. (One row of 16 + 2 heads of 128: 6.2 us in place of a step's chain element by element, 2.3 so.)
+// the row needs is loaded at once and stays in registers. (One row of 16 + 2 heads of 128: 6.2 us in place of a step's chain element by element, 2.3 so.
+// 2048 rows of 3 + 1 heads of 20: 8.7 us with two pieces a thread, 6.9 with one.)
 template <typename T, int EQ>
 __global__ void __launch_bounds__(256) qk_norm_kv_append_kernel(const T* __restrict__ proj, int ld, const float* __restrict__ qn_w,
                                                                 const float* __restrict__ kn_w, float eps, float* __restrict__ q_out,
@@ -1444,7 +1445,8 @@ int qk_norm_kv_append(int dt, const void* proj, int ld, const float* qn_w, const
             chained(qk_norm_kv_append_kernel<bf16, E>, S, 256, 0, s)((const bf16*)proj, ld, qn_w, kn_w, eps, q_out, (bf16*)k_pages,       \
                                                                      (bf16*)v_pages, page_table, page_size, S, Hq, G, D, DV, pos);        \
     } while (0)
-    if (vec && nq <= 2048) LCC_QKN(2);
+    if (vec && nq <= 1024) LCC_QKN(1);
+    else if (vec && nq <= 2048) LCC_QKN(2);
     else if (vec && nq <= 4096) LCC_QKN(4);
     else LCC_QKN(0);
 #undef LCC_QKN

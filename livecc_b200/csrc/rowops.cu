@@ -474,7 +474,8 @@ __device__ __forceinline__ float norm_apply(const NormSpec& n, float v, float rn
 }
 
 // One CTA per wanted row. E: pieces of V columns per thread, kept in registers (0: wider rows are read again in each pass). One row of 2048 columns in a
-// step: 5.8 us with single columns and a pass over memory for the sum and one for the result, 3.6 so.
+// step: 5.8 us with single columns and a pass over memory for the sum and one for the result, 3.6 so. (No more pieces than a row has: 2048 rows of 64 columns
+// 4.2 us with two, 3.8 with one.)
 template <typename T, int E, bool VEC>
 __global__ void __launch_bounds__(256) gather_norm_kernel(const float* __restrict__ x32, const int* __restrict__ rows, NormSpec n,
                                                           T* __restrict__ out, int W) {
@@ -867,8 +868,8 @@ int embed_sinusoid(int dt, const int64_t* ids, const int* seq_len, const void* t
                    const float* inv_freq, float* x32, void* xa, int S, int W, SeqPos pos, cudaStream_t s, int copies) {
     if (!ids || !table || !x32 || S < 1 || W < 1 || copies < 1) return -2;
     count_launch();
-    // (up to 148 rows the chip is not full: there a column per thread is the shorter chain)
-    if (S > kSms && (W % 4) == 0 && (((uintptr_t)table | (uintptr_t)x32 | (uintptr_t)xa | (uintptr_t)inv_freq) % 16) == 0) {
+    // (up to 148 rows the chip is not full: there a column per thread is the shorter chain. Below 256 columns most threads would have nothing: 1024 x 64 2.2 us for 2.6)
+    if (S > kSms && W >= 256 && (W % 4) == 0 && (((uintptr_t)table | (uintptr_t)x32 | (uintptr_t)xa | (uintptr_t)inv_freq) % 16) == 0) {
         if (dt == DT_F32)
             chained(embed_sinusoid4_kernel<float>, S, 256, 0, s)(ids, seq_len, (const float*)table, vocab, scale, inv_freq, x32, (float*)xa, S, W, pos, copies);
         else
@@ -1040,7 +1041,9 @@ int gather_norm(int dt, const float* x32, const int* rows, const NormSpec& n, vo
         else chained(gather_norm_kernel<bf16, E, VECB>, n_rows, 256, 0, s)(x32, rows, n, (bf16*)out, W);                  \
     } while (0)
 #define LCC_GN(E) do { if (vec) LCC_GN2(E, true); else LCC_GN2(E, false); } while (0)
-    if (pieces <= 2) LCC_GN(2);
+    if (pieces <= 1) LCC_GN(1);
+    else if (pieces <= 2) LCC_GN(2);
+    else if (pieces <= 4) LCC_GN(4);
     else if (pieces <= 8) LCC_GN(8);
     else LCC_GN(0);
 #undef LCC_GN

@@ -69,7 +69,7 @@ def test_cap_and_scale_of_many_rows_equal_those_of_one(rows, vocab, cap, scale):
 
 
 # either side of the rows from which the embedding takes four columns per thread, widths off 4 and past a pass of 1024; norm groups of a warp: up to 128, 256, 512, and past it
-@pytest.mark.parametrize("rows,width", [(148, 24), (149, 24), (149, 255), (150, 1028)])
+@pytest.mark.parametrize("rows,width", [(148, 24), (149, 24), (149, 255), (150, 1028), (149, 252), (149, 256), (148, 256), (150, 260)])
 def test_embedding_of_many_rows(rows, width):
     from livecc_b200.seq_engine import SeqLMForCausalLM
 
