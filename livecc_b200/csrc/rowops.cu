@@ -1,5 +1,6 @@
 // Row-wise ops of the hybrid decoder models. The residual stream, every norm and every sum of squares is fp32; `xa` /
 // `out` copies in the model's storage type feed the next linear layer.
+#include <limits.h>
 #include <math.h>
 
 #include <algorithm>
@@ -109,9 +110,10 @@ __device__ __forceinline__ float2 block_sum2(float a, float b, float* red) {
 // Two normed branches, averaged, behind a post-norm residual: one CTA per row. Rows of up to 256 * kRowCache pieces are read once
 // into registers (E pieces of V columns per thread, every load in flight together, the norms' weights too: behind a sum they would wait once more);
 // wider rows (E = 0) are re-read from L1/L2 in each of the three passes. One row of 2048 columns: 5.7 us in place of a step's chain with single
-// columns, weights loaded where they are used and a sum for each branch; 3.7 here.
+// columns, weights loaded where they are used and a sum for each branch; 3.7 here. KEEP: the weights are loaded first; with more than two rows per SM other
+// CTAs fill the wait and the registers cost more. Kept | not, us, bf16: 149 x 2048 3.3 | 3.9, 300 x 4096 6.5 | 6.0, 2048 x 512 11.6 | 7.4, 2048 x 2048 14.7 | 12.3.
 constexpr int kRowCache = 16;
-template <typename T, int E, bool VEC>
+template <typename T, int E, bool VEC, bool KEEP>
 __global__ void __launch_bounds__(256) postnorm_residual_kernel(float* __restrict__ x32, T* __restrict__ xa, const T* __restrict__ a,
                                                                 int ld_a, const float* __restrict__ wa, const T* __restrict__ b,
                                                                 int ld_b, const float* __restrict__ wb, const float* __restrict__ w,
@@ -125,21 +127,32 @@ __global__ void __launch_bounds__(256) postnorm_residual_kernel(float* __restric
     T* o = xa + (size_t)r * W;
     constexpr int V = VEC ? 4 : 1, EN = E > 0 ? E : 1;
     if (E > 0) {
-        float va[EN][V], vb[EN][V], vx[EN][V], ka[EN][V], kb[EN][V], kw[EN][V], sa = 0.f, sb = 0.f;
+        constexpr int KN = KEEP ? EN : 1;
+        float va[EN][V], vb[EN][V], vx[EN][V], ka[KN][V], kb[KN][V], kw[KN][V], sa = 0.f, sb = 0.f;
+        auto weights = [&](int i, int c) {
+            if (VEC) {
+                ld4(wa + c, (float(&)[4])ka[i % KN]); ld4(wb + c, (float(&)[4])kb[i % KN]);
+            } else {
+                ka[i % KN][0] = wa[c]; kb[i % KN][0] = wb[c];
+            }
+            if (KEEP) { if (VEC) ld4(w + c, (float(&)[4])kw[i % KN]); else kw[i % KN][0] = w[c]; }
+        };
 #pragma unroll
         for (int i = 0; i < EN; ++i) {
             const int c = (threadIdx.x + i * 256) * V;
             if (c < W) {
                 if (VEC) {
                     ld4(ar + c, (float(&)[4])va[i]); ld4(br + c, (float(&)[4])vb[i]); ld4(x + c, (float(&)[4])vx[i]);
-                    ld4(wa + c, (float(&)[4])ka[i]); ld4(wb + c, (float(&)[4])kb[i]); ld4(w + c, (float(&)[4])kw[i]);
                 } else {
                     va[i][0] = ldf(ar + c); vb[i][0] = ldf(br + c); vx[i][0] = x[c];
-                    ka[i][0] = wa[c]; kb[i][0] = wb[c]; kw[i][0] = w[c];
                 }
+                if (KEEP) weights(i, c);
             } else {
 #pragma unroll
-                for (int u = 0; u < V; ++u) va[i][u] = vb[i][u] = vx[i][u] = ka[i][u] = kb[i][u] = kw[i][u] = 0.f;
+                for (int u = 0; u < V; ++u) va[i][u] = vb[i][u] = vx[i][u] = 0.f;
+                if (KEEP)
+#pragma unroll
+                    for (int u = 0; u < V; ++u) ka[i % KN][u] = kb[i % KN][u] = kw[i % KN][u] = 0.f;
             }
         }
 #pragma unroll
@@ -150,20 +163,23 @@ __global__ void __launch_bounds__(256) postnorm_residual_kernel(float* __restric
         const float ra = 1.f / sqrtf(s.x / (float)W + eps), rb = 1.f / sqrtf(s.y / (float)W + eps);
         float ss = 0.f;
 #pragma unroll
-        for (int i = 0; i < EN; ++i)
+        for (int i = 0; i < EN; ++i) {
+            if (!KEEP) { const int c = (threadIdx.x + i * 256) * V; if (c >= W) continue; weights(i, c); }
 #pragma unroll
             for (int u = 0; u < V; ++u) {
-                const float m = 0.5f * (va[i][u] * ra * ka[i][u] + vb[i][u] * rb * kb[i][u]);
+                const float m = 0.5f * (va[i][u] * ra * ka[i % KN][u] + vb[i][u] * rb * kb[i % KN][u]);
                 vx[i][u] = fmaf(alpha, vx[i][u], m);
                 ss = fmaf(vx[i][u], vx[i][u], ss);
             }
+        }
         const float rn = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
 #pragma unroll
         for (int i = 0; i < EN; ++i) {
             const int c = (threadIdx.x + i * 256) * V;
             if (c >= W) continue;
+            if (!KEEP) { if (VEC) ld4(w + c, (float(&)[4])kw[0]); else kw[0][0] = w[c]; }
 #pragma unroll
-            for (int u = 0; u < V; ++u) vx[i][u] = vx[i][u] * rn * kw[i][u];
+            for (int u = 0; u < V; ++u) vx[i][u] = vx[i][u] * rn * kw[i % KN][u];
             if (VEC) { st4(x + c, (const float(&)[4])vx[i]); st4(o + c, (const float(&)[4])vx[i]); }
             else { x[c] = vx[i][0]; stf(o + c, vx[i][0]); }
         }
@@ -196,7 +212,7 @@ __global__ void __launch_bounds__(256) postnorm_residual_kernel(float* __restric
 // feed-forward's weighted sum of expert rows. ls: a factor per column, or null. The new row stays in registers between its sum of
 // squares and its store (E pieces of V columns per thread; E = 0: rows wider than 256 * 16 pieces keep it in x32). A column's sum runs in
 // the same order for every S.
-template <typename T, int E, bool VEC>
+template <typename T, int E, bool VEC, bool FEW>
 __global__ void __launch_bounds__(256) postnorm_branch_kernel(float* __restrict__ x32, T* __restrict__ xa, const T* __restrict__ a, int ld_a,
                                                               bool has_mc, MoeCombine mc, const float* __restrict__ ls,
                                                               const float* __restrict__ w, float alpha, float eps, int W) {
@@ -209,7 +225,7 @@ __global__ void __launch_bounds__(256) postnorm_branch_kernel(float* __restrict_
     float* x = x32 + (size_t)r * W;
     const int top = has_mc ? mc.top : 0;
     const bool cached = top <= kCombineTop;
-    constexpr bool KEEP = E > 0 && E <= 4;      // the norm's weights too (behind the sum they would wait once more)
+    constexpr bool KEEP = FEW && E > 0 && E <= 4;      // the norm's weights too (behind the sum they would wait once more)
     float vx[EN][V], kw[KEEP ? EN : 1][V];
     if (E > 0) {            // the residual row's loads fly while the routed row's places are read
 #pragma unroll
@@ -897,13 +913,17 @@ int postnorm_residual(int dt, float* x32, void* xa, const void* a, int ld_a, con
         auto ok4 = [&](const void* p, int ld) { return !p || ((ld % 4) == 0 && ((uintptr_t)p % (4 * es)) == 0); };
         const bool vec = (W % 4) == 0 && (((uintptr_t)x32 | (uintptr_t)w | (uintptr_t)ls) % 16) == 0 && ok4(a, ld_a) && ok4(xa, W) &&
                          (!mc || (ok4(m.eo, m.ld_eo) && ok4(m.so, m.ld_so)));
-#define LCC_PNB2(E, VECB)                                                                                                      \
+#define LCC_PNB3(E, VECB, FEWB)                                                                                                \
     do {                                                                                                                       \
-        if (dt == DT_F32) chained(postnorm_branch_kernel<float, E, VECB>, S, 256, 0, s)(x32, (float*)xa, (const float*)a, ld_a, mc != nullptr, m, ls, w, alpha, eps, W); \
-        else chained(postnorm_branch_kernel<bf16, E, VECB>, S, 256, 0, s)(x32, (bf16*)xa, (const bf16*)a, ld_a, mc != nullptr, m, ls, w, alpha, eps, W);                 \
+        if (dt == DT_F32) chained(postnorm_branch_kernel<float, E, VECB, FEWB>, S, 256, 0, s)(x32, (float*)xa, (const float*)a, ld_a, mc != nullptr, m, ls, w, alpha, eps, W); \
+        else chained(postnorm_branch_kernel<bf16, E, VECB, FEWB>, S, 256, 0, s)(x32, (bf16*)xa, (const bf16*)a, ld_a, mc != nullptr, m, ls, w, alpha, eps, W);                 \
     } while (0)
+#define LCC_PNB2(E, VECB) do { if (E > 0 && E <= 4 && (E == 1 || S <= few)) LCC_PNB3(E, VECB, true); else LCC_PNB3(E, VECB, false); } while (0)
 #define LCC_PNB(E) do { if (vec) LCC_PNB2(E, true); else LCC_PNB2(E, false); } while (0)
-        const int pieces = (W / (vec ? 4 : 1) + 255) / 256;      // per thread: the form depends on the row's width alone
+        const int pieces = (W / (vec ? 4 : 1) + 255) / 256;      // per thread: a row's sums depend on its width alone
+        // Rows from which weights that are kept cost more (registers: fewer CTAs) than they save. Kept | not, us: bf16 148 x 2048 2.0 | 2.3, 1024 x 2048 4.7 | 4.4,
+        // 1024 x 4096 7.9 | 9.1, 2048 x 4096 13.8 | 12.5; fp32 2048 x 2048 8.4 | 8.7, 1024 x 4096 9.1 | 10.6, 2048 x 4096 22.3 | 19.7; up to 1024 columns always kept.
+        const int few = pieces > 2 ? 8 * kSms : dt == DT_F32 ? INT_MAX : 2 * kSms;
         if (pieces <= 1) LCC_PNB(1);
         else if (pieces <= 2) LCC_PNB(2);
         else if (pieces <= 4) LCC_PNB(4);
@@ -912,24 +932,29 @@ int postnorm_residual(int dt, float* x32, void* xa, const void* a, int ld_a, con
         else LCC_PNB(0);
 #undef LCC_PNB
 #undef LCC_PNB2
+#undef LCC_PNB3
         return done();
     }
     auto row4 = [&](const void* p, int ld) { return (ld % 4) == 0 && ((uintptr_t)p % (dt == DT_F32 ? 16 : 8)) == 0; };
     const bool vec = (W % 4) == 0 && (((uintptr_t)x32 | (uintptr_t)w | (uintptr_t)wa | (uintptr_t)wb) % 16) == 0 && row4(a, ld_a) && row4(b, ld_b) && row4(xa, W);
-#define LCC_PNR2(E, VECB)                                                                                                   \
+#define LCC_PNR3(E, VECB, KEEPB)                                                                                            \
     do {                                                                                                                    \
         if (dt == DT_F32)                                                                                                   \
-            chained(postnorm_residual_kernel<float, E, VECB>, S, 256, 0, s)(x32, (float*)xa, (const float*)a, ld_a, wa, (const float*)b, ld_b, wb, w, alpha, eps, W); \
+            chained(postnorm_residual_kernel<float, E, VECB, KEEPB>, S, 256, 0, s)(x32, (float*)xa, (const float*)a, ld_a, wa, (const float*)b, ld_b, wb, w, alpha, eps, W); \
         else                                                                                                                \
-            chained(postnorm_residual_kernel<bf16, E, VECB>, S, 256, 0, s)(x32, (bf16*)xa, (const bf16*)a, ld_a, wa, (const bf16*)b, ld_b, wb, w, alpha, eps, W); \
+            chained(postnorm_residual_kernel<bf16, E, VECB, KEEPB>, S, 256, 0, s)(x32, (bf16*)xa, (const bf16*)a, ld_a, wa, (const bf16*)b, ld_b, wb, w, alpha, eps, W); \
     } while (0)
+#define LCC_PNR2(E, VECB) do { if (keep) LCC_PNR3(E, VECB, true); else LCC_PNR3(E, VECB, false); } while (0)
 #define LCC_PNR(E) do { if (vec) LCC_PNR2(E, true); else LCC_PNR2(E, false); } while (0)
     const int per = (W / (vec ? 4 : 1) + 255) / 256;
-    if (per <= 2) LCC_PNR(2);
+    const bool keep = S <= 2 * kSms;
+    if (per <= 1) LCC_PNR(1);
+    else if (per <= 2) LCC_PNR(2);
     else if (per <= 4) LCC_PNR(4);
-    else if (vec || per > kRowCache) LCC_PNR2(0, false);     // more than 4096 columns
+    else if (vec || per > kRowCache) LCC_PNR3(0, false, false);     // more than 4096 columns
     else if (per <= 8) LCC_PNR2(8, false);
     else LCC_PNR2(16, false);
+#undef LCC_PNR3
 #undef LCC_PNR2
 #undef LCC_PNR
     return done();
