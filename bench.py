@@ -42,7 +42,7 @@ def parse_args():
     ap.add_argument("--steps", type=int, default=3)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="native", choices=["native", "reference", "hf_gpu"],
-                    help="native: this repo; reference: the reference's CPU path (driver arm); hf_gpu: the reference's GPU "
+                    help="native: this repo; reference: the reference's CPU path; hf_gpu: the reference's GPU "
                          "path (HF bf16 + flash_attention_2, optionally --liger) on the same B200 = the kernel to beat")
     ap.add_argument("--liger", action="store_true", help="hf_gpu: apply_liger_kernel_to_qwen2_vl() first (REF/demo/infer.py:2-3)")
     ap.add_argument("--model", default="7b", choices=["7b", "small"])
@@ -234,19 +234,7 @@ def load_peaks():
     if os.path.exists(p):
         d = json.load(open(p))
         return float(d["hbm_gbs"]), "measured (MEASURED_PEAKS.json)"
-    return 6650.0, "fallback (B200_PROFILING.md)"
-
-
-def recorded_pool_peak():
-    """The driver-measured HBM figure BASELINE.md §2 quotes from MEASURED_PEAKS.json (GB/s), or None. Only used to annotate
-    the roofline blocks when MEASURED_PEAKS.json itself is absent from the snapshot (the fractions then use the fallback)."""
-    import re
-
-    try:
-        m = re.search(r"HBM copy bandwidth\s*\|\s*([0-9.]+)\s*GB/s", open(os.path.join(ROOT, "BASELINE.md")).read())
-        return float(m.group(1)) if m else None
-    except OSError:
-        return None
+    return 6650.0, "fallback"
 
 
 def time_gateup_kernel(eng, iters=5):
@@ -625,7 +613,7 @@ def main():
     traffic, traffic_src = None, None
     try:  # dram bytes of the same kernel from the committed `ncu --set full` capture (7B dims only)
         if args.model == "7b":
-            tr = json.load(open(os.path.join(ROOT, "profiles", "r01_gateup_ncu.json")))
+            tr = json.load(open(os.path.join(ROOT, "profiles", "early_gateup_ncu.json")))
             traffic = tr["dram_bytes_read"] + tr["dram_bytes_write"]
             traffic_src = "static: one `ncu --set full` capture of this kernel, not measured in this run"
     except Exception:
@@ -679,13 +667,6 @@ def main():
                              "bound": "hbm", "bytes_per_step_mean": int(bytes_avg), "ms_per_step": ms_per_dstep,
                              "achieved": bytes_avg / (ms_per_dstep / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                              "frac": bytes_avg / (ms_per_dstep / 1e3) / 1e9 / peak, "decode_steps": dsteps}
-    if peak_src.startswith("fallback"):
-        rec = recorded_pool_peak()
-        if rec:
-            note = (f"MEASURED_PEAKS.json absent: fractions use the {peak:.0f} GB/s fallback; against the driver-measured "
-                    f"{rec} GB/s recorded in BASELINE.md they are ")
-            line["roofline"]["peak_note"] = note + f"{line['roofline']['achieved'] / rec:.4f}"
-            line["roofline_step"]["peak_note"] = note + f"{line['roofline_step']['achieved'] / rec:.4f}"
     if not args.no_batch and world == 1:
         # multi-stream batching on one GPU: aggregate tokens/s of B concurrent streams over the same clip
         ms = {}

@@ -54,8 +54,8 @@ inline cudaError_t launch_kernel(void (*kern)(KArgs...), dim3 grid, dim3 block, 
 // weights of a linear layer loaded before the wait, a prompt of 128 tokens and 31 replayed steps took 8.29 ms for 8.48 (recurrent design, then
 // 45 kernels a step) and 4.86 for 5.14 (routed, two layers), one step launched by the host 0.32 ms for 0.38 and 0.33 for 0.36 (four layers each).
 // Matrix products, row kernels and attention of the vision tower and of a prefill are chained too: what they set up (barriers, tensor memory, tensor
-// maps) and their launch lie beside the kernel in front. A turn that reads 281 tokens behind 17 k 1.42 -> 1.32 ms, 24 behind 8 k 1.00 -> 0.84, eight
-// streams' prefill 2.0 -> 1.6, 1024 and 8192 patches 456 -> 442 and 980 -> 948 us, prompts of the hybrid models 1.72 -> 1.67 and 0.56 -> 0.525 ms.
+// maps) and their launch lie beside the kernel in front. A turn that reads 281 tokens behind 17 k 1.45 -> 1.39 ms, eight streams' turn 11.99 -> 11.93,
+// 1024 and 8192 patches 453 -> 440 and 1132 -> 1105 us, prompts of the hybrid models 1.72 -> 1.67 and 0.56 -> 0.525 ms.
 // A kernel that takes tensor memory takes it before it opens the door to the next one: that one could otherwise hold what this one waits for.
 // (The first stages' weights asked for before the wait changed little, turn by turn -1 to +0.6 %.) Prompt attention of the hybrid models (few and large
 // CTAs) stays outside: chained, its CTAs go where there is room while the kernel in front still holds the other SMs, and stay there two to an SM.

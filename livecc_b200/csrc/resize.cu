@@ -105,9 +105,10 @@ int resize_aa_table(int in_size, int out_size, int32_t* xmin_out, int32_t* xsize
 // The result r differs from the stated one by at most `bound` (plan: rounding errors of both, from the very tables). Where r is further than that from
 // every rounding boundary its byte is the stated one's. The other pixels (0.1 to 0.3 % of noise) are summed again in the stated order by the whole
 // warp, a lane per source row; where they are many (pictures that sit on a boundary) the whole tile is.
-// Two frames of 1080p -> 448x796: 18.2 us (stated order throughout: 32.8), six 45 (88), 360p -> 448x796 9.9 (13.1), three 1080p -> 140x140 36 (181); a
-// checkerboard at half size, every tile twice, 46 (33). What is left is latency (issue slots 55 % used): CTAs start (6 us), a lone warp's doubtful pixel
-// holds its CTA (4 us). No gain: CTAs that go through planes with two row buffers (21 us, less of them fit), 128 threads (21), those pixels without
+// Two frames of 1080p -> 448x796 replayed from a graph: 17.7 us (20 as a call of its own; with the filter on the CUDA cores 31.4), one 10.7 (17.7), six 43 (86),
+// 16 110 (222); two of 2160p 47 (139), of 1080p -> 140x140 24.5 (124), six of 360p -> 448x796 22.4 (30.5). A checkerboard of single pixels, where every
+// byte is in doubt and every tile is summed twice, 50 (32), at half size 35 (24); edges of 12 x 20 pixels 20.6. What is left is latency (issue slots 55 % used): CTAs start (6 us), a lone
+// warp's doubtful pixel holds its CTA (4 us). No gain: CTAs that go through planes with two row buffers (21 us, less of them fit), 128 threads (21), those pixels without
 // loops (19: code that runs once is fetched).
 struct ResizeParams {
     const uint8_t* src;
@@ -605,7 +606,8 @@ ResizePlan* resize_plan_create(int h, int w, int H, int W, int th_override) {
     const double off = 128.0 * std::max(std::max(fabs(sum_lo * hs_lo - 1), fabs(sum_hi * hs_hi - 1)), std::max(fabs(sum_lo * hs_hi - 1), fabs(sum_hi * hs_lo - 1)));
     const double bound = 1.02 * (e_w * ah + e_h + f_w * ah + f_h + off) + 1e-6;
 
-    // ---- tile: of those that fit, the one with the least estimated time for two frames. A CTA's instructions are counted, and some 2500 cycles of its
+    // ---- tile: of those that fit, the one with the least estimated time for two frames (of 20 tiles timed at eight sizes it is within 5 % of the best for two frames but
+    // for 1080p -> 140x140, 24.4 us for 22.1; one frame up to 1.2 times the best, 1.5 at 140x140; 16 frames up to 1.27 and 1.36). A CTA's instructions are counted, and some 2500 cycles of its
     // life (loads, two barriers) are no issue slots; at most 8 CTAs of an SM share its four schedulers.
     struct Tile { int tw, th, rows, rows16, stride; size_t smem; } best{};
     double best_t = 1e30;

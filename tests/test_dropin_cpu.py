@@ -1,4 +1,4 @@
-"""Executes the UNMODIFIED reference orchestrator (REF/demo/infer.py) under the import swap INTEGRATION.md §A
+"""Executes the UNMODIFIED reference orchestrator (REF/demo/infer.py) under the import swap of this package
 describes and diffs everything it does against livecc_b200.streaming.LiveCCDemoInfer: every generate() call
 (ids, cache length, pixel rows, kwargs incl. the ThresholdLogitsProcessor the canonical caller REF/demo/cli.py:16-19
 asks for), every yielded ((start, stop), text) and the `state` contract. The model is a deterministic recording mock
@@ -59,7 +59,7 @@ class RecordingModel:
 
 
 def _load_reference_class(cfg, model):
-    """REF/demo/infer.py imported verbatim with the module swap of INTEGRATION.md §A."""
+    """REF/demo/infer.py imported verbatim with the module swap."""
     real_tf = importlib.import_module("transformers")
     ours = importlib.import_module("livecc_b200.livecc_utils")
 

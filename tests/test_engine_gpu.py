@@ -214,7 +214,7 @@ def test_long_cache_split_kv_prefill(small):
 
 
 def test_gpu_frame_ingest_is_bit_identical(small):
-    """§8(f) rank 1: uint8 frames -> fused normalize+patchify kernel == host patchify + f32 rows, bit for bit
+    """uint8 frames -> fused normalize+patchify kernel == host patchify + f32 rows, bit for bit
     (video features and therefore logits), including an odd frame count (last frame repeated)."""
     cfg, sd, eng, rs = small
     from livecc_b200.processing import patchify_video

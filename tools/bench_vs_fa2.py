@@ -1,6 +1,6 @@
 """Head-to-head with "the kernel to beat": flash-attn 2 (the reference's attention,
 REF/demo/infer.py:46) vs the tcgen05/TMEM kernels of this repo at the
-§8 shapes, on the same B200, CUDA-event timed, L2 flushed between iterations. Writes a markdown table to stdout
+shapes of a streaming turn, on the same B200, CUDA-event timed, L2 flushed between iterations. Writes a markdown table to stdout
 (copy under profiles/). flash-attn is LIBRARY code used here only as the measured competitor."""
 import os
 import sys
