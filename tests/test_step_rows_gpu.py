@@ -128,3 +128,18 @@ def test_post_norms_with_and_without_kept_weights(rows, width, branches):
     for dtype, tol in (("float32", F32_TOL), ("bfloat16", BF16_TOL)):
         m = SeqLMForCausalLM.from_state_dict(cfg, t, dtype, max_tokens=2048)
         assert rel(run(m, toks, [rows]), want) < tol
+
+
+@pytest.mark.parametrize("width", [260, 1030, 1536])
+def test_post_norms_have_the_same_bits_for_few_and_many_rows(width):
+    """320 rows load the norms' weights behind the sums, 256 and 64 in front. The scans in front are cut at the same blocks of 64 rows, and the products in
+    fp32 storage are those of many rows on the CUDA cores."""
+    from livecc_b200.seq_engine import SeqLMForCausalLM
+
+    par = seq_cases.par(**(dict(heads=2, kv_heads=1, dim=10, vdim=8) if width % 4 else dict(heads=4, kv_heads=2, dim=16, vdim=8)), ff=None)
+    d = seq_cases.config([seq_cases.ssd(heads=2, vdim=8, state=8, groups=1, norm_groups=1), par], width=width, vocab=40)
+    cfg = SeqModelConfig.from_json(d)
+    m = SeqLMForCausalLM.from_state_dict(cfg, synthetic_seq_tensors(cfg, seed=5), "float32", max_tokens=512)
+    toks = seq_cases.tokens(320, 40, seed=width)
+    many, few = run(m, toks, [320]), run(m, toks, [256, 320])
+    assert torch.equal(many, few)
