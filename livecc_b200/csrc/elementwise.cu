@@ -236,9 +236,10 @@ __global__ void __launch_bounds__(TEAM) norm_rows_kernel(const bf16* __restrict_
 }
 
 // Many rows of up to 1536 columns: a warp per row needs no barrier. Its sums run as a team's above do, so a row's result does not depend on
-// the form. 8192 rows of 1280: 14.3 us, 18.4 as teams of 192; 1024 rows: 6.3 us (profiled), 4.7 as teams.
+// the form. 8192 rows of 1280: 14.3 us, 18.4 as teams of 192; 1024 rows: 6.3 us (profiled), 4.7 as teams. Four CTAs per SM: without the bound the layer
+// norm takes 80 registers, room for three (repeated 8.1 and 9.1 us, 4096 rows 5.2 and 6.7).
 template <bool RMS>
-__global__ void __launch_bounds__(256) norm_rows_warp_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w,
+__global__ void __launch_bounds__(256, 4) norm_rows_warp_kernel(const bf16* __restrict__ x, int ldx, const bf16* __restrict__ w,
                                                              const bf16* __restrict__ b, bf16* __restrict__ y, int ldy, int rows, int dim,
                                                              float eps) {
     chain_begin(x);
